@@ -170,3 +170,18 @@ def check(rc: int) -> None:
 
 def launch_count() -> int:
     return int(lib().light_b200_launch_count())
+
+
+class _MissingHost:
+    """Stands in for light_b200._host until it is built: any use is an error (there is no other path)."""
+
+    def __getattr__(self, name):
+        raise Light200Error(-100, f"{os.path.join(HERE, '_host.so')} is missing or does not load: run `python -m light_b200.build`")
+
+
+if os.path.exists(LIB_PATH) and os.path.exists(os.path.join(HERE, "_host.so")):
+    import torch  # noqa: F401  (its libraries are what _host.so links against)
+
+    from . import _host as host
+else:
+    host = _MissingHost()

@@ -1,4 +1,5 @@
-"""Builds liblight_b200.so in-tree with nvcc for sm_100a (the only target)."""
+"""Builds liblight_b200.so in-tree with nvcc for sm_100a (the only target), and _host.so, the native host path in
+front of its hot entry points (csrc/host.cpp), against the installed torch."""
 from __future__ import annotations
 
 import os
@@ -9,6 +10,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "liblight_b200.so")
+HOST = os.path.join(HERE, "_host.so")
 SOURCES = ["abi.cu", "gguf_dequant.cu", "gguf_matmul_generic.cu", "gguf_gemv_fast.cu", "gguf_gemv_batch.cu", "prefill_umma.cu", "decode_umma.cu", "int4.cu", "fp8_block.cu",
            "moe.cu", "peer_gather.cu", "decode_attn.cu", "norm_rope.cu", "w8a8.cu", "moe_route.cu", "decode_chain.cu", "gemv_bf16.cu", "moe_elementwise.cu", "gguf_decode_nt.cu", "gguf_decode_ts.cu"]
 NVCC_FLAGS = os.environ.get("LIGHT_B200_NVCC_EXTRA", "").split() + ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
@@ -56,7 +58,30 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link of liblight_b200.so failed")
+    build_host(force)
     return LIB
+
+
+def build_host(force: bool = False) -> str:
+    """Compiles csrc/host.cpp as the extension module light_b200._host, linked to liblight_b200.so beside it."""
+    import sysconfig
+
+    import torch
+
+    src = os.path.join(CSRC, "host.cpp")
+    if not (force or _stale(HOST, [src, os.path.join(HERE, "..", "include", "light_b200.h")])):
+        return HOST
+    inc = os.path.join(os.path.dirname(torch.__file__), "include")
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"), "-isystem", cuda, "-isystem", sysconfig.get_paths()["include"],
+           src, "-o", HOST, "-L" + libs, "-L" + HERE, "-l:liblight_b200.so", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("g++ failed on host.cpp")
+    return HOST
 
 
 if __name__ == "__main__":

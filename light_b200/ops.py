@@ -17,6 +17,7 @@ from typing import Optional, Sequence
 import torch
 
 from . import _lib
+from ._lib import host as _host
 from ._lib import BF16, F16, F32, Q4_0, Q4_K, Q5_0, Q5_K, Q6_K, Q8_0, Light200Error, MoeArgs  # noqa: F401
 
 GGUF_NAMES = {Q4_0: "Q4_0", Q5_0: "Q5_0", Q8_0: "Q8_0", Q4_K: "Q4_K", Q5_K: "Q5_K", Q6_K: "Q6_K"}
@@ -121,6 +122,7 @@ def ensure_workspace(device_index: int, nbytes: int) -> None:
     off = (-buf.data_ptr()) % 1024
     _lib.check(_lib.lib().light_b200_set_workspace(device_index, C.c_void_p(buf.data_ptr() + off), buf.numel() - 1024))
     _workspaces[device_index] = buf
+    _host.set_workspace(device_index, buf.numel() - 1024)
 
 
 def prefill_status(device_index: int = 0) -> int:
@@ -132,6 +134,10 @@ def prefill_status(device_index: int = 0) -> int:
 
 def MatMulQ(x: torch.Tensor, w: QTensor) -> torch.Tensor:
     """ops.MatMulQ (ops/matmul_q.go:27-75): out (M, N) f32 = x (M, K) f32 . dequant(w (N, K))^T."""
+    if len(w.shape) == 2 and x.dim() == 2:
+        y = _host.linear_q(x, w.data, w.ggml_type, w.shape[0], w.shape[1])
+        if y is not None:
+            return y
     if x.dim() != 2 or len(w.shape) != 2:
         raise ValueError(f"MatMulQ: want x (M,K) and w (N,K); got {tuple(x.shape)}, {tuple(w.shape)}")
     if x.dtype != torch.float32:
@@ -414,6 +420,10 @@ def MoEInt4(x: torch.Tensor, gate_up: Sequence[Int4], down: Sequence[Int4], rout
 
 def MatMulInt4(x: torch.Tensor, w: Int4) -> torch.Tensor:
     """ops.MatMulInt4 (ops/int4.go:66-127): x (M, K) F32 or BF16 -> (M, N) at x's dtype."""
+    if w.perm is None and x.dim() == 2:
+        y = _host.linear_int4(x, w.codes, w.scales, w.zeros, w.group)
+        if y is not None:
+            return y
     if x.dim() != 2 or x.shape[1] != w.K():
         raise ValueError(f"ops.MatMulInt4: x {tuple(x.shape)}, weight ({w.N()}, {w.K()})")
     if x.dtype not in (torch.float32, torch.bfloat16):
@@ -457,6 +467,10 @@ def DequantizeF8Block(w: torch.Tensor, scale: torch.Tensor, block_r: int, block_
 
 def MatMulF8Block(x: torch.Tensor, w: torch.Tensor, scale: torch.Tensor, block_r: int, block_c: int) -> torch.Tensor:
     """ops.MatMulF8Block (ops/fp8_block.go:165-233): x (M, K) F32 or BF16 -> (M, N) at x's dtype."""
+    if x.dim() == 2:
+        y = _host.linear_f8(x, w, scale, block_r, block_c)
+        if y is not None:
+            return y
     if x.dim() != 2 or w.dim() != 2 or x.shape[1] != w.shape[1]:
         raise ValueError(f"ops.MatMulF8Block: x {tuple(x.shape)}, w {tuple(w.shape)}")
     if x.dtype not in (torch.float32, torch.bfloat16):
@@ -647,6 +661,9 @@ def MoEGemmF8Block(x: torch.Tensor, w: torch.Tensor, scale: torch.Tensor, block_
 def MoECombine(pair_out: torch.Tensor, topk: int) -> torch.Tensor:
     """ops.MoECombine (ops/moe.go:206-240): sum of the topk slot rows, (M, N) -> (T, N), slot 0 first, every sum
     rounded to the tensor's dtype (the reference adds the slots one after the other with its Add kernel): one launch."""
+    y = _host.combine(pair_out, topk)
+    if y is not None:
+        return y
     M, N = pair_out.shape
     if M % topk:
         raise ValueError(f"moe_combine: {M} rows not divisible by topk {topk}")
@@ -683,6 +700,9 @@ def MoECombineWeighted(rows: torch.Tensor, index: Optional[torch.Tensor], weight
 def MoEGateMul(h: torch.Tensor, gelu: bool = False) -> torch.Tensor:
     """The step between the two grouped matmuls of a sparse block (nn/moe.go:206-224): h (M, 2 I) -> act(h[:, :I]) * h[:, I:],
     act SiLU or GELU-erf, the activation rounded to the tensor's dtype before the product: one launch."""
+    y = _host.gate_mul(h, gelu)
+    if y is not None:
+        return y
     if h.dim() != 2 or h.shape[1] % 16 or h.dtype not in _ACT:
         raise ValueError(f"moe_gate_mul: want (M, 2 I) with I a multiple of 8 at F32 / BF16 / F16, got {tuple(h.shape)} {h.dtype}")
     M, I2 = h.shape
@@ -731,6 +751,9 @@ def DecodeAttention(q: torch.Tensor, kbuf: torch.Tensor, vbuf: torch.Tensor, pos
     buffers -> (B, NH, 1, HD).  With k_new / v_new (B, KH, 1, HD) the same launch appends them at pos first
     (KVCache.decodeAttend, models/llama.go:1156-1160, does the two ops back to back); with rope_base the launch
     also rotates q and k_new at that position (the two ops.RoPE calls before it, models/llama.go:1136-1146)."""
+    y = _host.decode_attention(q, kbuf, vbuf, pos, scale, window, k_new, v_new, rope_base)
+    if y is not None:
+        return y
     _check_cache(kbuf, vbuf, "DecodeAttention")
     if q.dim() != 4 or q.shape[2] != 1:
         raise ValueError(f"ops.DecodeAttention: want q (B, NH, 1, HD), got {tuple(q.shape)}")
