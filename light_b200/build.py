@@ -2,6 +2,7 @@
 front of its hot entry points (csrc/host.cpp), against the installed torch."""
 from __future__ import annotations
 
+import concurrent.futures
 import os
 import shutil
 import subprocess
@@ -12,7 +13,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "liblight_b200.so")
 HOST = os.path.join(HERE, "_host.so")
 SOURCES = ["abi.cu", "gguf_dequant.cu", "gguf_matmul_generic.cu", "gguf_gemv_fast.cu", "gguf_gemv_batch.cu", "prefill_umma.cu", "decode_umma.cu", "int4.cu", "fp8_block.cu",
-           "moe.cu", "peer_gather.cu", "decode_attn.cu", "norm_rope.cu", "w8a8.cu", "moe_route.cu", "decode_chain.cu", "gemv_bf16.cu", "moe_elementwise.cu", "gguf_decode_nt.cu", "gguf_decode_ts.cu"]
+           "moe.cu", "peer_gather.cu", "decode_attn.cu", "norm_rope.cu", "w8a8.cu", "moe_route.cu", "decode_chain.cu", "gemv_bf16.cu", "moe_elementwise.cu", "gguf_decode_nt.cu", "gguf_decode_ts.cu",
+           "gemm_tmem.cu"]
 NVCC_FLAGS = os.environ.get("LIGHT_B200_NVCC_EXTRA", "").split() + ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
               "-Xcompiler", "-fvisibility=hidden", "-Xptxas", "-v"]
 
@@ -38,14 +40,18 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(objdir, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     headers.append(os.path.join(HERE, "..", "include", "light_b200.h"))
-    objs = []
-    for src in SOURCES:
-        s = os.path.join(CSRC, src)
-        o = os.path.join(objdir, src.replace(".cu", ".o"))
-        objs.append(o)
+    objs = [os.path.join(objdir, src.replace(".cu", ".o")) for src in SOURCES]
+
+    def compile_one(src_obj):
+        s, o = os.path.join(CSRC, src_obj[0]), src_obj[1]
         if force or _stale(o, [s] + headers):
-            cmd = [nvcc, *NVCC_FLAGS, "-c", s, "-o", o]
-            r = subprocess.run(cmd, capture_output=True, text=True)
+            return src_obj, subprocess.run([nvcc, *NVCC_FLAGS, "-c", s, "-o", o], capture_output=True, text=True)
+        return src_obj, None
+
+    with concurrent.futures.ThreadPoolExecutor(os.cpu_count() or 1) as pool:
+        for (src, o), r in pool.map(compile_one, zip(SOURCES, objs)):
+            if r is None:
+                continue
             if verbose or r.returncode:
                 sys.stderr.write(r.stdout + r.stderr)
             if r.returncode:

@@ -148,8 +148,8 @@ int light_b200_matmul_q_tp(int t, const float *x, const void *const *w, float *c
 
 int light_b200_prefill_status(int device) {
   if (int rc = bind(device)) return rc;
-  const int a = prefill_status(device), b = decode_umma_status(), c = decode_nt_status(), d = decode_ts_status();
-  return a ? a : b ? b : c ? c : d;
+  const int a = prefill_status(device), b = decode_umma_status(), c = decode_nt_status(), d = decode_ts_status(), e = gemm_tmem_status();
+  return a ? a : b ? b : c ? c : d ? d : e;
 }
 unsigned long long light_b200_matmul_q_workspace_bytes(int M, int K) {
   if (M < 1 || K <= 0) return 0;

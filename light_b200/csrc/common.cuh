@@ -133,6 +133,30 @@ int moe_route_deepseek(const float *logits, const float *bias, int64_t *ids, flo
 int moe_route_topk(const float *probs, int64_t *ids, float *weights, int T, int E, int topk, int normalize, cudaStream_t st);
 void *workspace_ptr(int device, size_t *bytes);
 size_t prefill_sk_ws_bytes();
+// one dequantize-and-multiply of gemm_tmem.cu: 1 = took the call, 0 = not covered, other = error
+struct TmemCall {
+  enum Kind { Q4K, Q6K, Q80, INT4, FP8, DENSE } kind;
+  const void *w;            // packed weights (E, N, K)
+  const float *s, *z;       // scales (INT4, FP8) and zeros (INT4)
+  int G, bR, bC;            // group (INT4); scale block (FP8)
+  const void *x16;          // (M, K) tokens at the operand type: bf16 (then the output is bf16) or f16 (f32)
+  bool bf16;
+  void *out;
+  long long M;
+  int N, K;
+  const int32_t *offsets;   // grouped: see gemm_tmem.cu (null: one matrix)
+  const int64_t *pairs;
+  const float *topkw;
+  long long size_m;
+  int E;
+  double mean_tokens;       // tokens per matrix (grouped: pairs / experts)
+  int min_run_k;            // fewest k a run covers
+  void *parts;              // room for partial tiles
+  size_t parts_bytes;
+};
+int gemm_tmem(const TmemCall &c, cudaStream_t st);
+size_t gemm_tmem_parts_bytes();
+int gemm_tmem_status();
 size_t decode_nt_ws_bytes(int M, int K);
 int gguf_decode_nt(int type, const float *x, const void *const *w, float *const *out, const int *n, int count, int M, int K, void *ws,
                    size_t ws_bytes, cudaStream_t st);

@@ -900,6 +900,39 @@ int launch(const CUtensorMap &tm, const typename Row::Ctx &ctx, const Group &grp
   return launched("prefill (tcgen05)");
 }
 
+TmemCall tmem_call(const GgufCtx &c, TmemCall::Kind kind) {
+  TmemCall t{};
+  t.kind = kind, t.w = c.w;
+  return t;
+}
+template <typename Row> TmemCall tmem_call(const typename Row::Ctx &c);
+template <> TmemCall tmem_call<Q4KRow>(const GgufCtx &c) { return tmem_call(c, TmemCall::Q4K); }
+template <> TmemCall tmem_call<Q6KRow>(const GgufCtx &c) { return tmem_call(c, TmemCall::Q6K); }
+template <> TmemCall tmem_call<Q80Row>(const GgufCtx &c) { return tmem_call(c, TmemCall::Q80); }
+template <> TmemCall tmem_call<Int4Row>(const Int4Ctx &c) {
+  TmemCall t{};
+  t.kind = TmemCall::INT4, t.w = c.codes, t.s = c.s, t.z = c.z, t.G = c.G;
+  return t;
+}
+template <> TmemCall tmem_call<Fp8Row>(const Fp8Ctx &c) {
+  TmemCall t{};
+  t.kind = TmemCall::FP8, t.w = c.w, t.s = c.scale, t.bR = c.bR, t.bC = c.bC;
+  return t;
+}
+template <> TmemCall tmem_call<DenseRow>(const DenseCtx &c) {
+  TmemCall t{};
+  t.kind = TmemCall::DENSE, t.w = c.w;
+  return t;
+}
+int use_tmem() {
+  static const int v = getenv("LIGHT_B200_TMEM") ? atoi(getenv("LIGHT_B200_TMEM")) : 1;
+  return v;
+}
+int tmem_min_run() {
+  static const int v = getenv("LIGHT_B200_TMEM_RUN") ? atoi(getenv("LIGHT_B200_TMEM_RUN")) : 1024;
+  return v;
+}
+
 // f32 activations run with f16 operands and f32 output, bf16 activations with bf16 operands and output
 template <typename Row>
 int launch_by_act(const void *x, int act_dtype, const typename Row::Ctx &ctx, void *out, int M, int N, int K, void *ws,
@@ -913,6 +946,12 @@ int launch_by_act(const void *x, int act_dtype, const typename Row::Ctx &ctx, vo
   const size_t x_bytes = act_dtype == LB200_F32 ? (((size_t)M * K * 2 + 1023) & ~(size_t)1023) : 0;
   void *sk = ws && ws_bytes > x_bytes ? (char *)ws + x_bytes : nullptr;
   const size_t sk_bytes = sk ? ws_bytes - x_bytes : 0;
+  if (use_tmem() && sk) {
+    TmemCall c = tmem_call<Row>(ctx);
+    c.x16 = act_dtype == LB200_F32 ? ws : x, c.bf16 = act_dtype != LB200_F32, c.out = out, c.M = M, c.N = N, c.K = K;
+    c.mean_tokens = M, c.min_run_k = tmem_min_run(), c.parts = sk, c.parts_bytes = sk_bytes;
+    if (int took = gemm_tmem(c, st)) return took == 1 ? 0 : took;
+  }
   if (act_dtype == LB200_F32) return launch<Row, false, float>(tm, ctx, none, (float *)out, M, N, K, st, sk, sk_bytes);
   if constexpr (!Row::KPERM) return launch<Row, true, __nv_bfloat16>(tm, ctx, none, (__nv_bfloat16 *)out, M, N, K, st, sk, sk_bytes);
   return LB200_E_DTYPE;
@@ -1049,6 +1088,13 @@ int moe_launch(const lb200_moe_args *a, const typename Row::Ctx &ctx, void *ws, 
   const Group grp{a->offsets, a->sorted_pairs, a->topk_weights, a->size_m, a->E};
   const size_t x_bytes = ((size_t)a->M * a->K * 2 + 1023) & ~(size_t)1023;
   void *sk = ws_bytes > x_bytes ? (char *)ws + x_bytes : nullptr;
+  if (use_tmem() && sk) {
+    TmemCall c = tmem_call<Row>(ctx);
+    c.x16 = ws, c.bf16 = BF16, c.out = a->out, c.M = a->M, c.N = a->N, c.K = a->K;
+    c.offsets = a->offsets, c.pairs = a->sorted_pairs, c.topkw = a->topk_weights, c.size_m = a->size_m, c.E = a->E;
+    c.mean_tokens = (double)a->M / a->E, c.min_run_k = tmem_min_run(), c.parts = sk, c.parts_bytes = ws_bytes - x_bytes;
+    if (int took = gemm_tmem(c, st)) return took == 1 ? 0 : took;
+  }
   return launch<Row, BF16, OutT>(tm, ctx, grp, (OutT *)a->out, (int)a->M, a->N, a->K, st, sk, sk ? ws_bytes - x_bytes : 0);
 }
 

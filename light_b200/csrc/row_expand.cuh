@@ -49,9 +49,9 @@ __device__ __forceinline__ void st_chunk(uint32_t addr, const uint4 &v) {
 }
 
 // ---- per-format row expanders: one thread, one weight row, one 256-element block at a time.
-// load(): fetch the block into registers.  step(j, ...): write the 64 weights k = 64j .. 64j+63 of
-// the block as 8 swizzled 16-byte chunks of row `r` of the B tile at shared address `tile`
-// (PART 0 / 1: only chunks 0-3 / 4-7, for two threads that share a row; 2: all eight).
+// load(): fetch the block into registers.  emit(j, sink): hand the 64 weights k = 64j .. 64j+63 of the
+// block to sink(c, chunk) as 8 chunks of eight values (PART 0 / 1: only chunks 0-3 / 4-7, for two threads
+// that share a row; 2: all eight); step() is emit() into a swizzled shared-memory tile.
 struct GgufCtx {
   const uint8_t *w;
 };
@@ -95,6 +95,10 @@ struct Q4KRow {
   __device__ __forceinline__ static __half2 u2h(uint32_t v) { return *reinterpret_cast<__half2 *>(&v); }
   template <bool BF16, int PART = 2>
   __device__ __forceinline__ void step(int j, uint32_t tile, int r) const {
+    emit<BF16, PART>(j, [&](int c, const uint4 &v) { st_chunk(tile + swz(r, c), v); });
+  }
+  template <bool BF16, int PART = 2, typename Sink>
+  __device__ __forceinline__ void emit(int j, Sink &&sink) const {
     // sub-blocks 2j (low nibbles of qs[32j .. 32j+31]) and 2j+1 (high nibbles)
     const __half2 dd = u2h(h.x);  // (d, dmin)
     uint32_t sc0, mn0, sc1, mn1;
@@ -120,8 +124,8 @@ struct Q4KRow {
 #pragma unroll
     for (int c = 0; c < 4; c++) {  // chunk c: k = 8c..8c+7 (low nibbles); chunk c+4: k = 32+8c.. (high nibbles)
       const uint32_t a = w[2 * c], b = w[2 * c + 1], a8 = a >> 8, b8 = b >> 8;
-      if (PART != 1) st_chunk(tile + swz(r, c), make_uint4(lo2(a), lo2(a8), lo2(b), lo2(b8)));
-      if (PART != 0) st_chunk(tile + swz(r, c + 4), make_uint4(hi2(a), hi2(a8), hi2(b), hi2(b8)));
+      if (PART != 1) sink(c, make_uint4(lo2(a), lo2(a8), lo2(b), lo2(b8)));
+      if (PART != 0) sink(c + 4, make_uint4(hi2(a), hi2(a8), hi2(b), hi2(b8)));
     }
   }
 };
@@ -195,6 +199,10 @@ struct Q6KRow {
   // and (1, 3), one HADD2 takes 1056 off (code - 32, exact), one HMUL2 applies d * sc rounded to f16.
   template <bool BF16, int PART = 2>
   __device__ __forceinline__ void step(int j, uint32_t tile, int r) const {
+    emit<BF16, PART>(j, [&](int c, const uint4 &v) { st_chunk(tile + swz(r, c), v); });
+  }
+  template <bool BF16, int PART = 2, typename Sink>
+  __device__ __forceinline__ void emit(int j, Sink &&sink) const {
     const __half2 off = __float2half2_rn(-1056.f);
 #pragma unroll
     for (int c = (PART == 1 ? 4 : 0); c < (PART == 0 ? 4 : 8); c++) {  // chunk c: k = 8c .. 8c+7 -> group q = 2j + c/4, l = 8 (c%4) ..
@@ -211,7 +219,7 @@ struct Q6KRow {
         const __half2 w13 = __hmul2(__hadd2(*reinterpret_cast<const __half2 *>(&p13), off), ds);
         o[2 * e] = *reinterpret_cast<const uint32_t *>(&w02), o[2 * e + 1] = *reinterpret_cast<const uint32_t *>(&w13);
       }
-      st_chunk(tile + swz(r, c), make_uint4(o[0], o[1], o[2], o[3]));
+      sink(c, make_uint4(o[0], o[1], o[2], o[3]));
     }
   }
 };
@@ -248,10 +256,17 @@ struct Q80Row {
   __device__ __forceinline__ void load_smem(uint32_t slot, int unit) {
     const uint32_t a = slot + (uint32_t)(unit & 1) * 136u;
 #pragma unroll
-    for (int i = 0; i < 34; i++) w[i] = lds32(a + 4 * i);
+    for (int i = 0; i < 17; i++) {
+      const uint2 v = lds64(a + 8 * i);
+      w[2 * i] = v.x, w[2 * i + 1] = v.y;
+    }
   }
   template <bool BF16, int PART = 2>
   __device__ __forceinline__ void step(int j, uint32_t tile, int r) const {
+    emit<BF16, PART>(j, [&](int c, const uint4 &v) { st_chunk(tile + swz(r, c), v); });
+  }
+  template <bool BF16, int PART = 2, typename Sink>
+  __device__ __forceinline__ void emit(int j, Sink &&sink) const {
     const __half2 off = __float2half2_rn(-1152.f);
 #pragma unroll
     for (int c = (PART == 1 ? 4 : 0); c < (PART == 0 ? 4 : 8); c++) {  // chunk c: k = 8c .. 8c+7 of block 2j + c/4
@@ -269,7 +284,7 @@ struct Q80Row {
         const __half2 w23 = __hmul2(__hadd2(*reinterpret_cast<const __half2 *>(&p23), off), d2);
         o[2 * e] = *reinterpret_cast<const uint32_t *>(&w01), o[2 * e + 1] = *reinterpret_cast<const uint32_t *>(&w23);
       }
-      st_chunk(tile + swz(r, c), make_uint4(o[0], o[1], o[2], o[3]));
+      sink(c, make_uint4(o[0], o[1], o[2], o[3]));
     }
   }
 };
@@ -290,8 +305,20 @@ struct Int4Row {
   static constexpr int STEPS = 4;
   const uint4 *row;
   const float *sr, *zr;
-  int G, unit;
+  int G;
+  struct Aux {  // of the four 64-element steps of a load unit; their loads are issued with (or before) the codes'
+    float s[4], z[4];
+  } aux;
   uint4 q[8];
+  __device__ __forceinline__ Aux fetch_aux(int u) const {
+    Aux a;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int grp = (u * 256 + j * 64) / G;
+      a.s[j] = __ldg(sr + grp), a.z[j] = __ldg(zr + grp);
+    }
+    return a;
+  }
   __device__ __forceinline__ void init(const Ctx &c, int e, int n, int N, int K) {
     const size_t r = (size_t)e * N + n;
     row = reinterpret_cast<const uint4 *>(c.codes + r * (K / 8));
@@ -304,19 +331,25 @@ struct Int4Row {
   __device__ __forceinline__ const uint8_t *raw_src_unaligned(int b) const { return raw_src(b); }
   __device__ __forceinline__ static size_t row_stride(const Ctx &, int K) { return (size_t)(K / 8) * 4; }
   __device__ __forceinline__ void load_smem(uint32_t slot, int u) {
-    unit = u;
+    aux = fetch_aux(u);
+    load_codes(slot);
+  }
+  __device__ __forceinline__ void load_codes(uint32_t slot) {
 #pragma unroll
     for (int i = 0; i < 8; i++) q[i] = lds128(slot + 16 * i);
   }
   __device__ __forceinline__ void load(int u) {
-    unit = u;
+    aux = fetch_aux(u);
 #pragma unroll
     for (int i = 0; i < 8; i++) q[i] = __ldg(row + (size_t)u * 8 + i);
   }
   template <bool BF16, int PART = 2>
   __device__ __forceinline__ void step(int j, uint32_t tile, int r) const {
-    const int grp = (unit * 256 + j * 64) / G;
-    const float sc = __ldg(sr + grp), z = __ldg(zr + grp);
+    emit<BF16, PART>(j, [&](int c, const uint4 &v) { st_chunk(tile + swz(r, c), v); });
+  }
+  template <bool BF16, int PART = 2, typename Sink>
+  __device__ __forceinline__ void emit(int j, Sink &&sink) const {
+    const float sc = aux.s[j], z = aux.z[j];
     const uint32_t w[8] = {q[2 * j].x, q[2 * j].y, q[2 * j].z, q[2 * j].w, q[2 * j + 1].x, q[2 * j + 1].y, q[2 * j + 1].z, q[2 * j + 1].w};
 #pragma unroll
     for (int c = (PART == 1 ? 4 : 0); c < (PART == 0 ? 4 : 8); c++) {  // chunk c = code word c: nibbles 0..7 in element order
@@ -326,7 +359,7 @@ struct Int4Row {
       o.y = pack2<BF16>(__fmul_rn(sc, __fsub_rn(byte_f32(lo, 1), z)), __fmul_rn(sc, __fsub_rn(byte_f32(hi, 1), z)));
       o.z = pack2<BF16>(__fmul_rn(sc, __fsub_rn(byte_f32(lo, 2), z)), __fmul_rn(sc, __fsub_rn(byte_f32(hi, 2), z)));
       o.w = pack2<BF16>(__fmul_rn(sc, __fsub_rn(byte_f32(lo, 3), z)), __fmul_rn(sc, __fsub_rn(byte_f32(hi, 3), z)));
-      st_chunk(tile + swz(r, c), o);
+      sink(c, o);
     }
   }
 };
@@ -345,8 +378,12 @@ struct Fp8Row {
   static constexpr int STEPS = 2;
   const uint4 *row;
   const float *sr;
-  int bC, unit;
+  int bC;
+  struct Aux {  // the scales of the two 64-element steps of a load unit
+    float s[2];
+  } aux;
   uint4 q[8];
+  __device__ __forceinline__ Aux fetch_aux(int u) const { return Aux{{__ldg(sr + u * 128 / bC), __ldg(sr + (u * 128 + 64) / bC)}}; }
   __device__ __forceinline__ void init(const Ctx &c, int e, int n, int N, int K) {
     row = reinterpret_cast<const uint4 *>(c.w + ((size_t)e * N + n) * K);
     sr = c.scale + ((size_t)e * (N / c.bR) + n / c.bR) * (K / c.bC), bC = c.bC;
@@ -358,12 +395,15 @@ struct Fp8Row {
   __device__ __forceinline__ const uint8_t *raw_src_unaligned(int b) const { return raw_src(b); }
   __device__ __forceinline__ static size_t row_stride(const Ctx &, int K) { return (size_t)K; }
   __device__ __forceinline__ void load_smem(uint32_t slot, int u) {
-    unit = u;
+    aux = fetch_aux(u);
+    load_codes(slot + 128 * (u & 1));
+  }
+  __device__ __forceinline__ void load_codes(uint32_t slot) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) q[i] = lds128(slot + 128 * (u & 1) + 16 * i);
+    for (int i = 0; i < 8; i++) q[i] = lds128(slot + 16 * i);
   }
   __device__ __forceinline__ void load(int u) {
-    unit = u;
+    aux = fetch_aux(u);
 #pragma unroll
     for (int i = 0; i < 8; i++) q[i] = __ldg(row + (size_t)u * 8 + i);
   }
@@ -376,13 +416,17 @@ struct Fp8Row {
   }
   template <bool BF16, int PART = 2>
   __device__ __forceinline__ void step(int j, uint32_t tile, int r) const {
-    const float sc = __ldg(sr + (unit * 128 + j * 64) / bC);
+    emit<BF16, PART>(j, [&](int c, const uint4 &v) { st_chunk(tile + swz(r, c), v); });
+  }
+  template <bool BF16, int PART = 2, typename Sink>
+  __device__ __forceinline__ void emit(int j, Sink &&sink) const {
+    const float sc = aux.s[j];
 #pragma unroll
     for (int c = (PART == 1 ? 2 : 0); c < (PART == 0 ? 2 : 4); c++) {  // 16 bytes = two chunks of 8 codes
       const uint4 v = q[4 * j + c];
       const uint2 a = four<BF16>(v.x, sc), b = four<BF16>(v.y, sc), e = four<BF16>(v.z, sc), f = four<BF16>(v.w, sc);
-      st_chunk(tile + swz(r, 2 * c), make_uint4(a.x, a.y, b.x, b.y));
-      st_chunk(tile + swz(r, 2 * c + 1), make_uint4(e.x, e.y, f.x, f.y));
+      sink(2 * c, make_uint4(a.x, a.y, b.x, b.y));
+      sink(2 * c + 1, make_uint4(e.x, e.y, f.x, f.y));
     }
   }
 };
@@ -401,14 +445,23 @@ struct DenseRow {
     row = reinterpret_cast<const uint4 *>(c.w + ((size_t)e * N + n) * K);
   }
   __device__ __forceinline__ void prefetch(int u) const { prefetch_l2(row + (size_t)u * 8, 128); }
+  __device__ __forceinline__ static size_t row_stride(const Ctx &, int K) { return (size_t)K * 2; }
+  __device__ __forceinline__ void load_codes(uint32_t slot) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) q[i] = lds128(slot + 16 * i);
+  }
   __device__ __forceinline__ void load(int u) {
 #pragma unroll
     for (int i = 0; i < 8; i++) q[i] = __ldg(row + (size_t)u * 8 + i);
   }
   template <bool BF16, int PART = 2>
-  __device__ __forceinline__ void step(int, uint32_t tile, int r) const {
+  __device__ __forceinline__ void step(int j, uint32_t tile, int r) const {
+    emit<BF16, PART>(j, [&](int c, const uint4 &v) { st_chunk(tile + swz(r, c), v); });
+  }
+  template <bool BF16, int PART = 2, typename Sink>
+  __device__ __forceinline__ void emit(int, Sink &&sink) const {
 #pragma unroll
-    for (int c = (PART == 1 ? 4 : 0); c < (PART == 0 ? 4 : 8); c++) st_chunk(tile + swz(r, c), q[c]);
+    for (int c = (PART == 1 ? 4 : 0); c < (PART == 0 ? 4 : 8); c++) sink(c, q[c]);
   }
 };
 
