@@ -9,13 +9,16 @@
 // Tokens are the N side, so a tile holds any multiple of 16 (32 when paired) of them: short prompts and the ragged
 // token counts of experts cost what they are, not the next multiple of 128.  Weight rows are the M side and always full.
 //
-//   warps 0-7    expanders.  Warps w and w + 4 own rows 32 (w & 3) .. + 31 (the TMEM lanes a warp can reach) and take
-//                turns at the K chunks: packed rows arrive by cp.async in the warp's own slots, are read into registers,
-//                and leave as 32 TMEM columns per 64 k (eight stages).
-//   warp  8      one lane: TMA of the token tiles.
-//   warp  9      one lane: MMAs and commits; in the second CTA of a pair: forwards "my half is ready" to the first.
-//   warps 10-13  epilogue: TMEM -> registers -> output rows (a warp's lanes hold 32 consecutive columns of a token's row:
-//                full lines without a transpose), while the next tile's MMAs run (token tiles up to 128 use two accumulators).
+//   warps 0-15   expanders.  The four warps w, w + 4, .. own rows 32 (w & 3) .. + 31 (the TMEM lanes a warp can reach) and
+//                take turns at the units of 128 k: a unit's packed rows arrive by cp.async in the warp's own slot, go into
+//                registers (the slot then takes the next copy) and leave as 64 TMEM columns.  Expansion is a chain of
+//                short dependent instructions: two warps per row quarter instead of four ran it at 4 to 8 clocks each
+//                and set the pace wherever a tile had few tokens (4-bit rows at 2048 tokens: 1092 against 1335 TFLOP/s).
+//   warp  16     one lane: TMA of the token tiles.
+//   warp  17     MMAs and commits; in the second CTA of a pair: forwards "my half is ready" to the first.
+//   warps 18-21  epilogue, while the next tile's MMAs run (token tiles up to 128 use two accumulators): TMEM -> registers ->
+//                a [token][row] strip in shared memory -> one bulk copy per token.  The run's last segment is finished by
+//                the expanders too, five warps to a row quarter, each 16 tokens at a time.
 //
 // Work is the list of (tile, K chunk) pairs, cut into equal runs, one per CTA (pair): stream-K.  A segment that does not
 // start its tile writes a partial tile and raises its flag, which it does first; the segment that starts the tile owns it
@@ -29,7 +32,7 @@
 
 #include "common.cuh"
 #include "mma_sync.cuh"
-#include "row_expand.cuh"
+#include "tmem_rows.cuh"
 #include "umma.cuh"
 
 namespace lb {
@@ -37,26 +40,19 @@ namespace {
 
 using namespace umma;
 
-constexpr int TMA_WARP = 8, MMA_WARP = 9, THREADS = 14 * 32;
-constexpr int NAS = 4;                        // TMEM stages of expanded weights, 64 columns (128 k) each
+constexpr int EXPANDERS = 16, TMA_WARP = 16, MMA_WARP = 17, EPI_WARP = 18, THREADS = 22 * 32;
+constexpr int KU = 128;                       // k of a unit: one TMEM stage, one stage of the token ring
+constexpr int NAS = 4;                        // stages of 128 k: 64 TMEM columns of expanded weights, and a token tile in shared memory
 constexpr int A_COL = 256;                    // columns 0-255: accumulators, 256-511: weight stages
 constexpr int MAX_E = 1024;                   // experts whose prefix sums fit the shared tables
 constexpr int MAX_GRID = 160;
+constexpr int BAR_BYTES = 640;                // barriers
 constexpr int PART_FLOATS = 256 * 128;        // one partial tile: [token][row]
 constexpr int SMEM_MAX = 227 * 1024 - 1024;   // dynamic; the static part (prefix tables, flags) is accounted below
 
 __device__ int g_status;                      // non-zero: a bounded wait gave up (sticky)
-__device__ unsigned int g_flags[MAX_GRID * 4];  // per epilogue warp: raised by the writer of a partial tile, lowered by its one reader
-
-// Per row format: k per chunk (one copy of a warp's 32 rows), its 16-byte granules per row, the slot pitch (an odd
-// number of granules spreads the rows over the banks), and the load units (Row::load_*) that make up a chunk.
-template <typename Row> struct Fmt;
-template <> struct Fmt<Q4KRow> { static constexpr int KU = 256, GR = 9, PITCH = 144, LOADS = 1; };
-template <> struct Fmt<Q6KRow> { static constexpr int KU = 256, GR = 14, PITCH = 240, LOADS = 2; };
-template <> struct Fmt<Q80Row> { static constexpr int KU = 256, GR = 17, PITCH = 272, LOADS = 2; };
-template <> struct Fmt<Int4Row> { static constexpr int KU = 256, GR = 8, PITCH = 144, LOADS = 1; };
-template <> struct Fmt<Fp8Row> { static constexpr int KU = 128, GR = 8, PITCH = 144, LOADS = 1; };
-template <> struct Fmt<DenseRow> { static constexpr int KU = 128, GR = 16, PITCH = 272, LOADS = 2; };
+__device__ unsigned int g_flags[MAX_GRID * 64];  // (CTA, row quarter, 16-token chunk): raised by the writer of that part of a partial tile,
+                                                // lowered by its one reader
 
 struct Args {
   const int32_t *offsets;   // grouped: expert e owns rows offsets[e] .. offsets[e + 1] of the (gathered) tokens; null: one matrix
@@ -66,7 +62,7 @@ struct Args {
   int E, M, N, K;
   int nt_max;               // most tokens of a tile
   int box;                  // token rows of one TMA box
-  int stage_bytes, nbs;     // of the token ring (a stage: 128 k), per CTA
+  int stage_bytes;          // of a token tile, per CTA
   int wmin;                 // grouped: a unit's weight is max(tokens of its tile, wmin)
   float *parts;
 };
@@ -85,21 +81,32 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
   return p != 0;
 }
+// Looks for up to a hardware-set time (the thread sleeps meanwhile): a waiting warp takes no issue slots from the expanders.
+// (Spinning, the four epilogue warps and the MMA warp issued a third of all instructions.)
+__device__ __forceinline__ bool mbar_sleep_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // A whole warp waits, together: every lane looks and all branches are on votes, so the warp never diverges here (what
 // follows are .aligned instructions and values the compiler keeps in the warp's uniform registers).
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort) {
-  if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity))) return true;
+  if (__all_sync(0xffffffffu, mbar_sleep_wait(bar, parity))) return true;
   const unsigned long long t0 = global_ns();
-  for (uint32_t i = 1;; i++) {
-    if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity))) return true;
-    if ((i & 63u) == 0) {
-      if (__any_sync(0xffffffffu, *abort != 0)) return false;
-      if (__any_sync(0xffffffffu, global_ns() - t0 > 1000000000ull)) break;
-      __nanosleep(32);
+  while (!__all_sync(0xffffffffu, mbar_sleep_wait(bar, parity))) {
+    if (__any_sync(0xffffffffu, *abort != 0)) return false;
+    if (__any_sync(0xffffffffu, global_ns() - t0 > 1000000000ull)) {
+      *abort = 1;
+      return false;
     }
   }
-  *abort = 1;
-  return false;
+  return true;
 }
 __device__ __forceinline__ void st_if(bool p, float *o, float v) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.f32 [%0], %1;\n\t}\n" ::"l"(o), "f"(v), "r"((int)p) : "memory");
@@ -150,28 +157,25 @@ __device__ __forceinline__ void commit(uint32_t bar) {  // CG = 2: on this barri
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(bar), "h"((uint16_t)3)
                  : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};\n" ::"r"(taddr),
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n" ::"r"(taddr),
       "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
-      "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]),
-      "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
-__device__ __forceinline__ bool wait_flag(const unsigned *flag, volatile int *abort) {  // whole warp
+__device__ __forceinline__ bool wait_flag(const unsigned *flag, bool mine, volatile int *abort) {  // whole warp, a flag to each lane that has one
   const unsigned long long t0 = global_ns();
   for (uint32_t i = 1;; i++) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(flag) : "memory");
+    unsigned v = 1;
+    if (mine) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(flag) : "memory");
     if (__all_sync(0xffffffffu, v != 0)) return true;
     if ((i & 15u) == 0) {
       if (__any_sync(0xffffffffu, *abort != 0)) return false;
       if (__any_sync(0xffffffffu, global_ns() - t0 > 1000000000ull)) break;
-      __nanosleep(64);
     }
   }
   *abort = 1;
@@ -184,8 +188,7 @@ __device__ __forceinline__ bool wait_flag(const unsigned *flag, volatile int *ab
 template <int CG>
 struct Work {
   const Args &a;
-  const int *preT;
-  const long long *preW;
+  const int *preT, *preW;
   int nb, nrt;
   __device__ __forceinline__ int count(int e) const { return a.offsets ? a.offsets[e + 1] - a.offsets[e] : a.M; }
   __device__ __forceinline__ int first(int e) const { return a.offsets ? a.offsets[e] : 0; }
@@ -193,93 +196,97 @@ struct Work {
     ntt = (cnt + a.nt_max - 1) / a.nt_max;
     nt = ntt ? ((cnt + ntt - 1) / ntt + 16 * CG - 1) / (16 * CG) * (16 * CG) : 0;
   }
-  __device__ __forceinline__ int weight(int nt) const { return a.offsets ? max(nt, a.wmin) : 1; }
-  __device__ __forceinline__ Tile tile(int t) const {
-    int lo = 0, hi = a.E - 1;  // the expert with preT[e] <= t < preT[e + 1]
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (preT[mid + 1] <= t) lo = mid + 1;
-      else hi = mid;
-    }
-    Tile T;
-    int ntt;
-    const int cnt = count(lo);
-    geo(cnt, ntt, T.nt);
-    const int r = t - preT[lo], rt = r / ntt, tt = r - rt * ntt;
-    T.expert = lo, T.n0 = rt * 128 * CG, T.m0 = first(lo) + tt * T.nt, T.m_end = min(first(lo) + cnt, T.m0 + T.nt);
-    return T;
-  }
-  // first unit (tile-major) of run j of G
-  __device__ __forceinline__ long long bound(int j, int G) const {
-    const long long W = preW[a.E], w = W * j / G;
-    if (j >= G) return (long long)preT[a.E] * nb;
+  __device__ __forceinline__ int weight(int nt) const { return a.offsets ? max(nt, a.wmin) / 16 : 1; }
+  __device__ __forceinline__ int expert_of(const int *pre, int v) const {  // the expert with pre[e] <= v < pre[e + 1]
     int lo = 0, hi = a.E - 1;
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
-      if (preW[mid + 1] <= w) lo = mid + 1;
+      if (pre[mid + 1] <= v) lo = mid + 1;
       else hi = mid;
     }
+    return lo;
+  }
+  __device__ __forceinline__ Tile tile(int t) const {
+    Tile T;
+    const int e = expert_of(preT, t);
+    int ntt;
+    const int cnt = count(e);
+    geo(cnt, ntt, T.nt);
+    const int r = t - preT[e], rt = r / ntt, tt = r - rt * ntt;
+    T.expert = e, T.n0 = rt * 128 * CG, T.m0 = first(e) + tt * T.nt, T.m_end = min(first(e) + cnt, T.m0 + T.nt);
+    return T;
+  }
+  // first unit (tile-major) of run j of G
+  __device__ __forceinline__ int bound(int j, int G) const {
+    if (j >= G) return preT[a.E] * nb;
+    const int W = preW[a.E], q = W / G, w = q * j + min(j, W - q * G);
+    if (!a.offsets) return w;
+    const int e = expert_of(preW, w);
     int ntt, nt;
-    geo(count(lo), ntt, nt);
-    return (long long)preT[lo] * nb + (w - preW[lo]) / weight(nt);
+    geo(count(e), ntt, nt);
+    return preT[e] * nb + (w - preW[e]) / weight(nt);
   }
 };
 
-template <typename Row>
-__device__ __forceinline__ const uint8_t *row_ptr(const Row &r) { return reinterpret_cast<const uint8_t *>(r.row); }
-template <typename Row> struct HasAux : std::false_type {};
-template <> struct HasAux<Int4Row> : std::true_type {};
-template <> struct HasAux<Fp8Row> : std::true_type {};
-
 // ------------------------------------------------------------------------------------ kernel
-template <typename Row, bool BF16, typename OutT, int CG, int NSLOT>
-__global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_constant__ CUtensorMap tmap, const typename Row::Ctx ctx,
+template <typename OutT>
+constexpr uint32_t STRIP = 32 * 128 * sizeof(OutT);  // 32 tokens of 128 output columns
+constexpr int STRIPS = 16384;                        // one strip of f32, two of bf16
+
+struct Maps {
+  CUtensorMap x, w[2];  // tokens; the weight rows, per box of the format
+};
+
+template <typename Row, bool BF16, typename OutT, int CG>
+__global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_constant__ Maps maps, const typename Row::Ctx ctx,
                                                               const __grid_constant__ Args a, OutT *__restrict__ out) {
-  using F = Fmt<Row>;
-  constexpr int SPC = F::KU / 64, SPL = SPC / F::LOADS;  // 64-k steps per chunk and per load unit
   extern __shared__ unsigned char smem_raw[];
   __shared__ int abort_flag;
   __shared__ uint32_t tmem_sh;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char *gen = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t ring_bytes = (uint32_t)a.nbs * a.stage_bytes;
-  const uint32_t sB = base, sRaw = base + ring_bytes, sBar = sRaw + 8u * NSLOT * 32 * F::PITCH;
-  const uint32_t a_full = sBar, a_empty = a_full + 8 * NAS, peer_full = a_empty + 8 * NAS, d_full = peer_full + 8 * NAS, d_empty = d_full + 16,
-                 b_full = d_empty + 16, b_empty = b_full + 8 * 16, drained = b_empty + 8 * 16;
-  long long *preW = reinterpret_cast<long long *>(gen + (sBar - base) + 512);
-  int *preT = reinterpret_cast<int *>(preW + a.E + 1);
+  const uint32_t sB = base, sRaw = base + NAS * (uint32_t)a.stage_bytes, sStrip = sRaw + (uint32_t)EXPANDERS * Row::SLOT, sBar = sStrip + STRIPS;
+  // full[s]: a stage's weights (four warps) and tokens (the TMA lane and its bytes) are there, and so are the other CTA's;
+  // empty[s]: its MMAs have completed
+  const uint32_t full = sBar, empty = full + 8 * NAS, d_full = empty + 8 * NAS, d_empty = d_full + 16, drained = d_empty + 16, w_full = drained + 8;
+  int *preW = reinterpret_cast<int *>(gen + (sBar - base) + BAR_BYTES), *preT = preW + a.E + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = CG == 2 ? (int)cluster_ctarank() : 0;
-  const Work<CG> wk{a, preT, preW, a.K / F::KU, (a.N + 128 * CG - 1) / (128 * CG)};
+  const Work<CG> wk{a, preT, preW, a.K / KU, (a.N + 128 * CG - 1) / (128 * CG)};
   const int nb = wk.nb;
   const int G = gridDim.x / CG, cta = blockIdx.x / CG;
 
   if (threadIdx.x == 0) {
+    prefetch_tmap(&maps.x);
+    if constexpr (Row::BOXES > 0) prefetch_tmap(&maps.w[0]);
+    if constexpr (Row::BOXES > 1) prefetch_tmap(&maps.w[1]);
     abort_flag = 0;
-    for (int i = 0; i < NAS; i++) mbar_init(a_full + 8 * i, 4), mbar_init(a_empty + 8 * i, 1), mbar_init(peer_full + 8 * i, 1);
+    for (int i = 0; i < NAS; i++) mbar_init(full + 8 * i, CG == 2 && rank == 0 ? 6 : 5), mbar_init(empty + 8 * i, 1);
     for (int i = 0; i < 2; i++) mbar_init(d_full + 8 * i, 1), mbar_init(d_empty + 8 * i, 4 * CG);
     mbar_init(drained, 1);
-    for (int i = 0; i < a.nbs; i++) mbar_init(b_full + 8 * i, 1), mbar_init(b_empty + 8 * i, 1);
+    for (int i = 0; i < EXPANDERS; i++) mbar_init(w_full + 8 * i, 1);
     fence_barrier_init();
   }
+  // (every CTA of this grid is resident once all have come by here: the next kernel's wait for room, and for its operands)
+  pdl_launch_dependents();
+  if (a.offsets) pdl_wait();
   for (int e = threadIdx.x; e < a.E; e += THREADS) {
     int ntt, nt;
     wk.geo(wk.count(e), ntt, nt);
     preT[e + 1] = ntt * wk.nrt;
-    preW[e + 1] = (long long)ntt * wk.nrt * nb * wk.weight(nt);
+    preW[e + 1] = ntt * wk.nrt * nb * wk.weight(nt);
   }
   if (warp == MMA_WARP) alloc512<CG>(smem_u32(&tmem_sh));
   __syncthreads();
   if (warp == 0) {  // inclusive prefix sums, 32 experts at a time
-    int ct = 0;
-    long long cw = 0;
+    int ct = 0, cw = 0;
     for (int e0 = 0; e0 < a.E; e0 += 32) {
       int t = e0 + lane < a.E ? preT[e0 + lane + 1] : 0;
-      long long w = e0 + lane < a.E ? preW[e0 + lane + 1] : 0;
+      int w = e0 + lane < a.E ? preW[e0 + lane + 1] : 0;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
         const int tt = __shfl_up_sync(0xffffffffu, t, d);
-        const long long ww = __shfl_up_sync(0xffffffffu, w, d);
+        const int ww = __shfl_up_sync(0xffffffffu, w, d);
         if (lane >= d) t += tt, w += ww;
       }
       if (e0 + lane < a.E) preT[e0 + lane + 1] = ct + t, preW[e0 + lane + 1] = cw + w;
@@ -293,50 +300,44 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   tc_fence_after();
   const uint32_t tmem = tmem_sh;
   volatile int *abort = &abort_flag;
-  const long long pos0 = wk.bound(cta, G), pos1 = wk.bound(cta + 1, G);
-  const int n = (int)(pos1 - pos0);  // units of this run
+  const int pos0 = wk.bound(cta, G), pos1 = wk.bound(cta + 1, G);
+  const int n = pos1 - pos0;  // units of this run
 
   if (warp == TMA_WARP) {
     if (lane == 0) {
-      prefetch_tmap(&tmap);
-      int bt = 0, ph = 1, issued = 0;
-      for (long long pos = pos0; pos < pos1 && !*abort;) {
-        const int t = (int)(pos / nb), u0 = (int)(pos - (long long)t * nb), u1 = (int)min((long long)nb, u0 + (pos1 - pos));
+      pdl_wait();  // the tokens may be the kernel before's; the weights are not
+      int issued = 0;
+      for (int pos = pos0; pos < pos1 && !*abort;) {
+        const int t = pos / nb, u0 = pos - t * nb, u1 = min(nb, u0 + (pos1 - pos));
         const Tile T = wk.tile(t);
         const int rows = T.nt / CG, boxes = (rows + a.box - 1) / a.box, y0 = T.m0 + rank * rows;
-        const uint32_t bytes = (uint32_t)(boxes * a.box) * 128u;
-        for (int k = u0 * SPC; k < u1 * SPC; k += 2) {
-          if (issued >= a.nbs && !mbar_wait(b_empty + 8 * bt, ph, abort)) break;
-          mbar_arrive_expect_tx(b_full + 8 * bt, 2 * bytes);
+        const uint32_t bytes = (uint32_t)(boxes * a.box) * 256u;
+        for (int u = u0; u < u1; u++, issued++) {
+          const int s = issued % NAS;
+          if (issued >= NAS) {
+            const uint32_t par = (uint32_t)(issued / NAS - 1) & 1u;
+            if (!mbar_sleep_wait(empty + 8 * s, par) && !mbar_wait(empty + 8 * s, par, abort)) break;
+          }
+          mbar_arrive_expect_tx(full + 8 * s, bytes);
           for (int i = 0; i < 2 * boxes; i++) {
             const int h = i & 1, bx = i >> 1;
-            tma_load_2d(sB + bt * a.stage_bytes + h * (a.stage_bytes / 2) + bx * a.box * 128, &tmap, b_full + 8 * bt, (k + h) * 64, y0 + bx * a.box);
+            tma_load_2d(sB + s * a.stage_bytes + h * (a.stage_bytes / 2) + bx * a.box * 128, &maps.x, full + 8 * s, u * 128 + h * 64, y0 + bx * a.box);
           }
-          issued++;
-          if (++bt == a.nbs) bt = 0, ph ^= 1;
         }
         pos += u1 - u0;
       }
-      if (*abort)  // the loads still in flight get a bounded time to land before the CTA retires
-        for (int k = issued > a.nbs ? issued - a.nbs : 0; k < issued; k++)
-          for (int i = 0; i < (1 << 14) && !mbar_test_wait(b_full + 8 * (k % a.nbs), (k / a.nbs) & 1); i++) {
-          }
     }
   } else if (warp == MMA_WARP) {
-    // The whole warp runs the loop and one elected lane issues.  A pass costs about 700 clocks of instruction latency
-    // (three barrier looks, fence, first MMA, two commits) whatever it issues, so a stage is 128 k: eight MMAs of 128 clocks;
-    // with 64 k per pass the tensor pipe stood at half its rate.  The next stage's barriers are looked at before this
-    // stage's turn ends.
+    // The whole warp runs the loop and one elected lane issues.  A pass is a chain of some 60 instructions that share their
+    // scheduler with the expanders: with 64 k and two or three barriers per pass it took 700 clocks and the tensor pipe
+    // stood at half its rate.  Hence 128 k to a stage, one barrier for all of its operands, and the look at the next
+    // stage's barrier issued before this stage's MMAs.
     const bool leader = elect_one();
     const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
-    int s = 0, par = 0, bt = 0, bph = 0, seg = 0;
+    int s = 0, par = 0, seg = 0;
     bool ok = true, wide_before = false;
-    auto look = [&]() {
-      const bool x = mbar_test_wait(a_full + 8 * s, par), y = mbar_test_wait(b_full + 8 * bt, bph);
-      return x && y && (CG == 1 || rank != 0 || mbar_test_wait(peer_full + 8 * s, par));
-    };
-    for (long long pos = pos0; pos < pos1 && ok; seg++) {
-      const int t = (int)(pos / nb), u0 = (int)(pos - (long long)t * nb), u1 = (int)min((long long)nb, u0 + (pos1 - pos));
+    for (int pos = pos0; pos < pos1 && ok; seg++) {
+      const int t = pos / nb, u0 = pos - t * nb, u1 = min(nb, u0 + (pos1 - pos));
       const int nt = __shfl_sync(0xffffffffu, wk.tile(t).nt, 0);
       const bool wide = nt > 128;
       if (rank == 0) {  // the accumulators this segment overwrites must have been read out
@@ -346,37 +347,34 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       wide_before = wide;
       const uint32_t d = tm + (wide ? 0 : 128 * (seg & 1));
       const uint32_t idesc = idesc_f16(128 * CG, 16, BF16) + ((uint32_t)((nt - 16) >> 3) << 17);
-      const int stages = (u1 - u0) * (SPC / 2);
+      const int stages = u1 - u0;
       uint32_t acc = 0;
-      bool ready = look();
+      bool ready = mbar_test_wait(full + 8 * s, par);
       for (int k = 0; k < stages; k++) {
-        if (!__all_sync(0xffffffffu, ready)) {
-          ok = warp_wait(a_full + 8 * s, par, abort) && warp_wait(b_full + 8 * bt, bph, abort);
-          if (CG == 2 && rank == 0) ok = ok && warp_wait(peer_full + 8 * s, par, abort);
-          if (!ok) break;
+        if (!__all_sync(0xffffffffu, ready) && !warp_wait(full + 8 * s, par, abort)) {
+          ok = false;
+          break;
         }
         tc_fence_after();
+        const uint64_t b0 = smem_desc_sw128(sB + s * a.stage_bytes), b1 = b0 + (uint64_t)(a.stage_bytes >> 5);
+        const uint32_t am = tm + A_COL + 64 * s, done = empty + 8 * s, fwd = full + 8 * s;
+        if (++s == NAS) s = 0, par ^= 1;
+        ready = mbar_test_wait(full + 8 * s, par);
         if (CG == 1 || rank == 0) {
-          const uint64_t b0 = smem_desc_sw128(sB + bt * a.stage_bytes), b1 = b0 + (uint64_t)(a.stage_bytes >> 5);
-          const uint32_t am = tm + A_COL + 64 * (s & (NAS - 1));
           if (leader) {
             mma_ts<CG>(d, am, b0, idesc, acc);
 #pragma unroll
             for (int j = 1; j < 4; j++) mma_ts<CG>(d, am + 8 * j, b0 + 2 * j, idesc, 1u);
 #pragma unroll
             for (int j = 0; j < 4; j++) mma_ts<CG>(d, am + 32 + 8 * j, b1 + 2 * j, idesc, 1u);
-            commit<CG>(a_empty + 8 * s);
-            commit<CG>(b_empty + 8 * bt);
+            commit<CG>(done);
           }
           acc = 1;
         } else {  // the pair's second CTA: its operands are ready, tell the one that issues
           tc_fence_before();
-          if (leader) mbar_arrive_remote(mapa(peer_full + 8 * s, 0));
+          if (leader) mbar_arrive_remote(mapa(fwd, 0));
         }
-        if (++bt == a.nbs) bt = 0, bph ^= 1;
-        if (++s == NAS) s = 0, par ^= 1;
         __syncwarp();
-        if (k + 1 < stages) ready = look();
       }
       if (ok && rank == 0 && leader) commit<CG>(d_full + 8 * (seg & 1));
       __syncwarp();
@@ -388,249 +386,322 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       for (int i = 0; i < (1 << 16) && !__all_sync(0xffffffffu, mbar_test_wait(drained, 0)); i++) {
       }
     }
-  } else if (warp < 8) {
-    // ================================================================ expanders
-    const int quad = warp & 3, half = warp >> 2;
-    const uint32_t wslot = sRaw + (uint32_t)warp * NSLOT * 32 * F::PITCH;
-    const size_t stride = Row::row_stride(ctx, a.K);
-    const int rofs = 128 * rank + quad * 32;  // the warp's first row within the tile
-    struct Cursor {
-      int c, u, t;  // chunk of the run, chunk within the tile, tile
-    };
-    auto at = [&](int c) {
-      const long long p = pos0 + c;
-      Cursor q;
-      q.c = c, q.t = (int)(p / nb), q.u = (int)(p - (long long)q.t * nb);
-      return q;
-    };
-    // ---- the copies run ahead of the expansion by NSLOT chunks of this warp
-    Cursor ic = at(half);
-    const uint8_t *ibase = nullptr, *ilim = nullptr;
-    uint32_t roff[F::GR];
-    constexpr bool SKEWED = std::is_same<Row, Q6KRow>::value;
-    auto aim = [&]() {
-      const Tile T = wk.tile(ic.t);
-      const int nw = min(T.n0 + rofs, a.N - 1);
-      Row r0;
-      r0.init(ctx, T.expert, nw, a.N, a.K);
-      ibase = row_ptr(r0);
-      if constexpr (SKEWED) ilim = r0.raw_end();
-#pragma unroll
-      for (int i = 0; i < F::GR; i++) {
-        const int q = lane + 32 * i, rr = q / F::GR, piece = q - rr * F::GR;
-        roff[i] = (uint32_t)(min(T.n0 + rofs + rr, a.N - 1) - nw) * (uint32_t)stride + (SKEWED ? 0 : piece * 16);
-      }
-    };
-    if (ic.c < n) aim();
-    int islot = 0;
-    constexpr int CBYTES = SKEWED ? 210 : std::is_same<Row, Q4KRow>::value ? 144 : std::is_same<Row, Q80Row>::value ? 272 : std::is_same<Row, DenseRow>::value ? 256 : 128;
-    auto issue = [&]() {  // always closes a commit group
-      if (ic.c < n) {
-        const uint8_t *src = ibase + (size_t)ic.u * CBYTES;
-        const uint32_t dst = wslot + islot * (32 * F::PITCH);
-#pragma unroll
-        for (int i = 0; i < F::GR; i++) {
-          const int q = lane + 32 * i, rr = q / F::GR, piece = q - rr * F::GR;
-          const uint32_t d = dst + (F::PITCH == F::GR * 16 ? (uint32_t)q * 16u : (uint32_t)(rr * F::PITCH + piece * 16));
-          if constexpr (SKEWED) {  // the 16-byte granules that cover the block
-            const uint8_t *s = reinterpret_cast<const uint8_t *>((uintptr_t)(src + roff[i]) & ~(uintptr_t)15) + piece * 16;
-            if (s + 16 <= ilim) cp_async16(d, s);
-            else if (s < ilim) cp_async16_part(d, s, (uint32_t)(ilim - s));
-          } else {
-            cp_async16(d, src + roff[i]);
-          }
-        }
-        islot = islot + 1 == NSLOT ? 0 : islot + 1;
-        ic.c += 2, ic.u += 2;
-        if (ic.u >= nb && ic.c < n) {
-          while (ic.u >= nb) ic.u -= nb, ic.t++;
-          aim();
-        }
-      }
-      cp_async_commit();
-    };
-#pragma unroll
-    for (int i = 0; i < NSLOT; i++) issue();
-
-    // ---- expansion
-    Cursor cc = at(half);
-    Row cur;
-    auto init_row = [&]() {
-      const Tile T = wk.tile(cc.t);
-      cur.init(ctx, T.expert, min(T.n0 + rofs + lane, a.N - 1), a.N, a.K);
-    };
-    auto advance = [&]() {
-      cc.c += 2, cc.u += 2;
-      if (cc.u >= nb && cc.c < n) {
-        while (cc.u >= nb) cc.u -= nb, cc.t++;
-        init_row();
-      }
-    };
-    if (cc.c < n) init_row();
-    if constexpr (HasAux<Row>::value) {
-      if (cc.c < n) cur.aux = cur.fetch_aux(cc.u);
-    }
-    int slot = 0, pending = -1;
-    bool ok = true;
-    const uint32_t lanes = (uint32_t)(quad * 32) << 16;
-    auto deliver = [&]() {  // the stage stored last is complete: hand it to the MMA warp
-      if (pending >= 0) {
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(a_full + 8 * pending);
-        pending = -1;
-      }
-    };
-    for (int c = half; c < n && ok; c += 2) {
-      cp_async_wait<NSLOT - 1>();
-      __syncwarp();
-      const uint32_t rs = wslot + slot * (32 * F::PITCH) + lane * F::PITCH;
-#pragma unroll
-      for (int l = 0; l < F::LOADS; l++) {
-        if constexpr (HasAux<Row>::value || std::is_same<Row, DenseRow>::value) cur.load_codes(rs + 128 * l);
-        else cur.load_smem(rs, cc.u * F::LOADS + l);
-        [[maybe_unused]] const Row here = cur;  // (registers; the pointers move on below)
-        if (l == F::LOADS - 1) {
-          __syncwarp();
-          issue();  // into the slot just read
-          advance();
-        }
-        if constexpr (HasAux<Row>::value) {  // the next chunk's scales arrive while this one is expanded
-          if (cc.c < n) cur.aux = cur.fetch_aux(cc.u);
-        }
-#pragma unroll
-        for (int j = 0; j < SPL; j++) {
-          const int it = c * SPC + l * SPL + j, s = (it >> 1) % NAS;
-          uint32_t o[32];
-          here.template emit<BF16>(j, [&](int ch, const uint4 &v) { o[4 * ch] = v.x, o[4 * ch + 1] = v.y, o[4 * ch + 2] = v.z, o[4 * ch + 3] = v.w; });
-          if (!((l * SPL + j) & 1)) {  // a new stage: hand over the one before, wait until this one's MMAs have completed
-            deliver();
-            if (it >= 2 * NAS) {
-              if (!warp_wait(a_empty + 8 * s, ((it / (2 * NAS)) - 1) & 1, abort)) {
-                ok = false;
-                break;
-              }
-              tc_fence_after();
-            }
-          }
-          __syncwarp();
-          tmem_st32(tmem + lanes + A_COL + 64 * s + 32 * (it & 1), o);
-          if ((l * SPL + j) & 1) pending = s;
-        }
-        if (!ok) break;
-      }
-      slot = slot + 1 == NSLOT ? 0 : slot + 1;
-    }
-    deliver();
-    cp_async_wait<0>();
   } else {
-    // ================================================================ epilogue
     const int quad = warp & 3, row = quad * 32 + lane;
     const uint32_t lanes = (uint32_t)(quad * 32) << 16;
-    float *const mine = a.parts + (size_t)blockIdx.x * PART_FLOATS + row;
-    int seg = 0;
-    for (long long pos = pos0; pos < pos1; seg++) {
-      const int t = (int)(pos / nb), u0 = (int)(pos - (long long)t * nb), u1 = (int)min((long long)nb, u0 + (pos1 - pos));
-      const Tile T = wk.tile(t);
-      pos += u1 - u0;
-      if (!warp_wait(d_full + 8 * (seg & 1), (seg >> 1) & 1, abort)) break;
-      tc_fence_after();
-      const uint32_t d = tmem + lanes + (T.nt > 128 ? 0 : 128 * (seg & 1));
-      const bool owner = u0 == 0, whole = owner && u1 == nb;
-      int jlast = cta;
-      bool ok = true;
-      if (owner && !whole) {  // the runs that hold the rest of this tile
-        const long long tile_end = (long long)(t + 1) * nb;
-        long long b = pos1;
-        while (jlast + 1 < G && b < tile_end) {
-          const long long b1 = wk.bound(++jlast + 1, G);
-          if (b1 > b && !wait_flag(g_flags + (jlast * CG + rank) * 4 + quad, abort)) ok = false;
-          b = b1;
+    // Columns c0 .. c0 + 31 of the accumulator at `d` into registers (a tile's last chunk may hold 16).
+    auto take = [&](uint32_t d, int c0, int nt, uint32_t (&v)[32]) {
+      __syncwarp();
+      if (c0 + 32 <= nt) {
+        tmem_ld32(d + c0, v);
+        tmem_ld_wait();
+      } else {
+        uint32_t h[16];
+        tmem_ld16(d + c0, h);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = h[i], v[16 + i] = 0u;
+      }
+    };
+    // Sixteen columns of a partial tile (those past the tile's tokens are written and read too); then, once all of a warp's
+    // chunks first, first + step, .. < nt are on their way, their flags.
+    auto put_part = [&](int c0, const uint32_t *v) {
+      float *mine = a.parts + (size_t)blockIdx.x * PART_FLOATS + row + c0 * 128;
+#pragma unroll
+      for (int i = 0; i < 16; i++) __stcg(mine + i * 128, __uint_as_float(v[i]));
+    };
+    auto raise_flags = [&](int first, int step, int nt) {
+      __threadfence();
+      __syncwarp();
+      const int c0 = first + lane * step;
+      if (c0 < nt) asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(g_flags + (blockIdx.x * 4 + quad) * 16 + (c0 >> 4)), "r"(1u) : "memory");
+    };
+    // Output row (-1: none) and routing weight of token c0 + lane of a tile.
+    auto route = [&](const Tile &T, int c0, int &prow, float &pw) {
+      prow = -1, pw = 1.f;
+      if (T.m0 + c0 + lane < T.m_end) {
+        prow = T.m0 + c0 + lane;
+        if (a.offsets) {
+          const long long p = a.pairs[prow];
+          prow = p >= 0 && p < a.size_m ? (int)p : -1;
+          if (prow >= 0 && a.topkw) pw = a.topkw[p];
         }
       }
-      const int ncol = T.m_end - T.m0, col = T.n0 + 128 * rank + row;
+    };
+    // The run's last segment, 16 tokens at a time: chunks first, first + step, ...  `shared`: five warps of this row quarter take
+    // turns (only where K is long enough that an expander cannot get here before the segment before the last but one is
+    // complete: the barrier's phase parity tells those two apart from one another, not from earlier ones).  What a chunk
+    // costs is latency (flags, partial sums, stores): the flags of all runs that hold a part of the tile are polled at
+    // once, a lane to each, and the partial sums of two runs are on their way together.
+    const bool shared = nb >= 8;
+    auto finish_last = [&](int first, int step) {
+      const int t = (pos1 - 1) / nb, u0 = max(pos0 - t * nb, 0), u1 = pos1 - t * nb, seg = t - pos0 / nb;
+      const Tile T = wk.tile(t);
+      if (first >= T.nt) return;
+      const bool owner = u0 == 0;
+      int jlast = cta;  // the runs that hold the rest of this tile
+      if (owner && u1 < nb)
+        while (jlast + 1 < G && wk.bound(jlast + 1, G) < (t + 1) * nb) jlast++;
+      const int col = T.n0 + 128 * rank + row;
       const bool live = col < a.N;
+      if (!warp_wait(d_full + 8 * (seg & 1), (seg >> 1) & 1, abort)) return;
+      tc_fence_after();
+      const uint32_t d = tmem + lanes + (T.nt > 128 ? 0 : 128 * (seg & 1));
+      if (jlast > cta) {  // all parts of this warp's chunks: (run, chunk) pairs, a lane to each
+        const int chunks = (T.nt - first + step - 1) / step;
+        for (int i0 = 0; i0 < (jlast - cta) * chunks; i0 += 32) {
+          const int i = i0 + lane, j = min(cta + 1 + i / chunks, jlast), c0 = first + (i % chunks) * step;
+          const bool has = i < (jlast - cta) * chunks && wk.bound(j, G) < wk.bound(j + 1, G);  // (an empty run writes nothing)
+          unsigned *flag = g_flags + ((j * CG + rank) * 4 + quad) * 16 + (c0 >> 4);
+          if (!wait_flag(flag, has, abort)) return;
+          if (has) *flag = 0u;  // for the next launch
+        }
+      }
 #pragma unroll 1
-      for (int c0 = 0; c0 < T.nt; c0 += 32) {
-        uint32_t v[32];
+      for (int c0 = first; c0 < T.nt; c0 += step) {
+        uint32_t v[16];
         __syncwarp();
-        if (c0 + 32 <= T.nt) {
-          tmem_ld32(d + c0, v);
-        } else {
-          uint32_t h[16];
-          tmem_ld16(d + c0, h);
-#pragma unroll
-          for (int i = 0; i < 16; i++) v[i] = h[i], v[16 + i] = 0u;
-        }
+        tmem_ld16(d + c0, v);
         tmem_ld_wait();
-        if (c0 + 32 >= T.nt) {  // the last of it is in registers: the accumulator is free
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if constexpr (CG == 1) mbar_arrive(d_empty + 8 * (seg & 1));
-            else mbar_arrive_remote(mapa(d_empty + 8 * (seg & 1), 0));
-          }
-        }
-        if (!owner) {  // (columns past the tile's tokens are written and read too: the slot has room for 256)
-#pragma unroll
-          for (int i = 0; i < 32; i++) __stcg(mine + (c0 + i) * 128, __uint_as_float(v[i]));
+        if (!owner) {
+          put_part(c0, v);
           continue;
         }
-        for (int j = cta + 1; j <= jlast && ok; j++) {
-          if (a.offsets && wk.bound(j, G) == wk.bound(j + 1, G)) continue;  // an empty run wrote nothing
-          const float *theirs = a.parts + (size_t)(j * CG + rank) * PART_FLOATS + row + c0 * 128;
-          float p[32];
+        for (int j0 = cta + 1; j0 <= jlast; j0 += 32) {
+          const int j = j0 + lane;
+          const bool has = j <= jlast && wk.bound(j, G) < wk.bound(j + 1, G);
+          unsigned left = __ballot_sync(0xffffffffu, has);
+          const float *theirs = a.parts + row + c0 * 128 + (size_t)rank * PART_FLOATS;
+          while (left) {
+            const int ja = j0 + __ffs(left) - 1;
+            left &= left - 1;
+            const int jb = left ? j0 + __ffs(left) - 1 : -1;
+            left &= left - 1;
+            float p[16], q[16];
 #pragma unroll
-          for (int i = 0; i < 32; i++) p[i] = __ldcg(theirs + i * 128);
+            for (int i = 0; i < 16; i++) p[i] = __ldcg(theirs + (size_t)ja * CG * PART_FLOATS + i * 128);
+            if (jb >= 0) {
 #pragma unroll
-          for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) + p[i]);
+              for (int i = 0; i < 16; i++) q[i] = __ldcg(theirs + (size_t)jb * CG * PART_FLOATS + i * 128);
+            }
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) + p[i]);
+            if (jb >= 0) {
+#pragma unroll
+              for (int i = 0; i < 16; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) + q[i]);
+            }
+          }
         }
         if (!a.offsets) {  // consecutive output rows
           OutT *o = out + (size_t)(T.m0 + c0) * a.N + col;
-          if (c0 + 32 <= ncol) {
+          const int ncol = T.m_end - T.m0 - c0;
 #pragma unroll
-            for (int i = 0; i < 32; i++, o += a.N) st_if(live, o, __uint_as_float(v[i]));
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; i++, o += a.N) st_if(live && c0 + i < ncol, o, __uint_as_float(v[i]));
-          }
+          for (int i = 0; i < 16; i++, o += a.N) st_if(live && i < ncol, o, __uint_as_float(v[i]));
         } else {
-          int prow = -1;  // output row and weight of token c0 + lane
-          float pw = 1.f;
-          if (c0 + lane < ncol) {
-            const long long p = a.pairs[T.m0 + c0 + lane];
-            if (p >= 0 && p < a.size_m) {
-              prow = (int)p;
-              if (a.topkw) pw = a.topkw[p];
-            }
-          }
+          int prow;
+          float pw;
+          route(T, c0, prow, pw);
           OutT *o = out + col;
 #pragma unroll
-          for (int i0 = 0; i0 < 32; i0 += 8) {
-            int m[8];
-            float f[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) m[i] = __shfl_sync(0xffffffffu, prow, i0 + i), f[i] = __shfl_sync(0xffffffffu, pw, i0 + i) * __uint_as_float(v[i0 + i]);
-#pragma unroll
-            for (int i = 0; i < 8; i++) st_if(live && m[i] >= 0, o + (long long)m[i] * a.N, f[i]);
+          for (int i = 0; i < 16; i++) {
+            const int m = __shfl_sync(0xffffffffu, prow, i);
+            const float f = __shfl_sync(0xffffffffu, pw, i) * __uint_as_float(v[i]);
+            st_if(live && m >= 0, o + (long long)m * a.N, f);
           }
         }
       }
-      __syncwarp();
-      if (!owner) {  // this warp's rows of the partial tile are written: raise its flag
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(g_flags + blockIdx.x * 4 + quad), "r"(1u) : "memory");
-      } else if (!whole) {  // the partials have been read: lower the flags for the next launch
-        for (int j = cta + 1 + lane; j <= jlast; j += 32) g_flags[(j * CG + rank) * 4 + quad] = 0u;
+      if (!owner) raise_flags(first, step, T.nt);
+    };
+
+    if (warp < EXPANDERS) {
+      // ================================================================ expanders
+      const int set = warp >> 2;
+      const uint32_t slot = sRaw + (uint32_t)warp * Row::SLOT, copied = w_full + 8 * warp;
+      const int rofs = 128 * rank + quad * 32;  // the warp's first row within the tile
+      if constexpr (std::is_same<Row, TmDense>::value) pdl_wait();  // (a dense weight may have been expanded just now)
+      // this warp's next unit: number in the run, in the tile, and the tile
+      int c = set, u, t;
+      t = (pos0 + c) / nb, u = pos0 + c - t * nb;
+      Row rowx(ctx);
+      [[maybe_unused]] int y = 0;                 // TMA: the warp's first row among all experts' rows
+      [[maybe_unused]] const uint8_t *src = nullptr;  // row copies: its address, and the rows of the matrix after it
+      [[maybe_unused]] int rows = 0;
+      auto aim = [&]() {
+        const Tile T = wk.tile(t);
+        const int nw = min(T.n0 + rofs, a.N - 1);
+        const size_t r0 = (size_t)T.expert * a.N;
+        y = (int)(r0 + nw);
+        if constexpr (Row::BOXES == 0) src = Row::base(ctx) + (r0 + nw) * Row::stride(a.K), rows = a.N - 1 - nw;
+        rowx.row(ctx, (int)r0 + min(nw + lane, a.N - 1), a.K);
+      };
+      auto issue = [&]() {
+        if constexpr (Row::BOXES > 0) {
+          if (lane == 0) {
+            mbar_arrive_expect_tx(copied, Row::BYTES);
+            Row::copy(slot, maps.w, copied, u, y);
+          }
+        } else {
+          // Lanes 10 r + i copy granule i of rows r, r + 3, ..: the granule's place in the block is the lane's own, and the
+          // next row is one addition away.
+          const int r0 = lane / 10, i = lane - 10 * r0;
+          const size_t step = Row::stride(a.K);
+          const uint8_t *at = src + (u >> 1) * 210;
+          const uint32_t dst = slot + r0 * Row::PITCH + 16 * i;
+          const int place = 16 * Row::number(u & 1, i);
+          if (lane < 30) {
+            if (rows >= 32) {  // (a whole row follows the last one: no copy passes the end of the matrix)
+              at += (size_t)r0 * step;
+#pragma unroll
+              for (int k = 0; k < 11; k++, at += 3 * step)
+                if (k < 10 || r0 < 2) cp_async16(dst + 3 * k * Row::PITCH, reinterpret_cast<const uint8_t *>((uintptr_t)at & ~(uintptr_t)15) + place);
+            } else {
+              const uint8_t *const end = Row::base(ctx) + (size_t)a.E * a.N * step;
+              for (int k = 0; k < 11; k++)
+                if (k < 10 || r0 < 2) {
+                  const uint8_t *g = reinterpret_cast<const uint8_t *>((uintptr_t)(at + (size_t)min(r0 + 3 * k, rows) * step) & ~(uintptr_t)15) + place;
+                  if (g + 16 <= end) cp_async16(dst + 3 * k * Row::PITCH, g);
+                  else if (g < end) cp_async16_part(dst + 3 * k * Row::PITCH, g, (uint32_t)(end - g));
+                }
+            }
+          }
+          cp_async_commit();
+        }
+      };
+      const uint32_t acol = tmem + lanes + A_COL + 64 * set;  // (four sets, four stages: always the same one)
+      if (c < n) {
+        aim();
+        issue();
+        rowx.fetch_scales(ctx, u);
       }
+      bool ok = true;
+      for (int round = 0; c < n && ok; round++) {
+        if constexpr (Row::BOXES > 0) {
+          if (!warp_wait(copied, round & 1, abort)) break;
+        } else {
+          cp_async_wait<0>();
+          __syncwarp();
+        }
+        rowx.load(slot, u);
+        const int now = u;
+        auto next = [&]() {  // everything of this unit is in registers: on to the next one
+          if constexpr (Row::BOXES > 0) fence_proxy_async();  // the reads above come before the copy that overwrites the slot
+          __syncwarp();
+          c += EXPANDERS / 4, u += EXPANDERS / 4;
+          if (c < n) {
+            if (u >= nb) {
+              while (u >= nb) u -= nb, t++;
+              aim();
+            }
+            issue();
+            rowx.fetch_scales(ctx, u);
+          }
+        };
+        if constexpr (!ReadsLate<Row>::value) next();
+        rowx.template expand<BF16>(now, [&](int p, const uint32_t (&o)[16]) {
+          if (p == 0 && round > 0) {  // the stage's MMAs of the round before
+            ok = warp_wait(empty + 8 * set, (round - 1) & 1, abort);
+            tc_fence_after();
+          }
+          __syncwarp();
+          if (ok) tmem_st16(acol + 16 * p, o);
+        });
+        if constexpr (ReadsLate<Row>::value) next();
+        if (!ok) break;
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full + 8 * set);
+      }
+      if constexpr (Row::BOXES == 0) cp_async_wait<0>();
+      __syncwarp();
+      pdl_wait();
+      if (ok && n > 0 && shared) finish_last(16 * (1 + set), 80);
+    } else {
+      // ================================================================ epilogue
+      pdl_wait();  // `out` and the partial tiles may still be in use by the kernel before
+      const uint32_t strip = sStrip, sbytes = STRIP<OutT>;
+      const bool bulk = ((size_t)a.N * sizeof(OutT)) % 16 == 0 && ((uintptr_t)out & 15) == 0;
+      int seg = 0, chunk = 0;
+      for (int pos = pos0; pos < pos1; seg++) {
+        const int t = pos / nb, u0 = pos - t * nb, u1 = min(nb, u0 + (pos1 - pos));
+        const Tile T = wk.tile(t);
+        pos += u1 - u0;
+        if (pos >= pos1) {
+          finish_last(0, shared ? 80 : 16);
+          break;
+        }
+        if (!warp_wait(d_full + 8 * (seg & 1), (seg >> 1) & 1, abort)) break;
+        tc_fence_after();
+        const uint32_t d = tmem + lanes + (T.nt > 128 ? 0 : 128 * (seg & 1));
+        const int n0 = T.n0 + 128 * rank, ncols = min(128, a.N - n0);  // (<= 0: no rows of the matrix here)
+#pragma unroll 1
+        for (int c0 = 0; c0 < T.nt; c0 += 32, chunk++) {
+          uint32_t v[32];
+          take(d, c0, T.nt, v);
+          if (c0 + 32 >= T.nt) {  // the last of it is in registers: the accumulator is free
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+              if constexpr (CG == 1) mbar_arrive(d_empty + 8 * (seg & 1));
+              else mbar_arrive_remote(mapa(d_empty + 8 * (seg & 1), 0));
+            }
+          }
+          if (u0 > 0) {
+            put_part(c0, v);
+            if (c0 + 16 < T.nt) put_part(c0 + 16, v + 16);
+            if (c0 + 32 >= T.nt) raise_flags(0, 16, T.nt);
+            continue;
+          }
+          int prow;
+          float pw;
+          route(T, c0, prow, pw);
+          if (a.topkw) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * __shfl_sync(0xffffffffu, pw, i));
+          }
+          if (bulk) {
+            constexpr bool two = 2 * STRIP<OutT> <= STRIPS;
+            const uint32_t buf = strip + (two ? (chunk & 1) * sbytes : 0);
+            if (two) asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");  // this lane's last copy from this strip
+            else asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+            asm volatile("bar.sync 1, 128;\n" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < 32; i++) {
+              if constexpr (sizeof(OutT) == 4) {
+                asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(buf + (uint32_t)(i * 128 + row) * 4u), "r"(v[i]) : "memory");
+              } else {
+                const __nv_bfloat16 h = __float2bfloat16_rn(__uint_as_float(v[i]));
+                asm volatile("st.shared.u16 [%0], %1;\n" ::"r"(buf + (uint32_t)(i * 128 + row) * 2u), "h"(*reinterpret_cast<const uint16_t *>(&h)) : "memory");
+              }
+            }
+            fence_proxy_async();
+            asm volatile("bar.sync 1, 128;\n" ::: "memory");
+            const int i = (warp - EPI_WARP) * 8 + (lane & 7), m = __shfl_sync(0xffffffffu, prow, i);  // a warp sends eight of the 32 tokens
+            if (lane < 8 && m >= 0 && ncols > 0)
+              asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(out + (long long)m * a.N + n0),
+                           "r"(buf + (uint32_t)(i * 128) * (uint32_t)sizeof(OutT)), "r"((uint32_t)ncols * (uint32_t)sizeof(OutT))
+                           : "memory");
+            asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+          } else {
+            OutT *o = out + n0 + row;
+#pragma unroll
+            for (int i = 0; i < 32; i++) {
+              const int m = __shfl_sync(0xffffffffu, prow, i);
+              st_if(row < ncols && m >= 0, o + (long long)m * a.N, __uint_as_float(v[i]));
+            }
+          }
+        }
+      }
+      asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
     }
   }
   __syncwarp();
-  if (abort_flag && threadIdx.x == 0) g_status = 1;
   tc_fence_before();
   __syncthreads();
+  if (abort_flag) {  // copies still in flight get some time to land before the CTA retires
+    __nanosleep(50000);
+    if (threadIdx.x == 0) g_status = 1;
+  }
   if constexpr (CG == 2) cluster_sync();  // nobody leaves while the peer may still signal its barriers
   if (warp == MMA_WARP) dealloc512<CG>(tmem);
 }
@@ -652,40 +723,47 @@ int knob(const char *name, int otherwise) {
   return e ? atoi(e) : otherwise;
 }
 
-template <typename Row> constexpr int narrow_slots() { return Fmt<Row>::PITCH > 144 ? 2 : 4; }
+template <typename Row>
+constexpr int fixed_smem(int E) { return EXPANDERS * Row::SLOT + STRIPS + BAR_BYTES + (E + 1) * 12 + 16 + 1024; }
 
-template <typename Row, bool BF16, typename OutT, int CG, int NSLOT>
+template <typename Row, bool BF16, typename OutT, int CG>
 int run(const typename Row::Ctx &ctx, const TmemCall &c, Args a, int nt_max, cudaStream_t st) {
-  using F = Fmt<Row>;
-  // token ring: what shared memory the weight slots leave, up to eight stages of 64 k
   a.nt_max = nt_max;
   const int rows = nt_max / CG;
-  a.box = c.offsets ? 32 : rows;
+  a.box = !c.offsets ? rows : rows % 32 ? 16 : 32;
   a.stage_bytes = (rows + a.box - 1) / a.box * a.box * 256;
-  const int fixed = 8 * NSLOT * 32 * F::PITCH + 512 + (a.E + 1) * 12 + 16 + 1024;
-  a.nbs = (SMEM_MAX - fixed) / a.stage_bytes;
-  if (a.nbs > 8) a.nbs = 8;
-  if (a.nbs < 2) return 0;
+  const int smem = NAS * a.stage_bytes + fixed_smem<Row>(a.E);
+  if (smem > SMEM_MAX) return 0;
   int G = sm_count() / CG;
   if (G * CG > MAX_GRID) G = MAX_GRID / CG;
   if (!c.offsets) {
     const int ntt = (int)((c.M + nt_max - 1) / nt_max);
-    const long long U = (long long)ntt * ((c.N + 128 * CG - 1) / (128 * CG)) * (c.K / F::KU), least = c.min_run_k / F::KU;
+    const long long U = (long long)ntt * ((c.N + 128 * CG - 1) / (128 * CG)) * (c.K / KU), least = c.min_run_k / KU;
+    if (U >= 1ll << 27) return 0;
     if (U / least < G) G = (int)(U / least > 0 ? U / least : 1);
   }
   if (c.parts_bytes < (size_t)G * CG * PART_FLOATS * 4) return 0;
   a.parts = (float *)c.parts;
   const EncodeTiledFn enc = encode_fn();
   if (!enc) return fail(LB200_E_DEVICE, "light_b200: cuTensorMapEncodeTiled is not available from the driver");
-  CUtensorMap tm;
+  Maps tm;
   const cuuint64_t dims[2] = {(cuuint64_t)c.K, (cuuint64_t)c.M};
   const cuuint64_t strides[1] = {(cuuint64_t)c.K * 2};
   const cuuint32_t box[2] = {64, (cuuint32_t)a.box}, estr[2] = {1, 1};
-  const CUresult r = enc(&tm, BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(c.x16), dims, strides, box, estr,
+  CUresult r = enc(&tm.x, BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(c.x16), dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  tm.w[0] = tm.w[1] = tm.x;
+  if constexpr (Row::BOXES > 0) {
+    const cuuint64_t wdims[2] = {(cuuint64_t)Row::stride(c.K), (cuuint64_t)a.E * c.N}, wstr[1] = {wdims[0]};
+    for (int i = 0; i < Row::BOXES && r == CUDA_SUCCESS; i++) {
+      const cuuint32_t wbox[2] = {(cuuint32_t)Row::BOX[i].bytes, 32};
+      const CUtensorMapSwizzle sw = Row::BOX[i].swizzle == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : Row::BOX[i].swizzle == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE;
+      r = enc(&tm.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(Row::base(ctx)), wdims, wstr, wbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    }
+  }
   if (r != CUDA_SUCCESS) return fail(LB200_E_SHAPE, "light_b200: cuTensorMapEncodeTiled failed (%d)", (int)r);
-  auto kern = gemm_tmem_kernel<Row, BF16, OutT, CG, NSLOT>;
-  const int smem = a.nbs * a.stage_bytes + fixed;
+  auto kern = gemm_tmem_kernel<Row, BF16, OutT, CG>;
   static DeviceOnce attr;
   cudaError_t e = attr.ensure([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX); });
   if (e != cudaSuccess) return fail((int)e, "light_b200: gemm (tmem): %s", cudaGetErrorString(e));
@@ -694,10 +772,12 @@ int run(const typename Row::Ctx &ctx, const TmemCall &c, Args a, int nt_max, cud
   cfg.blockDim = dim3(THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = CG, at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = 1;
-  cfg.attrs = at, cfg.numAttrs = CG > 1 ? 1 : 0;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = CG, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
+  cfg.attrs = at, cfg.numAttrs = CG > 1 ? 2 : 1;
   e = cudaLaunchKernelEx(&cfg, kern, tm, ctx, a, (OutT *)c.out);
   if (e != cudaSuccess) return fail((int)e, "light_b200: gemm (tmem): %s", cudaGetErrorString(e));
   if (int rc = launched("gemm (weights through tensor memory)")) return rc;
@@ -706,23 +786,31 @@ int run(const typename Row::Ctx &ctx, const TmemCall &c, Args a, int nt_max, cud
 
 template <typename Row, bool BF16, typename OutT>
 int pick(const typename Row::Ctx &ctx, const TmemCall &c, cudaStream_t st) {
-  if (c.K % Fmt<Row>::KU || c.E > MAX_E) return 0;
+  if (c.K % KU || c.E > MAX_E || (c.offsets && (c.M / 16 + c.E) * ((c.N + 127) / 128) * (c.K / KU) >= 1ll << 31)) return 0;
   Args a = {};
   a.offsets = c.offsets, a.pairs = c.pairs, a.topkw = c.topkw, a.size_m = c.size_m;
   a.E = c.offsets ? c.E : 1, a.M = (int)c.M, a.N = c.N, a.K = c.K;
-  static const int k_cg = knob("LIGHT_B200_TMEM_CG", 0), k_nt = knob("LIGHT_B200_TMEM_NT", 0), k_wmin = knob("LIGHT_B200_TMEM_WMIN", 96);
+  static const int k_cg = knob("LIGHT_B200_TMEM_CG", 0), k_nt = knob("LIGHT_B200_TMEM_NT", 0), k_wmin = knob("LIGHT_B200_TMEM_WMIN", 128), k_pair = knob("LIGHT_B200_TMEM_PAIR", 0);
   a.wmin = k_wmin;
-  // the token tile: at most 256, all tiles of a matrix alike
-  const int cap = k_nt ? k_nt : 256;
-  int cg = k_cg ? k_cg : c.mean_tokens > 192 ? 2 : 1;
+  // The token tile: at most 256 (two SMs; less where the weight slots leave less room), all tiles of a matrix alike.  One SM
+  // alone takes up to 128, with two accumulators.
+  int rows = (SMEM_MAX - fixed_smem<Row>(a.E)) / (NAS * 256) / 16 * 16;
+  if (rows > 128) rows = 128;
+  // Two SMs to a tile halve the token traffic and the number of times a weight is expanded, one SM has the shorter chain of
+  // hand-overs.  Measured crossing: 32 units per SM (333 tokens, 4096 x 4096: 21.6 us alone, 22.9 in pairs; 4096 x 14336: 46
+  // against 40); grouped, 64 tokens per expert on average (64 experts of 2048 x 2048, 64 tokens: 95 against 88 us).
+  const bool big = c.offsets ? c.mean_tokens >= (k_pair ? k_pair : 64)
+                             : c.M > 128 && (long long)((c.N + 127) / 128) * ((c.M + 127) / 128) * (c.K / KU) >= (k_pair ? k_pair : 32) * sm_count();
+  const int cg = k_cg ? k_cg : big ? 2 : 1;
+  int cap = rows * cg;
+  if (k_nt && k_nt < cap) cap = k_nt;
   int nt = cap;
   if (!c.offsets) {
     const int ntt = (int)((c.M + cap - 1) / cap);
     nt = (int)((c.M + ntt - 1) / ntt + 16 * cg - 1) / (16 * cg) * (16 * cg);
   }
-  if (cg == 2) return run<Row, BF16, OutT, 2, 1>(ctx, c, a, nt, st);
-  if (nt <= 64) return run<Row, BF16, OutT, 1, narrow_slots<Row>()>(ctx, c, a, nt, st);
-  return run<Row, BF16, OutT, 1, 1>(ctx, c, a, nt, st);
+  if (cg == 2) return run<Row, BF16, OutT, 2>(ctx, c, a, nt, st);
+  return run<Row, BF16, OutT, 1>(ctx, c, a, nt, st);
 }
 
 }  // namespace
@@ -731,16 +819,18 @@ size_t gemm_tmem_parts_bytes() { return (size_t)MAX_GRID * PART_FLOATS * 4; }
 
 int gemm_tmem(const TmemCall &c, cudaStream_t st) {
   switch (c.kind) {
-    case TmemCall::Q4K: return pick<Q4KRow, false, float>(GgufCtx{(const uint8_t *)c.w}, c, st);
-    case TmemCall::Q6K: return pick<Q6KRow, false, float>(GgufCtx{(const uint8_t *)c.w}, c, st);
-    case TmemCall::Q80: return pick<Q80Row, false, float>(GgufCtx{(const uint8_t *)c.w}, c, st);
-    case TmemCall::INT4:
-      if (c.bf16) return pick<Int4Row, true, __nv_bfloat16>(Int4Ctx{(const uint32_t *)c.w, c.s, c.z, c.G}, c, st);
-      return pick<Int4Row, false, float>(Int4Ctx{(const uint32_t *)c.w, c.s, c.z, c.G}, c, st);
-    case TmemCall::FP8:
-      if (c.bf16) return pick<Fp8Row, true, __nv_bfloat16>(Fp8Ctx{(const uint8_t *)c.w, c.s, c.bR, c.bC}, c, st);
-      return pick<Fp8Row, false, float>(Fp8Ctx{(const uint8_t *)c.w, c.s, c.bR, c.bC}, c, st);
-    case TmemCall::DENSE: return pick<DenseRow, true, __nv_bfloat16>(DenseCtx{(const uint16_t *)c.w}, c, st);
+    case TmemCall::Q4K: return pick<TmQ4K, false, float>({(const uint8_t *)c.w}, c, st);
+    case TmemCall::Q6K: return pick<TmQ6K, false, float>({(const uint8_t *)c.w}, c, st);
+    case TmemCall::Q80: return pick<TmQ80, false, float>({(const uint8_t *)c.w}, c, st);
+    case TmemCall::INT4: {
+      const TmInt4::Ctx x{(const uint32_t *)c.w, c.s, c.z, c.G, Div::of(c.G / 64)};
+      return c.bf16 ? pick<TmInt4, true, __nv_bfloat16>(x, c, st) : pick<TmInt4, false, float>(x, c, st);
+    }
+    case TmemCall::FP8: {
+      const TmFp8::Ctx x{(const uint8_t *)c.w, c.s, c.bR, c.bC, Div::of(c.bC / 64)};
+      return c.bf16 ? pick<TmFp8, true, __nv_bfloat16>(x, c, st) : pick<TmFp8, false, float>(x, c, st);
+    }
+    case TmemCall::DENSE: return pick<TmDense, true, __nv_bfloat16>({(const uint16_t *)c.w}, c, st);
   }
   return 0;
 }

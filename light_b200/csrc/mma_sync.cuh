@@ -1,5 +1,6 @@
 // Small PTX wrappers shared by the register-fed (mma.sync) decode kernels.
 #pragma once
+#include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace lb {
@@ -54,6 +55,17 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+// Launches a kernel that calls pdl_wait() itself: its CTAs may start while the kernel before is still running.
+template <typename... P, typename... A>
+cudaError_t launch_early(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid, cfg.blockDim = block, cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at, cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
 
 }  // namespace
 }  // namespace lb

@@ -727,6 +727,8 @@ __global__ void __launch_bounds__(THREADS, 1) prefill_sk_kernel(const __grid_con
 // PERM: every four consecutive k are stored in the order 0, 2, 1, 3 (what a KPERM row expander pairs them with).
 template <bool PERM>
 __global__ void __launch_bounds__(256) x_to_f16_kernel(const float4 *__restrict__ x, uint2 *__restrict__ y, long long n4) {
+  pdl_launch_dependents();
+  pdl_wait();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
     float4 v = __ldg(x + i);
     v.x = fminf(fmaxf(v.x, -65504.f), 65504.f), v.y = fminf(fmaxf(v.y, -65504.f), 65504.f);
@@ -767,9 +769,9 @@ int make_x_map(CUtensorMap *tm, const void *x, int act_dtype, int M, int K, void
     long long blocks = (n4 + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
     if (perm)
-      x_to_f16_kernel<true><<<(unsigned)blocks, 256, 0, st>>>((const float4 *)x, (uint2 *)ws, n4);
+      launch_early(x_to_f16_kernel<true>, dim3((unsigned)blocks), dim3(256), st, (const float4 *)x, (uint2 *)ws, n4);
     else
-      x_to_f16_kernel<false><<<(unsigned)blocks, 256, 0, st>>>((const float4 *)x, (uint2 *)ws, n4);
+      launch_early(x_to_f16_kernel<false>, dim3((unsigned)blocks), dim3(256), st, (const float4 *)x, (uint2 *)ws, n4);
     if (int rc = launched("prefill: activations to f16")) return rc;
     src = ws;
     dt = CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
@@ -924,6 +926,7 @@ template <> TmemCall tmem_call<DenseRow>(const DenseCtx &c) {
   t.kind = TmemCall::DENSE, t.w = c.w;
   return t;
 }
+constexpr int NOT_COVERED = -1000;
 int use_tmem() {
   static const int v = getenv("LIGHT_B200_TMEM") ? atoi(getenv("LIGHT_B200_TMEM")) : 1;
   return v;
@@ -936,7 +939,7 @@ int tmem_min_run() {
 // f32 activations run with f16 operands and f32 output, bf16 activations with bf16 operands and output
 template <typename Row>
 int launch_by_act(const void *x, int act_dtype, const typename Row::Ctx &ctx, void *out, int M, int N, int K, void *ws,
-                  size_t ws_bytes, cudaStream_t st) {
+                  size_t ws_bytes, cudaStream_t st, bool older = true) {
   CUtensorMap tm;
   if (Row::KPERM && act_dtype != LB200_F32)
     return fail(LB200_E_DTYPE, "light_b200: prefill: this weight format takes f32 activations only");
@@ -952,6 +955,7 @@ int launch_by_act(const void *x, int act_dtype, const typename Row::Ctx &ctx, vo
     c.mean_tokens = M, c.min_run_k = tmem_min_run(), c.parts = sk, c.parts_bytes = sk_bytes;
     if (int took = gemm_tmem(c, st)) return took == 1 ? 0 : took;
   }
+  if (!older) return NOT_COVERED;
   if (act_dtype == LB200_F32) return launch<Row, false, float>(tm, ctx, none, (float *)out, M, N, K, st, sk, sk_bytes);
   if constexpr (!Row::KPERM) return launch<Row, true, __nv_bfloat16>(tm, ctx, none, (__nv_bfloat16 *)out, M, N, K, st, sk, sk_bytes);
   return LB200_E_DTYPE;
@@ -996,10 +1000,12 @@ void pf_knobs() {
 // does not allow it, any other value is an error.
 int gguf_prefill(int type, const float *x, const void *w, float *out, int M, int N, int K, int device, cudaStream_t st) {
   if (M < PREFILL_MIN_M || K % 256) return 0;
+  bool older = true;
   if (type == LB200_Q4_K) {
     if ((uintptr_t)w & 15) return 0;
   } else if (type == LB200_Q6_K) {
-    if (((uintptr_t)w & 3) || ((size_t)(K >> 8) * 210) % 4) return 0;  // rows must start 4-byte aligned
+    older = !((uintptr_t)w & 3) && (K >> 8) % 2 == 0;  // (the older kernel wants rows that start 4-byte aligned)
+    if (!older && !use_tmem()) return 0;
   } else if (type == LB200_Q8_0) {
     if ((uintptr_t)w & 15) return 0;  // K % 256 == 0 makes every row a whole number of 16-byte granules
   } else {
@@ -1010,8 +1016,9 @@ int gguf_prefill(int type, const float *x, const void *w, float *out, int M, int
   if (!get_ws(device, LB200_F32, M, K, &ws, &wsb)) return 0;
   GgufCtx ctx{(const uint8_t *)w};
   int rc = type == LB200_Q4_K   ? launch_by_act<Q4KRow>(x, LB200_F32, ctx, out, M, N, K, ws, wsb, st)
-           : type == LB200_Q6_K ? launch_by_act<Q6KRow>(x, LB200_F32, ctx, out, M, N, K, ws, wsb, st)
+           : type == LB200_Q6_K ? launch_by_act<Q6KRow>(x, LB200_F32, ctx, out, M, N, K, ws, wsb, st, older)
                                 : launch_by_act<Q80Row>(x, LB200_F32, ctx, out, M, N, K, ws, wsb, st);
+  if (rc == NOT_COVERED) return 0;
   return rc ? rc : 1;
 }
 
@@ -1046,6 +1053,8 @@ template <typename TI, bool PERM>
 __global__ void __launch_bounds__(256) gather_rows_kernel(const TI *__restrict__ in, const int64_t *__restrict__ pairs,
                                                           uint16_t *__restrict__ dst, long long Mp, int K, int topk,
                                                           int row_per_pair, long long size_m) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   for (long long i = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); i < Mp; i += (long long)gridDim.x * 8) {
     const long long p = pairs[i];
@@ -1069,12 +1078,12 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const TI *__restrict__
 }
 
 template <typename Row, bool BF16, typename OutT, typename TI>
-int moe_launch(const lb200_moe_args *a, const typename Row::Ctx &ctx, void *ws, size_t ws_bytes, cudaStream_t st) {
+int moe_launch(const lb200_moe_args *a, const typename Row::Ctx &ctx, void *ws, size_t ws_bytes, cudaStream_t st, bool older = true) {
   if (int rc = ensure_encode()) return rc;
   long long blocks = (a->M + 7) / 8;
   if (blocks > 148 * 32) blocks = 148 * 32;
-  gather_rows_kernel<TI, Row::KPERM && sizeof(TI) == 4><<<(unsigned)blocks, 256, 0, st>>>((const TI *)a->input, a->sorted_pairs, (uint16_t *)ws, a->M, a->K,
-                                                          a->topk, a->row_per_pair, a->size_m);
+  launch_early(gather_rows_kernel<TI, Row::KPERM && sizeof(TI) == 4>, dim3((unsigned)blocks), dim3(256), st, (const TI *)a->input, a->sorted_pairs,
+               (uint16_t *)ws, (long long)a->M, a->K, a->topk, a->row_per_pair, (long long)a->size_m);
   if (int rc = launched("moe: gather rows")) return rc;
   CUtensorMap tm;
   const cuuint64_t dims[2] = {(cuuint64_t)a->K, (cuuint64_t)a->M};
@@ -1095,6 +1104,7 @@ int moe_launch(const lb200_moe_args *a, const typename Row::Ctx &ctx, void *ws, 
     c.mean_tokens = (double)a->M / a->E, c.min_run_k = tmem_min_run(), c.parts = sk, c.parts_bytes = ws_bytes - x_bytes;
     if (int took = gemm_tmem(c, st)) return took == 1 ? 0 : took;
   }
+  if (!older) return NOT_COVERED;
   return launch<Row, BF16, OutT>(tm, ctx, grp, (OutT *)a->out, (int)a->M, a->N, a->K, st, sk, sk ? ws_bytes - x_bytes : 0);
 }
 
@@ -1104,7 +1114,10 @@ int moe_launch(const lb200_moe_args *a, const typename Row::Ctx &ctx, void *ws, 
 // (a->dtype = BF16 only), 1 GGUF (a->dtype = Q4_K / Q6_K, x f32), 2 block-scaled FP8 (a->dtype = F32 / BF16
 // activations).  Returns 1 when taken, 0 when not covered, other values are errors.
 int moe_umma(const lb200_moe_args *a, int kind, const float *w_scale, int bR, int bC, int device, cudaStream_t st) {
-  if (a->M < 256 || a->M > 0x7fffffffLL || ((uintptr_t)a->input & 15) || ((uintptr_t)a->weights & 15) || a->K % 64) return 0;
+  // Fewer than 256 pairs (a decode step): where the fallback multiplies the same 16-bit values as the tensor cores do (bf16
+  // activations); others keep their f32 products.
+  const bool few = a->M < 256;
+  if ((few && !(use_tmem() && kind != 1 && a->dtype == LB200_BF16 && a->K % 128 == 0 && a->E <= 1024)) || a->M > 0x7fffffffLL || ((uintptr_t)a->input & 15) || ((uintptr_t)a->weights & 15) || a->K % 64) return 0;
   void *ws;
   size_t wsb;
   {
@@ -1115,13 +1128,13 @@ int moe_umma(const lb200_moe_args *a, int kind, const float *w_scale, int bR, in
   int rc = 0;
   if (kind == 0) {
     if (a->dtype != LB200_BF16) return 0;
-    rc = moe_launch<DenseRow, true, __nv_bfloat16, __nv_bfloat16>(a, DenseCtx{(const uint16_t *)a->weights}, ws, wsb, st);
+    rc = moe_launch<DenseRow, true, __nv_bfloat16, __nv_bfloat16>(a, DenseCtx{(const uint16_t *)a->weights}, ws, wsb, st, !few);
   } else if (kind == 1) {
     if (a->K % 256) return 0;
     if (a->dtype == LB200_Q4_K)
       rc = moe_launch<Q4KRow, false, float, float>(a, GgufCtx{(const uint8_t *)a->weights}, ws, wsb, st);
-    else if (a->dtype == LB200_Q6_K && ((size_t)(a->K >> 8) * 210) % 4 == 0)
-      rc = moe_launch<Q6KRow, false, float, float>(a, GgufCtx{(const uint8_t *)a->weights}, ws, wsb, st);
+    else if (a->dtype == LB200_Q6_K)  // (the older kernel wants rows that start 4-byte aligned)
+      rc = moe_launch<Q6KRow, false, float, float>(a, GgufCtx{(const uint8_t *)a->weights}, ws, wsb, st, (a->K >> 8) % 2 == 0);
     else if (a->dtype == LB200_Q8_0 && !((uintptr_t)a->weights & 15))
       rc = moe_launch<Q80Row, false, float, float>(a, GgufCtx{(const uint8_t *)a->weights}, ws, wsb, st);
     else
@@ -1130,12 +1143,13 @@ int moe_umma(const lb200_moe_args *a, int kind, const float *w_scale, int bR, in
     if (a->K % 128 || bC % 64 || bR <= 0 || a->N % bR || a->K % bC) return 0;
     const Fp8Ctx ctx{(const uint8_t *)a->weights, w_scale, bR, bC};
     if (a->dtype == LB200_BF16)
-      rc = moe_launch<Fp8Row, true, __nv_bfloat16, __nv_bfloat16>(a, ctx, ws, wsb, st);
+      rc = moe_launch<Fp8Row, true, __nv_bfloat16, __nv_bfloat16>(a, ctx, ws, wsb, st, !few);
     else if (a->dtype == LB200_F32)
       rc = moe_launch<Fp8Row, false, float, float>(a, ctx, ws, wsb, st);
     else
       return 0;
   }
+  if (rc == NOT_COVERED) return 0;
   return rc ? rc : 1;
 }
 

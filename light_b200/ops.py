@@ -595,8 +595,8 @@ def _moe_dispatch(op: str, key_dtype: int, quant: bool, inp: torch.Tensor, weigh
         raise ValueError(f"{op}: topkWeights must be F32 with {M} elements")
     dev = _dev(inp, op)
     inc = inp.contiguous()
-    if M >= 256:  # tensor-core grouped path: the token rows gathered in expert order, the persistent kernel's partial tiles
-        ensure_workspace(dev, int(_lib.lib().light_b200_matmul_q_workspace_bytes(M, K)))
+    if M:  # tensor-core grouped path: the token rows gathered in expert order, and behind them the partial tiles
+        ensure_workspace(dev, int(_lib.lib().light_b200_matmul_q_workspace_bytes(max(M, 65), K)))
     counts = torch.zeros(E, dtype=torch.int32, device=inp.device)
     offsets = torch.zeros(E + 1, dtype=torch.int32, device=inp.device)
     out = torch.zeros((M, N), dtype=out_dtype, device=inp.device)

@@ -1,0 +1,70 @@
+"""The tensor-memory matmul (weights expanded into TMEM, stream-K over CTAs or CTA pairs) where it can go wrong: one token more
+than a tile, ragged row counts (with and without whole 16-byte output rows), the shortest K, runs that start and end inside
+tiles, and grouped launches with empty experts, single tokens and ids outside the experts.
+
+Bounds: operands are rounded once each to f16 (2^-12 relative on average over a product: 1e-3 with room, the bound of the other
+tensor-core paths) or are the bf16 values themselves, when the bf16 output's rounding (2^-9 at most) is what remains."""
+import pytest
+import torch
+
+from helpers import rel_l2
+from light_b200 import ops, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _weight(kind, N, K, dev):
+    if kind in ("q4_k", "q6_k", "q8_0"):
+        dt = {"q4_k": ops.Q4_K, "q6_k": ops.Q6_K, "q8_0": ops.Q8_0}[kind]
+        w = ops.QTensor(synth.gaussian_weight(N + K, dt, N, K, device=dev).reshape(-1), dt, (N, K))
+        return (lambda x: ops.MatMulQ(x, w)), ops.Dequantize(w).double(), torch.float32
+    if kind == "int4":
+        g = torch.Generator(device=dev).manual_seed(N + K)
+        w = ops.Int4(torch.randint(-2**31, 2**31, (N, K // 8), generator=g, device=dev, dtype=torch.int32), torch.rand(N, K // 64, generator=g, device=dev) * 0.02,
+                     torch.randint(0, 31, (N, K // 64), generator=g, device=dev).float() / 2, 64)   # half of the zero points are no whole numbers
+        return (lambda x: ops.MatMulInt4(x, w)), ops.DequantizeInt4(w, torch.bfloat16).double(), torch.bfloat16
+    codes, scale = synth.random_fp8_block(N + K, N, K, 4, 64, device=dev)
+    return (lambda x: ops.MatMulF8Block(x, codes, scale, 4, 64)), ops.DequantizeF8Block(codes, scale, 4, 64, torch.bfloat16).double(), torch.bfloat16
+
+
+@pytest.mark.parametrize("kind", ["q4_k", "q6_k", "q8_0", "int4", "fp8"])
+@pytest.mark.parametrize("M,N,K", [(65, 132, 256), (129, 128, 1280), (200, 300, 512), (257, 4100, 2304), (1100, 1024, 768), (513, 8192, 2048)])
+def test_plain(cuda, kind, M, N, K):
+    if kind == "fp8" and N % 4:
+        pytest.skip("blocks of four rows")
+    f, w, dt = _weight(kind, N, K, cuda)
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(cuda, dt)
+    y = f(x)
+    assert torch.equal(y, f(x)), "partial tiles must be added in a fixed order"
+    assert ops.prefill_status(0) == 0
+    want = x.double() @ w.t()
+    assert rel_l2(y.cpu().double().numpy(), want.cpu().numpy()) <= (1e-3 if dt == torch.float32 else 3e-3)
+
+
+@pytest.mark.parametrize("M,E,topk,N,K", [(1, 8, 2, 256, 256), (5, 300, 3, 132, 128), (40, 4, 1, 128, 1024), (700, 6, 2, 520, 384)])
+def test_grouped_fp8(cuda, M, E, topk, N, K):
+    codes, scale = synth.random_fp8_block(7, E * N, K, 4, 64, device=cuda)
+    w = ops.DequantizeF8Block(codes, scale, 4, 64, torch.bfloat16).double().reshape(E, N, K)
+    g = torch.Generator().manual_seed(E)
+    x = torch.randn(M, K, generator=g).to(cuda, torch.bfloat16)
+    ids = torch.randint(0, E, (M, topk), generator=g).to(cuda)
+    ids[ids == 1] = 0                                    # expert 1 stays empty
+    wt = torch.rand(M * topk, generator=g).to(cuda)
+    r = ops.MoERouteFromIDs(ids, wt, M, topk)
+    y = ops.MoEGemmF8Block(x, codes.reshape(E, N, K), scale.reshape(E, N // 4, K // 64), 4, 64, r, wt, topk)
+    want = torch.einsum("mk,mnk->mn", x.double().repeat_interleave(topk, 0), w[ids.reshape(-1)]) * wt.double()[:, None]
+    assert ops.prefill_status(0) == 0
+    assert rel_l2(y.cpu().double().numpy(), want.cpu().numpy()) <= 3e-3
+
+
+def test_grouped_q6_k_rows_at_odd_offsets(cuda):
+    E, N, K, M, topk = 5, 260, 768, 333, 2                # 630-byte rows: not a multiple of four
+    q = ops.QTensor(synth.gaussian_weight(3, ops.Q6_K, E * N, K, device=cuda).reshape(-1), ops.Q6_K, (E, N, K))
+    w = ops.Dequantize(q).double().reshape(E, N, K)
+    g = torch.Generator().manual_seed(5)
+    x = torch.randn(M, K, generator=g).to(cuda)
+    ids = torch.randint(0, E, (M, topk), generator=g).to(cuda)
+    r = ops.MoERouteFromIDs(ids, torch.ones(M * topk, device=cuda), M, topk)
+    y = ops.MoEGemmQ(x, q, r, None, topk)
+    want = torch.einsum("mk,mnk->mn", x.double().repeat_interleave(topk, 0), w[ids.reshape(-1)])
+    assert rel_l2(y.cpu().double().numpy(), want.cpu().numpy()) <= 1e-3
