@@ -81,6 +81,41 @@ __device__ __forceinline__ void load_row(const __nv_bfloat16 *p, float (&f)[PER]
   }
 }
 
+// The CTAs of a cluster: rank r writes elements r (g D) / KS .. of the group's output from all ranks' (max, sum, sum p v).  BASE2:
+// the maxima are in units of log2 e.
+template <typename T, bool BASE2>
+__device__ __forceinline__ void cluster_combine(const AttnArgs &a, const float *cpart, int g, int D, int ROW, int KS, int rank, int b, int kh, int threads) {
+  const int tot = g * D, e0 = tot * rank / KS, e1 = tot * (rank + 1) / KS;
+  const uint32_t cbase = (uint32_t)__cvta_generic_to_shared(cpart);
+  for (int idx = e0 + threadIdx.x; idx < e1; idx += threads) {
+    const int h = idx / D, d = idx - h * D;
+    const uint32_t ra = cbase + (uint32_t)(h * ROW) * 4u;
+    float M = -INFINITY, L = 0.f, A = 0.f;
+    if (KS > 1) {
+      float mr[8], lr[8], ar[8];  // all remote loads at once
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        const uint32_t peer = umma::map_to_rank(ra, (uint32_t)(r < KS ? r : 0));
+        mr[r] = umma::ld_cluster_f32(peer), lr[r] = umma::ld_cluster_f32(peer + 4u), ar[r] = umma::ld_cluster_f32(peer + 8u + (uint32_t)d * 4u);
+      }
+#pragma unroll
+      for (int r = 0; r < 8; r++)
+        if (r < KS) M = fmaxf(M, mr[r]);
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        if (r < KS && mr[r] > -INFINITY) {  // a rank without keys holds (-inf, 0, 0)
+          const float e = BASE2 ? exp2f(mr[r] - M) : __expf(mr[r] - M);
+          L = fmaf(e, lr[r], L), A = fmaf(e, ar[r], A);
+        }
+      }
+    } else {
+      L = cpart[h * ROW + 1], A = cpart[h * ROW + 2 + d];
+    }
+    st_act(static_cast<T *>(a.out), ((long long)b * a.NH + (long long)kh * g + h) * D + d, A / L);
+  }
+  if (KS > 1) umma::cluster_sync();  // nobody leaves while a peer still reads its partials
+}
+
 template <int PER, int GH_>
 struct AttnCfg {
   static constexpr int D = PER * 32;
@@ -103,6 +138,18 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attn_kernel(AttnArgs a) 
   const int KS = gridDim.y, rank = blockIdx.y, bkh = blockIdx.x;
   const int g = a.NH / a.KH, b = bkh / a.KH, kh = bkh - b * a.KH;
   float *wpart = sm, *cpart = sm + Cfg::WPART;
+  __shared__ float trig[D];  // cos, sin of the rotation's D / 2 angles
+  {
+    // The cached rows of this CTA on their way to L2 while the launch before still runs.  Only a hint: the position may be
+    // one short here, and every row is read after the wait.
+    const long long p = a.pos[0];
+    const int n = (int)(p < 0 ? 0 : p < a.Cap ? p + 1 : a.Cap), s0 = a.window > 0 ? max(0, n - a.window) : 0, ch = (n - s0 + KS - 1) / KS;
+    const int f = s0 + rank * ch, e = min(n, f + ch);
+    const char *kp = static_cast<const char *>(a.kbuf) + ((size_t)bkh * a.Cap + f) * D * sizeof(T), *vp = static_cast<const char *>(a.vbuf) + ((size_t)bkh * a.Cap + f) * D * sizeof(T);
+    const int lines = min((e - f) * (int)(D * sizeof(T)) / 128, 4 * DA_THREADS);
+    for (int i = threadIdx.x; i < lines; i += DA_THREADS)
+      asm volatile("prefetch.global.L2 [%0];\n\tprefetch.global.L2 [%1];\n" ::"l"(kp + (size_t)i * 128), "l"(vp + (size_t)i * 128));
+  }
   pdl_wait();  // q, k_new, v_new are the previous launch's output; pos is older
   long long pos = a.pos[0];
   // A position outside the cache: reported, nothing is appended (as kv_append_kernel), and the launch attends
@@ -124,11 +171,16 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attn_kernel(AttnArgs a) 
   // which is lane ^ 16 here); cached keys were rotated when they were appended
   const bool roped = a.rope_k != 0.0;
   float rc[PER], rs[PER];
-  if (roped) {
+  if (roped) {  // each angle once per CTA (a chain of f64 operations): four in a row per lane took 2 us
+    for (int i = threadIdx.x; i < D / 2; i += DA_THREADS) {
+      const float2 cs = rope_cos_sin(pos, i, a.rope_k);
+      trig[i] = cs.x, trig[D / 2 + i] = cs.y;
+    }
+    __syncthreads();
 #pragma unroll
     for (int p = 0; p < PER; p++) {
-      const float2 cs = rope_cos_sin(pos, (lane * PER + p) & (D / 2 - 1), a.rope_k);
-      rc[p] = cs.x, rs[p] = cs.y;
+      const int i = (lane * PER + p) & (D / 2 - 1);
+      rc[p] = trig[i], rs[p] = trig[D / 2 + i];
     }
   }
   auto rotate = [&](float (&v)[PER]) {
@@ -143,7 +195,7 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attn_kernel(AttnArgs a) 
     const size_t dst = ((size_t)bkh * a.Cap + (size_t)pos) * D + threadIdx.x;
     if (roped) {
       const int i = threadIdx.x & (D / 2 - 1);
-      const float2 cs = rope_cos_sin(pos, i, a.rope_k);
+      const float2 cs = make_float2(trig[i], trig[D / 2 + i]);
       const float x0 = ld_act(ks, i), x1 = ld_act(ks, i + D / 2);
       st_act(static_cast<T *>(a.kbuf), (long long)dst, (int)threadIdx.x < D / 2 ? x0 * cs.x - x1 * cs.y : x0 * cs.y + x1 * cs.x);
     } else {
@@ -303,37 +355,265 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attn_kernel(AttnArgs a) 
     }
     __syncthreads();
   }
-  // ---- the CTAs of this cluster: rank r writes elements r (g D) / KS .. of the group's output
   if (KS > 1) umma::cluster_sync();
-  {
-    const int tot = g * D, e0 = tot * rank / KS, e1 = tot * (rank + 1) / KS;
-    const uint32_t cbase = (uint32_t)__cvta_generic_to_shared(cpart);
-    for (int idx = e0 + threadIdx.x; idx < e1; idx += DA_THREADS) {
-      const int h = idx / D, d = idx - h * D;
-      const uint32_t ra = cbase + (uint32_t)(h * ROW) * 4u;
-      float M = -INFINITY, L = 0.f, A = 0.f;
-      if (KS > 1) {
-        float mr[8];
+  cluster_combine<T, false>(a, cpart, g, D, ROW, KS, rank, b, kh, DA_THREADS);
+}
+
+// ------------------------------------------------------------------------------------ bf16 caches on the tensor cores
+// The kernel above spends about 60 instructions of a warp per key (unpacking, 2 D FMAs per head and key over 32 lanes, the
+// reduce-scatter), which bounds a bf16 cache at 1.2 TB/s (8 sequences, 8192 keys, 8 KV heads of 128: 231 us).  Here a warp takes
+// 16 keys at a time through mma.sync (bf16 x bf16 -> f32), straight from global memory to fragments, about 13 instructions
+// per key, and what remains is the memory.
+//   * S = Q K^T: the query heads are the rows.  Rotated q is f32 and is split into bf16 hi + lo: up to eight heads, rows 0-7
+//     hold hi and rows 8-15 lo of the same heads and one MMA does both; up to sixteen, two MMAs.  Relative error 2^-17.
+//   * O += P V the same way: p split into hi + lo; the S fragment of a lane IS its P fragment (no exchange).
+//   * The order of the dims inside a contraction is free as long as both sides agree, so a lane's K fragments are 32
+//     consecutive bytes of its key (one 256-bit load feeds two MMAs), and the assignment of dims to V's columns gives a lane
+//     32 consecutive bytes of each of its four keys; pairs of keys are interleaved by PRMT.
+//   * Loads for the next 16 keys are issued as soon as the registers are free: K behind the QK MMAs, V behind the PV MMAs.
+// Four warps to a CTA, two or three CTAs per SM, a cluster of up to eight CTAs along the keys.
+constexpr int MA_WARPS = 4, MA_THREADS = MA_WARPS * 32;
+constexpr int mma_ctas(int D) { return D == 64 ? 3 : 2; }  // CTAs per SM: what the registers allow
+
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<uint32_t *>(&h);
+}
+__device__ __forceinline__ uint32_t pack_rest(float a, float b, uint32_t hi) {  // what rounding to bf16 left, as bf16
+  return pack_bf16(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xFFFF0000u));
+}
+// W words (8 or 4) of a cached row: read once, so no room in L1
+template <int W>
+__device__ __forceinline__ void ld_stream(const void *p, uint32_t (&v)[W]) {
+  if constexpr (W == 8)
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "l"(p));
+  else
+    asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(p));
+}
+
+template <int D, bool G16>
+__global__ void __launch_bounds__(MA_THREADS, mma_ctas(D)) decode_attn_mma_kernel(AttnArgs a) {
+  constexpr int KL = D / 64;        // 32-byte loads of a key row per lane; each feeds two 16-dim steps
+  constexpr int NT = D / 8;         // column tiles of O, and consecutive dims of a V row per lane
+  constexpr int VW = NT / 2;        // words of a V row per lane
+  constexpr int HMAX = G16 ? 16 : 8, ROW = D + 2;
+  extern __shared__ __align__(16) float sm[];
+  float *qs = sm;                                    // [HMAX][D] rotated q; later the warps' partial results [warp][HMAX][ROW]
+  float *cpart = sm + MA_WARPS * HMAX * ROW;         // [HMAX][ROW] of this CTA
+  float *trig = cpart + HMAX * ROW;                  // cos, sin of D / 2 angles
+  uint32_t *fresh = reinterpret_cast<uint32_t *>(trig + D);  // the new key and value, bf16
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
+  const int KS = gridDim.y, rank = blockIdx.y, bkh = blockIdx.x;
+  const int g = a.NH / a.KH, b = bkh / a.KH, kh = bkh - b * a.KH;
+  pdl_wait();
+  long long pos = a.pos[0];
+  const bool in_range = pos >= 0 && pos < a.Cap;
+  if (!in_range) {
+    if (threadIdx.x == 0) atomicOr(&g_attn_status, 1u);
+    pos = pos < 0 ? 0 : a.Cap - 1;
+  }
+  const int n = (int)pos + 1, start = a.window > 0 ? max(0, n - a.window) : 0;
+  const int chunk = ((n - start + KS - 1) / KS + 15) & ~15;
+  const int j0 = min(n, start + rank * chunk), j1 = min(n, j0 + chunk);
+  const bool append = a.k_new && in_range;
+  const __nv_bfloat16 *Kb = static_cast<const __nv_bfloat16 *>(a.kbuf) + (size_t)bkh * a.Cap * D;
+  const __nv_bfloat16 *Vb = static_cast<const __nv_bfloat16 *>(a.vbuf) + (size_t)bkh * a.Cap * D;
+
+  // ---- this warp's first keys are on their way while the query is prepared
+  uint32_t kf[2][KL][8], vf[4][VW];
+  auto fetch_k = [&](int j) {
 #pragma unroll
-        for (int r = 0; r < 8; r++) {
-          mr[r] = r < KS ? umma::ld_cluster_f32(umma::map_to_rank(ra, (uint32_t)r)) : -INFINITY;
-          M = fmaxf(M, mr[r]);
-        }
+    for (int t = 0; t < 2; t++) {
+      const __nv_bfloat16 *p = Kb + (size_t)min(j + 8 * t + r, n - 1) * D + c * 16;
 #pragma unroll
-        for (int r = 0; r < 8; r++) {
-          if (r < KS && mr[r] > -INFINITY) {  // a rank without keys holds (-inf, 0, 0)
-            const float e = __expf(mr[r] - M);
-            L = fmaf(e, umma::ld_cluster_f32(umma::map_to_rank(ra + 4u, (uint32_t)r)), L);
-            A = fmaf(e, umma::ld_cluster_f32(umma::map_to_rank(ra + 8u + (uint32_t)d * 4u, (uint32_t)r)), A);
-          }
-        }
-      } else {
-        L = cpart[h * ROW + 1], A = cpart[h * ROW + 2 + d];
-      }
-      st_act(static_cast<T *>(a.out), ((long long)b * a.NH + (long long)kh * g + h) * D + d, A / L);
+      for (int i = 0; i < KL; i++) ld_stream<8>(p + 64 * i, kf[t][i]);
+    }
+  };
+  auto fetch_v = [&](int j) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) ld_stream<VW>(Vb + (size_t)min(j + 2 * c + (k & 1) + 8 * (k >> 1), n - 1) * D + r * NT, vf[k]);
+  };
+  int j = j0 + warp * 16;
+  if (j < j1) fetch_k(j), fetch_v(j);
+
+  const bool roped = a.rope_k != 0.0;
+  if (roped) {
+    for (int i = threadIdx.x; i < D / 2; i += MA_THREADS) {
+      const float2 cs = rope_cos_sin(pos, i, a.rope_k);
+      trig[i] = cs.x, trig[D / 2 + i] = cs.y;
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < g * (D / 2); i += MA_THREADS) {
+    const int h = i / (D / 2), d = i - h * (D / 2);
+    const __nv_bfloat16 *q = static_cast<const __nv_bfloat16 *>(a.q) + ((size_t)b * a.NH + (size_t)kh * g + h) * D;
+    const float x0 = __bfloat162float(q[d]), x1 = __bfloat162float(q[d + D / 2]);
+    const float cs = roped ? trig[d] : 1.f, sn = roped ? trig[D / 2 + d] : 0.f;
+    qs[h * D + d] = x0 * cs - x1 * sn, qs[h * D + d + D / 2] = x0 * sn + x1 * cs;
+  }
+  if (append && threadIdx.x < D / 2) {  // the new row: the cache gets it from rank 0, this CTA reads it from shared memory
+    const __nv_bfloat16 *kn = static_cast<const __nv_bfloat16 *>(a.k_new) + (size_t)bkh * D, *vn = static_cast<const __nv_bfloat16 *>(a.v_new) + (size_t)bkh * D;
+    const int d = threadIdx.x;
+    const float x0 = __bfloat162float(kn[d]), x1 = __bfloat162float(kn[d + D / 2]), cs = roped ? trig[d] : 1.f, sn = roped ? trig[D / 2 + d] : 0.f;
+    __nv_bfloat16 *fk = reinterpret_cast<__nv_bfloat16 *>(fresh), *fv = fk + D;
+    fk[d] = roped ? __float2bfloat16_rn(x0 * cs - x1 * sn) : kn[d], fk[d + D / 2] = roped ? __float2bfloat16_rn(x0 * sn + x1 * cs) : kn[d + D / 2];
+    fv[d] = vn[d], fv[d + D / 2] = vn[d + D / 2];
+    if (rank == 0) {
+      const size_t dst = ((size_t)bkh * a.Cap + (size_t)pos) * D + d;
+      static_cast<__nv_bfloat16 *>(a.kbuf)[dst] = fk[d], static_cast<__nv_bfloat16 *>(a.kbuf)[dst + D / 2] = fk[d + D / 2];
+      static_cast<__nv_bfloat16 *>(a.vbuf)[dst] = fv[d], static_cast<__nv_bfloat16 *>(a.vbuf)[dst + D / 2] = fv[d + D / 2];
     }
   }
-  if (KS > 1) umma::cluster_sync();  // nobody leaves while a peer still reads its partials
+  __syncthreads();
+
+  // ---- Q fragments: step s covers, for column c, dims 64 (s / 4) + 16 c + 4 (s % 4) .. + 3 of every key (its two registers)
+  uint32_t qh[D / 16][2], ql[D / 16][2], qh8[G16 ? D / 16 : 1][2], ql8[G16 ? D / 16 : 1][2];
+#pragma unroll
+  for (int s = 0; s < D / 16; s++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int d = 64 * (s >> 2) + 16 * c + 4 * (s & 3) + 2 * e;
+      const float x0 = r < g ? qs[r * D + d] : 0.f, x1 = r < g ? qs[r * D + d + 1] : 0.f;
+      qh[s][e] = pack_bf16(x0, x1), ql[s][e] = pack_rest(x0, x1, qh[s][e]);
+      if constexpr (G16) {
+        const float y0 = r + 8 < g ? qs[(r + 8) * D + d] : 0.f, y1 = r + 8 < g ? qs[(r + 8) * D + d + 1] : 0.f;
+        qh8[s][e] = pack_bf16(y0, y1), ql8[s][e] = pack_rest(y0, y1, qh8[s][e]);
+      }
+    }
+  __syncthreads();  // qs is reused for the partial results
+
+  const float sc = a.scale * 1.4426950408889634f;  // scores in units of log2 e
+  float m[G16 ? 2 : 1], l[G16 ? 2 : 1], o[NT][4];
+#pragma unroll
+  for (int i = 0; i < (G16 ? 2 : 1); i++) m[i] = -INFINITY, l[i] = 0.f;
+#pragma unroll
+  for (int t = 0; t < NT; t++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) o[t][e] = 0.f;
+
+  for (; j < j1; j += MA_WARPS * 16) {
+    if (append && j <= (int)pos && (int)pos < j + 16) {  // (pos is the last key: these loads cannot have its new row)
+      const int x = (int)pos - j;
+#pragma unroll
+      for (int t = 0; t < 2; t++)
+        if (x == 8 * t + r) {
+#pragma unroll
+          for (int i = 0; i < KL; i++)
+#pragma unroll
+            for (int e = 0; e < 8; e++) kf[t][i][e] = fresh[32 * i + 8 * c + e];
+        }
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int y = 2 * c + (k & 1) + 8 * (k >> 1);
+        if (y >= x) {  // (rows past it were read from its place, which holds anything: their weight is 0, so they must be finite)
+#pragma unroll
+          for (int e = 0; e < VW; e++) vf[k][e] = y == x ? fresh[D / 2 + VW * r + e] : 0u;
+        }
+      }
+    }
+    float s[2][4] = {};
+#pragma unroll
+    for (int st = 0; st < D / 16; st++)
+#pragma unroll
+      for (int t = 0; t < 2; t++) {
+        const uint32_t b0 = kf[t][st >> 2][2 * (st & 3)], b1 = kf[t][st >> 2][2 * (st & 3) + 1];
+        if constexpr (G16) {
+          mma_bf16(s[t], qh[st][0], qh8[st][0], qh[st][1], qh8[st][1], b0, b1);
+          mma_bf16(s[t], ql[st][0], ql8[st][0], ql[st][1], ql8[st][1], b0, b1);
+        } else {
+          mma_bf16(s[t], qh[st][0], ql[st][0], qh[st][1], ql[st][1], b0, b1);
+        }
+      }
+    const int jn = j + MA_WARPS * 16;
+    if (jn < j1) fetch_k(jn);
+    uint32_t ph[2][2], pl[2][2];  // [tile][row half]: P as A fragments
+    float mx[G16 ? 2 : 1];
+#pragma unroll
+    for (int i = 0; i < (G16 ? 2 : 1); i++) {
+      float v[4];
+#pragma unroll
+      for (int t = 0; t < 2; t++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const float x = G16 ? s[t][2 * i + e] : s[t][e] + s[t][2 + e];
+          v[2 * t + e] = j + 8 * t + 2 * c + e < j1 ? x * sc : -INFINITY;
+        }
+      mx[i] = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3]));
+      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
+      mx[i] = fmaxf(m[i], fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2)));
+      float p[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) p[e] = exp2f(v[e] - mx[i]);  // (a block holds a key: mx is finite)
+      const float corr = exp2f(m[i] - mx[i]);
+      l[i] = l[i] * corr + ((p[0] + p[1]) + (p[2] + p[3]));
+#pragma unroll
+      for (int t = 0; t < 2; t++) ph[t][i] = pack_bf16(p[2 * t], p[2 * t + 1]), pl[t][i] = pack_rest(p[2 * t], p[2 * t + 1], ph[t][i]);
+    }
+    bool same = mx[0] == m[0];
+    if constexpr (G16) same = same && mx[1] == m[1];
+    if (!__all_sync(0xffffffffu, same)) {
+#pragma unroll
+      for (int t = 0; t < NT; t++) {
+        const float c0 = exp2f(m[0] - mx[0]), c1 = G16 ? exp2f(m[G16 ? 1 : 0] - mx[G16 ? 1 : 0]) : c0;
+        o[t][0] *= c0, o[t][1] *= c0, o[t][2] *= c1, o[t][3] *= c1;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < (G16 ? 2 : 1); i++) m[i] = mx[i];
+#pragma unroll
+    for (int t = 0; t < NT; t++) {  // column r of tile t is dim NT r + t
+      const uint32_t sel = t & 1 ? 0x7632u : 0x5410u;
+      const uint32_t b0 = __byte_perm(vf[0][t >> 1], vf[1][t >> 1], sel), b1 = __byte_perm(vf[2][t >> 1], vf[3][t >> 1], sel);
+      if constexpr (G16) {
+        mma_bf16(o[t], ph[0][0], ph[0][1], ph[1][0], ph[1][1], b0, b1);
+        mma_bf16(o[t], pl[0][0], pl[0][1], pl[1][0], pl[1][1], b0, b1);
+      } else {
+        mma_bf16(o[t], ph[0][0], pl[0][0], ph[1][0], pl[1][0], b0, b1);
+      }
+    }
+    if (jn < j1) fetch_v(jn);
+  }
+  // ---- the warps of this CTA: O fragment element (row r, column 2 c + e of tile t) is dim NT (2 c + e) + t
+  float *mine = sm + warp * HMAX * ROW;
+#pragma unroll
+  for (int i = 0; i < (G16 ? 2 : 1); i++) {
+    l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1), l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
+    float *row = mine + (r + 8 * i) * ROW;
+    if (c == 0) row[0] = m[i], row[1] = l[i];
+#pragma unroll
+    for (int t = 0; t < NT; t++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) row[2 + NT * (2 * c + e) + t] = G16 ? o[t][2 * i + e] : o[t][e] + o[t][2 + e];
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < g * D; idx += MA_THREADS) {
+    const int h = idx / D, d = idx - h * D;
+    float M = -INFINITY, L = 0.f, A = 0.f;
+#pragma unroll
+    for (int w = 0; w < MA_WARPS; w++) M = fmaxf(M, sm[(w * HMAX + h) * ROW]);
+    if (M > -INFINITY) {
+#pragma unroll
+      for (int w = 0; w < MA_WARPS; w++) {
+        const float *row = sm + (w * HMAX + h) * ROW;
+        const float e = exp2f(row[0] - M);
+        L = fmaf(e, row[1], L), A = fmaf(e, row[2 + d], A);
+      }
+    }
+    cpart[h * ROW + 2 + d] = A;
+    if (d == 0) cpart[h * ROW] = M, cpart[h * ROW + 1] = L;
+  }
+  if (KS > 1) umma::cluster_sync();
+  else __syncthreads();
+  cluster_combine<__nv_bfloat16, true>(a, cpart, g, D, ROW, KS, rank, b, kh, MA_THREADS);
 }
 
 template <typename T>
@@ -406,6 +686,23 @@ int launch_attn_g(const AttnArgs &a, int ks, cudaStream_t st) {
   return launch_attn<T, PER, GMAX>(a, ks, st);
 }
 
+template <int D, bool G16>
+int launch_mma(const AttnArgs &a, cudaStream_t st) {
+  auto kern = decode_attn_mma_kernel<D, G16>;
+  constexpr int HMAX = G16 ? 16 : 8;
+  constexpr size_t smem = (size_t)((MA_WARPS + 1) * HMAX * (D + 2) + D + D) * sizeof(float);
+  static DeviceOnce smem_set;
+  cudaError_t e = smem_set.ensure([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }, smem);
+  if (e != cudaSuccess) return fail((int)e, "light_b200: decode_attn: %s", cudaGetErrorString(e));
+  // as many CTAs along the keys as fit on the SMs at once, with 64 keys of the capacity (a block of each warp) or more for each
+  const int slots = mma_ctas(D) * sm_count();
+  int ks = 1;
+  while (ks < 8 && a.B * a.KH * (ks + 1) <= slots && a.Cap >= 64 * (ks + 1)) ks++;
+  e = launch_chain(kern, dim3((unsigned)(a.B * a.KH), (unsigned)ks), dim3(MA_THREADS), smem, (unsigned)ks, st, a);
+  if (e != cudaSuccess) return fail((int)e, "light_b200: decode_attn: %s", cudaGetErrorString(e));
+  return launched("decode_attn");
+}
+
 template <typename T>
 int launch_attn_d(const AttnArgs &a, int D, int ks, cudaStream_t st) {
   switch (D / 32) {
@@ -436,6 +733,11 @@ int decode_attn(const lb200_decode_attn_args *p, cudaStream_t st) {
   if (p->rope_base < 0.f) return fail(LB200_E_SHAPE, "light_b200: decode_attn: rope_base %g", (double)p->rope_base);
   const double rope_k = p->rope_base > 0.f ? -2.0 * log2((double)p->rope_base) / (double)p->D : 0.0;
   AttnArgs a{p->q, p->k_new, p->v_new, p->kbuf, p->vbuf, p->out, (const long long *)p->pos, p->B, p->NH, p->KH, p->Cap, p->window, p->scale, rope_k};
+  // bf16 caches with 64- or 128-wide heads: the tensor-core kernel (its 256-bit loads want rows on 32 bytes)
+  if (p->dtype == LB200_BF16 && (p->D == 64 || p->D == 128) && !(((uintptr_t)p->kbuf | (uintptr_t)p->vbuf) & 31)) {
+    if (p->D == 64) return g <= 8 ? launch_mma<64, false>(a, st) : launch_mma<64, true>(a, st);
+    return g <= 8 ? launch_mma<128, false>(a, st) : launch_mma<128, true>(a, st);
+  }
   // enough CTAs to fill the GPU, at least 32 keys of the capacity each, a portable cluster
   int ks = 1;
   while (ks < 8 && p->B * p->KH * ks < 148 && p->Cap >= 64 * ks) ks *= 2;

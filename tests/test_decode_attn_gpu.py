@@ -131,3 +131,30 @@ def test_limits_are_reported_not_asserted(cuda):
         ops.DecodeAttention(q, kbuf, kbuf.clone(), pos, 1.0)
     with pytest.raises(ValueError):
         ops.DecodeAttention(q, kbuf, kbuf.clone(), pos.to(torch.int32), 1.0)
+
+
+# ---- the tensor-core kernel of bf16 caches: block edges (16 keys a warp, 64 a CTA), one key, head groups on both sides of
+# eight, a window that starts inside a block, and a row at pos that held NaN before the append.  Against f64; the bf16 output's
+# rounding (2^-9 at most) is what remains.
+@pytest.mark.parametrize("B,NH,KH,D,n,win", [(1, 1, 1, 64, 1, 0), (2, 8, 1, 128, 16, 0), (1, 9, 1, 64, 17, 0), (3, 16, 1, 128, 65, 0), (2, 4, 4, 64, 128, 50),
+                                             (1, 24, 8, 128, 1000, 300)])
+def test_tensor_core_kernel(cuda, B, NH, KH, D, n, win):
+    g = torch.Generator().manual_seed(n)
+    kb, vb, q, k, v = (torch.randn(s, generator=g).to(cuda, torch.bfloat16)
+                       for s in ((B, KH, n, D), (B, KH, n, D), (B, NH, 1, D), (B, KH, 1, D), (B, KH, 1, D)))
+    kb[:, :, n - 1], vb[:, :, n - 1] = float("nan"), float("nan")
+    pos = torch.full((1,), n - 1, dtype=torch.int64, device=cuda)
+    got = ops.DecodeAttention(q, kb, vb, pos, D ** -0.5, win, k, v, rope_base=10000.0)
+    ang = (n - 1) * 10000.0 ** (-torch.arange(D // 2, dtype=torch.float64, device=cuda) * 2 / D)
+
+    def rot(x):
+        a, b = x.double().chunk(2, -1)
+        return torch.cat([a * ang.cos() - b * ang.sin(), a * ang.sin() + b * ang.cos()], -1)
+
+    assert torch.equal(kb[:, :, n - 1], rot(k)[:, :, 0].float().to(torch.bfloat16)) or (kb[:, :, n - 1].double() - rot(k)[:, :, 0]).abs().max() < 2 ** -6
+    assert torch.equal(vb[:, :, n - 1], v[:, :, 0])
+    s = max(0, n - win) if win else 0
+    K, V = kb.double()[:, :, s:], vb.double()[:, :, s:]
+    want = torch.softmax(rot(q).reshape(B, KH, NH // KH, D) @ K.transpose(-1, -2) * D ** -0.5, -1) @ V
+    err = (got.double().reshape(want.shape) - want).norm() / want.norm()
+    assert float(err) <= 3e-3 and ops.decode_attn_status(0) == 0
