@@ -299,6 +299,11 @@ LB200_API int light_b200_moe_gemm_static_scratch(const lb200_moe_args *args, int
  * x f32, GGUF block-quantized experts, out f32. */
 LB200_API int light_b200_moe_gemm_q(const lb200_moe_args *args, int device, void *stream);
 
+/* Zeroes the rows (of row_bytes each) of out (rows, ..) that no sorted pair with an expert id in [0, E) writes; the grouped
+ * matmuls leave those untouched.  bits: ceil(rows / 32) words of scratch.  Replaces clearing all of `out` beforehand. */
+LB200_API int light_b200_moe_clear_unrouted(const int64_t *sorted_pairs, const int64_t *expert_ids, uint32_t *bits, void *out, int64_t M,
+                                            int64_t rows, int64_t row_bytes, int E, int device, void *stream);
+
 /* ---- decode-step attention against a fixed-capacity KV cache (the step beside the quantized matmuls)
  *
  * Registry keys {kv_append, CUDA, F32|BF16}, {decode_attn, CUDA, F32|BF16}, {inc_i64, CUDA, I64}

@@ -189,6 +189,10 @@ int light_b200_matmul_q(int t, const float *x, const void *w, float *out, int M,
   took = gguf_gemv_fast(t, x, w, out, M, N, K, st);
   if (took < 0) return took;
   if (took) return 0;
+  if (t == LB200_Q8_0 && M <= 64) {
+    took = gguf_prefill(t, x, w, out, M, N, K, device, st);
+    if (took != 0) return took == 1 ? 0 : took;
+  }
   if (M >= 2 && M <= 64) {  // tokens as MMA columns over activations staged once (needs the workspace)
     size_t wsb = 0;
     void *ws = workspace_ptr(device, &wsb);
@@ -443,6 +447,20 @@ int light_b200_moe_gemm(const lb200_moe_args *a, int device, void *stream) {
   if (int rc = moe_check(a, "moe_gemm", false)) return rc;
   if (int rc = bind(device)) return rc;
   return moe_gemm(a, device, (cudaStream_t)stream);
+}
+
+int light_b200_moe_clear_unrouted(const int64_t *sorted_pairs, const int64_t *expert_ids, uint32_t *bits, void *out, int64_t M, int64_t rows,
+                                  int64_t row_bytes, int E, int device, void *stream) {
+  if (M < 0 || rows < 0 || row_bytes < 0 || row_bytes % 2 || E < 0 || M > 0x7fffffffLL || rows > 0x7fffffffLL)
+    return fail(LB200_E_SHAPE, "light_b200: moe_clear_unrouted: M=%lld rows=%lld of %lld bytes", (long long)M, (long long)rows, (long long)row_bytes);
+  if (M) {
+    REQUIRE_PTR(sorted_pairs, "moe_clear_unrouted");
+    REQUIRE_PTR(expert_ids, "moe_clear_unrouted");
+  }
+  REQUIRE_PTR(bits, "moe_clear_unrouted");
+  REQUIRE_PTR(out, "moe_clear_unrouted");
+  if (int rc = bind(device)) return rc;
+  return moe_clear_unrouted(sorted_pairs, expert_ids, bits, out, M, rows, row_bytes, E, (cudaStream_t)stream);
 }
 
 int light_b200_moe_gemm_static_scratch(const lb200_moe_args *a, int device, void *stream) {

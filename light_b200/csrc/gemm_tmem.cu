@@ -42,7 +42,8 @@ using namespace umma;
 
 constexpr int EXPANDERS = 16, TMA_WARP = 16, MMA_WARP = 17, EPI_WARP = 18, THREADS = 22 * 32;
 constexpr int KU = 128;                       // k of a unit: one TMEM stage, one stage of the token ring
-constexpr int NAS = 4;                        // stages of 128 k: 64 TMEM columns of expanded weights, and a token tile in shared memory
+constexpr int NAS = 4;                        // stages of expanded weights: 128 k, 64 TMEM columns each
+constexpr int NBS = 12;                       // most stages of the token ring, 128 k each
 constexpr int A_COL = 256;                    // columns 0-255: accumulators, 256-511: weight stages
 constexpr int MAX_E = 1024;                   // experts whose prefix sums fit the shared tables
 constexpr int MAX_GRID = 160;
@@ -62,7 +63,7 @@ struct Args {
   int E, M, N, K;
   int nt_max;               // most tokens of a tile
   int box;                  // token rows of one TMA box
-  int stage_bytes;          // of a token tile, per CTA
+  int stage_bytes, nbs;     // of the token ring, per CTA
   int wmin;                 // grouped: a unit's weight is max(tokens of its tile, wmin)
   float *parts;
 };
@@ -206,14 +207,33 @@ struct Work {
     }
     return lo;
   }
-  __device__ __forceinline__ Tile tile(int t) const {
+  // A walk over the list: the search once, then one tile after the other.
+  struct Walk {
+    int t, e, rt, tt, ntt, nt, first, cnt;
+  };
+  __device__ __forceinline__ Walk walk(int t) const {
+    Walk w;
+    w.t = t, w.e = expert_of(preT, t), w.cnt = count(w.e), w.first = first(w.e);
+    geo(w.cnt, w.ntt, w.nt);
+    const int r = t - preT[w.e];
+    w.rt = w.ntt ? r / w.ntt : 0, w.tt = r - w.rt * w.ntt;
+    return w;
+  }
+  __device__ __forceinline__ void next(Walk &w) const {
+    w.t++;
+    if (++w.tt < w.ntt) return;
+    w.tt = 0;
+    if (++w.rt < nrt) return;
+    w.rt = 0;
+    do w.e++;
+    while (w.e < a.E && count(w.e) == 0);
+    if (w.e >= a.E) return;  // (the list's end)
+    w.cnt = count(w.e), w.first = first(w.e);
+    geo(w.cnt, w.ntt, w.nt);
+  }
+  __device__ __forceinline__ Tile tile(const Walk &w) const {
     Tile T;
-    const int e = expert_of(preT, t);
-    int ntt;
-    const int cnt = count(e);
-    geo(cnt, ntt, T.nt);
-    const int r = t - preT[e], rt = r / ntt, tt = r - rt * ntt;
-    T.expert = e, T.n0 = rt * 128 * CG, T.m0 = first(e) + tt * T.nt, T.m_end = min(first(e) + cnt, T.m0 + T.nt);
+    T.expert = w.e, T.nt = w.nt, T.n0 = w.rt * 128 * CG, T.m0 = w.first + w.tt * w.nt, T.m_end = min(w.first + w.cnt, T.m0 + w.nt);
     return T;
   }
   // first unit (tile-major) of run j of G
@@ -245,10 +265,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   __shared__ uint32_t tmem_sh;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char *gen = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t sB = base, sRaw = base + NAS * (uint32_t)a.stage_bytes, sStrip = sRaw + (uint32_t)EXPANDERS * Row::SLOT, sBar = sStrip + STRIPS;
-  // full[s]: a stage's weights (four warps) and tokens (the TMA lane and its bytes) are there, and so are the other CTA's;
-  // empty[s]: its MMAs have completed
-  const uint32_t full = sBar, empty = full + 8 * NAS, d_full = empty + 8 * NAS, d_empty = d_full + 16, drained = d_empty + 16, w_full = drained + 8;
+  const uint32_t sB = base, sRaw = base + (uint32_t)a.nbs * a.stage_bytes, sStrip = sRaw + (uint32_t)EXPANDERS * Row::SLOT, sBar = sStrip + STRIPS;
+  // full[s]: a stage's weights are there (four warps; in the first CTA of a pair also: the other CTA's weights and tokens);
+  // empty[s]: its MMAs have completed.  t_full, t_empty: the token ring's, which runs further ahead: a token tile takes a TMA
+  // latency to refill, and with only four stages that, not the tensor core, set the pace of narrow tiles.
+  const uint32_t full = sBar, empty = full + 8 * NAS, d_full = empty + 8 * NAS, d_empty = d_full + 16, drained = d_empty + 16, w_full = drained + 8,
+                 t_full = w_full + 8 * EXPANDERS, t_empty = t_full + 8 * NBS;
   int *preW = reinterpret_cast<int *>(gen + (sBar - base) + BAR_BYTES), *preT = preW + a.E + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = CG == 2 ? (int)cluster_ctarank() : 0;
@@ -261,7 +283,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
     if constexpr (Row::BOXES > 0) prefetch_tmap(&maps.w[0]);
     if constexpr (Row::BOXES > 1) prefetch_tmap(&maps.w[1]);
     abort_flag = 0;
-    for (int i = 0; i < NAS; i++) mbar_init(full + 8 * i, CG == 2 && rank == 0 ? 6 : 5), mbar_init(empty + 8 * i, 1);
+    for (int i = 0; i < NAS; i++) mbar_init(full + 8 * i, CG == 2 && rank == 0 ? 5 : 4), mbar_init(empty + 8 * i, 1);
+    for (int i = 0; i < a.nbs; i++) mbar_init(t_full + 8 * i, 1), mbar_init(t_empty + 8 * i, 1);
     for (int i = 0; i < 2; i++) mbar_init(d_full + 8 * i, 1), mbar_init(d_empty + 8 * i, 4 * CG);
     mbar_init(drained, 1);
     for (int i = 0; i < EXPANDERS; i++) mbar_init(w_full + 8 * i, 1);
@@ -306,23 +329,22 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   if (warp == TMA_WARP) {
     if (lane == 0) {
       pdl_wait();  // the tokens may be the kernel before's; the weights are not
-      int issued = 0;
-      for (int pos = pos0; pos < pos1 && !*abort;) {
-        const int t = pos / nb, u0 = pos - t * nb, u1 = min(nb, u0 + (pos1 - pos));
-        const Tile T = wk.tile(t);
+      int bt = 0, par = 1;
+      bool wrapped = false;
+      auto W = wk.walk(pos0 / nb);
+      for (int pos = pos0; pos < pos1 && !*abort; wk.next(W)) {
+        const int u0 = pos - W.t * nb, u1 = min(nb, u0 + (pos1 - pos));
+        const Tile T = wk.tile(W);
         const int rows = T.nt / CG, boxes = (rows + a.box - 1) / a.box, y0 = T.m0 + rank * rows;
         const uint32_t bytes = (uint32_t)(boxes * a.box) * 256u;
-        for (int u = u0; u < u1; u++, issued++) {
-          const int s = issued % NAS;
-          if (issued >= NAS) {
-            const uint32_t par = (uint32_t)(issued / NAS - 1) & 1u;
-            if (!mbar_sleep_wait(empty + 8 * s, par) && !mbar_wait(empty + 8 * s, par, abort)) break;
-          }
-          mbar_arrive_expect_tx(full + 8 * s, bytes);
+        for (int u = u0; u < u1; u++) {
+          if (wrapped && !mbar_sleep_wait(t_empty + 8 * bt, par) && !mbar_wait(t_empty + 8 * bt, par, abort)) break;
+          mbar_arrive_expect_tx(t_full + 8 * bt, bytes);
           for (int i = 0; i < 2 * boxes; i++) {
             const int h = i & 1, bx = i >> 1;
-            tma_load_2d(sB + s * a.stage_bytes + h * (a.stage_bytes / 2) + bx * a.box * 128, &maps.x, full + 8 * s, u * 128 + h * 64, y0 + bx * a.box);
+            tma_load_2d(sB + bt * a.stage_bytes + h * (a.stage_bytes / 2) + bx * a.box * 128, &maps.x, t_full + 8 * bt, u * 128 + h * 64, y0 + bx * a.box);
           }
+          if (++bt == a.nbs) bt = 0, par ^= 1, wrapped = true;
         }
         pos += u1 - u0;
       }
@@ -330,15 +352,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   } else if (warp == MMA_WARP) {
     // The whole warp runs the loop and one elected lane issues.  A pass is a chain of some 60 instructions that share their
     // scheduler with the expanders: with 64 k and two or three barriers per pass it took 700 clocks and the tensor pipe
-    // stood at half its rate.  Hence 128 k to a stage, one barrier for all of its operands, and the look at the next
-    // stage's barrier issued before this stage's MMAs.
+    // stood at half its rate.  Hence 128 k to a stage, and the look at the next stage's barriers issued
+    // before this stage's MMAs.
     const bool leader = elect_one();
     const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
-    int s = 0, par = 0, seg = 0;
+    int s = 0, par = 0, bt = 0, bpar = 0, seg = 0;
     bool ok = true, wide_before = false;
-    for (int pos = pos0; pos < pos1 && ok; seg++) {
-      const int t = pos / nb, u0 = pos - t * nb, u1 = min(nb, u0 + (pos1 - pos));
-      const int nt = __shfl_sync(0xffffffffu, wk.tile(t).nt, 0);
+    auto W = wk.walk(pos0 / nb);
+    for (int pos = pos0; pos < pos1 && ok; seg++, wk.next(W)) {
+      const int u0 = pos - W.t * nb, u1 = min(nb, u0 + (pos1 - pos));
+      const int nt = __shfl_sync(0xffffffffu, W.nt, 0);
       const bool wide = nt > 128;
       if (rank == 0) {  // the accumulators this segment overwrites must have been read out
         if (seg >= 2 && !warp_wait(d_empty + 8 * (seg & 1), ((seg - 2) >> 1) & 1, abort)) break;
@@ -349,17 +372,18 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       const uint32_t idesc = idesc_f16(128 * CG, 16, BF16) + ((uint32_t)((nt - 16) >> 3) << 17);
       const int stages = u1 - u0;
       uint32_t acc = 0;
-      bool ready = mbar_test_wait(full + 8 * s, par);
+      bool ready = mbar_test_wait(full + 8 * s, par), tokens = mbar_test_wait(t_full + 8 * bt, bpar);
       for (int k = 0; k < stages; k++) {
-        if (!__all_sync(0xffffffffu, ready) && !warp_wait(full + 8 * s, par, abort)) {
+        if (!__all_sync(0xffffffffu, ready && tokens) && !(warp_wait(t_full + 8 * bt, bpar, abort) && warp_wait(full + 8 * s, par, abort))) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint64_t b0 = smem_desc_sw128(sB + s * a.stage_bytes), b1 = b0 + (uint64_t)(a.stage_bytes >> 5);
-        const uint32_t am = tm + A_COL + 64 * s, done = empty + 8 * s, fwd = full + 8 * s;
+        const uint64_t b0 = smem_desc_sw128(sB + bt * a.stage_bytes), b1 = b0 + (uint64_t)(a.stage_bytes >> 5);
+        const uint32_t am = tm + A_COL + 64 * s, done = empty + 8 * s, fwd = full + 8 * s, tdone = t_empty + 8 * bt;
         if (++s == NAS) s = 0, par ^= 1;
-        ready = mbar_test_wait(full + 8 * s, par);
+        if (++bt == a.nbs) bt = 0, bpar ^= 1;
+        ready = mbar_test_wait(full + 8 * s, par), tokens = mbar_test_wait(t_full + 8 * bt, bpar);
         if (CG == 1 || rank == 0) {
           if (leader) {
             mma_ts<CG>(d, am, b0, idesc, acc);
@@ -368,6 +392,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
 #pragma unroll
             for (int j = 0; j < 4; j++) mma_ts<CG>(d, am + 32 + 8 * j, b1 + 2 * j, idesc, 1u);
             commit<CG>(done);
+            commit<CG>(tdone);
           }
           acc = 1;
         } else {  // the pair's second CTA: its operands are ready, tell the one that issues
@@ -436,7 +461,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
     const bool shared = nb >= 8;
     auto finish_last = [&](int first, int step) {
       const int t = (pos1 - 1) / nb, u0 = max(pos0 - t * nb, 0), u1 = pos1 - t * nb, seg = t - pos0 / nb;
-      const Tile T = wk.tile(t);
+      const Tile T = wk.tile(wk.walk(t));
       if (first >= T.nt) return;
       const bool owner = u0 == 0;
       int jlast = cta;  // the runs that hold the rest of this tile
@@ -520,14 +545,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       const int rofs = 128 * rank + quad * 32;  // the warp's first row within the tile
       if constexpr (std::is_same<Row, TmDense>::value) pdl_wait();  // (a dense weight may have been expanded just now)
       // this warp's next unit: number in the run, in the tile, and the tile
-      int c = set, u, t;
-      t = (pos0 + c) / nb, u = pos0 + c - t * nb;
+      int c = set, t = (pos0 + c) / nb, u = pos0 + c - t * nb;  // (a walk's state would cost these warps registers: they search)
       Row rowx(ctx);
       [[maybe_unused]] int y = 0;                 // TMA: the warp's first row among all experts' rows
       [[maybe_unused]] const uint8_t *src = nullptr;  // row copies: its address, and the rows of the matrix after it
       [[maybe_unused]] int rows = 0;
       auto aim = [&]() {
-        const Tile T = wk.tile(t);
+        const Tile T = wk.tile(wk.walk(t));
         const int nw = min(T.n0 + rofs, a.N - 1);
         const size_t r0 = (size_t)T.expert * a.N;
         y = (int)(r0 + nw);
@@ -622,9 +646,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       const uint32_t strip = sStrip, sbytes = STRIP<OutT>;
       const bool bulk = ((size_t)a.N * sizeof(OutT)) % 16 == 0 && ((uintptr_t)out & 15) == 0;
       int seg = 0, chunk = 0;
-      for (int pos = pos0; pos < pos1; seg++) {
-        const int t = pos / nb, u0 = pos - t * nb, u1 = min(nb, u0 + (pos1 - pos));
-        const Tile T = wk.tile(t);
+      auto W = wk.walk(pos0 / nb);
+      for (int pos = pos0; pos < pos1; seg++, wk.next(W)) {
+        const int u0 = pos - W.t * nb, u1 = min(nb, u0 + (pos1 - pos));
+        const Tile T = wk.tile(W);
         pos += u1 - u0;
         if (pos >= pos1) {
           finish_last(0, shared ? 80 : 16);
@@ -732,7 +757,10 @@ int run(const typename Row::Ctx &ctx, const TmemCall &c, Args a, int nt_max, cud
   const int rows = nt_max / CG;
   a.box = !c.offsets ? rows : rows % 32 ? 16 : 32;
   a.stage_bytes = (rows + a.box - 1) / a.box * a.box * 256;
-  const int smem = NAS * a.stage_bytes + fixed_smem<Row>(a.E);
+  a.nbs = (SMEM_MAX - fixed_smem<Row>(a.E)) / a.stage_bytes;
+  if (a.nbs > NBS) a.nbs = NBS;
+  if (a.nbs < 3) return 0;
+  const int smem = a.nbs * a.stage_bytes + fixed_smem<Row>(a.E);
   if (smem > SMEM_MAX) return 0;
   int G = sm_count() / CG;
   if (G * CG > MAX_GRID) G = MAX_GRID / CG;
@@ -794,7 +822,7 @@ int pick(const typename Row::Ctx &ctx, const TmemCall &c, cudaStream_t st) {
   a.wmin = k_wmin;
   // The token tile: at most 256 (two SMs; less where the weight slots leave less room), all tiles of a matrix alike.  One SM
   // alone takes up to 128, with two accumulators.
-  int rows = (SMEM_MAX - fixed_smem<Row>(a.E)) / (NAS * 256) / 16 * 16;
+  int rows = (SMEM_MAX - fixed_smem<Row>(a.E)) / (3 * 256) / 16 * 16;
   if (rows > 128) rows = 128;
   // Two SMs to a tile halve the token traffic and the number of times a weight is expanded, one SM has the shorter chain of
   // hand-overs.  Measured crossing: 32 units per SM (333 tokens, 4096 x 4096: 21.6 us alone, 22.9 in pairs; 4096 x 14336: 46

@@ -179,6 +179,85 @@ PyObject *decode_attention(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
   return give(light_b200_decode_attn(&d, dev, stream_of(dev)), out);
 }
 
+// A route's expert sort: ids I64 (T, topk) and weights are the first two of the answer, then the sorted pairs and their experts.
+PyObject *sorted_route(const at::Tensor &ids, const at::Tensor &w, long long E, int dev) {
+  const int64_t M = ids.numel();
+  const auto i32 = ids.options().dtype(at::kInt);
+  at::Tensor sp = at::empty({M}, ids.options()), se = at::empty({M}, ids.options());
+  at::Tensor scratch = at::empty({M + (M + 1023) / 1024 * E + 1 + 2 * E + 1}, i32);
+  int *s = scratch.data_ptr<int>(), *counts = s, *offsets = s + E;
+  if (light_b200_moe_sort_pairs(ids.const_data_ptr<int64_t>(), counts, offsets, sp.data_ptr<int64_t>(), se.data_ptr<int64_t>(), s + 2 * E + 1, M, (int)E, dev,
+                                stream_of(dev)) != 0)
+    Py_RETURN_NONE;
+  PyObject *t = PyTuple_New(4);
+  const at::Tensor flat = w.reshape({M});
+  PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(ids)), PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(flat));
+  PyTuple_SET_ITEM(t, 2, THPVariable_Wrap(sp)), PyTuple_SET_ITEM(t, 3, THPVariable_Wrap(se));
+  return t;
+}
+
+// (scores F32 (T, E), bias F32 (E) or None, topk, normalize, sigmoid) -> (ids, weights, sorted pairs, sorted experts)
+PyObject *moe_route(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+  ARGS(5)
+  Arg x, b;
+  long long topk;
+  NEED(x.ok(a[0]) && long_of(a[2], topk) && cuda_contig(*x.t) && x.t->dim() == 2 && x.t->scalar_type() == at::kFloat && x.t->numel() > 0);
+  const int dev = x.t->get_device(), norm = PyObject_IsTrue(a[3]), sigmoid = PyObject_IsTrue(a[4]);
+  const int64_t T = x.t->size(0), E = x.t->size(1);
+  NEED(topk >= 1 && topk <= E && topk <= 32 && E <= 1024 && T * topk < (1ll << 31));
+  if (a[1] != Py_None)
+    NEED(sigmoid && b.ok(a[1]) && cuda_contig(*b.t) && b.t->scalar_type() == at::kFloat && b.t->numel() == E && b.t->get_device() == dev);
+  at::Tensor ids = at::empty({T, topk}, x.t->options().dtype(at::kLong)), w = at::empty({T, topk}, x.t->options());
+  const float *in = x.t->const_data_ptr<float>();
+  const int rc = sigmoid ? light_b200_moe_route_sigmoid(in, b.t ? b.t->const_data_ptr<float>() : nullptr, ids.data_ptr<int64_t>(), w.data_ptr<float>(), (int)T, (int)E,
+                                                        (int)topk, norm, dev, stream_of(dev))
+                         : light_b200_moe_route_topk(in, ids.data_ptr<int64_t>(), w.data_ptr<float>(), (int)T, (int)E, (int)topk, norm, dev, stream_of(dev));
+  if (rc != 0) Py_RETURN_NONE;
+  return sorted_route(ids, w, E, dev);
+}
+
+// (input (rows, K), weights, scale or None, block rows, block columns, ggml type (-1: block FP8), E, N, K, sorted pairs, sorted
+// experts, pair weights or None, topk) -> (M, N) at the input's type
+PyObject *moe_gemm(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+  ARGS(13)
+  Arg x, w, s, sp, se, tw;
+  long long bR, bC, type, E, N, K, topk;
+  NEED(x.ok(a[0]) && w.ok(a[1]) && long_of(a[3], bR) && long_of(a[4], bC) && long_of(a[5], type) && long_of(a[6], E) && long_of(a[7], N) && long_of(a[8], K) &&
+       sp.ok(a[9]) && se.ok(a[10]) && long_of(a[12], topk));
+  NEED(cuda_contig(*x.t) && cuda_contig(*w.t) && cuda_contig(*sp.t) && cuda_contig(*se.t) && x.t->dim() == 2 && x.t->size(1) == K && x.t->numel() > 0);
+  const int dev = x.t->get_device();
+  const int64_t M = sp.t->numel(), rows = x.t->size(0);
+  NEED(sp.t->scalar_type() == at::kLong && se.t->scalar_type() == at::kLong && sp.t->dim() == 1 && se.t->dim() == 1 && se.t->numel() == M && M > 0 && M < (1ll << 31) &&
+       topk > 0 && E > 0 && N > 0 && N < (1ll << 31) && (rows == M || rows == M / topk));
+  NEED(w.t->get_device() == dev && sp.t->get_device() == dev && se.t->get_device() == dev);
+  const auto dt = x.t->scalar_type();
+  if (type >= 0) {
+    const int be = light_b200_block_elems((int)type);
+    NEED(dt == at::kFloat && be > 0 && K % be == 0 && w.t->scalar_type() == at::kByte && w.t->numel() == E * N * (K / be) * light_b200_block_bytes((int)type));
+  } else {
+    NEED((dt == at::kFloat || dt == at::kBFloat16) && s.ok(a[2]) && cuda_contig(*s.t) && s.t->scalar_type() == at::kFloat && s.t->get_device() == dev && bR > 0 &&
+         bC > 0 && N % bR == 0 && K % bC == 0 && w.t->element_size() == 1 && w.t->numel() == E * N * K && s.t->numel() == E * (N / bR) * (K / bC));
+  }
+  if (a[11] != Py_None) NEED(tw.ok(a[11]) && cuda_contig(*tw.t) && tw.t->scalar_type() == at::kFloat && tw.t->numel() == M && tw.t->get_device() == dev);
+  NEED(workspace_fits(dev, M > 65 ? M : 65, K));
+  // Rows that no pair writes are zero: cleared as a whole while that is cheaper than finding them.
+  const int64_t row_bytes = N * (int64_t)x.t->element_size(), words = (M + 31) / 32;
+  const bool find = M * row_bytes > (8 << 20);
+  at::Tensor out = find ? at::empty({M, N}, x.t->options()) : at::zeros({M, N}, x.t->options());
+  at::Tensor scratch = at::empty({2 * E + 1 + (find ? words : 0)}, sp.t->options().dtype(at::kInt));
+  int *sc = scratch.data_ptr<int>();
+  void *st = stream_of(dev);
+  if (find && light_b200_moe_clear_unrouted(sp.t->const_data_ptr<int64_t>(), se.t->const_data_ptr<int64_t>(), (uint32_t *)(sc + 2 * E + 1), out.data_ptr(), M, M,
+                                            row_bytes, (int)E, dev, st) != 0)
+    Py_RETURN_NONE;
+  lb200_moe_args m{};
+  m.input = x.t->const_data_ptr(), m.weights = w.t->const_data_ptr(), m.sorted_pairs = sp.t->const_data_ptr<int64_t>();
+  m.expert_ids = se.t->const_data_ptr<int64_t>(), m.counts = sc, m.offsets = sc + E, m.topk_weights = tw.t ? tw.t->const_data_ptr<float>() : nullptr;
+  m.out = out.data_ptr(), m.M = M, m.size_m = M, m.E = (int)E, m.N = (int)N, m.K = (int)K, m.topk = (int)topk, m.row_per_pair = rows == M;
+  m.dtype = type >= 0 ? (int)type : act_of(*x.t);
+  return give(type >= 0 ? light_b200_moe_gemm_q(&m, dev, st) : light_b200_moe_gemm_f8block(&m, s.t->const_data_ptr<float>(), (int)bR, (int)bC, dev, st), out);
+}
+
 #define FN(f, doc) {#f, (PyCFunction)(void (*)(void))f, METH_FASTCALL, doc}
 PyMethodDef kMethods[] = {FN(set_workspace, "registers a device's workspace size"),
                           FN(linear_q, "x . W^T, GGUF blocks"),
@@ -186,6 +265,8 @@ PyMethodDef kMethods[] = {FN(set_workspace, "registers a device's workspace size
                           FN(linear_f8, "x . W^T, block-scaled FP8"),
                           FN(gate_mul, "act(gate) * up"),
                           FN(combine, "sum of the top-k slot rows"),
+                          FN(moe_route, "top-k experts of each token and the pairs sorted by expert"),
+                          FN(moe_gemm, "grouped x . W^T"),
                           FN(decode_attention, "append + rotary embedding + attention"),
                           {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host", "native host path of light_b200", -1, kMethods, nullptr, nullptr, nullptr, nullptr};

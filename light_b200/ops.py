@@ -502,6 +502,9 @@ def MoERoute(probs: torch.Tensor, topk: int, normalize: bool) -> MoERouting:
     """ops.MoERoute (ops/moe.go:29-71): router probabilities (T, E) F32 -> the k largest experts per token, their
     probabilities (renormalised when `normalize`), and the pairs sorted by expert.  Selection and sort run on the
     device (light_b200_moe_route_topk + light_b200_moe_sort_pairs); ties keep the lower expert id."""
+    r = _host.moe_route(probs, None, topk, normalize, False)
+    if r is not None:
+        return MoERouting(*r)
     if probs.dim() != 2 or probs.dtype != torch.float32:
         raise ValueError(f"moe_route: probs must be (T, E) F32, got {tuple(probs.shape)} {probs.dtype}")
     T, E = probs.shape
@@ -539,6 +542,9 @@ def MoERouteDeepseek(logits: torch.Tensor, bias: Optional[torch.Tensor], topk: i
 def MoERouteSigmoid(logits: torch.Tensor, bias: Optional[torch.Tensor], topk: int, norm_topk: bool = True, E_sort: Optional[int] = None) -> MoERouting:
     """The DeepSeek-V3 router (models/deepseek_route.go:30-133, sigmoid branch, one group) and the expert sort of
     ops.MoERouteFromIDs (ops/moe.go:73-99), both on the device: logits (T, E) F32, bias (E) F32 or None."""
+    r = _host.moe_route(logits, bias, topk, norm_topk, True)
+    if r is not None:
+        return MoERouting(*r)
     if logits.dim() != 2 or logits.dtype != torch.float32:
         raise ValueError(f"moe_route: logits must be (T, E) F32, got {tuple(logits.shape)} {logits.dtype}")
     T, E = logits.shape
@@ -631,6 +637,10 @@ def MoEGemm(inp: torch.Tensor, weights: torch.Tensor, routing: MoERouting, topk_
 def MoEGemmQ(x: torch.Tensor, w: QTensor, routing: MoERouting, topk_weights: Optional[torch.Tensor],
              topk: int) -> torch.Tensor:
     """ops.MoEGemmQ (ops/moe.go:242-265): GGUF block-quantized experts (E, N, K), x f32, out f32."""
+    if type(w) is QTensor and len(w.shape) == 3:
+        y = _host.moe_gemm(x, w.data, None, 0, 0, w.ggml_type, *w.shape, routing.sorted_pairs, routing.sorted_expts, topk_weights, topk)
+        if y is not None:
+            return y
     if x.dtype != torch.float32:
         raise ValueError(f"moe_gemm_q: x must be F32, got {x.dtype}")
     if len(w.shape) != 3:
@@ -645,6 +655,10 @@ def MoEGemmF8Block(x: torch.Tensor, w: torch.Tensor, scale: torch.Tensor, block_
     f32 (E, N/bR, K/bC), x F32 or BF16 (rows per token or per pair), output (M, N) at x's dtype.  The
     reference runs this as a host loop over experts (models/moe_routed.go:34-79: IndexSelect, one
     ops.MatMulF8Block per expert, scatter); the contract per pair is the same as MoEGemm's."""
+    if w.dim() == 3:
+        y = _host.moe_gemm(x, w, scale, block_r, block_c, -1, *w.shape, routing.sorted_pairs, routing.sorted_expts, topk_weights, topk)
+        if y is not None:
+            return y
     if x.dtype not in (torch.float32, torch.bfloat16):
         raise ValueError(f"moe_gemm_f8block: activations {x.dtype}, want F32 or BF16")
     if w.dim() != 3 or scale.dim() != 3:
