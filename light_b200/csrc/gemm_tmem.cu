@@ -219,7 +219,11 @@ struct Work {
     w.rt = w.ntt ? r / w.ntt : 0, w.tt = r - w.rt * w.ntt;
     return w;
   }
-  __device__ __forceinline__ void next(Walk &w) const {
+  __device__ __forceinline__ void next(Walk &w, int stride) const {
+    if (stride > 1) {
+      if (w.t + stride < preT[a.E]) w = walk(w.t + stride);
+      return;
+    }
     w.t++;
     if (++w.tt < w.ntt) return;
     w.tt = 0;
@@ -251,7 +255,8 @@ struct Work {
 // ------------------------------------------------------------------------------------ kernel
 template <typename OutT>
 constexpr uint32_t STRIP = 32 * 128 * sizeof(OutT);  // 32 tokens of 128 output columns
-constexpr int STRIPS = 16384;                        // one strip of f32, two of bf16
+template <typename OutT>
+constexpr int STRIPS = 2 * STRIP<OutT>;
 
 struct Maps {
   CUtensorMap x, w[2];  // tokens; the weight rows, per box of the format
@@ -265,7 +270,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   __shared__ uint32_t tmem_sh;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char *gen = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t sB = base, sRaw = base + (uint32_t)a.nbs * a.stage_bytes, sStrip = sRaw + (uint32_t)EXPANDERS * Row::SLOT, sBar = sStrip + STRIPS;
+  const uint32_t sB = base, sRaw = base + (uint32_t)a.nbs * a.stage_bytes, sStrip = sRaw + (uint32_t)EXPANDERS * Row::SLOT, sBar = sStrip + STRIPS<OutT>;
   // full[s]: a stage's weights are there (four warps; in the first CTA of a pair also: the other CTA's weights and tokens);
   // empty[s]: its MMAs have completed.  t_full, t_empty: the token ring's, which runs further ahead: a token tile takes a TMA
   // latency to refill, and with only four stages that, not the tensor core, set the pace of narrow tiles.
@@ -323,17 +328,24 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   tc_fence_after();
   const uint32_t tmem = tmem_sh;
   volatile int *abort = &abort_flag;
-  const int pos0 = wk.bound(cta, G), pos1 = wk.bound(cta + 1, G);
-  const int n = pos1 - pos0;  // units of this run
+  // This CTA (pair)'s run: n units from unit v0 of tile tf on, then tile tf + stride, ...  Where there are plenty of tiles a grouped
+  // launch deals them out in turn instead: the tiles in flight are then neighbours, of a few experts whose tokens
+  // stay in L2.  (Contiguous runs, one far from the other, read the tokens of 74 experts at once, more than L2 holds, and
+  // from HBM again for every row tile.)
+  const int total = preT[a.E];
+  const bool dealt = a.offsets && total >= 16 * G;
+  const int pos0 = dealt ? cta * nb : wk.bound(cta, G), tf = pos0 / nb, v0 = pos0 - tf * nb, stride = dealt ? G : 1;
+  const int n = dealt ? (total > cta ? (total - 1 - cta) / G + 1 : 0) * nb : wk.bound(cta + 1, G) - pos0;
+  const int v1 = v0 + n;
 
   if (warp == TMA_WARP) {
     if (lane == 0) {
       pdl_wait();  // the tokens may be the kernel before's; the weights are not
       int bt = 0, par = 1;
       bool wrapped = false;
-      auto W = wk.walk(pos0 / nb);
-      for (int pos = pos0; pos < pos1 && !*abort; wk.next(W)) {
-        const int u0 = pos - W.t * nb, u1 = min(nb, u0 + (pos1 - pos));
+      auto W = wk.walk(tf);
+      for (int v = v0; v < v1 && !*abort; wk.next(W, stride)) {
+        const int u0 = v % nb, u1 = min(nb, u0 + (v1 - v));
         const Tile T = wk.tile(W);
         const int rows = T.nt / CG, boxes = (rows + a.box - 1) / a.box, y0 = T.m0 + rank * rows;
         const uint32_t bytes = (uint32_t)(boxes * a.box) * 256u;
@@ -346,7 +358,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
           }
           if (++bt == a.nbs) bt = 0, par ^= 1, wrapped = true;
         }
-        pos += u1 - u0;
+        v += u1 - u0;
       }
     }
   } else if (warp == MMA_WARP) {
@@ -358,9 +370,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
     const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
     int s = 0, par = 0, bt = 0, bpar = 0, seg = 0;
     bool ok = true, wide_before = false;
-    auto W = wk.walk(pos0 / nb);
-    for (int pos = pos0; pos < pos1 && ok; seg++, wk.next(W)) {
-      const int u0 = pos - W.t * nb, u1 = min(nb, u0 + (pos1 - pos));
+    auto W = wk.walk(tf);
+    for (int v = v0; v < v1 && ok; seg++, wk.next(W, stride)) {
+      const int u0 = v % nb, u1 = min(nb, u0 + (v1 - v));
       const int nt = __shfl_sync(0xffffffffu, W.nt, 0);
       const bool wide = nt > 128;
       if (rank == 0) {  // the accumulators this segment overwrites must have been read out
@@ -403,7 +415,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       }
       if (ok && rank == 0 && leader) commit<CG>(d_full + 8 * (seg & 1));
       __syncwarp();
-      pos += u1 - u0;
+      v += u1 - u0;
     }
     if (rank == 0) {  // no MMA may be in flight when tensor memory is given back, whichever way the loop ended
       if (leader) commit<CG>(drained);
@@ -460,7 +472,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
     // once, a lane to each, and the partial sums of two runs are on their way together.
     const bool shared = nb >= 8;
     auto finish_last = [&](int first, int step) {
-      const int t = (pos1 - 1) / nb, u0 = max(pos0 - t * nb, 0), u1 = pos1 - t * nb, seg = t - pos0 / nb;
+      const int seg = (v1 - 1) / nb, t = tf + seg * stride, u0 = seg ? 0 : v0, u1 = v1 - seg * nb;
       const Tile T = wk.tile(wk.walk(t));
       if (first >= T.nt) return;
       const bool owner = u0 == 0;
@@ -545,7 +557,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       const int rofs = 128 * rank + quad * 32;  // the warp's first row within the tile
       if constexpr (std::is_same<Row, TmDense>::value) pdl_wait();  // (a dense weight may have been expanded just now)
       // this warp's next unit: number in the run, in the tile, and the tile
-      int c = set, t = (pos0 + c) / nb, u = pos0 + c - t * nb;  // (a walk's state would cost these warps registers: they search)
+      int c = set, t = tf + (v0 + c) / nb * stride, u = (v0 + c) % nb;  // (a walk's state would cost these warps registers: they search)
       Row rowx(ctx);
       [[maybe_unused]] int y = 0;                 // TMA: the warp's first row among all experts' rows
       [[maybe_unused]] const uint8_t *src = nullptr;  // row copies: its address, and the rows of the matrix after it
@@ -613,7 +625,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
           c += EXPANDERS / 4, u += EXPANDERS / 4;
           if (c < n) {
             if (u >= nb) {
-              while (u >= nb) u -= nb, t++;
+              while (u >= nb) u -= nb, t += stride;
               aim();
             }
             issue();
@@ -646,12 +658,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       const uint32_t strip = sStrip, sbytes = STRIP<OutT>;
       const bool bulk = ((size_t)a.N * sizeof(OutT)) % 16 == 0 && ((uintptr_t)out & 15) == 0;
       int seg = 0, chunk = 0;
-      auto W = wk.walk(pos0 / nb);
-      for (int pos = pos0; pos < pos1; seg++, wk.next(W)) {
-        const int u0 = pos - W.t * nb, u1 = min(nb, u0 + (pos1 - pos));
+      auto W = wk.walk(tf);
+      for (int v = v0; v < v1; seg++, wk.next(W, stride)) {
+        const int u0 = v % nb, u1 = min(nb, u0 + (v1 - v));
         const Tile T = wk.tile(W);
-        pos += u1 - u0;
-        if (pos >= pos1) {
+        v += u1 - u0;
+        if (v >= v1) {
           finish_last(0, shared ? 80 : 16);
           break;
         }
@@ -685,10 +697,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
             for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * __shfl_sync(0xffffffffu, pw, i));
           }
           if (bulk) {
-            constexpr bool two = 2 * STRIP<OutT> <= STRIPS;
-            const uint32_t buf = strip + (two ? (chunk & 1) * sbytes : 0);
-            if (two) asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");  // this lane's last copy from this strip
-            else asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
+            const uint32_t buf = strip + (chunk & 1) * sbytes;
+            asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");  // this lane's last copy from this strip
             asm volatile("bar.sync 1, 128;\n" ::: "memory");
 #pragma unroll
             for (int i = 0; i < 32; i++) {
@@ -748,8 +758,8 @@ int knob(const char *name, int otherwise) {
   return e ? atoi(e) : otherwise;
 }
 
-template <typename Row>
-constexpr int fixed_smem(int E) { return EXPANDERS * Row::SLOT + STRIPS + BAR_BYTES + (E + 1) * 12 + 16 + 1024; }
+template <typename Row, typename OutT>
+constexpr int fixed_smem(int E) { return EXPANDERS * Row::SLOT + STRIPS<OutT> + BAR_BYTES + (E + 1) * 12 + 16 + 1024; }
 
 template <typename Row, bool BF16, typename OutT, int CG>
 int run(const typename Row::Ctx &ctx, const TmemCall &c, Args a, int nt_max, cudaStream_t st) {
@@ -757,10 +767,10 @@ int run(const typename Row::Ctx &ctx, const TmemCall &c, Args a, int nt_max, cud
   const int rows = nt_max / CG;
   a.box = !c.offsets ? rows : rows % 32 ? 16 : 32;
   a.stage_bytes = (rows + a.box - 1) / a.box * a.box * 256;
-  a.nbs = (SMEM_MAX - fixed_smem<Row>(a.E)) / a.stage_bytes;
+  a.nbs = (SMEM_MAX - fixed_smem<Row, OutT>(a.E)) / a.stage_bytes;
   if (a.nbs > NBS) a.nbs = NBS;
   if (a.nbs < 3) return 0;
-  const int smem = a.nbs * a.stage_bytes + fixed_smem<Row>(a.E);
+  const int smem = a.nbs * a.stage_bytes + fixed_smem<Row, OutT>(a.E);
   if (smem > SMEM_MAX) return 0;
   int G = sm_count() / CG;
   if (G * CG > MAX_GRID) G = MAX_GRID / CG;
@@ -822,7 +832,7 @@ int pick(const typename Row::Ctx &ctx, const TmemCall &c, cudaStream_t st) {
   a.wmin = k_wmin;
   // The token tile: at most 256 (two SMs; less where the weight slots leave less room), all tiles of a matrix alike.  One SM
   // alone takes up to 128, with two accumulators.
-  int rows = (SMEM_MAX - fixed_smem<Row>(a.E)) / (3 * 256) / 16 * 16;
+  int rows = (SMEM_MAX - fixed_smem<Row, OutT>(a.E)) / (3 * 256) / 16 * 16;
   if (rows > 128) rows = 128;
   // Two SMs to a tile halve the token traffic and the number of times a weight is expanded, one SM has the shorter chain of
   // hand-overs.  Measured crossing: 32 units per SM (333 tokens, 4096 x 4096: 21.6 us alone, 22.9 in pairs; 4096 x 14336: 46
