@@ -15,7 +15,9 @@ namespace {
 
 constexpr int RT_MAX_PER_LANE = 32;  // experts per lane: E <= 1024
 
-// one warp per token
+// One warp per token.  PER: experts per lane, rounded up to a power of two, so that the scores stay in registers (indexed by a
+// run-time loop they lay in local memory, and a choice of eight out of 256 experts took 14 us).
+template <int PER>
 __global__ void __launch_bounds__(256) moe_route_sigmoid_kernel(const float *__restrict__ logits, const float *__restrict__ bias,
                                                                 long long *__restrict__ ids, float *__restrict__ weights, int T, int E,
                                                                 int topk, int norm_topk) {
@@ -23,10 +25,9 @@ __global__ void __launch_bounds__(256) moe_route_sigmoid_kernel(const float *__r
   pdl_wait();
   const int tok = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (tok >= T) return;
-  const int per = (E + 31) / 32;
-  double score[RT_MAX_PER_LANE], choice[RT_MAX_PER_LANE];
-#pragma unroll 1
-  for (int i = 0; i < per; i++) {
+  double score[PER], choice[PER];
+#pragma unroll
+  for (int i = 0; i < PER; i++) {
     const int e = i * 32 + lane;  // expert e sits in slot e / 32 of lane e % 32
     if (e < E) {
       score[i] = 1.0 / (1.0 + exp(-(double)logits[(size_t)tok * E + e]));
@@ -40,11 +41,11 @@ __global__ void __launch_bounds__(256) moe_route_sigmoid_kernel(const float *__r
   long long mine_id = 0;
   for (int k = 0; k < topk; k++) {
     // this lane's best free slot (the lowest expert id among equals: slots ascend with the id)
-    double bv = -INFINITY;
+    double bv = -INFINITY, sc = 0.0;
     int be = 0x7fffffff;
-#pragma unroll 1
-    for (int i = 0; i < per; i++)
-      if (!(taken >> i & 1u) && i * 32 + lane < E && choice[i] > bv) bv = choice[i], be = i * 32 + lane;
+#pragma unroll
+    for (int i = 0; i < PER; i++)
+      if (!(taken >> i & 1u) && i * 32 + lane < E && choice[i] > bv) bv = choice[i], be = i * 32 + lane, sc = score[i];
     // the warp's best: larger choice, then lower expert id
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -52,11 +53,8 @@ __global__ void __launch_bounds__(256) moe_route_sigmoid_kernel(const float *__r
       const int oe = __shfl_xor_sync(0xffffffffu, be, o);
       if (ov > bv || (ov == bv && oe < be)) bv = ov, be = oe;
     }
-    double sc = 0.0;
-    if ((be & 31) == lane && be < E) {
-      taken |= 1u << (be >> 5);
-      sc = score[be >> 5];
-    }
+    if ((be & 31) == lane && be < E) taken |= 1u << (be >> 5);
+    else sc = 0.0;
     sc = __shfl_sync(0xffffffffu, sc, be & 31);
     den += sc;
     if (lane == k % 32) mine_w = sc, mine_id = be;  // lane k keeps selection k (topk <= 32)
@@ -196,24 +194,24 @@ __global__ void __launch_bounds__(256) moe_route_deepseek_kernel(const float *__
 
 // ops.MoERoute's selection (ops/moe.go:29-50): the k largest router probabilities of a token (ties keep the lower
 // expert id), their values as weights, divided by their f32 sum (added in selection order) when normalize.
+template <int PER>
 __global__ void __launch_bounds__(256) moe_route_topk_kernel(const float *__restrict__ probs, long long *__restrict__ ids, float *__restrict__ weights,
                                                              int T, int E, int topk, int normalize) {
   pdl_launch_dependents();
   pdl_wait();
   const int tok = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (tok >= T) return;
-  const int per = (E + 31) / 32;
-  float v[RT_MAX_PER_LANE];
-#pragma unroll 1
-  for (int i = 0; i < per; i++) v[i] = i * 32 + lane < E ? probs[(size_t)tok * E + i * 32 + lane] : 0.f;
+  float v[PER];
+#pragma unroll
+  for (int i = 0; i < PER; i++) v[i] = i * 32 + lane < E ? probs[(size_t)tok * E + i * 32 + lane] : 0.f;
   unsigned taken = 0;
   float sum = 0.f, mine_w = 0.f;
   long long mine_id = 0;
   for (int k = 0; k < topk; k++) {
     float bv = 0.f;
     int be = 0x7fffffff;
-#pragma unroll 1
-    for (int i = 0; i < per; i++)
+#pragma unroll
+    for (int i = 0; i < PER; i++)
       if (!(taken >> i & 1u) && i * 32 + lane < E && (be == 0x7fffffff || v[i] > bv)) bv = v[i], be = i * 32 + lane;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -269,6 +267,59 @@ __global__ void __launch_bounds__(SORT_BLOCK) moe_sort_local_kernel(const long l
   if (p < M) local_rank[p] = warp_hist[warp * E + (int)e] + r;
 }
 
+// Up to 1024 pairs: the whole sort in one CTA and one launch (a decode step sorts a few dozen; three dependent launches took 25 us).
+__global__ void __launch_bounds__(SORT_BLOCK) moe_sort_small_kernel(const long long *__restrict__ ids, int *__restrict__ counts, int *__restrict__ offsets,
+                                                                    long long *__restrict__ sorted_pairs, long long *__restrict__ sorted_expts, int M, int E,
+                                                                    unsigned int *__restrict__ status) {
+  extern __shared__ int warp_hist[];  // [warps in use][E], then [E] experts' first positions
+  pdl_launch_dependents();
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = (M + 31) / 32;
+  int *base = warp_hist + warps * E;
+  for (int i = threadIdx.x; i < warps * E; i += SORT_BLOCK) warp_hist[i] = 0;
+  __syncthreads();
+  const int p = threadIdx.x;
+  long long e = p < M ? ids[p] : -1;
+  if (p < M && (e < 0 || e >= E)) {  // reported, and parked with expert 0 so that nothing is written out of range
+    atomicOr(status, 1u);
+    e = 0;
+  }
+  const unsigned same = __match_any_sync(0xffffffffu, e);
+  const int r = __popc(same & ((1u << lane) - 1u));
+  if (e >= 0 && r == 0) warp_hist[warp * E + (int)e] = __popc(same);
+  __syncthreads();
+  for (int x = threadIdx.x; x < E; x += SORT_BLOCK) {
+    int run = 0;
+    for (int w = 0; w < warps; w++) {
+      const int c = warp_hist[w * E + x];
+      warp_hist[w * E + x] = run;
+      run += c;
+    }
+    counts[x] = run, base[x] = run;
+  }
+  __syncthreads();
+  if (warp == 0) {  // exclusive prefix over the experts
+    int carry = 0;
+    for (int x0 = 0; x0 < E; x0 += 32) {
+      const int c = x0 + lane < E ? base[x0 + lane] : 0;
+      int v = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+      }
+      if (x0 + lane < E) base[x0 + lane] = offsets[x0 + lane] = carry + v - c;
+      carry += __shfl_sync(0xffffffffu, v, 31);
+    }
+    if (lane == 0) offsets[E] = carry;
+  }
+  __syncthreads();
+  if (p < M) {
+    const int pos = base[e] + warp_hist[warp * E + (int)e] + r;
+    sorted_pairs[pos] = p, sorted_expts[pos] = e;
+  }
+}
+
 // counts, offsets, and the base of every (block, expert) run: one CTA
 __global__ void __launch_bounds__(1024) moe_sort_scan_kernel(int *__restrict__ block_hist, int *__restrict__ counts, int *__restrict__ offsets,
                                                              int nblocks, int E) {
@@ -277,20 +328,35 @@ __global__ void __launch_bounds__(1024) moe_sort_scan_kernel(int *__restrict__ b
   pdl_wait();
   for (int x = threadIdx.x; x < E; x += 1024) {
     int run = 0;
-#pragma unroll 1
-    for (int b = 0; b < nblocks; b++) {
-      const int c = block_hist[(size_t)b * E + x];
-      block_hist[(size_t)b * E + x] = run;  // pairs of expert x in earlier blocks
-      run += c;
+    for (int b0 = 0; b0 < nblocks; b0 += 16) {  // sixteen loads on their way at once
+      int c[16];
+#pragma unroll
+      for (int i = 0; i < 16; i++) c[i] = b0 + i < nblocks ? block_hist[(size_t)(b0 + i) * E + x] : 0;
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        if (b0 + i < nblocks) block_hist[(size_t)(b0 + i) * E + x] = run;  // pairs of expert x in earlier blocks
+        run += c[i];
+      }
     }
     tot[x] = run;
     counts[x] = run;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int x = 0; x < E; x++) offsets[x] = run, run += tot[x];
-    offsets[E] = run;
+  if (threadIdx.x < 32) {  // exclusive prefix over the experts
+    const int lane = threadIdx.x;
+    int carry = 0;
+    for (int x0 = 0; x0 < E; x0 += 32) {
+      const int c = x0 + lane < E ? tot[x0 + lane] : 0;
+      int v = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+      }
+      if (x0 + lane < E) offsets[x0 + lane] = carry + v - c;
+      carry += __shfl_sync(0xffffffffu, v, 31);
+    }
+    if (lane == 0) offsets[E] = carry;
   }
 }
 
@@ -328,8 +394,13 @@ cudaError_t launch_chain(Kern kern, unsigned grid, unsigned block, size_t smem, 
 int moe_route_sigmoid(const float *logits, const float *bias, int64_t *ids, float *weights, int T, int E, int topk, int norm_topk,
                       cudaStream_t st) {
   if (T == 0) return 0;
-  cudaError_t e = launch_chain(moe_route_sigmoid_kernel, (unsigned)((T + 7) / 8), 256, 0, st, logits, bias, (long long *)ids, weights, T, E, topk,
-                               norm_topk);
+  auto go = [&](auto kern) { return launch_chain(kern, (unsigned)((T + 7) / 8), 256, 0, st, logits, bias, (long long *)ids, weights, T, E, topk, norm_topk); };
+  const cudaError_t e = E <= 32    ? go(moe_route_sigmoid_kernel<1>)
+                        : E <= 64  ? go(moe_route_sigmoid_kernel<2>)
+                        : E <= 128 ? go(moe_route_sigmoid_kernel<4>)
+                        : E <= 256 ? go(moe_route_sigmoid_kernel<8>)
+                        : E <= 512 ? go(moe_route_sigmoid_kernel<16>)
+                                   : go(moe_route_sigmoid_kernel<RT_MAX_PER_LANE>);
   if (e != cudaSuccess) return fail((int)e, "light_b200: moe_route_sigmoid: %s", cudaGetErrorString(e));
   return launched("moe_route_sigmoid");
 }
@@ -345,7 +416,13 @@ int moe_route_deepseek(const float *logits, const float *bias, int64_t *ids, flo
 
 int moe_route_topk(const float *probs, int64_t *ids, float *weights, int T, int E, int topk, int normalize, cudaStream_t st) {
   if (T == 0) return 0;
-  cudaError_t e = launch_chain(moe_route_topk_kernel, (unsigned)((T + 7) / 8), 256, 0, st, probs, (long long *)ids, weights, T, E, topk, normalize);
+  auto go = [&](auto kern) { return launch_chain(kern, (unsigned)((T + 7) / 8), 256, 0, st, probs, (long long *)ids, weights, T, E, topk, normalize); };
+  const cudaError_t e = E <= 32    ? go(moe_route_topk_kernel<1>)
+                        : E <= 64  ? go(moe_route_topk_kernel<2>)
+                        : E <= 128 ? go(moe_route_topk_kernel<4>)
+                        : E <= 256 ? go(moe_route_topk_kernel<8>)
+                        : E <= 512 ? go(moe_route_topk_kernel<16>)
+                                   : go(moe_route_topk_kernel<RT_MAX_PER_LANE>);
   if (e != cudaSuccess) return fail((int)e, "light_b200: moe_route_topk: %s", cudaGetErrorString(e));
   return launched("moe_route_topk");
 }
@@ -364,10 +441,17 @@ int moe_sort_pairs(const int64_t *ids, int *counts, int *offsets, int64_t *sorte
   if (e == cudaSuccess)
     e = attr_done.ensure([&] {  // the first call on a device: make it outside stream capture
       cudaError_t r = cudaFuncSetAttribute(moe_sort_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 1024 * 4);
+      if (r == cudaSuccess) r = cudaFuncSetAttribute(moe_sort_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 33 * 1024 * 4);
       return r != cudaSuccess ? r : cudaGetSymbolAddress((void **)&status_of[dev], g_route_status);
     });
   if (e != cudaSuccess) return fail((int)e, "light_b200: moe_sort_pairs: %s", cudaGetErrorString(e));
   unsigned int *status = status_of[dev];
+  if (nblocks == 1) {
+    e = launch_chain(moe_sort_small_kernel, 1u, SORT_BLOCK, (size_t)((M + 31) / 32 + 1) * E * 4, st, (const long long *)ids, counts, offsets,
+                     (long long *)sorted_pairs, (long long *)sorted_expts, (int)M, E, status);
+    if (e != cudaSuccess) return fail((int)e, "light_b200: moe_sort_pairs: %s", cudaGetErrorString(e));
+    return launched("moe_sort_pairs");
+  }
   if (e == cudaSuccess && nblocks > 0)
     e = launch_chain(moe_sort_local_kernel, (unsigned)nblocks, SORT_BLOCK, (size_t)32 * E * 4, st, (const long long *)ids, local_rank, block_hist, M, E,
                      status);

@@ -48,6 +48,35 @@ def test_sort_pairs(cuda, oracle, M, E):
     assert ops.moe_route_status(0) == 0
 
 
+@pytest.mark.parametrize("M,E", [(1, 1024), (31, 8), (32, 33), (33, 1), (1023, 256), (1024, 1024)])
+def test_sort_pairs_in_one_launch(cuda, M, E):
+    """Up to 1024 pairs one CTA sorts: the edges of its warps and the most experts it holds."""
+    ids = torch.randint(0, E, (M,), generator=torch.Generator().manual_seed(920 + M))
+    sp, se, counts, offsets = ops.MoESortPairs(ids.to(cuda), E)
+    we, wp = torch.sort(ids, stable=True)
+    c = torch.bincount(ids, minlength=E)
+    assert torch.equal(sp.cpu(), wp) and torch.equal(se.cpu(), we)
+    assert torch.equal(counts.cpu().long(), c) and torch.equal(offsets.cpu().long(), torch.cat([torch.zeros(1, dtype=torch.int64), c.cumsum(0)]))
+
+
+@pytest.mark.parametrize("E", [32, 33, 64, 65, 128, 129, 257, 512, 513, 1024])
+def test_route_at_every_width_of_a_lane(cuda, E):
+    """1 to 32 experts per lane, at both ends of each compiled width; ids exact, weights to 1e-6 of the f64 ones."""
+    T, topk = 9, 7
+    g = torch.Generator().manual_seed(930 + E)
+    logits, bias = torch.randn(T, E, generator=g), torch.randn(E, generator=g)
+    score = torch.sigmoid(logits.double())
+    want = torch.sort(score + bias.double(), dim=1, descending=True, stable=True).indices[:, :topk]
+    w = score.gather(1, want)
+    r = ops.MoERouteSigmoid(logits.to(cuda), bias.to(cuda), topk, True)
+    assert torch.equal(r.topk_ids.cpu(), want)
+    assert (r.weights.reshape(T, topk).cpu() - w / w.sum(1, keepdim=True)).abs().max() <= 1e-6
+    probs = torch.softmax(logits, dim=1)
+    want = torch.sort(probs, dim=1, descending=True, stable=True).indices[:, :topk]
+    r = ops.MoERoute(probs.to(cuda), topk, False)
+    assert torch.equal(r.topk_ids.cpu(), want) and torch.equal(r.weights.reshape(T, topk).cpu(), probs.gather(1, want))
+
+
 @pytest.mark.parametrize("E,topk,n_group,topk_group,sigmoid", [(256, 8, 8, 4, True), (64, 6, 8, 3, False), (160, 6, 1, 1, False), (256, 8, 1, 1, True),
                                                                  (96, 4, 4, 2, True), (33, 5, 1, 1, False)])
 def test_deepseek_router_every_branch(cuda, oracle, E, topk, n_group, topk_group, sigmoid):
