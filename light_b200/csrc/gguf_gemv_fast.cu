@@ -94,22 +94,75 @@ __device__ __forceinline__ float stage_block(const float4 (&xv)[2], uint32_t sla
   return up;
 }
 
+// ---- the activations as whole numbers.  A block's 256 values become 31-bit fixed point (rounded at 2^-30 of the power of two above
+// the block's largest) and are cut into four signed bytes, the LIMBS: X = l0 + 256 l1 + 65536 l2 + 2^24 l3, limb j of element e at
+// plane j, byte e.  mma.m16n8k32 then multiplies the weights' integer codes, four to a register as they come out of a LOP3, with the
+// limbs, EXACTLY, and its eight columns are the four limbs of two sub-blocks: B is block diagonal, k slots 0..15 (registers a0, a1
+// and b0) belong to sub-block A and columns 0..3, slots 16..31 (a2, a3, b1) to sub-block B and columns 4..7.  Lane (g, t) of the
+// result holds rows g and g + 8 of limbs 2 (t & 1) and 2 (t & 1) + 1 of sub-block A (t < 2) or B, and V = D[c] + 256 D[c + 1] is still
+// a whole number below 2^31.  Against f16 codes and x as f16 hi + lo: half the MMAs, no offset to take off again, two to three
+// instructions per four weights instead of seven, and no x below 2^-24 is lost.
+constexpr int LIMB_PLANE = 264;                // bytes per plane: 256 and a pad that spreads the planes over the banks
+constexpr int LIMB_BYTES = 4 * LIMB_PLANE;
+
+__device__ __forceinline__ void imma16832_u8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// four 8 x 16-byte matrices: lane (g, t) gets bytes 4t .. 4t+3 of row g of each; lane l gives the address of row l & 7 of matrix l >> 3
+__device__ __forceinline__ uint4 ldmatrix4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(addr), "r"(v)); }
+// byte k of w as 2^23 + byte: an f32 whose mantissa is the byte.  sel = limb_sel(k).
+__device__ __forceinline__ uint32_t limb_sel(int k) { return 0x7440u + (uint32_t)k; }
+__device__ __forceinline__ float byte_2p23(uint32_t w, uint32_t sel) { return __uint_as_float(__byte_perm(w, 0x4B000000u, sel)); }
+// what the result of lane t counts in, limb pair and the 16 of a code taken from the high nibble in place
+__device__ __forceinline__ float limb_weight(int t, bool high_nibbles_in_place) {
+  return (t & 1 ? 65536.f : 1.f) * (t >= 2 && high_nibbles_in_place ? 0.0625f : 1.f);
+}
+
+// One block (two float4 per lane: elements 4 lane .. and 128 + 4 lane ..) into limbs at `slab`; xs = the values in fixed point, as
+// f32 before rounding.  Returns the power of two they count in (NaN for a block with an infinity or a NaN: the row's result is NaN).
+__device__ __forceinline__ float stage_limbs(const float4 (&xv)[2], uint32_t slab, int lane, float (&xs)[2][4]) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    m = max(m, __float_as_uint(xv[i].x) & 0x7fffffffu);
+    m = max(m, __float_as_uint(xv[i].y) & 0x7fffffffu);
+    m = max(m, __float_as_uint(xv[i].z) & 0x7fffffffu);
+    m = max(m, __float_as_uint(xv[i].w) & 0x7fffffffu);
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  const int s = min(156 - (int)(m >> 23), 126);  // |x| 2^s < 2^30
+  const float scale = __uint_as_float((uint32_t)(127 + s) << 23), up = m >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : __uint_as_float((uint32_t)(127 - s) << 23);
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    xs[i][0] = xv[i].x * scale, xs[i][1] = xv[i].y * scale, xs[i][2] = xv[i].z * scale, xs[i][3] = xv[i].w * scale;
+    uint32_t y[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) y[j] = ((uint32_t)__float2int_rn(xs[i][j]) + 0x808080u) ^ 0x808080u;  // the bytes are now the signed limbs
+    const uint32_t lo01 = __byte_perm(y[0], y[1], 0x5140), lo23 = __byte_perm(y[2], y[3], 0x5140);
+    const uint32_t hi01 = __byte_perm(y[0], y[1], 0x7362), hi23 = __byte_perm(y[2], y[3], 0x7362);
+    const uint32_t a = slab + i * 128 + lane * 4;
+    sts32(a, __byte_perm(lo01, lo23, 0x5410));
+    sts32(a + LIMB_PLANE, __byte_perm(lo01, lo23, 0x7632));
+    sts32(a + 2 * LIMB_PLANE, __byte_perm(hi01, hi23, 0x5410));
+    sts32(a + 3 * LIMB_PLANE, __byte_perm(hi01, hi23, 0x7632));
+  }
+  return up;
+}
+
 // ------------------------------------------------------------------------------------ Q4_K
 //
 // Block (144 B): [f16 d | f16 dmin | scales[12] | qs[128]]; byte qs[32p + l] holds element
 // 64p + l (low nibble, sub-block 2p) and 64p + 32 + l (high nibble, sub-block 2p+1).
-// Lane (g, t) loads the 32 qs bytes of pair p = t of rows g and g+8 (two 16-byte loads each)
-// and the 16-byte header of both rows.  Code word i (bytes 4i..4i+3) feeds two MMAs:
-//   even sub-block 2t:   a0 = codes(b0.lo, b2.lo)  a2 = codes(b1.lo, b3.lo)  (k slots 2t,2t+1 | 2t+8,2t+9)
-//   odd  sub-block 2t+1: the same with the high nibbles.
-// All four come out as f16 (64 + code): (word >> {-4, 4, 0, 8}) & 0x00F000F0 | 0x54005400.
-// The B lane (col c, tid) is non-zero only when c == 2*tid (even MMA) or c == 2*tid+1 (odd MMA);
-// all other lanes read a page of zeros.
-
-struct Q4KTile {
-  uint4 h0, h1, qa0, qa1, qb0, qb1;  // headers of rows g, g+8; the 32 code bytes of pair t of each
-};
-
+// ldmatrix gives lane (g, t) bytes 4t .. 4t+3 of each 16-byte quarter of a row's codes.  The low nibbles of such a word, as bytes,
+// are four k slots of the even sub-block (A), the high nibbles left in place, 16 times the code, four of the odd one (B).
 
 // ---- row-split execution over several GPUs, with the exchange inside the matmul launches.
 // A rank computes rows [rank n, (rank + 1) n) of an output of `world` n rows.  Instead of a gather
@@ -187,7 +240,7 @@ __device__ __forceinline__ float gate_act(float v, int act) {
 
 constexpr int Q4K_TILE_BYTES = ROWS * 144;  // one K block of 16 rows, dense in shared memory
 constexpr int GROUP = 4;                    // row tiles whose partial sums a CTA holds at a time
-constexpr int Q4K_SLAB = Slab<32>::BYTES + 16;  // a block's activations + its prescale factor
+constexpr int Q4K_SX = LIMB_BYTES, Q4K_UP = Q4K_SX + 32, Q4K_SLAB = Q4K_UP + 8;  // a block's limbs, eight sub-block sums, scale
 
 // One CTA per SM slot walks a contiguous range of row tiles (a balanced share of N/16), GROUP tiles
 // at a time; its warps take the K blocks round-robin and meet once per group to add up their parts.
@@ -216,37 +269,27 @@ struct NormArgs {
   float eps;
 };
 
-template <int S, int MINB, bool TP, bool NORM = false>
-__global__ void __launch_bounds__(WARPS * 32, MINB) q4k_gemv_mma_kernel(const float *__restrict__ x,
+template <int S, bool TP, bool NORM = false>
+__global__ void __launch_bounds__(WARPS * 32, 2) q4k_gemv_mma_kernel(const float *__restrict__ x,
                                                                        const __grid_constant__ MultiArgs a,
                                                                        const __grid_constant__ TpArgs tp,
                                                                        const __grid_constant__ NormArgs nrm, int tiles, int K) {
   __shared__ float nrm_part[WARPS];
-  using SL = Slab<32>;
   extern __shared__ __align__(16) unsigned char dyn[];  // [ring: WARPS x S tiles][slabs: K/256]
-  __shared__ __align__(16) unsigned char zero[SL::ZERO_BYTES];
   __shared__ __align__(16) float2 red[2][WARPS * GROUP * 32];  // by group parity
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int nb = K >> 8;
   const uint32_t row_bytes = (uint32_t)nb * 144u;
-  for (int i = threadIdx.x; i < SL::ZERO_BYTES / 4; i += WARPS * 32) reinterpret_cast<uint32_t *>(zero)[i] = 0u;
 
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(dyn) + warp * (S * Q4K_TILE_BYTES);
   const uint32_t slabs = (uint32_t)__cvta_generic_to_shared(dyn) + WARPS * S * Q4K_TILE_BYTES;
-  const uint32_t szero = (uint32_t)__cvta_generic_to_shared(zero);
   const uint32_t red_lane = (uint32_t)__cvta_generic_to_shared(&red[0][warp * GROUP * 32 + lane]);
   constexpr uint32_t RED_PARITY = WARPS * GROUP * 32 * 8;
-  // B addresses inside a slab.  The even MMA works on sub-block 2t of A-lane t: its column 2t
-  // carries the hi half of x and the otherwise unused column 2t+1 the lo half, so one MMA does
-  // both.  The odd MMA (sub-block 2t+1) has hi in column 2t+1 and lo in column 2t.  Every other
-  // column reads zeros.
-  const bool mine = (g >> 1) == t;
-  const uint32_t pe_off = (2 * t) * SL::SUB_BYTES + ((g & 1) ? SL::LO_OFF : 0);
-  const uint32_t po_off = (2 * t + 1) * SL::SUB_BYTES + ((g & 1) ? 0 : SL::LO_OFF);
-  const bool hdr_hi = t >= 2;
-  const int hdr_sh = (t & 1) * 16;
-  const uint32_t mask = 0x00F000F0u, magic = 0x54005400u;  // f16 (64 + nibble)
+  const uint32_t b_off = (g & 3) * LIMB_PLANE + 32 * (g >> 2) + 4 * t;  // limb g & 3 of the even (g < 4) or odd sub-block of a pair
+  const uint32_t m_off = ((lane & 7) + 8 * ((lane >> 3) & 1)) * 144 + 16 + 16 * (lane >> 4);  // ldmatrix row of this lane
+  const uint32_t sc_sel = limb_sel(t >> 1), mn_sel = limb_sel(2 * (t & 1));
+  const float lane_w = limb_weight(t, true);
 
   // this CTA's share [t0, t1) of the tile list (whole gate/up pairs when act != 0)
   const int unit = a.act ? 2 : 1, lt = tiles / unit;
@@ -260,7 +303,6 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) q4k_gemv_mma_kernel(const fl
     const uint32_t c = lane + 32 * i, row = c / 9u;
     soff[i] = row * row_bytes + (c - 9u * row) * 16u;
   }
-  const uint32_t ld_off = g * 144u + 32u * t;
   // The requests run S units ahead of the arithmetic; both walk (group, block, tile) in this order.
   int i_gt = t0, i_gs = min(GROUP, t1 - t0), i_b = warp, i_rt = 0, i_slot = 0;
   auto issue = [&]() {  // always closes a commit group, so that group counts stay uniform
@@ -316,8 +358,15 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) q4k_gemv_mma_kernel(const fl
       }
     }
     const uint32_t slab = slabs + b * Q4K_SLAB;
-    const float up = stage_block<32>(xv, slab, lane);
-    if (lane == 0) asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(slab + SL::BYTES), "f"(up));
+    float xs[2][4];
+    const float up = stage_limbs(xv, slab, lane, xs);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {  // eight lanes per sub-block
+      float v = (xs[i][0] + xs[i][1]) + (xs[i][2] + xs[i][3]);
+      v += __shfl_xor_sync(0xffffffffu, v, 1), v += __shfl_xor_sync(0xffffffffu, v, 2), v += __shfl_xor_sync(0xffffffffu, v, 4);
+      if ((lane & 7) == 0) sts32(slab + Q4K_SX + (4 * i + (lane >> 3)) * 4, __float_as_uint(v));
+    }
+    if (lane == 0) sts32(slab + Q4K_UP, __float_as_uint(up));
   }
   if constexpr (NORM) {
     nrm_ss = warp_sum(nrm_ss);
@@ -337,45 +386,47 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) q4k_gemv_mma_kernel(const fl
     const uint32_t red_g = red_lane + parity * RED_PARITY;
     for (int b = warp; b < nb; b += WARPS) {
       const uint32_t slab = slabs + b * Q4K_SLAB;
-      const uint32_t pe = mine ? slab + pe_off : szero, po = mine ? slab + po_off : szero;
-      float2 sx;
-      float up;
-      asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];\n" : "=f"(sx.x), "=f"(sx.y) : "r"(slab + SL::SX_OFF + 8 * t));
-      asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(up) : "r"(slab + SL::BYTES));
+      uint32_t bl[4][2];  // B of pair p, half h: in b0 for the even sub-block's columns, in b1 for the odd one's
+#pragma unroll
+      for (int p = 0; p < 4; p++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) bl[p][h] = lds32(slab + b_off + 64 * p + 16 * h);
+      const uint2 sx = lds64(slab + Q4K_SX + 8 * t);
+      const float up = __uint_as_float(lds32(slab + Q4K_UP));
       for (int rt = 0; rt < gs; rt++) {
         cp_async_wait<S - 1>();  // this lane's chunks of the tile have landed ...
         __syncwarp();            // ... and so have the other lanes'
-        const uint32_t sb = ring + slot * Q4K_TILE_BYTES + ld_off;
+        const uint32_t sb = ring + slot * Q4K_TILE_BYTES;
         slot = (slot + 1) & (S - 1);
-        const uint4 h0 = lds128(sb - 32u * t), h1 = lds128(sb - 32u * t + 8 * 144);
-        const uint4 qa0 = lds128(sb + 16), qa1 = lds128(sb + 32);
-        const uint4 qb0 = lds128(sb + 8 * 144 + 16), qb1 = lds128(sb + 8 * 144 + 32);
+        const uint4 hd[2] = {lds128(sb + g * 144u), lds128(sb + g * 144u + 8 * 144)};
+        uint4 q[4];  // quarters 2p: rows g, g+8; 2p+1: rows g, g+8
+#pragma unroll
+        for (int p = 0; p < 4; p++) q[p] = ldmatrix4(sb + m_off + 32 * p);
         __syncwarp();  // the slot is free again
         issue();
-        float dsc[2][2], dmn[2][2];
-        q4k_scales(h0, hdr_hi, hdr_sh, dsc[0], dmn[0]);
-        q4k_scales(h1, hdr_hi, hdr_sh, dsc[1], dmn[1]);
-        float de[4] = {0.f, 0.f, 0.f, 0.f}, dq[4] = {0.f, 0.f, 0.f, 0.f};  // even / odd sub-block chains
-        const uint32_t qg[8] = {qa0.x, qa0.y, qa0.z, qa0.w, qa1.x, qa1.y, qa1.z, qa1.w};
-        const uint32_t qh[8] = {qb0.x, qb0.y, qb0.z, qb0.w, qb1.x, qb1.y, qb1.z, qb1.w};
+        int D[4][4];
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const uint32_t vg = qg[i], vh = qh[i];
-          const uint32_t e0 = and_or(vg << 4, mask, magic), e1 = and_or(vh << 4, mask, magic);
-          const uint32_t e2 = and_or(vg >> 4, mask, magic), e3 = and_or(vh >> 4, mask, magic);
-          const uint32_t o0 = and_or(vg, mask, magic), o1 = and_or(vh, mask, magic);
-          const uint32_t o2 = and_or(vg >> 8, mask, magic), o3 = and_or(vh >> 8, mask, magic);
-          const uint2 be = lds64(pe + i * 8), bo = lds64(po + i * 8);
-          mma16816(de, e0, e1, e2, e3, be.x, be.y);
-          mma16816(dq, o0, o1, o2, o3, bo.x, bo.y);
+        for (int p = 0; p < 4; p++) {
+          D[p][0] = D[p][1] = D[p][2] = D[p][3] = 0;
+          const uint32_t lo = 0x0F0F0F0Fu, hi = 0xF0F0F0F0u;
+          imma16832_u8(D[p], q[p].x & lo, q[p].y & lo, q[p].x & hi, q[p].y & hi, g < 4 ? bl[p][0] : 0u, g < 4 ? 0u : bl[p][0]);
+          imma16832_u8(D[p], q[p].z & lo, q[p].w & lo, q[p].z & hi, q[p].w & hi, g < 4 ? bl[p][1] : 0u, g < 4 ? 0u : bl[p][1]);
         }
-        // lane (g, t): de[0] + de[1] = row g, sub-block 2t (hi + lo parts of x); dq[0] + dq[1] =
-        // row g, sub-block 2t+1; [2], [3] the same for row g+8.
+        // row g + 8 r: sum over this lane's four sub-blocks 2p + (t >> 1) of d sc V, less dmin m Sx of sub-blocks 2t and 2t + 1
         float vr[2];
 #pragma unroll
         for (int r = 0; r < 2; r++) {
-          float v = dsc[r][0] * (de[2 * r] + de[2 * r + 1]) - (64.f * dsc[r][0] + dmn[r][0]) * sx.x;
-          v += dsc[r][1] * (dq[2 * r] + dq[2 * r + 1]) - (64.f * dsc[r][1] + dmn[r][1]) * sx.y;
+          const uint4 h = hd[r];
+          const float2 df = __half22float2(*reinterpret_cast<const __half2 *>(&h.x));  // (d, dmin)
+          const uint32_t sc_lo = h.y & 0x3F3F3F3Fu, sc_hi = (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);
+          const uint32_t mn = t >= 2 ? (((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u)) : (h.z & 0x3F3F3F3Fu);
+          const float d = df.x * lane_w, d23 = -8388608.f * d, m23 = -8388608.f * df.y;  // fma(2^23 + byte, d, -2^23 d) = byte d, rounded once
+          float v = 0.f;
+#pragma unroll
+          for (int p = 0; p < 4; p++)
+            v = fmaf(fmaf(byte_2p23(p < 2 ? sc_lo : sc_hi, sc_sel + 2 * (p & 1)), d, d23), (float)(D[p][2 * r] + 256 * D[p][2 * r + 1]), v);
+          v -= fmaf(byte_2p23(mn, mn_sel), df.y, m23) * __uint_as_float(sx.x);
+          v -= fmaf(byte_2p23(mn, mn_sel + 1), df.y, m23) * __uint_as_float(sx.y);
           vr[r] = v * up;
         }
         // the warp's first block of a group overwrites what an earlier group left behind
@@ -1862,26 +1913,25 @@ int launch_pdl(void (*kern)(Args...), unsigned grid, size_t dyn_smem, cudaStream
 
 #define g_sms (sm_count())  // SMs of the calling thread's current device (every entry point binds it first)
 int g_waves = 2;       // LIGHT_B200_GEMV_WAVES: CTAs per SM of the persistent kernels' grids (1 or 2)
-int g_q4k_stages = 4;  // LIGHT_B200_Q4K_STAGES: ring depth (2 or 4)
-constexpr size_t MAX_DYN_SMEM = 96 * 1024;  // keeps two launches resident per SM
+int g_q4k_stages = 4;  // LIGHT_B200_Q4K_STAGES: deepest ring (2 or 4)
+constexpr size_t MAX_DYN_SMEM = 96 * 1024;   // leaves room for two CTAs per SM
+constexpr size_t MOST_DYN_SMEM = 200 * 1024;  // one CTA per SM
 
 }  // namespace
 
 int gguf_gemv_fast_init(int device) {
   if (const char *e = getenv("LIGHT_B200_GEMV_WAVES")) g_waves = atoi(e) == 1 ? 1 : 2;
   if (const char *e = getenv("LIGHT_B200_Q4K_STAGES")) g_q4k_stages = atoi(e) == 2 ? 2 : 4;
-  cudaError_t err = cudaFuncSetAttribute(q4k_gemv_mma_kernel<4, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(q4k_gemv_mma_kernel<2, 3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM);
+  cudaError_t err = cudaSuccess;
+  auto most = [&](auto kern) { if (err == cudaSuccess) err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST_DYN_SMEM); };
+  most(q4k_gemv_mma_kernel<4, false>), most(q4k_gemv_mma_kernel<2, false>);
+  most(q4k_gemv_mma_kernel<4, true>), most(q4k_gemv_mma_kernel<2, true>);
+  most(q4k_gemv_mma_kernel<4, false, true>), most(q4k_gemv_mma_kernel<2, false, true>);
   if (err == cudaSuccess)
     err = cudaFuncSetAttribute(q6k_gemv_mma_kernel<Q6K_STAGES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                WARPS * Q6K_STAGES * Q6K_TILE_BYTES);
   if (err == cudaSuccess)
     err = cudaFuncSetAttribute(q80_gemv_mma_kernel<Q80_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, WARPS * Q80_STAGES * Q80_TILE_BYTES);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(q4k_gemv_mma_kernel<4, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM);
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute(q4k_gemv_mma_kernel<4, 2, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_DYN_SMEM);
   if (err == cudaSuccess)
     err = cudaFuncSetAttribute(q6k_gemv_mma_kernel<Q6K_STAGES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                WARPS * Q6K_STAGES * Q6K_TILE_BYTES);
@@ -1897,15 +1947,18 @@ int gguf_gemv_fast_init(int device) {
 // path does not apply, < 0 or a CUDA code on error.
 static const NormArgs NO_NORM = {};
 static int q4k_launch(const float *x, const MultiArgs &a, const TpArgs &tp, int tiles, int K, cudaStream_t st, const NormArgs &nrm = NO_NORM) {
-  const size_t dyn = (size_t)WARPS * (tp.step || nrm.weight ? 4 : g_q4k_stages) * Q4K_TILE_BYTES + (size_t)(K >> 8) * Q4K_SLAB;
-  if (dyn > MAX_DYN_SMEM) return 0;  // very long rows: the activations do not fit beside the rings
-  const int lt = a.act ? tiles / 2 : tiles;
-  const int per_sm = (g_q4k_stages == 2 && !tp.step && !nrm.weight) ? 3 : g_waves;  // the 2-deep ring leaves room for three CTAs per SM
+  // The row's activations lie beside the rings: with four tiles per warp two CTAs fit an SM up to K = 5376, with two up to 14336 (the
+  // 74 KB in flight still cover the latency); longer rows take the deep ring and an SM to themselves, up to K = 30208.
+  const size_t slabs = (size_t)(K >> 8) * Q4K_SLAB, deep = (size_t)WARPS * 4 * Q4K_TILE_BYTES + slabs, flat = (size_t)WARPS * 2 * Q4K_TILE_BYTES + slabs;
+  const bool two = (g_q4k_stages == 2 || deep > MAX_DYN_SMEM) && flat <= MAX_DYN_SMEM;
+  const size_t dyn = two ? flat : deep;
+  if (dyn > MOST_DYN_SMEM) return 0;
+  const int lt = a.act ? tiles / 2 : tiles, per_sm = dyn > MAX_DYN_SMEM ? 1 : g_waves;
   const unsigned grid = (unsigned)(lt < g_sms * per_sm ? lt : g_sms * per_sm);
-  int rc = nrm.weight         ? launch_pdl(q4k_gemv_mma_kernel<4, 2, false, true>, grid, dyn, st, x, a, tp, nrm, tiles, K)
-           : tp.step           ? launch_pdl(q4k_gemv_mma_kernel<4, 2, true>, grid, dyn, st, x, a, tp, nrm, tiles, K)
-           : g_q4k_stages == 2 ? launch_pdl(q4k_gemv_mma_kernel<2, 3, false>, grid, dyn, st, x, a, tp, nrm, tiles, K)
-                               : launch_pdl(q4k_gemv_mma_kernel<4, 2, false>, grid, dyn, st, x, a, tp, nrm, tiles, K);
+  auto go = [&](auto kern) { return launch_pdl(kern, grid, dyn, st, x, a, tp, nrm, tiles, K); };
+  int rc = nrm.weight ? (two ? go(q4k_gemv_mma_kernel<2, false, true>) : go(q4k_gemv_mma_kernel<4, false, true>))
+           : tp.step  ? (two ? go(q4k_gemv_mma_kernel<2, true>) : go(q4k_gemv_mma_kernel<4, true>))
+                      : (two ? go(q4k_gemv_mma_kernel<2, false>) : go(q4k_gemv_mma_kernel<4, false>));
   if (rc) return rc;
   rc = launched("matmul_q (decode)");
   return rc ? rc : 1;
