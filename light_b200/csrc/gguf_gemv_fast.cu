@@ -906,9 +906,9 @@ __global__ void __launch_bounds__(DT_THREADS, 2) q4k_decode_tile_kernel(const fl
 // and bits 2q..2q+1 of qh[32h + l]; its sub-block of 16 is s = e / 16 = 8h + 2q + l/16.
 // For each (h, u = l/16), lane (g, t) takes l = 16u + 4t .. +3 of rows g and g+8: one word of
 // ql[64h + l], one of ql[64h + 32 + l] and one of qh[32h + l] -- every byte of the block is
-// read by exactly one lane.  From the three words come the four
-// groups' 6-bit codes as bytes, then f16x2 (1024 + code) with PRMT, and group q feeds ONE MMA
-// whose 16 k slots are exactly sub-block 8h + 2q + u, live column 2q + u.
+// read by exactly one lane.  From the three words come the four groups' 6-bit codes (code + 32) as bytes, and two integer
+// MMAs against the limbs of x: groups 0 and 2 (sub-blocks 8h + u and 8h + 4 + u, out of the same word), then 1 and 3.  The int8
+// scales multiply the whole-number results, and the 32 comes off in the accumulator's start, -32 times the limbs' sums.
 
 // The tiles travel through a per-warp ring of shared memory like the Q4_K ones.  A 16-byte
 // asynchronous copy keeps the byte offset inside its 16-byte granule, and a 210-byte block starts
@@ -920,6 +920,7 @@ __global__ void __launch_bounds__(DT_THREADS, 2) q4k_decode_tile_kernel(const fl
 constexpr int Q6K_PITCH = 240;
 constexpr int Q6K_TILE_BYTES = ROWS * Q6K_PITCH;
 constexpr int Q6K_STAGES = 2;
+constexpr int Q6K_SX = LIMB_BYTES, Q6K_SLAB = Q6K_SX + 16 * 16;  // a block's limbs, and -32 x the four limb sums of each sub-block
 
 __device__ __forceinline__ uint32_t lds16(uint32_t addr) {
   uint16_t v;
@@ -938,33 +939,22 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float
                                                                     const uint8_t *__restrict__ w,
                                                                     float *__restrict__ out, const __grid_constant__ TpArgs tp,
                                                                     int N, int K) {
-  using SL = Slab<16>;
   extern __shared__ __align__(16) unsigned char dyn[];  // ring: WARPS x S tiles
-  __shared__ __align__(16) unsigned char slabs[WARPS][SL::BYTES];
-  __shared__ __align__(16) unsigned char zero[SL::ZERO_BYTES];
+  __shared__ __align__(16) unsigned char slabs[WARPS][Q6K_SLAB];
   __shared__ __align__(16) float2 red[2][WARPS * GROUP * 32];  // by group parity
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int nb = K >> 8;
   const uint32_t row_bytes = (uint32_t)nb * 210u;  // a multiple of 4 (nb is even: checked by the launcher)
   const uint8_t *w_end = w + (size_t)N * row_bytes;
-  for (int i = threadIdx.x; i < SL::ZERO_BYTES / 4; i += WARPS * 32) reinterpret_cast<uint32_t *>(zero)[i] = 0u;
 
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(dyn) + warp * (S * Q6K_TILE_BYTES);
   const uint32_t slab = (uint32_t)__cvta_generic_to_shared(slabs[warp]);
-  const uint32_t szero = (uint32_t)__cvta_generic_to_shared(zero);
   const uint32_t red_lane = (uint32_t)__cvta_generic_to_shared(&red[0][warp * GROUP * 32 + lane]);
   constexpr uint32_t RED_PARITY = WARPS * GROUP * 32 * 8;
-  // B address of the MMA of (group q, u), which works on sub-block 8h + 2q + u: column 2q + u
-  // carries the hi half of x, the neighbouring column 2q + 1 - u (unused in this accumulator) the
-  // lo half; a lane of those columns reads elements 4t..4t+3 (h adds an immediate).  All other
-  // columns read zeros.
-  uint32_t pb[4][2];
-#pragma unroll
-  for (int q = 0; q < 4; q++)
-#pragma unroll
-    for (int u = 0; u < 2; u++)
-      pb[q][u] = (g >> 1) == q ? slab + (2 * q + u) * SL::SUB_BYTES + 8 * t + ((g & 1) == u ? 0 : SL::LO_OFF) : szero;
+  const uint32_t b_off = slab + (g & 3) * LIMB_PLANE + 64 * (g >> 2) + 4 * t;  // limb g & 3 of groups 0, 1 (g < 4) or 2, 3
+  const uint32_t c_off = slab + Q6K_SX + 64 * (t >> 1) + 8 * (t & 1);          // its sums: this lane's two limbs
+  const float lane_w = limb_weight(t, false);
   const uint32_t m0f = 0x0F0F0F0Fu;
 
   const int tiles = (N + ROWS - 1) / ROWS;
@@ -1031,10 +1021,10 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float
   };
   if (warp < nb) load_x(warp);
 
-  // one unit: rows g, g+8 of one tile x one K block, out of ring slot `sb`
-  auto unit = [&](auto odd_tag, uint32_t sb, uint32_t skew, const float2 (&sx)[2], float up, float (&vr)[2]) {
+  // One unit: rows g, g+8 of one tile x one K block, out of ring slot `sb`.  bl[h][u][i]: B of groups i and 2 + i.
+  auto unit = [&](auto odd_tag, uint32_t sb, uint32_t skew, const uint32_t (&bl)[2][2][2], float up, float (&vr)[2]) {
     constexpr bool ODD = decltype(odd_tag)::value;
-    uint32_t wa[2][4], wc[2][4], wh[2][4], scw[2];
+    uint32_t wa[2][4], wc[2][4], wh[2][4], scw[2][2];
     float dd[2];
 #pragma unroll
     for (int r = 0; r < 2; r++) {
@@ -1046,47 +1036,38 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float
         wc[r][hu] = lds32_skew<ODD>(blk + 4 * (16 * h + 8 + 4 * u + t));
         wh[r][hu] = lds32_skew<ODD>(blk + 4 * (32 + 8 * h + 4 * u + t));
       }
-      scw[r] = lds16(blk + 192 + 2 * t) | (lds16(blk + 200 + 2 * t) << 16);  // scales 2t, 2t+1 | 8+2t, 8+2t+1
+      scw[r][0] = lds32_skew<ODD>(blk + 192 + 4 * (t >> 1)), scw[r][1] = lds32_skew<ODD>(blk + 200 + 4 * (t >> 1));  // scales of this lane's eight
       dd[r] = f16_bits_to_f32((uint16_t)lds16(blk + 208));
     }
     __syncwarp();  // the slot is free again
     issue();
-    vr[0] = vr[1] = 0.f;
+    int acc[2][2] = {};  // [row][limb]: sum over sub-blocks of scale x (code - 32) . limb, below 2^28
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};  // u = 0 / u = 1 chains
+    for (int h = 0; h < 2; h++)
 #pragma unroll
       for (int u = 0; u < 2; u++) {
         const int hu = 2 * h + u;
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int i = 0; i < 2; i++) {
           uint32_t a[4];
 #pragma unroll
           for (int r = 0; r < 2; r++) {
-            const uint32_t lo4 = (q & 1) ? wc[r][hu] : wa[r][hu];
-            const uint32_t nib = (q >> 1) ? (lo4 >> 4) : lo4;
-            const uint32_t hi2 = q == 0 ? (wh[r][hu] << 4) : q == 1 ? (wh[r][hu] << 2) : q == 2 ? wh[r][hu] : (wh[r][hu] >> 2);
-            const uint32_t v = and_or(nib, m0f, hi2 & 0x30303030u);
-            a[r] = __byte_perm(v, 0x64646464u, 0x4240);      // f16x2 (1024 + b0, 1024 + b2)
-            a[2 + r] = __byte_perm(v, 0x64646464u, 0x4341);  // f16x2 (1024 + b1, 1024 + b3)
+            const uint32_t q4 = i ? wc[r][hu] : wa[r][hu], hq = wh[r][hu];
+            a[r] = and_or(q4, m0f, (i ? hq << 2 : hq << 4) & 0x30303030u);           // group i
+            a[2 + r] = and_or(q4 >> 4, m0f, (i ? hq >> 2 : hq) & 0x30303030u);       // group 2 + i
           }
-          const uint2 bh = lds64(pb[q][u] + h * (8 * SL::SUB_BYTES));
-          if (u == 0)
-            mma16816(d0, a[0], a[1], a[2], a[3], bh.x, bh.y);
-          else
-            mma16816(d1, a[0], a[1], a[2], a[3], bh.x, bh.y);
+          const uint2 c = lds64(c_off + 128 * h + 16 * u + 32 * i);
+          int D[4] = {(int)c.x, (int)c.y, (int)c.x, (int)c.y};
+          imma16832_u8(D, a[0], a[1], a[2], a[3], g < 4 ? bl[h][u][i] : 0u, g < 4 ? 0u : bl[h][u][i]);
+#pragma unroll
+          for (int r = 0; r < 2; r++) {
+            const int sc = (int)(int8_t)(scw[r][h] >> (8 * (2 * i + u)));
+            acc[r][0] += sc * D[2 * r], acc[r][1] += sc * D[2 * r + 1];
+          }
         }
       }
-      // lane (g, t): d0[0] + d0[1] = row g, sub-block 8h+2t; d1[0] + d1[1] = row g, sub-block 8h+2t+1;
-      // [2], [3] the same for row g+8
 #pragma unroll
-      for (int r = 0; r < 2; r++) {
-        const float s0 = dd[r] * (float)(int8_t)((scw[r] >> (16 * h)) & 0xff);
-        const float s1 = dd[r] * (float)(int8_t)((scw[r] >> (16 * h + 8)) & 0xff);
-        vr[r] += s0 * (d0[2 * r] + d0[2 * r + 1] - 1056.f * sx[h].x) + s1 * (d1[2 * r] + d1[2 * r + 1] - 1056.f * sx[h].y);
-      }
-    }
-    vr[0] *= up, vr[1] *= up;
+    for (int r = 0; r < 2; r++) vr[r] = dd[r] * lane_w * fmaf(256.f, (float)acc[r][1], (float)acc[r][0]) * up;
   };
 
   int slot = 0, parity = 0;
@@ -1101,11 +1082,27 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float
         if (b + WARPS < nb || gt + GROUP < t1) load_x(bn);
       }
       __syncwarp();  // every lane is done reading the previous block's slab
-      const float up = stage_block<16>(xv, slab, lane);
+      float xs[2][4];
+      const float up = stage_limbs(xv, slab, lane, xs);
       __syncwarp();
-      float2 sx[2];
-      asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];\n" : "=f"(sx[0].x), "=f"(sx[0].y) : "r"(slab + SL::SX_OFF + 8 * t));
-      asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];\n" : "=f"(sx[1].x), "=f"(sx[1].y) : "r"(slab + SL::SX_OFF + 32 + 8 * t));
+      {  // -32 times the sum of each limb over each sub-block: lane l adds up limbs 2 (l & 1), 2 (l & 1) + 1 of sub-block l >> 1
+        int sum[2];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          sum[j] = 0;
+#pragma unroll
+          for (int i = 0; i < 4; i++) sum[j] = __dp4a((int)lds32(slab + (2 * (lane & 1) + j) * LIMB_PLANE + 16 * (lane >> 1) + 4 * i), 0x01010101, sum[j]);
+        }
+        sts64(slab + Q6K_SX + 16 * (lane >> 1) + 8 * (lane & 1), (uint32_t)(-32 * sum[0]), (uint32_t)(-32 * sum[1]));
+      }
+      __syncwarp();
+      uint32_t bl[2][2][2];
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+#pragma unroll
+          for (int i = 0; i < 2; i++) bl[h][u][i] = lds32(b_off + 128 * h + 32 * i + 16 * u);
       for (int rt = 0; rt < gs; rt++) {
         cp_async_wait<S - 1>();  // this lane's granules of the tile have landed ...
         __syncwarp();            // ... and so have the other lanes'
@@ -1115,9 +1112,9 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float
         const uint32_t skew = ((uint32_t)r0 * row_bytes + (uint32_t)b * 210u + (uint32_t)g * row_bytes) & 15u;
         float vr[2];
         if (b & 1)
-          unit(std::true_type{}, sb, skew, sx, up, vr);
+          unit(std::true_type{}, sb, skew, bl, up, vr);
         else
-          unit(std::false_type{}, sb, skew, sx, up, vr);
+          unit(std::false_type{}, sb, skew, bl, up, vr);
         // the warp's first block of a group overwrites what an earlier group left behind
         const uint32_t ra = red_g + rt * (32 * 8);
         float2 o = make_float2(0.f, 0.f);

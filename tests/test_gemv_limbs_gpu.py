@@ -1,0 +1,44 @@
+"""One activation row in fixed-point limbs (gguf_gemv_fast.cu) against an f64 product with the dequantized weights.
+
+Bound per output: the fixed point rounds an activation at 2^-30 of the power of two above its block's largest, so at most
+2^-30 max|x| sum|w|; scales, sums over lanes, warps and blocks are f32, fewer than 64 roundings of terms that together stay below
+four times sum|w x| (a Q4_K weight is a difference of two products): 2^-16 sum|w x|."""
+import pytest
+import torch
+
+from light_b200 import ops, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def check(y, x, W):
+    W, x = W.double(), x.double()
+    bound = 2.0**-30 * x.abs().amax() * W.abs().sum(1) + 2.0**-16 * (W.abs() @ x.abs().t()).squeeze(1)
+    assert ((y.double().squeeze(0) - W @ x.squeeze(0)).abs() <= bound).all()
+
+
+def gguf(seed, dt, n, k):
+    return ops.QTensor(synth.gaussian_weight(seed, dt, n, k, device="cuda").reshape(-1), dt, (n, k))
+
+
+# both sides of each change of ring depth (K = 5376 and 14336 with Q4_K), the shortest rows, rows that are no whole tile
+@pytest.mark.parametrize("fmt,n,k", [("Q4_K", 16, 256), ("Q4_K", 161, 5376), ("Q4_K", 161, 5632), ("Q4_K", 48, 14336), ("Q4_K", 48, 14592),
+                                     ("Q4_K", 5000, 4096), ("Q6_K", 16, 512), ("Q6_K", 161, 1536), ("Q6_K", 5000, 4096)])
+@pytest.mark.parametrize("kind", ["normal", "outlier", "tiny", "huge"])
+def test_one_row(cuda, fmt, n, k, kind):
+    x = torch.randn(1, k, generator=torch.Generator().manual_seed(n + k)).to(cuda)
+    if kind == "outlier":
+        x[0, 5] = 1000.0
+    x = x * {"tiny": 2.0**-90, "huge": 2.0**90}.get(kind, 1.0)
+    w = gguf(n + k, getattr(ops, fmt), n, k)
+    check(ops.MatMulQ(x, w), x, ops.Dequantize(w))
+
+
+@pytest.mark.parametrize("fmt", ["Q4_K", "Q6_K"])
+def test_a_nan_reaches_every_row(cuda, fmt):
+    x = torch.zeros(1, 1024, device=cuda)
+    w = gguf(3, getattr(ops, fmt), 40, 1024)
+    assert (ops.MatMulQ(x, w) == 0).all()
+    for v in (float("nan"), float("inf")):
+        x[0, 700] = v
+        assert torch.isnan(ops.MatMulQ(x, w)).all()
