@@ -111,12 +111,19 @@ __device__ __forceinline__ void imma16832_u8(int (&d)[4], uint32_t a0, uint32_t 
       : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ void imma16832_s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
 // four 8 x 16-byte matrices: lane (g, t) gets bytes 4t .. 4t+3 of row g of each; lane l gives the address of row l & 7 of matrix l >> 3
 __device__ __forceinline__ uint4 ldmatrix4(uint32_t addr) {
   uint4 v;
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
   return v;
 }
+__device__ __forceinline__ void sts16(uint32_t addr, uint32_t v) { asm volatile("st.shared.u16 [%0], %1;\n" ::"r"(addr), "h"((uint16_t)v)); }
 __device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(addr), "r"(v)); }
 // byte k of w as 2^23 + byte: an f32 whose mantissa is the byte.  sel = limb_sel(k).
 __device__ __forceinline__ uint32_t limb_sel(int k) { return 0x7440u + (uint32_t)k; }
@@ -126,8 +133,14 @@ __device__ __forceinline__ float limb_weight(int t, bool high_nibbles_in_place) 
   return (t & 1 ? 65536.f : 1.f) * (t >= 2 && high_nibbles_in_place ? 0.0625f : 1.f);
 }
 
+// Where a plane keeps element e: at byte e (PLAIN); WORD8: of each eight elements first the even-numbered, then the odd ones (the low
+// and the high nibbles of a code word); Q8: of each even 32-element block the elements 2 .. 29, then 0, 1, 30, 31 (the order of the
+// aligned words of a block that starts two bytes into one), odd blocks plainly.
+enum { LIMB_PLAIN, LIMB_WORD8, LIMB_Q8 };
+
 // One block (two float4 per lane: elements 4 lane .. and 128 + 4 lane ..) into limbs at `slab`; xs = the values in fixed point, as
 // f32 before rounding.  Returns the power of two they count in (NaN for a block with an infinity or a NaN: the row's result is NaN).
+template <int ORDER = LIMB_PLAIN>
 __device__ __forceinline__ float stage_limbs(const float4 (&xv)[2], uint32_t slab, int lane, float (&xs)[2][4]) {
   uint32_t m = 0;
 #pragma unroll
@@ -146,13 +159,25 @@ __device__ __forceinline__ float stage_limbs(const float4 (&xv)[2], uint32_t sla
     uint32_t y[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) y[j] = ((uint32_t)__float2int_rn(xs[i][j]) + 0x808080u) ^ 0x808080u;  // the bytes are now the signed limbs
+    if constexpr (ORDER == LIMB_WORD8) {
+      const uint32_t u = y[1];
+      y[1] = y[2], y[2] = u;
+    }
     const uint32_t lo01 = __byte_perm(y[0], y[1], 0x5140), lo23 = __byte_perm(y[2], y[3], 0x5140);
     const uint32_t hi01 = __byte_perm(y[0], y[1], 0x7362), hi23 = __byte_perm(y[2], y[3], 0x7362);
-    const uint32_t a = slab + i * 128 + lane * 4;
-    sts32(a, __byte_perm(lo01, lo23, 0x5410));
-    sts32(a + LIMB_PLANE, __byte_perm(lo01, lo23, 0x7632));
-    sts32(a + 2 * LIMB_PLANE, __byte_perm(hi01, hi23, 0x5410));
-    sts32(a + 3 * LIMB_PLANE, __byte_perm(hi01, hi23, 0x7632));
+    const uint32_t pl[4] = {__byte_perm(lo01, lo23, 0x5410), __byte_perm(lo01, lo23, 0x7632), __byte_perm(hi01, hi23, 0x5410), __byte_perm(hi01, hi23, 0x7632)};
+    const uint32_t a = slab + i * 128;
+    if constexpr (ORDER == LIMB_PLAIN) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) sts32(a + j * LIMB_PLANE + lane * 4, pl[j]);
+    } else {
+      const int c = 4 * (lane & 7), blk = 32 * (lane >> 3);  // Q8: four elements from c of 32-element block `blk`; blocks 0 and 2 are the even ones
+      const bool odd = (lane >> 3) & 1;
+      const uint32_t p0 = ORDER == LIMB_WORD8 ? 8 * (lane >> 1) + 2 * (lane & 1) : blk + (odd ? c : c == 0 ? 28 : c - 2);
+      const uint32_t p1 = ORDER == LIMB_WORD8 ? p0 + 4 : blk + (odd ? c + 2 : c == 28 ? 30 : c);
+#pragma unroll
+      for (int j = 0; j < 4; j++) sts16(a + j * LIMB_PLANE + p0, pl[j]), sts16(a + j * LIMB_PLANE + p1, pl[j] >> 16);
+    }
   }
   return up;
 }
@@ -1143,11 +1168,12 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float
 
 // ------------------------------------------------------------------------------------ Q8_0
 //
-// The Q6_K kernel's structure (per-warp ring of 16-row tiles, activations staged per run of 256 k with the
-// next run requested ahead, one MMA per 16-element sub-block with the hi and lo halves of x in
-// neighbouring columns) on 34-byte blocks: a run of 256 k is eight blocks = 272 bytes = 17 granules per
-// row, rows are whole granules (K % 256 == 0), and a 272-byte pitch puts rows g and lanes t on 32
-// different banks.  reference: matmul_q8_0_f32_mv, kernels/cuda/src/matmul_q.cu:58-431.
+// The Q6_K kernel's structure on 34-byte blocks of signed bytes, which are the MMA's operand as they lie in memory: a run of 256 k is
+// eight blocks = 272 bytes = 17 granules per row, rows are whole granules (K % 256 == 0), and a 272-byte pitch puts rows g and lanes t
+// on 32 different banks and the granules of a tile one behind the other.  Pairs of blocks are the sub-blocks A and B of two MMAs; their
+// f16 scales multiply V.  Loads from shared memory were the bound (49 % of the cycles with x as f16 hi + lo: codes, and sixteen B
+// fragments a tile); B now stays in registers.  28672 x 4096: 25.5 -> 22.5 us.  reference: matmul_q8_0_f32_mv,
+// kernels/cuda/src/matmul_q.cu:58-431.
 constexpr int Q80_PITCH = 272;
 constexpr int Q80_TILE_BYTES = ROWS * Q80_PITCH;
 constexpr int Q80_STAGES = 2;
@@ -1155,50 +1181,40 @@ constexpr int Q80_STAGES = 2;
 template <int S>
 __global__ void __launch_bounds__(WARPS * 32, 2) q80_gemv_mma_kernel(const float *__restrict__ x, const uint8_t *__restrict__ w,
                                                                     float *__restrict__ out, int N, int K) {
-  using SL = Slab<16>;
   extern __shared__ __align__(16) unsigned char dyn[];  // ring: WARPS x S tiles
-  __shared__ __align__(16) unsigned char slabs[WARPS][SL::BYTES];
-  __shared__ __align__(16) unsigned char zero[SL::ZERO_BYTES];
+  __shared__ __align__(16) unsigned char slabs[WARPS][LIMB_BYTES];
   __shared__ __align__(16) float2 red[2][WARPS * GROUP * 32];  // by group parity
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int nb = K >> 8;
   const uint32_t row_bytes = (uint32_t)nb * 272u;  // eight 34-byte blocks per 256 elements: rows are whole granules
-  for (int i = threadIdx.x; i < SL::ZERO_BYTES / 4; i += WARPS * 32) reinterpret_cast<uint32_t *>(zero)[i] = 0u;
 
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(dyn) + warp * (S * Q80_TILE_BYTES);
   const uint32_t slab = (uint32_t)__cvta_generic_to_shared(slabs[warp]);
-  const uint32_t szero = (uint32_t)__cvta_generic_to_shared(zero);
   const uint32_t red_lane = (uint32_t)__cvta_generic_to_shared(&red[0][warp * GROUP * 32 + lane]);
   constexpr uint32_t RED_PARITY = WARPS * GROUP * 32 * 8;
-  // B address of the MMA of (group q, u), which works on sub-block 8h + 2q + u: column 2q + u
-  // carries the hi half of x, the neighbouring column 2q + 1 - u (unused in this accumulator) the
-  // lo half; a lane of those columns reads elements 4t..4t+3 (h adds an immediate).  All other
-  // columns read zeros.
-  uint32_t pb[4][2];
-#pragma unroll
-  for (int q = 0; q < 4; q++)
-#pragma unroll
-    for (int u = 0; u < 2; u++)
-      pb[q][u] = (g >> 1) == q ? slab + (2 * q + u) * SL::SUB_BYTES + 8 * t + ((g & 1) == u ? 0 : SL::LO_OFF) : szero;
+  const uint32_t b_off = slab + (g & 3) * LIMB_PLANE + 32 * (g >> 2) + 4 * t;  // limb g & 3 of the even (g < 4) or odd block of a pair
+  const float lane_w = limb_weight(t, false);
 
   const int tiles = (N + ROWS - 1) / ROWS;
   const int t0 = (int)((uint32_t)tiles * blockIdx.x / gridDim.x), t1 = (int)((uint32_t)tiles * (blockIdx.x + 1) / gridDim.x);
 
-  // requests: lanes 0..15 / 16..31 copy granules 0..15 of rows 2i / 2i+1, i = 0..7; lanes 0 / 16 also the 17th
-  const uint32_t c_rsub = lane >> 4, c_piece = lane & 15;
+  // requests: a tile is 272 granules in shared order; lane l takes l, l + 32, ...
+  uint32_t soff[9];
+#pragma unroll
+  for (int i = 0; i < 9; i++) {
+    const uint32_t c = lane + 32 * i, row = c / 17u;
+    soff[i] = row * row_bytes + (c - 17u * row) * 16u;
+  }
   int i_gt = t0, i_gs = min(GROUP, t1 - t0), i_b = warp, i_rt = 0, i_slot = 0;
   auto issue = [&]() {  // always closes a commit group, so that group counts stay uniform
     if (i_gt < t1 && warp < nb) {
       const int r0 = min((i_gt + i_rt) * ROWS, N - ROWS);
-      const uint8_t *src = w + ((size_t)(r0 + c_rsub) * row_bytes + (uint32_t)i_b * 272u + c_piece * 16);
-      uint32_t dst = ring + i_slot * Q80_TILE_BYTES + c_rsub * Q80_PITCH + c_piece * 16;
+      const uint8_t *base = w + ((size_t)r0 * row_bytes + (uint32_t)i_b * 272u);
+      const uint32_t dst = ring + i_slot * Q80_TILE_BYTES + lane * 16;
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        cp_async16(dst, src);
-        if (c_piece == 0) cp_async16(dst + 256, src + 256);
-        src += 2 * row_bytes, dst += 2 * Q80_PITCH;
-      }
+      for (int i = 0; i < 8; i++) cp_async16(dst + i * 512, base + soff[i]);
+      if (lane < 16) cp_async16(dst + 4096, base + soff[8]);
       i_slot = (i_slot + 1) & (S - 1);
       if (++i_rt == i_gs) {
         i_rt = 0, i_b += WARPS;
@@ -1219,54 +1235,37 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q80_gemv_mma_kernel(const float
   };
   if (warp < nb) load_x(warp);
 
-  // One unit: rows g, g+8 of one tile x one run of 256 k (eight 34-byte blocks), out of ring slot `sb`.
-  // Sub-block s = 8h + 2q + u (16 codes) is half s & 1 of block s >> 1; lane t takes its word t.  Even
-  // blocks start 2 bytes into a word (34 j + 2), odd ones on a word boundary.  XOR 0x80 makes the codes
-  // unsigned and PRMT gives f16 (1024 + 128 + q): the MMA sums (1152 + q) x, and 1152 sum(x) comes off.
-  auto unit = [&](uint32_t sb, const float2 (&sx)[2], float up, float (&vr)[2]) {
-    uint32_t wq[2][16];
-    float dd[2][2];
+  // One unit: rows g, g+8 of one tile x one run of 256 k, out of ring slot `sb`.  bl[p][h]: B of blocks 2p, 2p + 1, half h.  Odd blocks
+  // have their codes on a word boundary; even ones start 2 bytes into a word, and lane t takes words 1 + t and 5 + t of nine, with the
+  // two half words at the ends for the missing eighth (LIMB_Q8 is that order).
+  const uint32_t w5 = t < 3 ? 4 * (5 + t) : 0, w5_sel = t < 3 ? 0x3210 : 0x5432;
+  auto unit = [&](uint32_t sb, const uint32_t (&bl)[4][2], float up, float (&vr)[2]) {
+    uint32_t ev[2][4][2], od[2][4][2];
+    float dd[2][4];
 #pragma unroll
     for (int r = 0; r < 2; r++) {
-      const uint32_t blk = sb + (g + 8 * r) * Q80_PITCH;
+      const uint32_t row = sb + (g + 8 * r) * Q80_PITCH;
 #pragma unroll
-      for (int s = 0; s < 16; s++) {
-        const uint32_t a = blk + 34 * (s >> 1) + 2 + 16 * (s & 1) + 4 * t;
-        wq[r][s] = (((s >> 1) & 1) ? lds32(a) : __funnelshift_r(lds32(a - 2), lds32(a + 2), 16)) ^ 0x80808080u;
+      for (int p = 0; p < 4; p++) {
+        const uint32_t blk = row + 68 * p;
+        ev[r][p][0] = lds32(blk + 4 + 4 * t);
+        ev[r][p][1] = __byte_perm(lds32(blk + w5), lds32(blk + 32), w5_sel);
+        od[r][p][0] = lds32(blk + 36 + 4 * t), od[r][p][1] = lds32(blk + 52 + 4 * t);
+        dd[r][p] = f16_bits_to_f32((uint16_t)lds16(blk + 34 * (t >> 1)));
       }
-      dd[r][0] = f16_bits_to_f32((uint16_t)lds16(blk + 34 * t)), dd[r][1] = f16_bits_to_f32((uint16_t)lds16(blk + 34 * (4 + t)));
     }
     __syncwarp();  // the slot is free again
     issue();
     vr[0] = vr[1] = 0.f;
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      float d0[4] = {0.f, 0.f, 0.f, 0.f}, d1[4] = {0.f, 0.f, 0.f, 0.f};  // u = 0 / u = 1 chains
+    for (int p = 0; p < 4; p++) {
+      int D[4] = {0, 0, 0, 0};
 #pragma unroll
-      for (int u = 0; u < 2; u++) {
+      for (int h = 0; h < 2; h++) imma16832_s8(D, ev[0][p][h], ev[1][p][h], od[0][p][h], od[1][p][h], g < 4 ? bl[p][h] : 0u, g < 4 ? 0u : bl[p][h]);
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-          const int s = 8 * h + 2 * q + u;
-          uint32_t a[4];
-#pragma unroll
-          for (int r = 0; r < 2; r++) {
-            a[r] = __byte_perm(wq[r][s], 0x64646464u, 0x4240);      // f16x2 (1024 + b0, 1024 + b2)
-            a[2 + r] = __byte_perm(wq[r][s], 0x64646464u, 0x4341);  // f16x2 (1024 + b1, 1024 + b3)
-          }
-          const uint2 bh = lds64(pb[q][u] + h * (8 * SL::SUB_BYTES));
-          if (u == 0)
-            mma16816(d0, a[0], a[1], a[2], a[3], bh.x, bh.y);
-          else
-            mma16816(d1, a[0], a[1], a[2], a[3], bh.x, bh.y);
-        }
-      }
-      // lane (g, t): d0[0] + d0[1] = row g, sub-block 8h+2t; d1[0] + d1[1] = row g, sub-block 8h+2t+1: the
-      // two halves of block 4h + t; [2], [3] the same for row g+8
-#pragma unroll
-      for (int r = 0; r < 2; r++)
-        vr[r] += dd[r][h] * ((d0[2 * r] + d0[2 * r + 1]) + (d1[2 * r] + d1[2 * r + 1]) - 1152.f * (sx[h].x + sx[h].y));
+      for (int r = 0; r < 2; r++) vr[r] = fmaf(dd[r][p], (float)(D[2 * r] + 256 * D[2 * r + 1]), vr[r]);
     }
-    vr[0] *= up, vr[1] *= up;
+    vr[0] *= lane_w * up, vr[1] *= lane_w * up;
   };
 
   int slot = 0, parity = 0;
@@ -1281,18 +1280,21 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q80_gemv_mma_kernel(const float
         if (b + WARPS < nb || gt + GROUP < t1) load_x(bn);
       }
       __syncwarp();  // every lane is done reading the previous block's slab
-      const float up = stage_block<16>(xv, slab, lane);
+      float xs[2][4];
+      const float up = stage_limbs<LIMB_Q8>(xv, slab, lane, xs);
       __syncwarp();
-      float2 sx[2];
-      asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];\n" : "=f"(sx[0].x), "=f"(sx[0].y) : "r"(slab + SL::SX_OFF + 8 * t));
-      asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];\n" : "=f"(sx[1].x), "=f"(sx[1].y) : "r"(slab + SL::SX_OFF + 32 + 8 * t));
+      uint32_t bl[4][2];
+#pragma unroll
+      for (int p = 0; p < 4; p++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) bl[p][h] = lds32(b_off + 64 * p + 16 * h);
       for (int rt = 0; rt < gs; rt++) {
         cp_async_wait<S - 1>();  // this lane's granules of the tile have landed ...
         __syncwarp();            // ... and so have the other lanes'
         const uint32_t sb = ring + slot * Q80_TILE_BYTES;
         slot = (slot + 1) & (S - 1);
         float vr[2];
-        unit(sb, sx, up, vr);
+        unit(sb, bl, up, vr);
         // the warp's first block of a group overwrites what an earlier group left behind
         const uint32_t ra = red_g + rt * (32 * 8);
         float2 o = make_float2(0.f, 0.f);
@@ -1502,81 +1504,35 @@ __global__ void __launch_bounds__(WARPS * 32, 2) fp8_gemv_mma_kernel(const XT *_
 // ------------------------------------------------------------------------------------ int4 (GPTQ / AWQ), one row of x
 //
 // The canonical 4-bit layout (codes u32 (N, K/8), nibble j of word c = element 8c + j; scales / zeros f32
-// (N, K/G)) through the Q4_K arithmetic: LOP3 turns nibble pairs into f16 (64 + code), the MMA columns are
-// sets of 32 elements that share a scale (here the even- and the odd-numbered elements of a lane's 64), and
-// acc += s (D - (64 + z) Sx).  Structure as the Q8_0 kernel (per-warp ring, activations staged per run of
-// 256 k, so any K fits); a tile row sits 16 bytes into a 144-byte slot, which keeps the Q4_K kernel's
-// conflict-free 16-byte loads.  Needs G % 64 == 0 and K % 256 == 0.  reference: int4_gemv_f32 / _bf16,
-// kernels/cuda/src/int4.cu:43-106.
+// (N, K/G)) through the Q4_K arithmetic: the low nibbles of a code word, as bytes, are four even-numbered elements (A), the high ones
+// left in place four odd-numbered ones (B), and the whole-number sums of 64 elements, which share a scale, meet in one lane of four:
+// acc += s (sum - z Sx).  Structure as the Q8_0 kernel (per-warp ring, activations staged per run of 256 k, so any K fits); a 144-byte
+// row pitch keeps ldmatrix on 32 banks.  28672 x 4096: 21.6 -> 16.5 us.  Needs G % 64 == 0 and K % 256 == 0.  reference:
+// int4_gemv_f32 / _bf16, kernels/cuda/src/int4.cu:43-106.
 constexpr int I4_PITCH = 144;
 constexpr int I4_TILE_BYTES = ROWS * I4_PITCH;
 constexpr int I4_STAGES = 4;
-
-// stage_block<32> for the int4 element order: lanes l, l^1 hold the eight elements of one code word; the even
-// lane assembles (x0, x4, x2, x6) for the even set, the odd lane (x1, x5, x3, x7) for the odd set.
-__device__ __forceinline__ float stage_block_int4(const float4 (&xv)[2], uint32_t slab, int lane) {
-  using S = Slab<32>;
-  uint32_t m = 0;
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    m = max(m, __float_as_uint(xv[i].x) & 0x7fffffffu);
-    m = max(m, __float_as_uint(xv[i].y) & 0x7fffffffu);
-    m = max(m, __float_as_uint(xv[i].z) & 0x7fffffffu);
-    m = max(m, __float_as_uint(xv[i].w) & 0x7fffffffu);
-  }
-  m = __reduce_max_sync(0xffffffffu, m);
-  int sh = (int)(m >> 23) - 127 - 14;
-  sh = sh < 0 ? 0 : (sh > 100 ? 100 : sh);
-  const float down = __uint_as_float((uint32_t)(127 - sh) << 23), up = __uint_as_float((uint32_t)(127 + sh) << 23);
-  const bool odd = lane & 1;
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    float4 v = xv[i];
-    if (sh) v.x *= down, v.y *= down, v.z *= down, v.w *= down;
-    // the even lane needs the partner's x and z, the odd lane the partner's y and w
-    const float ra = __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1), rb = __shfl_xor_sync(0xffffffffu, odd ? v.z : v.w, 1);
-    const float s0 = odd ? ra : v.x, s1 = odd ? v.y : ra, s2 = odd ? rb : v.z, s3 = odd ? v.w : rb;  // slots 0..3 of this word
-    __half2 h01 = __floats2half2_rn(s0, s1), h23 = __floats2half2_rn(s2, s3);
-    float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
-    __half2 l01 = __floats2half2_rn(s0 - f01.x, s1 - f01.y), l23 = __floats2half2_rn(s2 - f23.x, s3 - f23.y);
-    const int t = 2 * i + (lane >> 4), w = (lane >> 1) & 7, vs = 2 * t + (lane & 1);  // lane quarter, word, set
-    const uint32_t a = slab + vs * S::SUB_BYTES + w * 8;
-    sts64(a, *reinterpret_cast<uint32_t *>(&h01), *reinterpret_cast<uint32_t *>(&h23));
-    sts64(a + S::LO_OFF, *reinterpret_cast<uint32_t *>(&l01), *reinterpret_cast<uint32_t *>(&l23));
-    float s = (s0 + s1) + (s2 + s3);
-    s += __shfl_xor_sync(0xffffffffu, s, 2), s += __shfl_xor_sync(0xffffffffu, s, 4), s += __shfl_xor_sync(0xffffffffu, s, 8);
-    if (w == 0) asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(slab + S::SX_OFF + vs * 4), "f"(s));
-  }
-  return up;
-}
 
 template <int S, typename XT>
 __global__ void __launch_bounds__(WARPS * 32, 2) int4_gemv_mma_kernel(const XT *__restrict__ x, const uint8_t *__restrict__ w,
                                                                      const float *__restrict__ scales, const float *__restrict__ zeros,
                                                                      XT *__restrict__ out, int N, int K, int G) {
-  using SL = Slab<32>;
   extern __shared__ __align__(16) unsigned char dyn[];  // ring: WARPS x S tiles
-  __shared__ __align__(16) unsigned char slabs[WARPS][SL::BYTES];
-  __shared__ __align__(16) unsigned char zero[SL::ZERO_BYTES];
+  __shared__ __align__(16) unsigned char slabs[WARPS][LIMB_BYTES + 16];  // limbs, the sums of four sets of 64
   __shared__ __align__(16) float2 red[2][WARPS * GROUP * 32];  // by group parity
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int nb = K >> 8;
   const uint32_t row_bytes = (uint32_t)K >> 1;  // 128 bytes of codes per 256 elements
   const int ngrp = K / G;
-  for (int i = threadIdx.x; i < SL::ZERO_BYTES / 4; i += WARPS * 32) reinterpret_cast<uint32_t *>(zero)[i] = 0u;
 
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(dyn) + warp * (S * I4_TILE_BYTES);
   const uint32_t slab = (uint32_t)__cvta_generic_to_shared(slabs[warp]);
-  const uint32_t szero = (uint32_t)__cvta_generic_to_shared(zero);
   const uint32_t red_lane = (uint32_t)__cvta_generic_to_shared(&red[0][warp * GROUP * 32 + lane]);
   constexpr uint32_t RED_PARITY = WARPS * GROUP * 32 * 8;
-  // B addresses inside the slab, as in the Q4_K kernel: the even MMA's column 2t carries the hi half of the
-  // even-numbered elements of lane t's 64, column 2t+1 their lo half; the odd MMA the other way round
-  const bool mine = (g >> 1) == t;
-  const uint32_t pe = mine ? slab + (2 * t) * SL::SUB_BYTES + ((g & 1) ? SL::LO_OFF : 0) : szero;
-  const uint32_t po = mine ? slab + (2 * t + 1) * SL::SUB_BYTES + ((g & 1) ? 0 : SL::LO_OFF) : szero;
-  const uint32_t mask = 0x00F000F0u, magic = 0x54005400u;  // f16 (64 + nibble)
+  const uint32_t b_off = slab + (g & 3) * LIMB_PLANE + 4 * (g >> 2) + 8 * t;  // limb g & 3 of the even (g < 4) or odd elements of word t
+  const uint32_t m_off = ((lane & 7) + 8 * ((lane >> 3) & 1)) * I4_PITCH + 16 * (lane >> 4);  // ldmatrix row of this lane
+  const float lane_w = limb_weight(t, true);
 
   const int tiles = (N + ROWS - 1) / ROWS;
   const int t0 = (int)((uint32_t)tiles * blockIdx.x / gridDim.x), t1 = (int)((uint32_t)tiles * (blockIdx.x + 1) / gridDim.x);
@@ -1588,7 +1544,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) int4_gemv_mma_kernel(const XT *
     if (i_gt < t1 && warp < nb) {
       const int r0 = min((i_gt + i_rt) * ROWS, N - ROWS);
       const uint8_t *src = w + ((size_t)(r0 + c_row) * row_bytes + (uint32_t)i_b * 128u + c_piece * 16);
-      uint32_t dst = ring + i_slot * I4_TILE_BYTES + c_row * I4_PITCH + 16 + c_piece * 16;
+      uint32_t dst = ring + i_slot * I4_TILE_BYTES + c_row * I4_PITCH + c_piece * 16;
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         cp_async16(dst, src);
@@ -1622,34 +1578,32 @@ __global__ void __launch_bounds__(WARPS * 32, 2) int4_gemv_mma_kernel(const XT *
   };
   if (warp < nb) load_x(warp);
 
-  // One unit: rows g, g+8 of one tile x one run of 256 k, out of ring slot `sb`.  Lane t owns words 8t .. 8t+7
-  // of both rows (elements 64t .. 64t+63, one quantization group).  Word i gives the even MMA the f16 pairs
-  // (64 + n0, 64 + n4), (64 + n2, 64 + n6) and the odd MMA (n1, n5), (n3, n7); the slab holds x in that order.
-  // acc += s ((D_even + D_odd) - (64 + z) (Sx_even + Sx_odd)).
-  auto unit = [&](uint32_t sb, const float (&sc)[2], const float (&zp)[2], const float2 sx, float up, float (&vr)[2]) {
-    const uint32_t la = sb + g * I4_PITCH + 32u * t;
-    const uint4 qa0 = lds128(la + 16), qa1 = lds128(la + 32);
-    const uint4 qb0 = lds128(la + 8 * I4_PITCH + 16), qb1 = lds128(la + 8 * I4_PITCH + 32);
+  // One unit: rows g, g+8 of one tile x one run of 256 k, out of ring slot `sb`.  bl[p][h]: B of words 8p + 4h + t.  Lane t ends up with
+  // elements 64t .. 64t+63 of both rows, of which it holds scale, zero and activation sum.
+  auto unit = [&](uint32_t sb, const float (&sc)[2], const float (&zp)[2], const uint32_t (&bl)[4][2], const float sx, float up, float (&vr)[2]) {
+    uint4 q[4];
+#pragma unroll
+    for (int p = 0; p < 4; p++) q[p] = ldmatrix4(sb + m_off + 32 * p);
     __syncwarp();  // the slot is free again
     issue();
-    float de[4] = {0.f, 0.f, 0.f, 0.f}, dq[4] = {0.f, 0.f, 0.f, 0.f};  // even / odd element chains
-    const uint32_t qg[8] = {qa0.x, qa0.y, qa0.z, qa0.w, qa1.x, qa1.y, qa1.z, qa1.w};
-    const uint32_t qh[8] = {qb0.x, qb0.y, qb0.z, qb0.w, qb1.x, qb1.y, qb1.z, qb1.w};
+    float v[2][4];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const uint32_t vg = qg[i], vh = qh[i];
-      const uint32_t e0 = and_or(vg << 4, mask, magic), e1 = and_or(vh << 4, mask, magic);
-      const uint32_t e2 = and_or(vg >> 4, mask, magic), e3 = and_or(vh >> 4, mask, magic);
-      const uint32_t o0 = and_or(vg, mask, magic), o1 = and_or(vh, mask, magic);
-      const uint32_t o2 = and_or(vg >> 8, mask, magic), o3 = and_or(vh >> 8, mask, magic);
-      const uint2 be = lds64(pe + i * 8), bo = lds64(po + i * 8);
-      mma16816(de, e0, e1, e2, e3, be.x, be.y);
-      mma16816(dq, o0, o1, o2, o3, bo.x, bo.y);
+    for (int p = 0; p < 4; p++) {
+      int D[4] = {0, 0, 0, 0};
+      const uint32_t lo = 0x0F0F0F0Fu, hi = 0xF0F0F0F0u;
+      imma16832_u8(D, q[p].x & lo, q[p].y & lo, q[p].x & hi, q[p].y & hi, g < 4 ? bl[p][0] : 0u, g < 4 ? 0u : bl[p][0]);
+      imma16832_u8(D, q[p].z & lo, q[p].w & lo, q[p].z & hi, q[p].w & hi, g < 4 ? bl[p][1] : 0u, g < 4 ? 0u : bl[p][1]);
+#pragma unroll
+      for (int r = 0; r < 2; r++) v[r][p] = (float)(D[2 * r] + 256 * D[2 * r + 1]) * lane_w;
     }
-    const float ssum = sx.x + sx.y;
 #pragma unroll
-    for (int r = 0; r < 2; r++)
-      vr[r] = sc[r] * (((de[2 * r] + de[2 * r + 1]) + (dq[2 * r] + dq[2 * r + 1])) - (64.f + zp[r]) * ssum) * up;
+    for (int r = 0; r < 2; r++) {  // four lanes' parts of four sums: lane t keeps sum t
+      const bool up2 = t & 2, up1 = t & 1;
+      const float s0 = __shfl_xor_sync(0xffffffffu, up2 ? v[r][0] : v[r][2], 2), s1 = __shfl_xor_sync(0xffffffffu, up2 ? v[r][1] : v[r][3], 2);
+      const float k0 = (up2 ? v[r][2] : v[r][0]) + s0, k1 = (up2 ? v[r][3] : v[r][1]) + s1;
+      const float sum = (up1 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, up1 ? k0 : k1, 1);
+      vr[r] = sc[r] * (sum - zp[r] * sx) * up;
+    }
   };
 
   int slot = 0, parity = 0;
@@ -1676,10 +1630,22 @@ __global__ void __launch_bounds__(WARPS * 32, 2) int4_gemv_mma_kernel(const XT *
           }
       }
       __syncwarp();  // every lane is done reading the previous block's slab
-      const float up = stage_block_int4(xv, slab, lane);
+      float xs[2][4];
+      const float up = stage_limbs<LIMB_WORD8>(xv, slab, lane, xs);
+#pragma unroll
+      for (int i = 0; i < 2; i++) {  // sixteen lanes per set of 64
+        float v = (xs[i][0] + xs[i][1]) + (xs[i][2] + xs[i][3]);
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if ((lane & 15) == 0) sts32(slab + LIMB_BYTES + (2 * i + (lane >> 4)) * 4, __float_as_uint(v));
+      }
       __syncwarp();
-      float2 sx;
-      asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];\n" : "=f"(sx.x), "=f"(sx.y) : "r"(slab + SL::SX_OFF + 8 * t));
+      uint32_t bl[4][2];
+#pragma unroll
+      for (int p = 0; p < 4; p++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) bl[p][h] = lds32(b_off + 64 * p + 32 * h);
+      const float sx = __uint_as_float(lds32(slab + LIMB_BYTES + 4 * t));
 #pragma unroll
       for (int rt = 0; rt < GROUP; rt++) {
         if (rt >= gs) break;
@@ -1688,7 +1654,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) int4_gemv_mma_kernel(const XT *
         const uint32_t sb = ring + slot * I4_TILE_BYTES;
         slot = (slot + 1) & (S - 1);
         float vr[2];
-        unit(sb, scg[rt], zpg[rt], sx, up, vr);
+        unit(sb, scg[rt], zpg[rt], bl, sx, up, vr);
         // the warp's first block of a group overwrites what an earlier group left behind
         const uint32_t ra = red_g + rt * (32 * 8);
         float2 o = make_float2(0.f, 0.f);

@@ -23,7 +23,8 @@ def gguf(seed, dt, n, k):
 
 # both sides of each change of ring depth (K = 5376 and 14336 with Q4_K), the shortest rows, rows that are no whole tile
 @pytest.mark.parametrize("fmt,n,k", [("Q4_K", 16, 256), ("Q4_K", 161, 5376), ("Q4_K", 161, 5632), ("Q4_K", 48, 14336), ("Q4_K", 48, 14592),
-                                     ("Q4_K", 5000, 4096), ("Q6_K", 16, 512), ("Q6_K", 161, 1536), ("Q6_K", 5000, 4096)])
+                                     ("Q4_K", 5000, 4096), ("Q6_K", 16, 512), ("Q6_K", 161, 1536), ("Q6_K", 5000, 4096), ("Q8_0", 16, 256),
+                                     ("Q8_0", 161, 2304), ("Q8_0", 5000, 4096)])
 @pytest.mark.parametrize("kind", ["normal", "outlier", "tiny", "huge"])
 def test_one_row(cuda, fmt, n, k, kind):
     x = torch.randn(1, k, generator=torch.Generator().manual_seed(n + k)).to(cuda)
@@ -34,7 +35,21 @@ def test_one_row(cuda, fmt, n, k, kind):
     check(ops.MatMulQ(x, w), x, ops.Dequantize(w))
 
 
-@pytest.mark.parametrize("fmt", ["Q4_K", "Q6_K"])
+@pytest.mark.parametrize("n,k,group", [(16, 256, 64), (161, 2304, 128), (5000, 4096, 256)])
+@pytest.mark.parametrize("kind", ["normal", "outlier", "tiny", "huge"])
+def test_one_row_int4(cuda, n, k, group, kind):
+    """F32 activations and results; sum - z Sx is a difference as in Q4_K."""
+    g = torch.Generator().manual_seed(n + k)
+    x = torch.randn(1, k, generator=g).to(cuda)
+    if kind == "outlier":
+        x[0, 5] = 1000.0
+    x = x * {"tiny": 2.0**-90, "huge": 2.0**90}.get(kind, 1.0)
+    w = ops.Int4(torch.randint(-2**31, 2**31, (n, k // 8), generator=g, dtype=torch.int32).to(cuda), (torch.rand(n, k // group, generator=g) + 0.5).to(cuda),
+                 torch.randint(0, 16, (n, k // group), generator=g).float().to(cuda), group)
+    check(ops.MatMulInt4(x, w), x, ops.DequantizeInt4(w, torch.float32))
+
+
+@pytest.mark.parametrize("fmt", ["Q4_K", "Q6_K", "Q8_0"])
 def test_a_nan_reaches_every_row(cuda, fmt):
     x = torch.zeros(1, 1024, device=cuda)
     w = gguf(3, getattr(ops, fmt), 40, 1024)
