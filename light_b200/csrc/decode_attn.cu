@@ -359,6 +359,249 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attn_kernel(AttnArgs a) 
   cluster_combine<T, false>(a, cpart, g, D, ROW, KS, rank, b, kh, DA_THREADS);
 }
 
+// ------------------------------------------------------------------------------------ f32 caches, heads of 64 or 128
+// One lane per 1/32 of a row (the first kernel) spends 17 shuffles and 25 exponentials' worth of latency on four keys: 6 us of a 12.4 us
+// launch for 1024 positions, and a third of the memory rate on long caches.  Here the keys come in tiles of 64 through shared memory
+// (16-byte asynchronous copies, a ring of S tiles: the bytes in flight; one bulk copy per padded row took 2.8 us a tile), and a lane owns a KEY: a quarter of its dot products with all the group's heads
+// (K rows are padded by 16 bytes, so 32 keys lie on 32 banks; the queries are broadcasts), one warp per head then turns the tile's
+// scores into weights, and a lane owns D / 32 dims of the values, a warp eight keys.  Three CTA barriers a tile, no shuffle per key.
+//   * What depends on the position alone (angles, L2 hints) runs before the wait, the first tiles, the queries and the position itself
+//     are requested together after it; the position may have moved by then, and everything is planned again if it has.
+//   * The new key and value are written into the last tile in shared memory, where the cache's row would have landed: the same bits.
+// About 14 shared-memory cycles per key of 128 f32 dims and four heads against 40 that its bytes take from HBM: 8 sequences of 8192
+// keys, 8 KV heads of 128 under 32 heads 196 -> 108 us (5.0 TB/s); one of 1024 keys, where the chain of latencies is all, 16.0 -> 7.5 us.
+constexpr int FT_WARPS = 8, FT_THREADS = FT_WARPS * 32, FT_KEYS = 64;
+
+template <int D, int GH>
+struct F32Cfg {
+  static constexpr int S = GH == 16 || (D == 64 && GH == 8) ? 2 : 3;  // tiles in the ring: what 227 KB (two CTAs of D = 64) hold beside the scores
+  static constexpr int KP = D * 4 + 16, KB = FT_KEYS * KP, STAGE = KB + FT_KEYS * D * 4, ROW = D + 2;
+  static constexpr int QS = S * STAGE, PART = QS + GH * D * 4, PS = PART + 4 * GH * FT_KEYS * 4, CP = PS + FT_KEYS * GH * 4, MISC = CP + GH * ROW * 4;
+  // MISC: max, sum, correction [GH] each | angles [D]
+  static constexpr int TRIG = MISC + 3 * GH * 4, SMEM = TRIG + D * 4;
+};
+
+template <int D, int GH>
+__global__ void __launch_bounds__(FT_THREADS, D == 64 ? 2 : 1) decode_attn_f32_kernel(AttnArgs a) {
+  using C = F32Cfg<D, GH>;
+  constexpr int S = C::S, DQ = D / 4, PV = D / 32, HW = (GH + FT_WARPS - 1) / FT_WARPS;
+  constexpr int QP = (GH * D / 2 + FT_THREADS - 1) / FT_THREADS;  // (q[i], q[i + D / 2]) pairs per thread
+  extern __shared__ __align__(128) unsigned char fsm[];
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int KS = gridDim.y, rank = blockIdx.y, bkh = blockIdx.x, g = a.NH / a.KH, b = bkh / a.KH, kh = bkh - b * a.KH;
+  const uint32_t base = umma::smem_u32(fsm);
+  float *qs = reinterpret_cast<float *>(fsm + C::QS), *part = reinterpret_cast<float *>(fsm + C::PART), *ps = reinterpret_cast<float *>(fsm + C::PS);
+  float *cpart = reinterpret_cast<float *>(fsm + C::CP), *ms = reinterpret_cast<float *>(fsm + C::MISC), *ls = ms + GH, *cs = ls + GH;
+  float *trig = reinterpret_cast<float *>(fsm + C::TRIG);
+  const float *kc = static_cast<const float *>(a.kbuf) + (size_t)bkh * a.Cap * D, *vc = static_cast<const float *>(a.vbuf) + (size_t)bkh * a.Cap * D;
+  const bool roped = a.rope_k != 0.0;
+
+  int pos, j0, n;  // this CTA's keys: j0 .. j0 + n
+  bool in_range, fresh;  // fresh: the last of them is the new one, which the cache does not hold yet
+  auto plan = [&](long long p) {
+    // a position outside the cache: nothing is appended (as kv_append_kernel), and the launch attends over the clamped range
+    in_range = p >= 0 && p < a.Cap;
+    pos = (int)(p < 0 ? 0ll : p < a.Cap ? p : (long long)a.Cap - 1);
+    const int start = a.window > 0 ? max(0, pos + 1 - a.window) : 0, end = pos + 1, ch = (end - start + KS - 1) / KS;
+    j0 = start + rank * ch, n = max(0, min(end, j0 + ch) - j0);
+    fresh = a.k_new && in_range && n > 0 && j0 + n == end;
+  };
+  auto angles = [&]() {
+    for (int i = tid; i < D / 2; i += FT_THREADS) {
+      const float2 v = rope_cos_sin(pos, i, a.rope_k);
+      trig[i] = v.x, trig[D / 2 + i] = v.y;
+    }
+  };
+  const long long seen = a.pos[0];
+  plan(seen);
+  {
+    const char *kp = reinterpret_cast<const char *>(kc + (size_t)j0 * D), *vp = reinterpret_cast<const char *>(vc + (size_t)j0 * D);
+    const int lines = min(n * (D * 4 / 128), 8 * FT_THREADS);
+    for (int i = tid; i < lines; i += FT_THREADS)
+      asm volatile("prefetch.global.L2 [%0];\n\tprefetch.global.L2 [%1];\n" ::"l"(kp + (size_t)i * 128), "l"(vp + (size_t)i * 128));
+  }
+  if (roped) angles();
+  __syncthreads();
+  pdl_wait();  // q, k_new, v_new are the previous launch's output; so may be the cache's last rows and the position
+  auto issue = [&](int t) {  // tile t into slot t % S: always one commit group
+    const int cnt = min(FT_KEYS, n - (fresh ? 1 : 0) - t * FT_KEYS);  // 0 for a tile of the new key alone
+    const uint32_t dst = base + (t % S) * C::STAGE;
+    const size_t row = (size_t)(j0 + t * FT_KEYS) * D;
+    constexpr int PIECES = D / 4;  // of 16 bytes per row
+    for (int i = tid; i < cnt * PIECES; i += FT_THREADS) {
+      const int r = i / PIECES, c = i % PIECES;
+      cp_async16(dst + r * C::KP + c * 16, kc + row + (size_t)i * 4);
+      cp_async16(dst + C::KB + i * 16, vc + row + (size_t)i * 4);
+    }
+    cp_async_commit();
+  };
+  auto fill = [&]() {
+#pragma unroll 1
+    for (int t = 0; t < S - 1; t++) issue(t);
+  };
+  fill();
+  const long long now = *(const volatile long long *)a.pos;
+  float2 qv[QP], kv = make_float2(0.f, 0.f), vv = kv;
+#pragma unroll
+  for (int i = 0; i < QP; i++) {
+    const int idx = tid + i * FT_THREADS, h = idx / (D / 2), d = idx % (D / 2);
+    const float *q = static_cast<const float *>(a.q) + ((size_t)b * a.NH + (size_t)kh * g + h) * D + d;
+    qv[i] = h < g ? make_float2(q[0], q[D / 2]) : make_float2(0.f, 0.f);
+  }
+  if (a.k_new && tid < D / 2) {
+    const float *k = static_cast<const float *>(a.k_new) + (size_t)bkh * D + tid, *v = static_cast<const float *>(a.v_new) + (size_t)bkh * D + tid;
+    kv = make_float2(k[0], k[D / 2]), vv = make_float2(v[0], v[D / 2]);
+  }
+  if (now != seen) {  // the position moved while the launch before ran (the same in every thread)
+    cp_async_wait<0>();
+    __syncthreads();
+    plan(now);
+    if (roped) angles();
+    __syncthreads();
+    fill();
+  }
+  auto rot = [&](float2 v, int d) { return roped ? make_float2(v.x * trig[d] - v.y * trig[D / 2 + d], v.x * trig[D / 2 + d] + v.y * trig[d]) : v; };
+#pragma unroll
+  for (int i = 0; i < QP; i++) {
+    const int idx = tid + i * FT_THREADS, h = idx / (D / 2), d = idx % (D / 2);
+    if (h < GH) {
+      const float2 v = rot(qv[i], d);
+      qs[h * D + d] = v.x, qs[h * D + d + D / 2] = v.y;
+    }
+  }
+  if (tid < D / 2) kv = rot(kv, tid);
+  __syncthreads();
+
+  float acc[GH][PV], m[HW], l[HW];  // m, l: of heads warp, warp + 8
+#pragma unroll
+  for (int h = 0; h < GH; h++)
+#pragma unroll
+    for (int i = 0; i < PV; i++) acc[h][i] = 0.f;
+#pragma unroll
+  for (int i = 0; i < HW; i++) m[i] = -INFINITY, l[i] = 0.f;
+  const int tiles = (n + FT_KEYS - 1) / FT_KEYS, qd = warp >> 1, key = (warp & 1) * 32 + lane;
+  for (int t = 0; t < tiles; t++) {
+    const int cnt = min(FT_KEYS, n - t * FT_KEYS);
+    unsigned char *kt = fsm + (t % S) * C::STAGE, *vt = kt + C::KB;
+    if (fresh && t == tiles - 1) {  // the slot is free, and no copy touches this row
+      if (tid < D / 2) {
+        float *k = reinterpret_cast<float *>(kt + (cnt - 1) * C::KP) + tid, *v = reinterpret_cast<float *>(vt + (cnt - 1) * (D * 4)) + tid;
+        k[0] = kv.x, k[D / 2] = kv.y, v[0] = vv.x, v[D / 2] = vv.y;
+      }
+    }
+    cp_async_wait<S - 2>();
+    __syncthreads();     // the tile is in place, and every warp is done with the one before it
+    issue(t + S - 1);    // into that one's slot
+    if (key < cnt || (warp & 1) * 32 < cnt) {  // a quarter of a key's products with every head (rows past cnt hold what they held)
+      float d[GH];
+#pragma unroll
+      for (int h = 0; h < GH; h++) d[h] = 0.f;
+#pragma unroll
+      for (int i = 0; i < DQ / 4; i++) {
+        const float4 k = *reinterpret_cast<const float4 *>(kt + key * C::KP + (qd * DQ + 4 * i) * 4);
+#pragma unroll
+        for (int h = 0; h < GH; h++) {
+          const float4 q = *reinterpret_cast<const float4 *>(qs + h * D + qd * DQ + 4 * i);
+          d[h] = fmaf(q.x, k.x, fmaf(q.y, k.y, fmaf(q.z, k.z, fmaf(q.w, k.w, d[h]))));
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < GH; h++) part[(qd * GH + h) * FT_KEYS + key] = d[h];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < HW; i++) {
+      const int h = warp + FT_WARPS * i;
+      if (h < GH) {
+        float v[2], mx = m[i];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const float *p = part + h * FT_KEYS + lane + 32 * u;
+          v[u] = lane + 32 * u < cnt ? ((p[0] + p[GH * FT_KEYS]) + (p[2 * GH * FT_KEYS] + p[3 * GH * FT_KEYS])) * a.scale : -INFINITY;
+          mx = fmaxf(mx, v[u]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float corr = __expf(m[i] - mx), e0 = __expf(v[0] - mx), e1 = __expf(v[1] - mx);  // m = -inf at first: 0
+        m[i] = mx;
+        l[i] = fmaf(l[i], corr, e0 + e1);  // each lane its own keys' part
+        ps[lane * GH + h] = e0, ps[(lane + 32) * GH + h] = e1;
+        if (lane == 0) cs[h] = corr;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < GH; h++) {
+      const float c = cs[h];
+#pragma unroll
+      for (int i = 0; i < PV; i++) acc[h][i] *= c;
+    }
+    auto add = [&](int k) {
+      float v[PV];
+      if constexpr (PV == 4) {
+        const float4 x = *reinterpret_cast<const float4 *>(vt + k * (D * 4) + lane * 16);
+        v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+      } else {
+        const float2 x = *reinterpret_cast<const float2 *>(vt + k * (D * 4) + lane * 8);
+        v[0] = x.x, v[1] = x.y;
+      }
+      float p[GH];
+      if constexpr (GH >= 4) {
+#pragma unroll
+        for (int h = 0; h < GH; h += 4) {
+          const float4 x = *reinterpret_cast<const float4 *>(ps + k * GH + h);
+          p[h] = x.x, p[h + 1] = x.y, p[h + 2] = x.z, p[h + 3] = x.w;
+        }
+      } else {
+#pragma unroll
+        for (int h = 0; h < GH; h++) p[h] = ps[k * GH + h];
+      }
+#pragma unroll
+      for (int h = 0; h < GH; h++)
+#pragma unroll
+        for (int i = 0; i < PV; i++) acc[h][i] = fmaf(p[h], v[i], acc[h][i]);
+    };
+    if (warp * 8 + 8 <= cnt) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) add(warp * 8 + k);
+    } else {
+      for (int k = warp * 8; k < cnt; k++) add(k);
+    }
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  // ---- the warps' values over the (drained) ring, the heads' maxima and sums
+  float *wpart = reinterpret_cast<float *>(fsm);
+#pragma unroll
+  for (int h = 0; h < GH; h++)
+#pragma unroll
+    for (int i = 0; i < PV; i++) wpart[(warp * GH + h) * D + lane * PV + i] = acc[h][i];
+#pragma unroll
+  for (int i = 0; i < HW; i++) {
+    const float sum = warp_sum(l[i]);
+    if (lane == 0 && warp + FT_WARPS * i < GH) ms[warp + FT_WARPS * i] = m[i], ls[warp + FT_WARPS * i] = sum;
+  }
+  __syncthreads();
+  for (int idx = tid; idx < g * D; idx += FT_THREADS) {
+    const int h = idx / D, d = idx - h * D;
+    float A = 0.f;
+#pragma unroll
+    for (int w = 0; w < FT_WARPS; w++) A += wpart[(w * GH + h) * D + d];
+    cpart[h * C::ROW + 2 + d] = A;
+    if (d == 0) cpart[h * C::ROW] = ms[h], cpart[h * C::ROW + 1] = ls[h];
+  }
+  if (fresh && tid < D / 2) {  // the append: nothing of this launch reads the row from the cache
+    const size_t dst = ((size_t)bkh * a.Cap + (size_t)pos) * D + tid;
+    float *k = static_cast<float *>(a.kbuf) + dst, *v = static_cast<float *>(a.vbuf) + dst;
+    k[0] = kv.x, k[D / 2] = kv.y, v[0] = vv.x, v[D / 2] = vv.y;
+  }
+  if (tid == 0 && !in_range) atomicOr(&g_attn_status, 1u);
+  __syncthreads();
+  if (KS > 1) umma::cluster_sync();
+  cluster_combine<float, false>(a, cpart, g, D, C::ROW, KS, rank, b, kh, FT_THREADS);
+}
+
 // ------------------------------------------------------------------------------------ bf16 caches on the tensor cores
 // The kernel above spends about 60 instructions of a warp per key (unpacking, 2 D FMAs per head and key over 32 lanes, the
 // reduce-scatter), which bounds a bf16 cache at 1.2 TB/s (8 sequences, 8192 keys, 8 KV heads of 128: 231 us).  Here a warp takes
@@ -703,12 +946,37 @@ int launch_mma(const AttnArgs &a, cudaStream_t st) {
   return launched("decode_attn");
 }
 
+template <int D, int GH>
+int launch_f32(const AttnArgs &a, cudaStream_t st) {
+  auto kern = decode_attn_f32_kernel<D, GH>;
+  constexpr size_t smem = F32Cfg<D, GH>::SMEM;
+  static DeviceOnce smem_set;
+  cudaError_t e = smem_set.ensure([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); }, smem);
+  if (e != cudaSuccess) return fail((int)e, "light_b200: decode_attn: %s", cudaGetErrorString(e));
+  // as many CTAs along the keys as fit on the SMs at once, with a tile of the capacity or more for each
+  const int slots = (D == 64 ? 2 : 1) * sm_count();
+  int ks = 1;
+  while (ks < 8 && a.B * a.KH * (ks + 1) <= slots && a.Cap >= FT_KEYS * (ks + 1)) ks++;
+  e = launch_chain(kern, dim3((unsigned)(a.B * a.KH), (unsigned)ks), dim3(FT_THREADS), smem, (unsigned)ks, st, a);
+  if (e != cudaSuccess) return fail((int)e, "light_b200: decode_attn: %s", cudaGetErrorString(e));
+  return launched("decode_attn");
+}
+
+template <int D>
+int launch_f32_g(const AttnArgs &a, int g, cudaStream_t st) {
+  return g == 1 ? launch_f32<D, 1>(a, st) : g == 2 ? launch_f32<D, 2>(a, st) : g <= 4 ? launch_f32<D, 4>(a, st) : g <= 8 ? launch_f32<D, 8>(a, st) : launch_f32<D, 16>(a, st);
+}
+
 template <typename T>
 int launch_attn_d(const AttnArgs &a, int D, int ks, cudaStream_t st) {
   switch (D / 32) {
     case 1: return launch_attn_g<T, 1>(a, ks, st);
-    case 2: return launch_attn_g<T, 2>(a, ks, st);
-    case 4: return launch_attn_g<T, 4>(a, ks, st);
+    case 2:
+      if constexpr (sizeof(T) == 2) return launch_attn_g<T, 2>(a, ks, st);  // a bf16 cache that is not on 32 bytes
+      break;
+    case 4:
+      if constexpr (sizeof(T) == 2) return launch_attn_g<T, 4>(a, ks, st);
+      break;
     case 8: return launch_attn_g<T, 8>(a, ks, st);
     case 16: return launch_attn_g<T, 16>(a, ks, st);
   }
@@ -738,6 +1006,8 @@ int decode_attn(const lb200_decode_attn_args *p, cudaStream_t st) {
     if (p->D == 64) return g <= 8 ? launch_mma<64, false>(a, st) : launch_mma<64, true>(a, st);
     return g <= 8 ? launch_mma<128, false>(a, st) : launch_mma<128, true>(a, st);
   }
+  if (p->dtype == LB200_F32 && p->D == 64) return launch_f32_g<64>(a, g, st);
+  if (p->dtype == LB200_F32 && p->D == 128) return launch_f32_g<128>(a, g, st);
   // enough CTAs to fill the GPU, at least 32 keys of the capacity each, a portable cluster
   int ks = 1;
   while (ks < 8 && p->B * p->KH * ks < 148 && p->Cap >= 64 * ks) ks *= 2;

@@ -158,3 +158,42 @@ def test_tensor_core_kernel(cuda, B, NH, KH, D, n, win):
     want = torch.softmax(rot(q).reshape(B, KH, NH // KH, D) @ K.transpose(-1, -2) * D ** -0.5, -1) @ V
     err = (got.double().reshape(want.shape) - want).norm() / want.norm()
     assert float(err) <= 3e-3 and ops.decode_attn_status(0) == 0
+
+
+def test_position_moves_right_before_the_launch(cuda):
+    """The launch starts while the increment before it still runs, and works ahead for the position as it stood: the same bits as with a
+    wait between the two."""
+    B, NH, KH, D, cap, steps = 2, 8, 2, 128, 256, 40
+    g = torch.Generator(device=cuda).manual_seed(5)
+    q, k, v = (torch.randn(steps, B, h, 1, D, generator=g, device=cuda) for h in (NH, KH, KH))
+    outs = []
+    for wait in (False, True):
+        kb, vb, pos = torch.zeros(B, KH, cap, D, device=cuda), torch.zeros(B, KH, cap, D, device=cuda), torch.full((1,), 29, device=cuda)
+        y = []
+        for s in range(steps):
+            ops.IncrementI64(pos)
+            if wait:
+                torch.cuda.synchronize()
+            y.append(ops.DecodeAttention(q[s], kb, vb, pos, D ** -0.5, 0, k[s], v[s], rope_base=10000.0))
+        outs.append(torch.cat([torch.stack(y).flatten(), kb.flatten(), vb.flatten()]))
+    assert torch.equal(*outs)
+
+
+@pytest.mark.parametrize("D,g", [(64, 1), (64, 2), (64, 3), (64, 8), (64, 16), (128, 1), (128, 2), (128, 4), (128, 5), (128, 16)])
+@pytest.mark.parametrize("n,window", [(1, 0), (64, 0), (65, 0), (513, 0), (1025, 0), (700, 100)])
+def test_f32_kernel(cuda, D, g, n, window):
+    """Every count of heads per pass, and tiles of 64 keys with nothing, one or all but one key in the last: against f64, 512 roundings of
+    2^-24 in the sums and 2^-20 of the exponentials' arguments stay below 1e-4 of the largest value."""
+    B, KH = 2, 3
+    gen = torch.Generator(device=cuda).manual_seed(D + g + n)
+    kb, vb = (torch.full((B, KH, n + 3, D), float("nan"), device=cuda) for _ in range(2))
+    kb[:, :, :n - 1], vb[:, :, :n - 1] = (torch.randn(B, KH, n - 1, D, generator=gen, device=cuda) for _ in range(2))
+    q = torch.randn(B, KH * g, 1, D, generator=gen, device=cuda)
+    k, v = (torch.randn(B, KH, 1, D, generator=gen, device=cuda) for _ in range(2))
+    pos = torch.full((1,), n - 1, device=cuda)
+    got = ops.DecodeAttention(q, kb, vb, pos, D ** -0.5, window, k, v)
+    assert torch.equal(kb[:, :, n - 1], k[:, :, 0]) and torch.equal(vb[:, :, n - 1], v[:, :, 0])
+    s0 = max(0, n - window) if window else 0
+    S = (q.double().reshape(B, KH, g, D) @ kb[:, :, s0:n].double().transpose(-1, -2) * D ** -0.5).softmax(-1)
+    want = (S @ vb[:, :, s0:n].double()).reshape(B, KH * g, 1, D)
+    assert (got.double() - want).abs().max() <= 1e-4 * v.abs().max()
