@@ -5,6 +5,7 @@
 // kernels/cuda/src/elementwise.cu:748-774, CPU kernels/cpu/misc_registry.go:27-92).
 #include "common.cuh"
 #include "mma_sync.cuh"
+#include "umma.cuh"
 
 namespace lb {
 namespace {
@@ -66,39 +67,60 @@ __global__ void rope_kernel(const T *__restrict__ x, const long long *__restrict
   st_act(out, o + half, x0 * sf + x1 * cf);
 }
 
-// Greedy sampling: the index of the largest element of every row (ties: the lowest index), as I64.  One CTA per
-// row; reference ops.Argmax on the last axis (ops/argmax.go:14-60, kernels/cuda/topk.go:56-90).
-__global__ void __launch_bounds__(1024) argmax_rows_kernel(const float *__restrict__ x, long long *__restrict__ out, int cols) {
+// Greedy sampling: the index of the largest element of every row (ties: the lowest index), as I64.  reference ops.Argmax on the last
+// axis (ops/argmax.go:14-60, kernels/cuda/topk.go:56-90).  A row is a cluster of ks CTAs, eight for a few long rows: one SM has
+// too few loads in flight (128256 columns: 15.7 us by one CTA with a load at a time).
+__global__ void __launch_bounds__(1024) argmax_rows_kernel(const float *__restrict__ x, long long *__restrict__ out, int cols, int ks) {
   __shared__ float bv[32];
   __shared__ int bi[32];
+  __shared__ float best_v;
+  __shared__ int best_i;
   pdl_launch_dependents();
   pdl_wait();
-  const float *row = x + (size_t)blockIdx.x * cols;
+  const int rank = blockIdx.x % ks, step = 1024 * ks;
+  const float *row = x + (size_t)(blockIdx.x / ks) * cols;
   float v = -INFINITY;
   int idx = 0x7fffffff;
-  for (int j = threadIdx.x; j < cols; j += 1024) {
-    const float c = row[j];
+  auto take = [&](float c, int j) {
     if (c > v || (c == v && j < idx) || idx == 0x7fffffff) v = c, idx = j;  // NaN never wins over a number; the first element seeds
-  }
-  auto better = [](float a, int ai, float b, int bi_) { return a > b || (a == b && ai < bi_); };
+  };
+  int j = rank * 1024 + threadIdx.x;
+  for (; j + 7ll * step < cols; j += 8 * step) {
+    float c[8];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-    if (oi != 0x7fffffff && (idx == 0x7fffffff || better(ov, oi, v, idx))) v = ov, idx = oi;
+    for (int i = 0; i < 8; i++) c[i] = row[j + i * step];
+#pragma unroll
+    for (int i = 0; i < 8; i++) take(c[i], j + i * step);
   }
-  if ((threadIdx.x & 31) == 0) bv[threadIdx.x >> 5] = v, bi[threadIdx.x >> 5] = idx;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    v = bv[threadIdx.x], idx = bi[threadIdx.x];
+  for (; j < cols; j += step) take(row[j], j);
+  auto better = [](float a, int ai, float b, int bi_) { return a > b || (a == b && ai < bi_); };
+  auto warp_best = [&]() {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float ov = __shfl_xor_sync(0xffffffffu, v, o);
       const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
       if (oi != 0x7fffffff && (idx == 0x7fffffff || better(ov, oi, v, idx))) v = ov, idx = oi;
     }
-    if (threadIdx.x == 0) out[blockIdx.x] = idx;
+  };
+  warp_best();
+  if ((threadIdx.x & 31) == 0) bv[threadIdx.x >> 5] = v, bi[threadIdx.x >> 5] = idx;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    v = bv[threadIdx.x], idx = bi[threadIdx.x];
+    warp_best();
+    if (threadIdx.x == 0) best_v = v, best_i = idx;
   }
+  if (ks > 1) {
+    umma::cluster_sync();
+    if (rank == 0 && threadIdx.x < 32) {
+      const uint32_t r = (uint32_t)min((int)threadIdx.x, ks - 1);
+      v = umma::ld_cluster_f32(umma::map_to_rank(umma::smem_u32(&best_v), r));
+      idx = __float_as_int(umma::ld_cluster_f32(umma::map_to_rank(umma::smem_u32(&best_i), r)));
+      warp_best();
+    }
+    umma::cluster_sync();  // nobody leaves while a peer still reads its best
+  }
+  if (rank == 0 && threadIdx.x == 0) out[blockIdx.x / ks] = idx;
 }
 
 template <typename K, typename... Args>
@@ -137,7 +159,16 @@ int argmax_rows(const float *x, int64_t *out, long long rows, int cols, cudaStre
   if (!x || !out) return fail(LB200_E_NULL, "light_b200: argmax: null pointer");
   if (rows < 0 || rows > 0x7fffffffLL || cols <= 0) return fail(LB200_E_SHAPE, "light_b200: argmax: rows %lld cols %d", rows, cols);
   if (rows == 0) return 0;
-  cudaError_t e = launch_chain(argmax_rows_kernel, (unsigned)rows, 1024u, st, x, (long long *)out, cols);
+  const bool split = cols >= 16384 && rows * 8 <= sm_count();  // two elements a thread or more, and SMs to spare
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)rows * (split ? 8u : 1u)), cfg.blockDim = dim3(1024), cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 8, attr[1].val.clusterDim.y = 1, attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr, cfg.numAttrs = split ? 2 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, argmax_rows_kernel, x, (long long *)out, cols, split ? 8 : 1);
   if (e != cudaSuccess) return fail((int)e, "light_b200: argmax: %s", cudaGetErrorString(e));
   return launched("argmax");
 }

@@ -98,3 +98,14 @@ def test_argmax(cuda, rows, cols):
     got = ops.Argmax(x.to(cuda)).cpu()
     want = torch.tensor([int(np.flatnonzero(r == r.max())[0]) for r in x.numpy()])
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 16383), (1, 16384), (18, 65537), (19, 65537)])
+def test_argmax_over_a_cluster(cuda, rows, cols):
+    """Long rows, a few of them by eight CTAs each: the largest, and twice the largest, anywhere."""
+    g = torch.Generator().manual_seed(rows + cols)
+    x = torch.randn(rows, cols, generator=g)
+    at = torch.randint(0, cols, (rows,), generator=g)
+    x[torch.arange(rows), at] = 9.0
+    x[:, cols - 1] = 9.0
+    assert torch.equal(ops.Argmax(x.to(cuda)).cpu().flatten(), at)
