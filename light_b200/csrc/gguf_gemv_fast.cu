@@ -231,8 +231,9 @@ __device__ __forceinline__ void st_slots(uint2 *const (&peer)[LB200_MAX_PEERS], 
 
 // Up to four weight matrices that share one activation row and one K, served by ONE launch: the
 // row tiles of all of them form one list, which the CTAs split evenly.  With act != 0 there are
-// two matrices of equal height (gate, up), their tiles alternate in the list, and the launch
-// stores act(gate . x) * (up . x) into out[0].
+// two matrices of equal height (gate, up), a tile is eight rows of the one above the same eight of
+// the other, and the launch stores act(gate . x) * (up . x) into out[0].  (Whole tiles of both, in
+// pairs, left a CTA of 14336 rows three or four pairs, and the four set the time: 17.5 -> 16.3 us.)
 struct MultiArgs {
   const uint8_t *w[4];
   float *out[4];
@@ -247,8 +248,8 @@ struct MultiArgs {
 // stores write identical values.
 __device__ __forceinline__ void resolve_tile(const MultiArgs &a, int T, int &j, int &r0) {
   if (a.act) {
-    j = T & 1;
-    r0 = min((T >> 1) * ROWS, a.n[0] - ROWS);
+    j = 0;
+    r0 = min(T * (ROWS / 2), a.n[0] - ROWS / 2);
     return;
   }
   j = 0;
@@ -316,10 +317,9 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q4k_gemv_mma_kernel(const float
   const uint32_t sc_sel = limb_sel(t >> 1), mn_sel = limb_sel(2 * (t & 1));
   const float lane_w = limb_weight(t, true);
 
-  // this CTA's share [t0, t1) of the tile list (whole gate/up pairs when act != 0)
-  const int unit = a.act ? 2 : 1, lt = tiles / unit;
-  const int t0 = (int)((uint32_t)lt * blockIdx.x / gridDim.x) * unit,  // lt * gridDim.x < 2^32 (launcher)
-            t1 = (int)((uint32_t)lt * (blockIdx.x + 1) / gridDim.x) * unit;
+  // this CTA's share [t0, t1) of the tile list
+  const int t0 = (int)((uint32_t)tiles * blockIdx.x / gridDim.x),  // tiles * gridDim.x < 2^32 (launcher)
+            t1 = (int)((uint32_t)tiles * (blockIdx.x + 1) / gridDim.x);
 
   // source offsets of this lane's chunks, relative to the tile's first byte (row 0, this block)
   uint32_t soff[5];
@@ -334,11 +334,12 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q4k_gemv_mma_kernel(const float
     if (i_gt < t1 && warp < nb) {
       int j, r0;
       resolve_tile(a, i_gt + i_rt, j, r0);
-      const uint8_t *base = a.w[j] + ((size_t)r0 * row_bytes + (uint32_t)i_b * 144u);
+      const size_t off = (size_t)r0 * row_bytes + (uint32_t)i_b * 144u;
+      const uint8_t *base = a.w[j] + off, *low = a.act ? a.w[1] + off - (ROWS / 2) * row_bytes : base;  // rows 0..7, 8..15
       const uint32_t dst = ring + i_slot * Q4K_TILE_BYTES + lane * 16;
-#pragma unroll
-      for (int i = 0; i < 4; i++) cp_async16(dst + i * 512, base + soff[i]);
-      if (lane < 16) cp_async16(dst + 2048, base + soff[4]);
+      cp_async16(dst, base + soff[0]), cp_async16(dst + 512, base + soff[1]);
+      cp_async16(dst + 1024, (lane < 8 ? base : low) + soff[2]), cp_async16(dst + 1536, low + soff[3]);
+      if (lane < 16) cp_async16(dst + 2048, low + soff[4]);
       i_slot = (i_slot + 1) & (S - 1);
       if (++i_rt == i_gs) {
         i_rt = 0, i_b += WARPS;
@@ -358,40 +359,56 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q4k_gemv_mma_kernel(const float
     if (tp.x_slots) asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(tp_t0));
   }
   float nrm_ss = 0.f;
-  for (int b = warp; b < nb; b += WARPS) {
-    float4 xv[2];
-    if (TP && tp.x_slots) {  // the peers' parts of x arrive as tagged slots
-      const uint2 *xs = tp.x_slots + (size_t)(tag & 1u) * K + b * 256 + lane * 4;
-      xv[0] = ld_slots4(xs, tag, tp_t0, tp_gave_up);
-      xv[1] = ld_slots4(xs + 128, tag, tp_t0, tp_gave_up);
-    } else {
-      xv[0] = __ldg(reinterpret_cast<const float4 *>(x + b * 256) + lane);
-      xv[1] = __ldg(reinterpret_cast<const float4 *>(x + b * 256 + 128) + lane);
-    }
-    if constexpr (NORM) {
+  for (int b0 = warp; b0 < nb; b0 += 2 * WARPS) {  // two blocks at a time: one trip to L2 for both
+    float4 xv[2][2], rv[2][2], wn[2][2];
 #pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const int e4 = b * 64 + i * 32 + lane;  // float4 index into the row
-        if (nrm.residual) {
-          const float4 r = __ldg(reinterpret_cast<const float4 *>(nrm.residual) + e4);
-          xv[i].x += r.x, xv[i].y += r.y, xv[i].z += r.z, xv[i].w += r.w;
-          if (blockIdx.x == 0) reinterpret_cast<float4 *>(nrm.sum_out)[e4] = xv[i];
+    for (int u = 0; u < 2; u++) {
+      const int b = min(b0 + u * WARPS, nb - 1);
+      if (TP && tp.x_slots) {  // the peers' parts of x arrive as tagged slots
+        const uint2 *xs = tp.x_slots + (size_t)(tag & 1u) * K + b * 256 + lane * 4;
+        xv[u][0] = ld_slots4(xs, tag, tp_t0, tp_gave_up);
+        xv[u][1] = ld_slots4(xs + 128, tag, tp_t0, tp_gave_up);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 2; i++) xv[u][i] = __ldg(reinterpret_cast<const float4 *>(x) + b * 64 + i * 32 + lane);
+      }
+      if constexpr (NORM) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          wn[u][i] = __ldg(reinterpret_cast<const float4 *>(nrm.weight) + b * 64 + i * 32 + lane);
+          if (nrm.residual) rv[u][i] = __ldg(reinterpret_cast<const float4 *>(nrm.residual) + b * 64 + i * 32 + lane);
         }
-        nrm_ss = fmaf(xv[i].x, xv[i].x, fmaf(xv[i].y, xv[i].y, fmaf(xv[i].z, xv[i].z, fmaf(xv[i].w, xv[i].w, nrm_ss))));
-        const float4 wn = __ldg(reinterpret_cast<const float4 *>(nrm.weight) + e4);
-        xv[i].x *= wn.x, xv[i].y *= wn.y, xv[i].z *= wn.z, xv[i].w *= wn.w;
       }
     }
-    const uint32_t slab = slabs + b * Q4K_SLAB;
-    float xs[2][4];
-    const float up = stage_limbs(xv, slab, lane, xs);
 #pragma unroll
-    for (int i = 0; i < 2; i++) {  // eight lanes per sub-block
-      float v = (xs[i][0] + xs[i][1]) + (xs[i][2] + xs[i][3]);
-      v += __shfl_xor_sync(0xffffffffu, v, 1), v += __shfl_xor_sync(0xffffffffu, v, 2), v += __shfl_xor_sync(0xffffffffu, v, 4);
-      if ((lane & 7) == 0) sts32(slab + Q4K_SX + (4 * i + (lane >> 3)) * 4, __float_as_uint(v));
+    for (int u = 0; u < 2; u++) {
+      const int b = b0 + u * WARPS;
+      if (b >= nb) break;
+      if constexpr (NORM) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          float4 &v = xv[u][i];
+          if (nrm.residual) {
+            const float4 r = rv[u][i];
+            v.x += r.x, v.y += r.y, v.z += r.z, v.w += r.w;
+            if (blockIdx.x == 0) reinterpret_cast<float4 *>(nrm.sum_out)[b * 64 + i * 32 + lane] = v;
+          }
+          nrm_ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, nrm_ss))));
+          const float4 w4 = wn[u][i];
+          v.x *= w4.x, v.y *= w4.y, v.z *= w4.z, v.w *= w4.w;
+        }
+      }
+      const uint32_t slab = slabs + b * Q4K_SLAB;
+      float xs[2][4];
+      const float up = stage_limbs(xv[u], slab, lane, xs);
+#pragma unroll
+      for (int i = 0; i < 2; i++) {  // eight lanes per sub-block
+        float v = (xs[i][0] + xs[i][1]) + (xs[i][2] + xs[i][3]);
+        v += __shfl_xor_sync(0xffffffffu, v, 1), v += __shfl_xor_sync(0xffffffffu, v, 2), v += __shfl_xor_sync(0xffffffffu, v, 4);
+        if ((lane & 7) == 0) sts32(slab + Q4K_SX + (4 * i + (lane >> 3)) * 4, __float_as_uint(v));
+      }
+      if (lane == 0) sts32(slab + Q4K_UP, __float_as_uint(up));
     }
-    if (lane == 0) sts32(slab + Q4K_UP, __float_as_uint(up));
   }
   if constexpr (NORM) {
     nrm_ss = warp_sum(nrm_ss);
@@ -403,7 +420,9 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q4k_gemv_mma_kernel(const float
     float tot = 0.f;
 #pragma unroll
     for (int i = 0; i < WARPS; i++) tot += nrm_part[i];
-    nrm_inv = (float)(1.0 / sqrt((double)(tot / (float)K) + (double)nrm.eps));
+    // 1 / sqrt by one Newton step in f64 from the f32 function (2^-43): f64 division and square root took 0.4 us of every launch
+    const double ms = (double)(tot / (float)K) + (double)nrm.eps, y = (double)rsqrtf((float)ms);
+    nrm_inv = ms > 1e-30 && ms < 1e30 ? (float)(y * (1.5 - 0.5 * ms * y * y)) : (float)(1.0 / sqrt(ms));
   }
   int slot = 0, parity = 0;
   for (int gt = t0; gt < t1; gt += GROUP, parity ^= 1) {
@@ -477,11 +496,11 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q4k_gemv_mma_kernel(const float
       return v;
     };
     if (a.act) {
-      for (int i = threadIdx.x; i < (gs >> 1) * ROWS; i += WARPS * 32) {
-        const int pr = i >> 4, row = i & 15;
+      for (int i = threadIdx.x; i < gs * (ROWS / 2); i += WARPS * 32) {
+        const int rt = i >> 3, row = i & 7;
         int j, r0;
-        resolve_tile(a, gt + 2 * pr, j, r0);
-        const float v = gate_act(row_sum(2 * pr, row) * nrm_inv, a.act) * (row_sum(2 * pr + 1, row) * nrm_inv);
+        resolve_tile(a, gt + rt, j, r0);
+        const float v = gate_act(row_sum(rt, row) * nrm_inv, a.act) * (row_sum(rt, row + 8) * nrm_inv);
         a.out[0][r0 + row] = v;
         if (TP && tp.peer[0][0]) st_slots(tp.peer[0], tp.world, (size_t)(tag & 1u) * a.n[0] * tp.world + (size_t)tp.rank * a.n[0] + r0 + row, v, tag);
       }
@@ -1916,8 +1935,8 @@ static int q4k_launch(const float *x, const MultiArgs &a, const TpArgs &tp, int 
   const bool two = (g_q4k_stages == 2 || deep > MAX_DYN_SMEM) && flat <= MAX_DYN_SMEM;
   const size_t dyn = two ? flat : deep;
   if (dyn > MOST_DYN_SMEM) return 0;
-  const int lt = a.act ? tiles / 2 : tiles, per_sm = dyn > MAX_DYN_SMEM ? 1 : g_waves;
-  const unsigned grid = (unsigned)(lt < g_sms * per_sm ? lt : g_sms * per_sm);
+  const int per_sm = dyn > MAX_DYN_SMEM ? 1 : g_waves;
+  const unsigned grid = (unsigned)(tiles < g_sms * per_sm ? tiles : g_sms * per_sm);
   auto go = [&](auto kern) { return launch_pdl(kern, grid, dyn, st, x, a, tp, nrm, tiles, K); };
   int rc = nrm.weight ? (two ? go(q4k_gemv_mma_kernel<2, false, true>) : go(q4k_gemv_mma_kernel<4, false, true>))
            : tp.step  ? (two ? go(q4k_gemv_mma_kernel<2, true>) : go(q4k_gemv_mma_kernel<4, true>))
@@ -2174,6 +2193,7 @@ int gguf_gemv_multi(int type, const float *x, const void *const *w, float *const
     a.w[i] = (const uint8_t *)w[i], a.out[i] = out[i], a.n[i] = n[i], a.tend[i] = tiles;
   }
   a.count = count, a.act = act;
+  if (act) tiles = (n[0] + ROWS / 2 - 1) / (ROWS / 2);
   return q4k_launch(x, a, NO_TP, tiles, K, st, nrm);
 }
 
