@@ -87,6 +87,8 @@ int gguf_gemv_multi(int type, const float *x, const void *const *w, float *const
 int gguf_gemv_batch(int type, const float *x, const void *w, float *out, int M, int N, int K, cudaStream_t st);
 // tensor-core prefill: 1 = took the call, 0 = shape / workspace not covered, other = error
 int gguf_prefill(int type, const float *x, const void *w, float *out, int M, int N, int K, int device, cudaStream_t st);
+int int4_narrow_tmem(const void *x, const uint32_t *codes, const float *s, const float *z, void *y, int act_dtype, int M, int N, int K, int G, int device,
+                     cudaStream_t st);
 int int4_prefill(const void *x, const uint32_t *codes, const float *s, const float *z, void *y, int act_dtype, int M, int N,
                  int K, int G, int device, cudaStream_t st);
 int fp8_prefill(const void *x, const uint8_t *w, const float *scale, void *y, int act_dtype, int M, int N, int K, int bR,
@@ -141,8 +143,9 @@ struct TmemCall {
   const void *w;            // packed weights (E, N, K)
   const float *s, *z;       // scales (INT4, FP8) and zeros (INT4)
   int G, bR, bC;            // group (INT4); scale block (FP8)
-  const void *x16;          // (M, K) tokens at the operand type: bf16 (then the output is bf16) or f16 (f32)
+  const void *x16;          // (M, K) tokens at the operand type: bf16 (then the output is bf16) or f16 (f32, or bf16 with out_bf16)
   bool bf16;
+  bool out_bf16;            // INT4 with f16 operands: the output is bf16 all the same
   void *out;
   long long M;
   int N, K;

@@ -862,6 +862,7 @@ int gemm_tmem(const TmemCall &c, cudaStream_t st) {
     case TmemCall::Q80: return pick<TmQ80, false, float>({(const uint8_t *)c.w}, c, st);
     case TmemCall::INT4: {
       const TmInt4::Ctx x{(const uint32_t *)c.w, c.s, c.z, c.G, Div::of(c.G / 64)};
+      if (c.out_bf16) return pick<TmInt4, false, __nv_bfloat16>(x, c, st);
       return c.bf16 ? pick<TmInt4, true, __nv_bfloat16>(x, c, st) : pick<TmInt4, false, float>(x, c, st);
     }
     case TmemCall::FP8: {

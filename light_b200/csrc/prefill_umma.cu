@@ -737,6 +737,21 @@ __global__ void __launch_bounds__(256) x_to_f16_kernel(const float4 *__restrict_
   }
 }
 
+// x bf16 -> f16 as the token-tile decode kernels stage it: exact but for values outside f16's range, which are clamped (or
+// fall among its subnormals).
+__global__ void __launch_bounds__(256) x_bf16_to_f16_kernel(const uint4 *__restrict__ x, uint4 *__restrict__ y, int n8) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n8) return;
+  const uint4 v = __ldg(x + i);
+  auto two = [](uint32_t w) {
+    const float lo = __uint_as_float(w << 16), hi = __uint_as_float(w & 0xFFFF0000u);
+    return pack_h2(fminf(fmaxf(lo, -65504.f), 65504.f), fminf(fmaxf(hi, -65504.f), 65504.f));
+  };
+  y[i] = make_uint4(two(v.x), two(v.y), two(v.z), two(v.w));
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1035,6 +1050,30 @@ int int4_prefill(const void *x, const uint32_t *codes, const float *s, const flo
   Int4Ctx ctx{codes, s, z, G};
   int rc = launch_by_act<Int4Row>(x, act_dtype, ctx, y, M, N, K, ws, wsb, st);
   return rc ? rc : 1;
+}
+
+// 17 to 64 bf16 rows of a 4-bit matrix: the tensor-memory kernel with the operands of the token-tile decode kernel (f16
+// weights (code - zero) * scale, here with one rounding where that kernel rounds the scale as well; x as f16), bf16 out.
+// That kernel's instructions grow with the tokens, this one's do not.  Device time with a cold L2, 28672 x 4096: 32 rows
+// 51.9 -> 44.0 us, 64 rows 73.6 -> 46.3; 4096 x 14336: 36.8 -> 30.4, 46.1 -> 34.4; 2560 x 4096: 21.9 -> 19.5, 23.6 -> 21.5.
+// At 16 rows the two are even, and at 2048 x 4096 and below the token tiles are: hence the lines.
+int int4_narrow_tmem(const void *x, const uint32_t *codes, const float *s, const float *z, void *y, int act_dtype, int M, int N, int K, int G, int device,
+                     cudaStream_t st) {
+  static const int min_m = getenv("LIGHT_B200_TMEM_INT4_MIN_M") ? atoi(getenv("LIGHT_B200_TMEM_INT4_MIN_M")) : 17;
+  if (act_dtype != LB200_BF16 || M < min_m || M > 64 || (long long)N * K < (10ll << 20) || K % 256 || G % 64 || ((uintptr_t)codes & 15) || ((uintptr_t)x & 15) ||
+      !use_tmem())
+    return 0;
+  void *ws;
+  size_t wsb;
+  const size_t x_bytes = ((size_t)M * K * 2 + 1023) & ~(size_t)1023;
+  if (!get_ws(device, LB200_F32, M, K, &ws, &wsb) || wsb < x_bytes + gemm_tmem_parts_bytes()) return 0;
+  const int n8 = (int)((long long)M * K / 8);
+  launch_early(x_bf16_to_f16_kernel, dim3((unsigned)((n8 + 255) / 256)), dim3(256), st, (const uint4 *)x, (uint4 *)ws, n8);
+  if (int rc = launched("int4: activations to f16")) return rc;
+  TmemCall c = tmem_call<Int4Row>(Int4Ctx{codes, s, z, G});
+  c.x16 = ws, c.out_bf16 = true, c.out = y, c.M = M, c.N = N, c.K = K;
+  c.mean_tokens = M, c.min_run_k = tmem_min_run(), c.parts = (char *)ws + x_bytes, c.parts_bytes = wsb - x_bytes;
+  return gemm_tmem(c, st);
 }
 
 int fp8_prefill(const void *x, const uint8_t *w, const float *scale, void *y, int act_dtype, int M, int N, int K, int bR,

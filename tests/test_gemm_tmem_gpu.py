@@ -68,3 +68,17 @@ def test_grouped_q6_k_rows_at_odd_offsets(cuda):
     y = ops.MoEGemmQ(x, q, r, None, topk)
     want = torch.einsum("mk,mnk->mn", x.double().repeat_interleave(topk, 0), w[ids.reshape(-1)])
     assert rel_l2(y.cpu().double().numpy(), want.cpu().numpy()) <= 1e-3
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 4096, 4096), (33, 8196, 2048), (48, 732, 14336), (64, 40964, 256)])
+def test_narrow_int4(cuda, M, N, K):
+    """17 to 64 bf16 rows of a 4-bit matrix of 10 * 2^20 weights or more: f16 operands (2^-12 each on average), then the bf16 output's
+    rounding, 2^-9 of a value at most."""
+    g = torch.Generator(device=cuda).manual_seed(N)
+    w = ops.Int4(torch.randint(-2**31, 2**31, (N, K // 8), generator=g, device=cuda, dtype=torch.int32), torch.rand(N, K // 64, generator=g, device=cuda) * 0.02,
+                 torch.randint(0, 31, (N, K // 64), generator=g, device=cuda).float() / 2, 64)
+    x = torch.randn(M, K, generator=g, device=cuda).bfloat16()
+    y = ops.MatMulInt4(x, w)
+    assert torch.equal(y, ops.MatMulInt4(x, w)) and ops.prefill_status(0) == 0
+    want = x.double() @ ops.DequantizeInt4(w, torch.float32).double().t()
+    assert rel_l2(y.cpu().double().numpy(), want.cpu().numpy()) <= 2.5e-3
