@@ -2148,7 +2148,7 @@ int gguf_decode_tile(int type, const float *x, const void *w, float *out, int M,
 
 // 2 .. 32 activation rows against up to four Q4_K matrices that share them (q, k, v; gate, up), one launch:
 // ops.LinearMulti for a small batch (the token-column kernel up to 8 rows, the eight-tiles-per-CTA kernel above:
-// q,k,v of configs[1] at 32 rows 23.4 us merged against 32.9 us as three launches; gate,up the same either way).  Returns 1 if launched, 0 if the shape is not covered.
+// q,k,v of an 8B layer at 32 rows 23.4 us merged against 32.9 us as three launches; gate,up the same either way).  Returns 1 if launched, 0 if the shape is not covered.
 int gguf_gemv_tok_multi(int type, const float *x, const void *const *w, float *const *out, const int *n, int count, int M, int K,
                         cudaStream_t st) {
   static int tile_multi = -1;  // LIGHT_B200_TILE_MULTI=0 (tuning knob): merge only up to 8 rows
