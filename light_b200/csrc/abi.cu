@@ -212,6 +212,7 @@ int light_b200_matmul_q(int t, const float *x, const void *w, float *out, int M,
   if (took != 0) return took == 1 ? 0 : took;
   took = gguf_gemv_batch(t, x, w, out, M, N, K, st);
   if (took != 0) return took == 1 ? 0 : took;
+  if (t == LB200_Q6_K && M > 64 && K % 256 == 0) return q6k_rows_dense(x, w, out, M, N, K, st);  // rows off 4-byte boundaries, or no workspace
   return gguf_matmul_generic(t, x, w, out, M, N, K, st);
 }
 

@@ -116,6 +116,8 @@ int fp8_block_rows_dot(const void *x, const uint8_t *w, const float *s, void *y,
                        cudaStream_t st);
 int moe_gemm(const lb200_moe_args *a, int device, cudaStream_t st);
 int moe_gemm_q(const lb200_moe_args *a, int device, cudaStream_t st);
+// Q6_K rows that start on any even byte, many activation rows: f32 products (moe.cu)
+int q6k_rows_dense(const float *x, const void *w, float *out, int M, int N, int K, cudaStream_t st);
 int moe_gemm_f8block(const lb200_moe_args *a, const float *w_scale, int bR, int bC, int device, cudaStream_t st);
 int moe_umma(const lb200_moe_args *a, int kind, const float *w_scale, int bR, int bC, int device, cudaStream_t st);
 int moe_clear_unrouted(const int64_t *pairs, const int64_t *ids, uint32_t *bits, void *out, long long M, long long rows, long long row_bytes, int E,

@@ -253,6 +253,119 @@ int moe_clear_unrouted(const int64_t *pairs, const int64_t *ids, uint32_t *bits,
   return launched("moe: clear unrouted rows");
 }
 
+// ------------------------------------------------------------------------------------ Q6_K rows that start on any even byte
+//
+// An odd number of 210-byte blocks per row: the tensor-core kernels would round both operands to 11 bits, and these rows have always had
+// f32 products, as below 256 pairs.  What bounds moe_gemm_kernel is the load unit: a warp to one weight row reads eight activation rows
+// for every eight weights, and the weights a byte at a time.  Here a warp owns NC rows of one expert and MT of its tokens: an
+// activation is loaded once for NC weights, a weight once for MT tokens, in 16-bit pieces.  Lanes split K, and the NC x MT sums end
+// in a reduce-scatter over the warp (31 shuffles for 32 sums, not 160).  616 pairs over 128 experts of 2048 x 768: 780 -> 245 us;
+// 2048 rows of 4096 x 14080: 42 -> 16 ms.
+// Elements 4 lane .. + 3 of both halves of a block: sixteen bytes of activations to a lane are then whole lines to a warp.
+__device__ __forceinline__ void q6k_eight(const uint8_t *b, int lane, float out[8]) {
+  const int grp = lane >> 3, l0 = 4 * (lane & 7);
+  const uint8_t *ql = b + (grp & 1) * 32 + l0, *qh = b + 128 + l0;
+  const float d = f16_bits_to_f32(__ldg(reinterpret_cast<const uint16_t *>(b + 208)));
+  auto word = [](const uint8_t *p) { return (uint32_t)__ldg(reinterpret_cast<const uint16_t *>(p)) | (uint32_t)__ldg(reinterpret_cast<const uint16_t *>(p) + 1) << 16; };
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const float ds = __fmul_rn(d, (float)__ldg(reinterpret_cast<const int8_t *>(b) + 192 + 8 * h + 2 * grp + (l0 >> 4)));
+    const uint32_t q = ((word(ql + 64 * h) >> (grp >> 1 ? 4 : 0)) & 0x0F0F0F0Fu) | ((word(qh + 32 * h) >> (2 * grp)) & 0x03030303u) << 4;
+#pragma unroll
+    for (int i = 0; i < 4; i++)  // 2^23 + code, less 2^23 + 32: exact
+      out[4 * h + i] = __fmul_rn(ds, __uint_as_float(__byte_perm(q, 0x4B000000u, 0x7440 + i)) - 8388640.f);
+  }
+}
+
+// CHAIN: a lane's products one after the other into its sum, as moe_gemm_kernel adds them; else eight at a time, as the shape-generic
+// matmul does (K = 14080: 1.6e-7 of the result against 3.8e-7).
+template <int NC, int MT, bool CHAIN>
+__global__ void __launch_bounds__(MOE_WARPS * 32, 2) q6k_rows_kernel(const float *__restrict__ in, const uint8_t *__restrict__ w, const int64_t *__restrict__ pairs,
+                                                                 const int32_t *__restrict__ offsets, const float *__restrict__ topkw, float *__restrict__ out,
+                                                                 long long M, long long size_m, int N, int K, int topk, int row_per_pair) {
+  static_assert(NC * MT % 32 == 0 && MT <= 32, "a lane per token, whole sums per lane");
+  const int lane = threadIdx.x & 31, n0 = (blockIdx.x * MOE_WARPS + (threadIdx.x >> 5)) * NC, e = blockIdx.y;
+  if (n0 >= N) return;
+  const size_t row_bytes = (size_t)(K >> 8) * 210;
+  const uint8_t *row[NC];
+#pragma unroll
+  for (int c = 0; c < NC; c++) row[c] = w + ((size_t)e * N + min(n0 + c, N - 1)) * row_bytes;
+  const long long i0 = offsets ? offsets[e] : 0, i1 = offsets ? offsets[e + 1] : M;
+  for (long long t = i0 + (long long)blockIdx.z * MT; t < i1; t += (long long)gridDim.z * MT) {
+    const int cnt = (int)min((long long)MT, i1 - t);
+    long long mine = -1;  // the pair of token `lane`
+    if (lane < cnt) {
+      mine = pairs ? pairs[t + lane] : t + lane;
+      if (mine < 0 || mine >= size_m) mine = -1;
+    }
+    const long long from = mine < 0 ? 0 : row_per_pair ? mine : mine / topk;
+    const float *x[MT];
+#pragma unroll
+    for (int m = 0; m < MT; m++) x[m] = in + (size_t)__shfl_sync(0xffffffffu, from, m) * K;
+    float acc[NC * MT];
+#pragma unroll
+    for (int i = 0; i < NC * MT; i++) acc[i] = 0.f;
+    for (int b = 0; b < K >> 8; b++) {
+      float wv[NC][8];
+#pragma unroll
+      for (int c = 0; c < NC; c++) q6k_eight(row[c] + b * 210, lane, wv[c]);
+#pragma unroll
+      for (int m = 0; m < MT; m++) {  // (a missing token reads row 0: with branches here the loads would wait for one another)
+        const float4 *xp = reinterpret_cast<const float4 *>(x[m] + b * 256) + lane;
+        const float4 u = __ldg(xp), v = __ldg(xp + 32);
+        const float xv[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+          if constexpr (CHAIN) {
+#pragma unroll
+            for (int j = 0; j < 8; j++) acc[m * NC + c] = fmaf(wv[c][j], xv[j], acc[m * NC + c]);
+          } else {
+            float s = wv[c][0] * xv[0];
+#pragma unroll
+            for (int j = 1; j < 8; j++) s = fmaf(wv[c][j], xv[j], s);
+            acc[m * NC + c] += s;
+          }
+        }
+      }
+    }
+    // Sum i of NC MT: a lane hands half of its sums to its partner at every step and keeps the other half.
+    int base = 0;  // of the sums this lane still holds
+#pragma unroll
+    for (int off = 16, n = NC * MT / 2; off >= 1; off >>= 1, n /= 2) {
+      const bool up = lane & off;
+#pragma unroll
+      for (int i = 0; i < NC * MT / 2; i++) {
+        if (i < n) {
+          const float send = up ? acc[i] : acc[i + n], keep = up ? acc[i + n] : acc[i];
+          acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+      }
+      if (up) base += n;
+    }
+#pragma unroll
+    for (int i = 0; i < NC * MT / 32; i++) {
+      const int m = (base + i) / NC, n = n0 + (base + i) % NC;
+      const long long p = __shfl_sync(0xffffffffu, mine, m);
+      if (p >= 0 && n < N) out[p * N + n] = topkw ? acc[i] * topkw[p] : acc[i];
+    }
+  }
+}
+
+template <bool CHAIN>
+static int q6k_rows(const float *in, const void *w, const int64_t *pairs, const int32_t *offsets, const float *topkw, float *out, long long M, long long size_m,
+                    int E, int N, int K, int topk, int row_per_pair, cudaStream_t st) {
+  constexpr int NC = 4, MT = 8;
+  const long long nb = (N + NC * MOE_WARPS - 1) / (NC * MOE_WARPS), tiles = (M + MT - 1) / MT, want = (8ll * sm_count() + nb * E - 1) / (nb * E);
+  const unsigned z = (unsigned)(want < tiles ? want : tiles);  // CTAs that share an expert's tokens, where experts and rows alone do not fill the GPU
+  q6k_rows_kernel<NC, MT, CHAIN><<<dim3((unsigned)nb, (unsigned)E, z), MOE_WARPS * 32, 0, st>>>(in, (const uint8_t *)w, pairs, offsets, topkw, out, M, size_m, N, K, topk,
+                                                                                     row_per_pair);
+  return launched("q6_k rows (f32)");
+}
+
+int q6k_rows_dense(const float *x, const void *w, float *out, int M, int N, int K, cudaStream_t st) {
+  return q6k_rows<false>(x, w, nullptr, nullptr, nullptr, out, M, M, 1, N, K, 1, 1, st);
+}
+
 template <typename TI, typename TO, typename Row>
 static int run(const lb200_moe_args *a, cudaStream_t st, RowAux aux = RowAux{nullptr, 0, 0, nullptr}) {
   if (a->M == 0 || a->N == 0) return 0;
@@ -362,6 +475,10 @@ int moe_gemm_q(const lb200_moe_args *a, int device, cudaStream_t st) {
   int rc = prep(a, st);
   if (rc) return rc;
   if (int took = moe_umma(a, 1, nullptr, 0, 0, device, st)) return took == 1 ? 0 : took;
+  // From as many pairs on as the tensor-core path takes of the other formats.
+  if (a->dtype == LB200_Q6_K && a->M >= 256 && a->K % 256 == 0 && a->E <= 65535 && a->N > 0)
+    return q6k_rows<true>((const float *)a->input, a->weights, a->sorted_pairs, a->offsets, a->topk_weights, (float *)a->out, a->M, a->size_m, a->E, a->N, a->K,
+                       a->topk, a->row_per_pair, st);
   switch (a->dtype) {
     case LB200_Q4_0: return run<float, float, QuantRow<LB200_Q4_0>>(a, st);
     case LB200_Q5_0: return run<float, float, QuantRow<LB200_Q5_0>>(a, st);

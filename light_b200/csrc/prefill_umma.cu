@@ -1019,12 +1019,12 @@ int gguf_prefill(int type, const float *x, const void *w, float *out, int M, int
   static const int q80_min = getenv("LIGHT_B200_TMEM_Q80_MIN_M") ? atoi(getenv("LIGHT_B200_TMEM_Q80_MIN_M")) : Q80_TMEM_MIN_M;
   const bool narrow = M < PREFILL_MIN_M;
   if ((narrow && !(type == LB200_Q8_0 && M >= q80_min && use_tmem())) || K % 256) return 0;
-  bool older = !narrow;
   if (type == LB200_Q4_K) {
     if ((uintptr_t)w & 15) return 0;
   } else if (type == LB200_Q6_K) {
-    older = !((uintptr_t)w & 3) && (K >> 8) % 2 == 0;  // (the older kernel wants rows that start 4-byte aligned)
-    if (!older && !use_tmem()) return 0;
+    // Rows that start 4-byte aligned only: the others belong to the shape-generic kernel, which multiplies f32 weights by f32
+    // activations, and f16 operands would take that precision from them.
+    if (((uintptr_t)w & 3) || (K >> 8) % 2) return 0;
   } else if (type == LB200_Q8_0) {
     if ((uintptr_t)w & 15) return 0;  // K % 256 == 0 makes every row a whole number of 16-byte granules
   } else {
@@ -1035,8 +1035,8 @@ int gguf_prefill(int type, const float *x, const void *w, float *out, int M, int
   if (!get_ws(device, LB200_F32, M, K, &ws, &wsb)) return 0;
   GgufCtx ctx{(const uint8_t *)w};
   int rc = type == LB200_Q4_K   ? launch_by_act<Q4KRow>(x, LB200_F32, ctx, out, M, N, K, ws, wsb, st)
-           : type == LB200_Q6_K ? launch_by_act<Q6KRow>(x, LB200_F32, ctx, out, M, N, K, ws, wsb, st, older)
-                                : launch_by_act<Q80Row>(x, LB200_F32, ctx, out, M, N, K, ws, wsb, st, older);
+           : type == LB200_Q6_K ? launch_by_act<Q6KRow>(x, LB200_F32, ctx, out, M, N, K, ws, wsb, st)
+                                : launch_by_act<Q80Row>(x, LB200_F32, ctx, out, M, N, K, ws, wsb, st, !narrow);
   if (rc == NOT_COVERED) return 0;
   return rc ? rc : 1;
 }
@@ -1176,8 +1176,8 @@ int moe_umma(const lb200_moe_args *a, int kind, const float *w_scale, int bR, in
     if (a->K % 256) return 0;
     if (a->dtype == LB200_Q4_K)
       rc = moe_launch<Q4KRow, false, float, float>(a, GgufCtx{(const uint8_t *)a->weights}, ws, wsb, st);
-    else if (a->dtype == LB200_Q6_K)  // (the older kernel wants rows that start 4-byte aligned)
-      rc = moe_launch<Q6KRow, false, float, float>(a, GgufCtx{(const uint8_t *)a->weights}, ws, wsb, st, (a->K >> 8) % 2 == 0);
+    else if (a->dtype == LB200_Q6_K && (a->K >> 8) % 2 == 0)  // (others keep their f32 products, as in gguf_prefill)
+      rc = moe_launch<Q6KRow, false, float, float>(a, GgufCtx{(const uint8_t *)a->weights}, ws, wsb, st);
     else if (a->dtype == LB200_Q8_0 && !((uintptr_t)a->weights & 15))
       rc = moe_launch<Q80Row, false, float, float>(a, GgufCtx{(const uint8_t *)a->weights}, ws, wsb, st);
     else

@@ -1,0 +1,33 @@
+"""Calls whose operands are multiplied as they are stay that way, whichever kernel takes the larger or better aligned ones of the same
+format.
+
+Bounds: a product of f32 values summed in f32 over K terms is off by at most about K / 2 * 2^-24 of the sum of magnitudes and by
+sqrt(K) * 2^-24 on average, below 1e-5 here; operands rounded to f16 give 2^-12 each, 3e-4 on the result."""
+import pytest
+import torch
+
+from helpers import rel_l2
+from light_b200 import ops, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K", [(65, 132, 256), (333, 300, 768), (1100, 128, 1280)])
+def test_q6_k_with_an_odd_number_of_blocks_per_row(cuda, M, N, K):
+    w = ops.QTensor(synth.gaussian_weight(N, ops.Q6_K, N, K, device=cuda).reshape(-1), ops.Q6_K, (N, K))
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(cuda)
+    want = x.double() @ ops.Dequantize(w).double().t()
+    assert rel_l2(ops.MatMulQ(x, w).cpu().double().numpy(), want.cpu().numpy()) <= 1e-5
+
+
+@pytest.mark.parametrize("M", [100, 333])   # 200 and 666 pairs
+def test_grouped_q6_k_with_an_odd_number_of_blocks_per_row(cuda, M):
+    E, N, K, topk = 5, 260, 768, 2
+    q = ops.QTensor(synth.gaussian_weight(3, ops.Q6_K, E * N, K, device=cuda).reshape(-1), ops.Q6_K, (E, N, K))
+    w = ops.Dequantize(q).double().reshape(E, N, K)
+    g = torch.Generator().manual_seed(5)
+    x = torch.randn(M, K, generator=g).to(cuda)
+    ids = torch.randint(0, E, (M, topk), generator=g).to(cuda)
+    r = ops.MoERouteFromIDs(ids, torch.ones(M * topk, device=cuda), M, topk)
+    want = torch.einsum("mk,mnk->mn", x.double().repeat_interleave(topk, 0), w[ids.reshape(-1)])
+    assert rel_l2(ops.MoEGemmQ(x, q, r, None, topk).cpu().double().numpy(), want.cpu().numpy()) <= 1e-5
