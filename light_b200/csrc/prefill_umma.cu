@@ -1060,7 +1060,9 @@ int int4_prefill(const void *x, const uint32_t *codes, const float *s, const flo
 int int4_narrow_tmem(const void *x, const uint32_t *codes, const float *s, const float *z, void *y, int act_dtype, int M, int N, int K, int G, int device,
                      cudaStream_t st) {
   static const int min_m = getenv("LIGHT_B200_TMEM_INT4_MIN_M") ? atoi(getenv("LIGHT_B200_TMEM_INT4_MIN_M")) : 17;
-  if (act_dtype != LB200_BF16 || M < min_m || M > 64 || (long long)N * K < (10ll << 20) || K % 256 || G % 64 || ((uintptr_t)codes & 15) || ((uintptr_t)x & 15) ||
+  // Groups of 128 only, whose token-tile kernel rounds x to f16 as well: the kernel that has other groups multiplies bf16 x as it is,
+  // and f16 would clamp values beyond 65504 and lose bits of those below 6e-5.
+  if (act_dtype != LB200_BF16 || M < min_m || M > 64 || (long long)N * K < (10ll << 20) || K % 256 || G != 128 || ((uintptr_t)codes & 15) || ((uintptr_t)x & 15) ||
       !use_tmem())
     return 0;
   void *ws;

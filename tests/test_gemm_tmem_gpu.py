@@ -82,3 +82,16 @@ def test_narrow_int4(cuda, M, N, K):
     assert torch.equal(y, ops.MatMulInt4(x, w)) and ops.prefill_status(0) == 0
     want = x.double() @ ops.DequantizeInt4(w, torch.float32).double().t()
     assert rel_l2(y.cpu().double().numpy(), want.cpu().numpy()) <= 2.5e-3
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 4096, 4096), (33, 8196, 2048), (48, 732, 14336), (64, 40964, 256)])
+def test_narrow_int4_in_groups_of_128(cuda, M, N, K):
+    """As test_narrow_int4, for the groups whose 17 to 64 rows this kernel has."""
+    g = torch.Generator(device=cuda).manual_seed(N)
+    w = ops.Int4(torch.randint(-2**31, 2**31, (N, K // 8), generator=g, device=cuda, dtype=torch.int32), torch.rand(N, K // 128, generator=g, device=cuda) * 0.02,
+                 torch.randint(0, 31, (N, K // 128), generator=g, device=cuda).float() / 2, 128)
+    x = torch.randn(M, K, generator=g, device=cuda).bfloat16()
+    y = ops.MatMulInt4(x, w)
+    assert torch.equal(y, ops.MatMulInt4(x, w)) and ops.prefill_status(0) == 0
+    want = x.double() @ ops.DequantizeInt4(w, torch.float32).double().t()
+    assert rel_l2(y.cpu().double().numpy(), want.cpu().numpy()) <= 2.5e-3

@@ -31,3 +31,17 @@ def test_grouped_q6_k_with_an_odd_number_of_blocks_per_row(cuda, M):
     r = ops.MoERouteFromIDs(ids, torch.ones(M * topk, device=cuda), M, topk)
     want = torch.einsum("mk,mnk->mn", x.double().repeat_interleave(topk, 0), w[ids.reshape(-1)])
     assert rel_l2(ops.MoEGemmQ(x, q, r, None, topk).cpu().double().numpy(), want.cpu().numpy()) <= 1e-5
+
+
+@pytest.mark.parametrize("G", [64, 256])
+@pytest.mark.parametrize("scale", [1e-6, 3e4])
+def test_int4_rows_beyond_f16(cuda, G, scale):
+    """17 to 64 bf16 rows of a 4-bit matrix whose groups are not 128: x is multiplied as bf16, whatever its range.  bf16 weights (2^-9 of a
+    weight at most, 1.1e-3 on average) and the bf16 output's rounding (the same) remain."""
+    M, N, K = 33, 4096, 4096
+    g = torch.Generator(device=cuda).manual_seed(G)
+    w = ops.Int4(torch.randint(-2**31, 2**31, (N, K // 8), generator=g, device=cuda, dtype=torch.int32), torch.rand(N, K // G, generator=g, device=cuda) * 0.02,
+                 torch.randint(0, 16, (N, K // G), generator=g, device=cuda).float(), G)
+    x = (torch.randn(M, K, generator=g, device=cuda) * scale).bfloat16()
+    want = x.double() @ ops.DequantizeInt4(w, torch.float32).double().t()
+    assert rel_l2(ops.MatMulInt4(x, w).cpu().double().numpy(), want.cpu().numpy()) <= 2.5e-3
