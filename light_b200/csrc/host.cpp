@@ -2,13 +2,16 @@
 // stream, C-ABI call.  A decode step's kernels run for 5 to 20 us; the same work in Python (ctypes argument boxing, tensor
 // attribute look-ups, torch.empty) costs 12 to 20 us per operator and leaves the GPU idle between them, here 4 to 6 us.
 //
-// Every function returns None when its arguments are not the common form (another type, layout or device, an error, a
-// workspace that has to grow first); the caller in ops.py / nn.py then takes the general path, which handles or rejects
-// them with the reference's messages.  Nothing is checked less: a call that succeeds here satisfies what that path checks.
+// Every function returns None when its arguments are not the common form (another type, layout or device, an error of the
+// library's, a workspace that has to grow first); the caller in ops.py / nn.py then takes the general path, which handles or
+// rejects them with the reference's messages.  Nothing is checked less: a call that succeeds here satisfies what that path
+// checks.  What torch throws on the way (no memory for the output, a tensor without storage) becomes the Python exception
+// that the same call raises from Python.
 #include <Python.h>
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <atomic>
@@ -258,7 +261,13 @@ PyObject *moe_gemm(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
   return give(type >= 0 ? light_b200_moe_gemm_q(&m, dev, st) : light_b200_moe_gemm_f8block(&m, s.t->const_data_ptr<float>(), (int)bR, (int)bC, dev, st), out);
 }
 
-#define FN(f, doc) {#f, (PyCFunction)(void (*)(void))f, METH_FASTCALL, doc}
+template <PyObject *(*F)(PyObject *, PyObject *const *, Py_ssize_t)>
+PyObject *guarded(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  return F(self, a, nargs);
+  END_HANDLE_TH_ERRORS
+}
+#define FN(f, doc) {#f, (PyCFunction)(void (*)(void))guarded<f>, METH_FASTCALL, doc}
 PyMethodDef kMethods[] = {FN(set_workspace, "registers a device's workspace size"),
                           FN(linear_q, "x . W^T, GGUF blocks"),
                           FN(linear_int4, "x . W^T, 4-bit groups"),

@@ -1,0 +1,41 @@
+"""The native host path of the hot operators under conditions that a server has to survive."""
+import pytest
+import torch
+
+from light_b200 import ops, synth
+from light_b200.nn import Linear
+
+pytestmark = pytest.mark.gpu
+
+
+def _calls(dev):
+    """Calls whose outputs are 64 MB or more each."""
+    M, K, N = 4096, 256, 4096
+    ops.ensure_workspace(0, 256 << 20)
+    x = torch.ones(M, K, device=dev)
+    lin = Linear(K, N, W=ops.QTensor(synth.gaussian_weight(1, ops.Q4_K, N, K, device=dev).reshape(-1), ops.Q4_K, (N, K)))
+    w4 = ops.Int4(torch.zeros(2 * N, K // 8, dtype=torch.int32, device=dev), torch.ones(2 * N, 2, device=dev), torch.zeros(2 * N, 2, device=dev), 128)
+    codes, scale = synth.random_fp8_block(1, 2 * N, K, device=dev)
+    h = torch.ones(4096, 8192, device=dev)
+    ids = torch.zeros(M, 1, dtype=torch.int64, device=dev)
+    r = ops.MoERouteFromIDs(ids, torch.ones(M, device=dev), M, 1)
+    b = x.bfloat16()
+    return {"linear_q": lambda: lin.forward(x), "linear_int4": lambda: ops.MatMulInt4(b, w4), "linear_f8": lambda: ops.MatMulF8Block(b, codes, scale, 128, 128),
+            "gate_mul": lambda: ops.MoEGateMul(h), "combine": lambda: ops.MoECombine(h, 2),
+            "moe_gemm": lambda: ops.MoEGemmF8Block(b, codes.reshape(1, 2 * N, K), scale.reshape(1, 2 * N // 128, K // 128), 128, 128, r, None, 1)}
+
+
+@pytest.mark.parametrize("name", ["linear_q", "linear_int4", "linear_f8", "gate_mul", "combine", "moe_gemm"])
+def test_no_memory_for_the_output_is_an_exception(cuda, name):
+    """torch.OutOfMemoryError, which a server can catch, and the same call runs once there is memory."""
+    call = _calls(cuda)[name]
+    want = call().clone()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.set_per_process_memory_fraction(1e-4)   # the caching allocator refuses to grow: nothing is exhausted
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            call(), call()                              # (one may still fit into a block that is cached)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(call(), want)
