@@ -34,8 +34,9 @@ struct Arg {
 bool cuda_contig(const at::Tensor &t) { return t.is_cuda() && t.is_contiguous() && !t.requires_grad(); }
 bool long_of(PyObject *o, long long &v) {
   if (!PyLong_Check(o)) return false;
-  v = PyLong_AsLongLong(o);
-  return !(v == -1 && PyErr_Occurred());
+  int overflow;
+  v = PyLong_AsLongLongAndOverflow(o, &overflow);  // (no Python error is set: the caller answers None)
+  return !overflow;
 }
 void *stream_of(int dev) { return (void *)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream(); }
 bool workspace_fits(int dev, long long M, long long K) {
@@ -73,7 +74,10 @@ bool rows_of(const at::Tensor &x, long long K, long long &M) {
 PyObject *set_workspace(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
   ARGS(2)
   long long dev, n;
-  if (!long_of(a[0], dev) || !long_of(a[1], n) || dev < 0 || dev >= 64) return nullptr;
+  if (!long_of(a[0], dev) || !long_of(a[1], n) || dev < 0 || dev >= 64) {
+    PyErr_SetString(PyExc_ValueError, "set_workspace: a device of 0 .. 63 and a size in bytes");
+    return nullptr;
+  }
   g_ws[dev].store((unsigned long long)n, std::memory_order_relaxed);
   Py_RETURN_NONE;
 }
@@ -134,6 +138,7 @@ PyObject *gate_mul(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
   Arg h;
   NEED(h.ok(a[0]) && h.t->dim() == 2 && cuda_contig(*h.t) && act_of(*h.t) >= 0 && h.t->size(1) % 16 == 0 && h.t->numel() > 0);
   const int gelu = PyObject_IsTrue(a[1]), dev = h.t->get_device();
+  if (gelu < 0) return nullptr;
   at::Tensor out = at::empty({h.t->size(0), h.t->size(1) / 2}, h.t->options());
   return give(light_b200_moe_gate_mul(h.t->const_data_ptr(), out.data_ptr(), act_of(*h.t), h.t->size(0), (int)(h.t->size(1) / 2), gelu, dev, stream_of(dev)), out);
 }
@@ -206,6 +211,7 @@ PyObject *moe_route(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
   long long topk;
   NEED(x.ok(a[0]) && long_of(a[2], topk) && cuda_contig(*x.t) && x.t->dim() == 2 && x.t->scalar_type() == at::kFloat && x.t->numel() > 0);
   const int dev = x.t->get_device(), norm = PyObject_IsTrue(a[3]), sigmoid = PyObject_IsTrue(a[4]);
+  if (norm < 0 || sigmoid < 0) return nullptr;
   const int64_t T = x.t->size(0), E = x.t->size(1);
   NEED(topk >= 1 && topk <= E && topk <= 32 && E <= 1024 && T * topk < (1ll << 31));
   if (a[1] != Py_None)

@@ -48,3 +48,21 @@ with FakeTensorMode():
         raise SystemExit(name + ": no exception")
 print("CASE OK")
 """)
+
+
+def test_numbers_beyond_64_bits_are_not_the_common_form():
+    """None, and no Python error left behind (which made it a SystemError)."""
+    import pytest
+    import torch
+
+    from light_b200 import ops
+
+    x, u8, big = torch.zeros(1, 256), torch.zeros(144, dtype=torch.uint8), 2**70
+    assert ops._host.linear_q(x, u8, ops.Q4_K, big, 256) is None
+    assert ops._host.linear_int4(x, x, x, x, big) is None
+    assert ops._host.linear_f8(x, x, x, -big, 1) is None
+    assert ops._host.combine(x, big) is None
+    assert ops._host.moe_route(x, None, big, True, True) is None
+    assert ops._host.decode_attention(x, x, x, x, 1.0, big, None, None, 0.0) is None
+    with pytest.raises(ValueError):
+        ops._host.set_workspace(64, 1)
