@@ -245,7 +245,8 @@ PyObject *moe_gemm(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     NEED(dt == at::kFloat && be > 0 && K % be == 0 && w.t->scalar_type() == at::kByte && w.t->numel() == E * N * (K / be) * light_b200_block_bytes((int)type));
   } else {
     NEED((dt == at::kFloat || dt == at::kBFloat16) && s.ok(a[2]) && cuda_contig(*s.t) && s.t->scalar_type() == at::kFloat && s.t->get_device() == dev && bR > 0 &&
-         bC > 0 && N % bR == 0 && K % bC == 0 && w.t->element_size() == 1 && w.t->numel() == E * N * K && s.t->numel() == E * (N / bR) * (K / bC));
+         bC > 0 && N % bR == 0 && K % bC == 0 && w.t->element_size() == 1 && w.t->numel() == E * N * K &&
+         s.t->sizes() == at::IntArrayRef({E, N / bR, K / bC}));
   }
   if (a[11] != Py_None) NEED(tw.ok(a[11]) && cuda_contig(*tw.t) && tw.t->scalar_type() == at::kFloat && tw.t->numel() == M && tw.t->get_device() == dev);
   NEED(workspace_fits(dev, M > 65 ? M : 65, K));

@@ -39,3 +39,18 @@ def test_no_memory_for_the_output_is_an_exception(cuda, name):
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert torch.equal(call(), want)
+
+
+def test_grouped_fp8_scale_of_another_shape_is_refused(cuda):
+    """A scale with the right number of elements and another shape: refused, as before the call went through the native path."""
+    E, N, K, bR, bC, M = 2, 256, 512, 64, 128, 8
+    codes, scale = synth.random_fp8_block(1, E * N, K, bR, bC, device=cuda)
+    codes, scale = codes.reshape(E, N, K), scale.reshape(E, N // bR, K // bC)
+    x = torch.randn(M, K, device=cuda).bfloat16()
+    r = ops.MoERouteFromIDs(torch.arange(M, device=cuda).reshape(M, 1) % E, torch.ones(M, device=cuda), M, 1)
+    good = ops.MoEGemmF8Block(x, codes, scale, bR, bC, r, None, 1)
+    assert torch.isfinite(good.float()).all()
+    s2 = torch.cat([scale, scale], 1)[:, :2, :].contiguous()      # (E, 2, 4) for blocks of (128, 128)
+    for bad, br, bc in ((s2.transpose(1, 2).contiguous(), 128, 128), (s2.reshape(E, 8, 1), 128, 128), (scale.reshape(-1), bR, bC), (scale[:, None], bR, bC)):
+        with pytest.raises(ValueError):
+            ops.MoEGemmF8Block(x, codes, bad, br, bc, r, None, 1)
