@@ -52,11 +52,13 @@ class Linear:
         if self.B is None:  # the common forms as one native call; None: not one of them, or an error to be named below
             y, w4 = None, self.W4
             if w4 is not None:
-                if w4.perm is None and x.dim() and x.shape[-1] == self.in_features:
+                if w4.perm is None and x.dim() and x.shape[-1] == self.in_features and w4.codes.shape[0] == self.out_features:
                     y = ops._host.linear_int4(x, w4.codes, w4.scales, w4.zeros, w4.group)
             elif type(w) is ops.QTensor:
-                y = ops._host.linear_q(x, w.data, w.ggml_type, self.out_features, self.in_features)
-            elif w is not None and w.dtype is torch.float8_e4m3fn and self.WBlockScale is not None and x.dim() and x.shape[-1] == self.in_features:
+                if w.shape == (self.out_features, self.in_features):
+                    y = ops._host.linear_q(x, w.data, w.ggml_type, self.out_features, self.in_features)
+            elif w is not None and w.dtype is torch.float8_e4m3fn and self.WBlockScale is not None and x.dim() and x.shape[-1] == self.in_features and \
+                    w.shape[0] == self.out_features:
                 y = ops._host.linear_f8(x, w, self.WBlockScale, *self.WBlock)
             if y is not None:
                 return y

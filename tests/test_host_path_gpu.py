@@ -54,3 +54,16 @@ def test_grouped_fp8_scale_of_another_shape_is_refused(cuda):
     for bad, br, bc in ((s2.transpose(1, 2).contiguous(), 128, 128), (s2.reshape(E, 8, 1), 128, 128), (scale.reshape(-1), bR, bC), (scale[:, None], bR, bC)):
         with pytest.raises(ValueError):
             ops.MoEGemmF8Block(x, codes, bad, br, bc, r, None, 1)
+
+
+def test_linear_whose_weight_has_another_shape_is_refused(cuda):
+    """A weight that was put into the layer without set_weight / set_int4 and is not (out, in): the general path's error."""
+    x = torch.randn(4, 256, device=cuda)
+    q = ops.QTensor(synth.gaussian_weight(1, ops.Q8_0, 256, 512, device=cuda).reshape(-1), ops.Q8_0, (256, 512))
+    with pytest.raises(ValueError, match="inner dim mismatch"):
+        Linear(256, 512, W=q).forward(x)                       # (in, out): as many blocks
+    w4 = ops.Int4(torch.zeros(512, 32, dtype=torch.int32, device=cuda), torch.ones(512, 2, device=cuda), torch.zeros(512, 2, device=cuda), 128)
+    codes, scale = synth.random_fp8_block(1, 512, 256, device=cuda)
+    for layer in (Linear(256, 384, W4=w4), Linear(256, 384, W=codes.view(torch.float8_e4m3fn), WBlockScale=scale, WBlock=(128, 128))):
+        with pytest.raises(RuntimeError):
+            layer.forward(x.bfloat16())
