@@ -109,6 +109,19 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
   }
   return true;
 }
+// The four epilogue warps, together: whether all of them are to go on.
+__device__ __forceinline__ bool epilogue_all(bool go) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %1, 0;\n\t"
+      "bar.red.and.pred q, 1, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"((uint32_t)go)
+      : "memory");
+  return r != 0;
+}
 __device__ __forceinline__ void st_if(bool p, float *o, float v) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.f32 [%0], %1;\n\t}\n" ::"l"(o), "f"(v), "r"((int)p) : "memory");
 }
@@ -667,7 +680,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
           finish_last(0, shared ? 80 : 16);
           break;
         }
-        if (!warp_wait(d_full + 8 * (seg & 1), (seg >> 1) & 1, abort)) break;
+        // The barriers of the chunks below want all four warps: one that gives up alone would leave the others waiting for good.
+        if (!epilogue_all(warp_wait(d_full + 8 * (seg & 1), (seg >> 1) & 1, abort))) break;
         tc_fence_after();
         const uint32_t d = tmem + lanes + (T.nt > 128 ? 0 : 128 * (seg & 1));
         const int n0 = T.n0 + 128 * rank, ncols = min(128, a.N - n0);  // (<= 0: no rows of the matrix here)
