@@ -21,8 +21,8 @@
 //                the expanders too, five warps to a row quarter, each 16 tokens at a time.
 //
 // Work is the list of (tile, K chunk) pairs, cut into equal runs, one per CTA (pair): stream-K.  A segment that does not
-// start its tile writes a partial tile and raises its flag, which it does first; the segment that starts the tile owns it
-// and adds the partials in run order.  In a grouped launch the units are weighted by their token count, so that runs are
+// start its tile writes a partial tile and sets its flags to the launch's tag, which it does first; the segment that starts the
+// tile owns it and adds the partials in run order.  In a grouped launch the units are weighted by their token count, so that runs are
 // equal in time.  Every wait is bounded; on giving up the status word is set, TMEM is freed and the CTA retires.
 #include <cuda.h>
 
@@ -52,8 +52,14 @@ constexpr int PART_FLOATS = 256 * 128;        // one partial tile: [token][row]
 constexpr int SMEM_MAX = 227 * 1024 - 1024;   // dynamic; the static part (prefix tables, flags) is accounted below
 
 __device__ int g_status;                      // non-zero: a bounded wait gave up (sticky)
-__device__ unsigned int g_flags[MAX_GRID * 64];  // (CTA, row quarter, 16-token chunk): raised by the writer of that part of a partial tile,
-                                                // lowered by its one reader
+// Which parts of the partial tiles are written: a flag per (CTA, row quarter, 16-token chunk) holds the tag of the launch that wrote the
+// part last.  A launch's tag is the epoch it finds, plus one; the last of its CTAs to have read the epoch raises it.  So no flag of an
+// earlier launch ever matches, one that gave up and left flags without a reader included, and nothing is cleared between launches.
+struct Sync {
+  unsigned epoch, readers;
+  unsigned flags[MAX_GRID * 64];
+};
+__device__ Sync g_sync;
 
 struct Args {
   const int32_t *offsets;   // grouped: expert e owns rows offsets[e] .. offsets[e + 1] of the (gathered) tokens; null: one matrix
@@ -181,12 +187,12 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
-__device__ __forceinline__ bool wait_flag(const unsigned *flag, bool mine, volatile int *abort) {  // whole warp, a flag to each lane that has one
+__device__ __forceinline__ bool wait_flag(const unsigned *flag, unsigned tag, bool mine, volatile int *abort) {  // whole warp, a flag to each lane that has one
   const unsigned long long t0 = global_ns();
   for (uint32_t i = 1;; i++) {
-    unsigned v = 1;
+    unsigned v = tag;
     if (mine) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(flag) : "memory");
-    if (__all_sync(0xffffffffu, v != 0)) return true;
+    if (__all_sync(0xffffffffu, v == tag)) return true;
     if ((i & 15u) == 0) {
       if (__any_sync(0xffffffffu, *abort != 0)) return false;
       if (__any_sync(0xffffffffu, global_ns() - t0 > 1000000000ull)) break;
@@ -281,6 +287,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   extern __shared__ unsigned char smem_raw[];
   __shared__ int abort_flag;
   __shared__ uint32_t tmem_sh;
+  __shared__ unsigned tag_sh;  // this launch's tag, there once `tagged` is complete
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char *gen = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t sB = base, sRaw = base + (uint32_t)a.nbs * a.stage_bytes, sStrip = sRaw + (uint32_t)EXPANDERS * Row::SLOT, sBar = sStrip + STRIPS<OutT>;
@@ -288,7 +295,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   // empty[s]: its MMAs have completed.  t_full, t_empty: the token ring's, which runs further ahead: a token tile takes a TMA
   // latency to refill, and with only four stages that, not the tensor core, set the pace of narrow tiles.
   const uint32_t full = sBar, empty = full + 8 * NAS, d_full = empty + 8 * NAS, d_empty = d_full + 16, drained = d_empty + 16, w_full = drained + 8,
-                 t_full = w_full + 8 * EXPANDERS, t_empty = t_full + 8 * NBS;
+                 t_full = w_full + 8 * EXPANDERS, t_empty = t_full + 8 * NBS, tagged = t_empty + 8 * NBS;
   int *preW = reinterpret_cast<int *>(gen + (sBar - base) + BAR_BYTES), *preT = preW + a.E + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = CG == 2 ? (int)cluster_ctarank() : 0;
@@ -304,7 +311,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
     for (int i = 0; i < NAS; i++) mbar_init(full + 8 * i, CG == 2 && rank == 0 ? 5 : 4), mbar_init(empty + 8 * i, 1);
     for (int i = 0; i < a.nbs; i++) mbar_init(t_full + 8 * i, 1), mbar_init(t_empty + 8 * i, 1);
     for (int i = 0; i < 2; i++) mbar_init(d_full + 8 * i, 1), mbar_init(d_empty + 8 * i, 4 * CG);
-    mbar_init(drained, 1);
+    mbar_init(drained, 1), mbar_init(tagged, 1);
     for (int i = 0; i < EXPANDERS; i++) mbar_init(w_full + 8 * i, 1);
     fence_barrier_init();
   }
@@ -460,11 +467,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
 #pragma unroll
       for (int i = 0; i < 16; i++) __stcg(mine + i * 128, __uint_as_float(v[i]));
     };
-    auto raise_flags = [&](int first, int step, int nt) {
+    auto raise_flags = [&](int first, int step, int nt, unsigned tag) {
       __threadfence();
       __syncwarp();
       const int c0 = first + lane * step;
-      if (c0 < nt) asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(g_flags + (blockIdx.x * 4 + quad) * 16 + (c0 >> 4)), "r"(1u) : "memory");
+      if (c0 < nt) asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(g_sync.flags + (blockIdx.x * 4 + quad) * 16 + (c0 >> 4)), "r"(tag) : "memory");
     };
     // Output row (-1: none) and routing weight of token c0 + lane of a tile.
     auto route = [&](const Tile &T, int c0, int &prow, float &pw) {
@@ -494,17 +501,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
         while (jlast + 1 < G && wk.bound(jlast + 1, G) < (t + 1) * nb) jlast++;
       const int col = T.n0 + 128 * rank + row;
       const bool live = col < a.N;
-      if (!warp_wait(d_full + 8 * (seg & 1), (seg >> 1) & 1, abort)) return;
+      if (!warp_wait(d_full + 8 * (seg & 1), (seg >> 1) & 1, abort) || !warp_wait(tagged, 0, abort)) return;
       tc_fence_after();
+      const unsigned tag = tag_sh;
       const uint32_t d = tmem + lanes + (T.nt > 128 ? 0 : 128 * (seg & 1));
       if (jlast > cta) {  // all parts of this warp's chunks: (run, chunk) pairs, a lane to each
         const int chunks = (T.nt - first + step - 1) / step;
         for (int i0 = 0; i0 < (jlast - cta) * chunks; i0 += 32) {
           const int i = i0 + lane, j = min(cta + 1 + i / chunks, jlast), c0 = first + (i % chunks) * step;
           const bool has = i < (jlast - cta) * chunks && wk.bound(j, G) < wk.bound(j + 1, G);  // (an empty run writes nothing)
-          unsigned *flag = g_flags + ((j * CG + rank) * 4 + quad) * 16 + (c0 >> 4);
-          if (!wait_flag(flag, has, abort)) return;
-          if (has) *flag = 0u;  // for the next launch
+          if (!wait_flag(g_sync.flags + ((j * CG + rank) * 4 + quad) * 16 + (c0 >> 4), tag, has, abort)) return;
         }
       }
 #pragma unroll 1
@@ -560,7 +566,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
           }
         }
       }
-      if (!owner) raise_flags(first, step, T.nt);
+      if (!owner) raise_flags(first, step, T.nt, tag);
     };
 
     if (warp < EXPANDERS) {
@@ -668,6 +674,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
     } else {
       // ================================================================ epilogue
       pdl_wait();  // `out` and the partial tiles may still be in use by the kernel before
+      if (warp == EPI_WARP && lane == 0) {
+        unsigned epoch;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(epoch) : "l"(&g_sync.epoch) : "memory");
+        tag_sh = epoch + 1;
+        mbar_arrive(tagged);
+        if (atomicInc(&g_sync.readers, gridDim.x - 1) == gridDim.x - 1) atomicExch(&g_sync.epoch, epoch + 1);  // every CTA has read it
+      }
+      __syncwarp();
+      warp_wait(tagged, 0, abort);
       const uint32_t strip = sStrip, sbytes = STRIP<OutT>;
       const bool bulk = ((size_t)a.N * sizeof(OutT)) % 16 == 0 && ((uintptr_t)out & 15) == 0;
       int seg = 0, chunk = 0;
@@ -700,7 +715,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
           if (u0 > 0) {
             put_part(c0, v);
             if (c0 + 16 < T.nt) put_part(c0 + 16, v + 16);
-            if (c0 + 32 >= T.nt) raise_flags(0, 16, T.nt);
+            if (c0 + 32 >= T.nt) raise_flags(0, 16, T.nt, tag_sh);
             continue;
           }
           int prow;

@@ -95,3 +95,19 @@ def test_narrow_int4_in_groups_of_128(cuda, M, N, K):
     assert torch.equal(y, ops.MatMulInt4(x, w)) and ops.prefill_status(0) == 0
     want = x.double() @ ops.DequantizeInt4(w, torch.float32).double().t()
     assert rel_l2(y.cpu().double().numpy(), want.cpu().numpy()) <= 2.5e-3
+
+
+def test_launches_of_different_runs_one_after_the_other(cuda):
+    """Launches whose tiles are cut in different places leave flags of their own behind: none may pass for a later launch's.  New
+    activations every time, so that a partial tile read too early is an old one; no host wait in between."""
+    shapes = [("q4_k", 130, 4096, 4096), ("q8_0", 70, 512, 8192), ("int4", 300, 1024, 2048), ("q6_k", 65, 640, 16384), ("fp8", 257, 4096, 1024)]
+    calls = [(m, *_weight(kind, n, k, cuda), k) for kind, m, n, k in shapes]
+    g = torch.Generator(device=cuda).manual_seed(1)
+    got = []
+    for i in range(40):
+        m, f, w, dt, k = calls[(i * i + i // 5) % len(calls)]
+        x = torch.randn(m, k, generator=g, device=cuda).to(dt)
+        got.append((f(x), x, w, dt))
+    for y, x, w, dt in got:
+        assert rel_l2(y.cpu().double().numpy(), (x.double() @ w.t()).cpu().numpy()) <= (1e-3 if dt == torch.float32 else 3e-3)
+    assert ops.prefill_status(0) == 0
