@@ -225,6 +225,14 @@ LB200_API int light_b200_moe_gemm(const lb200_moe_args *args, int device, void *
 LB200_API int light_b200_moe_gemm_f8block(const lb200_moe_args *args, const float *w_scale, int block_r, int block_c,
                                           int device, void *stream);
 
+/* The same two calls (w_scale null: light_b200_moe_gemm; else light_b200_moe_gemm_f8block) with memory of their own: `scratch`, device
+ * memory of light_b200_moe_scratch_bytes(M, K) or more, 256-byte aligned, uninitialised, which nothing else uses until the call has run.
+ * Fewer than 256 pairs of bf16 activations then take the tensor-core path too (K % 128 == 0; block_c % 64 == 0), without the
+ * workspace: such calls may overlap on the GPU.  With 256 pairs or more, or scratch = null, nothing differs. */
+LB200_API unsigned long long light_b200_moe_scratch_bytes(int64_t M, int K);
+LB200_API int light_b200_moe_gemm_scratch(const lb200_moe_args *args, const float *w_scale, int block_r, int block_c, void *scratch,
+                                          unsigned long long scratch_bytes, int device, void *stream);
+
 /* ---- multi-GPU: all-gather of row-split outputs over NVLink peer memory (no counterpart in the
  * reference, which is single-GPU: STATUS.md:474).  Each rank r of `world` (<= LB200_MAX_PEERS) GPUs of one
  * node owns rows [r N/P, (r+1) N/P) of a weight and so produces an (M, N/P) column block of the output.

@@ -116,6 +116,8 @@ SYMBOLS = {
     "light_b200_moe_gemm": (C.c_int, [C.POINTER(MoeArgs), C.c_int, C.c_void_p]),
     "light_b200_moe_gemm_q": (C.c_int, [C.POINTER(MoeArgs), C.c_int, C.c_void_p]),
     "light_b200_moe_gemm_f8block": (C.c_int, [C.POINTER(MoeArgs), C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]),
+    "light_b200_moe_scratch_bytes": (C.c_ulonglong, [C.c_int64, C.c_int]),
+    "light_b200_moe_gemm_scratch": (C.c_int, [C.POINTER(MoeArgs), C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_ulonglong, C.c_int, C.c_void_p]),
     "light_b200_moe_clear_unrouted": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_int, C.c_int, C.c_void_p]),
     "light_b200_moe_gemm_static_scratch": (C.c_int, [C.POINTER(MoeArgs), C.c_int, C.c_void_p]),
     "light_b200_kv_append": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int,

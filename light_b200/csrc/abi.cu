@@ -737,8 +737,7 @@ int light_b200_decode_attn_status(int device) {
   return decode_attn_status();
 }
 
-int light_b200_moe_gemm_f8block(const lb200_moe_args *a, const float *w_scale, int block_r, int block_c, int device,
-                                 void *stream) {
+static int moe_f8_check(const lb200_moe_args *a, const float *w_scale, int block_r, int block_c) {
   if (!a) return fail(LB200_E_NULL, "light_b200: moe_gemm_f8block: null argument block");
   if (a->M < 0 || a->size_m < 0 || a->E <= 0 || a->N < 0 || a->K <= 0 || a->topk < 1 || block_r <= 0 || block_c <= 0)
     return fail(LB200_E_SHAPE, "light_b200: moe_gemm_f8block: bad shape");
@@ -747,9 +746,26 @@ int light_b200_moe_gemm_f8block(const lb200_moe_args *a, const float *w_scale, i
   if (!a->counts || !a->offsets || !w_scale) return fail(LB200_E_NULL, "light_b200: moe_gemm_f8block: counts / offsets / scale missing");
   if (a->M > 0 && (!a->input || !a->weights || !a->sorted_pairs || !a->expert_ids || !a->out))
     return fail(LB200_E_NULL, "light_b200: moe_gemm_f8block: null tensor pointer");
+  return 0;
+}
+
+int light_b200_moe_gemm_f8block(const lb200_moe_args *a, const float *w_scale, int block_r, int block_c, int device,
+                                 void *stream) {
+  if (int rc = moe_f8_check(a, w_scale, block_r, block_c)) return rc;
   if (int rc = bind(device)) return rc;
   if (a->M == 0) return 0;
   return moe_gemm_f8block(a, w_scale, block_r, block_c, device, (cudaStream_t)stream);
+}
+
+unsigned long long light_b200_moe_scratch_bytes(int64_t M, int K) { return M < 0 || K <= 0 ? 0 : moe_scratch_bytes(M, K); }
+
+int light_b200_moe_gemm_scratch(const lb200_moe_args *a, const float *w_scale, int block_r, int block_c, void *scratch,
+                                unsigned long long scratch_bytes, int device, void *stream) {
+  if (int rc = w_scale ? moe_f8_check(a, w_scale, block_r, block_c) : moe_check(a, "moe_gemm", false)) return rc;
+  if (!aligned(scratch, 256)) return fail(LB200_E_ALIGN, "light_b200: moe_gemm_scratch: scratch must be 256-byte aligned");
+  if (int rc = bind(device)) return rc;
+  if (!w_scale) return moe_gemm(a, device, (cudaStream_t)stream, scratch, (size_t)scratch_bytes);
+  return a->M == 0 ? 0 : moe_gemm_f8block(a, w_scale, block_r, block_c, device, (cudaStream_t)stream, scratch, (size_t)scratch_bytes);
 }
 
 int light_b200_moe_gemm_q(const lb200_moe_args *a, int device, void *stream) {

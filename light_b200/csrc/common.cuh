@@ -114,12 +114,16 @@ int fp8_block_dequant(const uint8_t *w, const float *s, void *out, int out_dtype
                       cudaStream_t st);
 int fp8_block_rows_dot(const void *x, const uint8_t *w, const float *s, void *y, int act_dtype, int M, int N, int K, int bR, int bC,
                        cudaStream_t st);
-int moe_gemm(const lb200_moe_args *a, int device, cudaStream_t st);
+int moe_gemm(const lb200_moe_args *a, int device, cudaStream_t st, void *scratch = nullptr, size_t scratch_bytes = 0);
 int moe_gemm_q(const lb200_moe_args *a, int device, cudaStream_t st);
 // Q6_K rows that start on any even byte, many activation rows: f32 products (moe.cu)
 int q6k_rows_dense(const float *x, const void *w, float *out, int M, int N, int K, cudaStream_t st);
-int moe_gemm_f8block(const lb200_moe_args *a, const float *w_scale, int bR, int bC, int device, cudaStream_t st);
-int moe_umma(const lb200_moe_args *a, int kind, const float *w_scale, int bR, int bC, int device, cudaStream_t st);
+int moe_gemm_f8block(const lb200_moe_args *a, const float *w_scale, int bR, int bC, int device, cudaStream_t st, void *scratch = nullptr,
+                     size_t scratch_bytes = 0);
+// scratch: this call's own memory of moe_scratch_bytes() or more, whose first gemm_tmem_sync_bytes() are zero when its kernels run
+int moe_umma(const lb200_moe_args *a, int kind, const float *w_scale, int bR, int bC, int device, cudaStream_t st, void *scratch = nullptr,
+             size_t scratch_bytes = 0);
+size_t moe_scratch_bytes(long long M, int K);
 int moe_clear_unrouted(const int64_t *pairs, const int64_t *ids, uint32_t *bits, void *out, long long M, long long rows, long long row_bytes, int E,
                        cudaStream_t st);
 int moe_gemm_static_scratch(const lb200_moe_args *a, int device, cudaStream_t st);
@@ -158,11 +162,13 @@ struct TmemCall {
   int E;
   double mean_tokens;       // tokens per matrix (grouped: pairs / experts)
   int min_run_k;            // fewest k a run covers
+  void *sync;               // gemm_tmem_sync_bytes() of zeros for this call alone, or null: the library's own, shared by calls that do not overlap
   void *parts;              // room for partial tiles
   size_t parts_bytes;
 };
 int gemm_tmem(const TmemCall &c, cudaStream_t st);
 size_t gemm_tmem_parts_bytes();
+size_t gemm_tmem_sync_bytes();
 int gemm_tmem_status();
 size_t decode_nt_ws_bytes(int M, int K);
 int gguf_decode_nt(int type, const float *x, const void *const *w, float *const *out, const int *n, int count, int M, int K, void *ws,

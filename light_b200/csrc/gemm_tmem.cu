@@ -59,7 +59,7 @@ struct Sync {
   unsigned epoch, readers;
   unsigned flags[MAX_GRID * 64];
 };
-__device__ Sync g_sync;
+__device__ Sync g_sync;  // of the launches without one of their own
 
 struct Args {
   const int32_t *offsets;   // grouped: expert e owns rows offsets[e] .. offsets[e + 1] of the (gathered) tokens; null: one matrix
@@ -71,6 +71,7 @@ struct Args {
   int box;                  // token rows of one TMA box
   int stage_bytes, nbs;     // of the token ring, per CTA
   int wmin;                 // grouped: a unit's weight is max(tokens of its tile, wmin)
+  struct Sync *sync;
   float *parts;
 };
 
@@ -445,6 +446,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
     }
   } else {
     const int quad = warp & 3, row = quad * 32 + lane;
+    auto sync = [&]() { return a.sync ? a.sync : &g_sync; };  // (looked up where it is used: held, it cost the expanders registers)
     const uint32_t lanes = (uint32_t)(quad * 32) << 16;
     // Columns c0 .. c0 + 31 of the accumulator at `d` into registers (a tile's last chunk may hold 16).
     auto take = [&](uint32_t d, int c0, int nt, uint32_t (&v)[32]) {
@@ -471,7 +473,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       __threadfence();
       __syncwarp();
       const int c0 = first + lane * step;
-      if (c0 < nt) asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(g_sync.flags + (blockIdx.x * 4 + quad) * 16 + (c0 >> 4)), "r"(tag) : "memory");
+      if (c0 < nt) asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(sync()->flags + (blockIdx.x * 4 + quad) * 16 + (c0 >> 4)), "r"(tag) : "memory");
     };
     // Output row (-1: none) and routing weight of token c0 + lane of a tile.
     auto route = [&](const Tile &T, int c0, int &prow, float &pw) {
@@ -510,7 +512,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
         for (int i0 = 0; i0 < (jlast - cta) * chunks; i0 += 32) {
           const int i = i0 + lane, j = min(cta + 1 + i / chunks, jlast), c0 = first + (i % chunks) * step;
           const bool has = i < (jlast - cta) * chunks && wk.bound(j, G) < wk.bound(j + 1, G);  // (an empty run writes nothing)
-          if (!wait_flag(g_sync.flags + ((j * CG + rank) * 4 + quad) * 16 + (c0 >> 4), tag, has, abort)) return;
+          if (!wait_flag(sync()->flags + ((j * CG + rank) * 4 + quad) * 16 + (c0 >> 4), tag, has, abort)) return;
         }
       }
 #pragma unroll 1
@@ -676,10 +678,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       pdl_wait();  // `out` and the partial tiles may still be in use by the kernel before
       if (warp == EPI_WARP && lane == 0) {
         unsigned epoch;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(epoch) : "l"(&g_sync.epoch) : "memory");
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(epoch) : "l"(&sync()->epoch) : "memory");
         tag_sh = epoch + 1;
         mbar_arrive(tagged);
-        if (atomicInc(&g_sync.readers, gridDim.x - 1) == gridDim.x - 1) atomicExch(&g_sync.epoch, epoch + 1);  // every CTA has read it
+        if (atomicInc(&sync()->readers, gridDim.x - 1) == gridDim.x - 1) atomicExch(&sync()->epoch, epoch + 1);  // every CTA has read it
       }
       __syncwarp();
       warp_wait(tagged, 0, abort);
@@ -810,7 +812,7 @@ int run(const typename Row::Ctx &ctx, const TmemCall &c, Args a, int nt_max, cud
     if (U / least < G) G = (int)(U / least > 0 ? U / least : 1);
   }
   if (c.parts_bytes < (size_t)G * CG * PART_FLOATS * 4) return 0;
-  a.parts = (float *)c.parts;
+  a.parts = (float *)c.parts, a.sync = (Sync *)c.sync;
   const EncodeTiledFn enc = encode_fn();
   if (!enc) return fail(LB200_E_DEVICE, "light_b200: cuTensorMapEncodeTiled is not available from the driver");
   Maps tm;
@@ -882,6 +884,7 @@ int pick(const typename Row::Ctx &ctx, const TmemCall &c, cudaStream_t st) {
 
 }  // namespace
 
+size_t gemm_tmem_sync_bytes() { return (sizeof(Sync) + 1023) & ~(size_t)1023; }
 size_t gemm_tmem_parts_bytes() { return (size_t)MAX_GRID * PART_FLOATS * 4; }
 
 int gemm_tmem(const TmemCall &c, cudaStream_t st) {

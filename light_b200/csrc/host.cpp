@@ -249,7 +249,10 @@ PyObject *moe_gemm(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
          s.t->sizes() == at::IntArrayRef({E, N / bR, K / bC}));
   }
   if (a[11] != Py_None) NEED(tw.ok(a[11]) && cuda_contig(*tw.t) && tw.t->scalar_type() == at::kFloat && tw.t->numel() == M && tw.t->get_device() == dev);
-  NEED(workspace_fits(dev, M > 65 ? M : 65, K));
+  // 256 pairs or more work in the device's workspace; fewer, of bf16 rows, in memory of this call alone, so that several streams may
+  // have one each (the caching allocator hands it to this stream's later work only).
+  const bool few = M < 256;
+  NEED(few || workspace_fits(dev, M, K));
   // Rows that no pair writes are zero: cleared as a whole while that is cheaper than finding them.
   const int64_t row_bytes = N * (int64_t)x.t->element_size(), words = (M + 31) / 32;
   const bool find = M * row_bytes > (8 << 20);
@@ -265,7 +268,11 @@ PyObject *moe_gemm(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
   m.expert_ids = se.t->const_data_ptr<int64_t>(), m.counts = sc, m.offsets = sc + E, m.topk_weights = tw.t ? tw.t->const_data_ptr<float>() : nullptr;
   m.out = out.data_ptr(), m.M = M, m.size_m = M, m.E = (int)E, m.N = (int)N, m.K = (int)K, m.topk = (int)topk, m.row_per_pair = rows == M;
   m.dtype = type >= 0 ? (int)type : act_of(*x.t);
-  return give(type >= 0 ? light_b200_moe_gemm_q(&m, dev, st) : light_b200_moe_gemm_f8block(&m, s.t->const_data_ptr<float>(), (int)bR, (int)bC, dev, st), out);
+  if (type >= 0) return give(light_b200_moe_gemm_q(&m, dev, st), out);
+  at::Tensor own;
+  const int64_t own_bytes = few && dt == at::kBFloat16 ? (int64_t)light_b200_moe_scratch_bytes(M, (int)K) : 0;
+  if (own_bytes) own = at::empty({own_bytes}, w.t->options().dtype(at::kByte));
+  return give(light_b200_moe_gemm_scratch(&m, s.t->const_data_ptr<float>(), (int)bR, (int)bC, own_bytes ? own.data_ptr() : nullptr, own_bytes, dev, st), out);
 }
 
 template <PyObject *(*F)(PyObject *, PyObject *const *, Py_ssize_t)>

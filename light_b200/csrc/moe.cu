@@ -24,11 +24,13 @@ __device__ unsigned int g_moe_bad_ids;
 // Nobody validates the ids before this kernel, so it does.  A search is monotone in e even over unsorted ids: the offsets never
 // decrease and stay in [0, M].  A negative id owns no range, an id >= E lies at or beyond offsets[E], outside every
 // expert's range (the matmul kernels skip both), and either sets the status word.
+// `clear`: words that the launches after this one want zero.
 __global__ void __launch_bounds__(256) moe_prep_kernel(const int64_t *__restrict__ ids, int32_t *__restrict__ offsets, int32_t *__restrict__ counts,
-                                                       long long M, int E) {
+                                                       long long M, int E, uint32_t *__restrict__ clear, int clear_words) {
   pdl_launch_dependents();
   pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int c = (int)i; c < clear_words; c += gridDim.x * 256) clear[c] = 0u;
   if (i < M) {
     const long long e = ids[i];
     if (e < 0 || e >= E) g_moe_bad_ids = 1u;
@@ -235,10 +237,13 @@ __global__ void __launch_bounds__(MOE_WARPS * 32) moe_gemm_kernel(
   }
 }
 
-static int prep(const lb200_moe_args *a, cudaStream_t st) {
+static int prep(const lb200_moe_args *a, cudaStream_t st, void *scratch = nullptr, size_t scratch_bytes = 0) {
   if (a->M > 0x7fffffffLL) return fail(LB200_E_TOO_LARGE, "light_b200: moe: %lld pairs", (long long)a->M);
-  const long long work = a->M > a->E + 1 ? a->M : a->E + 1;
-  launch_early(moe_prep_kernel, dim3((unsigned)((work + 255) / 256)), dim3(256), st, a->expert_ids, a->offsets, a->counts, (long long)a->M, a->E);
+  const int words = scratch && scratch_bytes >= moe_scratch_bytes(a->M, a->K) ? (int)(gemm_tmem_sync_bytes() / 4) : 0;
+  long long work = a->M > a->E + 1 ? a->M : a->E + 1;
+  if (words && work < 4096) work = 4096;  // (a few words a thread)
+  launch_early(moe_prep_kernel, dim3((unsigned)((work + 255) / 256)), dim3(256), st, a->expert_ids, a->offsets, a->counts, (long long)a->M, a->E,
+               (uint32_t *)scratch, words);
   return launched("moe expert offsets");
 }
 
@@ -410,10 +415,14 @@ int moe_bad_ids_status() {
   return (int)v;
 }
 
-int moe_gemm(const lb200_moe_args *a, int device, cudaStream_t st) {
-  int rc = prep(a, st);
+size_t moe_scratch_bytes(long long M, int K) {
+  return gemm_tmem_sync_bytes() + (((size_t)M * K * 2 + 1023) & ~(size_t)1023) + gemm_tmem_parts_bytes();
+}
+
+int moe_gemm(const lb200_moe_args *a, int device, cudaStream_t st, void *scratch, size_t scratch_bytes) {
+  int rc = prep(a, st, scratch, scratch_bytes);
   if (rc) return rc;
-  if (int took = moe_umma(a, 0, nullptr, 0, 0, device, st)) return took == 1 ? 0 : took;
+  if (int took = moe_umma(a, 0, nullptr, 0, 0, device, st, scratch, scratch_bytes)) return took == 1 ? 0 : took;
   switch (a->dtype) {
     case LB200_F32: return run<float, float, DenseRow<float>>(a, st);
     case LB200_BF16: return run<__nv_bfloat16, __nv_bfloat16, DenseRow<__nv_bfloat16>>(a, st);
@@ -455,13 +464,13 @@ int moe_gemm_static_scratch(const lb200_moe_args *a, int device, cudaStream_t st
   return moe_gemm(&b, device, st);
 }
 
-int moe_gemm_f8block(const lb200_moe_args *a, const float *w_scale, int bR, int bC, int device, cudaStream_t st) {
-  int rc = prep(a, st);
+int moe_gemm_f8block(const lb200_moe_args *a, const float *w_scale, int bR, int bC, int device, cudaStream_t st, void *scratch, size_t scratch_bytes) {
+  int rc = prep(a, st, scratch, scratch_bytes);
   if (rc) return rc;
-  int took = moe_umma(a, 2, w_scale, bR, bC, device, st);
+  int took = moe_umma(a, 2, w_scale, bR, bC, device, st, scratch, scratch_bytes);
   if (took == 1) return 0;
   if (took) return took;
-  // Few pairs (a decode step), or a shape the tensor-core path does not take: one warp per output column and
+  // Few pairs (a decode step) without scratch of the call's own, or a shape the tensor-core path does not take: one warp per output column and
   // tile of sorted pairs, the weight row read once per tile.
   if (bR <= 0 || bC <= 0 || bC % 8 || a->K % bC || a->N % bR || a->K % 8)
     return fail(LB200_E_SHAPE, "light_b200: moe_gemm_f8block: N=%d K=%d with blocks (%d, %d): block_c must be a multiple of 8 and the blocks must tile the weight",

@@ -1123,7 +1123,7 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const TI *__restrict__
 }
 
 template <typename Row, bool BF16, typename OutT, typename TI>
-int moe_launch(const lb200_moe_args *a, const typename Row::Ctx &ctx, void *ws, size_t ws_bytes, cudaStream_t st, bool older = true) {
+int moe_launch(const lb200_moe_args *a, const typename Row::Ctx &ctx, void *ws, size_t ws_bytes, cudaStream_t st, void *sync = nullptr, bool older = true) {
   if (int rc = ensure_encode()) return rc;
   long long blocks = (a->M + 7) / 8;
   if (blocks > 148 * 32) blocks = 148 * 32;
@@ -1146,7 +1146,7 @@ int moe_launch(const lb200_moe_args *a, const typename Row::Ctx &ctx, void *ws, 
     TmemCall c = tmem_call<Row>(ctx);
     c.x16 = ws, c.bf16 = BF16, c.out = a->out, c.M = a->M, c.N = a->N, c.K = a->K;
     c.offsets = a->offsets, c.pairs = a->sorted_pairs, c.topkw = a->topk_weights, c.size_m = a->size_m, c.E = a->E;
-    c.mean_tokens = (double)a->M / a->E, c.min_run_k = tmem_min_run(), c.parts = sk, c.parts_bytes = ws_bytes - x_bytes;
+    c.mean_tokens = (double)a->M / a->E, c.min_run_k = tmem_min_run(), c.parts = sk, c.parts_bytes = ws_bytes - x_bytes, c.sync = sync;
     if (int took = gemm_tmem(c, st)) return took == 1 ? 0 : took;
   }
   if (!older) return NOT_COVERED;
@@ -1158,14 +1158,20 @@ int moe_launch(const lb200_moe_args *a, const typename Row::Ctx &ctx, void *ws, 
 // Grouped matmul on the tensor cores; the expert offsets must already be in a->offsets.  kind: 0 dense
 // (a->dtype = BF16 only), 1 GGUF (a->dtype = Q4_K / Q6_K, x f32), 2 block-scaled FP8 (a->dtype = F32 / BF16
 // activations).  Returns 1 when taken, 0 when not covered, other values are errors.
-int moe_umma(const lb200_moe_args *a, int kind, const float *w_scale, int bR, int bC, int device, cudaStream_t st) {
+int moe_umma(const lb200_moe_args *a, int kind, const float *w_scale, int bR, int bC, int device, cudaStream_t st, void *scratch, size_t scratch_bytes) {
   // Fewer than 256 pairs (a decode step): where the fallback multiplies the same 16-bit values as the tensor cores do (bf16
-  // activations); others keep their f32 products.
+  // activations; others keep their f32 products), and only in scratch of the call's own: the fallback shares no memory with
+  // other calls, so that sparse blocks of few tokens may run on several streams at once.
   const bool few = a->M < 256;
-  if ((few && !(use_tmem() && kind != 1 && a->dtype == LB200_BF16 && a->K % 128 == 0 && a->E <= 1024)) || a->M > 0x7fffffffLL || ((uintptr_t)a->input & 15) || ((uintptr_t)a->weights & 15) || a->K % 64) return 0;
-  void *ws;
+  if ((few && !(use_tmem() && kind != 1 && a->dtype == LB200_BF16 && a->K % 128 == 0 && a->E <= 1024 && scratch && scratch_bytes >= moe_scratch_bytes(a->M, a->K))) ||
+      a->M > 0x7fffffffLL || ((uintptr_t)a->input & 15) || ((uintptr_t)a->weights & 15) || a->K % 64)
+    return 0;
+  void *ws, *sync = nullptr;
   size_t wsb;
-  {
+  if (few) {
+    const size_t sb = gemm_tmem_sync_bytes();
+    sync = scratch, ws = (char *)scratch + sb, wsb = scratch_bytes - sb;
+  } else {
     std::lock_guard<std::mutex> lk(g_mu);
     if (!g_ws[device].ptr || g_ws[device].bytes < (size_t)a->M * a->K * 2) return 0;
     ws = g_ws[device].ptr, wsb = g_ws[device].bytes;
@@ -1173,7 +1179,7 @@ int moe_umma(const lb200_moe_args *a, int kind, const float *w_scale, int bR, in
   int rc = 0;
   if (kind == 0) {
     if (a->dtype != LB200_BF16) return 0;
-    rc = moe_launch<DenseRow, true, __nv_bfloat16, __nv_bfloat16>(a, DenseCtx{(const uint16_t *)a->weights}, ws, wsb, st, !few);
+    rc = moe_launch<DenseRow, true, __nv_bfloat16, __nv_bfloat16>(a, DenseCtx{(const uint16_t *)a->weights}, ws, wsb, st, sync, !few);
   } else if (kind == 1) {
     if (a->K % 256) return 0;
     if (a->dtype == LB200_Q4_K)
@@ -1188,7 +1194,7 @@ int moe_umma(const lb200_moe_args *a, int kind, const float *w_scale, int bR, in
     if (a->K % 128 || bC % 64 || bR <= 0 || a->N % bR || a->K % bC) return 0;
     const Fp8Ctx ctx{(const uint8_t *)a->weights, w_scale, bR, bC};
     if (a->dtype == LB200_BF16)
-      rc = moe_launch<Fp8Row, true, __nv_bfloat16, __nv_bfloat16>(a, ctx, ws, wsb, st, !few);
+      rc = moe_launch<Fp8Row, true, __nv_bfloat16, __nv_bfloat16>(a, ctx, ws, wsb, st, sync, !few);
     else if (a->dtype == LB200_F32)
       rc = moe_launch<Fp8Row, false, float, float>(a, ctx, ws, wsb, st);
     else

@@ -601,8 +601,11 @@ def _moe_dispatch(op: str, key_dtype: int, quant: bool, inp: torch.Tensor, weigh
         raise ValueError(f"{op}: topkWeights must be F32 with {M} elements")
     dev = _dev(inp, op)
     inc = inp.contiguous()
-    if M:  # tensor-core grouped path: the token rows gathered in expert order, and behind them the partial tiles
-        ensure_workspace(dev, int(_lib.lib().light_b200_matmul_q_workspace_bytes(max(M, 65), K)))
+    own = None
+    if M >= 256:  # tensor-core grouped path: the token rows gathered in expert order, and behind them the partial tiles
+        ensure_workspace(dev, int(_lib.lib().light_b200_matmul_q_workspace_bytes(M, K)))
+    elif M and not quant and inp.dtype == torch.bfloat16:  # the same for few pairs, in memory of this call alone
+        own = torch.empty(int(_lib.lib().light_b200_moe_scratch_bytes(M, K)), dtype=torch.uint8, device=inp.device)
     counts = torch.zeros(E, dtype=torch.int32, device=inp.device)
     offsets = torch.zeros(E + 1, dtype=torch.int32, device=inp.device)
     out = torch.zeros((M, N), dtype=out_dtype, device=inp.device)
@@ -611,12 +614,11 @@ def _moe_dispatch(op: str, key_dtype: int, quant: bool, inp: torch.Tensor, weigh
                 offsets=offsets.data_ptr(),
                 topk_weights=0 if topk_weights is None else topk_weights.contiguous().data_ptr(), out=out.data_ptr(),
                 M=M, size_m=M, E=E, N=N, K=K, topk=topk, row_per_pair=int(row_per_pair), dtype=key_dtype)
-    if f8 is not None:
-        scale, bR, bC = f8
-        _lib.check(_lib.lib().light_b200_moe_gemm_f8block(C.byref(a), _ptr(scale.contiguous()), bR, bC, dev, _stream(dev)))
+    if quant:
+        _lib.check(_lib.lib().light_b200_moe_gemm_q(C.byref(a), dev, _stream(dev)))
         return out
-    fn = _lib.lib().light_b200_moe_gemm_q if quant else _lib.lib().light_b200_moe_gemm
-    _lib.check(fn(C.byref(a), dev, _stream(dev)))
+    scale, bR, bC = (None, 0, 0) if f8 is None else (f8[0].contiguous(), f8[1], f8[2])
+    _lib.check(_lib.lib().light_b200_moe_gemm_scratch(C.byref(a), _ptr(scale), bR, bC, _ptr(own), 0 if own is None else own.numel(), dev, _stream(dev)))
     return out
 
 

@@ -111,3 +111,65 @@ def test_launches_of_different_runs_one_after_the_other(cuda):
     for y, x, w, dt in got:
         assert rel_l2(y.cpu().double().numpy(), (x.double() @ w.t()).cpu().numpy()) <= (1e-3 if dt == torch.float32 else 3e-3)
     assert ops.prefill_status(0) == 0
+
+
+def _few(dev, seed, T, E, topk, N, K, dense):
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(T, K, generator=g).to(dev, torch.bfloat16)
+    ids = torch.rand(T, E, generator=g).topk(topk, -1).indices.to(dev)
+    r = ops.MoERouteFromIDs(ids, torch.rand(T * topk, generator=g).to(dev), T, topk)
+    if dense:
+        w = torch.randn(E, N, K, generator=g).to(dev, torch.bfloat16)
+        return lambda: ops.MoEGemm(x, w, r, r.weights, topk)
+    codes, scale = synth.random_fp8_block(seed, E * N, K, device=dev)
+    return lambda: ops.MoEGemmF8Block(x, codes.reshape(E, N, K), scale.reshape(E, N // 128, K // 128), 128, 128, r, r.weights, topk)
+
+
+@pytest.mark.parametrize("dense", [False, True])
+def test_grouped_calls_of_few_pairs_on_two_streams(cuda, dense):
+    """Fewer than 256 pairs share nothing with other calls: flags, partial tiles and gathered tokens are the call's own."""
+    calls = [_few(cuda, 1, 9, 24, 3, 512, 4096, dense), _few(cuda, 2, 31, 16, 8, 384, 2048, dense)]
+    want = [f() for f in calls]
+    streams = [torch.cuda.Stream() for _ in calls]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(40):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(calls[i]())
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert all(torch.equal(want[i], y) for y in got[i])
+    assert ops.prefill_status(0) == 0
+
+
+def test_scratch_of_a_call_may_hold_anything(cuda):
+    """Flags that look raised, and an epoch of any value, are cleared by the call that is given the memory."""
+    import ctypes as C
+
+    from light_b200 import _lib
+
+    T, E, topk, N, K = 8, 12, 4, 256, 4096
+    g = torch.Generator().manual_seed(4)
+    x, w = torch.randn(T, K, generator=g).to(cuda, torch.bfloat16), torch.randn(E, N, K, generator=g).to(cuda, torch.bfloat16)
+    ids = torch.rand(T, E, generator=g).topk(topk, -1).indices.to(cuda)
+    r = ops.MoERouteFromIDs(ids, torch.ones(T * topk, device=cuda), T, topk)
+    M = T * topk
+    want = torch.einsum("mk,mnk->mn", x.double().repeat_interleave(topk, 0), w.double()[ids.reshape(-1)])
+    counts, offsets = torch.empty(E, dtype=torch.int32, device=cuda), torch.empty(E + 1, dtype=torch.int32, device=cuda)
+    L = _lib.lib()
+    nbytes = L.light_b200_moe_scratch_bytes(M, K)
+    for fill in (1, 0, -1, 0x7f7f7f7f):
+        scratch = torch.full((nbytes // 4 + 64,), fill, dtype=torch.int32, device=cuda)
+        out = torch.zeros(M, N, dtype=torch.bfloat16, device=cuda)
+        a = _lib.MoeArgs(input=x.data_ptr(), weights=w.data_ptr(), sorted_pairs=r.sorted_pairs.data_ptr(), expert_ids=r.sorted_expts.data_ptr(),
+                         counts=counts.data_ptr(), offsets=offsets.data_ptr(), topk_weights=0, out=out.data_ptr(), M=M, size_m=M, E=E, N=N, K=K, topk=topk,
+                         row_per_pair=0, dtype=_lib.BF16)
+        before = _lib.launch_count()
+        _lib.check(L.light_b200_moe_gemm_scratch(C.byref(a), None, 0, 0, C.c_void_p(scratch.data_ptr()), nbytes, 0,
+                                                 C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        assert _lib.launch_count() - before == 3      # offsets, token rows, the matmul: not the kernel for calls without scratch (2)
+        assert rel_l2(out.cpu().double().numpy(), want.cpu().numpy()) <= 3e-3
+        assert L.light_b200_moe_gemm_scratch(C.byref(a), None, 0, 0, C.c_void_p(scratch.data_ptr() + 64), nbytes, 0, None) == -4   # not on 256 bytes
+        assert bool((scratch[nbytes // 4:] == fill).all())
+    assert ops.prefill_status(0) == 0
