@@ -116,6 +116,13 @@ __device__ __forceinline__ void cluster_combine(const AttnArgs &a, const float *
   if (KS > 1) umma::cluster_sync();  // nobody leaves while a peer still reads its partials
 }
 
+// The position: read before the wait as a hint and once more after it, so never from a line that the first read left in L1.
+__device__ __forceinline__ long long load_pos(const long long *p) {
+  long long v;
+  asm volatile("ld.relaxed.gpu.global.s64 %0, [%1];\n" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
 template <int PER, int GH_>
 struct AttnCfg {
   static constexpr int D = PER * 32;
@@ -142,7 +149,7 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attn_kernel(AttnArgs a) 
   {
     // The cached rows of this CTA on their way to L2 while the launch before still runs.  Only a hint: the position may be
     // one short here, and every row is read after the wait.
-    const long long p = a.pos[0];
+    const long long p = load_pos(a.pos);
     const int n = (int)(p < 0 ? 0 : p < a.Cap ? p + 1 : a.Cap), s0 = a.window > 0 ? max(0, n - a.window) : 0, ch = (n - s0 + KS - 1) / KS;
     const int f = s0 + rank * ch, e = min(n, f + ch);
     const char *kp = static_cast<const char *>(a.kbuf) + ((size_t)bkh * a.Cap + f) * D * sizeof(T), *vp = static_cast<const char *>(a.vbuf) + ((size_t)bkh * a.Cap + f) * D * sizeof(T);
@@ -150,8 +157,8 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attn_kernel(AttnArgs a) 
     for (int i = threadIdx.x; i < lines; i += DA_THREADS)
       asm volatile("prefetch.global.L2 [%0];\n\tprefetch.global.L2 [%1];\n" ::"l"(kp + (size_t)i * 128), "l"(vp + (size_t)i * 128));
   }
-  pdl_wait();  // q, k_new, v_new are the previous launch's output; pos is older
-  long long pos = a.pos[0];
+  pdl_wait();  // q, k_new, v_new are the previous launch's output, and so may be pos
+  long long pos = load_pos(a.pos);
   // A position outside the cache: reported, nothing is appended (as kv_append_kernel), and the launch attends
   // over the cached rows of the clamped range, so that append-inside stays equal to append-then-attend.
   const bool in_range = pos >= 0 && pos < a.Cap;
@@ -413,7 +420,7 @@ __global__ void __launch_bounds__(FT_THREADS, D == 64 ? 2 : 1) decode_attn_f32_k
       trig[i] = v.x, trig[D / 2 + i] = v.y;
     }
   };
-  const long long seen = a.pos[0];
+  const long long seen = load_pos(a.pos);
   plan(seen);
   {
     const char *kp = reinterpret_cast<const char *>(kc + (size_t)j0 * D), *vp = reinterpret_cast<const char *>(vc + (size_t)j0 * D);
@@ -441,7 +448,7 @@ __global__ void __launch_bounds__(FT_THREADS, D == 64 ? 2 : 1) decode_attn_f32_k
     for (int t = 0; t < S - 1; t++) issue(t);
   };
   fill();
-  const long long now = *(const volatile long long *)a.pos;
+  const long long now = load_pos(a.pos);
   float2 qv[QP], kv = make_float2(0.f, 0.f), vv = kv;
 #pragma unroll
   for (int i = 0; i < QP; i++) {
@@ -658,7 +665,7 @@ __global__ void __launch_bounds__(MA_THREADS, mma_ctas(D)) decode_attn_mma_kerne
   const int KS = gridDim.y, rank = blockIdx.y, bkh = blockIdx.x;
   const int g = a.NH / a.KH, b = bkh / a.KH, kh = bkh - b * a.KH;
   pdl_wait();
-  long long pos = a.pos[0];
+  long long pos = load_pos(a.pos);
   const bool in_range = pos >= 0 && pos < a.Cap;
   if (!in_range) {
     if (threadIdx.x == 0) atomicOr(&g_attn_status, 1u);

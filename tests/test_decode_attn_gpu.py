@@ -179,6 +179,27 @@ def test_position_moves_right_before_the_launch(cuda):
     assert torch.equal(*outs)
 
 
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("D", [32, 64, 128, 256, 512])
+def test_position_moves_right_before_the_launch_in_every_kernel(cuda, D, dtype):
+    """As above for each kernel: one that keeps the position of its early look overwrites the key before and drops a position."""
+    B, NH, KH, cap, steps, dt = 2, 8, 2, 256, 40, {"f32": torch.float32, "bf16": torch.bfloat16}[dtype]
+    g = torch.Generator(device=cuda).manual_seed(D)
+    q, k, v = (torch.randn(steps, B, h, 1, D, generator=g, device=cuda).to(dt) for h in (NH, KH, KH))
+    outs = []
+    for wait in (False, True):
+        kb, vb = (torch.zeros(B, KH, cap, D, device=cuda, dtype=dt) for _ in range(2))
+        pos = torch.full((1,), 29, device=cuda)
+        y = []
+        for s in range(steps):
+            ops.IncrementI64(pos)
+            if wait:
+                torch.cuda.synchronize()
+            y.append(ops.DecodeAttention(q[s], kb, vb, pos, D ** -0.5, 0, k[s], v[s], rope_base=10000.0))
+        outs.append(torch.cat([torch.stack(y).flatten(), kb.flatten(), vb.flatten()]))
+    assert torch.equal(*outs)
+
+
 @pytest.mark.parametrize("D,g", [(64, 1), (64, 2), (64, 3), (64, 8), (64, 16), (128, 1), (128, 2), (128, 4), (128, 5), (128, 16)])
 @pytest.mark.parametrize("n,window", [(1, 0), (64, 0), (65, 0), (513, 0), (1025, 0), (700, 100)])
 def test_f32_kernel(cuda, D, g, n, window):
