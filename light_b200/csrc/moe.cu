@@ -19,6 +19,17 @@ namespace lb {
 // reports it together with the routing kernels' own word).
 __device__ unsigned int g_moe_bad_ids;
 
+// First sorted index whose expert id is >= e.
+__device__ __forceinline__ int first_of(const int64_t *ids, long long M, long long e) {
+  int lo = 0, hi = (int)M;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (ids[mid] < e) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
 // offsets[e] = first sorted index whose expert id is >= e, for e <= E (so offsets[E] = M when every id is an expert), and
 // counts[e], each by its own binary search: every entry is written whatever the ids are, so nothing has to be cleared before.
 // Nobody validates the ids before this kernel, so it does.  A search is monotone in e even over unsorted ids: the offsets never
@@ -36,31 +47,26 @@ __global__ void __launch_bounds__(256) moe_prep_kernel(const int64_t *__restrict
     if (e < 0 || e >= E) g_moe_bad_ids = 1u;
   }
   if (i > E) return;
-  auto first = [&](long long e) {
-    int lo = 0, hi = (int)M;
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (ids[mid] < e) lo = mid + 1;
-      else hi = mid;
-    }
-    return lo;
-  };
-  const int o = first(i);
+  const int o = first_of(ids, M, i);
   offsets[i] = o;
-  if (i < E) counts[i] = first(i + 1) - o;
+  if (i < E) counts[i] = first_of(ids, M, i + 1) - o;
 }
 
 // The output rows that no pair of the routing writes (ids that are no experts, pair ids out of range or missing) are zero.  A bit
-// per row is set by the pairs that do write, and the rows without one are cleared: clearing all of `out` instead costs a pass
-// over it (32768 x 7168 bf16: 110 us against 5).
+// per row is set by the pairs that are sure to write, and the rows without one are cleared: clearing all of `out` instead costs a
+// pass over it (32768 x 7168 bf16: 110 us against 5).  Sure are those with an expert's id that lie in [offsets[0], offsets[E]) as
+// well: some of the matmul kernels go by the one, some by the other, and over ids that are not sorted the two differ.
 __global__ void __launch_bounds__(256) moe_mark_kernel(const int64_t *__restrict__ pairs, const int64_t *__restrict__ ids, uint32_t *__restrict__ bits,
                                                        long long M, long long rows, int E) {
   pdl_launch_dependents();
   pdl_wait();
+  __shared__ int range[2];
+  if (threadIdx.x < 2) range[threadIdx.x] = first_of(ids, M, threadIdx.x ? E : 0);
+  __syncthreads();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= M) return;
   const long long p = pairs[i], e = ids[i];
-  if (p >= 0 && p < rows && e >= 0 && e < E) atomicOr(bits + (p >> 5), 1u << (p & 31));
+  if (p >= 0 && p < rows && e >= 0 && e < E && i >= range[0] && i < range[1]) atomicOr(bits + (p >> 5), 1u << (p & 31));
 }
 __global__ void __launch_bounds__(256) moe_clear_kernel(const uint32_t *__restrict__ bits, char *__restrict__ out, long long rows, long long row_bytes) {
   pdl_launch_dependents();

@@ -1,6 +1,6 @@
 """The tensor-memory matmul (weights expanded into TMEM, stream-K over CTAs or CTA pairs) where it can go wrong: one token more
 than a tile, ragged row counts (with and without whole 16-byte output rows), the shortest K, runs that start and end inside
-tiles, and grouped launches with empty experts, single tokens and ids outside the experts.
+tiles, grouped launches with empty experts and single tokens, and launches on two streams.
 
 Bounds: operands are rounded once each to f16 (2^-12 relative on average over a product: 1e-3 with room, the bound of the other
 tensor-core paths) or are the bf16 values themselves, when the bf16 output's rounding (2^-9 at most) is what remains."""
