@@ -69,7 +69,8 @@ __global__ void rope_kernel(const T *__restrict__ x, const long long *__restrict
 
 // Greedy sampling: the index of the largest element of every row (ties: the lowest index), as I64.  reference ops.Argmax on the last
 // axis (ops/argmax.go:14-60, kernels/cuda/topk.go:56-90).  A row is a cluster of ks CTAs, eight for a few long rows: one SM has
-// too few loads in flight (128256 columns: 15.7 us by one CTA with a load at a time).
+// too few loads in flight (128256 columns: 15.7 us by one CTA with a load at a time).  A scan that starts with the first element and
+// moves on to larger ones: a NaN at index 0 stays, one anywhere else is never chosen, whichever thread meets it first.
 __global__ void __launch_bounds__(1024) argmax_rows_kernel(const float *__restrict__ x, long long *__restrict__ out, int cols, int ks) {
   __shared__ float bv[32];
   __shared__ int bi[32];
@@ -81,18 +82,20 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(const float *__restri
   const float *row = x + (size_t)(blockIdx.x / ks) * cols;
   float v = -INFINITY;
   int idx = 0x7fffffff;
-  auto take = [&](float c, int j) {
-    if (c > v || (c == v && j < idx) || idx == 0x7fffffff) v = c, idx = j;  // NaN never wins over a number; the first element seeds
+  bool first_is_nan = false;
+  auto take = [&](float c, unsigned j) {  // (j ascends)
+    if (j == 0) first_is_nan = c != c;
+    if (c > v || (idx == 0x7fffffff && c == c)) v = c, idx = (int)j;
   };
-  int j = rank * 1024 + threadIdx.x;
-  for (; j + 7ll * step < cols; j += 8 * step) {
+  unsigned j = rank * 1024 + threadIdx.x;
+  for (; j + 7u * step < (unsigned)cols; j += 8u * step) {
     float c[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) c[i] = row[j + i * step];
 #pragma unroll
     for (int i = 0; i < 8; i++) take(c[i], j + i * step);
   }
-  for (; j < cols; j += step) take(row[j], j);
+  for (; j < (unsigned)cols; j += step) take(row[j], j);
   auto better = [](float a, int ai, float b, int bi_) { return a > b || (a == b && ai < bi_); };
   auto warp_best = [&]() {
 #pragma unroll
@@ -120,7 +123,7 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(const float *__restri
     }
     umma::cluster_sync();  // nobody leaves while a peer still reads its best
   }
-  if (rank == 0 && threadIdx.x == 0) out[blockIdx.x / ks] = idx;
+  if (rank == 0 && threadIdx.x == 0) out[blockIdx.x / ks] = first_is_nan ? 0 : idx;
 }
 
 template <typename K, typename... Args>

@@ -109,3 +109,24 @@ def test_argmax_over_a_cluster(cuda, rows, cols):
     x[torch.arange(rows), at] = 9.0
     x[:, cols - 1] = 9.0
     assert torch.equal(ops.Argmax(x.to(cuda)).cpu().flatten(), at)
+
+
+@pytest.mark.parametrize("cols", [1000, 16383, 128256])
+def test_argmax_with_nan(cuda, cols):
+    """A scan from the first element on: a NaN is never larger, so one after the first is passed over, wherever the largest is; one at the
+    start stays, and so a row of nothing else answers 0."""
+    g = torch.Generator().manual_seed(cols)
+    for nans in ([1], [5, 7], [cols // 3, cols // 2], [cols - 1], [0], [0, 9]):
+        x = torch.randn(1, cols, generator=g)
+        x[0, nans] = float("nan")
+        for at in (2, cols // 3 + 1, nans[-1] + 1024, nans[-1] + 8192, nans[-1] + 65536, cols - 2):   # a thread's or a warp's next elements
+            if 0 < at < cols and at not in nans:
+                y = x.clone()
+                y[0, at] = 9.0
+                assert int(ops.Argmax(y.to(cuda))) == (0 if 0 in nans else at), (nans, at)
+    assert int(ops.Argmax(torch.full((1, cols), float("nan"), device=cuda))) == 0
+    assert int(ops.Argmax(torch.full((1, cols), -float("inf"), device=cuda))) == 0
+    y = torch.full((1, cols), -float("inf"), device=cuda)
+    y[0, 3] = float("nan")
+    y[0, 4] = -1e30
+    assert int(ops.Argmax(y)) == 4
