@@ -649,6 +649,39 @@ __device__ __forceinline__ void ld_stream(const void *p, uint32_t (&v)[W]) {
     asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(p));
 }
 
+// One head's partial result of a warp, the 16 keys from j0 on and every MA_WARPS-th 16 after them, in f32 from end to end, into `row`
+// (max in units of log2 e, sum, sum p v).  For caches that hold infinities: the hi and lo parts of a split operand multiply those to
+// infinities of either sign, or to NaN, where the product itself is an infinity, or a score of -inf whose key counts for nothing.
+template <int D>
+__device__ __noinline__ void attend_plain(const __nv_bfloat16 *q, const __nv_bfloat16 *K, const __nv_bfloat16 *V, const __nv_bfloat16 *fresh, int pos_new,
+                                          const float *trig, float sc, int j0, int j1, float *row) {
+  constexpr int P = D / 32;
+  const int lane = threadIdx.x & 31;
+  float qf[P], acc[P], m = -INFINITY, l = 0.f;
+#pragma unroll
+  for (int i = 0; i < P; i++) {
+    const int d = lane * P + i, e = d & (D / 2 - 1);
+    const float x0 = __bfloat162float(q[e]), x1 = __bfloat162float(q[e + D / 2]);
+    const float cs = trig ? trig[e] : 1.f, sn = trig ? trig[D / 2 + e] : 0.f;
+    qf[i] = !trig ? __bfloat162float(q[d]) : d < D / 2 ? x0 * cs - x1 * sn : x0 * sn + x1 * cs, acc[i] = 0.f;
+  }
+  for (int i0 = 0, j = j0; j < j1; j = ++i0 % 16 ? j + 1 : j + 1 + 16 * (MA_WARPS - 1)) {
+    const __nv_bfloat16 *k = j == pos_new ? fresh : K + (size_t)j * D, *v = j == pos_new ? fresh + D : V + (size_t)j * D;
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < P; i++) s = fmaf(qf[i], __bfloat162float(k[lane * P + i]), s);
+    s = warp_sum(s) * sc;
+    if (s == -INFINITY) continue;
+    const float mx = fmaxf(m, s), corr = exp2f(m - mx), e = exp2f(s - mx);
+    m = mx, l = fmaf(l, corr, e);
+#pragma unroll
+    for (int i = 0; i < P; i++) acc[i] = fmaf(e, __bfloat162float(v[lane * P + i]), acc[i] * corr);
+  }
+  if (lane == 0) row[0] = m, row[1] = l;
+#pragma unroll
+  for (int i = 0; i < P; i++) row[2 + lane * P + i] = acc[i];
+}
+
 template <int D, bool G16>
 __global__ void __launch_bounds__(MA_THREADS, mma_ctas(D)) decode_attn_mma_kernel(AttnArgs a) {
   constexpr int KL = D / 64;        // 32-byte loads of a key row per lane; each feeds two 16-dim steps
@@ -843,6 +876,17 @@ __global__ void __launch_bounds__(MA_THREADS, mma_ctas(D)) decode_attn_mma_kerne
     for (int t = 0; t < NT; t++)
 #pragma unroll
       for (int e = 0; e < 2; e++) row[2 + NT * (2 * c + e) + t] = G16 ? o[t][2 * i + e] : o[t][e] + o[t][2 + e];
+  }
+  float sum = 0.f;
+#pragma unroll
+  for (int t = 0; t < NT; t++) sum += (o[t][0] + o[t][1]) + (o[t][2] + o[t][3]);
+#pragma unroll
+  for (int i = 0; i < (G16 ? 2 : 1); i++) sum += l[i];
+  if (__any_sync(0xffffffffu, sum != sum)) {  // NaN: of infinities met by hi and lo, or truly; the warp's keys once more tell which
+    __syncwarp();
+    for (int h = 0; h < g; h++)
+      attend_plain<D>(static_cast<const __nv_bfloat16 *>(a.q) + ((size_t)b * a.NH + (size_t)kh * g + h) * D, Kb, Vb, reinterpret_cast<const __nv_bfloat16 *>(fresh),
+                      append ? (int)pos : -1, roped ? trig : nullptr, sc, j0 + warp * 16, j1, mine + h * ROW);
   }
   __syncthreads();
   for (int idx = threadIdx.x; idx < g * D; idx += MA_THREADS) {

@@ -218,3 +218,33 @@ def test_f32_kernel(cuda, D, g, n, window):
     S = (q.double().reshape(B, KH, g, D) @ kb[:, :, s0:n].double().transpose(-1, -2) * D ** -0.5).softmax(-1)
     want = (S @ vb[:, :, s0:n].double()).reshape(B, KH * g, 1, D)
     assert (got.double() - want).abs().max() <= 1e-4 * v.abs().max()
+
+
+@pytest.mark.parametrize("D,g", [(64, 4), (64, 12), (128, 8), (128, 16)])
+@pytest.mark.parametrize("n,append", [(1, False), (37, False), (300, True), (2000, False)])
+def test_infinities_in_a_bf16_cache(cuda, D, g, n, append):
+    """An infinite value answers an infinity in its dimension alone; a key whose score is -inf counts for nothing; NaN stays NaN: what f32
+    arithmetic gives, in a kernel that splits its operands into two bf16 parts.  Against f64; the bf16 output's rounding remains."""
+    B, KH = 1, 2
+    gen = torch.Generator(device=cuda).manual_seed(n + g)
+    kb, vb = (torch.randn(B, KH, n + 1, D, generator=gen, device=cuda).bfloat16() for _ in range(2))
+    q = torch.randn(B, KH * g, 1, D, generator=gen, device=cuda).bfloat16()
+    q[..., 5] = q[..., 5].abs() + 0.5
+    k, v = (torch.randn(B, KH, 1, D, generator=gen, device=cuda).bfloat16() for _ in range(2))
+    inf = float("inf")
+    vb[0, 0, n // 2, 3] = inf
+    vb[0, 0, n - 1, 7] = -inf                               # the last row: read again for the places past it
+    kb[0, 1, : n // 2, 5] = -inf                            # the second head's first half: scores of -inf, whole blocks of them
+    vb[0, 1, n // 2, 9] = float("nan")
+    pos = torch.full((1,), n if append else n - 1, device=cuda)
+    new = (k, v) if append else (None, None)
+    got = ops.DecodeAttention(q, kb, vb, pos, D ** -0.5, 0, *new).double().reshape(KH, g, D)
+    m = int(pos) + 1
+    S = (q.double().reshape(KH, g, D) @ kb[0, :, :m].double().transpose(-1, -2) * D ** -0.5).softmax(-1)
+    want = S @ vb[0, :, :m].double()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[want.isinf()], want[want.isinf()])
+    fin = want.isfinite()
+    assert float((got[fin] - want[fin]).norm() / want[fin].norm()) <= 3e-3
+    if n > 1:
+        assert bool(want[0, :, 3].isinf().all()) and int(fin.sum()) >= KH * g * (D - 4)
