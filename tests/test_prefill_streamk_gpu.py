@@ -1,7 +1,9 @@
-"""The persistent tensor-core kernel (an even split of all K blocks over one CTA per SM, partial tiles summed in a fixed
-order) takes a call only where the split pays; here every shape of the prefill, int4 / block-FP8 and grouped (MoE) parity
-tests runs through it (LIGHT_B200_PREFILL_SK=2): one K block per CTA with a tile shared by eight of them, runs that start
-and end inside tiles, more CTAs than blocks (empty runs), ragged and empty expert groups; the status word stays zero."""
+"""The two tensor-core kernels that stage expanded weights in shared memory, which have the shapes that the tensor-memory kernel does not
+take (dense experts with K an odd multiple of 64, more than 1024 experts, a workspace without room for partial tiles).  With that
+kernel off (LIGHT_B200_TMEM=0) every shape of the prefill, int4 / block-FP8 and grouped (MoE) parity tests runs through them: the
+persistent one (LIGHT_B200_PREFILL_SK=2: an even split of all K blocks over one CTA per SM, partial tiles summed in a fixed order; one
+K block per CTA with a tile shared by eight of them, runs that start and end inside tiles, more CTAs than blocks (empty runs), ragged
+and empty expert groups) and the one with a CTA per tile (LIGHT_B200_PREFILL_SK=0); the status word stays zero."""
 import os
 import subprocess
 import sys
@@ -13,8 +15,9 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 FILES = ["test_prefill_gpu.py", "test_moe_gpu.py", "test_int4_fp8_gpu.py", "test_nn_gpu.py"]
 
 
-def test_parity_suites_through_the_persistent_kernel():
-    env = {**os.environ, "LIGHT_B200_PREFILL_SK": "2"}
+@pytest.mark.parametrize("sk", ["2", "0"])
+def test_parity_suites_through_the_older_kernels(sk):
+    env = {**os.environ, "LIGHT_B200_TMEM": "0", "LIGHT_B200_PREFILL_SK": sk}
     r = subprocess.run([sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider"] + [os.path.join(ROOT, "tests", f) for f in FILES],
                        capture_output=True, text=True, timeout=1500, env=env, cwd=ROOT)
     assert r.returncode == 0, r.stdout[-4000:] + r.stderr[-2000:]
@@ -36,6 +39,8 @@ print("CASE OK")
 """ % ROOT
 
 
-def test_same_bits_twice():
-    r = subprocess.run([sys.executable, "-c", CHILD], capture_output=True, text=True, timeout=600, env={**os.environ, "LIGHT_B200_PREFILL_SK": "2"})
+@pytest.mark.parametrize("sk", ["2", "0"])
+def test_same_bits_twice(sk):
+    r = subprocess.run([sys.executable, "-c", CHILD], capture_output=True, text=True, timeout=600,
+                       env={**os.environ, "LIGHT_B200_TMEM": "0", "LIGHT_B200_PREFILL_SK": sk})
     assert r.returncode == 0 and "CASE OK" in r.stdout, r.stdout + r.stderr[-3000:]
