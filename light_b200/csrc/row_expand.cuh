@@ -445,11 +445,6 @@ struct DenseRow {
     row = reinterpret_cast<const uint4 *>(c.w + ((size_t)e * N + n) * K);
   }
   __device__ __forceinline__ void prefetch(int u) const { prefetch_l2(row + (size_t)u * 8, 128); }
-  __device__ __forceinline__ static size_t row_stride(const Ctx &, int K) { return (size_t)K * 2; }
-  __device__ __forceinline__ void load_codes(uint32_t slot) {
-#pragma unroll
-    for (int i = 0; i < 8; i++) q[i] = lds128(slot + 16 * i);
-  }
   __device__ __forceinline__ void load(int u) {
 #pragma unroll
     for (int i = 0; i < 8; i++) q[i] = __ldg(row + (size_t)u * 8 + i);
