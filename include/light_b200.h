@@ -79,18 +79,23 @@ LB200_API unsigned long long light_b200_launch_count(void);
 /* Hands the library a per-device workspace it may use between calls on that device (device
  * memory, 1024-byte aligned, owned by the caller, valid until replaced; ptr = NULL withdraws it).
  * The reference keeps the same kind of buffer, one reusable weight scratch per device
- * (ops/fp8_block.go:105-154 weightScratch).  Here it holds the f16 copy of the activations that the
- * tensor-core prefill path streams by TMA: matmul_q with M > 64 needs M * K * 2 bytes; without a
- * large enough workspace such calls run the slower shape-generic kernel.  Batched decode (matmul_q and
- * matmul_q_multi_rows with 2 <= M <= 64 on Q4_K / Q6_K) keeps there the activations staged as f16 fragment
- * records and the split-K partial sums of its persistent grid.  Calls that use the workspace must not overlap
- * on the GPU. */
+ * (ops/fp8_block.go:105-154 weightScratch).  Who uses it, and for what:
+ *   matmul_q, _multi_rows   M > 64: the f16 copy of the activations that the tensor-core path streams by TMA (M * K * 2 bytes;
+ *                           without it the call runs a slower kernel) and partial tiles behind it; 2 <= M <= 64 of Q4_K, Q6_K and
+ *                           Q8_0: the activations staged as f16 and partial sums
+ *   int4_gemv               bf16 rows from 4 to 64 (staged as f16) and M > 64; f32 rows above 64
+ *   fp8_block_gemv          the same
+ *   moe_gemm, _q, _f8block  256 pairs or more: the gathered token rows, and partial tiles behind them.  Fewer pairs never use it
+ *                           (light_b200_moe_gemm_scratch below)
+ * One row (M = 1) never uses it.  Calls that use the workspace must not overlap on the GPU: neither on two streams nor in two
+ * branches of a graph. */
 LB200_API int light_b200_set_workspace(int device, void *ptr, size_t bytes);
 
 /* The workspace size with which light_b200_matmul_q / _multi_rows (and the int4, block-FP8 and grouped matmuls, M
- * then the number of activation rows or routed pairs) take their fastest path for M rows of K: above 64 rows the f16
- * copy of x plus about 42 MB of partial tiles for the persistent tensor-core kernel; with less, those calls run the
- * kernel that needs the copy alone. */
+ * then the number of activation rows or routed pairs) take their fastest path for M rows of K: the f16
+ * copy of x plus about 42 MB of partial tiles above 64 rows; with less, those calls run a kernel that needs the copy alone.  Up to
+ * 64 rows: what the token-tile kernels stage, or the f16 copy plus 21 MB where the tensor-memory kernel has such calls (Q8_0 from 4
+ * rows, bf16 rows of 4-bit weights from 17). */
 LB200_API unsigned long long light_b200_matmul_q_workspace_bytes(int M, int K);
 
 /* 0 if no bounded device-side wait of the tensor-core kernels ever gave up on this device, 1 if one

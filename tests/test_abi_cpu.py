@@ -98,3 +98,10 @@ def test_missing_library_fails_loudly(monkeypatch):
     monkeypatch.setattr(_lib, "LIB_PATH", "/nonexistent/liblight_b200.so")
     with pytest.raises(_lib.Light200Error, match="no CPU or PyTorch fallback"):
         _lib.lib()
+
+
+@pytest.mark.parametrize("M", [4, 17, 64, 65, 2048])
+@pytest.mark.parametrize("K", [256, 4096, 14336])
+def test_workspace_holds_the_partial_tiles_of_the_fastest_path(M, K):
+    """The f16 copy of the activations, rounded up to 1 KB, and behind it a 128 KB tile for each of 160 CTAs."""
+    assert _lib.lib().light_b200_matmul_q_workspace_bytes(M, K) >= (M * K * 2 + 1023) // 1024 * 1024 + 160 * 128 * 1024
