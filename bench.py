@@ -647,7 +647,7 @@ def moe_extras(device, peaks):
            "finite": bool(torch.isfinite(state["out"].float()).all().item()), "route_status": ops.moe_route_status(device.index or 0)}
     if "bf16_tflops" in peaks:  # the experts are expanded to bf16 for the tensor core: the bf16 peak bounds the matmuls
         res["layer_frac_of_measured_bf16_burst"] = res["layer_tflops"] / peaks["bf16_tflops"]
-    # the same block for one decode step's tokens (few pairs per expert: the warp-per-column kernel)
+    # the same block for one decode step's tokens (few pairs per expert)
     xd = x[:8].contiguous()
     rd = ops.MoERouteSigmoid(logits[:8].contiguous(), bias, topk, True)
 
@@ -657,8 +657,9 @@ def moe_extras(device, peaks):
 
     small()
     msd = timed(small, 5, 2, device, lambda: None) / 5
-    touched = 8 * topk * (2 * I * H + H * I)  # bytes of expert weights 64 pairs read (distinct experts assumed)
-    res["decode_8_tokens"] = {"ms": msd, "expert_bytes": touched, "gbs": touched / (msd * 1e-3) / 1e9}
+    used = int(rd.sorted_expts.unique().numel())
+    touched = used * (2 * I * H + H * I)  # bytes of the weights of the experts that the 64 pairs choose
+    res["decode_8_tokens"] = {"ms": msd, "experts": used, "expert_bytes": touched, "gbs": touched / (msd * 1e-3) / 1e9}
     del w1, w2, s1, s2
     torch.cuda.empty_cache()
     return res

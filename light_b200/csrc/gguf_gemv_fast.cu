@@ -1,26 +1,22 @@
-// Decode (few activation rows) fused dequant-matmul for Q4_K and Q6_K: HBM-bound GEMV.
+// Decode (few activation rows) fused dequant-matmul for Q4_K, Q6_K, Q8_0, 4-bit and block-FP8 weights: HBM-bound GEMV.
 //
-// The weights are read exactly once, coalesced, and never expanded to f32.  The arithmetic runs
-// on the tensor cores although this is a matrix-vector product:
+// The weights are read exactly once, coalesced, and never expanded.  The arithmetic runs on the tensor cores although this is a
+// matrix-vector product:
 //
-//   * a warp owns one 256-element K block and walks down RT tiles of 16 weight rows (the M of
-//     mma.m16n8k16), so the activations of its block are converted once and reused;
-//   * the packed integer codes become exact f16 values with one LOP3 / PRMT per pair of weights
-//     ((code bits) | magic exponent = offset + code) and form the A fragment directly in
-//     registers -- no int -> float conversion, no per-weight scale multiply, no CUDA-core FMA;
-//   * the eight columns of the MMA are not eight tokens but EIGHT SUB-BLOCKS: the B fragment
-//     holds the activations block-diagonally, B[k][c] = x[k] if element k lies in sub-block c,
-//     else 0.  D[row][c] is then sum_{k in sub-block c} (offset + code) * x[k], the per-sub-block
-//     integer dot product that a scale applies to, accumulated over the whole 256-element block
-//     by the tensor core.  The CUDA cores touch each (row, sub-block) once:
+//   * a warp owns one 256-element K block and walks down a list of tiles of 16 weight rows (the M of the MMA), so the
+//     activations of its block are prepared once and reused;
+//   * one row, GGUF and 4-bit: whole numbers.  The activations of a block become 31-bit fixed point in four signed bytes, the
+//     limbs, and mma.m16n8k32 multiplies the weights' codes, as bytes, with them exactly (stage_limbs below);
+//   * one row of FP8, and the kernels for a few rows: codes become exact f16 values with one LOP3 / PRMT per pair of weights
+//     ((code bits) | magic exponent = offset + code) and form the A fragment of mma.m16n8k16 directly in registers, x as
+//     f16 hi + lo after an exact power-of-two prescale (one row) or rounded to f16 (several);
+//   * the columns of the MMA are not tokens (one row) but SUB-BLOCKS: the B fragment holds the activations block-diagonally, and
+//     D is the dot product of whole codes that a scale applies to.  The CUDA cores touch each (row, sub-block) once:
 //         acc += (d*sc) * (D - offset * Sx) - (dmin*m) * Sx,     Sx = sum of x over the sub-block;
-//   * lane (g, t) of the warp ends up holding exactly the D columns whose scales it decoded
-//     (sub-blocks 2t and 2t+1 of rows g and g+8), so there is no cross-lane traffic until the
-//     final reduction;
-//   * activations stay f32-accurate: x is split as f16 hi + f16 lo (two MMAs into the same
-//     accumulator) after an exact power-of-two prescale that keeps it inside f16 range.
+//   * a lane ends up holding exactly the D columns whose scales it decoded, so there is no cross-lane traffic until the
+//     final reduction.
 //
-// A CTA covers 16*RT rows and all of K (its warps take K blocks round-robin and reduce through
+// A CTA covers whole tiles and all of K (its warps take K blocks round-robin and reduce through
 // shared memory), so every output element is written once, deterministically, without atomics.
 // The kernels are launched with programmatic dependent launch: the first weight tile is
 // requested before griddepcontrol.wait, so the head of each launch overlaps the tail of the one
@@ -1191,7 +1187,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float
 // eight blocks = 272 bytes = 17 granules per row, rows are whole granules (K % 256 == 0), and a 272-byte pitch puts rows g and lanes t
 // on 32 different banks and the granules of a tile one behind the other.  Pairs of blocks are the sub-blocks A and B of two MMAs; their
 // f16 scales multiply V.  Loads from shared memory were the bound (49 % of the cycles with x as f16 hi + lo: codes, and sixteen B
-// fragments a tile); B now stays in registers.  28672 x 4096: 25.5 -> 22.5 us.  reference: matmul_q8_0_f32_mv,
+// fragments a tile); B now stays in registers.  28672 x 4096: 25.1 -> 22.9 us.  reference: matmul_q8_0_f32_mv,
 // kernels/cuda/src/matmul_q.cu:58-431.
 constexpr int Q80_PITCH = 272;
 constexpr int Q80_TILE_BYTES = ROWS * Q80_PITCH;
@@ -1526,7 +1522,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) fp8_gemv_mma_kernel(const XT *_
 // (N, K/G)) through the Q4_K arithmetic: the low nibbles of a code word, as bytes, are four even-numbered elements (A), the high ones
 // left in place four odd-numbered ones (B), and the whole-number sums of 64 elements, which share a scale, meet in one lane of four:
 // acc += s (sum - z Sx).  Structure as the Q8_0 kernel (per-warp ring, activations staged per run of 256 k, so any K fits); a 144-byte
-// row pitch keeps ldmatrix on 32 banks.  28672 x 4096: 21.6 -> 16.5 us.  Needs G % 64 == 0 and K % 256 == 0.  reference:
+// row pitch keeps ldmatrix on 32 banks.  28672 x 4096: 20.0 -> 17.0 us.  Needs G % 64 == 0 and K % 256 == 0.  reference:
 // int4_gemv_f32 / _bf16, kernels/cuda/src/int4.cu:43-106.
 constexpr int I4_PITCH = 144;
 constexpr int I4_TILE_BYTES = ROWS * I4_PITCH;
