@@ -173,3 +173,30 @@ def test_scratch_of_a_call_may_hold_anything(cuda):
         assert L.light_b200_moe_gemm_scratch(C.byref(a), None, 0, 0, C.c_void_p(scratch.data_ptr() + 64), nbytes, 0, None) == -4   # not on 256 bytes
         assert bool((scratch[nbytes // 4:] == fill).all())
     assert ops.prefill_status(0) == 0
+
+
+@pytest.mark.parametrize("T,N", [(8, 512), (600, 4096)])   # few pairs in memory of the call's own; 4800 pairs with rows looked for
+def test_grouped_calls_in_a_graph(cuda, T, N):
+    E, topk, K = 16, 8, 1024
+    g = torch.Generator().manual_seed(T)
+    codes, scale = synth.random_fp8_block(2, E * N, K, device=cuda)
+    codes, scale = codes.reshape(E, N, K), scale.reshape(E, N // 128, K // 128)
+    x = torch.randn(T, K, generator=g).to(cuda, torch.bfloat16)
+    logits = torch.randn(T, E, generator=g).to(cuda)
+
+    def block():
+        r = ops.MoERouteSigmoid(logits, None, topk)
+        return ops.MoECombine(ops.MoEGemmF8Block(x, codes, scale, 128, 128, r, r.weights, topk), topk)
+
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        block()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            y = block()
+    for _ in range(3):                                      # other tokens and another routing at every replay
+        x.copy_(torch.randn(T, K, generator=g)), logits.copy_(torch.randn(T, E, generator=g))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, block())
+    assert ops.prefill_status(0) == 0
