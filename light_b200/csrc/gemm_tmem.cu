@@ -14,9 +14,13 @@
 //                registers (the slot then takes the next copy) and leave as 64 TMEM columns.  Expansion is a chain of
 //                short dependent instructions: two warps per row quarter instead of four ran it at 4 to 8 clocks each
 //                and set the pace wherever a tile had few tokens (4-bit rows at 2048 tokens: 1092 against 1335 TFLOP/s).
-//   warp  16     one lane: TMA of the token tiles.
-//   warp  17     MMAs and commits; in the second CTA of a pair: forwards "my half is ready" to the first.
-//   warps 18-21  epilogue, while the next tile's MMAs run (token tiles up to 128 use two accumulators): TMEM -> registers ->
+//   warps 16-17  one lane of each: TMA of the token tiles, 64 of a unit's 128 k to each warp, one box to a unit.  (One lane for
+//                both halves, in boxes of 16 or 32 tokens where groups are ragged, chosen by its number instead of elected so that
+//                operands went through vector registers: 240 clocks to a box, 470 to 730 per unit, and the MMAs of a tile of few
+//                tokens waited for those: 64 bf16 pairs over 64 experts of 4096 x 7168 247 -> 220 us, with 128 tokens to an expert
+//                744 -> 704, Q4_K experts of 1536 x 2048 with 5 tokens each 109 -> 95.)
+//   warp  18     MMAs and commits; in the second CTA of a pair: forwards "my half is ready" to the first.
+//   warps 19-22  epilogue, while the next tile's MMAs run (token tiles up to 128 use two accumulators): TMEM -> registers ->
 //                a [token][row] strip in shared memory -> one bulk copy per token.  The run's last segment is finished by
 //                the expanders too, five warps to a row quarter, each 16 tokens at a time.
 //
@@ -40,7 +44,7 @@ namespace {
 
 using namespace umma;
 
-constexpr int EXPANDERS = 16, TMA_WARP = 16, MMA_WARP = 17, EPI_WARP = 18, THREADS = 22 * 32;
+constexpr int EXPANDERS = 16, TMA_WARP = 16, MMA_WARP = 18, EPI_WARP = 19, THREADS = 23 * 32;
 constexpr int KU = 128;                       // k of a unit: one TMEM stage, one stage of the token ring
 constexpr int NAS = 4;                        // stages of expanded weights: 128 k, 64 TMEM columns each
 constexpr int NBS = 12;                       // most stages of the token ring, 128 k each
@@ -48,6 +52,7 @@ constexpr int A_COL = 256;                    // columns 0-255: accumulators, 25
 constexpr int MAX_E = 1024;                   // experts whose prefix sums fit the shared tables
 constexpr int MAX_GRID = 160;
 constexpr int BAR_BYTES = 640;                // barriers
+constexpr int MAX_ROWS = 128;                 // most token rows of a stage (one SM's)
 constexpr int PART_FLOATS = 256 * 128;        // one partial tile: [token][row]
 constexpr int SMEM_MAX = 227 * 1024 - 1024;   // dynamic; the static part (prefix tables, flags) is accounted below
 
@@ -68,7 +73,6 @@ struct Args {
   long long size_m;
   int E, M, N, K;
   int nt_max;               // most tokens of a tile
-  int box;                  // token rows of one TMA box
   int stage_bytes, nbs;     // of the token ring, per CTA
   int wmin;                 // grouped: a unit's weight is max(tokens of its tile, wmin)
   struct Sync *sync;
@@ -279,7 +283,7 @@ template <typename OutT>
 constexpr int STRIPS = 2 * STRIP<OutT>;
 
 struct Maps {
-  CUtensorMap x, w[2];  // tokens; the weight rows, per box of the format
+  CUtensorMap x[MAX_ROWS / 16], w[2];  // tokens, by the rows of a box (16, 32, ..); the weight rows, per box of the format
 };
 
 template <typename Row, bool BF16, typename OutT, int CG>
@@ -305,12 +309,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   const int G = gridDim.x / CG, cta = blockIdx.x / CG;
 
   if (threadIdx.x == 0) {
-    prefetch_tmap(&maps.x);
+    if (!a.offsets) prefetch_tmap(&maps.x[a.nt_max / CG / 16 - 1]);
     if constexpr (Row::BOXES > 0) prefetch_tmap(&maps.w[0]);
     if constexpr (Row::BOXES > 1) prefetch_tmap(&maps.w[1]);
     abort_flag = 0;
     for (int i = 0; i < NAS; i++) mbar_init(full + 8 * i, CG == 2 && rank == 0 ? 5 : 4), mbar_init(empty + 8 * i, 1);
-    for (int i = 0; i < a.nbs; i++) mbar_init(t_full + 8 * i, 1), mbar_init(t_empty + 8 * i, 1);
+    for (int i = 0; i < a.nbs; i++) mbar_init(t_full + 8 * i, 2), mbar_init(t_empty + 8 * i, 1);
     for (int i = 0; i < 2; i++) mbar_init(d_full + 8 * i, 1), mbar_init(d_empty + 8 * i, 4 * CG);
     mbar_init(drained, 1), mbar_init(tagged, 1);
     for (int i = 0; i < EXPANDERS; i++) mbar_init(w_full + 8 * i, 1);
@@ -359,25 +363,28 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   const int n = dealt ? (total > cta ? (total - 1 - cta) / G + 1 : 0) * nb : wk.bound(cta + 1, G) - pos0;
   const int v1 = v0 + n;
 
-  if (warp == TMA_WARP) {
-    if (lane == 0) {
+  if (warp >= TMA_WARP && warp < MMA_WARP) {
+    if (elect_one()) {
       pdl_wait();  // the tokens may be the kernel before's; the weights are not
+      const int half = warp - TMA_WARP;
+      const uint32_t first = sB + half * (a.stage_bytes / 2);
+      uint32_t dst = first;
       int bt = 0, par = 1;
       bool wrapped = false;
       auto W = wk.walk(tf);
       for (int v = v0; v < v1 && !*abort; wk.next(W, stride)) {
         const int u0 = v % nb, u1 = min(nb, u0 + (v1 - v));
         const Tile T = wk.tile(W);
-        const int rows = T.nt / CG, boxes = (rows + a.box - 1) / a.box, y0 = T.m0 + rank * rows;
-        const uint32_t bytes = (uint32_t)(boxes * a.box) * 256u;
-        for (int u = u0; u < u1; u++) {
+        const int rows = T.nt / CG, y = T.m0 + rank * rows;
+        const CUtensorMap *const map = &maps.x[rows / 16 - 1];
+        int x = u0 * 128 + half * 64;
+        for (int u = u0; u < u1; u++, x += 128) {
+          const uint32_t bar = t_full + 8 * bt;
           if (wrapped && !mbar_sleep_wait(t_empty + 8 * bt, par) && !mbar_wait(t_empty + 8 * bt, par, abort)) break;
-          mbar_arrive_expect_tx(t_full + 8 * bt, bytes);
-          for (int i = 0; i < 2 * boxes; i++) {
-            const int h = i & 1, bx = i >> 1;
-            tma_load_2d(sB + bt * a.stage_bytes + h * (a.stage_bytes / 2) + bx * a.box * 128, &maps.x, t_full + 8 * bt, u * 128 + h * 64, y0 + bx * a.box);
-          }
-          if (++bt == a.nbs) bt = 0, par ^= 1, wrapped = true;
+          mbar_arrive_expect_tx(bar, (uint32_t)rows * 128u);
+          tma_load_2d(dst, map, bar, x, y);
+          dst += a.stage_bytes;
+          if (++bt == a.nbs) bt = 0, par ^= 1, wrapped = true, dst = first;
         }
         v += u1 - u0;
       }
@@ -593,7 +600,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       };
       auto issue = [&]() {
         if constexpr (Row::BOXES > 0) {
-          if (lane == 0) {
+          if (elect_one()) {
             mbar_arrive_expect_tx(copied, Row::BYTES);
             Row::copy(slot, maps.w, copied, u, y);
           }
@@ -796,8 +803,7 @@ template <typename Row, bool BF16, typename OutT, int CG>
 int run(const typename Row::Ctx &ctx, const TmemCall &c, Args a, int nt_max, cudaStream_t st) {
   a.nt_max = nt_max;
   const int rows = nt_max / CG;
-  a.box = !c.offsets ? rows : rows % 32 ? 16 : 32;
-  a.stage_bytes = (rows + a.box - 1) / a.box * a.box * 256;
+  a.stage_bytes = rows * 256;
   a.nbs = (SMEM_MAX - fixed_smem<Row, OutT>(a.E)) / a.stage_bytes;
   if (a.nbs > NBS) a.nbs = NBS;
   if (a.nbs < 3) return 0;
@@ -815,13 +821,16 @@ int run(const typename Row::Ctx &ctx, const TmemCall &c, Args a, int nt_max, cud
   a.parts = (float *)c.parts, a.sync = (Sync *)c.sync;
   const EncodeTiledFn enc = encode_fn();
   if (!enc) return fail(LB200_E_DEVICE, "light_b200: cuTensorMapEncodeTiled is not available from the driver");
-  Maps tm;
+  Maps tm = {};
   const cuuint64_t dims[2] = {(cuuint64_t)c.K, (cuuint64_t)c.M};
   const cuuint64_t strides[1] = {(cuuint64_t)c.K * 2};
-  const cuuint32_t box[2] = {64, (cuuint32_t)a.box}, estr[2] = {1, 1};
-  CUresult r = enc(&tm.x, BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(c.x16), dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  tm.w[0] = tm.w[1] = tm.x;
+  const cuuint32_t estr[2] = {1, 1};
+  CUresult r = CUDA_SUCCESS;
+  for (int i = c.offsets ? 16 : rows; i <= rows && r == CUDA_SUCCESS; i += 16) {  // (one matrix: all its tiles are alike)
+    const cuuint32_t box[2] = {64, (cuuint32_t)i};
+    r = enc(&tm.x[i / 16 - 1], BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(c.x16), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  }
   if constexpr (Row::BOXES > 0) {
     const cuuint64_t wdims[2] = {(cuuint64_t)Row::stride(c.K), (cuuint64_t)a.E * c.N}, wstr[1] = {wdims[0]};
     for (int i = 0; i < Row::BOXES && r == CUDA_SUCCESS; i++) {
