@@ -20,9 +20,12 @@
 //                tokens waited for those: 64 bf16 pairs over 64 experts of 4096 x 7168 247 -> 220 us, with 128 tokens to an expert
 //                744 -> 704, Q4_K experts of 1536 x 2048 with 5 tokens each 109 -> 95.)
 //   warp  18     MMAs and commits; in the second CTA of a pair: forwards "my half is ready" to the first.
-//   warps 19-22  epilogue, while the next tile's MMAs run (token tiles up to 128 use two accumulators): TMEM -> registers ->
-//                a [token][row] strip in shared memory -> one bulk copy per token.  The run's last segment is finished by
-//                the expanders too, five warps to a row quarter, each 16 tokens at a time.
+//   warps 19-22  epilogue, while the next tile's MMAs run (token tiles up to 128 use two accumulators; beyond, the MMAs wait until the
+//                last chunk is out of tensor memory): TMEM -> registers -> a [token][row] strip of the warp's own in shared memory
+//                -> a box of 16 tokens, or 16 bytes a lane where tokens go to rows of their own.  (One strip for the four warps, two
+//                barriers and a bulk copy per token: 1600 clocks for 32 tokens; Q4_K 28672 x 4096, 2048 tokens 388 -> 375 us, a
+//                4-bit layer of 4096 tokens 1830 -> 1786.)  The run's last segment is finished by the expanders too, five warps to
+//                a row quarter, each 16 tokens at a time.
 //
 // Work is the list of (tile, K chunk) pairs, cut into equal runs, one per CTA (pair): stream-K.  A segment that does not
 // start its tile writes a partial tile and sets its flags to the launch's tag, which it does first; the segment that starts the
@@ -119,19 +122,6 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatil
     }
   }
   return true;
-}
-// The four epilogue warps, together: whether all of them are to go on.
-__device__ __forceinline__ bool epilogue_all(bool go) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %1, 0;\n\t"
-      "bar.red.and.pred q, 1, 128, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}\n"
-      : "=r"(r)
-      : "r"((uint32_t)go)
-      : "memory");
-  return r != 0;
 }
 __device__ __forceinline__ void st_if(bool p, float *o, float v) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.f32 [%0], %1;\n\t}\n" ::"l"(o), "f"(v), "r"((int)p) : "memory");
@@ -284,6 +274,7 @@ constexpr int STRIPS = 2 * STRIP<OutT>;
 
 struct Maps {
   CUtensorMap x[MAX_ROWS / 16], w[2];  // tokens, by the rows of a box (16, 32, ..); the weight rows, per box of the format
+  CUtensorMap out;                     // one matrix: 16 tokens of 32 output columns
 };
 
 template <typename Row, bool BF16, typename OutT, int CG>
@@ -692,7 +683,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       }
       __syncwarp();
       warp_wait(tagged, 0, abort);
-      const uint32_t strip = sStrip, sbytes = STRIP<OutT>;
+      constexpr uint32_t SB = STRIP<OutT> / 4;  // of one warp
+      const uint32_t strip = sStrip + 2 * SB * quad;
       const bool bulk = ((size_t)a.N * sizeof(OutT)) % 16 == 0 && ((uintptr_t)out & 15) == 0;
       int seg = 0, chunk = 0;
       auto W = wk.walk(tf);
@@ -704,11 +696,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
           finish_last(0, shared ? 80 : 16);
           break;
         }
-        // The barriers of the chunks below want all four warps: one that gives up alone would leave the others waiting for good.
-        if (!epilogue_all(warp_wait(d_full + 8 * (seg & 1), (seg >> 1) & 1, abort))) break;
+        if (!warp_wait(d_full + 8 * (seg & 1), (seg >> 1) & 1, abort)) break;
         tc_fence_after();
         const uint32_t d = tmem + lanes + (T.nt > 128 ? 0 : 128 * (seg & 1));
-        const int n0 = T.n0 + 128 * rank, ncols = min(128, a.N - n0);  // (<= 0: no rows of the matrix here)
+        const int n0 = T.n0 + 128 * rank + 32 * quad;  // the warp's first output column (beyond N: no rows of the matrix here)
 #pragma unroll 1
         for (int c0 = 0; c0 < T.nt; c0 += 32, chunk++) {
           uint32_t v[32];
@@ -734,33 +725,46 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
 #pragma unroll
             for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * __shfl_sync(0xffffffffu, pw, i));
           }
-          if (bulk) {
-            const uint32_t buf = strip + (chunk & 1) * sbytes;
-            asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");  // this lane's last copy from this strip
-            asm volatile("bar.sync 1, 128;\n" ::: "memory");
+          if (bulk) {  // through a strip of the warp's own: [32 tokens][32 rows], no other warp to wait for
+            const uint32_t buf = strip + (chunk & 1) * SB;
+            asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory");  // this lane's copies from this strip, if any (every lane closes a group per chunk)
+            __syncwarp();
 #pragma unroll
             for (int i = 0; i < 32; i++) {
               if constexpr (sizeof(OutT) == 4) {
-                asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(buf + (uint32_t)(i * 128 + row) * 4u), "r"(v[i]) : "memory");
+                asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(buf + (uint32_t)(i * 32 + lane) * 4u), "r"(v[i]) : "memory");
               } else {
                 const __nv_bfloat16 h = __float2bfloat16_rn(__uint_as_float(v[i]));
-                asm volatile("st.shared.u16 [%0], %1;\n" ::"r"(buf + (uint32_t)(i * 128 + row) * 2u), "h"(*reinterpret_cast<const uint16_t *>(&h)) : "memory");
+                asm volatile("st.shared.u16 [%0], %1;\n" ::"r"(buf + (uint32_t)(i * 32 + lane) * 2u), "h"(*reinterpret_cast<const uint16_t *>(&h)) : "memory");
               }
             }
-            fence_proxy_async();
-            asm volatile("bar.sync 1, 128;\n" ::: "memory");
-            const int i = (warp - EPI_WARP) * 8 + (lane & 7), m = __shfl_sync(0xffffffffu, prow, i);  // a warp sends eight of the 32 tokens
-            if (lane < 8 && m >= 0 && ncols > 0)
-              asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(out + (long long)m * a.N + n0),
-                           "r"(buf + (uint32_t)(i * 128) * (uint32_t)sizeof(OutT)), "r"((uint32_t)ncols * (uint32_t)sizeof(OutT))
-                           : "memory");
-            asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+            if (!a.offsets) {
+              fence_proxy_async();
+              __syncwarp();
+#pragma unroll
+              for (int j = 0; j < 2; j++)  // (16 tokens each: a tile's last chunk may hold no more, and what follows is the next tile's)
+                if (n0 < a.N && T.m0 + c0 + 16 * j < T.m_end && elect_one())
+                  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];\n" ::"l"(&maps.out), "r"(buf + j * (SB / 2)), "r"(n0),
+                               "r"(T.m0 + c0 + 16 * j)
+                               : "memory");
+              asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+            } else {
+              constexpr int LPT = 2 * (int)sizeof(OutT);  // lanes to a token, 16 bytes each
+              const int seg16 = lane % LPT, n = n0 + seg16 * (32 / LPT);
+              __syncwarp();
+#pragma unroll
+              for (int i = lane / LPT; i < 32; i += 32 / LPT) {
+                const int m = __shfl_sync(0xffffffffu, prow, i);
+                const uint4 q = lds128(buf + (uint32_t)(i * LPT + seg16) * 16u);
+                if (m >= 0 && n < a.N) *reinterpret_cast<uint4 *>(out + (long long)m * a.N + n) = q;
+              }
+            }
           } else {
-            OutT *o = out + n0 + row;
+            OutT *o = out + n0 + lane;
 #pragma unroll
             for (int i = 0; i < 32; i++) {
               const int m = __shfl_sync(0xffffffffu, prow, i);
-              st_if(row < ncols && m >= 0, o + (long long)m * a.N, __uint_as_float(v[i]));
+              st_if(n0 + lane < a.N && m >= 0, o + (long long)m * a.N, __uint_as_float(v[i]));
             }
           }
         }
@@ -830,6 +834,12 @@ int run(const typename Row::Ctx &ctx, const TmemCall &c, Args a, int nt_max, cud
     const cuuint32_t box[2] = {64, (cuuint32_t)i};
     r = enc(&tm.x[i / 16 - 1], BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(c.x16), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  }
+  if (!c.offsets && ((size_t)c.N * sizeof(OutT)) % 16 == 0 && ((uintptr_t)c.out & 15) == 0 && r == CUDA_SUCCESS) {  // (as the kernel has it: else plain stores)
+    const cuuint64_t odims[2] = {(cuuint64_t)c.N, (cuuint64_t)c.M}, ostr[1] = {(cuuint64_t)c.N * sizeof(OutT)};
+    const cuuint32_t obox[2] = {32, 16};
+    r = enc(&tm.out, sizeof(OutT) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, c.out, odims, ostr, obox, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   }
   if constexpr (Row::BOXES > 0) {
     const cuuint64_t wdims[2] = {(cuuint64_t)Row::stride(c.K), (cuuint64_t)a.E * c.N}, wstr[1] = {wdims[0]};
