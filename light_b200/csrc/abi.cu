@@ -148,8 +148,8 @@ int light_b200_matmul_q_tp(int t, const float *x, const void *const *w, float *c
 
 int light_b200_prefill_status(int device) {
   if (int rc = bind(device)) return rc;
-  const int a = prefill_status(device), b = decode_umma_status(), c = decode_nt_status(), d = decode_ts_status(), e = gemm_tmem_status();
-  return a ? a : b ? b : c ? c : d ? d : e;
+  const int a = prefill_status(device), b = decode_umma_status(), c = decode_nt_status(), d = decode_ts_status(), e = gemm_tmem_status(), f = q6k_limbs_status();
+  return a ? a : b ? b : c ? c : d ? d : e ? e : f;
 }
 unsigned long long light_b200_matmul_q_workspace_bytes(int M, int K) {
   if (M < 1 || K <= 0) return 0;
@@ -158,6 +158,7 @@ unsigned long long light_b200_matmul_q_workspace_bytes(int M, int K) {
   else if (M >= 4) f16_copy = ((f16_copy + 1023) & ~1023ull) + gemm_tmem_parts_bytes();  // those of the tensor-memory kernel (Q8_0, 4-bit)
   unsigned long long staged = M <= 64 ? decode_nt_ws_bytes(M, K) : 0;
   if (M <= 64 && decode_ts_ws_bytes(M, K) > staged) staged = decode_ts_ws_bytes(M, K);
+  if (M > 64 && K % 256 == 0 && (K >> 8) % 2 && q6k_limbs_ws_bytes(M, K) > f16_copy) f16_copy = q6k_limbs_ws_bytes(M, K);  // Q6_K rows that start on any even byte
   return f16_copy > staged ? f16_copy : staged;
 }
 unsigned long long light_b200_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
@@ -213,7 +214,7 @@ int light_b200_matmul_q(int t, const float *x, const void *w, float *out, int M,
   if (took != 0) return took == 1 ? 0 : took;
   took = gguf_gemv_batch(t, x, w, out, M, N, K, st);
   if (took != 0) return took == 1 ? 0 : took;
-  if (t == LB200_Q6_K && M > 64 && K % 256 == 0) return q6k_rows_dense(x, w, out, M, N, K, st);  // rows off 4-byte boundaries, or no workspace
+  if (t == LB200_Q6_K && M > 64 && K % 256 == 0) return q6k_rows_dense(x, w, out, M, N, K, device, st);  // rows off 4-byte boundaries, or no workspace
   return gguf_matmul_generic(t, x, w, out, M, N, K, st);
 }
 

@@ -12,6 +12,7 @@
 
 #include "gguf_decode.cuh"
 #include "mma_sync.cuh"
+#include "umma.cuh"
 
 namespace lb {
 
@@ -363,6 +364,311 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) q6k_rows_kernel(const float
   }
 }
 
+// ------------------------------------------------------------------------------------ the same products in whole numbers
+//
+// What bounds q6k_rows_kernel is f32 issue: eight multiply-adds per lane, token and weight row for every block.  Here a block's 256
+// activations become 31-bit fixed point, as in the one-row kernels, cut into three signed whole numbers of 11 bits (LIMBS), which f16 holds,
+// as it does a code.  One MMA (m16n8k16: 16 rows, 8 tokens, one limb) is then a sub-block's exact sum: three of them and 12 f32 operations
+// a lane (limbs together, times the sub-block's scale) replace 64 multiply-adds, and rounding starts where those 12 do.  Building
+// the operand takes some 900 of the 1550 instructions per 16 rows, block and 16 tokens, and issue is what bounds this kernel
+// (61 % of the slots, the tensor pipe 30 %).
+//   616 pairs over 128 experts of 2048 x 768:  247 -> 117 us;   2048 rows of 4096 x 14080:  16.2 -> 5.4 ms;   65 rows of 4096 x 2816:
+//   110 -> 68 us.  Blocks are added with their rounding errors kept (5 % of the time): 2.1e-8 to 3.6e-8 off against 64 bits where the f32
+//   sums were 5.3e-8 to 1.3e-7 off (K = 256 to 14080; without, 1.1e-7 at 11008).
+// Tried: limbs of eight bits and the integer MMAs (m16n8k32), 194 us and 19.5 ms: they run at a fraction of the f16 rate here; limbs
+// straight from L2, 152 us and 8.8 ms; 32 rows to a warp and half the warps, 115 us and 5.5 ms.
+// Tokens with infinities or NaN (whose limbs mean nothing; their power of two is NaN) are multiplied again in f32.
+constexpr int LIMB_RECORD = 1536;  // a token's block: [sub-block][t][limbs 0, 1 of four k], then [sub-block][t][limb 2 of four k]
+constexpr int LIMB_PASS = 16, LIMB_WARPS = 8, LIMB_RT = 1, LIMB_ROWS = 16 * LIMB_RT;
+constexpr int LIMB_RING = 2, LIMB_PITCH = 240, LIMB_SLOT = LIMB_ROWS * LIMB_PITCH;  // blocks of a warp's rows on their way
+constexpr int LIMB_TOKEN = LIMB_RECORD + 64, LIMB_STAGE = LIMB_PASS * LIMB_TOKEN;   // the pass's tokens, in shared memory for all warps; the pad
+                                                                                   // puts neighbours' 64 bytes on different banks
+constexpr int LIMB_SMEM = LIMB_WARPS * LIMB_RING * LIMB_SLOT + 2 * LIMB_STAGE;      // (two CTAs to an SM)
+__device__ int g_limb_status;  // non-zero: a bounded wait gave up (sticky)
+
+__global__ void __launch_bounds__(256) x_limbs_kernel(const float *__restrict__ in, const int64_t *__restrict__ pairs, uint8_t *__restrict__ limbs, float *__restrict__ ups,
+                                                      long long M, int K, int topk, int row_per_pair, long long size_m) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int nb = K >> 8, lane = threadIdx.x & 31;
+  const long long rec = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (rec >= M * nb) return;
+  const long long i = rec / nb;
+  const int b = (int)(rec - i * nb);
+  long long p = pairs ? pairs[i] : i;
+  if (p < 0 || p >= size_m) p = 0;  // (not stored)
+  const float4 *x = reinterpret_cast<const float4 *>(in + (size_t)(row_per_pair ? p : p / topk) * K + b * 256);
+  const float4 v[2] = {__ldg(x + lane), __ldg(x + lane + 32)};
+  uint32_t m = 0;
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+    m = max(max(m, max(__float_as_uint(v[j].x) & 0x7fffffffu, __float_as_uint(v[j].y) & 0x7fffffffu)),
+            max(__float_as_uint(v[j].z) & 0x7fffffffu, __float_as_uint(v[j].w) & 0x7fffffffu));
+  m = __reduce_max_sync(0xffffffffu, m);
+  const int s = min(156 - (int)(m >> 23), 126);  // |x| 2^s < 2^30
+  const float scale = __uint_as_float((uint32_t)(127 + s) << 23);
+  if (lane == 0) ups[rec] = m >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : __uint_as_float((uint32_t)(127 - s) << 23);
+  uint8_t *dst = limbs + (size_t)rec * LIMB_RECORD;
+#pragma unroll
+  for (int j = 0; j < 2; j++) {  // elements 128 j + 4 lane ..: sub-block 8 j + lane / 4, t = lane % 4
+    const float xs[4] = {v[j].x * scale, v[j].y * scale, v[j].z * scale, v[j].w * scale};
+    uint32_t l[3][2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      float f[3][2];
+#pragma unroll
+      for (int c = 0; c < 2; c++) {  // X = l0 + 2^11 l1 + 2^22 l2, l0 and l1 in [-1024, 1023]
+        const int X = __float2int_rn(xs[2 * k + c]), l0 = ((X + 1024) & 2047) - 1024, X1 = (X - l0) >> 11, l1 = ((X1 + 1024) & 2047) - 1024;
+        f[0][c] = (float)l0, f[1][c] = (float)l1, f[2][c] = (float)((X1 - l1) >> 11);
+      }
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const __half2 h = __floats2half2_rn(f[c][0], f[c][1]);
+        l[c][k] = *reinterpret_cast<const uint32_t *>(&h);
+      }
+    }
+    const int at = (8 * j + (lane >> 2)) * 4 + (lane & 3);
+    *reinterpret_cast<uint4 *>(dst + at * 16) = make_uint4(l[0][0], l[0][1], l[1][0], l[1][1]);
+    *reinterpret_cast<uint2 *>(dst + 1024 + at * 8) = make_uint2(l[2][0], l[2][1]);
+  }
+}
+
+__device__ __forceinline__ void mma_from_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+
+__global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const float *__restrict__ in, const uint8_t *__restrict__ w, const uint8_t *__restrict__ limbs,
+                                                                   const float *__restrict__ ups, const int64_t *__restrict__ pairs, const int32_t *__restrict__ offsets,
+                                                                   const float *__restrict__ topkw, float *__restrict__ out, long long M, long long size_m, int E, int N,
+                                                                   int K, int topk, int row_per_pair) {
+  extern __shared__ __align__(16) unsigned char ring_mem[];
+  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ int abort_flag;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, e = blockIdx.y;
+  const uint32_t bar0 = umma::smem_u32(bars), stages = umma::smem_u32(ring_mem) + LIMB_WARPS * LIMB_RING * LIMB_SLOT;
+  if (threadIdx.x == 0) {
+    umma::mbar_init(bar0, 1), umma::mbar_init(bar0 + 8, 1);
+    umma::fence_barrier_init();
+    abort_flag = 0;
+  }
+  pdl_launch_dependents();
+  pdl_wait();
+  __syncthreads();
+  const long long i0 = offsets ? offsets[e] : 0, i1 = offsets ? offsets[e + 1] : M;
+  if (i0 + (long long)blockIdx.z * LIMB_PASS >= i1) return;
+  const int r0 = min((int)(blockIdx.x * LIMB_WARPS + warp) * LIMB_ROWS, N - LIMB_ROWS), nb = K >> 8;  // the last rows are pulled back: duplicates store equal values
+  const size_t row_bytes = (size_t)nb * 210;
+  const uint8_t *const rows = w + ((size_t)e * N + r0) * row_bytes, *const w_end = w + (size_t)E * N * row_bytes;
+  const uint32_t ring = umma::smem_u32(ring_mem) + warp * (LIMB_RING * LIMB_SLOT);
+  const uint32_t skew0 = (uint32_t)(uintptr_t)(rows + g * row_bytes);  // (rows g, g + 8, .. lie multiples of 16 bytes apart)
+  // Lanes 0 .. 13 / 16 .. 29 copy the 14 granules that cover a block of rows 2 i / 2 i + 1.
+  auto issue = [&](int b, int slot) {
+    if ((lane & 15) < 14 && b < nb) {
+      const uint8_t *at = rows + (size_t)(lane >> 4) * row_bytes + (size_t)b * 210;
+      uint32_t dst = ring + slot * LIMB_SLOT + (lane >> 4) * LIMB_PITCH + (lane & 15) * 16;
+#pragma unroll 4
+      for (int i = 0; i < LIMB_ROWS / 2; i++, at += 2 * row_bytes, dst += 2 * LIMB_PITCH) {
+        const uint8_t *src = reinterpret_cast<const uint8_t *>((uintptr_t)at & ~(uintptr_t)15) + (lane & 15) * 16;
+        if (src + 16 <= w_end) cp_async16(dst, src);
+        else if (src < w_end) cp_async16_part(dst, src, (uint32_t)(w_end - src));
+      }
+    }
+    cp_async_commit();
+  };
+  uint32_t used = 0;  // stages consumed so far
+  for (long long t0 = i0 + (long long)blockIdx.z * LIMB_PASS; t0 < i1; t0 += (long long)gridDim.z * LIMB_PASS) {
+    const int cnt = (int)min((long long)LIMB_PASS, i1 - t0);
+    const bool two = cnt > 8;  // groups of eight tokens
+    for (int b = 0; b < LIMB_RING - 1; b++) issue(b, b);
+    auto fetch = [&](int b) {  // the tokens' records of block b, by the first warp
+      if (warp == 0 && b < nb) {
+        const uint32_t at = (used + b) & 1u, bar = bar0 + 8 * at;
+        if (lane == 0) umma::mbar_arrive_expect_tx(bar, (uint32_t)(cnt * LIMB_RECORD));
+        __syncwarp();
+        if (lane < cnt)
+          asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(stages + at * LIMB_STAGE + lane * LIMB_TOKEN),
+                       "l"(limbs + ((size_t)(t0 + lane) * nb + b) * LIMB_RECORD), "r"(LIMB_RECORD), "r"(bar)
+                       : "memory");
+      }
+    };
+    fetch(0), fetch(1);
+    float acc[LIMB_RT][2][4], rest[LIMB_RT][2][4];  // [16 rows][group][rows g, g + 8 x tokens 2 t, 2 t + 1]: sum, and what its roundings left out
+#pragma unroll
+    for (int i = 0; i < 8 * LIMB_RT; i++) acc[i >> 3][(i >> 2) & 1][i & 3] = rest[i >> 3][(i >> 2) & 1][i & 3] = 0.f;
+    int slot = 0;
+    for (int b = 0; b < nb; b++) {
+      issue(b + LIMB_RING - 1, slot == 0 ? LIMB_RING - 1 : slot - 1);
+      float two_to[2][2];  // what the tokens' limbs count in
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+#pragma unroll
+        for (int c = 0; c < 2; c++) two_to[j][c] = __ldg(ups + (size_t)(t0 + min(8 * j + 2 * t + c, cnt - 1)) * nb + b);
+      cp_async_wait<LIMB_RING - 1>();
+      const uint32_t at = (used + b) & 1u, xs = stages + at * LIMB_STAGE + g * LIMB_TOKEN;  // operand column g: token g of each group
+      if (!umma::mbar_wait(bar0 + 8 * at, ((used + b) >> 1) & 1u, &abort_flag)) g_limb_status = 1;
+      if (__syncthreads_or(abort_flag)) return;  // (all warps, together)
+      const uint32_t blk = ring + slot * LIMB_SLOT + g * LIMB_PITCH + ((skew0 + (uint32_t)b * 210u) & 15u);  // row g's block
+      const uint32_t al = blk & ~3u, sh = (blk & 2u) * 8u;
+      auto word = [&](int r, int at) {  // of row g + 8 r
+        const uint32_t a = al + r * (8 * LIMB_PITCH) + at;
+        return __funnelshift_r(lds32(a), lds32(a + 4), sh);
+      };
+      float top[LIMB_RT][2][4], low[LIMB_RT][2][4];  // scale x sub-block's sum: limb 2 (whole, and exact below 2^24), limbs 1 and 0
+#pragma unroll
+      for (int i = 0; i < 8 * LIMB_RT; i++) top[i >> 3][(i >> 2) & 1][i & 3] = low[i >> 3][(i >> 2) & 1][i & 3] = 0.f;
+#pragma unroll 1
+      for (int hu = 0; hu < 4; hu++) {  // half h of the block, elements 16 u .. of each of its four groups
+        const int h = hu >> 1, u = hu & 1;
+        uint32_t wa[2 * LIMB_RT], wc[2 * LIMB_RT], wh[2 * LIMB_RT], sc[2 * LIMB_RT];
+#pragma unroll
+        for (int r = 0; r < 2 * LIMB_RT; r++) {
+          wa[r] = word(r, 64 * h + 16 * u + 4 * t), wc[r] = word(r, 64 * h + 32 + 16 * u + 4 * t), wh[r] = word(r, 128 + 32 * h + 16 * u + 4 * t);
+          sc[r] = __byte_perm(word(r, 192 + 8 * h), word(r, 196 + 8 * h), u ? 0x7531 : 0x6420) ^ 0x80808080u;  // of the four groups, plus 128
+        }
+        const int first = (8 * h + u) * 4 + t;  // the record's place of sub-block 8 h + u; group q's is 8 q further
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          uint4 x01[2];
+          uint2 x2[2];
+#pragma unroll
+          for (int j = 0; j < 2; j++) {
+            if (j == 0 || two) {
+              x01[j] = lds128(xs + j * (8 * LIMB_TOKEN) + 16 * (first + 8 * q)), x2[j] = lds64(xs + j * (8 * LIMB_TOKEN) + 1024 + 8 * (first + 8 * q));
+            }
+          }
+#pragma unroll
+          for (int rt = 0; rt < LIMB_RT; rt++) {
+            uint32_t a[4];
+            float f[2];
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+              const int i = 2 * rt + r;
+              const uint32_t nib = (q & 1 ? wc[i] : wa[i]) >> (q & 2 ? 4 : 0), bits = q == 0 ? wh[i] << 4 : q == 1 ? wh[i] << 2 : q == 2 ? wh[i] : wh[i] >> 2;
+              const uint32_t code = and_or(nib, 0x0F0F0F0Fu, bits & 0x30303030u);  // code + 32
+              const __half2 off = __float2half2_rn(-1056.f);
+              auto f16 = [&](uint32_t bits) {
+                const __half2 v = __hadd2(*reinterpret_cast<const __half2 *>(&bits), off);
+                return *reinterpret_cast<const uint32_t *>(&v);
+              };
+              a[r] = f16(__byte_perm(code, 0x64646464u, 0x4140)), a[2 + r] = f16(__byte_perm(code, 0x64646464u, 0x4342));
+              f[r] = __uint_as_float(__byte_perm(sc[i], 0x4B000000u, 0x7440 + q)) - 8388736.f;
+            }
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+              if (j == 0 || two) {
+                float d0[4], d1[4], d2[4];
+                mma_from_zero(d0, a, x01[j].x, x01[j].y);
+                mma_from_zero(d1, a, x01[j].z, x01[j].w);
+                mma_from_zero(d2, a, x2[j].x, x2[j].y);
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                  top[rt][j][c] = fmaf(f[c >> 1], d2[c], top[rt][j][c]), low[rt][j][c] = fmaf(f[c >> 1], fmaf(2048.f, d1[c], d0[c]), low[rt][j][c]);
+              }
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 2 * LIMB_RT; r++) {
+        uint16_t dh;
+        asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(dh) : "r"(blk + r * (8 * LIMB_PITCH) + 208));
+        const float d = f16_bits_to_f32(dh);
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+          for (int c = 0; c < 2; c++) {
+            // acc + d 2^.. (2^22 top + low), the roundings of the product and of the sum kept (d 2^.. has eleven bits: exact)
+            const int i = 2 * (r & 1) + c;
+            float &y = acc[r >> 1][j][i];
+            const float s = d * two_to[j][c], s22 = s * 4194304.f, v = s22 * top[r >> 1][j][i], t = y + v, z = t - y;
+            rest[r >> 1][j][i] += ((y - (t - z)) + (v - z)) + fmaf(s, low[r >> 1][j][i], fmaf(s22, top[r >> 1][j][i], -v));
+            y = t;
+          }
+      }
+      slot = slot + 1 == LIMB_RING ? 0 : slot + 1;
+      __syncthreads();  // every warp is done with the stage, and with its own slot
+      fetch(b + 2);
+    }
+    used += nb;
+    cp_async_wait<0>();
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        const int mine = 8 * j + 2 * t + c;
+        long long p = -1;
+        if (mine < cnt) {
+          p = pairs ? pairs[t0 + mine] : t0 + mine;
+          if (p >= size_m) p = -1;
+        }
+        bool nan = false;
+        if (p >= 0) {
+          const float f = topkw ? topkw[p] : 1.f;
+#pragma unroll
+          for (int r = 0; r < 2 * LIMB_RT; r++) {
+            const float y = acc[r >> 1][j][2 * (r & 1) + c] + rest[r >> 1][j][2 * (r & 1) + c];
+            nan |= y != y;
+            out[p * N + r0 + g + 8 * r] = topkw ? y * f : y;
+          }
+        }
+        unsigned odd = __ballot_sync(0xffffffffu, nan);
+        while (odd) {  // not a number: this token's rows once more, one after the other
+          const int tt = (__ffs(odd) - 1) & 3;
+          odd &= ~(0x11111111u << tt);  // (the lanes of that token)
+          const long long i = t0 + 8 * j + 2 * tt + c, q = pairs ? pairs[i] : i;
+          const float4 *x = reinterpret_cast<const float4 *>(in + (size_t)(row_per_pair ? q : q / topk) * K) + lane;
+          __syncwarp();  // (after the stores above)
+          for (int r = 0; r < LIMB_ROWS; r++) {
+            float y = 0.f;
+            for (int b = 0; b < nb; b++) {
+              float wv[8];
+              q6k_eight(rows + r * row_bytes + (size_t)b * 210, lane, wv);
+              const float4 u = __ldg(x + b * 64), v = __ldg(x + b * 64 + 32);
+              y = fmaf(wv[0], u.x, y), y = fmaf(wv[1], u.y, y), y = fmaf(wv[2], u.z, y), y = fmaf(wv[3], u.w, y);
+              y = fmaf(wv[4], v.x, y), y = fmaf(wv[5], v.y, y), y = fmaf(wv[6], v.z, y), y = fmaf(wv[7], v.w, y);
+            }
+            y = warp_sum(y);
+            if (lane == 0) out[q * N + r0 + r] = topkw ? y * topkw[q] : y;
+          }
+        }
+      }
+  }
+}
+
+size_t q6k_limbs_ws_bytes(long long M, int K) { return (size_t)M * (K >> 8) * LIMB_RECORD + (((size_t)M * (K >> 8) * 4 + 1023) & ~(size_t)1023); }
+
+// 1: took the call; 0: no room in the workspace, or fewer rows than a warp's
+static int q6k_limbs(const float *in, const void *w, const int64_t *pairs, const int32_t *offsets, const float *topkw, float *out, long long M, long long size_m,
+                     int E, int N, int K, int topk, int row_per_pair, int device, cudaStream_t st) {
+  size_t bytes = 0;
+  uint8_t *ws = (uint8_t *)workspace_ptr(device, &bytes);
+  const long long records = M * (K >> 8);
+  if (!ws || bytes < q6k_limbs_ws_bytes(M, K) || N < LIMB_ROWS || ((uintptr_t)in & 15) || (records + 7) / 8 > 0x7fffffffll) return 0;
+  float *ups = (float *)(ws + (size_t)records * LIMB_RECORD);
+  launch_early(x_limbs_kernel, dim3((unsigned)((records + 7) / 8)), dim3(256), st, in, pairs, ws, ups, M, K, topk, row_per_pair, size_m);
+  if (int rc = launched("q6_k: activations to limbs")) return rc;
+  static DeviceOnce attr;
+  const cudaError_t err = attr.ensure([] { return cudaFuncSetAttribute(q6k_limbs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LIMB_SMEM); });
+  if (err != cudaSuccess) return fail((int)err, "light_b200: q6_k rows: %s", cudaGetErrorString(err));
+  const long long nb = (N + LIMB_ROWS * LIMB_WARPS - 1) / (LIMB_ROWS * LIMB_WARPS), passes = (M + LIMB_PASS - 1) / LIMB_PASS, want = (4ll * sm_count() + nb * E - 1) / (nb * E);
+  long long z = want < passes ? want : passes;  // CTAs that share an expert's tokens, where experts and rows alone do not fill the GPU
+  if (z > 65535) z = 65535;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nb, (unsigned)E, (unsigned)z), cfg.blockDim = dim3(LIMB_WARPS * 32), cfg.dynamicSmemBytes = LIMB_SMEM, cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at, cfg.numAttrs = 1;
+  const cudaError_t e2 = cudaLaunchKernelEx(&cfg, q6k_limbs_kernel, in, (const uint8_t *)w, (const uint8_t *)ws, (const float *)ups, pairs, offsets, topkw, out, M, size_m, E,
+                                            N, K, topk, row_per_pair);
+  if (e2 != cudaSuccess) return fail((int)e2, "light_b200: q6_k rows: %s", cudaGetErrorString(e2));
+  if (int rc = launched("q6_k rows (limbs)")) return rc;
+  return 1;
+}
+
 template <bool CHAIN>
 static int q6k_rows(const float *in, const void *w, const int64_t *pairs, const int32_t *offsets, const float *topkw, float *out, long long M, long long size_m,
                     int E, int N, int K, int topk, int row_per_pair, cudaStream_t st) {
@@ -374,7 +680,8 @@ static int q6k_rows(const float *in, const void *w, const int64_t *pairs, const 
   return launched("q6_k rows (f32)");
 }
 
-int q6k_rows_dense(const float *x, const void *w, float *out, int M, int N, int K, cudaStream_t st) {
+int q6k_rows_dense(const float *x, const void *w, float *out, int M, int N, int K, int device, cudaStream_t st) {
+  if (int took = q6k_limbs(x, w, nullptr, nullptr, nullptr, out, M, M, 1, N, K, 1, 1, device, st)) return took == 1 ? 0 : took;
   return q6k_rows<false>(x, w, nullptr, nullptr, nullptr, out, M, M, 1, N, K, 1, 1, st);
 }
 
@@ -413,6 +720,12 @@ int fp8_block_rows_dot(const void *x, const uint8_t *w, const float *s, void *y,
   const RowAux aux{s, bR, bC, nullptr};
   if (act_dtype == LB200_F32) return run_plain<float, F8BlockRow<float>>(x, w, y, M, N, K, aux, st);
   return run_plain<__nv_bfloat16, F8BlockRow<__nv_bfloat16>>(x, w, y, M, N, K, aux, st);
+}
+
+int q6k_limbs_status() {
+  int v = 0;
+  const cudaError_t e = cudaMemcpyFromSymbol(&v, g_limb_status, sizeof(int));
+  return e == cudaSuccess ? v : -(int)e;
 }
 
 int moe_bad_ids_status() {
@@ -492,9 +805,13 @@ int moe_gemm_q(const lb200_moe_args *a, int device, cudaStream_t st) {
   if (rc) return rc;
   if (int took = moe_umma(a, 1, nullptr, 0, 0, device, st)) return took == 1 ? 0 : took;
   // From as many pairs on as the tensor-core path takes of the other formats.
-  if (a->dtype == LB200_Q6_K && a->M >= 256 && a->K % 256 == 0 && a->E <= 65535 && a->N > 0)
+  if (a->dtype == LB200_Q6_K && a->M >= 256 && a->K % 256 == 0 && a->E <= 65535 && a->N > 0) {
+    if (int took = q6k_limbs((const float *)a->input, a->weights, a->sorted_pairs, a->offsets, a->topk_weights, (float *)a->out, a->M, a->size_m, a->E, a->N, a->K, a->topk,
+                             a->row_per_pair, device, st))
+      return took == 1 ? 0 : took;
     return q6k_rows<true>((const float *)a->input, a->weights, a->sorted_pairs, a->offsets, a->topk_weights, (float *)a->out, a->M, a->size_m, a->E, a->N, a->K,
                        a->topk, a->row_per_pair, st);
+  }
   switch (a->dtype) {
     case LB200_Q4_0: return run<float, float, QuantRow<LB200_Q4_0>>(a, st);
     case LB200_Q5_0: return run<float, float, QuantRow<LB200_Q5_0>>(a, st);

@@ -45,3 +45,36 @@ def test_int4_rows_beyond_f16(cuda, G, scale):
     x = (torch.randn(M, K, generator=g, device=cuda) * scale).bfloat16()
     want = x.double() @ ops.DequantizeInt4(w, torch.float32).double().t()
     assert rel_l2(ops.MatMulInt4(x, w).cpu().double().numpy(), want.cpu().numpy()) <= 2.5e-3
+
+
+# whole passes of 16 tokens and one more, rows that are no whole tile, one block per row, runs of more than the ring's blocks
+@pytest.mark.parametrize("M,N,K", [(65, 32, 256), (80, 33, 768), (81, 300, 1280), (500, 130, 2816)])
+@pytest.mark.parametrize("kind", ["normal", "outlier", "tiny", "huge"])
+def test_q6_k_in_limbs(cuda, M, N, K, kind):
+    """Per output: the fixed point rounds an activation at 2^-30 of the power of two above its block's largest, 2^-30 max|x| sum|w| in all;
+    per block and limb pair the whole sums and their scaling are rounded three times, blocks are added in f32: fewer than 16 + K / 256
+    roundings of terms that together stay below four times sum|w x|."""
+    w = ops.QTensor(synth.gaussian_weight(N + K, ops.Q6_K, N, K, device=cuda).reshape(-1), ops.Q6_K, (N, K))
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(cuda)
+    if kind == "outlier":
+        x[:, 5] = 1000.0
+    x = x * {"tiny": 2.0**-90, "huge": 2.0**90}.get(kind, 1.0)
+    W, X = ops.Dequantize(w).double(), x.double()
+    bound = 2.0**-30 * X.abs().amax(1, keepdim=True) * W.abs().sum(1) + (16 + K / 256) * 2.0**-22 * (X.abs() @ W.abs().t())
+    assert bool(((ops.MatMulQ(x, w).double() - X @ W.t()).abs() <= bound).all())
+
+
+def test_q6_k_in_limbs_infinities_and_nan(cuda):
+    """Tokens with infinities or NaN give what f32 products give; the others are not touched by them."""
+    M, N, K = 70, 40, 768
+    w = ops.QTensor(synth.gaussian_weight(1, ops.Q6_K, N, K, device=cuda).reshape(-1), ops.Q6_K, (N, K))
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(2)).to(cuda)
+    inf = float("inf")
+    x[3, 7], x[4, 700], x[5, 0], x[6, 9], x[6, 300], x[69, 1] = inf, -inf, float("nan"), inf, -inf, inf
+    W = ops.Dequantize(w).double().cpu()
+    want = (x.double().cpu()[:, None, :] * W[None]).sum(-1)
+    y = ops.MatMulQ(x, w).double().cpu()
+    assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isinf(), want.isinf())
+    assert torch.equal(y[y.isinf()].sign(), want[want.isinf()].sign())
+    fin = want.isfinite()
+    assert rel_l2(y[fin].numpy(), want[fin].numpy()) <= 1e-6
