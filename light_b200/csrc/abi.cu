@@ -148,8 +148,8 @@ int light_b200_matmul_q_tp(int t, const float *x, const void *const *w, float *c
 
 int light_b200_prefill_status(int device) {
   if (int rc = bind(device)) return rc;
-  const int a = prefill_status(device), b = decode_umma_status(), c = decode_nt_status(), d = decode_ts_status(), e = gemm_tmem_status(), f = q6k_limbs_status();
-  return a ? a : b ? b : c ? c : d ? d : e ? e : f;
+  const int a = prefill_status(device), b = decode_umma_status(), c = decode_nt_status(), d = decode_ts_status(), e = gemm_tmem_status(), f = q6k_limbs_status(), g = decode_tmem_status();
+  return a ? a : b ? b : c ? c : d ? d : e ? e : f ? f : g;
 }
 unsigned long long light_b200_matmul_q_workspace_bytes(int M, int K) {
   if (M < 1 || K <= 0) return 0;
@@ -201,6 +201,8 @@ int light_b200_matmul_q(int t, const float *x, const void *w, float *out, int M,
     const void *wv[1] = {w};
     float *ov[1] = {out};
     const int nv[1] = {N};
+    took = gguf_decode_tmem(t, x, w, out, M, N, K, ws, wsb, st);
+    if (took != 0) return took == 1 ? 0 : took;
     took = gguf_decode_nt(t, x, wv, ov, nv, 1, M, K, ws, wsb, st);
     if (took != 0) return took == 1 ? 0 : took;
   }

@@ -39,13 +39,12 @@
 
 #include "common.cuh"
 #include "mma_sync.cuh"
+#include "tmem_ops.cuh"
 #include "tmem_rows.cuh"
 #include "umma.cuh"
 
 namespace lb {
 namespace {
-
-using namespace umma;
 
 constexpr int EXPANDERS = 16, TMA_WARP = 16, MMA_WARP = 18, EPI_WARP = 19, THREADS = 23 * 32;
 constexpr int KU = 128;                       // k of a unit: one TMEM stage, one stage of the token ring
@@ -53,21 +52,12 @@ constexpr int NAS = 4;                        // stages of expanded weights: 128
 constexpr int NBS = 12;                       // most stages of the token ring, 128 k each
 constexpr int A_COL = 256;                    // columns 0-255: accumulators, 256-511: weight stages
 constexpr int MAX_E = 1024;                   // experts whose prefix sums fit the shared tables
-constexpr int MAX_GRID = 160;
 constexpr int BAR_BYTES = 640;                // barriers
 constexpr int MAX_ROWS = 128;                 // most token rows of a stage (one SM's)
 constexpr int PART_FLOATS = 256 * 128;        // one partial tile: [token][row]
-constexpr int SMEM_MAX = 227 * 1024 - 1024;   // dynamic; the static part (prefix tables, flags) is accounted below
 
 __device__ int g_status;                      // non-zero: a bounded wait gave up (sticky)
-// Which parts of the partial tiles are written: a flag per (CTA, row quarter, 16-token chunk) holds the tag of the launch that wrote the
-// part last.  A launch's tag is the epoch it finds, plus one; the last of its CTAs to have read the epoch raises it.  So no flag of an
-// earlier launch ever matches, one that gave up and left flags without a reader included, and nothing is cleared between launches.
-struct Sync {
-  unsigned epoch, readers;
-  unsigned flags[MAX_GRID * 64];
-};
-__device__ Sync g_sync;  // of the launches without one of their own
+__device__ Sync g_sync;  // of the launches without one of their own; a flag per (CTA, row quarter, 16-token chunk)
 
 struct Args {
   const int32_t *offsets;   // grouped: expert e owns rows offsets[e] .. offsets[e + 1] of the (gathered) tokens; null: one matrix
@@ -86,43 +76,6 @@ struct Tile {
   int expert, n0, m0, m_end, nt;
 };
 
-// ------------------------------------------------------------------------------------ PTX forms this file adds
-__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) { return map_to_rank(addr, rank); }
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
-  return p != 0;
-}
-// Looks for up to a hardware-set time (the thread sleeps meanwhile): a waiting warp takes no issue slots from the expanders.
-// (Spinning, the four epilogue warps and the MMA warp issued a third of all instructions.)
-__device__ __forceinline__ bool mbar_sleep_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// A whole warp waits, together: every lane looks and all branches are on votes, so the warp never diverges here (what
-// follows are .aligned instructions and values the compiler keeps in the warp's uniform registers).
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int *abort) {
-  if (__all_sync(0xffffffffu, mbar_sleep_wait(bar, parity))) return true;
-  const unsigned long long t0 = global_ns();
-  while (!__all_sync(0xffffffffu, mbar_sleep_wait(bar, parity))) {
-    if (__any_sync(0xffffffffu, *abort != 0)) return false;
-    if (__any_sync(0xffffffffu, global_ns() - t0 > 1000000000ull)) {
-      *abort = 1;
-      return false;
-    }
-  }
-  return true;
-}
 __device__ __forceinline__ void st_if(bool p, float *o, float v) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.f32 [%0], %1;\n\t}\n" ::"l"(o), "f"(v), "r"((int)p) : "memory");
 }
@@ -131,72 +84,6 @@ __device__ __forceinline__ void st_if(bool p, __nv_bfloat16 *o, float v) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.b16 [%0], %1;\n\t}\n" ::"l"(o), "h"(*reinterpret_cast<const uint16_t *>(&b)), "r"((int)p)
                : "memory");
 }
-template <int CG>
-__device__ __forceinline__ void alloc512(uint32_t smem_dst) {
-  if constexpr (CG == 1) {
-    tmem_alloc(smem_dst, 512);
-    tmem_relinquish();
-  } else {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_dst) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
-  }
-}
-template <int CG>
-__device__ __forceinline__ void dealloc512(uint32_t taddr) {
-  if constexpr (CG == 1) tmem_dealloc(taddr, 512);
-  else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;\n" ::"r"(taddr) : "memory");
-}
-// D[tmem] (+)= A[tmem] x B[smem]; with CG = 2 each CTA of the pair holds half of the rows of A and D and half of the
-// columns (tokens) of B at the same addresses, and the first CTA issues for both
-template <int CG>
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  if constexpr (CG == 1)
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-  else
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-template <int CG>
-__device__ __forceinline__ void commit(uint32_t bar) {  // CG = 2: on this barrier of both CTAs
-  if constexpr (CG == 1) mma_commit(bar);
-  else
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(bar), "h"((uint16_t)3)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
-      "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
-
-__device__ __forceinline__ bool wait_flag(const unsigned *flag, unsigned tag, bool mine, volatile int *abort) {  // whole warp, a flag to each lane that has one
-  const unsigned long long t0 = global_ns();
-  for (uint32_t i = 1;; i++) {
-    unsigned v = tag;
-    if (mine) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(flag) : "memory");
-    if (__all_sync(0xffffffffu, v == tag)) return true;
-    if ((i & 15u) == 0) {
-      if (__any_sync(0xffffffffu, *abort != 0)) return false;
-      if (__any_sync(0xffffffffu, global_ns() - t0 > 1000000000ull)) break;
-    }
-  }
-  *abort = 1;
-  return false;
-}
-
 // ------------------------------------------------------------------------------------ work list
 // Experts with their token tiles: preT[e] tiles and preW[e] weighted units before expert e.  Within an expert the token
 // tiles of one row tile follow one another, so that its packed weights are read from HBM once and from L2 after that.
@@ -784,22 +671,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
 }
 
 // ------------------------------------------------------------------------------------ host
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-  static const EncodeTiledFn fn = [] {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    const cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q);
-    return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? (EncodeTiledFn)p : (EncodeTiledFn) nullptr;
-  }();
-  return fn;
-}
-int knob(const char *name, int otherwise) {
-  const char *e = getenv(name);
-  return e ? atoi(e) : otherwise;
-}
-
 template <typename Row, typename OutT>
 constexpr int fixed_smem(int E) { return EXPANDERS * Row::SLOT + STRIPS<OutT> + BAR_BYTES + (E + 1) * 12 + 16 + 1024; }
 
