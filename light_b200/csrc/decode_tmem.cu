@@ -9,8 +9,9 @@
 //
 //   warps 0-15   expanders, as gemm_tmem.cu's: the four warps w, w + 4, .. own rows 32 (w & 3) .. + 31, set w / 4 has every fourth unit of 128 k
 //                (sets 0 and 2 the first halves of blocks, 1 and 3 the second).
-//   warps 16-17  one lane of each: TMA of the tokens, 64 of a unit's 128 k each; the second one also their sub-blocks' sums.
-//   warp  18     MMAs and commits.
+//   warps 16-17  one lane of each: TMA of the tokens, half a block each; the second one also their sub-blocks' sums.
+//   warp  18     MMAs and commits, a block at a time: 18 MMAs take some 900 clocks, and a pass 400 more of waits and commits that the tensor
+//                pipe does not cover (half a block at a time: 28672 x 4096, 32 rows 33.2 us where this takes 30.9).
 //   warps 19-26  drain: row quarter w & 3 and every second chunk of 16 tokens; per block sums += d x D; at a tile's end the minimums'
 //                sums are added and the tile leaves, or is left for, or put together from, the runs it is cut into.
 //
@@ -27,9 +28,10 @@ namespace lb {
 namespace {
 
 constexpr int EXPANDERS = 16, TMA_WARP = 16, MMA_WARP = 18, DRAIN_WARP = 19, DRAINS = 8, THREADS = 27 * 32;
-constexpr int NAS = 4, NBS = 8;               // stages of weights; most stages of tokens
+constexpr int NBS = 4;                        // most blocks of tokens on their way (of weights: two)
 constexpr int MAX_NT = 64;
-// tensor memory: two buffers of a block's sums, the minimums' sums, the minimums (8 columns per stage), the weights
+// tensor memory: buffers of a block's sums (two, or four where 32 columns are enough), the minimums' sums, the minimums (8 columns per
+// half block), the weights
 constexpr int P_COL = 2 * MAX_NT, M_COL = 3 * MAX_NT, A_COL = 256;
 constexpr int BAR_BYTES = 512;
 constexpr int PART_FLOATS = MAX_NT * 128;     // one partial tile: [token][row]
@@ -40,6 +42,7 @@ __device__ Sync g_sync;                       // a flag per (CTA, drain warp)
 struct Args {
   int M, N, K, nt;            // nt: tokens of a tile, a multiple of 16
   int stage_bytes, stages;    // of the tokens
+  int bufs;                   // buffers of a block's sums: a power of two
   float *parts;
 };
 struct Maps {
@@ -155,12 +158,12 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
   __shared__ int abort_flag;
   __shared__ uint32_t tmem_sh;
   __shared__ unsigned tag_sh;
-  __shared__ float scales[4][128];  // d of a block's rows, by the block's number in the run
+  __shared__ float scales[8][128];  // d of a block's rows, by the block's number in the run
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sB = base, sRaw = base + (uint32_t)a.stages * a.stage_bytes, sBar = sRaw + (uint32_t)EXPANDERS * Row::SLOT;
-  // full[s], empty[s]: a unit's weights are there, its MMAs have completed; t_full, t_empty: its tokens; d_full, d_empty: a block's sums are
+  // full, empty: a block's weights are there, its MMAs have completed; t_full, t_empty: its tokens; d_full, d_empty: its sums are
   // complete, are read out; p_empty: the minimums' sums are.
-  const uint32_t full = sBar, empty = full + 8 * NAS, d_full = empty + 8 * NAS, d_empty = d_full + 16, p_empty = d_empty + 16, w_full = p_empty + 8,
+  const uint32_t full = sBar, empty = full + 16, d_full = empty + 16, d_empty = d_full + 32, p_empty = d_empty + 32, w_full = p_empty + 8,
                  t_full = w_full + 8 * EXPANDERS, t_empty = t_full + 8 * NBS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nb = a.K >> 8, G = gridDim.x, cta = blockIdx.x, U = (a.N + 127) / 128 * nb;
@@ -172,9 +175,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
     if constexpr (Row::MINS) prefetch_tmap(&maps.sums);
     if constexpr (Row::BOXES > 0) prefetch_tmap(&maps.w[0]), prefetch_tmap(&maps.w[1]);
     abort_flag = 0;
-    for (int i = 0; i < NAS; i++) mbar_init(full + 8 * i, 4), mbar_init(empty + 8 * i, 1);
+    for (int i = 0; i < 2; i++) mbar_init(full + 8 * i, 8), mbar_init(empty + 8 * i, 1);
     for (int i = 0; i < a.stages; i++) mbar_init(t_full + 8 * i, 2), mbar_init(t_empty + 8 * i, 1);
-    for (int i = 0; i < 2; i++) mbar_init(d_full + 8 * i, 1), mbar_init(d_empty + 8 * i, DRAINS);
+    for (int i = 0; i < a.bufs; i++) mbar_init(d_full + 8 * i, 1), mbar_init(d_empty + 8 * i, DRAINS);
     mbar_init(p_empty, DRAINS);
     for (int i = 0; i < EXPANDERS; i++) mbar_init(w_full + 8 * i, 1);
     fence_barrier_init();
@@ -185,62 +188,64 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_sh;
+  const uint32_t tmem = tmem_sh, bmask = (uint32_t)a.bufs - 1, cols = 2 * MAX_NT / a.bufs;
+  const int blog = a.bufs == 4 ? 2 : 1;
   volatile int *abort = &abort_flag;
 
   if (warp >= TMA_WARP && warp < MMA_WARP) {
     if (elect_one()) {
       pdl_wait();  // the tokens are the kernel before's
       const int half = warp - TMA_WARP;
-      const uint32_t bytes = (uint32_t)a.nt * (Row::MINS && half ? 160u : 128u);
-      int s = 0, par = 1, u = v0 % nb * 2;
+      const uint32_t bytes = (uint32_t)a.nt * (Row::MINS && half ? 320u : 256u), tile = (uint32_t)a.nt * 128u;
+      int s = 0, par = 1, kb = v0 % nb;
       bool wrapped = false;
-      for (int i = 0; i < 2 * n; i++) {
+      for (int i = 0; i < n; i++) {
         const uint32_t bar = t_full + 8 * s, dst = sB + s * a.stage_bytes;
         if (wrapped && !mbar_sleep_wait(t_empty + 8 * s, par) && !mbar_wait(t_empty + 8 * s, par, abort)) break;
         mbar_arrive_expect_tx(bar, bytes);
-        tma_load_2d(dst + half * a.nt * 128, &maps.x, bar, u * 128 + half * 64, 0);
-        if (Row::MINS && half) tma_load_2d(dst + a.nt * 256, &maps.sums, bar, u * 16, 0);
-        if (++u == 2 * nb) u = 0;
+        tma_load_2d(dst + 2 * half * tile, &maps.x, bar, kb * 256 + half * 128, 0);
+        tma_load_2d(dst + (2 * half + 1) * tile, &maps.x, bar, kb * 256 + half * 128 + 64, 0);
+        if (Row::MINS && half) {
+          tma_load_2d(dst + 4 * tile, &maps.sums, bar, kb * 32, 0);
+          tma_load_2d(dst + 4 * tile + tile / 4, &maps.sums, bar, kb * 32 + 16, 0);
+        }
+        if (++kb == nb) kb = 0;
         if (++s == a.stages) s = 0, par ^= 1, wrapped = true;
       }
     }
   } else if (warp == MMA_WARP) {
     const uint32_t idesc = idesc_f16(128, 16, false) + ((uint32_t)((a.nt - 16) >> 3) << 17);
-    int s = 0, par = 0, t = 0, tpar = 0, kb = v0 % nb, seg = 0;
-    bool ok = true, first = true;  // first: of the tile's blocks in this run
-    bool ready = false, room = false;  // the next unit's barriers and its block's buffer, looked at before this one's MMAs are issued
-    for (int i = 0; i < n && ok; i++) {
-      const uint32_t d = tmem + MAX_NT * (i & 1);
-      if (i >= 2 && !__all_sync(0xffffffffu, room) && !warp_wait(d_empty + 8 * (i & 1), ((i >> 1) - 1) & 1, abort)) break;
+    const uint32_t tile = (uint32_t)a.nt * 128u;
+    int t = 0, tpar = 0, kb = v0 % nb, seg = 0;
+    bool first = true;                  // of the tile's blocks in this run
+    bool ready = false, room = false;   // the next block's barriers and buffer, looked at before this one's MMAs are issued
+    for (int i = 0; i < n; i++) {
+      if (i >= a.bufs && !__all_sync(0xffffffffu, room) && !warp_wait(d_empty + 8 * (i & bmask), ((i >> blog) - 1) & 1, abort)) break;
       if (Row::MINS && first && seg > 0 && !warp_wait(p_empty, (seg - 1) & 1, abort)) break;
-#pragma unroll 1
-      for (int half = 0; half < 2; half++) {
-        if (!__all_sync(0xffffffffu, ready) && !(warp_wait(t_full + 8 * t, tpar, abort) && warp_wait(full + 8 * s, par, abort))) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t st = sB + t * a.stage_bytes, am = tmem + A_COL + 64 * s, mins = tmem + M_COL + 8 * s, done = empty + 8 * s, tdone = t_empty + 8 * t;
-        if (++s == NAS) s = 0, par ^= 1;
-        if (++t == a.stages) t = 0, tpar ^= 1;
-        const bool weights = mbar_test_wait(full + 8 * s, par), tokens = mbar_test_wait(t_full + 8 * t, tpar);
-        room = i > 0 && mbar_test_wait(d_empty + 8 * ((i + 1) & 1), (((i + 1) >> 1) - 1) & 1);
-        ready = weights && tokens;
-        if (elect_one()) {
-          const uint64_t b0 = smem_desc_sw128(st), b1 = smem_desc_sw128(st + a.nt * 128);
-          mma_ts<1>(d, am, b0, idesc, half);
+      if (!__all_sync(0xffffffffu, ready) && !(warp_wait(t_full + 8 * t, tpar, abort) && warp_wait(full + 8 * (i & 1), (i >> 1) & 1, abort))) break;
+      tc_fence_after();
+      const uint32_t d = tmem + cols * (i & bmask), st = sB + t * a.stage_bytes, tdone = t_empty + 8 * t;
+      if (++t == a.stages) t = 0, tpar ^= 1;
+      const bool weights = mbar_test_wait(full + 8 * ((i + 1) & 1), ((i + 1) >> 1) & 1), tokens = mbar_test_wait(t_full + 8 * t, tpar);
+      room = i + 1 >= a.bufs && mbar_test_wait(d_empty + 8 * ((i + 1) & bmask), (((i + 1) >> blog) - 1) & 1);
+      ready = weights && tokens;
+      if (elect_one()) {
+        const uint32_t am = tmem + A_COL + 128 * (i & 1), mins = tmem + M_COL + 16 * (i & 1);
 #pragma unroll
-          for (int j = 1; j < 4; j++) mma_ts<1>(d, am + 8 * j, b0 + 2 * j, idesc, 1u);
+        for (int q = 0; q < 4; q++) {
+          const uint64_t b = smem_desc_sw128(st + q * tile);
 #pragma unroll
-          for (int j = 0; j < 4; j++) mma_ts<1>(d, am + 32 + 8 * j, b1 + 2 * j, idesc, 1u);
-          if constexpr (Row::MINS) mma_ts<1>(tmem + P_COL, mins, smem_desc_sw32(st + a.nt * 256), idesc, first && half == 0 ? 0u : 1u);
-          mma_commit(done);
-          mma_commit(tdone);
-          if (half) mma_commit(d_full + 8 * (i & 1));
+          for (int j = 0; j < 4; j++) mma_ts<1>(d, am + 32 * q + 8 * j, b + 2 * j, idesc, q || j ? 1u : 0u);
         }
-        __syncwarp();
+        if constexpr (Row::MINS) {
+          mma_ts<1>(tmem + P_COL, mins, smem_desc_sw32(st + 4 * tile), idesc, first ? 0u : 1u);
+          mma_ts<1>(tmem + P_COL, mins + 8, smem_desc_sw32(st + 4 * tile + tile / 4), idesc, 1u);
+        }
+        mma_commit(empty + 8 * (i & 1));
+        mma_commit(d_full + 8 * (i & bmask));
+        mma_commit(tdone);
       }
+      __syncwarp();
       first = false;
       if (++kb == nb) kb = 0, first = true, seg++;
     }
@@ -312,10 +317,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
         }
         issue();
       }
-      if (round > 0 && !warp_wait(empty + 8 * set, (round - 1) & 1, abort)) break;  // the stage's MMAs of the round before
+      if (round > 0 && !warp_wait(empty + 8 * (set >> 1), (round - 1) & 1, abort)) break;  // the MMAs of the block two before
       tc_fence_after();
-      // (the drain is done with the block four before: the MMAs of the one two before, complete now, have waited for it)
-      if (half == 0) scales[now & 3][quad * 32 + lane] = rowx.scale();
+      // (the drain is done with the block eight before: the MMAs of the one two before, complete now, have waited for a later one)
+      if (half == 0) scales[now & 7][quad * 32 + lane] = rowx.scale();
       if constexpr (Row::MINS) {
         uint32_t m[8];
         rowx.mins(u, m);
@@ -329,7 +334,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(full + 8 * set);
+      if (lane == 0) mbar_arrive(full + 8 * (set >> 1));
     }
     if constexpr (Row::BOXES == 0) cp_async_wait<0>();
   } else {
@@ -354,18 +359,18 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
 #pragma unroll
         for (int k = 0; k < 16; k++) acc[c][k] = 0.f;
       for (int kb = k0; kb < k1; kb++, i++) {
-        if (!warp_wait(d_full + 8 * (i & 1), (i >> 1) & 1, abort)) {
+        if (!warp_wait(d_full + 8 * (i & bmask), (i >> blog) & 1, abort)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const float s = scales[i & 3][row];
+        const float s = scales[i & 7][row];
 #pragma unroll
         for (int c = 0; c < 2; c++) {
           const int c0 = 16 * (2 * c + grp);
           if (c0 < a.nt) {
             uint32_t w[16];
-            tmem_ld16(tmem + lanes + MAX_NT * (i & 1) + c0, w);
+            tmem_ld16(tmem + lanes + cols * (i & bmask) + c0, w);
             tmem_ld_wait();
 #pragma unroll
             for (int k = 0; k < 16; k++) acc[c][k] = fmaf(__uint_as_float(w[k]), s, acc[c][k]);
@@ -373,7 +378,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(d_empty + 8 * (i & 1));
+        if (lane == 0) mbar_arrive(d_empty + 8 * (i & bmask));
       }
       if (!ok) break;
       if constexpr (Row::MINS) {  // (complete: committed before the last block's sums)
@@ -476,12 +481,13 @@ int run(const typename Row::Ctx &ctx, const float *x, float *out, int M, int N, 
   const EncodeTiledFn enc = encode_fn();
   if (!enc) return fail(LB200_E_DEVICE, "light_b200: cuTensorMapEncodeTiled is not available from the driver");
   Args a = {};
-  a.M = M, a.N = N, a.K = K, a.nt = (M + 15) / 16 * 16;
-  a.stage_bytes = (a.nt * (Row::MINS ? 288 : 256) + 1023) & ~1023;
-  const int fixed = EXPANDERS * Row::SLOT + BAR_BYTES + 1024 + 3072;  // (the last: static shared memory)
+  a.M = M, a.N = N, a.K = K, a.nt = (M + 15) / 16 * 16, a.bufs = a.nt <= 32 ? 4 : 2;
+  a.stage_bytes = (a.nt * (Row::MINS ? 576 : 512) + 1023) & ~1023;
+  const int fixed = EXPANDERS * Row::SLOT + BAR_BYTES + 1024 + 5120;  // (the last: static shared memory)
   a.stages = (SMEM_MAX - fixed) / a.stage_bytes;
   if (a.stages > NBS) a.stages = NBS;
-  const int smem = fixed - 3072 + a.stages * a.stage_bytes;
+  if (a.stages < 2) return 0;
+  const int smem = fixed - 5120 + a.stages * a.stage_bytes;
   char *const w8 = (char *)ws;
   a.parts = (float *)(w8 + x_bytes + sum_bytes);
   Maps tm = {};
@@ -503,7 +509,7 @@ int run(const typename Row::Ctx &ctx, const float *x, float *out, int M, int N, 
   if (int rc = launched("decode: activations to f16")) return rc;
   auto kern = decode_tmem_kernel<Row>;
   static DeviceOnce attr;
-  cudaError_t e = attr.ensure([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 3072); });
+  cudaError_t e = attr.ensure([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 5120); });
   if (e != cudaSuccess) return fail((int)e, "light_b200: decode (tmem): %s", cudaGetErrorString(e));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)G), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = smem, cfg.stream = st;
@@ -519,11 +525,11 @@ int run(const typename Row::Ctx &ctx, const float *x, float *out, int M, int N, 
 
 }  // namespace
 
-// Where this beats the token tiles (us per call of a chain with a cold L2, tiles / here): Q4_K 28672 x 4096, 32 rows 42.6 / 33.8, 64 rows
-// 67.1 / 38.6; 6144 x 4096 18.6 / 15.0, 23.7 / 17.8; 8192 x 2048 17.3 / 13.1, 16.7 / 15.1; 4096 x 14336 29.4 / 23.5, 40.8 / 29.0.  At 4096 x
+// Where this beats the token tiles (us per call of a chain with a cold L2, tiles / here): Q4_K 28672 x 4096, 32 rows 42.6 / 30.9, 64 rows
+// 67.1 / 36.3; 6144 x 4096 18.6 / 14.7, 23.7 / 17.8; 8192 x 2048 17.3 / 12.9, 16.7 / 15.2; 4096 x 14336 29.4 / 21.8, 40.8 / 27.8.  At 4096 x
 // 4096 they are even (13.6 / 13.9, 17.6 / 17.4) and below the tiles are ahead (4096 x 2048 9.3 / 9.8, 1024 x 4096 9.3 / 10.7): a
-// tile is cut into too many parts.  Q6_K: 4096 x 14336 32.8 / 29.3, 44.5 / 34.0; 2048 x 5632 19.7 / 15.9, but 64 rows 20.7 / 21.8; 2048 x 2048
-// 11.4 / 9.3; 128256 x 4096 186 / 151, 307 / 165.  Up to 16 rows the tiles multiply half as much (28672 x 4096 32.8 / 33).
+// tile is cut into too many parts.  Q6_K: 4096 x 14336 32.8 / 29.7, 44.5 / 33.7; 2048 x 5632 19.7 / 15.9, but 64 rows 20.7 / 21.8; 2048 x 2048
+// 11.4 / 9.0; 128256 x 4096 186 / 156, 307 / 170.  Up to 16 rows the tiles multiply half as much (28672 x 4096 32.8 / 33).
 int gguf_decode_tmem(int type, const float *x, const void *w, float *out, int M, int N, int K, void *ws, size_t ws_bytes, cudaStream_t st) {
   static const int min_m = knob("LIGHT_B200_DECODE_TMEM_MIN_M", 17);
   const long long size = (long long)N * K;
