@@ -154,7 +154,7 @@ int light_b200_prefill_status(int device) {
 unsigned long long light_b200_matmul_q_workspace_bytes(int M, int K) {
   if (M < 1 || K <= 0) return 0;
   unsigned long long f16_copy = M > 1 ? (unsigned long long)M * K * 2 : 0;  // the tensor-core paths' f16 copy of x
-  if (M > 64) f16_copy += prefill_sk_ws_bytes();  // and, behind it, the partial tiles of the persistent prefill kernel
+  if (M > 64) f16_copy += prefill_sk_ws_bytes() + (((unsigned long long)M * 4 + 2047) & ~1023ull);  // and, behind it, partial tiles and a factor per row
   else if (M >= 4) f16_copy = ((f16_copy + 1023) & ~1023ull) + gemm_tmem_parts_bytes();  // those of the tensor-memory kernel (Q8_0, 4-bit)
   unsigned long long staged = M <= 64 ? decode_nt_ws_bytes(M, K) : 0;
   if (M <= 64 && decode_ts_ws_bytes(M, K) > staged) staged = decode_ts_ws_bytes(M, K);

@@ -160,6 +160,7 @@ struct TmemCall {
   const int32_t *offsets;   // grouped: see gemm_tmem.cu (null: one matrix)
   const int64_t *pairs;
   const float *topkw;
+  const float *factor;      // FP8, grouped: x16 holds f16 rows over a power of two each, which this multiplies by again (bf16 output)
   long long size_m;
   int E;
   double mean_tokens;       // tokens per matrix (grouped: pairs / experts)

@@ -63,6 +63,7 @@ struct Args {
   const int32_t *offsets;   // grouped: expert e owns rows offsets[e] .. offsets[e + 1] of the (gathered) tokens; null: one matrix
   const int64_t *pairs;     // grouped: token row i goes to output row pairs[i] ...
   const float *topkw;       // ... scaled by its routing weight (or null)
+  const float *factor;      // f16 tokens over a power of two each: token row i is to be multiplied by factor[i] (null: as they are)
   long long size_m;
   int E, M, N, K;
   int nt_max;               // most tokens of a tile
@@ -365,11 +366,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       prow = -1, pw = 1.f;
       if (T.m0 + c0 + lane < T.m_end) {
         prow = T.m0 + c0 + lane;
+        const float f = a.factor ? a.factor[prow] : 1.f;
         if (a.offsets) {
           const long long p = a.pairs[prow];
           prow = p >= 0 && p < a.size_m ? (int)p : -1;
           if (prow >= 0 && a.topkw) pw = a.topkw[p];
         }
+        pw *= f;
       }
     };
     // The run's last segment, 16 tokens at a time: chunks first, first + step, ...  `shared`: five warps of this row quarter take
@@ -388,6 +391,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
         while (jlast + 1 < G && wk.bound(jlast + 1, G) < (t + 1) * nb) jlast++;
       const int col = T.n0 + 128 * rank + row;
       const bool live = col < a.N;
+      [[maybe_unused]] float scale = 1.f;
+      if constexpr (Unscales<Row>::value) scale = Row::unscale(ctx, T.expert * a.N + min(T.n0 + 128 * rank + quad * 32, a.N - 1));
       if (!warp_wait(d_full + 8 * (seg & 1), (seg >> 1) & 1, abort) || !warp_wait(tagged, 0, abort)) return;
       tc_fence_after();
       const unsigned tag = tag_sh;
@@ -448,7 +453,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
 #pragma unroll
           for (int i = 0; i < 16; i++) {
             const int m = __shfl_sync(0xffffffffu, prow, i);
-            const float f = __shfl_sync(0xffffffffu, pw, i) * __uint_as_float(v[i]);
+            const float y = Unscales<Row>::value ? __uint_as_float(v[i]) * scale : __uint_as_float(v[i]), f = __shfl_sync(0xffffffffu, pw, i) * y;
             st_if(live && m >= 0, o + (long long)m * a.N, f);
           }
         }
@@ -583,6 +588,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
           finish_last(0, shared ? 80 : 16);
           break;
         }
+        [[maybe_unused]] float scale = 1.f;
+        if constexpr (Unscales<Row>::value) scale = Row::unscale(ctx, T.expert * a.N + min(T.n0 + 128 * rank + quad * 32, a.N - 1));
         if (!warp_wait(d_full + 8 * (seg & 1), (seg >> 1) & 1, abort)) break;
         tc_fence_after();
         const uint32_t d = tmem + lanes + (T.nt > 128 ? 0 : 128 * (seg & 1));
@@ -608,7 +615,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
           int prow;
           float pw;
           route(T, c0, prow, pw);
-          if (a.topkw) {
+          if constexpr (Unscales<Row>::value) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * scale);
+          }
+          if (a.topkw || a.factor) {
 #pragma unroll
             for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * __shfl_sync(0xffffffffu, pw, i));
           }
@@ -747,7 +758,7 @@ template <typename Row, bool BF16, typename OutT>
 int pick(const typename Row::Ctx &ctx, const TmemCall &c, cudaStream_t st) {
   if (c.K % KU || c.E > MAX_E || (c.offsets && (c.M / 16 + c.E) * ((c.N + 127) / 128) * (c.K / KU) >= 1ll << 31)) return 0;
   Args a = {};
-  a.offsets = c.offsets, a.pairs = c.pairs, a.topkw = c.topkw, a.size_m = c.size_m;
+  a.offsets = c.offsets, a.pairs = c.pairs, a.topkw = c.topkw, a.factor = c.factor, a.size_m = c.size_m;
   a.E = c.offsets ? c.E : 1, a.M = (int)c.M, a.N = c.N, a.K = c.K;
   static const int k_cg = knob("LIGHT_B200_TMEM_CG", 0), k_nt = knob("LIGHT_B200_TMEM_NT", 0), k_wmin = knob("LIGHT_B200_TMEM_WMIN", 128), k_pair = knob("LIGHT_B200_TMEM_PAIR", 0);
   a.wmin = k_wmin;
@@ -788,6 +799,10 @@ int gemm_tmem(const TmemCall &c, cudaStream_t st) {
       return c.bf16 ? pick<TmInt4, true, __nv_bfloat16>(x, c, st) : pick<TmInt4, false, float>(x, c, st);
     }
     case TmemCall::FP8: {
+      if (c.factor) {
+        if (c.bR % 128 || c.bC % KU || c.N % c.bR) return 0;
+        return pick<TmFp8H, false, __nv_bfloat16>({(const uint8_t *)c.w, c.s, c.bR, Div::of(c.bC / KU), c.K / c.bC}, c, st);
+      }
       const TmFp8::Ctx x{(const uint8_t *)c.w, c.s, c.bR, c.bC, Div::of(c.bC / 64)};
       return c.bf16 ? pick<TmFp8, true, __nv_bfloat16>(x, c, st) : pick<TmFp8, false, float>(x, c, st);
     }

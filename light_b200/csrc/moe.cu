@@ -736,7 +736,7 @@ int moe_bad_ids_status() {
 }
 
 size_t moe_scratch_bytes(long long M, int K) {
-  return gemm_tmem_sync_bytes() + (((size_t)M * K * 2 + 1023) & ~(size_t)1023) + gemm_tmem_parts_bytes();
+  return gemm_tmem_sync_bytes() + (((size_t)M * K * 2 + 1023) & ~(size_t)1023) + (((size_t)M * 4 + 1023) & ~(size_t)1023) + gemm_tmem_parts_bytes();
 }
 
 int moe_gemm(const lb200_moe_args *a, int device, cudaStream_t st, void *scratch, size_t scratch_bytes) {

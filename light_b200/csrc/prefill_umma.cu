@@ -1122,6 +1122,73 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const TI *__restrict__
   }
 }
 
+// Rows of bf16 tokens in expert order as f16, over a power of two each that puts the row's largest element at [2^14, 2^15): exact for elements
+// down to 2^-31 of it, and factor[i] = the power.  (A row with infinities or NaN keeps them, and its other elements only their sign:
+// they do not matter beside those.)  A CTA to a row, held in registers (up to 8192 elements; the rest is read twice).
+constexpr int SCALED_THREADS = 128, SCALED_KEPT = 8;
+__global__ void __launch_bounds__(SCALED_THREADS) gather_rows_scaled_kernel(const uint4 *__restrict__ in, const int64_t *__restrict__ pairs, uint4 *__restrict__ dst,
+                                                                           float *__restrict__ factor, int K, int topk, int row_per_pair, long long size_m) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ uint32_t tops[SCALED_THREADS / 32];
+  const long long i = blockIdx.x, p = pairs[i];
+  const bool ok = p >= 0 && p < size_m;
+  const int n = K >> 3;  // pieces of eight elements
+  const uint4 *src = in + (ok ? (size_t)(row_per_pair ? p : p / topk) * n : 0);
+  auto larger = [](uint32_t top, const uint4 &q) {  // magnitudes, as bits, of the even and odd elements
+    return __vmaxu2(__vmaxu2(top, __vmaxu2(q.x & 0x7FFF7FFFu, q.y & 0x7FFF7FFFu)), __vmaxu2(q.z & 0x7FFF7FFFu, q.w & 0x7FFF7FFFu));
+  };
+  uint4 kept[SCALED_KEPT];
+  uint32_t top = 0;
+#pragma unroll
+  for (int j = 0; j < SCALED_KEPT; j++) {
+    const int k = threadIdx.x + j * SCALED_THREADS;
+    kept[j] = ok && k < n ? __ldg(src + k) : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int j = 0; j < SCALED_KEPT; j++) top = larger(top, kept[j]);
+  if (ok)
+    for (int k = threadIdx.x + SCALED_KEPT * SCALED_THREADS; k < n; k += SCALED_THREADS) top = larger(top, __ldg(src + k));
+  uint32_t mx = __reduce_max_sync(0xffffffffu, max(top & 0xFFFFu, top >> 16));
+  if ((threadIdx.x & 31) == 0) tops[threadIdx.x >> 5] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < SCALED_THREADS / 32; j++) mx = max(mx, tops[j]);
+  const bool finite = mx < 0x7F80u;
+  const int e = max((int)(mx >> 7), 1), sb = finite ? min(253, 268 - e) : 127;  // biased exponent of the multiplier
+  const float f = __uint_as_float((uint32_t)sb << 23);
+  if (threadIdx.x == 0) factor[i] = __uint_as_float((uint32_t)(254 - sb) << 23);
+  uint4 *to = dst + (size_t)i * n;
+  auto two = [&](uint32_t w) {
+    const float x = __uint_as_float(w << 16), y = __uint_as_float(w & 0xFFFF0000u);
+    if (finite) return pack_h2(x * f, y * f);
+    auto keep = [](float v) { return isfinite(v) ? copysignf(0.f, v) : v; };
+    return pack_h2(keep(x), keep(y));
+  };
+  auto put = [&](int k, const uint4 &q) { to[k] = make_uint4(two(q.x), two(q.y), two(q.z), two(q.w)); };
+#pragma unroll
+  for (int j = 0; j < SCALED_KEPT; j++) {
+    const int k = threadIdx.x + j * SCALED_THREADS;
+    if (k < n) put(k, kept[j]);
+  }
+  for (int k = threadIdx.x + SCALED_KEPT * SCALED_THREADS; k < n; k += SCALED_THREADS) put(k, ok ? __ldg(src + k) : make_uint4(0, 0, 0, 0));
+}
+
+// bf16 tokens times FP8 weights in whole 128 x 128 blocks, grouped, with f16 operands.  1: took the call, 0: not covered, other: error.
+int moe_fp8_f16(const lb200_moe_args *a, const float *w_scale, int bR, int bC, void *ws, size_t ws_bytes, void *sync, cudaStream_t st) {
+  const size_t x_bytes = ((size_t)a->M * a->K * 2 + 1023) & ~(size_t)1023, f_bytes = ((size_t)a->M * 4 + 1023) & ~(size_t)1023;
+  if (!use_tmem() || bR % 128 || bC % 128 || ws_bytes < x_bytes + f_bytes + gemm_tmem_parts_bytes() || a->E > 1024 || (long long)a->E * a->N > 0x7fffffffll) return 0;
+  float *factor = (float *)((char *)ws + x_bytes);
+  launch_early(gather_rows_scaled_kernel, dim3((unsigned)a->M), dim3(SCALED_THREADS), st, (const uint4 *)a->input, a->sorted_pairs, (uint4 *)ws, factor, a->K, a->topk,
+               a->row_per_pair, (long long)a->size_m);
+  if (int rc = launched("moe: gather rows")) return rc;
+  TmemCall c = tmem_call<Fp8Row>(Fp8Ctx{(const uint8_t *)a->weights, w_scale, bR, bC});
+  c.x16 = ws, c.out_bf16 = true, c.out = a->out, c.M = a->M, c.N = a->N, c.K = a->K, c.factor = factor;
+  c.offsets = a->offsets, c.pairs = a->sorted_pairs, c.topkw = a->topk_weights, c.size_m = a->size_m, c.E = a->E;
+  c.mean_tokens = (double)a->M / a->E, c.min_run_k = tmem_min_run(), c.parts = (char *)ws + x_bytes + f_bytes, c.parts_bytes = ws_bytes - x_bytes - f_bytes, c.sync = sync;
+  return gemm_tmem(c, st);
+}
+
 template <typename Row, bool BF16, typename OutT, typename TI>
 int moe_launch(const lb200_moe_args *a, const typename Row::Ctx &ctx, void *ws, size_t ws_bytes, cudaStream_t st, void *sync = nullptr, bool older = true) {
   if (int rc = ensure_encode()) return rc;
@@ -1192,6 +1259,8 @@ int moe_umma(const lb200_moe_args *a, int kind, const float *w_scale, int bR, in
       return 0;
   } else {
     if (a->K % 128 || bC % 64 || bR <= 0 || a->N % bR || a->K % bC) return 0;
+    if (a->dtype == LB200_BF16)
+      if (int took = moe_fp8_f16(a, w_scale, bR, bC, ws, wsb, sync, st)) return took;
     const Fp8Ctx ctx{(const uint8_t *)a->weights, w_scale, bR, bC};
     if (a->dtype == LB200_BF16)
       rc = moe_launch<Fp8Row, true, __nv_bfloat16, __nv_bfloat16>(a, ctx, ws, wsb, st, sync, !few);

@@ -339,6 +339,68 @@ struct TmFp8 {
   }
 };
 
+// ---- the same for f16 operands, whole blocks of 128 rows and 128 k under one scale.  A code is exact in f16 and one conversion gives
+// two of them; the scale, over a power of two that puts the row block's largest at [64, 128) (the epilogue multiplies by it again), is
+// rounded to f16 and so is the product: 2^-12 each where the bf16 weight has 2^-9.  Five instructions per four weights
+// instead of a dozen through f32: 64 pairs over 64 experts of 4096 x 7168 220 -> 205 us (5.6 TB/s of weights), with 128 tokens to an expert
+// 712 -> 694 (there the clock falls with the power), error against 64 bits 2.2e-3 -> 1.66e-3, of which the bf16 output is 1.64e-3.  Scales below 2^-11 of the largest lose bits of their smallest codes, at most 2^-40 of the largest weights.
+struct TmFp8H {
+  struct Ctx {
+    const uint8_t *w;
+    const float *scale;
+    int bR;
+    Div per;  // units of a block
+    int cols; // blocks of a row
+  };
+  static constexpr int SLOT = 32 * 128, BYTES = 32 * 128, BOXES = 1;
+  static constexpr Box BOX[1] = {{128, 128}};
+  static __host__ __device__ __forceinline__ size_t stride(int K) { return (size_t)K; }
+  static __host__ __device__ __forceinline__ const uint8_t *base(const Ctx &c) { return c.w; }
+  static __device__ __forceinline__ void copy(uint32_t slot, const CUtensorMap *m, uint32_t bar, int u, int y) { tma_rows(slot, m, bar, (uint32_t)(u * 128), y); }
+  // Exponent (biased) of the power of two that a row's scales are multiplied by; the whole warp, rows of one block.
+  static __device__ __forceinline__ int exponent(const Ctx &c, int r) {
+    const float *s = c.scale + (size_t)(r / c.bR) * c.cols;
+    uint32_t top = 0;
+    for (int i = threadIdx.x & 31; i < c.cols; i += 32) {
+      const uint32_t b = __float_as_uint(__ldg(s + i)) & 0x7fffffffu;
+      if (b < 0x7f800000u) top = max(top, b);
+    }
+    return min(253, 260 - max((int)(__reduce_max_sync(0xffffffffu, top) >> 23), 1));
+  }
+  static __device__ __forceinline__ float unscale(const Ctx &c, int r) { return __uint_as_float((uint32_t)(254 - exponent(c, r)) << 23); }
+  const float *sr;
+  float mult, ns;
+  __half2 s2;
+  uint32_t q[32];
+  __device__ __forceinline__ TmFp8H(const Ctx &) {}
+  __device__ __forceinline__ void row(const Ctx &c, int r, int) {
+    sr = c.scale + (size_t)(r / c.bR) * c.cols;
+    mult = __uint_as_float((uint32_t)exponent(c, r) << 23);
+  }
+  __device__ __forceinline__ void fetch_scales(const Ctx &c, int u) { ns = __ldg(sr + c.per(u)) * mult; }
+  __device__ __forceinline__ void load(uint32_t slot, int) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) to_words(lds128(slot + sw128(threadIdx.x & 31, j)), q + 4 * j);
+    s2 = __float2half2_rn(ns);
+  }
+  template <bool BF16, typename Put>
+  __device__ __forceinline__ void expand(int, Put &&put) const {
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+      uint32_t o[16];
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const uint32_t w = q[8 * p + i];
+        o[2 * i] = h2_bits(__hmul2(__half2(__nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w & 0xFFFFu), __NV_E4M3)), s2));
+        o[2 * i + 1] = h2_bits(__hmul2(__half2(__nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w >> 16), __NV_E4M3)), s2));
+      }
+      put(p, o);
+    }
+  }
+};
+template <typename Row> struct Unscales : std::false_type {};  // rows that carry a power of two less: the epilogue multiplies by unscale()
+template <> struct Unscales<TmFp8H> : std::true_type {};
+
 // ---- dense 16-bit rows (nothing to expand: pieces are read from the slot as they are stored)
 struct TmDense {
   struct Ctx { const uint16_t *w; };
