@@ -1526,15 +1526,15 @@ __global__ void __launch_bounds__(WARPS * 32, 2) fp8_gemv_mma_kernel(const XT *_
 // int4_gemv_f32 / _bf16, kernels/cuda/src/int4.cu:43-106.
 constexpr int I4_PITCH = 144;
 constexpr int I4_TILE_BYTES = ROWS * I4_PITCH;
-constexpr int I4_STAGES = 4;
+constexpr int I4_STAGES = 4, I4_WIDE = 16;  // ring depth; warps of the CTA for few row tiles
 
-template <int S, typename XT>
-__global__ void __launch_bounds__(WARPS * 32, 2) int4_gemv_mma_kernel(const XT *__restrict__ x, const uint8_t *__restrict__ w,
+template <int S, int W, int GRP, typename XT>
+__global__ void __launch_bounds__(W * 32, 16 / W) int4_gemv_mma_kernel(const XT *__restrict__ x, const uint8_t *__restrict__ w,
                                                                      const float *__restrict__ scales, const float *__restrict__ zeros,
                                                                      XT *__restrict__ out, int N, int K, int G) {
-  extern __shared__ __align__(16) unsigned char dyn[];  // ring: WARPS x S tiles
-  __shared__ __align__(16) unsigned char slabs[WARPS][LIMB_BYTES + 16];  // limbs, the sums of four sets of 64
-  __shared__ __align__(16) float2 red[2][WARPS * GROUP * 32];  // by group parity
+  extern __shared__ __align__(16) unsigned char dyn[];  // ring: W x S tiles
+  __shared__ __align__(16) unsigned char slabs[W][LIMB_BYTES + 16];  // limbs, the sums of four sets of 64
+  __shared__ __align__(16) float2 red[2][W * GRP * 32];  // by group parity
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int nb = K >> 8;
@@ -1543,8 +1543,8 @@ __global__ void __launch_bounds__(WARPS * 32, 2) int4_gemv_mma_kernel(const XT *
 
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(dyn) + warp * (S * I4_TILE_BYTES);
   const uint32_t slab = (uint32_t)__cvta_generic_to_shared(slabs[warp]);
-  const uint32_t red_lane = (uint32_t)__cvta_generic_to_shared(&red[0][warp * GROUP * 32 + lane]);
-  constexpr uint32_t RED_PARITY = WARPS * GROUP * 32 * 8;
+  const uint32_t red_lane = (uint32_t)__cvta_generic_to_shared(&red[0][warp * GRP * 32 + lane]);
+  constexpr uint32_t RED_PARITY = W * GRP * 32 * 8;
   const uint32_t b_off = slab + (g & 3) * LIMB_PLANE + 4 * (g >> 2) + 8 * t;  // limb g & 3 of the even (g < 4) or odd elements of word t
   const uint32_t m_off = ((lane & 7) + 8 * ((lane >> 3) & 1)) * I4_PITCH + 16 * (lane >> 4);  // ldmatrix row of this lane
   const float lane_w = limb_weight(t, true);
@@ -1554,7 +1554,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) int4_gemv_mma_kernel(const XT *
 
   // requests: a tile is 16 rows x 8 granules; lane l copies granule l & 7 of rows (l >> 3) + 4 i, i = 0..3
   const uint32_t c_row = lane >> 3, c_piece = lane & 7;
-  int i_gt = t0, i_gs = min(GROUP, t1 - t0), i_b = warp, i_rt = 0, i_slot = 0;
+  int i_gt = t0, i_gs = min(GRP, t1 - t0), i_b = warp, i_rt = 0, i_slot = 0;
   auto issue = [&]() {  // always closes a commit group, so that group counts stay uniform
     if (i_gt < t1 && warp < nb) {
       const int r0 = min((i_gt + i_rt) * ROWS, N - ROWS);
@@ -1567,8 +1567,8 @@ __global__ void __launch_bounds__(WARPS * 32, 2) int4_gemv_mma_kernel(const XT *
       }
       i_slot = (i_slot + 1) & (S - 1);
       if (++i_rt == i_gs) {
-        i_rt = 0, i_b += WARPS;
-        if (i_b >= nb) i_b = warp, i_gt += i_gs, i_gs = min(GROUP, t1 - i_gt);
+        i_rt = 0, i_b += W;
+        if (i_b >= nb) i_b = warp, i_gt += i_gs, i_gs = min(GRP, t1 - i_gt);
       }
     }
     cp_async_commit();
@@ -1622,22 +1622,22 @@ __global__ void __launch_bounds__(WARPS * 32, 2) int4_gemv_mma_kernel(const XT *
   };
 
   int slot = 0, parity = 0;
-  for (int gt = t0; gt < t1; gt += GROUP, parity ^= 1) {
-    const int gs = min(GROUP, t1 - gt);
+  for (int gt = t0; gt < t1; gt += GRP, parity ^= 1) {
+    const int gs = min(GRP, t1 - gt);
     const uint32_t red_g = red_lane + parity * RED_PARITY;
-    for (int b = warp; b < nb; b += WARPS) {
+    for (int b = warp; b < nb; b += W) {
       // this block's activations into the warp's slab; the next block's are requested meanwhile
       const float4 xv[2] = {xn[0], xn[1]};
       {
-        const int bn = b + WARPS < nb ? b + WARPS : warp;
-        if (b + WARPS < nb || gt + GROUP < t1) load_x(bn);
+        const int bn = b + W < nb ? b + W : warp;
+        if (b + W < nb || gt + GRP < t1) load_x(bn);
       }
       // scales and zeros of this block's row tiles: requested here, used after the staging and the first MMAs
-      float scg[GROUP][2], zpg[GROUP][2];
+      float scg[GRP][2], zpg[GRP][2];
       {
         const int grp = (b * 256 + 64 * t) / G;
 #pragma unroll
-        for (int rt = 0; rt < GROUP; rt++)
+        for (int rt = 0; rt < GRP; rt++)
 #pragma unroll
           for (int r = 0; r < 2; r++) {
             const size_t o = (size_t)(min((gt + min(rt, gs - 1)) * ROWS, N - ROWS) + g + 8 * r) * ngrp + grp;
@@ -1662,7 +1662,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) int4_gemv_mma_kernel(const XT *
         for (int h = 0; h < 2; h++) bl[p][h] = lds32(b_off + 64 * p + 32 * h);
       const float sx = __uint_as_float(lds32(slab + LIMB_BYTES + 4 * t));
 #pragma unroll
-      for (int rt = 0; rt < GROUP; rt++) {
+      for (int rt = 0; rt < GRP; rt++) {
         if (rt >= gs) break;
         cp_async_wait<S - 1>();  // this lane's granules of the tile have landed ...
         __syncwarp();            // ... and so have the other lanes'
@@ -1678,13 +1678,13 @@ __global__ void __launch_bounds__(WARPS * 32, 2) int4_gemv_mma_kernel(const XT *
       }
     }
     __syncthreads();  // also orders this group's reads of red[parity] before its reuse two groups on
-    for (int i = threadIdx.x; i < gs * ROWS; i += WARPS * 32) {
+    for (int i = threadIdx.x; i < gs * ROWS; i += W * 32) {
       const int rt = i >> 4, row = i & 15, gg = row & 7, hi = row >> 3;
       float v = 0.f;
 #pragma unroll
-      for (int wq = 0; wq < WARPS; wq++) {
+      for (int wq = 0; wq < W; wq++) {
         if (wq >= nb) break;  // a warp without a K block never wrote its part
-        const float2 *p = &red[parity][(wq * GROUP + rt) * 32 + gg * 4];
+        const float2 *p = &red[parity][(wq * GRP + rt) * 32 + gg * 4];
 #pragma unroll
         for (int tt = 0; tt < 4; tt++) v += hi ? p[tt].y : p[tt].x;
       }
@@ -1873,10 +1873,10 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_tok_kernel(const float
 }
 
 template <typename... Args>
-int launch_pdl(void (*kern)(Args...), unsigned grid, size_t dyn_smem, cudaStream_t st, Args... args) {
+int launch_pdl_warps(int warps, void (*kern)(Args...), unsigned grid, size_t dyn_smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(WARPS * 32);
+  cfg.blockDim = dim3(warps * 32);
   cfg.dynamicSmemBytes = dyn_smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -1887,6 +1887,11 @@ int launch_pdl(void (*kern)(Args...), unsigned grid, size_t dyn_smem, cudaStream
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
   if (e != cudaSuccess) return fail((int)e, "light_b200: matmul_q (decode): %s", cudaGetErrorString(e));
   return 0;
+}
+
+template <typename... Args>
+int launch_pdl(void (*kern)(Args...), unsigned grid, size_t dyn_smem, cudaStream_t st, Args... args) {
+  return launch_pdl_warps(WARPS, kern, grid, dyn_smem, st, args...);
 }
 
 #define g_sms (sm_count())  // SMs of the calling thread's current device (every entry point binds it first)
@@ -1997,22 +2002,35 @@ int int4_gemv_fast(const void *x, const uint32_t *codes, const float *s, const f
   static DeviceOnce attr_done;
   {
     cudaError_t e = attr_done.ensure([&] {
-      cudaError_t r = cudaFuncSetAttribute(int4_gemv_mma_kernel<I4_STAGES, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, WARPS * I4_STAGES * I4_TILE_BYTES);
-      return r != cudaSuccess ? r : cudaFuncSetAttribute(int4_gemv_mma_kernel<I4_STAGES, __nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, WARPS * I4_STAGES * I4_TILE_BYTES);
+      cudaError_t r = cudaSuccess;
+      auto room = [&](auto kern, int warps) {
+        if (r == cudaSuccess) r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, warps * I4_STAGES * I4_TILE_BYTES);
+      };
+      room(int4_gemv_mma_kernel<I4_STAGES, WARPS, GROUP, float>, WARPS), room(int4_gemv_mma_kernel<I4_STAGES, WARPS, GROUP, __nv_bfloat16>, WARPS);
+      room(int4_gemv_mma_kernel<I4_STAGES, I4_WIDE, 2, float>, I4_WIDE), room(int4_gemv_mma_kernel<I4_STAGES, I4_WIDE, 2, __nv_bfloat16>, I4_WIDE);
+      return r;
     });
     if (e != cudaSuccess) return fail((int)e, "light_b200: int4_gemv (decode): %s", cudaGetErrorString(e));
   }
   const int tiles = (N + ROWS - 1) / ROWS;
-  const unsigned grid = (unsigned)(tiles < g_sms * g_waves ? tiles : g_sms * g_waves);
-  const size_t dyn = (size_t)WARPS * I4_STAGES * I4_TILE_BYTES;
+  // Few row tiles: one CTA of sixteen warps to an SM instead of two of eight.  Each warp then stages half as many blocks of
+  // activations, which is most of its work when a block serves one tile, and for as many as two tiles together: 3584 x 18944 18.3 -> 12.9 us, 4096 x 4096
+  // 6.7 -> 5.2, 4736 x 8192 12.0 -> 9.0, 1024 x 1024 2.3 -> 2.1.
+  const bool wide = tiles <= 2 * g_sms;
+  const int warps = wide ? I4_WIDE : WARPS, most = wide ? g_sms : g_sms * g_waves;
+  const unsigned grid = (unsigned)(tiles < most ? tiles : most);
+  const size_t dyn = (size_t)warps * I4_STAGES * I4_TILE_BYTES;
   for (int m = 0; m < M; m++) {
     int rc;
+    auto go = [&](auto kern, const auto *xm, auto *ym) {
+      return launch_pdl_warps(warps, kern, grid, dyn, st, xm + (size_t)m * K, (const uint8_t *)codes, s, z, ym + (size_t)m * N, N, K, G);
+    };
     if (act_dtype == LB200_F32)
-      rc = launch_pdl(int4_gemv_mma_kernel<I4_STAGES, float>, grid, dyn, st, (const float *)x + (size_t)m * K, (const uint8_t *)codes, s, z,
-                      (float *)y + (size_t)m * N, N, K, G);
+      rc = wide ? go(int4_gemv_mma_kernel<I4_STAGES, I4_WIDE, 2, float>, (const float *)x, (float *)y)
+                : go(int4_gemv_mma_kernel<I4_STAGES, WARPS, GROUP, float>, (const float *)x, (float *)y);
     else
-      rc = launch_pdl(int4_gemv_mma_kernel<I4_STAGES, __nv_bfloat16>, grid, dyn, st, (const __nv_bfloat16 *)x + (size_t)m * K, (const uint8_t *)codes,
-                      s, z, (__nv_bfloat16 *)y + (size_t)m * N, N, K, G);
+      rc = wide ? go(int4_gemv_mma_kernel<I4_STAGES, I4_WIDE, 2, __nv_bfloat16>, (const __nv_bfloat16 *)x, (__nv_bfloat16 *)y)
+                : go(int4_gemv_mma_kernel<I4_STAGES, WARPS, GROUP, __nv_bfloat16>, (const __nv_bfloat16 *)x, (__nv_bfloat16 *)y);
     if (rc) return rc;
     if (int l = launched("int4_gemv (decode)")) return l;
   }
