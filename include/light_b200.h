@@ -94,7 +94,8 @@ LB200_API int light_b200_set_workspace(int device, void *ptr, size_t bytes);
 /* The workspace size with which light_b200_matmul_q / _multi_rows (and the int4, block-FP8 and grouped matmuls, M
  * then the number of activation rows or routed pairs) take their fastest path for M rows of K: the f16
  * copy of x plus about 42 MB of partial tiles above 64 rows; with less, those calls run a kernel that needs the copy alone.  Where K / 256
- * is odd, Q6_K rows multiply in f32 accuracy and keep six bytes per activation instead (without room for them: a slower kernel).  Up to
+ * is odd, Q6_K rows multiply in f32 accuracy and keep six bytes per activation of 4096 rows at a time instead (without room for them: a
+ * slower kernel).  Up to
  * 64 rows: what the token-tile kernels stage, or the f16 copy plus 21 MB where the tensor-memory kernel has such calls (Q8_0 from 4
  * rows, bf16 rows of 4-bit weights from 17). */
 LB200_API unsigned long long light_b200_matmul_q_workspace_bytes(int M, int K);

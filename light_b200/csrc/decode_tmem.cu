@@ -1,4 +1,4 @@
-// Batched decode, 17 to 64 activation rows (tokens) of Q4_K and Q6_K: the weights go through TENSOR MEMORY as WHOLE NUMBERS.
+// Batched decode, up to 64 activation rows (tokens), from 9 of Q4_K and from 17 of Q6_K: the weights go through TENSOR MEMORY as WHOLE NUMBERS.
 //
 // What bounds the token tiles on mma.sync (gguf_decode_nt.cu): they expand a weight in registers once per warp and multiply by the legacy
 // tensor path, which holds the pipe 8 clocks per 16 x 16 x 8; neither pipe nor issue is half busy, and time grows with the tokens
@@ -529,11 +529,12 @@ int run(const typename Row::Ctx &ctx, const float *x, float *out, int M, int N, 
 // 67.1 / 36.3; 6144 x 4096 18.6 / 14.7, 23.7 / 17.8; 8192 x 2048 17.3 / 12.9, 16.7 / 15.2; 4096 x 14336 29.4 / 21.8, 40.8 / 27.8.  At 4096 x
 // 4096 they are even (13.6 / 13.9, 17.6 / 17.4) and below the tiles are ahead (4096 x 2048 9.3 / 9.8, 1024 x 4096 9.3 / 10.7): a
 // tile is cut into too many parts.  Q6_K: 4096 x 14336 32.8 / 29.7, 44.5 / 33.7; 2048 x 5632 19.7 / 15.9, but 64 rows 20.7 / 21.8; 2048 x 2048
-// 11.4 / 9.0; 128256 x 4096 186 / 156, 307 / 170.  Up to 16 rows the tiles multiply half as much (28672 x 4096 32.8 / 33).
+// 11.4 / 9.0; 128256 x 4096 186 / 156, 307 / 170.  9 to 16 rows of Q4_K: 28672 x 4096 32.9 / 28.3, 14336 x 4096 21.2 / 19.2, 6144 x 4096 14.5 /
+// 14.2, 4096 x 14336 23.0 / 20.5, but Q6_K 4096 x 14336 28.1 / 28.8.
 int gguf_decode_tmem(int type, const float *x, const void *w, float *out, int M, int N, int K, void *ws, size_t ws_bytes, cudaStream_t st) {
-  static const int min_m = knob("LIGHT_B200_DECODE_TMEM_MIN_M", 17);
+  static const int q4_min = knob("LIGHT_B200_DECODE_TMEM_MIN_M", 9), q6_min = q4_min > 17 ? q4_min : 17;
   const long long size = (long long)N * K;
-  if (M < min_m || M > MAX_NT || K % 256 || !ws || N < 128 || size >> 8 > 1ll << 30 || ((uintptr_t)x & 15)) return 0;
+  if (M < (type == LB200_Q4_K ? q4_min : q6_min) || M > MAX_NT || K % 256 || !ws || N < 128 || size >> 8 > 1ll << 30 || ((uintptr_t)x & 15)) return 0;
   if (type == LB200_Q4_K && size >= 16ll << 20 && (N > 4096 || K > 4096) && !((uintptr_t)w & 15)) return run<ExQ4K>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);
   if (type == LB200_Q6_K && size >= (M > 32 ? 16ll : 4ll) << 20 && !((uintptr_t)w & 3) && (K >> 8) % 2 == 0)
     return run<ExQ6K>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);

@@ -379,6 +379,7 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) q6k_rows_kernel(const float
 // straight from L2, 152 us and 8.8 ms; 32 rows to a warp and half the warps, 115 us and 5.5 ms.
 // Tokens with infinities or NaN (whose limbs mean nothing; their power of two is NaN) are multiplied again in f32.
 constexpr int LIMB_RECORD = 1536;  // a token's block: [sub-block][t][limbs 0, 1 of four k], then [sub-block][t][limb 2 of four k]
+constexpr int LIMB_CHUNK = 4096;   // rows whose limbs are kept at a time: six bytes per activation
 constexpr int LIMB_PASS = 16, LIMB_WARPS = 8, LIMB_RT = 1, LIMB_ROWS = 16 * LIMB_RT;
 constexpr int LIMB_RING = 2, LIMB_PITCH = 240, LIMB_SLOT = LIMB_ROWS * LIMB_PITCH;  // blocks of a warp's rows on their way
 constexpr int LIMB_TOKEN = LIMB_RECORD + 64, LIMB_STAGE = LIMB_PASS * LIMB_TOKEN;   // the pass's tokens, in shared memory for all warps; the pad
@@ -386,8 +387,9 @@ constexpr int LIMB_TOKEN = LIMB_RECORD + 64, LIMB_STAGE = LIMB_PASS * LIMB_TOKEN
 constexpr int LIMB_SMEM = LIMB_WARPS * LIMB_RING * LIMB_SLOT + 2 * LIMB_STAGE;      // (two CTAs to an SM)
 __device__ int g_limb_status;  // non-zero: a bounded wait gave up (sticky)
 
+// Records of rows (of pairs, in expert order) first .. first + M - 1.
 __global__ void __launch_bounds__(256) x_limbs_kernel(const float *__restrict__ in, const int64_t *__restrict__ pairs, uint8_t *__restrict__ limbs, float *__restrict__ ups,
-                                                      long long M, int K, int topk, int row_per_pair, long long size_m) {
+                                                      long long first, long long M, int K, int topk, int row_per_pair, long long size_m) {
   pdl_launch_dependents();
   pdl_wait();
   const int nb = K >> 8, lane = threadIdx.x & 31;
@@ -395,7 +397,7 @@ __global__ void __launch_bounds__(256) x_limbs_kernel(const float *__restrict__ 
   if (rec >= M * nb) return;
   const long long i = rec / nb;
   const int b = (int)(rec - i * nb);
-  long long p = pairs ? pairs[i] : i;
+  long long p = pairs ? pairs[first + i] : first + i;
   if (p < 0 || p >= size_m) p = 0;  // (not stored)
   const float4 *x = reinterpret_cast<const float4 *>(in + (size_t)(row_per_pair ? p : p / topk) * K + b * 256);
   const float4 v[2] = {__ldg(x + lane), __ldg(x + lane + 32)};
@@ -442,8 +444,8 @@ __device__ __forceinline__ void mma_from_zero(float (&d)[4], const uint32_t (&a)
 
 __global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const float *__restrict__ in, const uint8_t *__restrict__ w, const uint8_t *__restrict__ limbs,
                                                                    const float *__restrict__ ups, const int64_t *__restrict__ pairs, const int32_t *__restrict__ offsets,
-                                                                   const float *__restrict__ topkw, float *__restrict__ out, long long M, long long size_m, int E, int N,
-                                                                   int K, int topk, int row_per_pair) {
+                                                                   const float *__restrict__ topkw, float *__restrict__ out, long long first, long long M, long long size_m, int E,
+                                                                   int N, int K, int topk, int row_per_pair) {
   extern __shared__ __align__(16) unsigned char ring_mem[];
   __shared__ __align__(8) uint64_t bars[2];
   __shared__ int abort_flag;
@@ -457,7 +459,7 @@ __global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const flo
   pdl_launch_dependents();
   pdl_wait();
   __syncthreads();
-  const long long i0 = offsets ? offsets[e] : 0, i1 = offsets ? offsets[e + 1] : M;
+  const long long i0 = max(offsets ? (long long)offsets[e] : 0ll, first), i1 = min(offsets ? (long long)offsets[e + 1] : first + M, first + M);
   if (i0 + (long long)blockIdx.z * LIMB_PASS >= i1) return;
   const int r0 = min((int)(blockIdx.x * LIMB_WARPS + warp) * LIMB_ROWS, N - LIMB_ROWS), nb = K >> 8;  // the last rows are pulled back: duplicates store equal values
   const size_t row_bytes = (size_t)nb * 210;
@@ -490,7 +492,7 @@ __global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const flo
         __syncwarp();
         if (lane < cnt)
           asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(stages + at * LIMB_STAGE + lane * LIMB_TOKEN),
-                       "l"(limbs + ((size_t)(t0 + lane) * nb + b) * LIMB_RECORD), "r"(LIMB_RECORD), "r"(bar)
+                       "l"(limbs + ((size_t)(t0 - first + lane) * nb + b) * LIMB_RECORD), "r"(LIMB_RECORD), "r"(bar)
                        : "memory");
       }
     };
@@ -505,7 +507,7 @@ __global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const flo
 #pragma unroll
       for (int j = 0; j < 2; j++)
 #pragma unroll
-        for (int c = 0; c < 2; c++) two_to[j][c] = __ldg(ups + (size_t)(t0 + min(8 * j + 2 * t + c, cnt - 1)) * nb + b);
+        for (int c = 0; c < 2; c++) two_to[j][c] = __ldg(ups + (size_t)(t0 - first + min(8 * j + 2 * t + c, cnt - 1)) * nb + b);
       cp_async_wait<LIMB_RING - 1>();
       const uint32_t at = (used + b) & 1u, xs = stages + at * LIMB_STAGE + g * LIMB_TOKEN;  // operand column g: token g of each group
       if (!umma::mbar_wait(bar0 + 8 * at, ((used + b) >> 1) & 1u, &abort_flag)) g_limb_status = 1;
@@ -638,34 +640,38 @@ __global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const flo
   }
 }
 
-size_t q6k_limbs_ws_bytes(long long M, int K) { return (size_t)M * (K >> 8) * LIMB_RECORD + (((size_t)M * (K >> 8) * 4 + 1023) & ~(size_t)1023); }
+size_t q6k_limbs_ws_bytes(long long M, int K) {
+  const size_t records = (size_t)(M < LIMB_CHUNK ? M : LIMB_CHUNK) * (K >> 8);
+  return records * LIMB_RECORD + ((records * 4 + 1023) & ~(size_t)1023);
+}
 
 // 1: took the call; 0: no room in the workspace, or fewer rows than a warp's
 static int q6k_limbs(const float *in, const void *w, const int64_t *pairs, const int32_t *offsets, const float *topkw, float *out, long long M, long long size_m,
                      int E, int N, int K, int topk, int row_per_pair, int device, cudaStream_t st) {
   size_t bytes = 0;
   uint8_t *ws = (uint8_t *)workspace_ptr(device, &bytes);
-  const long long records = M * (K >> 8);
-  if (!ws || bytes < q6k_limbs_ws_bytes(M, K) || N < LIMB_ROWS || ((uintptr_t)in & 15) || (records + 7) / 8 > 0x7fffffffll) return 0;
-  float *ups = (float *)(ws + (size_t)records * LIMB_RECORD);
-  launch_early(x_limbs_kernel, dim3((unsigned)((records + 7) / 8)), dim3(256), st, in, pairs, ws, ups, M, K, topk, row_per_pair, size_m);
-  if (int rc = launched("q6_k: activations to limbs")) return rc;
+  if (!ws || bytes < q6k_limbs_ws_bytes(M, K) || N < LIMB_ROWS || ((uintptr_t)in & 15)) return 0;
   static DeviceOnce attr;
   const cudaError_t err = attr.ensure([] { return cudaFuncSetAttribute(q6k_limbs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LIMB_SMEM); });
   if (err != cudaSuccess) return fail((int)err, "light_b200: q6_k rows: %s", cudaGetErrorString(err));
-  const long long nb = (N + LIMB_ROWS * LIMB_WARPS - 1) / (LIMB_ROWS * LIMB_WARPS), passes = (M + LIMB_PASS - 1) / LIMB_PASS, want = (4ll * sm_count() + nb * E - 1) / (nb * E);
-  long long z = want < passes ? want : passes;  // CTAs that share an expert's tokens, where experts and rows alone do not fill the GPU
-  if (z > 65535) z = 65535;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)nb, (unsigned)E, (unsigned)z), cfg.blockDim = dim3(LIMB_WARPS * 32), cfg.dynamicSmemBytes = LIMB_SMEM, cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at, cfg.numAttrs = 1;
-  const cudaError_t e2 = cudaLaunchKernelEx(&cfg, q6k_limbs_kernel, in, (const uint8_t *)w, (const uint8_t *)ws, (const float *)ups, pairs, offsets, topkw, out, M, size_m, E,
-                                            N, K, topk, row_per_pair);
-  if (e2 != cudaSuccess) return fail((int)e2, "light_b200: q6_k rows: %s", cudaGetErrorString(e2));
-  if (int rc = launched("q6_k rows (limbs)")) return rc;
+  for (long long first = 0; first < M; first += LIMB_CHUNK) {
+    const long long m = M - first < LIMB_CHUNK ? M - first : LIMB_CHUNK, records = m * (K >> 8);
+    float *ups = (float *)(ws + (size_t)records * LIMB_RECORD);
+    launch_early(x_limbs_kernel, dim3((unsigned)((records + 7) / 8)), dim3(256), st, in, pairs, ws, ups, first, m, K, topk, row_per_pair, size_m);
+    if (int rc = launched("q6_k: activations to limbs")) return rc;
+    const long long nb = (N + LIMB_ROWS * LIMB_WARPS - 1) / (LIMB_ROWS * LIMB_WARPS), passes = (m + LIMB_PASS - 1) / LIMB_PASS, want = (4ll * sm_count() + nb * E - 1) / (nb * E);
+    const long long z = want < passes ? want : passes;  // CTAs that share an expert's tokens, where experts and rows alone do not fill the GPU
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)nb, (unsigned)E, (unsigned)z), cfg.blockDim = dim3(LIMB_WARPS * 32), cfg.dynamicSmemBytes = LIMB_SMEM, cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at, cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, q6k_limbs_kernel, in, (const uint8_t *)w, (const uint8_t *)ws, (const float *)ups, pairs, offsets, topkw, out, first, m,
+                                             size_m, E, N, K, topk, row_per_pair);
+    if (e != cudaSuccess) return fail((int)e, "light_b200: q6_k rows: %s", cudaGetErrorString(e));
+    if (int rc = launched("q6_k rows (limbs)")) return rc;
+  }
   return 1;
 }
 

@@ -1,4 +1,4 @@
-"""Q4_K and Q6_K with 17 to 64 rows as whole numbers through tensor memory, where it can go wrong: rows that are no whole tile, one block per
+"""Q4_K with 9 to 64 rows and Q6_K with 17 to 64 as whole numbers through tensor memory, where it can go wrong: rows that are no whole tile, one block per
 row, runs that start and end inside tiles and tiles cut into many runs, token counts on both sides of a chunk.
 
 x is rounded to f16 (taken out of the comparison), a Q4_K weight is exact, a Q6_K weight's scale x code is rounded to 11 bits: 2^-11 of it at
@@ -18,7 +18,7 @@ def test_whole_numbers(cuda, dt, N, K):
     w = ops.QTensor(synth.gaussian_weight(N + K, dt, N, K, device=cuda).reshape(-1), dt, (N, K))
     W = ops.Dequantize(w).double()
     g = torch.Generator().manual_seed(N)
-    for M in (17, 32, 33, 48, 49, 64):
+    for M in (9, 16, 17, 32, 33, 48, 49, 64):
         x = torch.randn(M, K, generator=g).to(cuda)
         y = ops.MatMulQ(x, w)
         assert torch.equal(y, ops.MatMulQ(x, w)), "partial tiles must be added in a fixed order"

@@ -47,8 +47,9 @@ def test_int4_rows_beyond_f16(cuda, G, scale):
     assert rel_l2(ops.MatMulInt4(x, w).cpu().double().numpy(), want.cpu().numpy()) <= 2.5e-3
 
 
-# whole passes of 16 tokens and one more, rows that are no whole tile, one block per row, runs of more than the ring's blocks
-@pytest.mark.parametrize("M,N,K", [(65, 32, 256), (80, 33, 768), (81, 300, 1280), (500, 130, 2816)])
+# whole passes of 16 tokens and one more, rows that are no whole tile, one block per row, runs of more than the ring's blocks, more rows
+# than limbs are kept of at a time
+@pytest.mark.parametrize("M,N,K", [(65, 32, 256), (4100, 48, 256), (80, 33, 768), (81, 300, 1280), (500, 130, 2816)])
 @pytest.mark.parametrize("kind", ["normal", "outlier", "tiny", "huge"])
 def test_q6_k_in_limbs(cuda, M, N, K, kind):
     """Per output: the fixed point rounds an activation at 2^-30 of the power of two above its block's largest, 2^-30 max|x| sum|w| in all;
@@ -62,6 +63,21 @@ def test_q6_k_in_limbs(cuda, M, N, K, kind):
     W, X = ops.Dequantize(w).double(), x.double()
     bound = 2.0**-30 * X.abs().amax(1, keepdim=True) * W.abs().sum(1) + (16 + K / 256) * 2.0**-22 * (X.abs() @ W.abs().t())
     assert bool(((ops.MatMulQ(x, w).double() - X @ W.t()).abs() <= bound).all())
+
+
+def test_grouped_q6_k_in_limbs_of_many_pairs(cuda):
+    """Experts on both sides of the 4096 pairs whose limbs are kept at a time, one of them across."""
+    E, T, topk, N, K = 3, 3000, 2, 40, 768
+    q = ops.QTensor(synth.gaussian_weight(4, ops.Q6_K, E * N, K, device=cuda).reshape(-1), ops.Q6_K, (E, N, K))
+    W = ops.Dequantize(q).double().reshape(E, N, K)
+    g = torch.Generator().manual_seed(6)
+    x = torch.randn(T, K, generator=g).to(cuda)
+    ids = torch.randint(0, E, (T, topk), generator=g).to(cuda)
+    wt = torch.rand(T * topk, generator=g).to(cuda)
+    y = ops.MoEGemmQ(x, q, ops.MoERouteFromIDs(ids, wt, T, topk), wt, topk)
+    want = torch.einsum("mk,mnk->mn", x.double().repeat_interleave(topk, 0), W[ids.reshape(-1)]) * wt.double()[:, None]
+    assert rel_l2(y.cpu().double().numpy(), want.cpu().numpy()) <= 1e-6
+    assert ops.prefill_status(0) == 0
 
 
 def test_q6_k_in_limbs_infinities_and_nan(cuda):
