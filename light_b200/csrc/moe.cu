@@ -370,8 +370,8 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) q6k_rows_kernel(const float
 // activations become 31-bit fixed point, as in the one-row kernels, cut into three signed whole numbers of 11 bits (LIMBS), which f16 holds,
 // as it does a code.  One MMA (m16n8k16: 16 rows, 8 tokens, one limb) is then a sub-block's exact sum: three of them and 12 f32 operations
 // a lane (limbs together, times the sub-block's scale) replace 64 multiply-adds, and rounding starts where those 12 do.  Building
-// the operand takes some 900 of the 1550 instructions per 16 rows, block and 16 tokens, and issue is what bounds this kernel
-// (61 % of the slots, the tensor pipe 30 %).
+// the operand takes some 900 of the 1665 instructions per 16 rows, block and 16 tokens, and issue is what bounds this kernel
+// (63 % of the slots, the tensor pipe 24 %).
 //   616 pairs over 128 experts of 2048 x 768:  247 -> 117 us;   2048 rows of 4096 x 14080:  16.2 -> 5.4 ms;   65 rows of 4096 x 2816:
 //   110 -> 68 us.  Blocks are added with their rounding errors kept (5 % of the time): 2.1e-8 to 3.6e-8 off against 64 bits where the f32
 //   sums were 5.3e-8 to 1.3e-7 off (K = 256 to 14080; without, 1.1e-7 at 11008).
