@@ -146,6 +146,9 @@ int moe_route_topk(const float *probs, int64_t *ids, float *weights, int T, int 
 void *workspace_ptr(int device, size_t *bytes);
 size_t prefill_sk_ws_bytes();
 // one dequantize-and-multiply of gemm_tmem.cu: 1 = took the call, 0 = not covered, other = error
+// Of an expert's word of TmemCall::modes, whose other bits mean nothing there: f16 does not hold its tokens or weights, they are bf16; some
+// row's factor is outside 2^-64 .. 2^64.
+constexpr int MODE_BF16 = (int)0x80000000, MODE_APART = 0x40000000;
 struct TmemCall {
   enum Kind { Q4K, Q6K, Q80, INT4, FP8, DENSE } kind;
   const void *w;            // packed weights (E, N, K)
@@ -161,6 +164,7 @@ struct TmemCall {
   const int64_t *pairs;
   const float *topkw;
   const float *factor;      // FP8, grouped: x16 holds f16 rows over a power of two each, which this multiplies by again (bf16 output)
+  const int32_t *modes;     // FP8, grouped, a word per expert (null: no matter): with factor the experts without MODE_BF16 are this call's, else those with it
   long long size_m;
   int E;
   double mean_tokens;       // tokens per matrix (grouped: pairs / experts)

@@ -64,6 +64,8 @@ struct Args {
   const int64_t *pairs;     // grouped: token row i goes to output row pairs[i] ...
   const float *topkw;       // ... scaled by its routing weight (or null)
   const float *factor;      // f16 tokens over a power of two each: token row i is to be multiplied by factor[i] (null: as they are)
+  const int32_t *modes;     // see TmemCall
+  int mode;                 // with modes: of the experts that are this launch's
   long long size_m;
   int E, M, N, K;
   int nt_max;               // most tokens of a tile
@@ -88,12 +90,13 @@ __device__ __forceinline__ void st_if(bool p, __nv_bfloat16 *o, float v) {
 // ------------------------------------------------------------------------------------ work list
 // Experts with their token tiles: preT[e] tiles and preW[e] weighted units before expert e.  Within an expert the token
 // tiles of one row tile follow one another, so that its packed weights are read from HBM once and from L2 after that.
-template <int CG>
+template <int CG, bool MODES>  // MODES: some experts may be another launch's
 struct Work {
   const Args &a;
-  const int *preT, *preW;
+  const int *preT, *preW, *counts;  // counts (MODES): of the experts that are this launch's, with MODE_APART
   int nb, nrt;
-  __device__ __forceinline__ int count(int e) const { return a.offsets ? a.offsets[e + 1] - a.offsets[e] : a.M; }
+  __device__ __forceinline__ int count_of(int e) const { return a.offsets ? a.offsets[e + 1] - a.offsets[e] : a.M; }
+  __device__ __forceinline__ int count(int e) const { return MODES ? counts[e] & (MODE_APART - 1) : count_of(e); }
   __device__ __forceinline__ int first(int e) const { return a.offsets ? a.offsets[e] : 0; }
   __device__ __forceinline__ void geo(int cnt, int &ntt, int &nt) const {
     ntt = (cnt + a.nt_max - 1) / a.nt_max;
@@ -131,6 +134,10 @@ struct Work {
     w.tt = 0;
     if (++w.rt < nrt) return;
     w.rt = 0;
+    if (MODES && a.modes && a.mode) {  // (few experts of many: no walk from one to the next)
+      if (w.t < preT[a.E]) w = walk(w.t);
+      return;
+    }
     do w.e++;
     while (w.e < a.E && count(w.e) == 0);
     if (w.e >= a.E) return;  // (the list's end)
@@ -181,9 +188,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   const uint32_t full = sBar, empty = full + 8 * NAS, d_full = empty + 8 * NAS, d_empty = d_full + 16, drained = d_empty + 16, w_full = drained + 8,
                  t_full = w_full + 8 * EXPANDERS, t_empty = t_full + 8 * NBS, tagged = t_empty + 8 * NBS;
   int *preW = reinterpret_cast<int *>(gen + (sBar - base) + BAR_BYTES), *preT = preW + a.E + 1;
+  [[maybe_unused]] int *const counts = preT + a.E + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = CG == 2 ? (int)cluster_ctarank() : 0;
-  const Work<CG> wk{a, preT, preW, a.K / KU, (a.N + 128 * CG - 1) / (128 * CG)};
+  const Work<CG, HasModes<Row>::value> wk{a, preT, preW, counts, a.K / KU, (a.N + 128 * CG - 1) / (128 * CG)};
   const int nb = wk.nb;
   const int G = gridDim.x / CG, cta = blockIdx.x / CG;
 
@@ -202,6 +210,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   // (every CTA of this grid is resident once all have come by here: the next kernel's wait for room, and for its operands)
   pdl_launch_dependents();
   if (a.offsets) pdl_wait();
+  if constexpr (HasModes<Row>::value) {
+    bool any = false;
+    for (int e = threadIdx.x; e < a.E; e += THREADS) {
+      const int cnt = wk.count_of(e), m = a.modes ? a.modes[e] : a.mode;
+      counts[e] = (m & MODE_BF16) == a.mode ? cnt | (m & MODE_APART) : 0;
+      any |= cnt > 0 && (m & MODE_BF16) == a.mode;
+    }
+    if (a.modes && a.mode && !__syncthreads_or(any)) return;  // (mostly: no expert is left to the bf16 launch)
+  }
   for (int e = threadIdx.x; e < a.E; e += THREADS) {
     int ntt, nt;
     wk.geo(wk.count(e), ntt, nt);
@@ -361,19 +378,28 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       const int c0 = first + lane * step;
       if (c0 < nt) asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(sync()->flags + (blockIdx.x * 4 + quad) * 16 + (c0 >> 4)), "r"(tag) : "memory");
     };
-    // Output row (-1: none) and routing weight of token c0 + lane of a tile.
-    auto route = [&](const Tile &T, int c0, int &prow, float &pw) {
+    // Rows over powers of two (Unscales): what a row block's sums are to be multiplied by (the warp's rows of the tile), negative where some token's
+    // factor times its routing weight may leave f32's range, so that they are multiplied by one after the other; a token row's factor.
+    [[maybe_unused]] auto unscale = [&](const Tile &T) {
+      if constexpr (Unscales<Row>::value)
+        return copysignf(Row::unscale(ctx, T.expert * a.N + min(T.n0 + 128 * rank + quad * 32, a.N - 1)), counts[T.expert] & MODE_APART ? -1.f : 1.f);
+      else
+        return 1.f;
+    };
+    [[maybe_unused]] auto factor = [&](const Tile &T, int c0) { return T.m0 + c0 + lane < T.m_end ? a.factor[T.m0 + c0 + lane] : 1.f; };
+    // Output row (-1: none) and routing weight, with the row's factor if `joint`, of token c0 + lane of a tile.
+    auto route = [&](const Tile &T, int c0, [[maybe_unused]] bool joint, int &prow, float &pw) {
       prow = -1, pw = 1.f;
       if (T.m0 + c0 + lane < T.m_end) {
         prow = T.m0 + c0 + lane;
-        const float f = a.factor ? a.factor[prow] : 1.f;
         if (a.offsets) {
           const long long p = a.pairs[prow];
           prow = p >= 0 && p < a.size_m ? (int)p : -1;
           if (prow >= 0 && a.topkw) pw = a.topkw[p];
         }
-        pw *= f;
       }
+      if constexpr (Unscales<Row>::value)
+        if (joint) pw *= factor(T, c0);
     };
     // The run's last segment, 16 tokens at a time: chunks first, first + step, ...  `shared`: five warps of this row quarter take
     // turns (only where K is long enough that an expander cannot get here before the segment before the last but one is
@@ -391,8 +417,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
         while (jlast + 1 < G && wk.bound(jlast + 1, G) < (t + 1) * nb) jlast++;
       const int col = T.n0 + 128 * rank + row;
       const bool live = col < a.N;
-      [[maybe_unused]] float scale = 1.f;
-      if constexpr (Unscales<Row>::value) scale = Row::unscale(ctx, T.expert * a.N + min(T.n0 + 128 * rank + quad * 32, a.N - 1));
+      const float scale = unscale(T);
       if (!warp_wait(d_full + 8 * (seg & 1), (seg >> 1) & 1, abort) || !warp_wait(tagged, 0, abort)) return;
       tc_fence_after();
       const unsigned tag = tag_sh;
@@ -448,12 +473,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
         } else {
           int prow;
           float pw;
-          route(T, c0, prow, pw);
+          route(T, c0, scale > 0.f, prow, pw);
+          [[maybe_unused]] const float power = scale < 0.f ? factor(T, c0) : 1.f;
           OutT *o = out + col;
 #pragma unroll
           for (int i = 0; i < 16; i++) {
             const int m = __shfl_sync(0xffffffffu, prow, i);
-            const float y = Unscales<Row>::value ? __uint_as_float(v[i]) * scale : __uint_as_float(v[i]), f = __shfl_sync(0xffffffffu, pw, i) * y;
+            const float y = Unscales<Row>::value ? __uint_as_float(v[i]) * fabsf(scale) : __uint_as_float(v[i]);
+            float f = __shfl_sync(0xffffffffu, pw, i) * y;
+            if constexpr (Unscales<Row>::value) f *= __shfl_sync(0xffffffffu, power, i);
             st_if(live && m >= 0, o + (long long)m * a.N, f);
           }
         }
@@ -588,8 +616,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
           finish_last(0, shared ? 80 : 16);
           break;
         }
-        [[maybe_unused]] float scale = 1.f;
-        if constexpr (Unscales<Row>::value) scale = Row::unscale(ctx, T.expert * a.N + min(T.n0 + 128 * rank + quad * 32, a.N - 1));
+        const float scale = unscale(T);
         if (!warp_wait(d_full + 8 * (seg & 1), (seg >> 1) & 1, abort)) break;
         tc_fence_after();
         const uint32_t d = tmem + lanes + (T.nt > 128 ? 0 : 128 * (seg & 1));
@@ -614,14 +641,21 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
           }
           int prow;
           float pw;
-          route(T, c0, prow, pw);
+          route(T, c0, scale > 0.f, prow, pw);
           if constexpr (Unscales<Row>::value) {
 #pragma unroll
-            for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * scale);
+            for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * fabsf(scale));
           }
           if (a.topkw || a.factor) {
 #pragma unroll
             for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * __shfl_sync(0xffffffffu, pw, i));
+          }
+          if constexpr (Unscales<Row>::value) {
+            if (scale < 0.f) {
+              const float power = factor(T, c0);
+#pragma unroll
+              for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * __shfl_sync(0xffffffffu, power, i));
+            }
           }
           if (bulk) {  // through a strip of the warp's own: [32 tokens][32 rows], no other warp to wait for
             const uint32_t buf = strip + (chunk & 1) * SB;
@@ -758,7 +792,7 @@ template <typename Row, bool BF16, typename OutT>
 int pick(const typename Row::Ctx &ctx, const TmemCall &c, cudaStream_t st) {
   if (c.K % KU || c.E > MAX_E || (c.offsets && (c.M / 16 + c.E) * ((c.N + 127) / 128) * (c.K / KU) >= 1ll << 31)) return 0;
   Args a = {};
-  a.offsets = c.offsets, a.pairs = c.pairs, a.topkw = c.topkw, a.factor = c.factor, a.size_m = c.size_m;
+  a.offsets = c.offsets, a.pairs = c.pairs, a.topkw = c.topkw, a.factor = c.factor, a.modes = c.modes, a.mode = c.factor ? 0 : MODE_BF16, a.size_m = c.size_m;
   a.E = c.offsets ? c.E : 1, a.M = (int)c.M, a.N = c.N, a.K = c.K;
   static const int k_cg = knob("LIGHT_B200_TMEM_CG", 0), k_nt = knob("LIGHT_B200_TMEM_NT", 0), k_wmin = knob("LIGHT_B200_TMEM_WMIN", 128), k_pair = knob("LIGHT_B200_TMEM_PAIR", 0);
   a.wmin = k_wmin;
@@ -799,7 +833,7 @@ int gemm_tmem(const TmemCall &c, cudaStream_t st) {
       return c.bf16 ? pick<TmInt4, true, __nv_bfloat16>(x, c, st) : pick<TmInt4, false, float>(x, c, st);
     }
     case TmemCall::FP8: {
-      if (c.factor) {
+      if (c.factor && c.modes) {
         if (c.bR % 128 || c.bC % KU || c.N % c.bR) return 0;
         return pick<TmFp8H, false, __nv_bfloat16>({(const uint8_t *)c.w, c.s, c.bR, Div::of(c.bC / KU), c.K / c.bC}, c, st);
       }

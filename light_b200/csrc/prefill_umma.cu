@@ -1122,15 +1122,39 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const TI *__restrict__
   }
 }
 
-// Rows of bf16 tokens in expert order as f16, over a power of two each that puts the row's largest element at [2^14, 2^15): exact for elements
-// down to 2^-31 of it, and factor[i] = the power.  (A row with infinities or NaN keeps them, and its other elements only their sign:
-// they do not matter beside those.)  A CTA to a row, held in registers (up to 8192 elements; the rest is read twice).
-constexpr int SCALED_THREADS = 128, SCALED_KEPT = 8;
+// Rows of bf16 tokens in expert order as f16, over a power of two each that puts the row's largest element at [2^14, 2^15), factor[i] = the power:
+// exact for elements down to 2^-31 of the largest, to 2^-40 of the largest below.  A CTA to a row, held in registers (up to
+// 8192 elements; the rest is read twice).  A row with infinities or NaN keeps them, and of its other elements the signs and zeros: beside
+// those they matter where they meet an infinity or NaN among the weights.  More CTAs look at the experts' scales, a warp to a row block.
+//
+// Where f16 would hold less than bf16 does, the expert's counts[] entry (which nothing reads after the launch that wrote it) gets MODE_BF16:
+// a finite row where f16 does not hold one in sixteen elements, or a row block whose scales are more than 2^16 apart (zeros aside), or so
+// large or small that a sum may leave f32's range between the multiplications by the two powers.  (Single elements below 2^-31 of the largest
+// are in every other row of a SiLU's outputs; an output that meets only those, all others' weights being zero, is off by 2^-40 of the
+// largest times its weight.)
+constexpr int SCALED_THREADS = 128, SCALED_WARPS = SCALED_THREADS / 32, SCALED_KEPT = 8;
 __global__ void __launch_bounds__(SCALED_THREADS) gather_rows_scaled_kernel(const uint4 *__restrict__ in, const int64_t *__restrict__ pairs, uint4 *__restrict__ dst,
-                                                                           float *__restrict__ factor, int K, int topk, int row_per_pair, long long size_m) {
+                                                                           float *__restrict__ factor, int M, int K, int topk, int row_per_pair, long long size_m,
+                                                                           const float *__restrict__ scale, int blocks, int cols, const int32_t *__restrict__ offsets,
+                                                                           int32_t *__restrict__ modes, int E) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ uint32_t tops[SCALED_THREADS / 32];
+  if ((int)blockIdx.x >= M) {
+    const int per = (blocks + SCALED_WARPS - 1) / SCALED_WARPS, rest = (int)blockIdx.x - M, e = rest / per;
+    const int b = (rest - e * per) * SCALED_WARPS + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (b >= blocks || offsets[e + 1] <= offsets[e]) return;
+    const float *s = scale + ((size_t)e * blocks + b) * cols;
+    const int x = fp8_scale_exponent(s, cols);
+    const float mult = __uint_as_float((uint32_t)x << 23);
+    bool wide = false;
+    for (int i = lane; i < cols; i += 32) {
+      const float v = fabsf(__ldg(s + i));
+      if (v > 0.f && isfinite(v)) wide |= v * mult < 0x1p-10f || v >= 0x1p64f || x > 197;  // (the last: the largest is below 2^-64)
+    }
+    if (__any_sync(0xffffffffu, wide) && lane == 0) atomicOr(modes + e, MODE_BF16);
+    return;
+  }
+  __shared__ uint32_t tops[SCALED_WARPS], losses[SCALED_WARPS];
   const long long i = blockIdx.x, p = pairs[i];
   const bool ok = p >= 0 && p < size_m;
   const int n = K >> 3;  // pieces of eight elements
@@ -1153,16 +1177,22 @@ __global__ void __launch_bounds__(SCALED_THREADS) gather_rows_scaled_kernel(cons
   if ((threadIdx.x & 31) == 0) tops[threadIdx.x >> 5] = mx;
   __syncthreads();
 #pragma unroll
-  for (int j = 0; j < SCALED_THREADS / 32; j++) mx = max(mx, tops[j]);
+  for (int j = 0; j < SCALED_WARPS; j++) mx = max(mx, tops[j]);
   const bool finite = mx < 0x7F80u;
-  const int e = max((int)(mx >> 7), 1), sb = finite ? min(253, 268 - e) : 127;  // biased exponent of the multiplier
-  const float f = __uint_as_float((uint32_t)sb << 23);
-  if (threadIdx.x == 0) factor[i] = __uint_as_float((uint32_t)(254 - sb) << 23);
+  const int e = max((int)(mx >> 7), 1), sb = finite && mx ? min(253, 268 - e) : 127;  // biased exponent of the multiplier
+  const float f = __uint_as_float((uint32_t)sb << 23), power = __uint_as_float((uint32_t)(254 - sb) << 23);
+  if (threadIdx.x == 0) factor[i] = power;
   uint4 *to = dst + (size_t)i * n;
+  int lost = 0;
   auto two = [&](uint32_t w) {
     const float x = __uint_as_float(w << 16), y = __uint_as_float(w & 0xFFFF0000u);
-    if (finite) return pack_h2(x * f, y * f);
-    auto keep = [](float v) { return isfinite(v) ? copysignf(0.f, v) : v; };
+    if (finite) {
+      const __half2 h = __floats2half2_rn(x * f, y * f);
+      const float2 back = __half22float2(h);
+      lost += (back.x * power != x) + (back.y * power != y);
+      return *reinterpret_cast<const uint32_t *>(&h);
+    }
+    auto keep = [](float v) { return isfinite(v) && v != 0.f ? copysignf(1.f, v) : v; };
     return pack_h2(keep(x), keep(y));
   };
   auto put = [&](int k, const uint4 &q) { to[k] = make_uint4(two(q.x), two(q.y), two(q.z), two(q.w)); };
@@ -1172,21 +1202,64 @@ __global__ void __launch_bounds__(SCALED_THREADS) gather_rows_scaled_kernel(cons
     if (k < n) put(k, kept[j]);
   }
   for (int k = threadIdx.x + SCALED_KEPT * SCALED_THREADS; k < n; k += SCALED_THREADS) put(k, ok ? __ldg(src + k) : make_uint4(0, 0, 0, 0));
+  lost = __reduce_add_sync(0xffffffffu, lost);
+  if ((threadIdx.x & 31) == 0) losses[threadIdx.x >> 5] = (uint32_t)lost;
+  __syncthreads();
+  if (threadIdx.x) return;
+  lost = 0;
+#pragma unroll
+  for (int j = 0; j < SCALED_WARPS; j++) lost += (int)losses[j];
+  const int mode = (lost > K / 16 ? MODE_BF16 : 0) | (power < 0x1p-64f || power > 0x1p64f ? MODE_APART : 0);
+  if (!mode) return;
+  int lo = 0, hi = E;  // the expert whose row this is, if any
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (offsets[mid + 1] <= (int)i) lo = mid + 1;
+    else hi = mid;
+  }
+  if (lo < E && offsets[lo] <= (int)i) atomicOr(modes + lo, mode);
 }
 
-// bf16 tokens times FP8 weights in whole 128 x 128 blocks, grouped, with f16 operands.  1: took the call, 0: not covered, other: error.
+// The rows of experts with bf16 operands once more, as they are.
+__global__ void __launch_bounds__(SCALED_THREADS) gather_rows_again_kernel(const uint4 *__restrict__ in, const int64_t *__restrict__ pairs, uint4 *__restrict__ dst, int K,
+                                                                          int topk, int row_per_pair, long long size_m, const int32_t *__restrict__ offsets,
+                                                                          const int32_t *__restrict__ modes) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int e = blockIdx.x, n = K >> 3;
+  if (!(modes[e] & MODE_BF16)) return;
+  for (int i = offsets[e] + (int)blockIdx.y; i < offsets[e + 1]; i += gridDim.y) {
+    const long long p = pairs[i];
+    const bool ok = p >= 0 && p < size_m;
+    const uint4 *src = in + (ok ? (size_t)(row_per_pair ? p : p / topk) * n : 0);
+    for (int k = threadIdx.x; k < n; k += SCALED_THREADS) dst[(size_t)i * n + k] = ok ? __ldg(src + k) : make_uint4(0, 0, 0, 0);
+  }
+}
+
+// bf16 tokens times FP8 weights in whole 128 x 128 blocks, grouped: f16 operands for the experts for which they hold what bf16 does, then
+// bf16 operands for the rest, mostly none: then the two launches take 13 us of a sparse block of 8 tokens (504 -> 517).  1: took the call, 0: not covered,
+// other: error.
 int moe_fp8_f16(const lb200_moe_args *a, const float *w_scale, int bR, int bC, void *ws, size_t ws_bytes, void *sync, cudaStream_t st) {
   const size_t x_bytes = ((size_t)a->M * a->K * 2 + 1023) & ~(size_t)1023, f_bytes = ((size_t)a->M * 4 + 1023) & ~(size_t)1023;
-  if (!use_tmem() || bR % 128 || bC % 128 || ws_bytes < x_bytes + f_bytes + gemm_tmem_parts_bytes() || a->E > 1024 || (long long)a->E * a->N > 0x7fffffffll) return 0;
+  const long long looks = (long long)a->E * ((a->N / bR + SCALED_WARPS - 1) / SCALED_WARPS);
+  if (!use_tmem() || bR % 128 || bC % 128 || ws_bytes < x_bytes + f_bytes + gemm_tmem_parts_bytes() || a->E > 1024 || (long long)a->E * a->N > 0x7fffffffll ||
+      a->M >= MODE_APART || a->M + looks > 0x7fffffffll)
+    return 0;
   float *factor = (float *)((char *)ws + x_bytes);
-  launch_early(gather_rows_scaled_kernel, dim3((unsigned)a->M), dim3(SCALED_THREADS), st, (const uint4 *)a->input, a->sorted_pairs, (uint4 *)ws, factor, a->K, a->topk,
-               a->row_per_pair, (long long)a->size_m);
+  launch_early(gather_rows_scaled_kernel, dim3((unsigned)(a->M + looks)), dim3(SCALED_THREADS), st, (const uint4 *)a->input, a->sorted_pairs, (uint4 *)ws, factor, (int)a->M, a->K,
+               a->topk, a->row_per_pair, (long long)a->size_m, w_scale, a->N / bR, a->K / bC, (const int32_t *)a->offsets, a->counts, a->E);
   if (int rc = launched("moe: gather rows")) return rc;
   TmemCall c = tmem_call<Fp8Row>(Fp8Ctx{(const uint8_t *)a->weights, w_scale, bR, bC});
-  c.x16 = ws, c.out_bf16 = true, c.out = a->out, c.M = a->M, c.N = a->N, c.K = a->K, c.factor = factor;
+  c.x16 = ws, c.out_bf16 = true, c.out = a->out, c.M = a->M, c.N = a->N, c.K = a->K, c.factor = factor, c.modes = a->counts;
   c.offsets = a->offsets, c.pairs = a->sorted_pairs, c.topkw = a->topk_weights, c.size_m = a->size_m, c.E = a->E;
   c.mean_tokens = (double)a->M / a->E, c.min_run_k = tmem_min_run(), c.parts = (char *)ws + x_bytes + f_bytes, c.parts_bytes = ws_bytes - x_bytes - f_bytes, c.sync = sync;
-  return gemm_tmem(c, st);
+  if (int took = gemm_tmem(c, st); took != 1) return took;
+  launch_early(gather_rows_again_kernel, dim3((unsigned)a->E, 8), dim3(SCALED_THREADS), st, (const uint4 *)a->input, a->sorted_pairs, (uint4 *)ws, a->K, a->topk, a->row_per_pair,
+               (long long)a->size_m, (const int32_t *)a->offsets, (const int32_t *)a->counts);
+  if (int rc = launched("moe: gather rows again")) return rc;
+  c.factor = nullptr, c.bf16 = true;
+  const int took = gemm_tmem(c, st);
+  return took ? took : fail(LB200_E_SHAPE, "light_b200: moe: no bf16 kernel behind the f16 one");
 }
 
 template <typename Row, bool BF16, typename OutT, typename TI>

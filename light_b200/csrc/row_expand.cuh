@@ -372,6 +372,15 @@ struct Fp8Ctx {
   const float *scale;
   int bR, bC;
 };
+// Exponent (biased) of the power of two that puts the largest finite of `cols` scales at [64, 128); the whole warp.
+__device__ __forceinline__ int fp8_scale_exponent(const float *__restrict__ s, int cols) {
+  uint32_t top = 0;
+  for (int i = threadIdx.x & 31; i < cols; i += 32) {
+    const uint32_t b = __float_as_uint(__ldg(s + i)) & 0x7fffffffu;
+    if (b < 0x7f800000u) top = max(top, b);
+  }
+  return min(253, 260 - max((int)(__reduce_max_sync(0xffffffffu, top) >> 23), 1));
+}
 struct Fp8Row {
   using Ctx = Fp8Ctx;
   static constexpr bool KPERM = false;

@@ -341,9 +341,13 @@ struct TmFp8 {
 
 // ---- the same for f16 operands, whole blocks of 128 rows and 128 k under one scale.  A code is exact in f16 and one conversion gives
 // two of them; the scale, over a power of two that puts the row block's largest at [64, 128) (the epilogue multiplies by it again), is
-// rounded to f16 and so is the product: 2^-12 each where the bf16 weight has 2^-9.  Five instructions per four weights
+// rounded to f16 and so is the product: 2^-11 each at most where the bf16 weight has 2^-8.  Five instructions per four weights
 // instead of a dozen through f32: 64 pairs over 64 experts of 4096 x 7168 220 -> 205 us (5.6 TB/s of weights), with 128 tokens to an expert
-// 712 -> 694 (there the clock falls with the power), error against 64 bits 2.2e-3 -> 1.66e-3, of which the bf16 output is 1.64e-3.  Scales below 2^-11 of the largest lose bits of their smallest codes, at most 2^-40 of the largest weights.
+// 712 -> 694 (there the clock falls with the power), error against 64 bits 2.2e-3 -> 1.66e-3, of which the bf16 output is 1.64e-3.
+//
+// f16 has the range for that while a row block's scales lie within 2^16 of each other: the smallest normal code then gives 2^-16 and is
+// as exact as in bf16.  Experts with scales further apart (zeros aside), or with a token that f16 does not hold, are left to a launch with
+// bf16 operands, as above, that follows.
 struct TmFp8H {
   struct Ctx {
     const uint8_t *w;
@@ -357,16 +361,7 @@ struct TmFp8H {
   static __host__ __device__ __forceinline__ size_t stride(int K) { return (size_t)K; }
   static __host__ __device__ __forceinline__ const uint8_t *base(const Ctx &c) { return c.w; }
   static __device__ __forceinline__ void copy(uint32_t slot, const CUtensorMap *m, uint32_t bar, int u, int y) { tma_rows(slot, m, bar, (uint32_t)(u * 128), y); }
-  // Exponent (biased) of the power of two that a row's scales are multiplied by; the whole warp, rows of one block.
-  static __device__ __forceinline__ int exponent(const Ctx &c, int r) {
-    const float *s = c.scale + (size_t)(r / c.bR) * c.cols;
-    uint32_t top = 0;
-    for (int i = threadIdx.x & 31; i < c.cols; i += 32) {
-      const uint32_t b = __float_as_uint(__ldg(s + i)) & 0x7fffffffu;
-      if (b < 0x7f800000u) top = max(top, b);
-    }
-    return min(253, 260 - max((int)(__reduce_max_sync(0xffffffffu, top) >> 23), 1));
-  }
+  static __device__ __forceinline__ int exponent(const Ctx &c, int r) { return fp8_scale_exponent(c.scale + (size_t)(r / c.bR) * c.cols, c.cols); }
   static __device__ __forceinline__ float unscale(const Ctx &c, int r) { return __uint_as_float((uint32_t)(254 - exponent(c, r)) << 23); }
   const float *sr;
   float mult, ns;
@@ -400,6 +395,9 @@ struct TmFp8H {
 };
 template <typename Row> struct Unscales : std::false_type {};  // rows that carry a power of two less: the epilogue multiplies by unscale()
 template <> struct Unscales<TmFp8H> : std::true_type {};
+template <typename Row> struct HasModes : std::false_type {};  // rows whose experts may be shared out over two launches
+template <> struct HasModes<TmFp8H> : std::true_type {};
+template <> struct HasModes<TmFp8> : std::true_type {};
 
 // ---- dense 16-bit rows (nothing to expand: pieces are read from the slot as they are stored)
 struct TmDense {
