@@ -364,12 +364,15 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) q6k_rows_kernel(const float
   }
 }
 
-// ------------------------------------------------------------------------------------ the same products in whole numbers
+// ------------------------------------------------------------------------------------ the same products on the tensor cores
 //
-// What bounds q6k_rows_kernel is f32 issue: eight multiply-adds per lane, token and weight row for every block.  Here a block's 256
-// activations become 31-bit fixed point, as in the one-row kernels, cut into three signed whole numbers of 11 bits (LIMBS), which f16 holds,
-// as it does a code.  One MMA (m16n8k16: 16 rows, 8 tokens, one limb) is then a sub-block's exact sum: three of them and 12 f32 operations
-// a lane (limbs together, times the sub-block's scale) replace 64 multiply-adds, and rounding starts where those 12 do.  Building
+// What bounds q6k_rows_kernel is f32 issue: eight multiply-adds per lane, token and weight row for every block.  Here an activation is the sum
+// of three f16 values (LIMBS), and a code is exact in f16.  The first limb is a whole number of 2^-8 of the power of two above the largest
+// of the block's 256, so that its sums are exact; the second and third are the rest, rounded to eleven bits and again.  An activation above
+// 2^-9 of that power so keeps all its bits, one below 23 of its own, down to 2^-38: f32 products hold 24.  (In fixed point to the
+// end, the third limb 2^-30 of that power, small activations lost bits: 512 outputs of 768 whose weights are zero at one
+// element of 1000 beside N(0, 0.05) were 5.5e-6 off; 9.5e-8 now, 8.9e-8 with f32 products.)  One MMA (m16n8k16: 16 rows, 8 tokens, one limb) is a sub-block's sum: three of
+// them and 12 f32 operations a lane (limbs together, times the sub-block's scale) replace 64 multiply-adds.  Building
 // the operand takes some 900 of the 1665 instructions per 16 rows, block and 16 tokens, and issue is what bounds this kernel
 // (63 % of the slots, the tensor pipe 24 %).
 //   616 pairs over 128 experts of 2048 x 768:  247 -> 117 us;   2048 rows of 4096 x 14080:  16.2 -> 5.4 ms;   65 rows of 4096 x 2816:
@@ -409,25 +412,20 @@ __global__ void __launch_bounds__(256) x_limbs_kernel(const float *__restrict__ 
   m = __reduce_max_sync(0xffffffffu, m);
   const int s = min(156 - (int)(m >> 23), 126);  // |x| 2^s < 2^30
   const float scale = __uint_as_float((uint32_t)(127 + s) << 23);
-  if (lane == 0) ups[rec] = m >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : __uint_as_float((uint32_t)(127 - s) << 23);
+  if (lane == 0) ups[rec] = m >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : __uint_as_float((uint32_t)(149 - s) << 23);  // of the first limb: 2^22
   uint8_t *dst = limbs + (size_t)rec * LIMB_RECORD;
 #pragma unroll
   for (int j = 0; j < 2; j++) {  // elements 128 j + 4 lane ..: sub-block 8 j + lane / 4, t = lane % 4
     const float xs[4] = {v[j].x * scale, v[j].y * scale, v[j].z * scale, v[j].w * scale};
     uint32_t l[3][2];
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-      float f[3][2];
-#pragma unroll
-      for (int c = 0; c < 2; c++) {  // X = l0 + 2^11 l1 + 2^22 l2, l0 and l1 in [-1024, 1023]
-        const int X = __float2int_rn(xs[2 * k + c]), l0 = ((X + 1024) & 2047) - 1024, X1 = (X - l0) >> 11, l1 = ((X1 + 1024) & 2047) - 1024;
-        f[0][c] = (float)l0, f[1][c] = (float)l1, f[2][c] = (float)((X1 - l1) >> 11);
-      }
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const __half2 h = __floats2half2_rn(f[c][0], f[c][1]);
-        l[c][k] = *reinterpret_cast<const uint32_t *>(&h);
-      }
+    for (int k = 0; k < 2; k++) {  // x 2^s = 2^22 l2 + 2^6 l1 + 2^-5 l0; every difference is exact
+      const float a = xs[2 * k], b = xs[2 * k + 1], ta = rintf(a * 0x1p-22f), tb = rintf(b * 0x1p-22f);
+      const float ra = fmaf(ta, -0x1p22f, a), rb = fmaf(tb, -0x1p22f, b);
+      const __half2 h2 = __floats2half2_rn(ta, tb), h1 = __floats2half2_rn(ra * 0x1p-6f, rb * 0x1p-6f);
+      const float2 back = __half22float2(h1);
+      const __half2 h0 = __floats2half2_rn(fmaf(back.x, -0x1p6f, ra) * 0x1p5f, fmaf(back.y, -0x1p6f, rb) * 0x1p5f);
+      l[0][k] = *reinterpret_cast<const uint32_t *>(&h0), l[1][k] = *reinterpret_cast<const uint32_t *>(&h1), l[2][k] = *reinterpret_cast<const uint32_t *>(&h2);
     }
     const int at = (8 * j + (lane >> 2)) * 4 + (lane & 3);
     *reinterpret_cast<uint4 *>(dst + at * 16) = make_uint4(l[0][0], l[0][1], l[1][0], l[1][1]);
@@ -503,7 +501,7 @@ __global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const flo
     int slot = 0;
     for (int b = 0; b < nb; b++) {
       issue(b + LIMB_RING - 1, slot == 0 ? LIMB_RING - 1 : slot - 1);
-      float two_to[2][2];  // what the tokens' limbs count in
+      float two_to[2][2];  // what the tokens' first limbs count in
 #pragma unroll
       for (int j = 0; j < 2; j++)
 #pragma unroll
@@ -518,7 +516,7 @@ __global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const flo
         const uint32_t a = al + r * (8 * LIMB_PITCH) + at;
         return __funnelshift_r(lds32(a), lds32(a + 4), sh);
       };
-      float top[LIMB_RT][2][4], low[LIMB_RT][2][4];  // scale x sub-block's sum: limb 2 (whole, and exact below 2^24), limbs 1 and 0
+      float top[LIMB_RT][2][4], low[LIMB_RT][2][4];  // scale x sub-block's sum: limb 2 (whole, and exact below 2^24), limbs 1 and 0 (in units of the latter)
 #pragma unroll
       for (int i = 0; i < 8 * LIMB_RT; i++) top[i >> 3][(i >> 2) & 1][i & 3] = low[i >> 3][(i >> 2) & 1][i & 3] = 0.f;
 #pragma unroll 1
@@ -582,11 +580,11 @@ __global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const flo
         for (int j = 0; j < 2; j++)
 #pragma unroll
           for (int c = 0; c < 2; c++) {
-            // acc + d 2^.. (2^22 top + low), the roundings of the product and of the sum kept (d 2^.. has eleven bits: exact)
+            // acc + d 2^.. (top + 2^-27 low), the roundings of both products and of both sums kept (d 2^.. has eleven bits: exact)
             const int i = 2 * (r & 1) + c;
             float &y = acc[r >> 1][j][i];
-            const float s = d * two_to[j][c], s22 = s * 4194304.f, v = s22 * top[r >> 1][j][i], t = y + v, z = t - y;
-            rest[r >> 1][j][i] += ((y - (t - z)) + (v - z)) + fmaf(s, low[r >> 1][j][i], fmaf(s22, top[r >> 1][j][i], -v));
+            const float s = d * two_to[j][c], l = low[r >> 1][j][i] * 0x1p-27f, v = s * top[r >> 1][j][i], w = fmaf(s, l, v), t = y + w, z = t - y;
+            rest[r >> 1][j][i] += ((y - (t - z)) + (w - z)) + (fmaf(s, l, v - w) + fmaf(s, top[r >> 1][j][i], -v));
             y = t;
           }
       }

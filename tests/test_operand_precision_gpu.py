@@ -52,7 +52,7 @@ def test_int4_rows_beyond_f16(cuda, G, scale):
 @pytest.mark.parametrize("M,N,K", [(65, 32, 256), (4100, 48, 256), (80, 33, 768), (81, 300, 1280), (500, 130, 2816)])
 @pytest.mark.parametrize("kind", ["normal", "outlier", "tiny", "huge"])
 def test_q6_k_in_limbs(cuda, M, N, K, kind):
-    """Per output: the fixed point rounds an activation at 2^-30 of the power of two above its block's largest, 2^-30 max|x| sum|w| in all;
+    """Per output: an activation is held to 2^-23 of itself or 2^-60 of its block's largest, less than 2^-30 max|x| sum|w| in all;
     per block and limb pair the whole sums and their scaling are rounded three times, blocks are added in f32: fewer than 16 + K / 256
     roundings of terms that together stay below four times sum|w x|."""
     w = ops.QTensor(synth.gaussian_weight(N + K, ops.Q6_K, N, K, device=cuda).reshape(-1), ops.Q6_K, (N, K))
@@ -94,3 +94,56 @@ def test_q6_k_in_limbs_infinities_and_nan(cuda):
     assert torch.equal(y[y.isinf()].sign(), want[want.isinf()].sign())
     fin = want.isfinite()
     assert rel_l2(y[fin].numpy(), want[fin].numpy()) <= 1e-6
+
+
+def _zero_at(w, N, K, column):
+    """The blocks with the code of 0 at this element (of 256) of every block."""
+    raw = w.reshape(N, K // 256, 210).clone()
+    assert column < 32
+    raw[:, :, column] &= 0xF0
+    raw[:, :, 128 + column] = (raw[:, :, 128 + column] & 0xFC) | 2
+    return raw.reshape(-1)
+
+
+@pytest.mark.parametrize("M,N,K", [(65, 64, 256), (100, 512, 768), (333, 130, 2816), (200, 64, 11008)])
+@pytest.mark.parametrize("large,sigma", [(0, 1.0), (5, 0.05), (1000, 1.0), (1000, 0.05), (1e6, 0.05), (1e9, 0.05)])
+def test_q6_k_small_activations_beside_large_ones(cuda, M, N, K, large, sigma):
+    """Outputs whose weights are zero where a block's large activation is.  The small ones keep 23 bits (2^-23 each, at random), what is done in
+    a block is rounded some 16 times, 2^-24 each: together about 2^-23 = 1.2e-7 (f32 products are 8.1e-8 to 1.46e-7 off at these sizes); without
+    large ones the sums of a sub-block are whole numbers and blocks are added exactly: 2.5e-8, and 5e-8 is twice that."""
+    raw = synth.gaussian_weight(N + K, ops.Q6_K, N, K, device=cuda)
+    w = ops.QTensor(_zero_at(raw, N, K, 9) if large else raw.reshape(-1), ops.Q6_K, (N, K))
+    W = ops.Dequantize(w).double()
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(cuda) * sigma
+    if large:
+        assert not W[:, 9::256].any()
+        x[:, 9::256] = large
+    y = ops.MatMulQ(x, w).double()
+    assert rel_l2(y.cpu().numpy(), (x.double() @ W.t()).cpu().numpy()) <= (2.0**-23 if large else 5e-8)
+
+
+def test_grouped_q6_k_small_activations_beside_large_ones(cuda):
+    E, T, topk, N, K = 4, 200, 2, 96, 768
+    raw = synth.gaussian_weight(2, ops.Q6_K, E * N, K, device=cuda)
+    q = ops.QTensor(_zero_at(raw, E * N, K, 9), ops.Q6_K, (E, N, K))
+    W = ops.Dequantize(q).double().reshape(E, N, K)
+    g = torch.Generator().manual_seed(3)
+    x = (0.05 * torch.randn(T, K, generator=g)).to(cuda)
+    x[:, 9::256] = 1e5
+    ids = torch.randint(0, E, (T, topk), generator=g).to(cuda)
+    y = ops.MoEGemmQ(x, q, ops.MoERouteFromIDs(ids, torch.ones(T * topk, device=cuda), T, topk), None, topk)
+    want = torch.einsum("mk,mnk->mn", x.double().repeat_interleave(topk, 0), W[ids.reshape(-1)])
+    assert rel_l2(y.cpu().double().numpy(), want.cpu().numpy()) <= 2.0**-23
+
+
+@pytest.mark.parametrize("kind", ["normal", "silu"])
+def test_q6_k_of_ordinary_activations_is_no_less_exact_than_f32_products(cuda, kind):
+    M, N, K = 300, 256, 2816
+    w = ops.QTensor(synth.gaussian_weight(8, ops.Q6_K, N, K, device=cuda).reshape(-1), ops.Q6_K, (N, K))
+    g = torch.Generator().manual_seed(9)
+    x = torch.randn(M, K, generator=g)
+    if kind == "silu":
+        x = torch.nn.functional.silu(4 * x) * torch.randn(M, K, generator=g)
+    x = x.to(cuda)
+    want = x.double() @ ops.Dequantize(w).double().t()
+    assert rel_l2(ops.MatMulQ(x, w).cpu().double().numpy(), want.cpu().numpy()) <= 6e-8   # f32 products: 1.0e-7
