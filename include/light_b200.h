@@ -93,9 +93,8 @@ LB200_API int light_b200_set_workspace(int device, void *ptr, size_t bytes);
 
 /* The workspace size with which light_b200_matmul_q / _multi_rows (and the int4, block-FP8 and grouped matmuls, M
  * then the number of activation rows or routed pairs) take their fastest path for M rows of K: the f16
- * copy of x plus about 42 MB of partial tiles above 64 rows; with less, those calls run a kernel that needs the copy alone.  Where K / 256
- * is odd, Q6_K rows multiply in f32 accuracy and keep six bytes per activation of 4096 rows at a time instead (without room for them: a
- * slower kernel).  Up to
+ * copy of x plus about 42 MB of partial tiles above 64 rows; with less, those calls run a kernel that needs the copy alone.  (Q6_K with an
+ * odd K / 256 uses none of it: light_b200_q6k_scratch_bytes below.)  Up to
  * 64 rows: what the token-tile kernels stage, or the f16 copy plus 21 MB where the tensor-memory kernel has such calls (Q8_0 from 4
  * rows, bf16 rows of 4-bit weights from 17). */
 LB200_API unsigned long long light_b200_matmul_q_workspace_bytes(int M, int K);
@@ -115,6 +114,15 @@ LB200_API int light_b200_block_bytes(int ggml_type);
  * dequantize + SGEMM; here one call covers decode and prefill). */
 LB200_API int light_b200_matmul_q(int ggml_type, const float *x, const void *w, float *out, int M, int N, int K, int device,
                         void *stream);
+
+/* Q6_K rows that start on any even byte (K / 256 odd, or w off a 4-byte, grouped a 16-byte boundary) multiply in f32 accuracy; above 64
+ * activation rows, grouped from 256 pairs, they do so on the tensor cores if the call is given memory of its own: `scratch`, device memory
+ * of light_b200_q6k_scratch_bytes (0: the call has no use for any) or more, 256-byte aligned, uninitialised, which nothing else uses
+ * until the call has run.  Six bytes per activation of up to 4096 rows.  Without, a kernel with f32 products runs that takes about three
+ * times as long.  Neither uses the workspace: such calls may overlap on the GPU. */
+LB200_API unsigned long long light_b200_q6k_scratch_bytes(int ggml_type, const void *w, int64_t rows, int K, int grouped);
+LB200_API int light_b200_matmul_q_scratch(int ggml_type, const float *x, const void *w, float *out, int M, int N, int K, void *scratch,
+                                          unsigned long long scratch_bytes, int device, void *stream);
 
 /* light_b200_matmul_q_multi for a small batch: x f32 (M, K) against up to four quantized matrices of one type
  * that share it, out[i] (M, n[i]) dense.  2 <= M <= 32 and Q4_K run as ONE launch (the token-column decode
@@ -313,6 +321,7 @@ LB200_API int light_b200_moe_gemm_static_scratch(const lb200_moe_args *args, int
 /* Registry key {moe_gemm_q, CUDA, <w dtype>} (reference kernels/cuda/moe.go:99-141):
  * x f32, GGUF block-quantized experts, out f32. */
 LB200_API int light_b200_moe_gemm_q(const lb200_moe_args *args, int device, void *stream);
+LB200_API int light_b200_moe_gemm_q_scratch(const lb200_moe_args *args, void *scratch, unsigned long long scratch_bytes, int device, void *stream);
 
 /* Zeroes the rows (of row_bytes each) of out (rows, ..) that no sorted pair with an expert id in [0, E) writes; the grouped
  * matmuls leave those untouched.  bits: ceil(rows / 32) words of scratch.  Replaces clearing all of `out` beforehand. */

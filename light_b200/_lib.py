@@ -79,6 +79,9 @@ SYMBOLS = {
     "light_b200_block_bytes": (C.c_int, [C.c_int]),
     "light_b200_matmul_q": (C.c_int, [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int,
                                       C.c_void_p]),
+    "light_b200_q6k_scratch_bytes": (C.c_ulonglong, [C.c_int, C.c_void_p, C.c_int64, C.c_int, C.c_int]),
+    "light_b200_matmul_q_scratch": (C.c_int, [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_ulonglong, C.c_int,
+                                              C.c_void_p]),
     "light_b200_matmul_q_multi": (C.c_int, [C.c_int, C.c_void_p, C.POINTER(C.c_void_p), C.POINTER(C.c_void_p),
                                             C.POINTER(C.c_int32), C.c_int, C.c_int, C.c_int, C.c_void_p]),
     "light_b200_matmul_q_multi_rows": (C.c_int, [C.c_int, C.c_void_p, C.POINTER(C.c_void_p), C.POINTER(C.c_void_p),
@@ -115,6 +118,7 @@ SYMBOLS = {
                                             C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p]),
     "light_b200_moe_gemm": (C.c_int, [C.POINTER(MoeArgs), C.c_int, C.c_void_p]),
     "light_b200_moe_gemm_q": (C.c_int, [C.POINTER(MoeArgs), C.c_int, C.c_void_p]),
+    "light_b200_moe_gemm_q_scratch": (C.c_int, [C.POINTER(MoeArgs), C.c_void_p, C.c_ulonglong, C.c_int, C.c_void_p]),
     "light_b200_moe_gemm_f8block": (C.c_int, [C.POINTER(MoeArgs), C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]),
     "light_b200_moe_scratch_bytes": (C.c_ulonglong, [C.c_int64, C.c_int]),
     "light_b200_moe_gemm_scratch": (C.c_int, [C.POINTER(MoeArgs), C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_ulonglong, C.c_int, C.c_void_p]),

@@ -158,14 +158,23 @@ unsigned long long light_b200_matmul_q_workspace_bytes(int M, int K) {
   else if (M >= 4) f16_copy = ((f16_copy + 1023) & ~1023ull) + gemm_tmem_parts_bytes();  // those of the tensor-memory kernel (Q8_0, 4-bit)
   unsigned long long staged = M <= 64 ? decode_nt_ws_bytes(M, K) : 0;
   if (M <= 64 && decode_ts_ws_bytes(M, K) > staged) staged = decode_ts_ws_bytes(M, K);
-  if (M > 64 && K % 256 == 0 && (K >> 8) % 2 && q6k_limbs_ws_bytes(M, K) > f16_copy) f16_copy = q6k_limbs_ws_bytes(M, K);  // Q6_K rows that start on any even byte
   return f16_copy > staged ? f16_copy : staged;
 }
 unsigned long long light_b200_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 int light_b200_block_elems(int t) { return block_elems(t); }
 int light_b200_block_bytes(int t) { return block_bytes(t); }
 
+// Q6_K rows that start on any even byte; where tensor memory takes the call after all, the scratch lies idle.
+unsigned long long light_b200_q6k_scratch_bytes(int t, const void *w, int64_t rows, int K, int grouped) {
+  if (t != LB200_Q6_K || rows < (grouped ? 256 : 65) || K <= 0 || K % 256 || ((K >> 8) % 2 == 0 && !((uintptr_t)w & (grouped ? 15 : 3)))) return 0;
+  return q6k_limbs_bytes(rows, K);
+}
+
 int light_b200_matmul_q(int t, const float *x, const void *w, float *out, int M, int N, int K, int device, void *stream) {
+  return light_b200_matmul_q_scratch(t, x, w, out, M, N, K, nullptr, 0, device, stream);
+}
+int light_b200_matmul_q_scratch(int t, const float *x, const void *w, float *out, int M, int N, int K, void *scratch, unsigned long long scratch_bytes, int device,
+                                void *stream) {
   const int be = block_elems(t);
   if (!be) return fail(LB200_E_DTYPE, "light_b200: matmul_q: ggml type %d has no fused kernel", t);
   if (M < 0 || N < 0 || K <= 0) return fail(LB200_E_SHAPE, "light_b200: matmul_q: bad shape M=%d N=%d K=%d", M, N, K);
@@ -176,6 +185,7 @@ int light_b200_matmul_q(int t, const float *x, const void *w, float *out, int M,
   REQUIRE_PTR(out, "matmul_q");
   if (!aligned(x, 16) || !aligned(out, 4) || !aligned(w, 2))
     return fail(LB200_E_ALIGN, "light_b200: matmul_q: x must be 16-byte, out 4-byte, w 2-byte aligned");
+  if (!aligned(scratch, 256)) return fail(LB200_E_ALIGN, "light_b200: matmul_q: scratch must be 256-byte aligned");
   if (int rc = bind(device)) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   int took = 0;
@@ -216,7 +226,7 @@ int light_b200_matmul_q(int t, const float *x, const void *w, float *out, int M,
   if (took != 0) return took == 1 ? 0 : took;
   took = gguf_gemv_batch(t, x, w, out, M, N, K, st);
   if (took != 0) return took == 1 ? 0 : took;
-  if (t == LB200_Q6_K && M > 64 && K % 256 == 0) return q6k_rows_dense(x, w, out, M, N, K, device, st);  // rows off 4-byte boundaries, or no workspace
+  if (t == LB200_Q6_K && M > 64 && K % 256 == 0) return q6k_rows_dense(x, w, out, M, N, K, scratch, (size_t)scratch_bytes, st);  // rows off 4-byte boundaries, or no workspace
   return gguf_matmul_generic(t, x, w, out, M, N, K, st);
 }
 
@@ -772,10 +782,12 @@ int light_b200_moe_gemm_scratch(const lb200_moe_args *a, const float *w_scale, i
   return a->M == 0 ? 0 : moe_gemm_f8block(a, w_scale, block_r, block_c, device, (cudaStream_t)stream, scratch, (size_t)scratch_bytes);
 }
 
-int light_b200_moe_gemm_q(const lb200_moe_args *a, int device, void *stream) {
+int light_b200_moe_gemm_q(const lb200_moe_args *a, int device, void *stream) { return light_b200_moe_gemm_q_scratch(a, nullptr, 0, device, stream); }
+int light_b200_moe_gemm_q_scratch(const lb200_moe_args *a, void *scratch, unsigned long long scratch_bytes, int device, void *stream) {
   if (int rc = moe_check(a, "moe_gemm_q", true)) return rc;
+  if (!aligned(scratch, 256)) return fail(LB200_E_ALIGN, "light_b200: moe_gemm_q: scratch must be 256-byte aligned");
   if (int rc = bind(device)) return rc;
-  return moe_gemm_q(a, device, (cudaStream_t)stream);
+  return moe_gemm_q(a, device, (cudaStream_t)stream, scratch, (size_t)scratch_bytes);
 }
 
 }  // extern "C"

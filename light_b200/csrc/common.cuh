@@ -115,10 +115,10 @@ int fp8_block_dequant(const uint8_t *w, const float *s, void *out, int out_dtype
 int fp8_block_rows_dot(const void *x, const uint8_t *w, const float *s, void *y, int act_dtype, int M, int N, int K, int bR, int bC,
                        cudaStream_t st);
 int moe_gemm(const lb200_moe_args *a, int device, cudaStream_t st, void *scratch = nullptr, size_t scratch_bytes = 0);
-int moe_gemm_q(const lb200_moe_args *a, int device, cudaStream_t st);
-// Q6_K rows that start on any even byte, many activation rows: f32 products (moe.cu)
-int q6k_rows_dense(const float *x, const void *w, float *out, int M, int N, int K, int device, cudaStream_t st);
-size_t q6k_limbs_ws_bytes(long long M, int K);
+int moe_gemm_q(const lb200_moe_args *a, int device, cudaStream_t st, void *scratch = nullptr, size_t scratch_bytes = 0);
+// Q6_K rows that start on any even byte, many activation rows (moe.cu): on the tensor cores with q6k_limbs_bytes() of scratch, else f32 products
+int q6k_rows_dense(const float *x, const void *w, float *out, int M, int N, int K, void *scratch, size_t scratch_bytes, cudaStream_t st);
+size_t q6k_limbs_bytes(long long M, int K);
 int q6k_limbs_status();
 int moe_gemm_f8block(const lb200_moe_args *a, const float *w_scale, int bR, int bC, int device, cudaStream_t st, void *scratch = nullptr,
                      size_t scratch_bytes = 0);

@@ -92,9 +92,11 @@ PyObject *linear_q(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
   const int be = light_b200_block_elems((int)type), dev = x.t->get_device();
   NEED(be > 0 && N > 0 && K % be == 0 && w.t->scalar_type() == at::kByte && w.t->numel() == N * (K / be) * light_b200_block_bytes((int)type));
   NEED(M == 1 || workspace_fits(dev, M, K));
-  at::Tensor out = out_like(*x.t, N);
-  return give(light_b200_matmul_q((int)type, x.t->const_data_ptr<float>(), w.t->const_data_ptr(), out.data_ptr<float>(), (int)M, (int)N, (int)K, dev,
-                                  stream_of(dev)), out);
+  at::Tensor out = out_like(*x.t, N), own;
+  const auto own_bytes = light_b200_q6k_scratch_bytes((int)type, w.t->const_data_ptr(), M, (int)K, 0);
+  if (own_bytes) own = at::empty({(int64_t)own_bytes}, w.t->options());
+  return give(light_b200_matmul_q_scratch((int)type, x.t->const_data_ptr<float>(), w.t->const_data_ptr(), out.data_ptr<float>(), (int)M, (int)N, (int)K,
+                                          own_bytes ? own.data_ptr() : nullptr, own_bytes, dev, stream_of(dev)), out);
 }
 
 // (x (..., K) F32 / BF16, codes I32 (N, K/8), scales, zeros F32 (N, K/G), G) -> (..., N) at x's type
@@ -268,8 +270,12 @@ PyObject *moe_gemm(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
   m.expert_ids = se.t->const_data_ptr<int64_t>(), m.counts = sc, m.offsets = sc + E, m.topk_weights = tw.t ? tw.t->const_data_ptr<float>() : nullptr;
   m.out = out.data_ptr(), m.M = M, m.size_m = M, m.E = (int)E, m.N = (int)N, m.K = (int)K, m.topk = (int)topk, m.row_per_pair = rows == M;
   m.dtype = type >= 0 ? (int)type : act_of(*x.t);
-  if (type >= 0) return give(light_b200_moe_gemm_q(&m, dev, st), out);
   at::Tensor own;
+  if (type >= 0) {
+    const auto q6k_bytes = light_b200_q6k_scratch_bytes((int)type, m.weights, M, (int)K, 1);
+    if (q6k_bytes) own = at::empty({(int64_t)q6k_bytes}, w.t->options());
+    return give(light_b200_moe_gemm_q_scratch(&m, q6k_bytes ? own.data_ptr() : nullptr, q6k_bytes, dev, st), out);
+  }
   const int64_t own_bytes = few && dt == at::kBFloat16 ? (int64_t)light_b200_moe_scratch_bytes(M, (int)K) : 0;
   if (own_bytes) own = at::empty({own_bytes}, w.t->options().dtype(at::kByte));
   return give(light_b200_moe_gemm_scratch(&m, s.t->const_data_ptr<float>(), (int)bR, (int)bC, own_bytes ? own.data_ptr() : nullptr, own_bytes, dev, st), out);

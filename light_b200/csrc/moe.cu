@@ -638,17 +638,17 @@ __global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const flo
   }
 }
 
-size_t q6k_limbs_ws_bytes(long long M, int K) {
+size_t q6k_limbs_bytes(long long M, int K) {
   const size_t records = (size_t)(M < LIMB_CHUNK ? M : LIMB_CHUNK) * (K >> 8);
   return records * LIMB_RECORD + ((records * 4 + 1023) & ~(size_t)1023);
 }
 
-// 1: took the call; 0: no room in the workspace, or fewer rows than a warp's
+// In memory of the call's own: these calls never shared the workspace, so that streams may have one each.  1: took the call; 0: no
+// (or too little) scratch, or fewer rows than a warp's.
 static int q6k_limbs(const float *in, const void *w, const int64_t *pairs, const int32_t *offsets, const float *topkw, float *out, long long M, long long size_m,
-                     int E, int N, int K, int topk, int row_per_pair, int device, cudaStream_t st) {
-  size_t bytes = 0;
-  uint8_t *ws = (uint8_t *)workspace_ptr(device, &bytes);
-  if (!ws || bytes < q6k_limbs_ws_bytes(M, K) || N < LIMB_ROWS || ((uintptr_t)in & 15)) return 0;
+                     int E, int N, int K, int topk, int row_per_pair, void *scratch, size_t bytes, cudaStream_t st) {
+  uint8_t *const ws = (uint8_t *)scratch;
+  if (!ws || bytes < q6k_limbs_bytes(M, K) || N < LIMB_ROWS || ((uintptr_t)in & 15)) return 0;
   static DeviceOnce attr;
   const cudaError_t err = attr.ensure([] { return cudaFuncSetAttribute(q6k_limbs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LIMB_SMEM); });
   if (err != cudaSuccess) return fail((int)err, "light_b200: q6_k rows: %s", cudaGetErrorString(err));
@@ -684,8 +684,8 @@ static int q6k_rows(const float *in, const void *w, const int64_t *pairs, const 
   return launched("q6_k rows (f32)");
 }
 
-int q6k_rows_dense(const float *x, const void *w, float *out, int M, int N, int K, int device, cudaStream_t st) {
-  if (int took = q6k_limbs(x, w, nullptr, nullptr, nullptr, out, M, M, 1, N, K, 1, 1, device, st)) return took == 1 ? 0 : took;
+int q6k_rows_dense(const float *x, const void *w, float *out, int M, int N, int K, void *scratch, size_t scratch_bytes, cudaStream_t st) {
+  if (int took = q6k_limbs(x, w, nullptr, nullptr, nullptr, out, M, M, 1, N, K, 1, 1, scratch, scratch_bytes, st)) return took == 1 ? 0 : took;
   return q6k_rows<false>(x, w, nullptr, nullptr, nullptr, out, M, M, 1, N, K, 1, 1, st);
 }
 
@@ -804,14 +804,14 @@ int moe_gemm_f8block(const lb200_moe_args *a, const float *w_scale, int bR, int 
   return run<__nv_bfloat16, __nv_bfloat16, F8BlockRow<__nv_bfloat16>>(a, st, aux);
 }
 
-int moe_gemm_q(const lb200_moe_args *a, int device, cudaStream_t st) {
+int moe_gemm_q(const lb200_moe_args *a, int device, cudaStream_t st, void *scratch, size_t scratch_bytes) {
   int rc = prep(a, st);
   if (rc) return rc;
   if (int took = moe_umma(a, 1, nullptr, 0, 0, device, st)) return took == 1 ? 0 : took;
   // From as many pairs on as the tensor-core path takes of the other formats.
   if (a->dtype == LB200_Q6_K && a->M >= 256 && a->K % 256 == 0 && a->E <= 65535 && a->N > 0) {
     if (int took = q6k_limbs((const float *)a->input, a->weights, a->sorted_pairs, a->offsets, a->topk_weights, (float *)a->out, a->M, a->size_m, a->E, a->N, a->K, a->topk,
-                             a->row_per_pair, device, st))
+                             a->row_per_pair, scratch, scratch_bytes, st))
       return took == 1 ? 0 : took;
     return q6k_rows<true>((const float *)a->input, a->weights, a->sorted_pairs, a->offsets, a->topk_weights, (float *)a->out, a->M, a->size_m, a->E, a->N, a->K,
                        a->topk, a->row_per_pair, st);

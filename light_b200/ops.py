@@ -153,9 +153,21 @@ def MatMulQ(x: torch.Tensor, w: QTensor) -> torch.Tensor:
     if M > 1:  # the batched paths keep an f16 copy of x (and split-K partial sums) in the workspace
         ensure_workspace(dev, int(_lib.lib().light_b200_matmul_q_workspace_bytes(M, K)))
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-    _lib.check(_lib.lib().light_b200_matmul_q(w.ggml_type, _ptr(xc), _ptr(w.data), _ptr(out), M, N, K, dev,
-                                              _stream(dev)))
+    _matmul_q(xc, w, out, M, N, K, dev)
     return out
+
+
+def _q6k_scratch(w: QTensor, rows: int, K: int, grouped: bool) -> Optional[torch.Tensor]:
+    """Memory of one call alone (Q6_K rows that start on any even byte; else None): on this stream's part of the caching allocator, so
+    that calls on several streams have one each."""
+    n = int(_lib.lib().light_b200_q6k_scratch_bytes(w.ggml_type, _ptr(w.data), rows, K, int(grouped)))
+    return torch.empty(n, dtype=torch.uint8, device=w.device) if n else None
+
+
+def _matmul_q(x: torch.Tensor, w: QTensor, out: torch.Tensor, M: int, N: int, K: int, dev: int) -> None:
+    own = _q6k_scratch(w, M, K, False)
+    _lib.check(_lib.lib().light_b200_matmul_q_scratch(w.ggml_type, _ptr(x), _ptr(w.data), _ptr(out), M, N, K, _ptr(own), 0 if own is None else own.numel(), dev,
+                                                      _stream(dev)))
 
 
 def _one_row(x: torch.Tensor, op: str) -> int:
@@ -192,6 +204,10 @@ def MatMulQMulti(x: torch.Tensor, ws: Sequence[QTensor], outs: Optional[Sequence
     nn = (C.c_int32 * n)(*[w.shape[0] for w in ws])
     if M > 1:
         ensure_workspace(dev, int(_lib.lib().light_b200_matmul_q_workspace_bytes(M, K)))
+    if M > 64 and ws[0].ggml_type == Q6_K and all(w.shape[0] > 0 for w in ws):  # a launch per matrix as it is, and some have use for memory of their own
+        for w, o in zip(ws, outs):
+            _matmul_q(xc, w, o, M, w.shape[0], K, dev)
+        return list(outs)
     _lib.check(_lib.lib().light_b200_matmul_q_multi_rows(ws[0].ggml_type, _ptr(xc), wp, op, nn, n, M, K, dev, _stream(dev)))
     return list(outs)
 
@@ -615,7 +631,11 @@ def _moe_dispatch(op: str, key_dtype: int, quant: bool, inp: torch.Tensor, weigh
                 topk_weights=0 if topk_weights is None else topk_weights.contiguous().data_ptr(), out=out.data_ptr(),
                 M=M, size_m=M, E=E, N=N, K=K, topk=topk, row_per_pair=int(row_per_pair), dtype=key_dtype)
     if quant:
-        _lib.check(_lib.lib().light_b200_moe_gemm_q(C.byref(a), dev, _stream(dev)))
+        own = None
+        n = int(_lib.lib().light_b200_q6k_scratch_bytes(key_dtype, _ptr(weights), M, K, 1))
+        if n:  # Q6_K rows that start on any even byte: memory of this call alone
+            own = torch.empty(n, dtype=torch.uint8, device=inp.device)
+        _lib.check(_lib.lib().light_b200_moe_gemm_q_scratch(C.byref(a), _ptr(own), n, dev, _stream(dev)))
         return out
     scale, bR, bC = (None, 0, 0) if f8 is None else (f8[0].contiguous(), f8[1], f8[2])
     _lib.check(_lib.lib().light_b200_moe_gemm_scratch(C.byref(a), _ptr(scale), bR, bC, _ptr(own), 0 if own is None else own.numel(), dev, _stream(dev)))

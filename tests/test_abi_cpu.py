@@ -105,3 +105,22 @@ def test_missing_library_fails_loudly(monkeypatch):
 def test_workspace_holds_the_partial_tiles_of_the_fastest_path(M, K):
     """The f16 copy of the activations, rounded up to 1 KB, and behind it a 128 KB tile for each of 160 CTAs."""
     assert _lib.lib().light_b200_matmul_q_workspace_bytes(M, K) >= (M * K * 2 + 1023) // 1024 * 1024 + 160 * 128 * 1024
+
+
+def test_workspace_of_many_rows_grows_with_k():
+    """The size asked for with the largest M and K is enough for the smaller ones, and holds the f16 copy and partial tiles alone."""
+    l = _lib.lib()
+    for M in (2, 8, 64, 65, 512, 4096):
+        sizes = [int(l.light_b200_matmul_q_workspace_bytes(M, K)) for K in range(256, 15000, 256)]
+        assert sizes == sorted(sizes)
+        assert M <= 64 or sizes[-1] <= 2 * M * 14848 + (50 << 20)
+
+
+def test_scratch_of_q6_k_rows_on_any_even_byte():
+    l = _lib.lib()
+    size = lambda t, w, rows, K, grouped: int(l.light_b200_q6k_scratch_bytes(t, C.c_void_p(w), rows, K, grouped))  # noqa: E731
+    assert size(14, 4096, 65, 768, 0) >= 65 * 768 * 6
+    assert size(14, 4096, 10**6, 768, 0) == size(14, 4096, 4096, 768, 0)      # so many rows at a time
+    assert size(14, 4096, 64, 768, 0) == size(14, 4096, 255, 768, 1) == 0     # too few rows
+    assert size(14, 4096, 65, 512, 0) == size(12, 4096, 65, 768, 0) == size(14, 4096, 65, 100, 0) == 0
+    assert size(14, 4098, 65, 512, 0) > 0 and size(14, 4104, 256, 512, 1) > 0  # rows of an even number of blocks, off the boundary

@@ -147,3 +147,45 @@ def test_q6_k_of_ordinary_activations_is_no_less_exact_than_f32_products(cuda, k
     x = x.to(cuda)
     want = x.double() @ ops.Dequantize(w).double().t()
     assert rel_l2(ops.MatMulQ(x, w).cpu().double().numpy(), want.cpu().numpy()) <= 6e-8   # f32 products: 1.0e-7
+
+
+def test_q6_k_in_limbs_shares_no_memory(cuda):
+    """Dense and grouped calls leave the workspace as it is, and several streams have calls at once."""
+    N, K, M, E, topk = 96, 1280, 300, 3, 2
+    q = ops.QTensor(synth.gaussian_weight(1, ops.Q6_K, E * N, K, device=cuda).reshape(-1), ops.Q6_K, (E, N, K))
+    w = ops.QTensor(q.data, ops.Q6_K, (E * N, K))
+    g = torch.Generator().manual_seed(2)
+    xs = [torch.randn(M, K, generator=g).to(cuda) for _ in range(4)]
+    ids = torch.randint(0, E, (M, topk), generator=g).to(cuda)
+    r = ops.MoERouteFromIDs(ids, torch.ones(M * topk, device=cuda), M, topk)
+    call = lambda x: (ops.MatMulQ(x, w), ops.MoEGemmQ(x, q, r, None, topk), ops.MatMulQMulti(x, [w])[0])  # noqa: E731
+    ops.ensure_workspace(0, 1 << 20)
+    want = [call(x) for x in xs]
+    ws = ops._workspaces[0]
+    ws.fill_(0x5A)
+    call(xs[0])
+    assert bool((ws == 0x5A).all())
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in xs]
+    got = []
+    for _ in range(3):
+        for x, s in zip(xs, streams):
+            with torch.cuda.stream(s):
+                got.append(call(x))
+    torch.cuda.synchronize()
+    for i, ys in enumerate(got):
+        assert all(torch.equal(y, z) for y, z in zip(ys, want[i % 4]))
+
+
+def test_q6_k_in_limbs_in_a_graph(cuda):
+    N, K, M = 64, 768, 100
+    w = ops.QTensor(synth.gaussian_weight(3, ops.Q6_K, N, K, device=cuda).reshape(-1), ops.Q6_K, (N, K))
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(4)).to(cuda)
+    want = ops.MatMulQ(x, w)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = ops.MatMulQ(x, w)
+    x.copy_(2 * x)
+    graph.replay()
+    assert torch.equal(y, 2 * want)
