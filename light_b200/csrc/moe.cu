@@ -509,7 +509,11 @@ __global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const flo
       cp_async_wait<LIMB_RING - 1>();
       const uint32_t at = (used + b) & 1u, xs = stages + at * LIMB_STAGE + g * LIMB_TOKEN;  // operand column g: token g of each group
       if (!umma::mbar_wait(bar0 + 8 * at, ((used + b) >> 1) & 1u, &abort_flag)) g_limb_status = 1;
-      if (__syncthreads_or(abort_flag)) return;  // (all warps, together)
+      if (__syncthreads_or(abort_flag)) {  // (all warps, together) copies still in flight get some time to land before the CTA retires
+        cp_async_wait<0>();
+        __nanosleep(50000);
+        return;
+      }
       const uint32_t blk = ring + slot * LIMB_SLOT + g * LIMB_PITCH + ((skew0 + (uint32_t)b * 210u) & 15u);  // row g's block
       const uint32_t al = blk & ~3u, sh = (blk & 2u) * 8u;
       auto word = [&](int r, int at) {  // of row g + 8 r
