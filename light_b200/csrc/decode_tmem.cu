@@ -162,9 +162,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t sB = base, sRaw = base + (uint32_t)a.stages * a.stage_bytes, sBar = sRaw + (uint32_t)EXPANDERS * Row::SLOT;
   // full, empty: a block's weights are there, its MMAs have completed; t_full, t_empty: its tokens; d_full, d_empty: its sums are
-  // complete, are read out; p_empty: the minimums' sums are.
+  // complete, are read out; p_empty: the minimums' sums are; drained: nothing of the MMA warp's is in flight.
   const uint32_t full = sBar, empty = full + 16, d_full = empty + 16, d_empty = d_full + 32, p_empty = d_empty + 32, w_full = p_empty + 8,
-                 t_full = w_full + 8 * EXPANDERS, t_empty = t_full + 8 * NBS;
+                 t_full = w_full + 8 * EXPANDERS, t_empty = t_full + 8 * NBS, drained = t_empty + 8 * NBS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nb = a.K >> 8, G = gridDim.x, cta = blockIdx.x, U = (a.N + 127) / 128 * nb;
   auto bound = [&](int j) { return (int)((long long)U * j / G); };
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
     for (int i = 0; i < 2; i++) mbar_init(full + 8 * i, 8), mbar_init(empty + 8 * i, 1);
     for (int i = 0; i < a.stages; i++) mbar_init(t_full + 8 * i, 2), mbar_init(t_empty + 8 * i, 1);
     for (int i = 0; i < a.bufs; i++) mbar_init(d_full + 8 * i, 1), mbar_init(d_empty + 8 * i, DRAINS);
-    mbar_init(p_empty, DRAINS);
+    mbar_init(p_empty, DRAINS), mbar_init(drained, 1);
     for (int i = 0; i < EXPANDERS; i++) mbar_init(w_full + 8 * i, 1);
     fence_barrier_init();
   }
@@ -248,6 +248,12 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
       __syncwarp();
       first = false;
       if (++kb == nb) kb = 0, first = true, seg++;
+    }
+    // No MMA, and none of the arrivals that nobody above waits for, may be in flight when the CTA gives its memory back, whichever way the
+    // loop ended.
+    if (elect_one()) mma_commit(drained);
+    __syncwarp();
+    for (int i = 0; i < (1 << 16) && !__all_sync(0xffffffffu, mbar_test_wait(drained, 0)); i++) {
     }
   } else if (warp < EXPANDERS) {
     // ================================================================ expanders
