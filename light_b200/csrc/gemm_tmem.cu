@@ -721,6 +721,7 @@ constexpr int fixed_smem(int E) { return EXPANDERS * Row::SLOT + STRIPS<OutT> + 
 
 template <typename Row, bool BF16, typename OutT, int CG>
 int run(const typename Row::Ctx &ctx, const TmemCall &c, Args a, int nt_max, cudaStream_t st) {
+  if (nt_max < 16 * CG || nt_max % (16 * CG) || nt_max > MAX_ROWS * CG) return 0;  // (the tensor maps and the kernel's own rounding of tiles go by sixteens)
   a.nt_max = nt_max;
   const int rows = nt_max / CG;
   a.stage_bytes = rows * 256;
@@ -733,7 +734,7 @@ int run(const typename Row::Ctx &ctx, const TmemCall &c, Args a, int nt_max, cud
   if (G * CG > MAX_GRID) G = MAX_GRID / CG;
   if (!c.offsets) {
     const int ntt = (int)((c.M + nt_max - 1) / nt_max);
-    const long long U = (long long)ntt * ((c.N + 128 * CG - 1) / (128 * CG)) * (c.K / KU), least = c.min_run_k / KU;
+    const long long U = (long long)ntt * ((c.N + 128 * CG - 1) / (128 * CG)) * (c.K / KU), least = c.min_run_k < KU ? 1 : c.min_run_k / KU;
     if (U >= 1ll << 27) return 0;
     if (U / least < G) G = (int)(U / least > 0 ? U / least : 1);
   }
@@ -795,7 +796,7 @@ int pick(const typename Row::Ctx &ctx, const TmemCall &c, cudaStream_t st) {
   a.offsets = c.offsets, a.pairs = c.pairs, a.topkw = c.topkw, a.factor = c.factor, a.modes = c.modes, a.mode = c.factor ? 0 : MODE_BF16, a.size_m = c.size_m;
   a.E = c.offsets ? c.E : 1, a.M = (int)c.M, a.N = c.N, a.K = c.K;
   static const int k_cg = knob("LIGHT_B200_TMEM_CG", 0), k_nt = knob("LIGHT_B200_TMEM_NT", 0), k_wmin = knob("LIGHT_B200_TMEM_WMIN", 128), k_pair = knob("LIGHT_B200_TMEM_PAIR", 0);
-  a.wmin = k_wmin;
+  a.wmin = k_wmin < 16 ? 16 : k_wmin > 1024 ? 1024 : k_wmin;
   // The token tile: at most 256 (two SMs; less where the weight slots leave less room), all tiles of a matrix alike.  One SM
   // alone takes up to 128, with two accumulators.
   int rows = (SMEM_MAX - fixed_smem<Row, OutT>(a.E)) / (3 * 256) / 16 * 16;
@@ -805,9 +806,9 @@ int pick(const typename Row::Ctx &ctx, const TmemCall &c, cudaStream_t st) {
   // against 40); grouped, 64 tokens per expert on average (64 experts of 2048 x 2048, 64 tokens: 95 against 88 us).
   const bool big = c.offsets ? c.mean_tokens >= (k_pair ? k_pair : 64)
                              : c.M > 128 && (long long)((c.N + 127) / 128) * ((c.M + 127) / 128) * (c.K / KU) >= (k_pair ? k_pair : 32) * sm_count();
-  const int cg = k_cg ? k_cg : big ? 2 : 1;
+  const int cg = (k_cg ? k_cg >= 2 : big) ? 2 : 1;
   int cap = rows * cg;
-  if (k_nt && k_nt < cap) cap = k_nt;
+  if (k_nt && k_nt < cap) cap = k_nt < 16 * cg ? 16 * cg : k_nt / (16 * cg) * (16 * cg);
   int nt = cap;
   if (!c.offsets) {
     const int ntt = (int)((c.M + cap - 1) / cap);
