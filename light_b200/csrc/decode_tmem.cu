@@ -531,19 +531,31 @@ int run(const typename Row::Ctx &ctx, const float *x, float *out, int M, int N, 
 
 }  // namespace
 
-// Where this beats the token tiles (us per call of a chain with a cold L2, tiles / here): Q4_K 28672 x 4096, 32 rows 42.6 / 30.9, 64 rows
-// 67.1 / 36.3; 6144 x 4096 18.6 / 14.7, 23.7 / 17.8; 8192 x 2048 17.3 / 12.9, 16.7 / 15.2; 4096 x 14336 29.4 / 21.8, 40.8 / 27.8.  At 4096 x
-// 4096 they are even (13.6 / 13.9, 17.6 / 17.4) and below the tiles are ahead (4096 x 2048 9.3 / 9.8, 1024 x 4096 9.3 / 10.7): a
-// tile is cut into too many parts.  Q6_K: 4096 x 14336 32.8 / 29.7, 44.5 / 33.7; 2048 x 5632 19.7 / 15.9, but 64 rows 20.7 / 21.8; 2048 x 2048
-// 11.4 / 9.0; 128256 x 4096 186 / 156, 307 / 170.  9 to 16 rows of Q4_K: 28672 x 4096 32.9 / 28.3, 14336 x 4096 21.2 / 19.2, 6144 x 4096 14.5 /
-// 14.2, 4096 x 14336 23.0 / 20.5, but Q6_K 4096 x 14336 28.1 / 28.8.
+// Where this beats the kernels that take the call otherwise (us per call of a chain with a cold L2, those / here).  What it costs beside its
+// blocks is the exchange of cut tiles and some 10 us of start and end, so the rules go by the list of (tile, block) and the runs it is cut into.
+//   Q4_K, 9 to 16 rows: lists of four blocks or more to an SM, which the token tiles have: 4096 x 5120 14.3 / 13.6, 4096 x 14336 23.0 / 20.5, 28672 x 4096
+//     32.8 / 28.1 (even from 20 to 32 Mi weights; K = 1024 loses, 28672 x 1024 9.8 / 11.9).  Shorter ones are the cluster kernel's (K split over a
+//     cluster, no pass over x): 4096 x 4096 8.9 / 12.8, 4096 x 4352 10.8 / 12.9, 3584 x 4864 11.2 / 13.5, 3072 x 5632 10.9 / 13.4, 2048 x 8192 13.0 / 14.3,
+//     unless the matrix is so tall that a tile is cut into four parts at most: 5120 x 3328 14.8 / 12.7, 6144 x 2816 15.7 / 12.2, 8192 x 2048 12.2 / 12.0.
+//   Q4_K, 17 to 32: from 16 Mi weights on: 28672 x 4096 42.6 / 30.9, 6144 x 4096 18.6 / 14.7, 8192 x 2048 16.6 / 12.6, 1024 x 16384 26.6 / 19.1,
+//     4096 x 4096 12.8 / 13.1; below, a tile is cut into too many parts (4096 x 2048 9.3 / 9.8, 1024 x 4096 9.3 / 10.7).
+//   33 to 64, where a part is a chunk more to each warp: not where a tile is cut into more than eight parts of few blocks: Q4_K 2048 x 8192 18.5 / 21.4, 1024 x
+//     20480 24.4 / 31.5, 2048 x 10240 21.3 / 23.5, but 2560 x 6656 20.6 / 18.8, 1536 x 16384 26.9 / 24.5, 28672 x 4096 66.7 / 35.7, 4096 x 14336 40.8 / 27.8.
+//     Q6_K 2048 x 8192 19.0 / 21.4, 2048 x 12288 24.2 / 24.6, but 2560 x 6656 21.9 / 20.4, 2048 x 16384 30.7 / 27.4, 4096 x 14336 44.0 / 33.6, 128256 x
+//     4096 307 / 170 (4096 x 4096 17.1 / 17.6, 8192 x 2048 16.3 / 16.2).
+//   Q6_K, 17 to 32: from 4 Mi on: 2048 x 2048 10.7 / 7.9, 2048 x 5632 19.7 / 15.9, 4096 x 14336 32.4 / 29.1, 128256 x 4096 186 / 156; 9 to 16 rows lose
+//     (4096 x 14336 28.1 / 28.8).
 int gguf_decode_tmem(int type, const float *x, const void *w, float *out, int M, int N, int K, void *ws, size_t ws_bytes, cudaStream_t st) {
   static const int q4_min = knob("LIGHT_B200_DECODE_TMEM_MIN_M", 9), q6_min = q4_min > 17 ? q4_min : 17;
+  const bool q4 = type == LB200_Q4_K;
   const long long size = (long long)N * K;
-  if (M < (type == LB200_Q4_K ? q4_min : q6_min) || M > MAX_NT || K % 256 || !ws || N < 128 || size >> 8 > 1ll << 30 || ((uintptr_t)x & 15)) return 0;
-  if (type == LB200_Q4_K && size >= 16ll << 20 && (N > 4096 || K > 4096) && !((uintptr_t)w & 15)) return run<ExQ4K>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);
-  if (type == LB200_Q6_K && size >= (M > 32 ? 16ll : 4ll) << 20 && !((uintptr_t)w & 3) && (K >> 8) % 2 == 0)
-    return run<ExQ6K>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);
+  if ((!q4 && type != LB200_Q6_K) || M < (q4 ? q4_min : q6_min) || M > MAX_NT || K % 256 || !ws || N < 128 || size >> 8 > 1ll << 30 || ((uintptr_t)x & 15)) return 0;
+  const long long tiles = (N + 127) / 128, U = tiles * (K >> 8), sms = sm_count();
+  if (size < (q4 || M > 32 ? 16ll : 4ll) << 20) return 0;
+  if (q4 && M <= 16 && U < 4 * sms && 4 * tiles < sms) return 0;
+  if (M > 32 && U < (q4 ? 5 : 6) * sms && 8 * tiles < sms) return 0;
+  if (q4 && !((uintptr_t)w & 15)) return run<ExQ4K>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);
+  if (!q4 && !((uintptr_t)w & 3) && (K >> 8) % 2 == 0) return run<ExQ6K>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);
   return 0;
 }
 

@@ -41,3 +41,17 @@ def test_calls_of_different_shapes_in_a_graph(cuda):
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
     assert ops.prefill_status(0) == 0
+
+
+# on both sides of each line of the dispatch: runs of four, five and six blocks to an SM, tiles cut into four and into eight parts
+@pytest.mark.parametrize("dt,N,K", [(ops.Q4_K, 4096, 4096), (ops.Q4_K, 4096, 4864), (ops.Q4_K, 4608, 3840), (ops.Q4_K, 4736, 3584), (ops.Q4_K, 2304, 8192),
+                                     (ops.Q4_K, 2432, 7168), (ops.Q4_K, 1024, 23552), (ops.Q4_K, 1024, 24064), (ops.Q6_K, 2304, 9728), (ops.Q6_K, 2432, 7168),
+                                     (ops.Q6_K, 1024, 28160), (ops.Q6_K, 1024, 28672), (ops.Q6_K, 2048, 2048)])
+def test_both_sides_of_the_dispatch(cuda, dt, N, K):
+    w = ops.QTensor(synth.gaussian_weight(N + K, dt, N, K, device=cuda).reshape(-1), dt, (N, K))
+    W = ops.Dequantize(w).double()
+    for M in (9, 16, 17, 32, 33, 64):
+        x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).to(cuda)
+        want = x.half().double() @ W.t()
+        assert rel_l2(ops.MatMulQ(x, w).cpu().double().numpy(), want.cpu().numpy()) <= (4e-6 if dt == ops.Q4_K else 2.0**-11)
+    assert ops.prefill_status(0) == 0
