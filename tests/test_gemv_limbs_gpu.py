@@ -57,3 +57,10 @@ def test_a_nan_reaches_every_row(cuda, fmt):
     for v in (float("nan"), float("inf")):
         x[0, 700] = v
         assert torch.isnan(ops.MatMulQ(x, w)).all()
+
+
+# eight warps with one block of k, sixteen beyond; one row tile to an SM, two, and more (of 148: 2368 and 4736 rows)
+@pytest.mark.parametrize("n", [2368, 2384, 4736, 4752])
+@pytest.mark.parametrize("k", [256, 512, 4096, 4352])
+def test_one_row_int4_both_sides_of_the_wide_cta(cuda, n, k):
+    test_one_row_int4(cuda, n, k, 128, "normal")
