@@ -267,8 +267,9 @@ int moe_clear_unrouted(const int64_t *pairs, const int64_t *ids, uint32_t *bits,
 
 // ------------------------------------------------------------------------------------ Q6_K rows that start on any even byte
 //
-// An odd number of 210-byte blocks per row: the tensor-core kernels would round both operands to 11 bits, and these rows have always had
-// f32 products, as below 256 pairs.  What bounds moe_gemm_kernel is the load unit: a warp to one weight row reads eight activation rows
+// An odd number of 210-byte blocks per row: the tensor-memory kernel would round both operands to 11 bits, where this call multiplies f32 by
+// f32 (as below 256 pairs it does at any K).  These are the products one by one, for calls without scratch; the limbs further down
+// are what calls with scratch have.  What bounds moe_gemm_kernel is the load unit: a warp to one weight row reads eight activation rows
 // for every eight weights, and the weights a byte at a time.  Here a warp owns NC rows of one expert and MT of its tokens: an
 // activation is loaded once for NC weights, a weight once for MT tokens, in 16-bit pieces.  Lanes split K, and the NC x MT sums end
 // in a reduce-scatter over the warp (31 shuffles for 32 sums, not 160).  616 pairs over 128 experts of 2048 x 768: 780 -> 245 us;
@@ -376,8 +377,8 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) q6k_rows_kernel(const float
 // the operand takes some 900 of the 1665 instructions per 16 rows, block and 16 tokens, and issue is what bounds this kernel
 // (63 % of the slots, the tensor pipe 24 %).
 //   616 pairs over 128 experts of 2048 x 768:  247 -> 117 us;   2048 rows of 4096 x 14080:  16.2 -> 5.4 ms;   65 rows of 4096 x 2816:
-//   110 -> 68 us.  Blocks are added with their rounding errors kept (5 % of the time): 2.1e-8 to 3.6e-8 off against 64 bits where the f32
-//   sums were 5.3e-8 to 1.3e-7 off (K = 256 to 14080; without, 1.1e-7 at 11008).
+//   110 -> 68 us.  Blocks are added with their rounding errors kept (5 % of the time): 2.5e-8 off against 64 bits with normal inputs where the
+//   f32 products are 8.1e-8 to 1.59e-7 off (K = 256 to 14080; without, 1.1e-7 at 11008).
 // Tried: limbs of eight bits and the integer MMAs (m16n8k32), 194 us and 19.5 ms: they run at a fraction of the f16 rate here; limbs
 // straight from L2, 152 us and 8.8 ms; 32 rows to a warp and half the warps, 115 us and 5.5 ms.
 // Tokens with infinities or NaN (whose limbs mean nothing; their power of two is NaN) are multiplied again in f32.

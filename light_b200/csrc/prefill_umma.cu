@@ -1324,7 +1324,7 @@ int moe_umma(const lb200_moe_args *a, int kind, const float *w_scale, int bR, in
     if (a->K % 256) return 0;
     if (a->dtype == LB200_Q4_K)
       rc = moe_launch<Q4KRow, false, float, float>(a, GgufCtx{(const uint8_t *)a->weights}, ws, wsb, st);
-    else if (a->dtype == LB200_Q6_K && (a->K >> 8) % 2 == 0)  // (others keep their f32 products, as in gguf_prefill)
+    else if (a->dtype == LB200_Q6_K && (a->K >> 8) % 2 == 0)  // (others: q6k_limbs or f32 products, as in gguf_prefill)
       rc = moe_launch<Q6KRow, false, float, float>(a, GgufCtx{(const uint8_t *)a->weights}, ws, wsb, st);
     else if (a->dtype == LB200_Q8_0 && !((uintptr_t)a->weights & 15))
       rc = moe_launch<Q80Row, false, float, float>(a, GgufCtx{(const uint8_t *)a->weights}, ws, wsb, st);

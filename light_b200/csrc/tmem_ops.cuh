@@ -14,7 +14,7 @@ namespace {
 using namespace umma;
 
 constexpr int MAX_GRID = 160;
-constexpr int SMEM_MAX = 227 * 1024 - 1024;   // dynamic; the static part (prefix tables, flags) is accounted below
+constexpr int SMEM_MAX = 227 * 1024 - 1024;   // dynamic; 1 KB is left for a kernel's static part, and one with more takes it off
 
 // Which parts of the partial tiles are written: a flag per part (the kernels say which) holds the tag of the launch that wrote the
 // part last.  A launch's tag is the epoch it finds, plus one; the last of its CTAs to have read the epoch raises it.  So no flag of an

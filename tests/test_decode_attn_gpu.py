@@ -135,7 +135,7 @@ def test_limits_are_reported_not_asserted(cuda):
 
 # ---- the tensor-core kernel of bf16 caches: block edges (16 keys a warp, 64 a CTA), one key, head groups on both sides of
 # eight, a window that starts inside a block, and a row at pos that held NaN before the append.  Against f64; the bf16 output's
-# rounding (2^-9 at most) is what remains.
+# rounding (2^-8 at most) is what remains.
 @pytest.mark.parametrize("B,NH,KH,D,n,win", [(1, 1, 1, 64, 1, 0), (2, 8, 1, 128, 16, 0), (1, 9, 1, 64, 17, 0), (3, 16, 1, 128, 65, 0), (2, 4, 4, 64, 128, 50),
                                              (1, 24, 8, 128, 1000, 300)])
 def test_tensor_core_kernel(cuda, B, NH, KH, D, n, win):

@@ -3,7 +3,7 @@ than a tile, ragged row counts (with and without whole 16-byte output rows), the
 tiles, grouped launches with empty experts and single tokens, and launches on two streams.
 
 Bounds: operands are rounded once each to f16 (2^-12 relative on average over a product: 1e-3 with room, the bound of the other
-tensor-core paths) or are the bf16 values themselves, when the bf16 output's rounding (2^-9 at most) is what remains."""
+tensor-core paths) or are the bf16 values themselves, when the bf16 output's rounding (2^-8 at most) is what remains."""
 import pytest
 import torch
 
@@ -73,7 +73,7 @@ def test_grouped_q6_k_rows_at_odd_offsets(cuda):
 @pytest.mark.parametrize("M,N,K", [(17, 4096, 4096), (33, 8196, 2048), (48, 732, 14336), (64, 40964, 256)])
 def test_narrow_int4(cuda, M, N, K):
     """17 to 64 bf16 rows of a 4-bit matrix of 10 * 2^20 weights or more: f16 operands (2^-12 each on average), then the bf16 output's
-    rounding, 2^-9 of a value at most."""
+    rounding, 2^-8 of a value at most."""
     g = torch.Generator(device=cuda).manual_seed(N)
     w = ops.Int4(torch.randint(-2**31, 2**31, (N, K // 8), generator=g, device=cuda, dtype=torch.int32), torch.rand(N, K // 64, generator=g, device=cuda) * 0.02,
                  torch.randint(0, 31, (N, K // 64), generator=g, device=cuda).float() / 2, 64)

@@ -2,7 +2,7 @@
 format.
 
 Bounds: a product of f32 values summed in f32 over K terms is off by at most about K / 2 * 2^-24 of the sum of magnitudes and by
-sqrt(K) * 2^-24 on average, below 1e-5 here; operands rounded to f16 give 2^-12 each, 3e-4 on the result."""
+sqrt(K) * 2^-24 on average, below 1e-5 here; operands rounded to f16 give 2^-11 each at most, 3e-4 on the result."""
 import pytest
 import torch
 
@@ -36,7 +36,7 @@ def test_grouped_q6_k_with_an_odd_number_of_blocks_per_row(cuda, M):
 @pytest.mark.parametrize("G", [64, 256])
 @pytest.mark.parametrize("scale", [1e-6, 3e4])
 def test_int4_rows_beyond_f16(cuda, G, scale):
-    """17 to 64 bf16 rows of a 4-bit matrix whose groups are not 128: x is multiplied as bf16, whatever its range.  bf16 weights (2^-9 of a
+    """17 to 64 bf16 rows of a 4-bit matrix whose groups are not 128: x is multiplied as bf16, whatever its range.  bf16 weights (2^-8 of a
     weight at most, 1.1e-3 on average) and the bf16 output's rounding (the same) remain."""
     M, N, K = 33, 4096, 4096
     g = torch.Generator(device=cuda).manual_seed(G)
