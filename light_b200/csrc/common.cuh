@@ -165,6 +165,8 @@ struct TmemCall {
   const float *topkw;
   const float *factor;      // FP8, grouped: x16 holds f16 rows over a power of two each, which this multiplies by again (bf16 output)
   const int32_t *modes;     // FP8, grouped, a word per expert (null: no matter): with factor the experts without MODE_BF16 are this call's, else those with it
+  const uint4 *tokens;      // with factor and modes: the bf16 tokens themselves; this call copies the rows of the other experts from there to x16, for the next
+  int topk, row_per_pair;
   long long size_m;
   int E;
   double mean_tokens;       // tokens per matrix (grouped: pairs / experts)

@@ -66,6 +66,9 @@ struct Args {
   const float *factor;      // f16 tokens over a power of two each: token row i is to be multiplied by factor[i] (null: as they are)
   const int32_t *modes;     // see TmemCall
   int mode;                 // with modes: of the experts that are this launch's
+  const uint4 *tokens;      // with factor: see TmemCall
+  uint4 *x16;
+  int topk, row_per_pair;
   long long size_m;
   int E, M, N, K;
   int nt_max;               // most tokens of a tile
@@ -161,6 +164,24 @@ struct Work {
   }
 };
 
+// The rows of experts that are left to the bf16 launch, as they are: nothing in this launch makes use of them.
+__device__ __noinline__ void copy_rows(const Args &a) {
+  const int lane = threadIdx.x & 31, pieces = a.K >> 3;
+  for (int e = 0; e < a.E; e += 32) {
+    unsigned left = __ballot_sync(0xffffffffu, e + lane < a.E && (a.modes[min(e + lane, a.E - 1)] & MODE_BF16));
+    while (left) {
+      const int f = e + __ffs(left) - 1;
+      left &= left - 1;
+      for (int i = a.offsets[f] + (int)blockIdx.x; i < a.offsets[f + 1]; i += gridDim.x) {
+        const long long p = a.pairs[i];
+        const bool ok = p >= 0 && p < a.size_m;
+        const uint4 *src = a.tokens + (ok ? (size_t)(a.row_per_pair ? p : p / a.topk) * pieces : 0);
+        for (int k = threadIdx.x; k < pieces; k += THREADS) a.x16[(size_t)i * pieces + k] = ok ? __ldg(src + k) : make_uint4(0, 0, 0, 0);
+      }
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------ kernel
 template <typename OutT>
 constexpr uint32_t STRIP = 32 * 128 * sizeof(OutT);  // 32 tokens of 128 output columns
@@ -210,12 +231,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   // (every CTA of this grid is resident once all have come by here: the next kernel's wait for room, and for its operands)
   pdl_launch_dependents();
   if (a.offsets) pdl_wait();
+  [[maybe_unused]] int others = 0;
   if constexpr (HasModes<Row>::value) {
     bool any = false;
     for (int e = threadIdx.x; e < a.E; e += THREADS) {
       const int cnt = wk.count_of(e), m = a.modes ? a.modes[e] : a.mode;
       counts[e] = (m & MODE_BF16) == a.mode ? cnt | (m & MODE_APART) : 0;
-      any |= cnt > 0 && (m & MODE_BF16) == a.mode;
+      any |= cnt > 0 && (m & MODE_BF16) == a.mode, others |= m & MODE_BF16;
     }
     if (a.modes && a.mode && !__syncthreads_or(any)) return;  // (mostly: no expert is left to the bf16 launch)
   }
@@ -226,7 +248,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
     preW[e + 1] = ntt * wk.nrt * nb * wk.weight(nt);
   }
   if (warp == MMA_WARP) alloc512<CG>(smem_u32(&tmem_sh));
-  __syncthreads();
+  if constexpr (Unscales<Row>::value) others = __syncthreads_or(others);
+  else __syncthreads();
+  if (Unscales<Row>::value && others) copy_rows(a);
   if (warp == 0) {  // inclusive prefix sums, 32 experts at a time
     int ct = 0, cw = 0;
     for (int e0 = 0; e0 < a.E; e0 += 32) {
@@ -794,6 +818,7 @@ int pick(const typename Row::Ctx &ctx, const TmemCall &c, cudaStream_t st) {
   if (c.K % KU || c.E > MAX_E || (c.offsets && (c.M / 16 + c.E) * ((c.N + 127) / 128) * (c.K / KU) >= 1ll << 31)) return 0;
   Args a = {};
   a.offsets = c.offsets, a.pairs = c.pairs, a.topkw = c.topkw, a.factor = c.factor, a.modes = c.modes, a.mode = c.factor ? 0 : MODE_BF16, a.size_m = c.size_m;
+  a.tokens = c.tokens, a.x16 = (uint4 *)const_cast<void *>(c.x16), a.topk = c.topk, a.row_per_pair = c.row_per_pair;
   a.E = c.offsets ? c.E : 1, a.M = (int)c.M, a.N = c.N, a.K = c.K;
   static const int k_cg = knob("LIGHT_B200_TMEM_CG", 0), k_nt = knob("LIGHT_B200_TMEM_NT", 0), k_wmin = knob("LIGHT_B200_TMEM_WMIN", 128), k_pair = knob("LIGHT_B200_TMEM_PAIR", 0);
   a.wmin = k_wmin < 16 ? 16 : k_wmin > 1024 ? 1024 : k_wmin;

@@ -2017,8 +2017,8 @@ int int4_gemv_fast(const void *x, const uint32_t *codes, const float *s, const f
   // activations, which is most of its work when a block serves one tile, and for as many as two tiles together: 3584 x 18944 18.3 -> 12.9 us, 4736 x
   // 8192 11.9 -> 8.7, 4096 x 4096 6.6 -> 5.1.  With few blocks it still gains, as most warps of either kind have none and the second tile
   // costs no second CTA: 4736 x 2048 4.0 -> 3.6, 2368 x 2048 2.65 -> 2.5, 4608 x 1024 2.4 -> 2.25, 3584 x 512 2.15 -> 2.05; with one block, the only busy
-  // warp has both tiles: 4096 x 256 1.9 -> 2.05.
-  const bool wide = tiles <= 2 * g_sms && K > 256;
+  // warp would have both tiles: 4096 x 256 1.88 -> 2.05, but one tile 2048 x 256 1.88 -> 1.80.
+  const bool wide = tiles <= (K > 256 ? 2 : 1) * g_sms;
   const int warps = wide ? I4_WIDE : WARPS, most = wide ? g_sms : g_sms * g_waves;
   const unsigned grid = (unsigned)(tiles < most ? tiles : most);
   const size_t dyn = (size_t)warps * I4_STAGES * I4_TILE_BYTES;

@@ -1187,10 +1187,9 @@ __global__ void __launch_bounds__(SCALED_THREADS) gather_rows_scaled_kernel(cons
   auto two = [&](uint32_t w) {
     const float x = __uint_as_float(w << 16), y = __uint_as_float(w & 0xFFFF0000u);
     if (finite) {
-      const __half2 h = __floats2half2_rn(x * f, y * f);
-      const float2 back = __half22float2(h);
-      lost += (back.x * power != x) + (back.y * power != y);
-      return *reinterpret_cast<const uint32_t *>(&h);
+      const float xs = x * f, ys = y * f;  // (the eight bits of 2^-17 and more fit above f16's last place, and so do bf16's own subnormals)
+      lost += (x != 0.f && fabsf(xs) < 0x1p-17f) + (y != 0.f && fabsf(ys) < 0x1p-17f);
+      return pack_h2(xs, ys);
     }
     auto keep = [](float v) { return isfinite(v) && v != 0.f ? copysignf(1.f, v) : v; };
     return pack_h2(keep(x), keep(y));
@@ -1220,25 +1219,9 @@ __global__ void __launch_bounds__(SCALED_THREADS) gather_rows_scaled_kernel(cons
   if (lo < E && offsets[lo] <= (int)i) atomicOr(modes + lo, mode);
 }
 
-// The rows of experts with bf16 operands once more, as they are.
-__global__ void __launch_bounds__(SCALED_THREADS) gather_rows_again_kernel(const uint4 *__restrict__ in, const int64_t *__restrict__ pairs, uint4 *__restrict__ dst, int K,
-                                                                          int topk, int row_per_pair, long long size_m, const int32_t *__restrict__ offsets,
-                                                                          const int32_t *__restrict__ modes) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int e = blockIdx.x, n = K >> 3;
-  if (!(modes[e] & MODE_BF16)) return;
-  for (int i = offsets[e] + (int)blockIdx.y; i < offsets[e + 1]; i += gridDim.y) {
-    const long long p = pairs[i];
-    const bool ok = p >= 0 && p < size_m;
-    const uint4 *src = in + (ok ? (size_t)(row_per_pair ? p : p / topk) * n : 0);
-    for (int k = threadIdx.x; k < n; k += SCALED_THREADS) dst[(size_t)i * n + k] = ok ? __ldg(src + k) : make_uint4(0, 0, 0, 0);
-  }
-}
-
 // bf16 tokens times FP8 weights in whole 128 x 128 blocks, grouped: f16 operands for the experts for which they hold what bf16 does, then
-// bf16 operands for the rest, mostly none: then the two launches take 13 us of a sparse block of 8 tokens (504 -> 517).  1: took the call, 0: not covered,
-// other: error.
+// bf16 operands for the rest, mostly none: the looks at tokens and scales and the empty launch take 11 us of a sparse block of 8 tokens (515 ->
+// 526), 40 of one of 4096 (5030 -> 5071).  1: took the call, 0: not covered, other: error.
 int moe_fp8_f16(const lb200_moe_args *a, const float *w_scale, int bR, int bC, void *ws, size_t ws_bytes, void *sync, cudaStream_t st) {
   const size_t x_bytes = ((size_t)a->M * a->K * 2 + 1023) & ~(size_t)1023, f_bytes = ((size_t)a->M * 4 + 1023) & ~(size_t)1023;
   const long long looks = (long long)a->E * ((a->N / bR + SCALED_WARPS - 1) / SCALED_WARPS);
@@ -1250,13 +1233,11 @@ int moe_fp8_f16(const lb200_moe_args *a, const float *w_scale, int bR, int bC, v
                a->topk, a->row_per_pair, (long long)a->size_m, w_scale, a->N / bR, a->K / bC, (const int32_t *)a->offsets, a->counts, a->E);
   if (int rc = launched("moe: gather rows")) return rc;
   TmemCall c = tmem_call<Fp8Row>(Fp8Ctx{(const uint8_t *)a->weights, w_scale, bR, bC});
-  c.x16 = ws, c.out_bf16 = true, c.out = a->out, c.M = a->M, c.N = a->N, c.K = a->K, c.factor = factor, c.modes = a->counts;
+  c.x16 = ws, c.out_bf16 = true, c.out = a->out, c.M = a->M, c.N = a->N, c.K = a->K, c.factor = factor, c.modes = a->counts, c.tokens = (const uint4 *)a->input, c.topk = a->topk,
+  c.row_per_pair = a->row_per_pair;
   c.offsets = a->offsets, c.pairs = a->sorted_pairs, c.topkw = a->topk_weights, c.size_m = a->size_m, c.E = a->E;
   c.mean_tokens = (double)a->M / a->E, c.min_run_k = tmem_min_run(), c.parts = (char *)ws + x_bytes + f_bytes, c.parts_bytes = ws_bytes - x_bytes - f_bytes, c.sync = sync;
   if (int took = gemm_tmem(c, st); took != 1) return took;
-  launch_early(gather_rows_again_kernel, dim3((unsigned)a->E, 8), dim3(SCALED_THREADS), st, (const uint4 *)a->input, a->sorted_pairs, (uint4 *)ws, a->K, a->topk, a->row_per_pair,
-               (long long)a->size_m, (const int32_t *)a->offsets, (const int32_t *)a->counts);
-  if (int rc = launched("moe: gather rows again")) return rc;
   c.factor = nullptr, c.bf16 = true;
   const int took = gemm_tmem(c, st);
   return took ? took : fail(LB200_E_SHAPE, "light_b200: moe: no bf16 kernel behind the f16 one");
