@@ -100,7 +100,8 @@ def test_infinities_and_nan(cuda, T):
 
 @pytest.mark.parametrize("T", [20, 300])   # pairs in memory of the call, in the workspace
 @pytest.mark.parametrize("kind", ["scales", "tokens", "both", "neither"])
-def test_operands_of_far_apart_sizes(cuda, T, kind):
+@pytest.mark.parametrize("per_pair", [False, True])
+def test_operands_of_far_apart_sizes(cuda, T, kind, per_pair):
     """What is small beside another block of the row, or another element of the token, counts where the large one meets zeros.  Even tokens
     go to experts 0 and 1, odd ones to 2 and 1; expert 0 has the scales, even tokens have the large elements."""
     E, topk, N, K = 3, 2, 256, 512
@@ -117,7 +118,8 @@ def test_operands_of_far_apart_sizes(cuda, T, kind):
     even = torch.arange(T) % 2 == 0
     ids = torch.stack([torch.where(even, 0, 2), torch.ones(T, dtype=torch.int64)], 1).to(cuda)
     wt = torch.rand(T * topk, generator=torch.Generator().manual_seed(7)).to(cuda)
-    y = _run(x, codes, scale, ids, wt, E, N, K, 128, 128).double().reshape(T, topk, N)
+    rows = x.repeat_interleave(topk, 0) if per_pair else x
+    y = _run(rows, codes, scale, ids, wt, E, N, K, 128, 128).double().reshape(T, topk, N)
     want = torch.einsum("tk,tsnk->tsn", x.double(), w[ids]) * wt.double().reshape(T, topk, 1)
     bf16 = {"scales": (0,), "tokens": (0, 1), "both": (0, 1), "neither": ()}[kind]
     for e in range(E):

@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from helpers import rel_l2
-from light_b200 import ops, synth
+from light_b200 import _lib, ops, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -189,3 +189,20 @@ def test_q6_k_in_limbs_in_a_graph(cuda):
     x.copy_(2 * x)
     graph.replay()
     assert torch.equal(y, 2 * want)
+
+
+@pytest.mark.parametrize("short", [None, 1])   # no scratch, too little of it
+def test_q6_k_without_scratch(cuda, short):
+    """f32 products: 8.8e-8 off at this K, whatever the sizes of a block's activations."""
+    M, N, K = 100, 64, 768
+    w = ops.QTensor(_zero_at(synth.gaussian_weight(4, ops.Q6_K, N, K, device=cuda), N, K, 9), ops.Q6_K, (N, K))
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(5)).to(cuda)
+    x[:, 9::256] = 1e6
+    L = _lib.lib()
+    need = int(L.light_b200_q6k_scratch_bytes(ops.Q6_K, w.data.data_ptr(), M, K, 0))
+    own = None if short is None else torch.empty(need - short, dtype=torch.uint8, device=cuda)
+    y = torch.empty(M, N, device=cuda)
+    _lib.check(L.light_b200_matmul_q_scratch(ops.Q6_K, x.data_ptr(), w.data.data_ptr(), y.data_ptr(), M, N, K, None if own is None else own.data_ptr(),
+                                             0 if own is None else own.numel(), 0, torch.cuda.current_stream().cuda_stream))
+    want = x.double() @ ops.Dequantize(w).double().t()
+    assert rel_l2(y.cpu().double().numpy(), want.cpu().numpy()) <= 2.0**-23
