@@ -165,10 +165,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
   // complete, are read out; p_empty: the minimums' sums are; drained: nothing of the MMA warp's is in flight.
   const uint32_t full = sBar, empty = full + 16, d_full = empty + 16, d_empty = d_full + 32, p_empty = d_empty + 32, w_full = p_empty + 8,
                  t_full = w_full + 8 * EXPANDERS, t_empty = t_full + 8 * NBS, drained = t_empty + 8 * NBS;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = same((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int nb = a.K >> 8, G = gridDim.x, cta = blockIdx.x, U = (a.N + 127) / 128 * nb;
   auto bound = [&](int j) { return (int)((long long)U * j / G); };
-  const int v0 = bound(cta), n = bound(cta + 1) - v0;  // this CTA's run of (tile, block)
+  const int v0 = same(bound(cta)), n = same(bound(cta + 1)) - v0;  // this CTA's run of (tile, block)
 
   if (threadIdx.x == 0) {
     prefetch_tmap(&maps.x);
@@ -188,20 +188,21 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_sh, bmask = (uint32_t)a.bufs - 1, cols = 2 * MAX_NT / a.bufs;
+  const uint32_t tmem = same(tmem_sh), bmask = (uint32_t)a.bufs - 1;
   const int blog = a.bufs == 4 ? 2 : 1;
+  const uint32_t cols = 2 * MAX_NT >> blog;
   volatile int *abort = &abort_flag;
 
   if (warp >= TMA_WARP && warp < MMA_WARP) {
-    if (elect_one()) {
-      pdl_wait();  // the tokens are the kernel before's
-      const int half = warp - TMA_WARP;
-      const uint32_t bytes = (uint32_t)a.nt * (Row::MINS && half ? 320u : 256u), tile = (uint32_t)a.nt * 128u;
-      int s = 0, par = 1, kb = v0 % nb;
-      bool wrapped = false;
-      for (int i = 0; i < n; i++) {
-        const uint32_t bar = t_full + 8 * s, dst = sB + s * a.stage_bytes;
-        if (wrapped && !mbar_sleep_wait(t_empty + 8 * s, par) && !mbar_wait(t_empty + 8 * s, par, abort)) break;
+    pdl_wait();  // the tokens are the kernel before's
+    const int half = warp - TMA_WARP;
+    const uint32_t bytes = (uint32_t)a.nt * (Row::MINS && half ? 320u : 256u), tile = (uint32_t)a.nt * 128u;
+    int s = 0, par = 1, kb = same(v0 % nb);
+    bool wrapped = false;
+    for (int i = 0; i < n; i++) {
+      const uint32_t bar = t_full + 8 * s, dst = sB + s * a.stage_bytes;
+      if (wrapped && !warp_wait(t_empty + 8 * s, par, abort)) break;
+      if (elect_one()) {
         mbar_arrive_expect_tx(bar, bytes);
         tma_load_2d(dst + 2 * half * tile, &maps.x, bar, kb * 256 + half * 128, 0);
         tma_load_2d(dst + (2 * half + 1) * tile, &maps.x, bar, kb * 256 + half * 128 + 64, 0);
@@ -209,14 +210,15 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
           tma_load_2d(dst + 4 * tile, &maps.sums, bar, kb * 32, 0);
           tma_load_2d(dst + 4 * tile + tile / 4, &maps.sums, bar, kb * 32 + 16, 0);
         }
-        if (++kb == nb) kb = 0;
-        if (++s == a.stages) s = 0, par ^= 1, wrapped = true;
       }
+      __syncwarp();
+      if (++kb == nb) kb = 0;
+      if (++s == a.stages) s = 0, par ^= 1, wrapped = true;
     }
   } else if (warp == MMA_WARP) {
     const uint32_t idesc = idesc_f16(128, 16, false) + ((uint32_t)((a.nt - 16) >> 3) << 17);
     const uint32_t tile = (uint32_t)a.nt * 128u;
-    int t = 0, tpar = 0, kb = v0 % nb, seg = 0;
+    int t = 0, tpar = 0, kb = same(v0 % nb), seg = 0;
     bool first = true;                  // of the tile's blocks in this run
     bool ready = false, room = false;   // the next block's barriers and buffer, looked at before this one's MMAs are issued
     for (int i = 0; i < n; i++) {
@@ -260,7 +262,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
     const int set = warp >> 2, quad = warp & 3, half = set & 1;
     const uint32_t slot = sRaw + (uint32_t)warp * Row::SLOT, copied = w_full + 8 * warp, lanes = (uint32_t)(quad * 32) << 16;
     Row rowx(ctx);
-    int i = set >> 1, kb = (v0 + i) % nb, tile = (v0 + i) / nb;  // this warp's next block: number in the run, in its rows, and the tile
+    int i = set >> 1, kb = same((v0 + i) % nb), tile = same((v0 + i) / nb);  // this warp's next block: number in the run, in its rows, and the tile
     [[maybe_unused]] int y = 0;
     [[maybe_unused]] const uint8_t *src = nullptr;
     [[maybe_unused]] int rows = 0;

@@ -189,7 +189,7 @@ template <typename OutT>
 constexpr int STRIPS = 2 * STRIP<OutT>;
 
 struct Maps {
-  CUtensorMap x[MAX_ROWS / 16], w[2];  // tokens, by the rows of a box (16, 32, ..); the weight rows, per box of the format
+  CUtensorMap x[MAX_ROWS / 16], w[3];  // tokens, by the rows of a box (16, 32, ..); the weight rows, per box of the format
   CUtensorMap out;                     // one matrix: 16 tokens of 32 output columns
 };
 
@@ -210,8 +210,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
                  t_full = w_full + 8 * EXPANDERS, t_empty = t_full + 8 * NBS, tagged = t_empty + 8 * NBS;
   int *preW = reinterpret_cast<int *>(gen + (sBar - base) + BAR_BYTES), *preT = preW + a.E + 1;
   [[maybe_unused]] int *const counts = preT + a.E + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = CG == 2 ? (int)cluster_ctarank() : 0;
+  const int warp = same((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int rank = CG == 2 ? same((int)cluster_ctarank()) : 0;
   const Work<CG, HasModes<Row>::value> wk{a, preT, preW, counts, a.K / KU, (a.N + 128 * CG - 1) / (128 * CG)};
   const int nb = wk.nb;
   const int G = gridDim.x / CG, cta = blockIdx.x / CG;
@@ -220,6 +220,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
     if (!a.offsets) prefetch_tmap(&maps.x[a.nt_max / CG / 16 - 1]);
     if constexpr (Row::BOXES > 0) prefetch_tmap(&maps.w[0]);
     if constexpr (Row::BOXES > 1) prefetch_tmap(&maps.w[1]);
+    if constexpr (Row::BOXES > 2) prefetch_tmap(&maps.w[2]);
     abort_flag = 0;
     for (int i = 0; i < NAS; i++) mbar_init(full + 8 * i, CG == 2 && rank == 0 ? 5 : 4), mbar_init(empty + 8 * i, 1);
     for (int i = 0; i < a.nbs; i++) mbar_init(t_full + 8 * i, 2), mbar_init(t_empty + 8 * i, 1);
@@ -271,43 +272,47 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
   __syncthreads();
   if constexpr (CG == 2) cluster_sync();  // the peer's barriers exist before anything arrives on them
   tc_fence_after();
-  const uint32_t tmem = tmem_sh;
+  const uint32_t tmem = same(tmem_sh);
   volatile int *abort = &abort_flag;
   // This CTA (pair)'s run: n units from unit v0 of tile tf on, then tile tf + stride, ...  Where there are plenty of tiles a grouped
   // launch deals them out in turn instead: the tiles in flight are then neighbours, of a few experts whose tokens
   // stay in L2.  (Contiguous runs, one far from the other, read the tokens of 74 experts at once, more than L2 holds, and
   // from HBM again for every row tile.)
-  const int total = preT[a.E];
+  const int total = same(preT[a.E]);
   const bool dealt = a.offsets && total >= 16 * G;
-  const int pos0 = dealt ? cta * nb : wk.bound(cta, G), tf = pos0 / nb, v0 = pos0 - tf * nb, stride = dealt ? G : 1;
-  const int n = dealt ? (total > cta ? (total - 1 - cta) / G + 1 : 0) * nb : wk.bound(cta + 1, G) - pos0;
+  const int pos0 = dealt ? cta * nb : same(wk.bound(cta, G)), tf = same(pos0 / nb), v0 = pos0 - tf * nb, stride = dealt ? G : 1;
+  const int n = dealt ? same(total > cta ? (total - 1 - cta) / G + 1 : 0) * nb : same(wk.bound(cta + 1, G)) - pos0;
   const int v1 = v0 + n;
 
   if (warp >= TMA_WARP && warp < MMA_WARP) {
-    if (elect_one()) {
-      pdl_wait();  // the tokens may be the kernel before's; the weights are not
-      const int half = warp - TMA_WARP;
-      const uint32_t first = sB + half * (a.stage_bytes / 2);
-      uint32_t dst = first;
-      int bt = 0, par = 1;
-      bool wrapped = false;
-      auto W = wk.walk(tf);
-      for (int v = v0; v < v1 && !*abort; wk.next(W, stride)) {
-        const int u0 = v % nb, u1 = min(nb, u0 + (v1 - v));
-        const Tile T = wk.tile(W);
-        const int rows = T.nt / CG, y = T.m0 + rank * rows;
-        const CUtensorMap *const map = &maps.x[rows / 16 - 1];
-        int x = u0 * 128 + half * 64;
-        for (int u = u0; u < u1; u++, x += 128) {
-          const uint32_t bar = t_full + 8 * bt;
-          if (wrapped && !mbar_sleep_wait(t_empty + 8 * bt, par) && !mbar_wait(t_empty + 8 * bt, par, abort)) break;
+    pdl_wait();  // the tokens may be the kernel before's; the weights are not
+    const int half = warp - TMA_WARP;
+    const uint32_t first = sB + half * (a.stage_bytes / 2);
+    uint32_t dst = first;
+    int bt = 0, par = 1;
+    bool wrapped = false, ok = true;
+    auto W = wk.walk(tf);
+    for (int v = v0; v < v1 && ok; wk.next(W, stride)) {
+      const int u0 = same(v % nb), u1 = min(nb, u0 + (v1 - v));
+      const Tile T = wk.tile(W);
+      const int rows = same(T.nt / CG), y = same(T.m0) + rank * rows;
+      const CUtensorMap *const map = &maps.x[rows / 16 - 1];
+      int x = u0 * 128 + half * 64;
+      for (int u = u0; u < u1; u++, x += 128) {
+        const uint32_t bar = t_full + 8 * bt;
+        if (wrapped && !warp_wait(t_empty + 8 * bt, par, abort)) {
+          ok = false;
+          break;
+        }
+        if (elect_one()) {
           mbar_arrive_expect_tx(bar, (uint32_t)rows * 128u);
           tma_load_2d(dst, map, bar, x, y);
-          dst += a.stage_bytes;
-          if (++bt == a.nbs) bt = 0, par ^= 1, wrapped = true, dst = first;
         }
-        v += u1 - u0;
+        __syncwarp();
+        dst += a.stage_bytes;
+        if (++bt == a.nbs) bt = 0, par ^= 1, wrapped = true, dst = first;
       }
+      v += u1 - u0;
     }
   } else if (warp == MMA_WARP) {
     // The whole warp runs the loop and one elected lane issues.  A pass is a chain of some 60 instructions that share their
@@ -315,20 +320,19 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
     // stood at half its rate.  Hence 128 k to a stage, and the look at the next stage's barriers issued
     // before this stage's MMAs.
     const bool leader = elect_one();
-    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
     int s = 0, par = 0, bt = 0, bpar = 0, seg = 0;
     bool ok = true, wide_before = false;
     auto W = wk.walk(tf);
     for (int v = v0; v < v1 && ok; seg++, wk.next(W, stride)) {
-      const int u0 = v % nb, u1 = min(nb, u0 + (v1 - v));
-      const int nt = __shfl_sync(0xffffffffu, W.nt, 0);
+      const int u0 = same(v % nb), u1 = min(nb, u0 + (v1 - v));
+      const int nt = same(W.nt);
       const bool wide = nt > 128;
       if (rank == 0) {  // the accumulators this segment overwrites must have been read out
         if (seg >= 2 && !warp_wait(d_empty + 8 * (seg & 1), ((seg - 2) >> 1) & 1, abort)) break;
         if (seg >= 1 && (wide || wide_before) && !warp_wait(d_empty + 8 * ((seg - 1) & 1), ((seg - 1) >> 1) & 1, abort)) break;
       }
       wide_before = wide;
-      const uint32_t d = tm + (wide ? 0 : 128 * (seg & 1));
+      const uint32_t d = tmem + (wide ? 0 : 128 * (seg & 1));
       const uint32_t idesc = idesc_f16(128 * CG, 16, BF16) + ((uint32_t)((nt - 16) >> 3) << 17);
       const int stages = u1 - u0;
       uint32_t acc = 0;
@@ -340,7 +344,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
         }
         tc_fence_after();
         const uint64_t b0 = smem_desc_sw128(sB + bt * a.stage_bytes), b1 = b0 + (uint64_t)(a.stage_bytes >> 5);
-        const uint32_t am = tm + A_COL + 64 * s, done = empty + 8 * s, fwd = full + 8 * s, tdone = t_empty + 8 * bt;
+        const uint32_t am = tmem + A_COL + 64 * s, done = empty + 8 * s, fwd = full + 8 * s, tdone = t_empty + 8 * bt;
         if (++s == NAS) s = 0, par ^= 1;
         if (++bt == a.nbs) bt = 0, bpar ^= 1;
         ready = mbar_test_wait(full + 8 * s, par), tokens = mbar_test_wait(t_full + 8 * bt, bpar);
@@ -365,11 +369,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
       __syncwarp();
       v += u1 - u0;
     }
-    if (rank == 0) {  // no MMA may be in flight when tensor memory is given back, whichever way the loop ended
-      if (leader) commit<CG>(drained);
-      __syncwarp();
-      for (int i = 0; i < (1 << 16) && !__all_sync(0xffffffffu, mbar_test_wait(drained, 0)); i++) {
-      }
+    // No MMA may be in flight when tensor memory is given back, whichever way the loop ended, nor an arrival on a barrier of the pair's second CTA when that
+    // one leaves: each waits for its own.
+    if (rank == 0 && leader) commit<CG>(drained);
+    __syncwarp();
+    for (int i = 0; i < (1 << 16) && !__all_sync(0xffffffffu, mbar_test_wait(drained, 0)); i++) {
     }
   } else {
     const int quad = warp & 3, row = quad * 32 + lane;
@@ -529,7 +533,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
         const Tile T = wk.tile(wk.walk(t));
         const int nw = min(T.n0 + rofs, a.N - 1);
         const size_t r0 = (size_t)T.expert * a.N;
-        y = (int)(r0 + nw);
+        y = same((int)(r0 + nw));
         if constexpr (Row::BOXES == 0) src = Row::base(ctx) + (r0 + nw) * Row::stride(a.K), rows = a.N - 1 - nw;
         rowx.row(ctx, (int)r0 + min(nw + lane, a.N - 1), a.K);
       };

@@ -29,6 +29,12 @@ __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) { return 
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
 }
+// A value that all lanes of the warp hold alike, told to the compiler: what follows from such values, branches on them included, stays in the warp's uniform
+// registers, where the operands of tcgen05.mma, its commits and TMA copies have to be.  From vector registers (a warp number as threadIdx.x >> 5, a
+// quotient or an address read from shared memory is enough) every MMA took 48 to 58 clocks to issue and a commit 100, whatever their size; so an MMA
+// takes 9 clocks with 16 columns, 16 with 32, 64 with 128: the tensor pipe's own.
+__device__ __forceinline__ int same(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ uint32_t same(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
