@@ -46,7 +46,7 @@ struct Args {
   float *parts;
 };
 struct Maps {
-  CUtensorMap x, sums, w[2];
+  CUtensorMap x, sums, w[3];
 };
 
 // D[tmem] += A[tmem] x B[smem], with B a tile of 16 k in the 32-byte swizzle
@@ -92,9 +92,14 @@ struct ExQ4K : TmQ4K {
     }
   }
 };
-struct ExQ6K : TmQ6K {
+template <typename Rows>
+struct ExQ6K : Rows {
+  using Rows::d;
+  using Rows::qh;
+  using Rows::ql;
+  using Rows::sc;
   static constexpr bool MINS = false;
-  __device__ __forceinline__ ExQ6K(const Ctx &c) : TmQ6K(c) {}
+  __device__ __forceinline__ ExQ6K(const typename Rows::Ctx &c) : Rows(c) {}
   __device__ __forceinline__ float scale() const { return d; }
   template <typename Put>
   __device__ __forceinline__ void whole(int, Put &&put) const {
@@ -173,7 +178,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_tmem_kernel(const __grid_co
   if (threadIdx.x == 0) {
     prefetch_tmap(&maps.x);
     if constexpr (Row::MINS) prefetch_tmap(&maps.sums);
-    if constexpr (Row::BOXES > 0) prefetch_tmap(&maps.w[0]), prefetch_tmap(&maps.w[1]);
+    for (int i = 0; i < Row::BOXES; i++) prefetch_tmap(&maps.w[i]);
     abort_flag = 0;
     for (int i = 0; i < 2; i++) mbar_init(full + 8 * i, 8), mbar_init(empty + 8 * i, 1);
     for (int i = 0; i < a.stages; i++) mbar_init(t_full + 8 * i, 2), mbar_init(t_empty + 8 * i, 1);
@@ -511,7 +516,7 @@ int run(const typename Row::Ctx &ctx, const float *x, float *out, int M, int N, 
   if constexpr (Row::BOXES > 0)
     for (int i = 0; i < Row::BOXES; i++)
       ok = ok && map(&tm.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, Row::base(ctx), Row::stride(K), N, Row::stride(K), Row::BOX[i].bytes, 32,
-                     Row::BOX[i].swizzle == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE);
+                     swizzle_of(Row::BOX[i].swizzle));
   if (!ok) return fail(LB200_E_SHAPE, "light_b200: cuTensorMapEncodeTiled failed");
   launch_early(x_rows_kernel<Row::MINS>, dim3((unsigned)((M * nb + 7) / 8)), dim3(256), st, (const float4 *)x, (uint2 *)w8, (uint4 *)(w8 + x_bytes), M, K);
   if (int rc = launched("decode: activations to f16")) return rc;
@@ -557,7 +562,8 @@ int gguf_decode_tmem(int type, const float *x, const void *w, float *out, int M,
   if (q4 && M <= 16 && U < 4 * sms && 4 * tiles < sms) return 0;
   if (M > 32 && U < (q4 ? 5 : 6) * sms && 8 * tiles < sms) return 0;
   if (q4 && !((uintptr_t)w & 15)) return run<ExQ4K>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);
-  if (!q4 && !((uintptr_t)w & 3) && (K >> 8) % 2 == 0) return run<ExQ6K>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);
+  if (!q4 && TmQ6KT::fits(w, K)) return run<ExQ6K<TmQ6KT>>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);
+  if (!q4 && !((uintptr_t)w & 3) && (K >> 8) % 2 == 0) return run<ExQ6K<TmQ6K>>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);
   return 0;
 }
 

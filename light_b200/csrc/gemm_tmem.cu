@@ -790,7 +790,7 @@ int run(const typename Row::Ctx &ctx, const TmemCall &c, Args a, int nt_max, cud
     const cuuint64_t wdims[2] = {(cuuint64_t)Row::stride(c.K), (cuuint64_t)a.E * c.N}, wstr[1] = {wdims[0]};
     for (int i = 0; i < Row::BOXES && r == CUDA_SUCCESS; i++) {
       const cuuint32_t wbox[2] = {(cuuint32_t)Row::BOX[i].bytes, 32};
-      const CUtensorMapSwizzle sw = Row::BOX[i].swizzle == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : Row::BOX[i].swizzle == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE;
+      const CUtensorMapSwizzle sw = swizzle_of(Row::BOX[i].swizzle);
       r = enc(&tm.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(Row::base(ctx)), wdims, wstr, wbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     }
@@ -855,7 +855,9 @@ size_t gemm_tmem_parts_bytes() { return (size_t)MAX_GRID * PART_FLOATS * 4; }
 int gemm_tmem(const TmemCall &c, cudaStream_t st) {
   switch (c.kind) {
     case TmemCall::Q4K: return pick<TmQ4K, false, float>({(const uint8_t *)c.w}, c, st);
-    case TmemCall::Q6K: return pick<TmQ6K, false, float>({(const uint8_t *)c.w}, c, st);
+    case TmemCall::Q6K:
+      if (TmQ6KT::fits(c.w, c.K)) return pick<TmQ6KT, false, float>({(const uint8_t *)c.w}, c, st);
+      return pick<TmQ6K, false, float>({(const uint8_t *)c.w}, c, st);
     case TmemCall::Q80: return pick<TmQ80, false, float>({(const uint8_t *)c.w}, c, st);
     case TmemCall::INT4: {
       const TmInt4::Ctx x{(const uint32_t *)c.w, c.s, c.z, c.G, Div::of(c.G / 64)};

@@ -4,9 +4,9 @@
 // that of row_expand.cuh, value for value.
 //
 // The copies are TMA boxes of 32 rows (copy(), issued by one lane): the same bytes by cp.async cost the warp 5 to 16
-// instructions per granule column, a sixth of everything it issued.  Boxes 64 or 128 bytes wide take the swizzle of that
+// instructions per granule column, a sixth of everything it issued.  Boxes 32, 64 or 128 bytes wide take the swizzle of that
 // width, others are an odd number of granules wide: either way a lane per row reads 16 bytes without bank conflicts.  Q6_K rows start
-// on any even byte, which TMA cannot address: they take the 16-byte cp.async
+// on any even byte, which TMA cannot address: but for rows of a multiple of eight blocks they take the 16-byte cp.async
 // of the granules that cover them (a bulk copy per row and run of granules was 1.5 times slower: its requests do not keep up).
 #pragma once
 #include <cuda.h>
@@ -62,6 +62,9 @@ __device__ __forceinline__ uint32_t pack2(F2 p) {
 struct Box {  // one tensor map: `bytes` wide at row offset x, or with its own pitch
   int bytes, swizzle;
 };
+inline CUtensorMapSwizzle swizzle_of(int bytes) {
+  return bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : bytes == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE;
+}
 // a 32-row box of the (rows, row bytes) matrix: columns x .., rows y ..
 __device__ __forceinline__ void tma_rows(uint32_t dst, const CUtensorMap *m, uint32_t bar, uint32_t x, int y) {
   umma::tma_load_2d(dst, m, bar, (int)x, y);
@@ -149,31 +152,9 @@ struct TmQ4K {
 
 // ---- Q6_K: a unit is half a 210-byte block: of the 14 granules that cover the block, five hold its 64 bytes of ql, three
 // its 32 of qh, and the last two the scales
-struct TmQ6K {
-  struct Ctx { const uint8_t *w; };
-  static constexpr int PITCH = 176, SLOT = 32 * PITCH, BYTES = 0, BOXES = 0;
-  static __host__ __device__ __forceinline__ size_t stride(int K) { return (size_t)(K >> 8) * 210; }
-  static __host__ __device__ __forceinline__ const uint8_t *base(const Ctx &c) { return c.w; }
-  // granule number (of the 14 that cover the block, the first one holding the block's first byte) of piece i of half h
-  static __device__ __forceinline__ int number(int h, int i) { return i < 5 ? 4 * h + i : i < 8 ? 3 + 2 * h + i : 4 + i; }
-  uint32_t low;  // low bits of the row's address: a block starts on any even byte
+struct Q6KUnit {
   uint32_t ql[16], qh[8], sc[2];
   float d;
-  __device__ __forceinline__ TmQ6K(const Ctx &) {}
-  __device__ __forceinline__ void row(const Ctx &c, int r, int K) { low = (uint32_t)(uintptr_t)(c.w + (size_t)r * stride(K)); }
-  __device__ __forceinline__ void fetch_scales(const Ctx &, int) {}
-  __device__ __forceinline__ void load(uint32_t slot, int u) {
-    slot += (threadIdx.x & 31) * PITCH;
-    const uint32_t skew = (low + (uint32_t)(u >> 1) * 210u) & 15u, sh = (skew & 2u) * 8u;
-    lds_skewed(slot, skew, ql);
-    lds_skewed(slot + 80, skew, qh);
-    const uint32_t sa = slot + 128 + 8 * (u & 1) + (skew & ~3u);  // piece 8 holds block bytes 192 ..: the scales, then d
-    const uint32_t c0 = lds32(sa), c1 = lds32(sa + 4), c2 = lds32(sa + 8);
-    sc[0] = __funnelshift_r(c0, c1, sh), sc[1] = __funnelshift_r(c1, c2, sh);
-    uint16_t dh;
-    asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(dh) : "r"(slot + 144 + skew));
-    d = f16_bits_to_f32(dh);
-  }
   template <bool BF16, typename Put>
   __device__ __forceinline__ void expand(int, Put &&put) const {
     const __half2 off = __float2half2_rn(-1056.f);
@@ -191,6 +172,82 @@ struct TmQ6K {
         o[2 * i + 1] = h2_bits(__hmul2(__hadd2(bits_h2(p13), off), ds));
       }
       put(q, o);
+    }
+  }
+};
+
+// Rows at any even byte, by cp.async.
+struct TmQ6K : Q6KUnit {
+  struct Ctx { const uint8_t *w; };
+  static constexpr int PITCH = 176, SLOT = 32 * PITCH, BYTES = 0, BOXES = 0;
+  static __host__ __device__ __forceinline__ size_t stride(int K) { return (size_t)(K >> 8) * 210; }
+  static __host__ __device__ __forceinline__ const uint8_t *base(const Ctx &c) { return c.w; }
+  // granule number (of the 14 that cover the block, the first one holding the block's first byte) of piece i of half h
+  static __device__ __forceinline__ int number(int h, int i) { return i < 5 ? 4 * h + i : i < 8 ? 3 + 2 * h + i : 4 + i; }
+  uint32_t low;  // low bits of the row's address: a block starts on any even byte
+  __device__ __forceinline__ TmQ6K(const Ctx &) {}
+  __device__ __forceinline__ void row(const Ctx &c, int r, int K) { low = (uint32_t)(uintptr_t)(c.w + (size_t)r * stride(K)); }
+  __device__ __forceinline__ void fetch_scales(const Ctx &, int) {}
+  __device__ __forceinline__ void load(uint32_t slot, int u) {
+    slot += (threadIdx.x & 31) * PITCH;
+    const uint32_t skew = (low + (uint32_t)(u >> 1) * 210u) & 15u, sh = (skew & 2u) * 8u;
+    lds_skewed(slot, skew, ql);
+    lds_skewed(slot + 80, skew, qh);
+    const uint32_t sa = slot + 128 + 8 * (u & 1) + (skew & ~3u);  // piece 8 holds block bytes 192 ..: the scales, then d
+    const uint32_t c0 = lds32(sa), c1 = lds32(sa + 4), c2 = lds32(sa + 8);
+    sc[0] = __funnelshift_r(c0, c1, sh), sc[1] = __funnelshift_r(c1, c2, sh);
+    uint16_t dh;
+    asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(dh) : "r"(slot + 144 + skew));
+    d = f16_bits_to_f32(dh);
+  }
+};
+
+// Rows of a multiple of eight blocks, which start on 16-byte boundaries, by TMA: a block then starts equally far into its first granule in every row,
+// so that the words move down by a count that the whole warp shares, and nothing is spent on the addresses and predicates of 11 copies a lane:
+// some 130 of 500 instructions that 32 rows x 128 k took, and issue is what bounds these rows.
+struct TmQ6KT : Q6KUnit {
+  struct Ctx { const uint8_t *w; };
+  static constexpr int SLOT = 32 * 160, BYTES = 32 * 160, BOXES = 3;  // ql, qh, scales and d
+  static constexpr Box BOX[3] = {{80, 0}, {48, 0}, {32, 32}};
+  static __host__ __forceinline__ bool fits(const void *w, int K) { return !((uintptr_t)w & 15) && (K >> 8) % 8 == 0; }
+  static __host__ __device__ __forceinline__ size_t stride(int K) { return (size_t)(K >> 8) * 210; }
+  static __host__ __device__ __forceinline__ const uint8_t *base(const Ctx &c) { return c.w; }
+  static __device__ __forceinline__ void copy(uint32_t slot, const CUtensorMap *m, uint32_t bar, int u, int y) {
+    const uint32_t x = ((uint32_t)(u >> 1) * 210u) & ~15u, h = u & 1;
+    tma_rows(slot, m, bar, x + 64 * h, y);
+    tma_rows(slot + 32 * 80, m + 1, bar, x + 128 + 32 * h, y);
+    tma_rows(slot + 32 * 128, m + 2, bar, x + 192, y);
+  }
+  __device__ __forceinline__ TmQ6KT(const Ctx &) {}
+  __device__ __forceinline__ void row(const Ctx &, int, int) {}
+  __device__ __forceinline__ void fetch_scales(const Ctx &, int) {}
+  template <int FIRST>  // the word of its first granule that a block starts in
+  __device__ __forceinline__ void take(uint32_t slot, uint32_t sh, bool second) {
+    const uint32_t r = threadIdx.x & 31;
+    uint32_t w[20];
+    lds_words(slot + 80 * r, w);
+#pragma unroll
+    for (int i = 0; i < 16; i++) ql[i] = __funnelshift_r(w[FIRST + i], w[FIRST + i + 1], sh);
+    uint32_t v[12];
+    lds_words(slot + 32 * 80 + 48 * r, v);
+#pragma unroll
+    for (int i = 0; i < 8; i++) qh[i] = __funnelshift_r(v[FIRST + i], v[FIRST + i + 1], sh);
+    const uint32_t at = slot + 32 * 128 + 32 * r, flip = (r >> 2 & 1) << 4;  // (32-byte swizzle)
+    uint32_t g[8];
+    to_words(lds128(at + flip), g), to_words(lds128(at + (flip ^ 16)), g + 4);
+    const uint32_t c0 = second ? g[FIRST + 2] : g[FIRST], c1 = second ? g[FIRST + 3] : g[FIRST + 1], c2 = second ? g[FIRST + 4] : g[FIRST + 2];
+    sc[0] = __funnelshift_r(c0, c1, sh), sc[1] = __funnelshift_r(c1, c2, sh);
+    d = f16_bits_to_f32((uint16_t)(g[FIRST + 4] >> sh));
+  }
+  __device__ __forceinline__ void load(uint32_t slot, int u) {
+    const uint32_t skew = ((uint32_t)(u >> 1) * 210u) & 15u, sh = (skew & 2u) * 8u;
+    const bool second = u & 1;
+    if (skew < 8) {
+      if (skew < 4) take<0>(slot, sh, second);
+      else take<1>(slot, sh, second);
+    } else {
+      if (skew < 12) take<2>(slot, sh, second);
+      else take<3>(slot, sh, second);
     }
   }
 };

@@ -1,0 +1,47 @@
+"""Rows of the tensor-memory kernels: matrices of few units and of many, last tiles of few rows, every row format; and the two ways Q6_K rows come in by, which
+carry the same arithmetic.
+
+Bounds: as in the tests of those kernels, 1e-3 for f16 operands with f32 outputs, 3e-3 with bf16 outputs."""
+import pytest
+import torch
+
+from helpers import rel_l2
+from light_b200 import ops, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", ["q4_k", "q6_k", "q8_0", "int4", "fp8"])
+@pytest.mark.parametrize("M,N,K", [(66, 128, 256), (70, 4, 512), (128, 1284, 2048), (257, 132, 6144), (96, 19000, 2048)])
+def test_many_rows(cuda, kind, M, N, K):
+    g = torch.Generator(device=cuda).manual_seed(N)
+    dt = torch.bfloat16 if kind in ("int4", "fp8") else torch.float32
+    x = torch.randn(M, K, generator=g, device=cuda).to(dt)
+    if kind == "int4":
+        w4 = ops.Int4(torch.randint(-2**31, 2**31, (N, K // 8), generator=g, device=cuda, dtype=torch.int32), torch.rand(N, K // 128, generator=g, device=cuda) * 0.02,
+                      torch.randint(0, 16, (N, K // 128), generator=g, device=cuda).float(), 128)
+        y, w = ops.MatMulInt4(x, w4), ops.DequantizeInt4(w4, torch.bfloat16).double()
+    elif kind == "fp8":
+        codes, scale = synth.random_fp8_block(N + K, N, K, 4, 64, device=cuda)
+        y, w = ops.MatMulF8Block(x, codes, scale, 4, 64), ops.DequantizeF8Block(codes, scale, 4, 64, torch.bfloat16).double()
+    else:
+        t = {"q4_k": ops.Q4_K, "q6_k": ops.Q6_K, "q8_0": ops.Q8_0}[kind]
+        q = ops.QTensor(synth.gaussian_weight(N + K, t, N, K, device=cuda).reshape(-1), t, (N, K))
+        y, w = ops.MatMulQ(x, q), ops.Dequantize(q).double()
+    assert ops.prefill_status(0) == 0
+    assert rel_l2(y.cpu().double().numpy(), (x.double() @ w.t()).cpu().numpy()) <= (1e-3 if dt == torch.float32 else 3e-3)
+
+
+@pytest.mark.parametrize("M,N,K", [(18, 4100, 2048), (33, 12804, 2048), (64, 2564, 14336), (65, 388, 4096), (333, 1028, 2048)])
+def test_q6_k_rows_by_tma_and_by_cp_async(cuda, M, N, K):
+    """Rows of a multiple of eight blocks at a 16-byte boundary come by TMA, four bytes off one they do not: value for value the same operands, in the same order."""
+    raw = synth.gaussian_weight(N + M, ops.Q6_K, N, K, device=cuda).reshape(-1)
+    off = torch.empty(raw.numel() + 16, dtype=raw.dtype, device=cuda)[4:4 + raw.numel()]
+    off.copy_(raw)
+    assert raw.data_ptr() % 16 == 0 and off.data_ptr() % 16 == 4
+    x = torch.randn(M, K, generator=torch.Generator(device=cuda).manual_seed(M), device=cuda)
+    y, z = (ops.MatMulQ(x, ops.QTensor(d, ops.Q6_K, (N, K))) for d in (raw, off))
+    assert ops.prefill_status(0) == 0
+    assert torch.equal(y, z)
+    w = ops.Dequantize(ops.QTensor(raw, ops.Q6_K, (N, K))).double()
+    assert rel_l2(y.cpu().double().numpy(), (x.double() @ w.t()).cpu().numpy()) <= 1e-3
