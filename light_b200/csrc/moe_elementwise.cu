@@ -21,21 +21,36 @@ struct alignas(16) Vec8 {  // eight elements: one 16-byte access (bf16 / f16) or
   T v[8];
 };
 
+// n / d with a 32-bit division where both fit, which a launch decides for all of its threads (a 64-bit one takes about as many instructions as the
+// eight elements that it places)
+__device__ __forceinline__ long long div_by(long long n, long long d, bool small) {
+  return small ? (long long)((uint32_t)n / (uint32_t)d) : n / d;
+}
+// n / d for a d of 1 or more: reciprocal, product and one correction by the remainder (P. Markstein, IBM J. Res. Dev. 34 (1990)), within one ulp.  Where an
+// infinity makes the remainder a NaN (d after exp overflows, n itself), the product is the quotient.
+__device__ __forceinline__ float quotient(float n, float d) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;\n" : "=f"(r) : "f"(d));
+  const float q = n * r, c = fmaf(fmaf(-q, d, n), r, q);
+  return c == c ? c : q;
+}
+
 // h (M, 2 I): gate = h[:, :I], up = h[:, I:] -> out (M, I) = act(gate) * up; eight elements per thread
 template <typename T>
 __global__ void __launch_bounds__(256) moe_gate_mul_kernel(const T *__restrict__ h, T *__restrict__ out, long long M, int I, int gelu) {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const long long per_row = I / 8, total = M * per_row;
+  const bool small = total < 1ll << 31;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long m = i / per_row;
+    const long long m = div_by(i, per_row, small);
     const int c = (int)(i - m * per_row) * 8;
     const Vec8<T> g = *reinterpret_cast<const Vec8<T> *>(h + m * 2 * I + c), u = *reinterpret_cast<const Vec8<T> *>(h + m * 2 * I + I + c);
     Vec8<T> o;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       const float gv = (float)g.v[j];
-      const float a = gelu ? 0.5f * gv * (1.f + erff(gv * 0.70710678118654752f)) : gv / (1.f + expf(-gv));
+      const float a = gelu ? 0.5f * gv * (1.f + erff(gv * 0.70710678118654752f)) : quotient(gv, 1.f + expf(-gv));
       o.v[j] = (T)(rnd<T>(a) * (float)u.v[j]);
     }
     *reinterpret_cast<Vec8<T> *>(out + m * I + c) = o;
@@ -48,8 +63,9 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const T *__restrict__ 
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const long long per_row = N / 8, total = tokens * per_row;
+  const bool small = total < 1ll << 31;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / per_row;
+    const long long t = div_by(i, per_row, small);
     const int c = (int)(i - t * per_row) * 8;
     const T *src = pair_out + t * topk * (long long)N + c;
     float acc[8];
@@ -80,8 +96,9 @@ __global__ void __launch_bounds__(256) moe_combine_weighted_kernel(const T *__re
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   const long long per_row = N / 8, total = tokens * per_row;
+  const bool small = total < 1ll << 31;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long t = i / per_row;
+    const long long t = div_by(i, per_row, small);
     const int c = (int)(i - t * per_row) * 8;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int s = 0; s < topk; s++) {
