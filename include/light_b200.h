@@ -415,6 +415,10 @@ LB200_API int light_b200_moe_route_deepseek(const float *logits, const float *bi
 LB200_API int light_b200_moe_route_topk(const float *probs, int64_t *ids, float *weights, int T, int E, int topk, int normalize,
                                         int device, void *stream);
 
+/* The router's logits: x (T, K) LB200_F32 or LB200_BF16 times w (E, K) F32 -> out (T, E) F32, in f32 arithmetic or better (operands in three bf16
+ * parts on the tensor cores).  K is whole granules of 16 bytes of x and of w; pointers 16-byte aligned. */
+LB200_API int light_b200_router_logits(const void *x, int act_dtype, const float *w, float *out, int T, int E, int K, int device, void *stream);
+
 /* The element-wise steps of a sparse MoE block around the two grouped matmuls, each as one launch with the roundings of
  * the reference's unfused sequence (nn/moe.go:206-236: Narrow gate / up -> SiLU -> Mul; ops.MoECombine, ops/moe.go:206-240).
  *   moe_gate_mul: h (M, 2 I), gate = h[:, :I], up = h[:, I:] -> out (M, I) = act(gate) * up, act SiLU (gelu = 0) or GELU-erf,

@@ -603,6 +603,19 @@ int light_b200_moe_route_topk(const float *probs, int64_t *ids, float *weights, 
   return moe_route_topk(probs, ids, weights, T, E, topk, normalize, (cudaStream_t)stream);
 }
 
+int light_b200_router_logits(const void *x, int act_dtype, const float *w, float *out, int T, int E, int K, int device, void *stream) {
+  if (act_dtype != LB200_F32 && act_dtype != LB200_BF16) return fail(LB200_E_DTYPE, "light_b200: router_logits: element type %d", act_dtype);
+  if (T < 0 || T > 1 << 21 || E < 1 || K < 1 || K % (act_dtype == LB200_F32 ? 4 : 8))
+    return fail(LB200_E_SHAPE, "light_b200: router_logits: T=%d E=%d K=%d (K whole 16-byte granules)", T, E, K);
+  if (T == 0) return 0;
+  REQUIRE_PTR(x, "router_logits");
+  REQUIRE_PTR(w, "router_logits");
+  REQUIRE_PTR(out, "router_logits");
+  if (!aligned(x, 16) || !aligned(w, 16)) return fail(LB200_E_ALIGN, "light_b200: router_logits: pointers not 16-byte aligned");
+  if (int rc = bind(device)) return rc;
+  return router_logits(x, act_dtype, w, out, T, E, K, (cudaStream_t)stream);
+}
+
 int light_b200_moe_gate_mul(const void *h, void *out, int dtype, int64_t M, int I, int gelu, int device, void *stream) {
   if (M < 0 || I <= 0 || I % 8) return fail(LB200_E_SHAPE, "light_b200: moe_gate_mul: M=%lld I=%d (I a positive multiple of 8)", (long long)M, I);
   if (M == 0) return 0;

@@ -195,6 +195,7 @@ int gguf_decode_ts(int type, const float *x, const void *const *w, float *const 
                    size_t ws_bytes, cudaStream_t st);
 int decode_ts_status();
 int gather_columns(const void *x, const int64_t *idx, void *out, int elt, long long M, int K, cudaStream_t st);
+int router_logits(const void *x, int dtype, const float *w, float *out, int T, int E, int K, cudaStream_t st);
 int moe_gate_mul(const void *h, void *out, int dtype, long long M, int I, int gelu, cudaStream_t st);
 int moe_combine(const void *pair_out, void *out, int dtype, long long tokens, int N, int topk, cudaStream_t st);
 int moe_combine_weighted(const void *rows, const int64_t *index, const float *weights, float *out, int dtype, long long tokens, int N,

@@ -514,6 +514,17 @@ def MoERouteFromIDs(ids: torch.Tensor, weights: torch.Tensor, T: int, topk: int)
     return MoERouting(ids.reshape(T, topk), weights.reshape(T * topk).float(), sorted_pairs, sorted_expts)
 
 
+def RouterLogits(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """The router's matmul of a sparse block (nn/moe.go:121-150): x (T, K) F32 or BF16, w (E, K) F32 -> (T, E) F32, in F32 arithmetic."""
+    if x.dim() != 2 or w.dim() != 2 or x.shape[1] != w.shape[1] or x.dtype not in (torch.float32, torch.bfloat16) or w.dtype != torch.float32:
+        raise ValueError(f"router_logits: x {tuple(x.shape)} {x.dtype}, w {tuple(w.shape)} {w.dtype}")
+    dev = _dev(x, "RouterLogits")
+    out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
+    _lib.check(_lib.lib().light_b200_router_logits(_ptr(x.contiguous()), _ACT[x.dtype], _ptr(w.contiguous()), _ptr(out), x.shape[0], w.shape[0], x.shape[1], dev,
+                                                   _stream(dev)))
+    return out
+
+
 def MoERoute(probs: torch.Tensor, topk: int, normalize: bool) -> MoERouting:
     """ops.MoERoute (ops/moe.go:29-71): router probabilities (T, E) F32 -> the k largest experts per token, their
     probabilities (renormalised when `normalize`), and the pairs sorted by expert.  Selection and sort run on the

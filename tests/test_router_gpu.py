@@ -1,0 +1,50 @@
+"""The router's matmul: f32 in effect.  Bound: f32 products summed in blocks of 32 and then in f32: 2^-24 of the sum of magnitudes per addition, of which K / 32 follow
+one another, and far below that on average: 2e-6 of sum |x w| with room."""
+import pytest
+import torch
+
+from light_b200 import nn, ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,E,K", [(1, 8, 8), (16, 256, 7168), (17, 60, 2048), (77, 128, 2040), (333, 33, 520), (1024, 256, 1024), (2400, 250, 264)])
+def test_against_64_bits(cuda, dtype, T, E, K):
+    g = torch.Generator(device=cuda).manual_seed(T + E)
+    x, w = torch.randn(T, K, generator=g, device=cuda).to(dtype), torch.randn(E, K, generator=g, device=cuda)
+    w[E // 2] *= 1e20
+    y = ops.RouterLogits(x, w)
+    assert torch.equal(y, ops.RouterLogits(x, w))
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert float(((y - want).abs() / size).max()) <= 2e-6
+    # no further off than the library's f32 matmul, but for chance
+    lib = x.float() @ w.t()
+    assert float(((y - want) / size).norm()) <= 1.25 * float(((lib - want) / size).norm()) + 1e-9
+
+
+def test_infinities_and_large_values(cuda):
+    x, w = torch.ones(20, 64, device=cuda), torch.ones(40, 64, device=cuda)
+    w[3, 5], w[4, 6], w[5, 7] = 3.4e38, float("inf"), float("nan")
+    x[7, 0], x[8, 1] = float("-inf"), float("nan")
+    y = ops.RouterLogits(x, w)
+    want = x @ w.t()
+    assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isinf(y), torch.isinf(want))
+    ok = torch.isfinite(want)
+    assert torch.allclose(y[ok], want[ok], rtol=1e-6)
+
+
+def test_sparse_block_takes_the_same_route(cuda):
+    """nn.SparseMoE chooses by these logits as by the library's; a gate that requires a gradient goes the library's way."""
+    g = torch.Generator(device=cuda).manual_seed(1)
+    H, I, E, T, k = 256, 128, 16, 40, 2
+    gate = nn.Linear(H, E, W=torch.randn(E, H, generator=g, device=cuda) / 16)
+    gu, dn = (torch.randn(E, n, m, generator=g, device=cuda).bfloat16() / 16 for n, m in ((2 * I, H), (H, I)))
+    x = torch.randn(T, H, generator=g, device=cuda).bfloat16()
+    seen = []
+    moe = nn.SparseMoE(gate, gu, dn, TopK=k, RouterF32=True, Router=lambda l: seen.append(l) or ops.MoERouteSigmoid(l, None, k))
+    y = moe.forward(x)
+    gate.W.requires_grad_()
+    z = moe.forward(x)
+    assert torch.allclose(seen[0], seen[1], rtol=1e-5, atol=1e-5) and seen[1].requires_grad and not seen[0].requires_grad
+    assert torch.equal(y, z)
