@@ -96,7 +96,7 @@ LB200_API int light_b200_set_workspace(int device, void *ptr, size_t bytes);
  * copy of x plus about 42 MB of partial tiles above 64 rows; with less, those calls run a kernel that needs the copy alone.  (Q6_K with an
  * odd K / 256 uses none of it: light_b200_q6k_scratch_bytes below.)  Up to
  * 64 rows: what the token-tile kernels stage, or the f16 copy plus 21 MB where the tensor-memory kernel has such calls (Q8_0 from 4
- * rows, bf16 rows of 4-bit weights from 17). */
+ * rows, bf16 rows of 4-bit weights from 4). */
 LB200_API unsigned long long light_b200_matmul_q_workspace_bytes(int M, int K);
 
 /* 0 if no bounded device-side wait of the tensor-core kernels ever gave up on this device, 1 if one

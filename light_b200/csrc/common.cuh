@@ -179,7 +179,7 @@ int gemm_tmem(const TmemCall &c, cudaStream_t st);
 size_t gemm_tmem_parts_bytes();
 size_t gemm_tmem_sync_bytes();
 int gemm_tmem_status();
-// whole numbers through tensor memory, 9 (Q6_K: 17) .. 64 rows of Q4_K / Q6_K: 1 = took the call, 0 = not covered, other = error
+// whole numbers through tensor memory, 9 .. 64 rows of Q4_K / Q6_K: 1 = took the call, 0 = not covered, other = error
 int gguf_decode_tmem(int type, const float *x, const void *w, float *out, int M, int N, int K, void *ws, size_t ws_bytes, cudaStream_t st);
 int decode_tmem_status();
 size_t decode_nt_ws_bytes(int M, int K);

@@ -1,4 +1,4 @@
-// Batched decode, up to 64 activation rows (tokens), from 9 of Q4_K and from 17 of Q6_K: the weights go through TENSOR MEMORY as WHOLE NUMBERS.
+// Batched decode, 9 to 64 activation rows (tokens) of Q4_K and Q6_K: the weights go through TENSOR MEMORY as WHOLE NUMBERS.
 //
 // What bounds the token tiles on mma.sync (gguf_decode_nt.cu): they expand a weight in registers once per warp and multiply by the legacy
 // tensor path, which holds the pipe 8 clocks per 16 x 16 x 8; neither pipe nor issue is half busy, and time grows with the tokens
@@ -10,8 +10,9 @@
 //   warps 0-15   expanders, as gemm_tmem.cu's: the four warps w, w + 4, .. own rows 32 (w & 3) .. + 31, set w / 4 has every fourth unit of 128 k
 //                (sets 0 and 2 the first halves of blocks, 1 and 3 the second).
 //   warps 16-17  one lane of each: TMA of the tokens, half a block each; the second one also their sub-blocks' sums.
-//   warp  18     MMAs and commits, a block at a time: 18 MMAs take some 900 clocks, and a pass 400 more of waits and commits that the tensor
-//                pipe does not cover (half a block at a time: 28672 x 4096, 32 rows 33.2 us where this takes 30.9).
+//   warp  18     MMAs and commits, a block at a time (half a block at a time a pass has the same looks at barriers for half the work).  18 MMAs of 32 columns
+//                are 290 clocks of the tensor pipe; beside the expanders' instructions they take some 750 to issue, of 1400 to 1500 a block (with
+//                operands in vector registers 900 whatever their columns: same(), tmem_ops.cuh).
 //   warps 19-26  drain: row quarter w & 3 and every second chunk of 16 tokens; per block sums += d x D; at a tile's end the minimums'
 //                sums are added and the tile leaves, or is left for, or put together from, the runs it is cut into.
 //
@@ -547,20 +548,24 @@ int run(const typename Row::Ctx &ctx, const float *x, float *out, int M, int N, 
 //   Q4_K, 17 to 32: from 16 Mi weights on: 28672 x 4096 42.6 / 30.9, 6144 x 4096 18.6 / 14.7, 8192 x 2048 16.6 / 12.6, 1024 x 16384 26.6 / 19.1,
 //     4096 x 4096 12.8 / 13.1; below, a tile is cut into too many parts (4096 x 2048 9.3 / 9.8, 1024 x 4096 9.3 / 10.7).
 //   33 to 64, where a part is a chunk more to each warp: not where a tile is cut into more than eight parts of few blocks: Q4_K 2048 x 8192 18.5 / 21.4, 1024 x
-//     20480 24.4 / 31.5, 2048 x 10240 21.3 / 23.5, but 2560 x 6656 20.6 / 18.8, 1536 x 16384 26.9 / 24.5, 28672 x 4096 66.7 / 35.7, 4096 x 14336 40.8 / 27.8.
-//     Q6_K 2048 x 8192 19.0 / 21.4, 2048 x 12288 24.2 / 24.6, but 2560 x 6656 21.9 / 20.4, 2048 x 16384 30.7 / 27.4, 4096 x 14336 44.0 / 33.6, 128256 x
-//     4096 307 / 170 (4096 x 4096 17.1 / 17.6, 8192 x 2048 16.3 / 16.2).
-//   Q6_K, 17 to 32: from 4 Mi on: 2048 x 2048 10.7 / 7.9, 2048 x 5632 19.7 / 15.9, 4096 x 14336 32.4 / 29.1, 128256 x 4096 186 / 156; 9 to 16 rows lose
-//     (4096 x 14336 28.1 / 28.8).
+//     8192 17.3 / 18.2, 1024 x 20480 24.4 / 31.5, 2048 x 10240 21.3 / 23.5, but 2048 x 2048 11.9 / 8.8, 1024 x 4096 14.9 / 11.7, 4096 x 2048 12.0 / 9.5,
+//     2048 x 4096 13.6 / 12.3, 2560 x 6656 20.6 / 18.8, 1536 x 16384 26.9 / 24.5, 28672 x 4096 65.2 / 33.2, 4096 x 14336 40.8 / 27.8.
+//     Q6_K 2048 x 8192 19.0 / 21.4, 2048 x 12288 24.2 / 24.6, but 1024 x 4096 14.8 / 11.0, 2048 x 2048 11.6 / 8.1, 2048 x 4096 13.6 / 12.0, 2560 x 6656 21.9 / 20.4, 2048 x 16384 30.7 /
+//     27.4, 4096 x 14336 43.2 / 26.5, 128256 x 4096 307 / 170 (4096 x 4096 17.1 / 15.6).
+//   Q6_K, 17 to 32: 1024 x 3584 10.7 / 7.9, 2048 x 2048 10.7 / 6.9, 2048 x 5632 19.0 / 14.3, 4096 x 14336 31.1 / 21.9, 128256 x 4096 186 / 156.  9 to 16, but for
+//     tiles in more than nine parts (2048 x 5632 16.2 / 14.1, 2048 x 7168 14.5 / 15.6): 4096 x 1024 8.0 / 6.2, 2048 x 2048 8.5 / 6.8, 1024 x 4096 9.3 / 8.0, 2048 x 4096
+//     10.8 / 8.9, 3072 x 9216 19.0 / 18.3, 4096 x 10240 22.2 / 17.8.
 int gguf_decode_tmem(int type, const float *x, const void *w, float *out, int M, int N, int K, void *ws, size_t ws_bytes, cudaStream_t st) {
-  static const int q4_min = knob("LIGHT_B200_DECODE_TMEM_MIN_M", 9), q6_min = q4_min > 17 ? q4_min : 17;
+  static const int min_m = knob("LIGHT_B200_DECODE_TMEM_MIN_M", 9);
   const bool q4 = type == LB200_Q4_K;
   const long long size = (long long)N * K;
-  if ((!q4 && type != LB200_Q6_K) || M < (q4 ? q4_min : q6_min) || M > MAX_NT || K % 256 || !ws || N < 128 || size >> 8 > 1ll << 30 || ((uintptr_t)x & 15)) return 0;
+  if ((!q4 && type != LB200_Q6_K) || M < min_m || M > MAX_NT || K % 256 || !ws || N < 128 || size >> 8 > 1ll << 30 || ((uintptr_t)x & 15)) return 0;
   const long long tiles = (N + 127) / 128, U = tiles * (K >> 8), sms = sm_count();
-  if (size < (q4 || M > 32 ? 16ll : 4ll) << 20) return 0;
+  const long long runs = U < 2 * sms ? U / 2 : sms;  // (as run() has them)
+  if (size < (q4 && M <= 32 ? 16ll : 2ll) << 20) return 0;  // (below 2 Mi a matrix is one of several that share x: the token tiles take those in one launch)
   if (q4 && M <= 16 && U < 4 * sms && 4 * tiles < sms) return 0;
-  if (M > 32 && U < (q4 ? 5 : 6) * sms && 8 * tiles < sms) return 0;
+  if (!q4 && M <= 16 && runs > 9 * tiles) return 0;
+  if (M > 32 && U < (q4 ? 5 : 6) * sms && runs > 8 * tiles) return 0;
   if (q4 && !((uintptr_t)w & 15)) return run<ExQ4K>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);
   if (!q4 && TmQ6KT::fits(w, K)) return run<ExQ6K<TmQ6KT>>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);
   if (!q4 && !((uintptr_t)w & 3) && (K >> 8) % 2 == 0) return run<ExQ6K<TmQ6K>>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);

@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tmem_kernel(const __grid_cons
     // The whole warp runs the loop and one elected lane issues.  A pass is a chain of some 60 instructions that share their
     // scheduler with the expanders: with 64 k and two or three barriers per pass it took 700 clocks and the tensor pipe
     // stood at half its rate.  Hence 128 k to a stage, and the look at the next stage's barriers issued
-    // before this stage's MMAs.
+    // before this stage's MMAs.  (128 x 16 x 128 in 8 MMAs and two commits: 110 clocks alone, 290 beside the expanders.)
     const bool leader = elect_one();
     int s = 0, par = 0, bt = 0, bpar = 0, seg = 0;
     bool ok = true, wide_before = false;

@@ -1059,10 +1059,13 @@ int int4_prefill(const void *x, const uint32_t *codes, const float *s, const flo
 // At 16 rows the two are even, and at 2048 x 4096 and below the token tiles are: hence the lines.
 int int4_narrow_tmem(const void *x, const uint32_t *codes, const float *s, const float *z, void *y, int act_dtype, int M, int N, int K, int G, int device,
                      cudaStream_t st) {
-  static const int min_m = getenv("LIGHT_B200_TMEM_INT4_MIN_M") ? atoi(getenv("LIGHT_B200_TMEM_INT4_MIN_M")) : 17;
+  static const int min_m = getenv("LIGHT_B200_TMEM_INT4_MIN_M") ? atoi(getenv("LIGHT_B200_TMEM_INT4_MIN_M")) : 4;
+  // us, the token tiles / here, a chain of calls with a cold L2.  4 and 16 rows: 1024 x 1024 6.4, 6.8 / 5.5, 5.6, 4096 x 1024 7.1, 7.6 / 5.6, 5.7, 2048 x 4096 9.4, 10.5 / 8.7, 9.2, 4096 x
+  // 4096 12.3, 14.2 / 10.6, 10.9, 14336 x 4096 19.6, 22.4 / 18.5, 18.4, 3584 x 18944 22.5, 25.3 / 19.8, 20.0, 37888 x 3584 27.3, 30.9 / 28.5, 28.6: so up to eight rows of the
+  // largest stay.  32 and 64 rows: 1024 x 1024 8.0, 9.7 / 6.0, 6.3, 2048 x 2048 10.8, 12.5 / 8.6, 9.4, 1024 x 8192 15.3, 17.9 / 10.8, 12.4, 3072 x 3072 12.4, 13.7 / 9.2, 10.9.
   // Groups of 128 only, whose token-tile kernel rounds x to f16 as well: the kernel that has other groups multiplies bf16 x as it is,
   // and f16 would clamp values beyond 65504 and lose bits of those below 6e-5.
-  if (act_dtype != LB200_BF16 || M < min_m || M > 64 || (long long)N * K < (10ll << 20) || K % 256 || G != 128 || ((uintptr_t)codes & 15) || ((uintptr_t)x & 15) ||
+  if (act_dtype != LB200_BF16 || M < min_m || M > 64 || (long long)N * K < (1ll << 20) || (M <= 8 && (long long)N * K >= (100ll << 20)) || K % 256 || G != 128 || ((uintptr_t)codes & 15) || ((uintptr_t)x & 15) ||
       !use_tmem())
     return 0;
   void *ws;

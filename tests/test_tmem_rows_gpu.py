@@ -45,3 +45,27 @@ def test_q6_k_rows_by_tma_and_by_cp_async(cuda, M, N, K):
     assert torch.equal(y, z)
     w = ops.Dequantize(ops.QTensor(raw, ops.Q6_K, (N, K))).double()
     assert rel_l2(y.cpu().double().numpy(), (x.double() @ w.t()).cpu().numpy()) <= 1e-3
+
+
+@pytest.mark.parametrize("M", [4, 8, 9, 16, 33])
+@pytest.mark.parametrize("N,K", [(1024, 1024), (1020, 1280), (4100, 256), (130, 8448), (409600, 256)])
+def test_few_rows_of_int4(cuda, M, N, K):
+    """From 2^20 weights on (100 * 2^20: from nine rows): x in f16, then the bf16 output's rounding (2^-8 of a value at most)."""
+    g = torch.Generator(device=cuda).manual_seed(N)
+    w = ops.Int4(torch.randint(-2**31, 2**31, (N, K // 8), generator=g, device=cuda, dtype=torch.int32), torch.rand(N, K // 128, generator=g, device=cuda) * 0.02,
+                 torch.randint(0, 16, (N, K // 128), generator=g, device=cuda).float(), 128)
+    x = torch.randn(M, K, generator=g, device=cuda).bfloat16()
+    y = ops.MatMulInt4(x, w)
+    assert torch.equal(y, ops.MatMulInt4(x, w)) and ops.prefill_status(0) == 0
+    want = x.double() @ ops.DequantizeInt4(w, torch.float32).double().t()
+    assert rel_l2(y.cpu().double().numpy(), want.cpu().numpy()) <= 2.5e-3
+
+
+@pytest.mark.parametrize("dt,M,N,K", [(ops.Q6_K, 9, 1024, 2048), (ops.Q6_K, 16, 1028, 3584), (ops.Q6_K, 12, 2048, 5632), (ops.Q6_K, 10, 4100, 512), (ops.Q6_K, 33, 1024, 2048),
+                                      (ops.Q4_K, 33, 1024, 2048), (ops.Q4_K, 64, 1030, 4096), (ops.Q4_K, 47, 2052, 2048), (ops.Q6_K, 64, 2052, 2560), (ops.Q4_K, 40, 1024, 8192)])
+def test_small_matrices_of_9_to_64_rows(cuda, dt, M, N, K):
+    q = ops.QTensor(synth.gaussian_weight(N + M, dt, N, K, device=cuda).reshape(-1), dt, (N, K))
+    x = torch.randn(M, K, generator=torch.Generator(device=cuda).manual_seed(K), device=cuda)
+    y = ops.MatMulQ(x, q)
+    assert torch.equal(y, ops.MatMulQ(x, q)) and ops.prefill_status(0) == 0
+    assert rel_l2(y.cpu().double().numpy(), (x.double() @ ops.Dequantize(q).double().t()).cpu().numpy()) <= 1e-3
