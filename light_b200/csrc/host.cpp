@@ -134,6 +134,23 @@ PyObject *linear_f8(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
                                         act_of(*x.t), (int)M, (int)N, (int)K, (int)bR, (int)bC, dev, stream_of(dev)), out);
 }
 
+// (x (T, K) F32 / BF16, w (E, K) F32) -> (T, E) F32.  F32 rows up to 2^18 logits: beyond, the library's f32 matmul is the faster one (router.cu).
+PyObject *router_logits(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+  ARGS(2)
+  Arg x, w;
+  NEED(x.ok(a[0]) && w.ok(a[1]) && x.t->dim() == 2 && w.t->dim() == 2 && cuda_contig(*x.t) && cuda_contig(*w.t) && w.t->scalar_type() == at::kFloat);
+  const auto dt = x.t->scalar_type();
+  const long long T = x.t->size(0), E = w.t->size(0), K = x.t->size(1);
+  NEED((dt == at::kBFloat16 || (dt == at::kFloat && T * E <= 1ll << 18)) && T > 0 && T <= 1ll << 21 && E > 0 && E < 1ll << 31 && K > 0 && K < 1ll << 31 && K % 8 == 0 && w.t->size(1) == K &&
+       w.t->get_device() == x.t->get_device());
+  const void *const xp = x.t->const_data_ptr();
+  const float *const wp = w.t->const_data_ptr<float>();
+  NEED(!((uintptr_t)xp & 15) && !((uintptr_t)wp & 15));
+  const int dev = x.t->get_device();
+  at::Tensor out = at::empty({T, E}, w.t->options());
+  return give(light_b200_router_logits(xp, act_of(*x.t), wp, out.data_ptr<float>(), (int)T, (int)E, (int)K, dev, stream_of(dev)), out);
+}
+
 // (h (M, 2 I), gelu) -> (M, I)
 PyObject *gate_mul(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
   ARGS(2)
@@ -292,6 +309,7 @@ PyMethodDef kMethods[] = {FN(set_workspace, "registers a device's workspace size
                           FN(linear_q, "x . W^T, GGUF blocks"),
                           FN(linear_int4, "x . W^T, 4-bit groups"),
                           FN(linear_f8, "x . W^T, block-scaled FP8"),
+                          FN(router_logits, "x . W^T, F32"),
                           FN(gate_mul, "act(gate) * up"),
                           FN(combine, "sum of the top-k slot rows"),
                           FN(moe_route, "top-k experts of each token and the pairs sorted by expert"),

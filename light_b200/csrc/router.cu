@@ -8,7 +8,7 @@
 // as many issue slots as the MMAs take clocks, and both are re-read for every 64 tokens.
 //   us, the library (with the pass to f32 for bf16) / here:  bf16 4096 x 256 x 7168 370 / 203, 1024 x 128 x 4096 82 / 27, 32 x 256 x 7168 54 / 23, 8 x 256 x 7168
 //   26.7 / 11.9;  f32 77 x 128 x 2048 24.7 / 12.9, 300 x 200 x 3072 64 / 24, 2048 x 64 x 2048 37 / 18, 1024 x 256 x 4096 78 / 58, but 4096 x 128 x 4096
-//   110 / 106, 2500 x 200 x 1536 47 / 74, 4096 x 256 x 4096 166 / 203: f32 rows come here up to 2^18 logits (SparseMoE._routes_here).
+//   110 / 106, 2500 x 200 x 1536 47 / 74, 4096 x 256 x 4096 166 / 203: f32 rows come here up to 2^18 logits (host.cpp).
 //
 // A CTA holds a tile of BM tokens x BN experts and a share of K; the CTAs of a cluster hold the others and add up through each other's shared memory, in their
 // order.  A sum that is not finite (an infinity times the zero rest of another operand is no number) is made again by multiply-adds.

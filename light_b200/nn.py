@@ -142,8 +142,9 @@ class SparseMoE:
         if x.shape[-1] != H:
             raise ValueError(f"nn.SparseMoE: last dim {x.shape[-1]} != hidden {H}")
         flat = x.contiguous().reshape(-1, H)
-        if self._routes_here(flat):
-            route = self._choose(ops.RouterLogits(flat, self.Gate.W))
+        logits = self._logits_here(flat)
+        if logits is not None:
+            route = self._choose(logits)
         else:
             route = self.route(flat.float() if (self.RouterF32 and flat.dtype != torch.float32) else flat)
         if self.GateUpQ4 is not None:
@@ -158,19 +159,15 @@ class SparseMoE:
             return self.Router(logits)
         return ops.MoERoute(torch.softmax(logits, -1), self.TopK, self.NormTopK)
 
-    def _routes_here(self, x: torch.Tensor) -> bool:
-        """Whether the router's matmul is ops.RouterLogits: a plain F32 gate on rows that it takes as they are, with nothing for autograd to record."""
+    def _logits_here(self, x: torch.Tensor) -> Optional[torch.Tensor]:
+        """The router's matmul as ops.RouterLogits: a plain F32 gate on rows that it takes as they are, with nothing for autograd to record; else None."""
         g = self.Gate
         w = g.W
-        if type(self).route is not SparseMoE.route or type(g) is not Linear or g.B is not None or g.W4 is not None or type(w) is not torch.Tensor or type(x) is not torch.Tensor:
-            return False
-        if x.dtype != torch.float32 and not (self.RouterF32 and x.dtype == torch.bfloat16):
-            return False
-        return x.is_cuda and w.device == x.device and w.dtype == torch.float32 and w.dim() == 2 and x.dim() == 2 and 0 < x.shape[0] <= 1 << 21 and \
-            (x.dtype != torch.float32 or x.shape[0] * w.shape[0] <= 1 << 18) and \
-            tuple(w.shape) == (g.out_features, g.in_features) and x.shape[1] == g.in_features and g.in_features % 8 == 0 and w.shape[0] > 0 and \
-            x.is_contiguous() and w.is_contiguous() and not x.data_ptr() % 16 and not w.data_ptr() % 16 and \
-            not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad)) and not torch.is_autocast_enabled("cuda")
+        if type(self).route is not SparseMoE.route or type(g) is not Linear or g.B is not None or g.W4 is not None or type(w) is not torch.Tensor or type(x) is not torch.Tensor or \
+                not (x.dtype == torch.float32 or (self.RouterF32 and x.dtype == torch.bfloat16)) or tuple(w.shape) != (g.out_features, g.in_features) or \
+                torch.is_autocast_enabled("cuda"):
+            return None
+        return ops._host.router_logits(x, w)
 
     def run_experts(self, flat: torch.Tensor, route: ops.MoERouting) -> torch.Tensor:
         gu, dn = self.GateUp, self.Down

@@ -518,6 +518,9 @@ def RouterLogits(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """The router's matmul of a sparse block (nn/moe.go:121-150): x (T, K) F32 or BF16, w (E, K) F32 -> (T, E) F32, in F32 arithmetic."""
     if x.dim() != 2 or w.dim() != 2 or x.shape[1] != w.shape[1] or x.dtype not in (torch.float32, torch.bfloat16) or w.dtype != torch.float32:
         raise ValueError(f"router_logits: x {tuple(x.shape)} {x.dtype}, w {tuple(w.shape)} {w.dtype}")
+    y = _host.router_logits(x, w)
+    if y is not None:
+        return y
     dev = _dev(x, "RouterLogits")
     out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
     _lib.check(_lib.lib().light_b200_router_logits(_ptr(x.contiguous()), _ACT[x.dtype], _ptr(w.contiguous()), _ptr(out), x.shape[0], w.shape[0], x.shape[1], dev,
