@@ -967,11 +967,12 @@ __device__ __forceinline__ uint32_t lds16(uint32_t addr) {
   asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(v) : "r"(addr));
   return v;
 }
-// word at a 2-byte aligned shared address: odd == false -> 4-byte aligned
-template <bool ODD>
+// word at a 2-byte aligned shared address, which is a multiple of 4 (SKEW 0), never one (1), or one in some lanes (2)
+template <int SKEW>
 __device__ __forceinline__ uint32_t lds32_skew(uint32_t addr) {
-  if constexpr (!ODD) return lds32(addr);
-  return __funnelshift_r(lds32(addr - 2), lds32(addr + 2), 16);
+  if constexpr (SKEW == 0) return lds32(addr);
+  if constexpr (SKEW == 1) return __funnelshift_r(lds32(addr - 2), lds32(addr + 2), 16);
+  return __funnelshift_r(lds32(addr & ~3u), lds32((addr & ~3u) + 4), (addr & 2u) * 8u);
 }
 
 template <int S, bool TP>
@@ -985,7 +986,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int nb = K >> 8;
-  const uint32_t row_bytes = (uint32_t)nb * 210u;  // a multiple of 4 (nb is even: checked by the launcher)
+  const uint32_t row_bytes = (uint32_t)nb * 210u;  // rows 8 apart lie equally far into a granule; with an odd nb every second row is off a word's boundary
   const uint8_t *w_end = w + (size_t)N * row_bytes;
 
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(dyn) + warp * (S * Q6K_TILE_BYTES);
@@ -1062,8 +1063,8 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float
   if (warp < nb) load_x(warp);
 
   // One unit: rows g, g+8 of one tile x one K block, out of ring slot `sb`.  bl[h][u][i]: B of groups i and 2 + i.
-  auto unit = [&](auto odd_tag, uint32_t sb, uint32_t skew, const uint32_t (&bl)[2][2][2], float up, float (&vr)[2]) {
-    constexpr bool ODD = decltype(odd_tag)::value;
+  auto unit = [&](auto skew_tag, uint32_t sb, uint32_t skew, const uint32_t (&bl)[2][2][2], float up, float (&vr)[2]) {
+    constexpr int SKEW = decltype(skew_tag)::value;
     uint32_t wa[2][4], wc[2][4], wh[2][4], scw[2][2];
     float dd[2];
 #pragma unroll
@@ -1072,11 +1073,11 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float
 #pragma unroll
       for (int hu = 0; hu < 4; hu++) {
         const int h = hu >> 1, u = hu & 1;
-        wa[r][hu] = lds32_skew<ODD>(blk + 4 * (16 * h + 4 * u + t));
-        wc[r][hu] = lds32_skew<ODD>(blk + 4 * (16 * h + 8 + 4 * u + t));
-        wh[r][hu] = lds32_skew<ODD>(blk + 4 * (32 + 8 * h + 4 * u + t));
+        wa[r][hu] = lds32_skew<SKEW>(blk + 4 * (16 * h + 4 * u + t));
+        wc[r][hu] = lds32_skew<SKEW>(blk + 4 * (16 * h + 8 + 4 * u + t));
+        wh[r][hu] = lds32_skew<SKEW>(blk + 4 * (32 + 8 * h + 4 * u + t));
       }
-      scw[r][0] = lds32_skew<ODD>(blk + 192 + 4 * (t >> 1)), scw[r][1] = lds32_skew<ODD>(blk + 200 + 4 * (t >> 1));  // scales of this lane's eight
+      scw[r][0] = lds32_skew<SKEW>(blk + 192 + 4 * (t >> 1)), scw[r][1] = lds32_skew<SKEW>(blk + 200 + 4 * (t >> 1));  // scales of this lane's eight
       dd[r] = f16_bits_to_f32((uint16_t)lds16(blk + 208));
     }
     __syncwarp();  // the slot is free again
@@ -1151,10 +1152,12 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float
         const int r0 = min((gt + rt) * ROWS, N - ROWS);
         const uint32_t skew = ((uint32_t)r0 * row_bytes + (uint32_t)b * 210u + (uint32_t)g * row_bytes) & 15u;
         float vr[2];
-        if (b & 1)
-          unit(std::true_type{}, sb, skew, bl, up, vr);
+        if (nb & 1)
+          unit(std::integral_constant<int, 2>{}, sb, skew, bl, up, vr);
+        else if (b & 1)
+          unit(std::integral_constant<int, 1>{}, sb, skew, bl, up, vr);
         else
-          unit(std::false_type{}, sb, skew, bl, up, vr);
+          unit(std::integral_constant<int, 0>{}, sb, skew, bl, up, vr);
         // the warp's first block of a group overwrites what an earlier group left behind
         const uint32_t ra = red_g + rt * (32 * 8);
         float2 o = make_float2(0.f, 0.f);
@@ -1950,7 +1953,12 @@ static int q4k_launch(const float *x, const MultiArgs &a, const TpArgs &tp, int 
 static const TpArgs NO_TP = {};
 
 int gguf_gemv_fast(int type, const float *x, const void *w, float *out, int M, int N, int K, cudaStream_t st) {
-  if (type == LB200_Q8_0 && M >= 2 && M <= 3) {  // no token-column kernel for this format: a pass per row beats the tensor-core kernel up to three rows
+  // No token-column kernel for Q8_0: a pass per row beats the tensor-core kernel up to three rows.  Nor for Q6_K rows of an odd number of blocks, where it
+  // beats the row kernel (us, that one / a pass per row): 4096 x 11008, 2 and 8 rows 62, 154 / 28, 110, 2048 x 5888, 2, 3 and 8 rows 20.7, 24.9, 45 / 14.6, 23.1, 61, 1024 x
+  // 3328, 3 rows 12.6 / 11.5, but 2048 x 768, 2 rows 4.0 / 4.5; limbs take 8 rows of 16384 x 1280 in 25 us, passes 52.
+  const long long size = (long long)N * K;
+  const bool odd = type == LB200_Q6_K && K % 512 == 256 && !((uintptr_t)w & 15);
+  if (M >= 2 && ((type == LB200_Q8_0 && M <= 3) || (odd && (M <= 3 ? size >= (3ll << 20) : M <= 8 && size >= (20ll << 20) && K >= 4096)))) {
     for (int m = 0; m < M; m++) {
       const int rc = gguf_gemv_fast(type, x + (size_t)m * K, w, out + (size_t)m * N, 1, N, K, st);
       if (rc != 1) return m == 0 ? rc : fail(rc < 0 ? rc : LB200_E_SHAPE, "light_b200: matmul_q (decode): row %d refused after row 0 was launched", m);
@@ -1960,9 +1968,8 @@ int gguf_gemv_fast(int type, const float *x, const void *w, float *out, int M, i
   if (M != 1 || K % 256 || N < ROWS) return 0;
   if (type != LB200_Q4_K && type != LB200_Q6_K && type != LB200_Q8_0) return 0;
   if ((uintptr_t)w & 15) return 0;
-  // Q6_K: an even number of blocks per row keeps every row's skew equal for rows 8 apart and
-  // word-aligned for even blocks; byte offsets are 32-bit
-  if (type == LB200_Q6_K && (((K >> 8) & 1) || (unsigned long long)N * (K >> 8) * 210ull >= (1ull << 32))) return 0;
+  // Q6_K: byte offsets are 32-bit
+  if (type == LB200_Q6_K && (unsigned long long)N * (K >> 8) * 210ull >= (1ull << 32)) return 0;
   const uint8_t *wb = (const uint8_t *)w;
   const int tiles = (N + ROWS - 1) / ROWS;
   if (type == LB200_Q4_K) {
