@@ -121,6 +121,8 @@ LB200_API int light_b200_matmul_q(int ggml_type, const float *x, const void *w, 
  * until the call has run.  Six bytes per activation of up to 4096 rows.  Without, a kernel with f32 products runs that takes about three
  * times as long.  Neither uses the workspace: such calls may overlap on the GPU. */
 LB200_API unsigned long long light_b200_q6k_scratch_bytes(int ggml_type, const void *w, int64_t rows, int K, int grouped);
+/* The same for M rows of one (N, K) matrix, 2 to 64 rows among them (0 where a call has no use for scratch). */
+LB200_API unsigned long long light_b200_matmul_q_scratch_bytes(int ggml_type, const void *w, int64_t M, int64_t N, int K);
 LB200_API int light_b200_matmul_q_scratch(int ggml_type, const float *x, const void *w, float *out, int M, int N, int K, void *scratch,
                                           unsigned long long scratch_bytes, int device, void *stream);
 

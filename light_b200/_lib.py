@@ -79,6 +79,7 @@ SYMBOLS = {
     "light_b200_block_bytes": (C.c_int, [C.c_int]),
     "light_b200_matmul_q": (C.c_int, [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int,
                                       C.c_void_p]),
+    "light_b200_matmul_q_scratch_bytes": (C.c_ulonglong, [C.c_int, C.c_void_p, C.c_int64, C.c_int64, C.c_int]),
     "light_b200_q6k_scratch_bytes": (C.c_ulonglong, [C.c_int, C.c_void_p, C.c_int64, C.c_int, C.c_int]),
     "light_b200_matmul_q_scratch": (C.c_int, [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_ulonglong, C.c_int,
                                               C.c_void_p]),

@@ -170,6 +170,15 @@ unsigned long long light_b200_q6k_scratch_bytes(int t, const void *w, int64_t ro
   return q6k_limbs_bytes(rows, K);
 }
 
+// Of one matrix: as above, and from 60000 outputs on.  The row kernel takes 3.6e-7 us for each weight and activation row, limbs 3 to 5 us for each block of k, whose CTAs
+// share out the outputs: 3072 x 9984, 33 and 64 rows 389, 722 / 157, 227 us, 4096 x 11008, 16 and 64 rows 283, 1056 / 219, 251, 2048 x 5888 33 rows 156 / 133, 1024 x 3328 64 rows
+// 87 / 76, 16384 x 1280, 4 and 16 rows 36, 126 / 25, 32; but 1024 x 3328, 33 and 50 rows 47, 68 / 53, 75, 3072 x 9984 9 rows 132 / 146 (16 rows 191 / 153).
+unsigned long long light_b200_matmul_q_scratch_bytes(int t, const void *w, int64_t M, int64_t N, int K) {
+  if (M > 64) return light_b200_q6k_scratch_bytes(t, w, M, K, 0);
+  if (t != LB200_Q6_K || M < 2 || N < 16 || M * N < 60000 || K <= 0 || K % 256 || ((K >> 8) % 2 == 0 && !((uintptr_t)w & 3))) return 0;
+  return q6k_limbs_bytes(M, K);
+}
+
 int light_b200_matmul_q(int t, const float *x, const void *w, float *out, int M, int N, int K, int device, void *stream) {
   return light_b200_matmul_q_scratch(t, x, w, out, M, N, K, nullptr, 0, device, stream);
 }
@@ -215,6 +224,10 @@ int light_b200_matmul_q_scratch(int t, const float *x, const void *w, float *out
     if (took != 0) return took == 1 ? 0 : took;
     took = gguf_decode_nt(t, x, wv, ov, nv, 1, M, K, ws, wsb, st);
     if (took != 0) return took == 1 ? 0 : took;
+  }
+  if (M <= 64 && scratch) {  // Q6_K rows that start on any even byte
+    const unsigned long long need = light_b200_matmul_q_scratch_bytes(t, w, M, N, K);
+    if (need && scratch_bytes >= need) return q6k_rows_dense(x, w, out, M, N, K, scratch, (size_t)scratch_bytes, st);
   }
   took = gguf_gemv_tok(t, x, w, out, M, N, K, st);
   if (took != 0) return took == 1 ? 0 : took;

@@ -93,7 +93,7 @@ PyObject *linear_q(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
   NEED(be > 0 && N > 0 && K % be == 0 && w.t->scalar_type() == at::kByte && w.t->numel() == N * (K / be) * light_b200_block_bytes((int)type));
   NEED(M == 1 || workspace_fits(dev, M, K));
   at::Tensor out = out_like(*x.t, N), own;
-  const auto own_bytes = light_b200_q6k_scratch_bytes((int)type, w.t->const_data_ptr(), M, (int)K, 0);
+  const auto own_bytes = light_b200_matmul_q_scratch_bytes((int)type, w.t->const_data_ptr(), M, N, (int)K);
   if (own_bytes) own = at::empty({(int64_t)own_bytes}, w.t->options());
   return give(light_b200_matmul_q_scratch((int)type, x.t->const_data_ptr<float>(), w.t->const_data_ptr(), out.data_ptr<float>(), (int)M, (int)N, (int)K,
                                           own_bytes ? own.data_ptr() : nullptr, own_bytes, dev, stream_of(dev)), out);

@@ -157,15 +157,15 @@ def MatMulQ(x: torch.Tensor, w: QTensor) -> torch.Tensor:
     return out
 
 
-def _q6k_scratch(w: QTensor, rows: int, K: int, grouped: bool) -> Optional[torch.Tensor]:
+def _q6k_scratch(w: QTensor, M: int, N: int, K: int) -> Optional[torch.Tensor]:
     """Memory of one call alone (Q6_K rows that start on any even byte; else None): on this stream's part of the caching allocator, so
     that calls on several streams have one each."""
-    n = int(_lib.lib().light_b200_q6k_scratch_bytes(w.ggml_type, _ptr(w.data), rows, K, int(grouped)))
+    n = int(_lib.lib().light_b200_matmul_q_scratch_bytes(w.ggml_type, _ptr(w.data), M, N, K))
     return torch.empty(n, dtype=torch.uint8, device=w.device) if n else None
 
 
 def _matmul_q(x: torch.Tensor, w: QTensor, out: torch.Tensor, M: int, N: int, K: int, dev: int) -> None:
-    own = _q6k_scratch(w, M, K, False)
+    own = _q6k_scratch(w, M, N, K)
     _lib.check(_lib.lib().light_b200_matmul_q_scratch(w.ggml_type, _ptr(x), _ptr(w.data), _ptr(out), M, N, K, _ptr(own), 0 if own is None else own.numel(), dev,
                                                       _stream(dev)))
 
