@@ -962,6 +962,11 @@ constexpr int Q6K_TILE_BYTES = ROWS * Q6K_PITCH;
 constexpr int Q6K_STAGES = 2;
 constexpr int Q6K_SX = LIMB_BYTES, Q6K_SLAB = Q6K_SX + 16 * 16;  // a block's limbs, and -32 x the four limb sums of each sub-block
 
+__device__ __forceinline__ uint32_t lds8(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u8 %0, [%1];\n" : "=r"(v) : "r"(addr));
+  return v;
+}
 __device__ __forceinline__ uint32_t lds16(uint32_t addr) {
   uint16_t v;
   asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(v) : "r"(addr));
@@ -975,13 +980,15 @@ __device__ __forceinline__ uint32_t lds32_skew(uint32_t addr) {
   return __funnelshift_r(lds32(addr & ~3u), lds32((addr & ~3u) + 4), (addr & 2u) * 8u);
 }
 
-template <int S, bool TP>
+// ODD: an odd number of blocks to a row (a kernel of its own: as a branch of this one it cost the others 1 % of a decode step).
+template <int S, bool TP, bool ODD = false>
 __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float *__restrict__ x,
                                                                     const uint8_t *__restrict__ w,
                                                                     float *__restrict__ out, const __grid_constant__ TpArgs tp,
                                                                     int N, int K) {
   extern __shared__ __align__(16) unsigned char dyn[];  // ring: WARPS x S tiles
   __shared__ __align__(16) unsigned char slabs[WARPS][Q6K_SLAB];
+  [[maybe_unused]] __shared__ __align__(8) uint2 rests[ODD ? WARPS : 1][ODD ? 256 : 1];  // elements, and what their fixed point leaves out
   __shared__ __align__(16) float2 red[2][WARPS * GROUP * 32];  // by group parity
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -1125,6 +1132,20 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float
       __syncwarp();  // every lane is done reading the previous block's slab
       float xs[2][4];
       const float up = stage_limbs(xv, slab, lane, xs);
+      [[maybe_unused]] int nrest = 0;
+      if constexpr (ODD) {
+        // The f32 products that these rows had keep every bit of a small activation beside a large one.  Fixed point keeps those above 2^-31 of the block's largest;
+        // the rest, of one element in forty with normal inputs, is multiplied on its own.  A block with an infinity or a NaN goes that way whole.
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const float v = j == 0 ? xv[i].x : j == 1 ? xv[i].y : j == 2 ? xv[i].z : xv[i].w, rest = up == up ? xs[i][j] - rintf(xs[i][j]) : v;
+            const unsigned some = __ballot_sync(0xffffffffu, rest != 0.f);  // (a NaN among them)
+            if (rest != 0.f) rests[warp][nrest + __popc(some & ((1u << lane) - 1u))] = make_uint2(128 * i + 4 * lane + j, __float_as_uint(rest));
+            nrest += __popc(some);
+          }
+      }
       __syncwarp();
       {  // -32 times the sum of each limb over each sub-block: lane l adds up limbs 2 (l & 1), 2 (l & 1) + 1 of sub-block l >> 1
         int sum[2];
@@ -1152,12 +1173,28 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q6k_gemv_mma_kernel(const float
         const int r0 = min((gt + rt) * ROWS, N - ROWS);
         const uint32_t skew = ((uint32_t)r0 * row_bytes + (uint32_t)b * 210u + (uint32_t)g * row_bytes) & 15u;
         float vr[2];
-        if (nb & 1)
+        if constexpr (ODD) {
+          float c[2];
+#pragma unroll
+          for (int r = 0; r < 2; r++) {
+            const uint32_t blk = sb + (g + 8 * r) * Q6K_PITCH + skew;
+            float v = 0.f;
+            for (int i = t; i < nrest; i += 4) {  // (each lane of a row a quarter)
+              const uint2 e = rests[warp][i];
+              const uint32_t h = e.x >> 7, q = (e.x >> 5) & 3, l = e.x & 31;
+              const uint32_t code = ((lds8(blk + 64 * h + 32 * (q & 1) + l) >> (4 * (q >> 1))) & 15u) | ((lds8(blk + 128 + 32 * h + l) >> (2 * q)) & 3u) << 4;
+              const int sc = (int)(int8_t)lds8(blk + 192 + 8 * h + 2 * q + (l >> 4));
+              v = fmaf(__uint_as_float(e.y), (float)(sc * ((int)code - 32)), v);
+            }
+            c[r] = v * f16_bits_to_f32((uint16_t)lds16(blk + 208));
+          }
           unit(std::integral_constant<int, 2>{}, sb, skew, bl, up, vr);
-        else if (b & 1)
-          unit(std::integral_constant<int, 1>{}, sb, skew, bl, up, vr);
-        else
-          unit(std::integral_constant<int, 0>{}, sb, skew, bl, up, vr);
+#pragma unroll
+          for (int r = 0; r < 2; r++) vr[r] = up == up ? fmaf(c[r], up, vr[r]) : c[r];
+        } else {
+          if (b & 1) unit(std::integral_constant<int, 1>{}, sb, skew, bl, up, vr);
+          else unit(std::integral_constant<int, 0>{}, sb, skew, bl, up, vr);
+        }
         // the warp's first block of a group overwrites what an earlier group left behind
         const uint32_t ra = red_g + rt * (32 * 8);
         float2 o = make_float2(0.f, 0.f);
@@ -1917,6 +1954,9 @@ int gguf_gemv_fast_init(int device) {
     err = cudaFuncSetAttribute(q6k_gemv_mma_kernel<Q6K_STAGES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                WARPS * Q6K_STAGES * Q6K_TILE_BYTES);
   if (err == cudaSuccess)
+    err = cudaFuncSetAttribute(q6k_gemv_mma_kernel<Q6K_STAGES, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               WARPS * Q6K_STAGES * Q6K_TILE_BYTES);
+  if (err == cudaSuccess)
     err = cudaFuncSetAttribute(q80_gemv_mma_kernel<Q80_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, WARPS * Q80_STAGES * Q80_TILE_BYTES);
   if (err == cudaSuccess)
     err = cudaFuncSetAttribute(q6k_gemv_mma_kernel<Q6K_STAGES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1954,11 +1994,12 @@ static const TpArgs NO_TP = {};
 
 int gguf_gemv_fast(int type, const float *x, const void *w, float *out, int M, int N, int K, cudaStream_t st) {
   // No token-column kernel for Q8_0: a pass per row beats the tensor-core kernel up to three rows.  Nor for Q6_K rows of an odd number of blocks, where it
-  // beats the row kernel (us, that one / a pass per row): 4096 x 11008, 2 and 8 rows 62, 154 / 28, 110, 2048 x 5888, 2, 3 and 8 rows 20.7, 24.9, 45 / 14.6, 23.1, 61, 1024 x
-  // 3328, 3 rows 12.6 / 11.5, but 2048 x 768, 2 rows 4.0 / 4.5; limbs take 8 rows of 16384 x 1280 in 25 us, passes 52.
+  // beats the row kernel (us, that one / a pass per row): 4096 x 11008, 2, 3 and 8 rows 62, 68, 154 / 34, 50, 134, 3072 x 9984, 8 rows 123 / 119, 1024 x 3328, 2 and 3 rows 10.5, 12.6 /
+  // 9.2, 13.9, 2048 x 5888 20.7, 24.9 / 19.0, 28.5, 2048 x 768, 2 rows 4.0 / 5.4; limbs take 8 rows of 16384 x 1280 in 25 us, passes 66.
   const long long size = (long long)N * K;
   const bool odd = type == LB200_Q6_K && K % 512 == 256 && !((uintptr_t)w & 15);
-  if (M >= 2 && ((type == LB200_Q8_0 && M <= 3) || (odd && (M <= 3 ? size >= (3ll << 20) : M <= 8 && size >= (20ll << 20) && K >= 4096)))) {
+  const bool passes = type == LB200_Q8_0 ? M <= 3 : odd && (M == 2 ? size >= (3ll << 20) : size >= (20ll << 20) && (M == 3 || (M <= 8 && K >= 4096)));
+  if (M >= 2 && passes) {
     for (int m = 0; m < M; m++) {
       const int rc = gguf_gemv_fast(type, x + (size_t)m * K, w, out + (size_t)m * N, 1, N, K, st);
       if (rc != 1) return m == 0 ? rc : fail(rc < 0 ? rc : LB200_E_SHAPE, "light_b200: matmul_q (decode): row %d refused after row 0 was launched", m);
@@ -1984,7 +2025,8 @@ int gguf_gemv_fast(int type, const float *x, const void *w, float *out, int M, i
     rc = launched("matmul_q (decode)");
     return rc ? rc : 1;
   }
-  int rc = launch_pdl(q6k_gemv_mma_kernel<Q6K_STAGES, false>, grid, (size_t)WARPS * Q6K_STAGES * Q6K_TILE_BYTES, st, x, wb, out, NO_TP, N, K);
+  int rc = odd ? launch_pdl(q6k_gemv_mma_kernel<Q6K_STAGES, false, true>, grid, (size_t)WARPS * Q6K_STAGES * Q6K_TILE_BYTES, st, x, wb, out, NO_TP, N, K)
+               : launch_pdl(q6k_gemv_mma_kernel<Q6K_STAGES, false>, grid, (size_t)WARPS * Q6K_STAGES * Q6K_TILE_BYTES, st, x, wb, out, NO_TP, N, K);
   if (rc) return rc;
   rc = launched("matmul_q (decode)");
   return rc ? rc : 1;

@@ -31,7 +31,7 @@ def test_one_row(cuda, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(2, 1024, 3328), (3, 1024, 3328), (4, 1024, 3328), (2, 2048, 768), (8, 3072, 9984), (9, 3072, 9984), (16, 3072, 9984), (4, 16384, 1280), (64, 930, 768), (64, 940, 768),
-                                   (33, 1850, 256), (17, 4100, 2816), (3, 15, 768), (64, 15, 768)])
+                                   (33, 1850, 256), (17, 4100, 2816), (3, 15, 768), (64, 15, 768), (1, 3072, 256), (1, 2048, 768)])
 def test_few_rows(cuda, M, N, K):
     _check(cuda, M, N, K)
 
@@ -53,3 +53,34 @@ def test_infinities_and_nan(cuda):
     keep = [m for m in range(40) if m not in (7, 20)]
     assert torch.equal(y[keep], clean[keep])
     assert not torch.isfinite(y[20]).any() and not torch.isfinite(y[7]).any()
+
+
+@pytest.mark.parametrize("M", [1, 2])
+@pytest.mark.parametrize("large", [1e3, 1e6, -3e30])
+def test_small_activations_beside_a_large_one(cuda, M, large):
+    """Outputs whose weights are zero at the large elements: what the others give keeps its f32 accuracy."""
+    N, K = 6000, 768
+    w = ops.QTensor(synth.gaussian_weight(9, ops.Q6_K, N, K, device=cuda).reshape(-1), ops.Q6_K, (N, K))
+    deq = ops.Dequantize(w).double()
+    x = torch.randn(M, K, generator=torch.Generator(device=cuda).manual_seed(3), device=cuda) * 0.05
+    x[:, 130] = large
+    rows = deq[:, 130] == 0
+    assert int(rows.sum()) > 20
+    want = x.double() @ deq.t()
+    got = ops.MatMulQ(x, w)
+    assert rel_l2(got[:, rows].cpu().double().numpy(), want[:, rows].cpu().numpy()) <= 3e-7
+    assert rel_l2(got.cpu().double().numpy(), want.cpu().numpy()) <= 3e-7
+
+
+def test_one_row_with_infinities_and_nan(cuda):
+    """As plain f32 arithmetic over the dequantized weights has it, infinity times zero among it."""
+    N, K = 4096, 1280
+    w = ops.QTensor(synth.gaussian_weight(11, ops.Q6_K, N, K, device=cuda).reshape(-1), ops.Q6_K, (N, K))
+    deq = ops.Dequantize(w)
+    x = torch.randn(1, K, generator=torch.Generator(device=cuda).manual_seed(3), device=cuda)
+    for at, v in ((300, float("inf")), (301, float("-inf")), (5, float("nan"))):
+        z = x.clone()
+        z[0, at] = v
+        y, want = ops.MatMulQ(z, w), (z.double() @ deq.double().t()).float()
+        assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isinf(y), torch.isinf(want))
+        assert torch.equal(y[torch.isinf(y)], want[torch.isinf(want)])
