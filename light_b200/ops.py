@@ -521,10 +521,12 @@ def RouterLogits(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     y = _host.router_logits(x, w)
     if y is not None:
         return y
+    if x.device != w.device:
+        raise ValueError(f"router_logits: x on {x.device} but w on {w.device}")
     dev = _dev(x, "RouterLogits")
+    xc, wc = x.contiguous(), w.contiguous()  # (named: a copy whose address alone is kept is gone before the next one is made)
     out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
-    _lib.check(_lib.lib().light_b200_router_logits(_ptr(x.contiguous()), _ACT[x.dtype], _ptr(w.contiguous()), _ptr(out), x.shape[0], w.shape[0], x.shape[1], dev,
-                                                   _stream(dev)))
+    _lib.check(_lib.lib().light_b200_router_logits(_ptr(xc), _ACT[x.dtype], _ptr(wc), _ptr(out), x.shape[0], w.shape[0], x.shape[1], dev, _stream(dev)))
     return out
 
 

@@ -48,3 +48,17 @@ def test_sparse_block_takes_the_same_route(cuda):
     z = moe.forward(x)
     assert torch.allclose(seen[0], seen[1], rtol=1e-5, atol=1e-5) and seen[1].requires_grad and not seen[0].requires_grad
     assert torch.equal(y, z)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_operands_that_are_not_contiguous(cuda, dtype):
+    g = torch.Generator(device=cuda).manual_seed(2)
+    x, w = torch.randn(512, 256, generator=g, device=cuda).to(dtype), torch.randn(512, 256, generator=g, device=cuda)
+    xs, ws = x.t().contiguous().t(), w.t().contiguous().t()
+    want = ops.RouterLogits(x, w)
+    assert torch.equal(ops.RouterLogits(xs, ws), want) and torch.equal(ops.RouterLogits(x, ws), want) and torch.equal(ops.RouterLogits(xs, w), want)
+
+
+def test_a_weight_on_the_host(cuda):
+    with pytest.raises(ValueError, match="router_logits: x on cuda:0 but w on cpu"):
+        ops.RouterLogits(torch.zeros(4, 8, device=cuda), torch.zeros(4, 8))
