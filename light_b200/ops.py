@@ -101,6 +101,12 @@ def _ptr(t: Optional[torch.Tensor]) -> C.c_void_p:
     return C.c_void_p(0 if t is None else t.data_ptr())
 
 
+def _whole(*ts: Optional[torch.Tensor]) -> list:
+    """The tensors as contiguous ones, for the caller to hold until its call returns.  (A copy of which nothing but the address is kept is freed at once: the
+    next copy or output, or another thread's, may take its memory before the kernel has read it.)"""
+    return [None if t is None else t.contiguous() for t in ts]
+
+
 # --------------------------------------------------------------------------- workspace
 
 _workspaces = {}  # device index -> torch uint8 buffer handed to the library
@@ -269,9 +275,9 @@ def GatedLinear(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, gelu: bool 
         if w.dim() != 2 or w.shape[1] != K or w.shape[0] != wg.shape[0] or w.dtype != torch.bfloat16 or w.device != x.device:
             raise ValueError(f"GatedLinear: weights must be (N, {K}) BF16 on {x.device}, got {tuple(wg.shape)} / {tuple(wu.shape)}")
     dev = _dev(x, "GatedLinear")
+    xc, wgc, wuc = _whole(x, wg, wu)
     out = torch.empty(tuple(x.shape[:-1]) + (wg.shape[0],), dtype=torch.bfloat16, device=x.device)
-    _lib.check(_lib.lib().light_b200_gemv_gated(_ptr(x.contiguous()), _ptr(wg.contiguous()), _ptr(wu.contiguous()), _ptr(out), wg.shape[0], K,
-                                                int(gelu), dev, _stream(dev)))
+    _lib.check(_lib.lib().light_b200_gemv_gated(_ptr(xc), _ptr(wgc), _ptr(wuc), _ptr(out), wg.shape[0], K, int(gelu), dev, _stream(dev)))
     return out
 
 
@@ -331,8 +337,8 @@ def MatMulW8A8(x: torch.Tensor, wq: torch.Tensor, ws: torch.Tensor) -> torch.Ten
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
     xq = torch.empty((M, K), dtype=torch.int8, device=x.device)
     xs = torch.empty((M,), dtype=torch.float32, device=x.device)
-    _lib.check(_lib.lib().light_b200_matmul_w8a8(_ptr(x.contiguous()), _ptr(wq.contiguous()), _ptr(ws.contiguous()), _ptr(out), _ptr(xq), _ptr(xs),
-                                                 M, N, K, dev, _stream(dev)))
+    xc, wc, wsc = _whole(x, wq, ws)
+    _lib.check(_lib.lib().light_b200_matmul_w8a8(_ptr(xc), _ptr(wc), _ptr(wsc), _ptr(out), _ptr(xq), _ptr(xs), M, N, K, dev, _stream(dev)))
     return out
 
 
@@ -369,8 +375,8 @@ def Int4FromCheckpoint(qweight: torch.Tensor, qzeros: torch.Tensor, scales: torc
     codes = torch.empty((N, K // 8), dtype=torch.int32, device=qweight.device)
     s = torch.empty((N, K // group), dtype=torch.float32, device=qweight.device)
     z = torch.empty_like(s)
-    _lib.check(_lib.lib().light_b200_int4_repack(_ptr(qweight.contiguous()), _ptr(qzeros.contiguous()), _ptr(scales.contiguous()), _ptr(codes),
-                                                 _ptr(s), _ptr(z), N, K, group, kind, dev, _stream(dev)))
+    qw, qz, sc = _whole(qweight, qzeros, scales)
+    _lib.check(_lib.lib().light_b200_int4_repack(_ptr(qw), _ptr(qz), _ptr(sc), _ptr(codes), _ptr(s), _ptr(z), N, K, group, kind, dev, _stream(dev)))
     return Int4(codes, s, z, group)
 
 
@@ -384,9 +390,9 @@ def DequantizeInt4(w: Int4, out_dtype: torch.dtype, out: Optional[torch.Tensor] 
     dev = _dev(w.codes, "DequantizeInt4")
     if out is None:
         out = torch.zeros((w.N(), w.K()), dtype=out_dtype, device=w.codes.device)
-    _lib.check(_lib.lib().light_b200_int4_dequant(_ptr(w.codes.contiguous()), _ptr(w.scales.contiguous()),
-                                                  _ptr(w.zeros.contiguous()), _ptr(out), _ACT[out_dtype], w.N(), w.K(),
-                                                  w.group, offset, dev, _stream(dev)))
+    codes, scales, zeros = _whole(w.codes, w.scales, w.zeros)
+    _lib.check(_lib.lib().light_b200_int4_dequant(_ptr(codes), _ptr(scales), _ptr(zeros), _ptr(out), _ACT[out_dtype], w.N(), w.K(), w.group, offset, dev,
+                                                  _stream(dev)))
     return out
 
 
@@ -396,8 +402,8 @@ def GatherColumns(x: torch.Tensor, idx: torch.Tensor) -> torch.Tensor:
         raise ValueError(f"gather_columns: x {tuple(x.shape)} {x.dtype}, idx {tuple(idx.shape)} {idx.dtype}")
     dev = _dev(x, "GatherColumns")
     out = torch.empty_like(x, memory_format=torch.contiguous_format)
-    _lib.check(_lib.lib().light_b200_gather_columns(_ptr(x.contiguous()), _ptr(idx.contiguous()), _ptr(out), _ACT[x.dtype], x.shape[0], x.shape[1], dev,
-                                                    _stream(dev)))
+    xc, ic = _whole(x, idx)
+    _lib.check(_lib.lib().light_b200_gather_columns(_ptr(xc), _ptr(ic), _ptr(out), _ACT[x.dtype], x.shape[0], x.shape[1], dev, _stream(dev)))
     return out
 
 
@@ -454,9 +460,8 @@ def MatMulInt4(x: torch.Tensor, w: Int4) -> torch.Tensor:
         # token tiles over activations staged once
         ensure_workspace(dev, int(_lib.lib().light_b200_matmul_q_workspace_bytes(M, w.K())))
     out = torch.zeros((M, N), dtype=x.dtype, device=x.device)
-    _lib.check(_lib.lib().light_b200_int4_gemv(_ptr(xc), _ptr(w.codes.contiguous()), _ptr(w.scales.contiguous()),
-                                               _ptr(w.zeros.contiguous()), _ptr(out), _ACT[x.dtype], M, N, w.K(),
-                                               w.group, dev, _stream(dev)))
+    codes, scales, zeros = _whole(w.codes, w.scales, w.zeros)
+    _lib.check(_lib.lib().light_b200_int4_gemv(_ptr(xc), _ptr(codes), _ptr(scales), _ptr(zeros), _ptr(out), _ACT[x.dtype], M, N, w.K(), w.group, dev, _stream(dev)))
     return out
 
 
@@ -476,8 +481,8 @@ def DequantizeF8Block(w: torch.Tensor, scale: torch.Tensor, block_r: int, block_
     out = torch.empty((R, Cc), dtype=out_dtype, device=w.device)
     if out_dtype not in (torch.float32, torch.bfloat16):
         raise ValueError(f"ops.DequantizeF8Block: output {out_dtype}, want F32 or BF16")
-    _lib.check(_lib.lib().light_b200_fp8_block_dequant(_ptr(w.contiguous()), _ptr(scale.contiguous()), _ptr(out),
-                                                       _ACT[out_dtype], R, Cc, block_r, block_c, dev, _stream(dev)))
+    wc, sc = _whole(w, scale)
+    _lib.check(_lib.lib().light_b200_fp8_block_dequant(_ptr(wc), _ptr(sc), _ptr(out), _ACT[out_dtype], R, Cc, block_r, block_c, dev, _stream(dev)))
     return out
 
 
@@ -497,9 +502,8 @@ def MatMulF8Block(x: torch.Tensor, w: torch.Tensor, scale: torch.Tensor, block_r
     if M > 64 or (4 <= M and x.dtype == torch.bfloat16):  # (as in MatMulInt4)
         ensure_workspace(dev, int(_lib.lib().light_b200_matmul_q_workspace_bytes(M, K)))
     out = torch.zeros((M, N), dtype=x.dtype, device=x.device)
-    _lib.check(_lib.lib().light_b200_fp8_block_gemv(_ptr(x.contiguous()), _ptr(w.contiguous()),
-                                                    _ptr(scale.contiguous()), _ptr(out), _ACT[x.dtype], M, N, K,
-                                                    block_r, block_c, dev, _stream(dev)))
+    xc, wc, sc = _whole(x, w, scale)
+    _lib.check(_lib.lib().light_b200_fp8_block_gemv(_ptr(xc), _ptr(wc), _ptr(sc), _ptr(out), _ACT[x.dtype], M, N, K, block_r, block_c, dev, _stream(dev)))
     return out
 
 
@@ -524,7 +528,7 @@ def RouterLogits(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     if x.device != w.device:
         raise ValueError(f"router_logits: x on {x.device} but w on {w.device}")
     dev = _dev(x, "RouterLogits")
-    xc, wc = x.contiguous(), w.contiguous()  # (named: a copy whose address alone is kept is gone before the next one is made)
+    xc, wc = _whole(x, w)
     out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
     _lib.check(_lib.lib().light_b200_router_logits(_ptr(xc), _ACT[x.dtype], _ptr(wc), _ptr(out), x.shape[0], w.shape[0], x.shape[1], dev, _stream(dev)))
     return out
@@ -545,7 +549,8 @@ def MoERoute(probs: torch.Tensor, topk: int, normalize: bool) -> MoERouting:
     dev = _dev(probs, "MoERoute")
     ids = torch.empty((T, topk), dtype=torch.int64, device=probs.device)
     w = torch.empty((T, topk), dtype=torch.float32, device=probs.device)
-    _lib.check(_lib.lib().light_b200_moe_route_topk(_ptr(probs.contiguous()), _ptr(ids), _ptr(w), T, E, topk, int(normalize), dev, _stream(dev)))
+    pc, = _whole(probs)
+    _lib.check(_lib.lib().light_b200_moe_route_topk(_ptr(pc), _ptr(ids), _ptr(w), T, E, topk, int(normalize), dev, _stream(dev)))
     sp, se, _, _ = MoESortPairs(ids.reshape(-1), E)
     return MoERouting(ids, w.reshape(-1), sp, se)
 
@@ -565,8 +570,8 @@ def MoERouteDeepseek(logits: torch.Tensor, bias: Optional[torch.Tensor], topk: i
     dev = _dev(logits, "MoERouteDeepseek")
     ids = torch.empty((T, topk), dtype=torch.int64, device=logits.device)
     w = torch.empty((T, topk), dtype=torch.float32, device=logits.device)
-    _lib.check(_lib.lib().light_b200_moe_route_deepseek(_ptr(logits.contiguous()), _ptr(None if bias is None else bias.contiguous()), _ptr(ids), _ptr(w),
-                                                        T, E, topk, n_group, topk_group, int(sigmoid), int(norm_topk), dev, _stream(dev)))
+    lc, bc = _whole(logits, bias)
+    _lib.check(_lib.lib().light_b200_moe_route_deepseek(_ptr(lc), _ptr(bc), _ptr(ids), _ptr(w), T, E, topk, n_group, topk_group, int(sigmoid), int(norm_topk), dev, _stream(dev)))
     sp, se, _, _ = MoESortPairs(ids.reshape(-1), E)
     return MoERouting(ids, w.reshape(-1), sp, se)
 
@@ -585,8 +590,8 @@ def MoERouteSigmoid(logits: torch.Tensor, bias: Optional[torch.Tensor], topk: in
     dev = _dev(logits, "MoERouteSigmoid")
     ids = torch.empty((T, topk), dtype=torch.int64, device=logits.device)
     w = torch.empty((T, topk), dtype=torch.float32, device=logits.device)
-    _lib.check(_lib.lib().light_b200_moe_route_sigmoid(_ptr(logits.contiguous()), _ptr(None if bias is None else bias.contiguous()), _ptr(ids),
-                                                       _ptr(w), T, E, topk, int(norm_topk), dev, _stream(dev)))
+    lc, bc = _whole(logits, bias)
+    _lib.check(_lib.lib().light_b200_moe_route_sigmoid(_ptr(lc), _ptr(bc), _ptr(ids), _ptr(w), T, E, topk, int(norm_topk), dev, _stream(dev)))
     sp, se, _, _ = MoESortPairs(ids.reshape(-1), E)
     return MoERouting(ids, w.reshape(-1), sp, se)
 
@@ -601,7 +606,8 @@ def MoESortPairs(ids: torch.Tensor, E: int):
     counts = torch.empty(E, dtype=torch.int32, device=ids.device)
     offsets = torch.empty(E + 1, dtype=torch.int32, device=ids.device)
     scratch = torch.empty(M + (M + 1023) // 1024 * E + 1, dtype=torch.int32, device=ids.device)
-    _lib.check(_lib.lib().light_b200_moe_sort_pairs(_ptr(ids.contiguous()), _ptr(counts), _ptr(offsets), _ptr(sp), _ptr(se), _ptr(scratch), M, E, dev,
+    ic, = _whole(ids)
+    _lib.check(_lib.lib().light_b200_moe_sort_pairs(_ptr(ic), _ptr(counts), _ptr(offsets), _ptr(sp), _ptr(se), _ptr(scratch), M, E, dev,
                                                     _stream(dev)))
     return sp, se, counts, offsets
 
@@ -632,7 +638,7 @@ def _moe_dispatch(op: str, key_dtype: int, quant: bool, inp: torch.Tensor, weigh
     if topk_weights is not None and (topk_weights.dtype != torch.float32 or topk_weights.numel() != M):
         raise ValueError(f"{op}: topkWeights must be F32 with {M} elements")
     dev = _dev(inp, op)
-    inc = inp.contiguous()
+    inc, pairs, expts, tw = _whole(inp, routing.sorted_pairs, routing.sorted_expts, topk_weights)
     own = None
     if M >= 256:  # tensor-core grouped path: the token rows gathered in expert order, and behind them the partial tiles
         ensure_workspace(dev, int(_lib.lib().light_b200_matmul_q_workspace_bytes(M, K)))
@@ -641,10 +647,8 @@ def _moe_dispatch(op: str, key_dtype: int, quant: bool, inp: torch.Tensor, weigh
     counts = torch.zeros(E, dtype=torch.int32, device=inp.device)
     offsets = torch.zeros(E + 1, dtype=torch.int32, device=inp.device)
     out = torch.zeros((M, N), dtype=out_dtype, device=inp.device)
-    a = MoeArgs(input=inc.data_ptr(), weights=weights.data_ptr(), sorted_pairs=routing.sorted_pairs.contiguous().data_ptr(),
-                expert_ids=routing.sorted_expts.contiguous().data_ptr(), counts=counts.data_ptr(),
-                offsets=offsets.data_ptr(),
-                topk_weights=0 if topk_weights is None else topk_weights.contiguous().data_ptr(), out=out.data_ptr(),
+    a = MoeArgs(input=inc.data_ptr(), weights=weights.data_ptr(), sorted_pairs=pairs.data_ptr(), expert_ids=expts.data_ptr(), counts=counts.data_ptr(),
+                offsets=offsets.data_ptr(), topk_weights=0 if tw is None else tw.data_ptr(), out=out.data_ptr(),
                 M=M, size_m=M, E=E, N=N, K=K, topk=topk, row_per_pair=int(row_per_pair), dtype=key_dtype)
     if quant:
         own = None
@@ -723,7 +727,8 @@ def MoECombine(pair_out: torch.Tensor, topk: int) -> torch.Tensor:
         raise ValueError(f"moe_combine: dtype {pair_out.dtype} / N {N} (a multiple of 8) unsupported")
     dev = _dev(pair_out, "MoECombine")
     out = torch.empty((M // topk, N), dtype=pair_out.dtype, device=pair_out.device)
-    _lib.check(_lib.lib().light_b200_moe_combine(_ptr(pair_out.contiguous()), _ptr(out), _ACT[pair_out.dtype], M // topk, N, topk, dev, _stream(dev)))
+    pc, = _whole(pair_out)
+    _lib.check(_lib.lib().light_b200_moe_combine(_ptr(pc), _ptr(out), _ACT[pair_out.dtype], M // topk, N, topk, dev, _stream(dev)))
     return out
 
 
@@ -741,11 +746,10 @@ def MoECombineWeighted(rows: torch.Tensor, index: Optional[torch.Tensor], weight
     if index is None and rows.shape[0] < M:
         raise ValueError(f"moe_combine_weighted: {rows.shape[0]} rows for {M} pairs and no index")
     dev = _dev(rows, "MoECombineWeighted")
-    rows = rows.contiguous()
+    rows, ic, wc = _whole(rows, index, weights)
     out = torch.empty((tokens, rows.shape[1]), dtype=torch.float32, device=rows.device)
-    _lib.check(_lib.lib().light_b200_moe_combine_weighted(_ptr(rows), _ptr(None if index is None else index.contiguous()),
-                                                          _ptr(None if weights is None else weights.contiguous()), _ptr(out), _ACT[rows.dtype],
-                                                          tokens, rows.shape[1], topk, rows.shape[0], dev, _stream(dev)))
+    _lib.check(_lib.lib().light_b200_moe_combine_weighted(_ptr(rows), _ptr(ic), _ptr(wc), _ptr(out), _ACT[rows.dtype], tokens, rows.shape[1], topk, rows.shape[0],
+                                                          dev, _stream(dev)))
     return out
 
 
@@ -760,7 +764,8 @@ def MoEGateMul(h: torch.Tensor, gelu: bool = False) -> torch.Tensor:
     M, I2 = h.shape
     dev = _dev(h, "MoEGateMul")
     out = torch.empty((M, I2 // 2), dtype=h.dtype, device=h.device)
-    _lib.check(_lib.lib().light_b200_moe_gate_mul(_ptr(h.contiguous()), _ptr(out), _ACT[h.dtype], M, I2 // 2, int(gelu), dev, _stream(dev)))
+    hc, = _whole(h)
+    _lib.check(_lib.lib().light_b200_moe_gate_mul(_ptr(hc), _ptr(out), _ACT[h.dtype], M, I2 // 2, int(gelu), dev, _stream(dev)))
     return out
 
 
@@ -793,7 +798,8 @@ def KVAppend(kbuf: torch.Tensor, vbuf: torch.Tensor, k: torch.Tensor, v: torch.T
     _check_pos(pos, kbuf, "KVAppend")
     dev = _dev(kbuf, "KVAppend")
     B, KH, cap, D = kbuf.shape
-    _lib.check(_lib.lib().light_b200_kv_append(_ptr(k.contiguous()), _ptr(v.contiguous()), _ptr(kbuf), _ptr(vbuf), _ptr(pos),
+    kc, vc = _whole(k, v)
+    _lib.check(_lib.lib().light_b200_kv_append(_ptr(kc), _ptr(vc), _ptr(kbuf), _ptr(vbuf), _ptr(pos),
                                                _ACT[k.dtype], B, KH, D, cap, dev, _stream(dev)))
 
 
@@ -877,9 +883,9 @@ def RoPE(x: torch.Tensor, positions: torch.Tensor, base: float) -> torch.Tensor:
     if positions.shape[0] != seq_len:
         raise ValueError(f"ops.RoPE: positions length {positions.shape[0]} != seqLen {seq_len}")
     dev = _dev(x, "RoPE")
-    xc = x.contiguous()
+    xc, pc = _whole(x, positions)
     out = torch.empty_like(xc)
-    _lib.check(_lib.lib().light_b200_rope(_ptr(xc), _ptr(positions.contiguous()), _ptr(out), _ACT[x.dtype], xc.numel() // head_dim, seq_len,
+    _lib.check(_lib.lib().light_b200_rope(_ptr(xc), _ptr(pc), _ptr(out), _ACT[x.dtype], xc.numel() // head_dim, seq_len,
                                           head_dim, float(base), dev, _stream(dev)))
     return out
 
