@@ -10,9 +10,13 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <atomic>
 
@@ -32,6 +36,12 @@ struct Arg {
 };
 
 bool cuda_contig(const at::Tensor &t) { return t.is_cuda() && t.is_contiguous() && !t.requires_grad(); }
+// Whether something beside the result is to come of an operator of torch's on this tensor (a forward-mode tangent), or somebody is to see it: function
+// transforms, torch-function and dispatch modes, tracing.  For operators that stand in for one of torch's.
+bool watched(const at::Tensor &t) {
+  return t._fw_grad(0).defined() || c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) ||
+         at::impl::PythonTorchFunctionTLS::stack_len() > 0 || c10::impl::TorchDispatchModeTLS::any_modes_set() || torch::jit::tracer::isTracing();
+}
 bool long_of(PyObject *o, long long &v) {
   if (!PyLong_Check(o)) return false;
   int overflow;
@@ -138,7 +148,7 @@ PyObject *linear_f8(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
 PyObject *router_logits(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
   ARGS(2)
   Arg x, w;
-  NEED(x.ok(a[0]) && w.ok(a[1]) && x.t->dim() == 2 && w.t->dim() == 2 && cuda_contig(*x.t) && cuda_contig(*w.t) && w.t->scalar_type() == at::kFloat);
+  NEED(x.ok(a[0]) && w.ok(a[1]) && !watched(*x.t) && !watched(*w.t) && x.t->dim() == 2 && w.t->dim() == 2 && cuda_contig(*x.t) && cuda_contig(*w.t) && w.t->scalar_type() == at::kFloat);
   const auto dt = x.t->scalar_type();
   const long long T = x.t->size(0), E = w.t->size(0), K = x.t->size(1);
   NEED((dt == at::kBFloat16 || (dt == at::kFloat && T * E <= 1ll << 18)) && T > 0 && T <= 1ll << 21 && E > 0 && E < 1ll << 31 && K > 0 && K < 1ll << 31 && K % 8 == 0 && w.t->size(1) == K &&

@@ -160,10 +160,13 @@ class SparseMoE:
         return ops.MoERoute(torch.softmax(logits, -1), self.TopK, self.NormTopK)
 
     def _logits_here(self, x: torch.Tensor) -> Optional[torch.Tensor]:
-        """The router's matmul as ops.RouterLogits: a plain F32 gate on rows that it takes as they are, with nothing for autograd to record; else None."""
+        """The router's matmul as ops.RouterLogits: a plain F32 gate on rows that it takes as they are, where nothing is to see the matmul or to take its place
+        (a route or a gate's forward of the program's own, on the class or on the object; autograd in either direction, transforms and modes: host.cpp);
+        else None."""
         g = self.Gate
         w = g.W
-        if type(self).route is not SparseMoE.route or type(g) is not Linear or g.B is not None or g.W4 is not None or type(w) is not torch.Tensor or type(x) is not torch.Tensor or \
+        if getattr(self.route, "__func__", None) is not _ROUTE or type(g) is not Linear or getattr(g.forward, "__func__", None) is not _LINEAR or g.B is not None or \
+                g.W4 is not None or type(w) is not torch.Tensor or type(x) is not torch.Tensor or \
                 not (x.dtype == torch.float32 or (self.RouterF32 and x.dtype == torch.bfloat16)) or tuple(w.shape) != (g.out_features, g.in_features) or \
                 torch.is_autocast_enabled("cuda"):
             return None
@@ -184,3 +187,6 @@ class SparseMoE:
         h = gemm(flat, gu, None)                          # (M, 2 I)
         pair = gemm(ops.MoEGateMul(h, self.Gelu), dn, route.weights)   # (M, H), routing-weighted
         return ops.MoECombine(pair, self.TopK)            # (T, H)
+
+
+_LINEAR, _ROUTE = Linear.forward, SparseMoE.route

@@ -62,3 +62,52 @@ def test_operands_that_are_not_contiguous(cuda, dtype):
 def test_a_weight_on_the_host(cuda):
     with pytest.raises(ValueError, match="router_logits: x on cuda:0 but w on cpu"):
         ops.RouterLogits(torch.zeros(4, 8, device=cuda), torch.zeros(4, 8))
+
+
+def _block(cuda):
+    g = torch.Generator(device=cuda).manual_seed(4)
+    moe = nn.SparseMoE(nn.Linear(64, 8, W=torch.randn(8, 64, generator=g, device=cuda)), TopK=2, Router=lambda logits: logits)
+    moe.run_experts = lambda flat, route: torch.cat([route] * 8, 1)  # (the block's output is its logits, eight times)
+    return moe, torch.randn(40, 64, generator=g, device=cuda), g
+
+
+def test_tangents_reach_the_router(cuda):
+    import torch.autograd.forward_ad as fwd
+
+    moe, x, g = _block(cuda)
+    t = torch.randn(40, 64, generator=g, device=cuda)
+    with fwd.dual_level():
+        value, tangent = fwd.unpack_dual(moe.forward(fwd.make_dual(x, t)))
+    assert tangent is not None and torch.equal(tangent[:, :8], t @ moe.Gate.W.t()) and torch.equal(value[:, :8], x @ moe.Gate.W.t())
+
+
+def test_function_transforms(cuda):
+    moe, x, _ = _block(cuda)
+    want = torch.cat([x @ moe.Gate.W.t()] * 8, 1)
+    assert torch.allclose(torch.vmap(lambda v: moe.forward(v[None])[0])(x), want, rtol=1e-5, atol=1e-5)
+    value, tangent = torch.func.jvp(moe.forward, (x,), (x,))
+    assert torch.allclose(value, want) and torch.allclose(tangent, want)
+
+
+def test_modes_see_the_matmul(cuda):
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    seen = []
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    class Function(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(getattr(func, "__name__", ""))
+            return func(*args, **(kwargs or {}))
+
+    moe, x, _ = _block(cuda)
+    for mode, name in ((Dispatch, "mm"), (Function, "matmul")):
+        seen.clear()
+        with mode():
+            moe.forward(x)
+        assert any(name in s for s in seen), seen
