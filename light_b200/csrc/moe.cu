@@ -370,9 +370,12 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) q6k_rows_kernel(const float
 // What bounds q6k_rows_kernel is f32 issue: eight multiply-adds per lane, token and weight row for every block.  Here an activation is the sum
 // of three f16 values (LIMBS), and a code is exact in f16.  The first limb is a whole number of 2^-8 of the power of two above the largest
 // of the block's 256, so that its sums are exact; the second and third are the rest, rounded to eleven bits and again.  An activation above
-// 2^-9 of that power so keeps all its bits, one below 23 of its own, down to 2^-38: f32 products hold 24.  (In fixed point to the
+// 2^-9 of that power so keeps all its bits, one below 23 of its own, down to 2^-37: f32 products hold 24.  (In fixed point to the
 // end, the third limb 2^-30 of that power, small activations lost bits: 512 outputs of 768 whose weights are zero at one
-// element of 1000 beside N(0, 0.05) were 5.5e-6 off; 9.5e-8 now, 8.9e-8 with f32 products.)  One MMA (m16n8k16: 16 rows, 8 tokens, one limb) is a sub-block's sum: three of
+// element of 1000 beside N(0, 0.05) were 5.5e-6 off; 9.5e-8 now, 8.9e-8 with f32 products.)  Below 2^-37 of it an element is off by up to 2^-52 of the
+// first limb's unit, all 256 of a block together by up to 2^-32 of that unit times |d| (a weight is at most 2^12 |d|).  Such blocks carry a mark (ups is negative), and
+// an output that is not 2^25 times as large as what its marked blocks may have lost is multiplied again, element by element: its weights are zero, or cancel, at the
+// large activations (beside 1e12 such outputs were 6.3e-6 off, beside 3e30 nothing was left of them).  One MMA (m16n8k16: 16 rows, 8 tokens, one limb) is a sub-block's sum: three of
 // them and 12 f32 operations a lane (limbs together, times the sub-block's scale) replace 64 multiply-adds.  Building
 // the operand takes some 900 of the 1665 instructions per 16 rows, block and 16 tokens, and issue is what bounds this kernel
 // (63 % of the slots, the tensor pipe 24 %).
@@ -381,7 +384,7 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) q6k_rows_kernel(const float
 //   f32 products are 8.1e-8 to 1.59e-7 off (K = 256 to 14080; without, 1.1e-7 at 11008).
 // Tried: limbs of eight bits and the integer MMAs (m16n8k32), 194 us and 19.5 ms: they run at a fraction of the f16 rate here; limbs
 // straight from L2, 152 us and 8.8 ms; 32 rows to a warp and half the warps, 115 us and 5.5 ms.
-// Tokens with infinities or NaN (whose limbs mean nothing; their power of two is NaN) are multiplied again in f32.
+// Tokens with infinities or NaN (whose limbs mean nothing; their power of two is NaN) are too.
 constexpr int LIMB_RECORD = 1536;  // a token's block: [sub-block][t][limbs 0, 1 of four k], then [sub-block][t][limb 2 of four k]
 constexpr int LIMB_CHUNK = 4096;   // rows whose limbs are kept at a time: six bytes per activation
 constexpr int LIMB_PASS = 16, LIMB_WARPS = 8, LIMB_RT = 1, LIMB_ROWS = 16 * LIMB_RT;
@@ -413,7 +416,16 @@ __global__ void __launch_bounds__(256) x_limbs_kernel(const float *__restrict__ 
   m = __reduce_max_sync(0xffffffffu, m);
   const int s = min(156 - (int)(m >> 23), 126);  // |x| 2^s < 2^30
   const float scale = __uint_as_float((uint32_t)(127 + s) << 23);
-  if (lane == 0) ups[rec] = m >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : __uint_as_float((uint32_t)(149 - s) << 23);  // of the first limb: 2^22
+  bool small = false;  // an element other than zero below 2^-37 of the power of two above the largest
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const float e[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) small |= e[k] != 0.f && fabsf(e[k] * scale) < 0x1p-7f;
+  }
+  small = __any_sync(0xffffffffu, small);
+  const uint32_t unit = (uint32_t)(149 - s) << 23 | (small ? 0x80000000u : 0u);  // of the first limb: 2^22
+  if (lane == 0) ups[rec] = __uint_as_float(m >= 0x7f800000u ? 0x7fc00000u : unit);
   uint8_t *dst = limbs + (size_t)rec * LIMB_RECORD;
 #pragma unroll
   for (int j = 0; j < 2; j++) {  // elements 128 j + 4 lane ..: sub-block 8 j + lane / 4, t = lane % 4
@@ -499,6 +511,7 @@ __global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const flo
     float acc[LIMB_RT][2][4], rest[LIMB_RT][2][4];  // [16 rows][group][rows g, g + 8 x tokens 2 t, 2 t + 1]: sum, and what its roundings left out
 #pragma unroll
     for (int i = 0; i < 8 * LIMB_RT; i++) acc[i >> 3][(i >> 2) & 1][i & 3] = rest[i >> 3][(i >> 2) & 1][i & 3] = 0.f;
+    float lost[2 * LIMB_RT][2][2] = {};  // [row][group][token] marked blocks: unit of the first limb times |d|
     int slot = 0;
     for (int b = 0; b < nb; b++) {
       issue(b + LIMB_RING - 1, slot == 0 ? LIMB_RING - 1 : slot - 1);
@@ -585,10 +598,11 @@ __global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const flo
         for (int j = 0; j < 2; j++)
 #pragma unroll
           for (int c = 0; c < 2; c++) {
+            lost[r][j][c] = fmaf(fmaxf(-two_to[j][c], 0.f), fabsf(d), lost[r][j][c]);
             // acc + d 2^.. (top + 2^-27 low), the roundings of both products and of both sums kept (d 2^.. has eleven bits: exact)
             const int i = 2 * (r & 1) + c;
             float &y = acc[r >> 1][j][i];
-            const float s = d * two_to[j][c], l = low[r >> 1][j][i] * 0x1p-27f, v = s * top[r >> 1][j][i], w = fmaf(s, l, v), t = y + w, z = t - y;
+            const float s = d * fabsf(two_to[j][c]), l = low[r >> 1][j][i] * 0x1p-27f, v = s * top[r >> 1][j][i], w = fmaf(s, l, v), t = y + w, z = t - y;
             rest[r >> 1][j][i] += ((y - (t - z)) + (w - z)) + (fmaf(s, l, v - w) + fmaf(s, top[r >> 1][j][i], -v));
             y = t;
           }
@@ -609,33 +623,42 @@ __global__ void __launch_bounds__(LIMB_WARPS * 32, 2) q6k_limbs_kernel(const flo
           p = pairs ? pairs[t0 + mine] : t0 + mine;
           if (p >= size_m) p = -1;
         }
-        bool nan = false;
+        bool again[2 * LIMB_RT] = {};  // not a number, or too small beside what may be lost (of a row by itself: a row that two warps have comes out alike)
         if (p >= 0) {
           const float f = topkw ? topkw[p] : 1.f;
 #pragma unroll
           for (int r = 0; r < 2 * LIMB_RT; r++) {
             const float y = acc[r >> 1][j][2 * (r & 1) + c] + rest[r >> 1][j][2 * (r & 1) + c];
-            nan |= y != y;
+            again[r] = !(fabsf(y) >= 0x1p-7f * lost[r][j][c]);
             out[p * N + r0 + g + 8 * r] = topkw ? y * f : y;
           }
         }
-        unsigned odd = __ballot_sync(0xffffffffu, nan);
-        while (odd) {  // not a number: this token's rows once more, one after the other
-          const int tt = (__ffs(odd) - 1) & 3;
-          odd &= ~(0x11111111u << tt);  // (the lanes of that token)
+        unsigned odd[2 * LIMB_RT], left = 0;
+#pragma unroll
+        for (int r = 0; r < 2 * LIMB_RT; r++) odd[r] = __ballot_sync(0xffffffffu, again[r]), left |= odd[r];
+        while (left) {  // those rows of a token once more, one after the other
+          const int tt = (__ffs(left) - 1) & 3;
+          left &= ~(0x11111111u << tt);  // (the lanes of that token: row g + 8 r is lane 4 g + tt's)
           const long long i = t0 + 8 * j + 2 * tt + c, q = pairs ? pairs[i] : i;
           const float4 *x = reinterpret_cast<const float4 *>(in + (size_t)(row_per_pair ? q : q / topk) * K) + lane;
           __syncwarp();  // (after the stores above)
           for (int r = 0; r < LIMB_ROWS; r++) {
-            float y = 0.f;
+            unsigned which = odd[0];
+#pragma unroll
+            for (int h = 1; h < 2 * LIMB_RT; h++) which = r >> 3 == h ? odd[h] : which;
+            if (!(which >> (4 * (r & 7) + tt) & 1u)) continue;
+            double sum = 0.;  // (in f32 one after the other they would be further off than limbs are where little is lost: 3.4e-7 at K = 11008)
             for (int b = 0; b < nb; b++) {
               float wv[8];
               q6k_eight(rows + r * row_bytes + (size_t)b * 210, lane, wv);
               const float4 u = __ldg(x + b * 64), v = __ldg(x + b * 64 + 32);
-              y = fmaf(wv[0], u.x, y), y = fmaf(wv[1], u.y, y), y = fmaf(wv[2], u.z, y), y = fmaf(wv[3], u.w, y);
-              y = fmaf(wv[4], v.x, y), y = fmaf(wv[5], v.y, y), y = fmaf(wv[6], v.z, y), y = fmaf(wv[7], v.w, y);
+              const float xv[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+#pragma unroll
+              for (int k = 0; k < 8; k++) sum = fma((double)wv[k], (double)xv[k], sum);
             }
-            y = warp_sum(y);
+#pragma unroll
+            for (int o = 16; o >= 1; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            const float y = (float)sum;
             if (lane == 0) out[q * N + r0 + r] = topkw ? y * topkw[q] : y;
           }
         }

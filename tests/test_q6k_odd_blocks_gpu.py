@@ -84,3 +84,43 @@ def test_one_row_with_infinities_and_nan(cuda):
         y, want = ops.MatMulQ(z, w), (z.double() @ deq.double().t()).float()
         assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isinf(y), torch.isinf(want))
         assert torch.equal(y[torch.isinf(y)], want[torch.isinf(want)])
+
+
+def _outlier(cuda, M, K, large):
+    x = torch.randn(M, K, generator=torch.Generator(device=cuda).manual_seed(3), device=cuda) * 0.05
+    x[:, 130] = large
+    x[M // 2] = 0
+    return x
+
+
+@pytest.mark.parametrize("M,N", [(4, 16000), (16, 6000), (40, 6000), (64, 6000), (65, 2000), (100, 2000)])
+@pytest.mark.parametrize("large", [1e3, 1e6, 1e10, 1e12, -3e30])
+def test_limbs_of_small_activations_beside_a_large_one(cuda, M, N, large):
+    """As above, where the products are those of limbs: from 60000 outputs on."""
+    K = 768
+    w = ops.QTensor(synth.gaussian_weight(9, ops.Q6_K, N, K, device=cuda).reshape(-1), ops.Q6_K, (N, K))
+    deq, x = ops.Dequantize(w).double(), _outlier(cuda, M, K, large)
+    rows = deq[:, 130] == 0
+    assert int(rows.sum()) > 20
+    got, want = ops.MatMulQ(x, w), x.double() @ deq.t()
+    assert rel_l2(got[:, rows].cpu().double().numpy(), want[:, rows].cpu().numpy()) <= 3e-7
+    assert rel_l2(got.cpu().double().numpy(), want.cpu().numpy()) <= 3e-7
+    assert not got[M // 2].any() and torch.equal(got, ops.MatMulQ(x, w))
+
+
+@pytest.mark.parametrize("large", [1e3, 1e12, -3e30])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_grouped_limbs_of_small_activations_beside_a_large_one(cuda, large, weighted):
+    E, N, K, T, topk = 5, 1500, 768, 150, 2
+    w = ops.QTensor(synth.gaussian_weight(9, ops.Q6_K, E * N, K, device=cuda).reshape(-1), ops.Q6_K, (E, N, K))
+    deq, x = ops.Dequantize(w).double(), _outlier(cuda, T, K, large)
+    g = torch.Generator(device=cuda).manual_seed(8)
+    ids = torch.rand(T, E, generator=g, device=cuda).topk(topk, -1).indices
+    tw = torch.rand(T * topk, generator=g, device=cuda) + 0.5
+    route = ops.MoERouteFromIDs(ids, tw, T, topk)
+    got = ops.MoEGemmQ(x, w, route, tw if weighted else None, topk).double()
+    e = ids.reshape(-1)
+    want = torch.stack([deq[int(e[p])] @ x[p // topk].double() * (float(tw[p]) if weighted else 1.0) for p in range(T * topk)])
+    off = deq[e, :, 130] == 0
+    assert int(off.sum()) > 1000
+    assert float((got - want)[off].norm() / want[off].norm()) <= 3e-7 and float((got - want).norm() / want.norm()) <= 3e-7
