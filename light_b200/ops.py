@@ -210,7 +210,8 @@ def MatMulQMulti(x: torch.Tensor, ws: Sequence[QTensor], outs: Optional[Sequence
     nn = (C.c_int32 * n)(*[w.shape[0] for w in ws])
     if M > 1:
         ensure_workspace(dev, int(_lib.lib().light_b200_matmul_q_workspace_bytes(M, K)))
-    if M > 64 and ws[0].ggml_type == Q6_K and all(w.shape[0] > 0 for w in ws):  # a launch per matrix as it is, and some have use for memory of their own
+    if ws[0].ggml_type == Q6_K and M > 1 and all(w.shape[0] > 0 for w in ws) and \
+            any(_lib.lib().light_b200_matmul_q_scratch_bytes(Q6_K, _ptr(w.data), M, w.shape[0], K) for w in ws):  # some have use for memory of their own
         for w, o in zip(ws, outs):
             _matmul_q(xc, w, o, M, w.shape[0], K, dev)
         return list(outs)

@@ -124,3 +124,13 @@ def test_grouped_limbs_of_small_activations_beside_a_large_one(cuda, large, weig
     off = deq[e, :, 130] == 0
     assert int(off.sum()) > 1000
     assert float((got - want)[off].norm() / want[off].norm()) <= 3e-7 and float((got - want).norm() / want.norm()) <= 3e-7
+
+
+@pytest.mark.parametrize("M", [2, 8, 40, 64, 65])
+def test_several_matrices_in_one_call(cuda, M):
+    """Each gives what it gives alone, bit for bit."""
+    K, sizes = 3328, (1600, 96, 2000)
+    ws = [ops.QTensor(synth.gaussian_weight(n, ops.Q6_K, n, K, device=cuda).reshape(-1), ops.Q6_K, (n, K)) for n in sizes]
+    x = torch.randn(M, K, generator=torch.Generator(device=cuda).manual_seed(M), device=cuda)
+    for y, w in zip(ops.MatMulQMulti(x, ws), ws):
+        assert torch.equal(y, ops.MatMulQ(x, w))
