@@ -26,13 +26,14 @@ struct alignas(16) Vec8 {  // eight elements: one 16-byte access (bf16 / f16) or
 __device__ __forceinline__ long long div_by(long long n, long long d, bool small) {
   return small ? (long long)((uint32_t)n / (uint32_t)d) : n / d;
 }
-// n / d for a d of 1 or more: reciprocal, product and one correction by the remainder (P. Markstein, IBM J. Res. Dev. 34 (1990)), within one ulp.  Where an
-// infinity makes the remainder a NaN (d after exp overflows, n itself), the product is the quotient.
+// n / d for a d of 1 or more: reciprocal, product and one correction by the remainder (P. Markstein, IBM J. Res. Dev. 34 (1990)); as 1 + exp(-n) is used here, the
+// division's bits for every one of the 2^32 n (compared one by one).  Where an infinity makes the remainder a NaN (d after exp overflows, n itself), the
+// product is the quotient; the correction of a zero loses its sign, which is n's.
 __device__ __forceinline__ float quotient(float n, float d) {
   float r;
   asm("rcp.approx.f32 %0, %1;\n" : "=f"(r) : "f"(d));
   const float q = n * r, c = fmaf(fmaf(-q, d, n), r, q);
-  return c == c ? c : q;
+  return copysignf(c == c ? c : q, n);
 }
 
 // h (M, 2 I): gate = h[:, :I], up = h[:, I:] -> out (M, I) = act(gate) * up; eight elements per thread

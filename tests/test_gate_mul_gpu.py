@@ -28,3 +28,22 @@ def test_extremes(cuda):
     assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isinf(y), torch.isinf(want))
     ok = torch.isfinite(want)
     assert bool(((y - want)[ok].abs() <= 4e-7 * want[ok].abs() + 2.0**-148).all())
+
+
+def test_bits_of_the_division(cuda):
+    """f32 gates of every exponent and both signs, zeros and infinities among them (every 1021st bit pattern): the bits that a correctly rounded division gives."""
+    bits = torch.arange(-2**31, 2**31, 1021, device=cuda, dtype=torch.int64)
+    v = torch.cat([bits.to(torch.int32).view(torch.float32), torch.tensor([0.0, -0.0, float("inf"), float("-inf")], device=cuda)])
+    v = torch.cat([v, v.new_full((-v.numel() % 8,), -0.0)]).reshape(-1, 8)
+    y, want = ops.MoEGateMul(torch.cat([v, torch.ones_like(v)], 1)), v / (1 + torch.exp(-v))
+    assert torch.equal(torch.isnan(y), torch.isnan(want))
+    number = ~torch.isnan(want)
+    assert torch.equal(y.view(torch.int32)[number], want.view(torch.int32)[number])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_zeros_keep_their_sign(cuda, dtype):
+    v = torch.tensor([0.0, -0.0] * 4, device=cuda, dtype=dtype)
+    for u in (1.0, -1.0):
+        y = ops.MoEGateMul(torch.cat([v, torch.full_like(v, u)])[None])[0]
+        assert torch.equal(torch.signbit(y), torch.signbit(v * u)) and not y.any()
