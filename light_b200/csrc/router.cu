@@ -24,6 +24,10 @@ namespace {
 constexpr int RT_KC = 32, RT_THREADS = 128;
 constexpr int RT_PITCH32 = 160, RT_PITCH16 = 80;  // bytes of a staged row of 32 f32 / bf16: an operand's reads meet every bank once
 
+// Operands are split 2^24 times as large as they are, so that the last bit of the smallest f32 (2^-149) still has its place in a normal bf16; as they are, operands
+// below 2^-109 lost theirs (w of 2^-120: 2e-5 of an output).  What leaves f32's range that way is not finite, and made again.
+constexpr float SPLIT_UP = 0x1p24f;
+
 struct RouterArgs {
   const void *x;
   const float *w;
@@ -37,14 +41,18 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// two f32 as three pairs of bf16 each, largest first
+// two f32 times SPLIT_UP as three pairs of bf16 each, largest first (sm_100 multiplies and adds two f32 with one instruction)
 __device__ __forceinline__ void split3(uint2 v, uint32_t (&p)[3]) {
-  float a = __uint_as_float(v.x), b = __uint_as_float(v.y);
+  uint64_t ab;
+  asm("{\n\t.reg .b64 x, up;\n\tmov.b64 x, {%1, %2};\n\tmov.b64 up, {%3, %3};\n\tmul.rn.f32x2 %0, x, up;\n\t}\n" : "=l"(ab) : "r"(v.x), "r"(v.y), "f"(SPLIT_UP));
 #pragma unroll
   for (int i = 0; i < 3; i++) {
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(a), "=f"(b) : "l"(ab));
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     p[i] = *reinterpret_cast<const uint32_t *>(&h);
-    a -= __uint_as_float(p[i] << 16), b -= __uint_as_float(p[i] & 0xFFFF0000u);
+    if (i < 2)  // what is left: exact
+      asm("{\n\t.reg .b64 h, m;\n\tmov.b64 h, {%1, %2};\n\tmov.b64 m, {%3, %3};\n\tfma.rn.f32x2 %0, h, m, %0;\n\t}\n" : "+l"(ab) : "r"(p[i] << 16), "r"(p[i] & 0xFFFF0000u), "f"(-1.f));
   }
 }
 
@@ -146,6 +154,8 @@ __global__ void __launch_bounds__(RT_THREADS, STAGES == 3 ? 4 : 3) router_kernel
       const float *w = a.w + (size_t)e * a.K;
       v = 0.f;
       for (int k = 0; k < a.K; k++) v = fmaf(ld_act(x, k), w[k], v);
+    } else {
+      v *= F32 ? 1.f / (SPLIT_UP * SPLIT_UP) : 1.f / SPLIT_UP;
     }
     a.out[(size_t)m * a.E + e] = v;
   }

@@ -111,3 +111,15 @@ def test_modes_see_the_matmul(cuda):
         with mode():
             moe.forward(x)
         assert any(name in s for s in seen), seen
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("of_x,of_w", [(0, -100), (0, -112), (0, -120), (-20, -100), (-112, 0), (-120, 0), (-130, 8), (-60, -60), (60, -118), (60, 40)])
+@pytest.mark.parametrize("T", [5, 70])
+def test_powers_of_two(cuda, dtype, of_x, of_w, T):
+    """Small operands keep their bits, down to subnormal ones; a sum is within the bound above, and an output's own last place where that is subnormal."""
+    g = torch.Generator(device=cuda).manual_seed(T)
+    x, w = (torch.randn(T, 512, generator=g, device=cuda) * 2.0**of_x).to(dtype), torch.randn(72, 512, generator=g, device=cuda) * 2.0**of_w
+    y = ops.RouterLogits(x, w).double()
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert float(want.abs().max()) > 0 and bool(((y - want).abs() <= 2e-6 * size + 2.0**-149).all())
