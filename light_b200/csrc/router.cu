@@ -6,9 +6,9 @@
 // largest products for f32 ones (what is left out is below 2^-26 of a product).  The tensor core's own sum is kept to 32 k, smallest terms first, and added to the
 // running sum in f32.  The error against 64 bits is a fifth to two thirds of the library's f32 matmul (K = 1024 to 7168).  Splitting the weights takes about
 // as many issue slots as the MMAs take clocks, and both are re-read for every 64 tokens.
-//   us, the library (with the pass to f32 for bf16) / here:  bf16 4096 x 256 x 7168 370 / 203, 1024 x 128 x 4096 82 / 27, 32 x 256 x 7168 54 / 23, 8 x 256 x 7168
-//   26.7 / 11.9;  f32 77 x 128 x 2048 24.7 / 12.9, 300 x 200 x 3072 64 / 24, 2048 x 64 x 2048 37 / 18, 1024 x 256 x 4096 78 / 58, but 4096 x 128 x 4096
-//   110 / 106, 2500 x 200 x 1536 47 / 74, 4096 x 256 x 4096 166 / 203: f32 rows come here up to 2^18 logits (host.cpp).
+//   us, the library (with the pass to f32 for bf16) / here:  bf16 4096 x 256 x 7168 369 / 212, 1024 x 128 x 4096 79 / 26, 32 x 256 x 7168 53 / 12.9, 8 x 256 x 7168
+//   22.3 / 11.4;  f32 77 x 128 x 2048 20.3 / 7.3, 300 x 200 x 3072 59 / 24, 2048 x 64 x 2048 38 / 20, 1024 x 256 x 4096 76 / 59, 4096 x 128 x 4096 119 / 114, but 3000 x
+//   200 x 1536 69 / 80, 4096 x 256 x 4096 170 / 214: which calls of a sparse block come here is nn.py's choice.
 //
 // A CTA holds a tile of BM tokens x BN experts and a share of K; the CTAs of a cluster hold the others and add up through each other's shared memory, in their
 // order.  A sum that is not finite (an infinity times the zero rest of another operand is no number) is made again by multiply-adds.
@@ -189,10 +189,16 @@ int go(const RouterArgs &a, cudaStream_t st) {
 
 }  // namespace
 
+// Tiles of 16 tokens by 32 experts while they take no more than 512 CTAs with their shares of K (about as many as the GPU holds of them at once), of 64 by 64
+// beyond.  us, 64 x 64 / 16 x 32 (tokens x experts x K):  f32 17 x 64 x 256 12.6 / 5.2, 77 x 128 x 2048 12.7 / 7.3, 256 x 256 x 512 15.8 / 7.6, 512 x 8 x 4096 21.4 /
+// 15.0, 1024 x 64 x 1024 13.8 / 13.6;  bf16 32 x 256 x 7168 23.7 / 12.9, 64 x 256 x 7168 23.9 / 15.4, 512 x 64 x 2048 9.9 / 8.5;  but f32 512 x 64 x 4096 21.8 / 23.3, 256 x 256 x
+// 2048 17.7 / 23.6, bf16 700 x 64 x 2048 11.0 / 11.9, 1024 x 256 x 2048 27.0 / 48.0.  (64 x 64 from 17 tokens on took longer than the library's matmul where K is
+// short: f32 17 x 64 x 256 12.6, the library 7.1.)
 int router_logits(const void *x, int dtype, const float *w, float *out, int T, int E, int K, cudaStream_t st) {
   if (T == 0 || E == 0) return 0;
   const RouterArgs a{x, w, out, T, E, K};
-  if (T <= 16) return dtype == LB200_F32 ? go<float, 1, 1, 1>(a, st) : go<__nv_bfloat16, 1, 1, 1>(a, st);
+  const long long narrow = ((long long)T + 15) / 16 * ((E + 31) / 32);
+  if (narrow * (K < 2048 ? K : 2048) <= 64 * 2048) return dtype == LB200_F32 ? go<float, 1, 1, 1>(a, st) : go<__nv_bfloat16, 1, 1, 1>(a, st);
   if (dtype == LB200_F32) return go<float, 2, 2, 4>(a, st);
   // Where the tiles fill the GPU, four CTAs of three chunks each to an SM (4096 x 256 x 7168: 226 -> 203 us), else three of four (1024 x 128 x 4096: 31.7 ->
   // 26.6): with a CTA or two to an SM the chunks on their way are what hides the latency.

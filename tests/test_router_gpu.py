@@ -123,3 +123,9 @@ def test_powers_of_two(cuda, dtype, of_x, of_w, T):
     y = ops.RouterLogits(x, w).double()
     want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
     assert float(want.abs().max()) > 0 and bool(((y - want).abs() <= 2e-6 * size + 2.0**-149).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,E,K", [(16, 513, 7168), (17, 33, 256), (64, 512, 2048), (65, 512, 2048), (1024, 64, 2040), (1025, 64, 1024), (8192, 32, 256), (8193, 32, 256), (1, 1, 8)])
+def test_both_sides_of_the_tiles(cuda, dtype, T, E, K):
+    test_against_64_bits(cuda, dtype, T, E, K)
