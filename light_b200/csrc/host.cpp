@@ -144,14 +144,14 @@ PyObject *linear_f8(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
                                         act_of(*x.t), (int)M, (int)N, (int)K, (int)bR, (int)bC, dev, stream_of(dev)), out);
 }
 
-// (x (T, K) F32 / BF16, w (E, K) F32) -> (T, E) F32.  F32 rows up to 2^18 logits: beyond, the library's f32 matmul is the faster one (router.cu).
+// (x (T, K) F32 / BF16, w (E, K) F32) -> (T, E) F32
 PyObject *router_logits(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
   ARGS(2)
   Arg x, w;
   NEED(x.ok(a[0]) && w.ok(a[1]) && !watched(*x.t) && !watched(*w.t) && x.t->dim() == 2 && w.t->dim() == 2 && cuda_contig(*x.t) && cuda_contig(*w.t) && w.t->scalar_type() == at::kFloat);
   const auto dt = x.t->scalar_type();
   const long long T = x.t->size(0), E = w.t->size(0), K = x.t->size(1);
-  NEED((dt == at::kBFloat16 || (dt == at::kFloat && T * E <= 1ll << 18)) && T > 0 && T <= 1ll << 21 && E > 0 && E < 1ll << 31 && K > 0 && K < 1ll << 31 && K % 8 == 0 && w.t->size(1) == K &&
+  NEED((dt == at::kBFloat16 || dt == at::kFloat) && T > 0 && T <= 1ll << 21 && E > 0 && E < 1ll << 31 && K > 0 && K < 1ll << 31 && K % 8 == 0 && w.t->size(1) == K &&
        w.t->get_device() == x.t->get_device());
   const void *const xp = x.t->const_data_ptr();
   const float *const wp = w.t->const_data_ptr<float>();

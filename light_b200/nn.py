@@ -116,6 +116,28 @@ class Linear:
         return y.reshape(*x.shape[:-1], self.out_features)
 
 
+def _router_is_faster(T: int, E: int, K: int, f32: bool) -> bool:
+    """Whether ops.RouterLogits takes less time than the library's f32 matmul does, with its pass over bf16 tokens to f32 (us, the library / here, tokens x experts x K).
+    One token is the library's matrix-vector product: f32 1 x 64 x 2048 7.5 / 5.7, 1 x 256 x 1024 6.7 / 5.8, but 1 x 256 x 2048 5.2 / 6.1, 1 x 64 x 4096 7.8 / 9.3, 1 x 64 x 512
+    3.6 / 6.0; bf16 1 x 256 x 4096 8.0 / 7.6, but 1 x 256 x 7168 9.2 / 11.4.  Short rows leave the tensor cores little to do beside the launch: f32 16 x 256 x 256 3.9 / 5.2, 512 x 256 x 768
+    15.6 / 20.3, bf16 4096 x 40 x 256 13.2 / 25.0.  Few experts leave most of a tile of 64 of them empty: f32 1500 x 8 x 1280 19.7 / 22.6, bf16 4096 x 4 x 512
+    19.8 / 26.0, 8192 x 8 x 1280 53 / 56.  F32 tokens cost six products to a weight where the library has one multiply-add: past 2^18 places in the tiles 3000 x 200 x 1536
+    69 / 80 (4096 x 64 x 4096 1.5 times as fast here)."""
+    wide, narrow = -(-T // 64) * -(-E // 64), -(-T // 16) * -(-E // 32)
+    short = narrow * K <= 1 << 17  # (tiles of 16 x 32 even so: router.cu)
+    if f32:
+        if T == 1:
+            return 1024 <= K < 1280 or (E <= 64 and 2048 <= K <= 3072)
+        if K < 1024:
+            return 16 < T <= 1024 and short and wide * 4096 <= 192 * K
+        return wide <= 64 and (E > 16 or K >= 2048 or T <= 1024)
+    if T == 1:
+        return K <= 3072 or (K <= 5120 and E * K <= 1 << 20)
+    if K < 512:
+        return short and T <= 2000
+    return E > 32 or K >= 2048 or T <= (4 * K if K < 1024 else 6 * K if E <= 16 else T)
+
+
 @dataclass
 class SparseMoE:
     """Routed gated-MLP block (nn/moe.go:27-60).  `GateUp` (E, 2 I, H) holds every expert's gate rows then up rows,
@@ -160,15 +182,15 @@ class SparseMoE:
         return ops.MoERoute(torch.softmax(logits, -1), self.TopK, self.NormTopK)
 
     def _logits_here(self, x: torch.Tensor) -> Optional[torch.Tensor]:
-        """The router's matmul as ops.RouterLogits: a plain F32 gate on rows that it takes as they are, where nothing is to see the matmul or to take its place
-        (a route or a gate's forward of the program's own, on the class or on the object; autograd in either direction, transforms and modes: host.cpp);
-        else None."""
+        """The router's matmul as ops.RouterLogits: a plain F32 gate on rows that it takes as they are, of a size where it is the faster one, where nothing is to
+        see the matmul or to take its place (a route or a gate's forward of the program's own, on the class or on the object; autograd in either direction, transforms and
+        modes: host.cpp); else None."""
         g = self.Gate
         w = g.W
         if getattr(self.route, "__func__", None) is not _ROUTE or type(g) is not Linear or getattr(g.forward, "__func__", None) is not _LINEAR or g.B is not None or \
                 g.W4 is not None or type(w) is not torch.Tensor or type(x) is not torch.Tensor or \
                 not (x.dtype == torch.float32 or (self.RouterF32 and x.dtype == torch.bfloat16)) or tuple(w.shape) != (g.out_features, g.in_features) or \
-                torch.is_autocast_enabled("cuda"):
+                torch.is_autocast_enabled("cuda") or not _router_is_faster(x.shape[0], *w.shape, x.dtype == torch.float32):
             return None
         return ops._host.router_logits(x, w)
 

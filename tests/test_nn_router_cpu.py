@@ -7,7 +7,7 @@ import torch
 
 from light_b200 import nn, ops
 
-H, E = 32, 8
+H, E = 1024, 8
 
 
 def _block(cls=nn.SparseMoE, gate=None):
@@ -73,3 +73,19 @@ def test_on_the_class(native, monkeypatch, cls, name):
     monkeypatch.setattr(cls, name, lambda self, v: 2 * plain(self, v))
     moe, x = _block()
     assert torch.equal(moe.forward(x), 2 * (x @ moe.Gate.W.t()).sum() + x) and not native
+
+
+@pytest.mark.parametrize("T,E,K,f32,bf16", [(1, 64, 2048, True, True), (1, 256, 2048, False, True), (1, 256, 1024, True, True), (1, 64, 7168, False, False), (1, 256, 7168, False, False),
+                                            (8, 256, 7168, True, True), (77, 128, 2048, True, True), (17, 64, 256, True, True), (16, 64, 256, False, True), (512, 256, 768, False, True),
+                                            (1024, 8, 1280, True, True), (1500, 8, 1280, False, True), (4096, 64, 1024, True, True), (4097, 64, 4096, False, True), (4096, 256, 7168, False, True),
+                                            (4096, 4, 512, False, False), (8192, 8, 1280, False, False), (4096, 40, 256, False, False), (16384, 8, 2560, False, True)])
+def test_sizes_where_it_is_the_faster_one(T, E, K, f32, bf16):
+    assert nn._router_is_faster(T, E, K, True) == f32 and nn._router_is_faster(T, E, K, False) == bf16
+
+
+def test_a_size_where_the_library_is(native):
+    g = torch.Generator().manual_seed(2)
+    moe = nn.SparseMoE(nn.Linear(64, E, W=torch.randn(E, 64, generator=g)), TopK=2, Router=lambda logits: logits)
+    moe.run_experts = lambda flat, route: route.sum() + flat
+    x = torch.randn(3, 64, generator=g)
+    assert torch.equal(moe.forward(x), (x @ moe.Gate.W.t()).sum() + x) and not native
