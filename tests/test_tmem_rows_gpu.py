@@ -69,3 +69,10 @@ def test_small_matrices_of_9_to_64_rows(cuda, dt, M, N, K):
     y = ops.MatMulQ(x, q)
     assert torch.equal(y, ops.MatMulQ(x, q)) and ops.prefill_status(0) == 0
     assert rel_l2(y.cpu().double().numpy(), (x.double() @ ops.Dequantize(q).double().t()).cpu().numpy()) <= 1e-3
+
+
+@pytest.mark.parametrize("kind", ["q4_k", "q8_0", "int4", "fp8"])
+@pytest.mark.parametrize("M,N,K", [(70, 260, 256), (100, 4100, 768), (66, 18944, 1536), (66, 19200, 1536), (129, 9480, 768), (80, 2052, 2048)])
+def test_short_rows(cuda, kind, M, N, K):
+    """Tiles of fewer units than a run, of between one and two, and of two; as many as there are SMs (148), and one more."""
+    test_many_rows(cuda, kind, M, N, K)
