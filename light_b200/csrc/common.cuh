@@ -183,6 +183,8 @@ int gemm_tmem_status();
 int gguf_decode_tmem(int type, const float *x, const void *w, float *out, int M, int N, int K, void *ws, size_t ws_bytes, cudaStream_t st);
 int decode_tmem_status();
 size_t decode_nt_ws_bytes(int M, int K);
+// Blocks of 256 k to a run of the token-tile kernels on (tiles of 128 rows) x nb of them, where all runs are equal parts of a tile or equal numbers of whole ones; 0 where they are not
+int decode_nt_equal_run(long long blocks, int nb);
 int gguf_decode_nt(int type, const float *x, const void *const *w, float *const *out, const int *n, int count, int M, int K, void *ws,
                    size_t ws_bytes, cudaStream_t st);
 int decode_nt_status();

@@ -1052,22 +1052,34 @@ int int4_prefill(const void *x, const uint32_t *codes, const float *s, const flo
   return rc ? rc : 1;
 }
 
-// 17 to 64 bf16 rows of a 4-bit matrix: the tensor-memory kernel with the operands of the token-tile decode kernel (f16
+// 4 to 64 bf16 rows of a 4-bit matrix: the tensor-memory kernel with the operands of the token-tile decode kernel (f16
 // weights (code - zero) * scale, here with one rounding where that kernel rounds the scale as well; x as f16), bf16 out.
-// That kernel's instructions grow with the tokens, this one's do not.  Device time with a cold L2, 28672 x 4096: 32 rows
-// 51.9 -> 44.0 us, 64 rows 73.6 -> 46.3; 4096 x 14336: 36.8 -> 30.4, 46.1 -> 34.4; 2560 x 4096: 21.9 -> 19.5, 23.6 -> 21.5.
-// At 16 rows the two are even, and at 2048 x 4096 and below the token tiles are: hence the lines.
+// That kernel's instructions grow with the tokens, this one's do not.  us, the token tiles / here, a chain of calls with a cold L2:
+//   4 and 16 rows: 1024 x 1024 6.4, 6.8 / 5.5, 5.6, 4096 x 1024 7.1, 7.6 / 5.6, 5.7, 2048 x 4096 9.4, 10.5 / 8.7, 9.2, 4096 x 4096 12.3, 14.2 / 10.6, 10.9, 14336 x 4096 19.6, 22.4 / 18.5,
+//   18.4, 3584 x 18944 22.5, 25.3 / 19.8, 20.0, 37888 x 3584 27.3, 30.9 / 28.5, 28.6: so up to eight rows of the largest stay.
+//   32 and 64 rows: 1024 x 1024 8.0, 9.7 / 6.0, 6.3, 2048 x 2048 10.8, 12.5 / 8.6, 9.4, 1024 x 8192 15.3, 17.9 / 10.8, 12.4, 3072 x 3072 12.4, 13.7 / 9.2, 10.9.
+//   Rows of one block: 4096 x 256 3.6 / 4.4, 12288 x 256 3.9 / 5.7, 17 rows 4.3 / 5.8 (65536 x 256, 17 rows 14.5 / 11.4).
+// Up to 16 rows the token tiles stay ahead where all their runs are alike (decode_nt_equal_run) and
+//   a run is whole tiles: 12288 x 512 5.0 / 6.0, 32768 x 1024 9.8 / 14.8 (8192 x 512, a block to a run, 7.2 / 4.8);
+//   a run is one of seven blocks or more (up to 8 rows; above, of seven or eight): 2560 x 1792 7.4 / 8.2, 1024 x 3328 8.6 / 9.6 (3072 x 1536 7.4 / 7.3);
+//   up to 8 rows: runs of four of more than 592 blocks, rows of up to 16: 8192 x 4096 14.5 / 15.3 (3072 x 8192 14.9 / 14.5); runs of three of a long row whose blocks are no multiple of eight: 1792 x 6912 10.6 / 11.7
+//   (2048 x 6144 11.7 / 10.0).
 int int4_narrow_tmem(const void *x, const uint32_t *codes, const float *s, const float *z, void *y, int act_dtype, int M, int N, int K, int G, int device,
                      cudaStream_t st) {
   static const int min_m = getenv("LIGHT_B200_TMEM_INT4_MIN_M") ? atoi(getenv("LIGHT_B200_TMEM_INT4_MIN_M")) : 4;
-  // us, the token tiles / here, a chain of calls with a cold L2.  4 and 16 rows: 1024 x 1024 6.4, 6.8 / 5.5, 5.6, 4096 x 1024 7.1, 7.6 / 5.6, 5.7, 2048 x 4096 9.4, 10.5 / 8.7, 9.2, 4096 x
-  // 4096 12.3, 14.2 / 10.6, 10.9, 14336 x 4096 19.6, 22.4 / 18.5, 18.4, 3584 x 18944 22.5, 25.3 / 19.8, 20.0, 37888 x 3584 27.3, 30.9 / 28.5, 28.6: so up to eight rows of the
-  // largest stay.  32 and 64 rows: 1024 x 1024 8.0, 9.7 / 6.0, 6.3, 2048 x 2048 10.8, 12.5 / 8.6, 9.4, 1024 x 8192 15.3, 17.9 / 10.8, 12.4, 3072 x 3072 12.4, 13.7 / 9.2, 10.9.
   // Groups of 128 only, whose token-tile kernel rounds x to f16 as well: the kernel that has other groups multiplies bf16 x as it is,
   // and f16 would clamp values beyond 65504 and lose bits of those below 6e-5.
-  if (act_dtype != LB200_BF16 || M < min_m || M > 64 || (long long)N * K < (1ll << 20) || (M <= 8 && (long long)N * K >= (100ll << 20)) || K % 256 || G != 128 || ((uintptr_t)codes & 15) || ((uintptr_t)x & 15) ||
-      !use_tmem())
+  if (act_dtype != LB200_BF16 || M < min_m || M > 64 || (long long)N * K < (1ll << 20) || (M <= 8 && (long long)N * K >= (100ll << 20)) || K % 256 || G != 128 ||
+      ((uintptr_t)codes & 15) || ((uintptr_t)x & 15) || !use_tmem())
     return 0;
+  if (K == 256 && (M <= 16 || N < 40960)) return 0;
+  if (M <= 16) {
+    const int nb = K >> 8;
+    const long long blocks = (long long)((N + 127) / 128) * nb;
+    const int run = decode_nt_equal_run(blocks, nb);
+    if ((run == 1 && nb >= 7 && nb <= (M <= 8 ? 16 : 8)) || (run > 1 && nb <= run)) return 0;
+    if (M <= 8 && ((run == 4 && blocks > 4ll * sm_count() && nb <= 16) || (run == 3 && nb > 16 && nb % 8))) return 0;
+  }
   void *ws;
   size_t wsb;
   const size_t x_bytes = ((size_t)M * K * 2 + 1023) & ~(size_t)1023;
