@@ -81,4 +81,4 @@ def test_short_rows(cuda, kind, M, N, K):
 @pytest.mark.parametrize("M", [4, 8, 9, 16, 17])
 @pytest.mark.parametrize("N,K", [(4096, 256), (40960, 256), (12288, 512), (8192, 512), (2560, 1792), (3072, 1536), (1024, 2304), (8192, 4096), (1792, 6912)])
 def test_int4_on_both_sides_of_the_token_tiles(cuda, M, N, K):
-    test_few_rows_of_int4(cuda, N, K, M)
+    test_few_rows_of_int4(cuda, M, N, K)
