@@ -552,6 +552,12 @@ int run(const typename Row::Ctx &ctx, const float *x, float *out, int M, int N, 
 //     2048 x 4096 13.6 / 12.3, 2560 x 6656 20.6 / 18.8, 1536 x 16384 26.9 / 24.5, 28672 x 4096 65.2 / 33.2, 4096 x 14336 40.8 / 27.8.
 //     Q6_K 2048 x 8192 19.0 / 21.4, 2048 x 12288 24.2 / 24.6, but 1024 x 4096 14.8 / 11.0, 2048 x 2048 11.6 / 8.1, 2048 x 4096 13.6 / 12.0, 2560 x 6656 21.9 / 20.4, 2048 x 16384 30.7 /
 //     27.4, 4096 x 14336 43.2 / 26.5, 128256 x 4096 307 / 170 (4096 x 4096 17.1 / 15.6).
+// And where the token tiles' runs are all alike (decode_nt_equal_run) they stay ahead of this kernel, whose hand-overs then weigh more:
+//   Q6_K, 9 to 16 (12 rows): whole tiles 12800 x 512 5.9 / 6.1; runs of two, from 250 blocks on 1792 x 4608 10.3 / 11.6 (1536 x 4608, 216 blocks, 11.5 / 9.2); runs of three or four on up to 138
+//     CTAs 4096 x 3072 10.9 / 13.5, 2304 x 7168 13.4 / 15.7, 4096 x 4096 12.0 / 12.8 (140 CTAs: 2560 x 7168 17.0 / 16.0); beyond 592 blocks rows of 2, 4 or 12: 32768 x 1024 13.9 / 16.1, 12288 x
+//     3072 18.5 / 20.7 (3072 x 8192 18.0 / 15.6).
+//   33 to 64: whole tiles of three or four blocks: Q4_K 64 rows 15360 x 768 9.7 / 11.4, 16000 x 1024 12.3 / 13.3, Q6_K 16000 x 1024 13.6 / 15.0 (two: Q4_K 16384 x 512 1.17 times as fast here).
+//   Rows of one block on fewer tiles than SMs: Q4_K 8192 x 256, 33 rows 5.0 / 5.6.
 //   Q6_K, 17 to 32: 1024 x 3584 10.7 / 7.9, 2048 x 2048 10.7 / 6.9, 2048 x 5632 19.0 / 14.3, 4096 x 14336 31.1 / 21.9, 128256 x 4096 186 / 156.  9 to 16, but for
 //     tiles in more than nine parts (2048 x 5632 16.2 / 14.1, 2048 x 7168 14.5 / 15.6): 4096 x 1024 8.0 / 6.2, 2048 x 2048 8.5 / 6.8, 1024 x 4096 9.3 / 8.0, 2048 x 4096
 //     10.8 / 8.9, 3072 x 9216 19.0 / 18.3, 4096 x 10240 22.2 / 17.8.
@@ -566,6 +572,10 @@ int gguf_decode_tmem(int type, const float *x, const void *w, float *out, int M,
   if (q4 && M <= 16 && U < 4 * sms && 4 * tiles < sms) return 0;
   if (!q4 && M <= 16 && runs > 9 * tiles) return 0;
   if (M > 32 && U < (q4 ? 5 : 6) * sms && runs > 8 * tiles) return 0;
+  const int nb = K >> 8, equal = decode_nt_equal_run(U, nb);
+  if (!q4 && M <= 16 && equal >= 2 && (nb <= equal || (equal == 2 ? U >= 250 : U <= 138 * equal) || (U > 4 * sms && nb <= 16 && nb % 8))) return 0;
+  if (M > 32 && equal >= 3 && nb <= equal && U <= 4 * sms) return 0;
+  if (nb == 1 && tiles <= sms) return 0;
   if (q4 && !((uintptr_t)w & 15)) return run<ExQ4K>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);
   if (!q4 && TmQ6KT::fits(w, K)) return run<ExQ6K<TmQ6KT>>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);
   if (!q4 && !((uintptr_t)w & 3) && (K >> 8) % 2 == 0) return run<ExQ6K<TmQ6K>>({(const uint8_t *)w}, x, out, M, N, K, ws, ws_bytes, st);

@@ -82,3 +82,10 @@ def test_short_rows(cuda, kind, M, N, K):
 @pytest.mark.parametrize("N,K", [(4096, 256), (40960, 256), (12288, 512), (8192, 512), (2560, 1792), (3072, 1536), (1024, 2304), (8192, 4096), (1792, 6912)])
 def test_int4_on_both_sides_of_the_token_tiles(cuda, M, N, K):
     test_few_rows_of_int4(cuda, M, N, K)
+
+
+@pytest.mark.parametrize("dt,N,K", [(ops.Q6_K, 4096, 3072), (ops.Q6_K, 3072, 4096), (ops.Q6_K, 1536, 4608), (ops.Q6_K, 1792, 4608), (ops.Q6_K, 2304, 7168), (ops.Q6_K, 2560, 7168), (ops.Q6_K, 12800, 512),
+                                    (ops.Q6_K, 12288, 3072), (ops.Q4_K, 16000, 1024), (ops.Q4_K, 12800, 768), (ops.Q4_K, 16384, 512), (ops.Q4_K, 16384, 256), (ops.Q4_K, 19200, 256)])
+def test_whole_numbers_on_both_sides_of_the_token_tiles(cuda, dt, N, K):
+    for M in (12, 16, 48):
+        test_small_matrices_of_9_to_64_rows(cuda, dt, M, N, K)
