@@ -1992,14 +1992,25 @@ static int q4k_launch(const float *x, const MultiArgs &a, const TpArgs &tp, int 
 
 static const TpArgs NO_TP = {};
 
-int gguf_gemv_fast(int type, const float *x, const void *w, float *out, int M, int N, int K, cudaStream_t st) {
-  // No token-column kernel for Q8_0: a pass per row beats the tensor-core kernel up to three rows.  Nor for Q6_K rows of an odd number of blocks, where it
-  // beats the row kernel (us, that one / a pass per row): 4096 x 11008, 2, 3 and 8 rows 62, 68, 154 / 34, 50, 134, 3072 x 9984, 8 rows 123 / 119, 1024 x 3328, 2 and 3 rows 10.5, 12.6 /
-  // 9.2, 13.9, 2048 x 5888 20.7, 24.9 / 19.0, 28.5, 2048 x 768, 2 rows 4.0 / 5.4; limbs take 8 rows of 16384 x 1280 in 25 us, passes 66.
+// 2 to 8 rows of Q6_K with an odd number of blocks: a pass of the one-row kernel for each, or the row kernel (from 60000 outputs on limbs, which passes were not compared with but for
+// 16384 x 1280, 8 rows 66 / 25).  us, the row kernel / passes:
+//   2 rows from 3 Mi weights on, not rows of one block: 4096 x 11008 62 / 34, 1024 x 3328 10.6 / 9.4, 2048 x 768 4.0 / 5.4, 16384 x 256 8.0 / 9.9
+//   3 rows from 20 Mi on: 4096 x 11008 68 / 50, 2048 x 5888 24.9 / 28.5
+//   more, of rows of 4096 and more, by how many weight rows share the row kernel's loads: 4 rows 4096 x 5376 41 / 37, 3072 x 8960 54 / 57, 2304 x 9472 50 / 57; 6 rows 4096 x 5376 66 / 56,
+//   2560 x 9472 85 / 88, 2048 x 11008 71 / 95; 8 rows 4096 x 5376 77 / 74, 3328 x 8448 105 / 108, 2304 x 9472 70 / 114, 6144 x 5376 106 / 117, 6144 x 11008 212 / 218
+static bool odd_rows_by_passes(int M, int N, int K) {
   const long long size = (long long)N * K;
+  if (M == 2) return size >= (3ll << 20) && K > 256;
+  if (M > 8 || size < (20ll << 20) || (M > 3 && K < 4096)) return false;
+  if (M == 3 || (long long)M * N >= 60000) return true;
+  if (M == 8 && N >= 6000) return K >= 8192 && size >= (28ll << 20);
+  return N >= (M >= 5 && M <= 7 ? 2400 : 3500) || size >= (34ll << 20);
+}
+
+int gguf_gemv_fast(int type, const float *x, const void *w, float *out, int M, int N, int K, cudaStream_t st) {
+  // No token-column kernel for Q8_0: a pass per row beats the tensor-core kernel up to three rows.  Nor for Q6_K rows of an odd number of blocks.
   const bool odd = type == LB200_Q6_K && K % 512 == 256 && !((uintptr_t)w & 15);
-  const bool passes = type == LB200_Q8_0 ? M <= 3 : odd && (M == 2 ? size >= (3ll << 20) : size >= (20ll << 20) && (M == 3 || (M <= 8 && K >= 4096)));
-  if (M >= 2 && passes) {
+  if (M >= 2 && (type == LB200_Q8_0 ? M <= 3 : odd && odd_rows_by_passes(M, N, K))) {
     for (int m = 0; m < M; m++) {
       const int rc = gguf_gemv_fast(type, x + (size_t)m * K, w, out + (size_t)m * N, 1, N, K, st);
       if (rc != 1) return m == 0 ? rc : fail(rc < 0 ? rc : LB200_E_SHAPE, "light_b200: matmul_q (decode): row %d refused after row 0 was launched", m);

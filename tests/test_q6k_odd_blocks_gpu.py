@@ -134,3 +134,9 @@ def test_several_matrices_in_one_call(cuda, M):
     x = torch.randn(M, K, generator=torch.Generator(device=cuda).manual_seed(M), device=cuda)
     for y, w in zip(ops.MatMulQMulti(x, ws), ws):
         assert torch.equal(y, ops.MatMulQ(x, w))
+
+
+@pytest.mark.parametrize("M,N,K", [(2, 16384, 256), (2, 4096, 768), (3, 4096, 5376), (4, 3499, 6400), (4, 3500, 6400), (4, 3300, 11008), (5, 2399, 9472), (6, 2400, 9472), (8, 3500, 6400), (8, 6016, 3840),
+                                   (8, 6016, 4352), (8, 6016, 8448), (8, 7500, 4352), (8, 3400, 9472)])
+def test_both_sides_of_the_passes(cuda, M, N, K):
+    _check(cuda, M, N, K)
