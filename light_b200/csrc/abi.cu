@@ -170,9 +170,10 @@ unsigned long long light_b200_q6k_scratch_bytes(int t, const void *w, int64_t ro
   return q6k_limbs_bytes(rows, K);
 }
 
-// Of one matrix: as above, and from 60000 outputs on.  The row kernel takes 3.6e-7 us for each weight and activation row, limbs 3 to 5 us for each block of k, whose CTAs
+// Of one matrix: as above, and from 60000 outputs on (that hand gguf_gemv_fast.cu has no passes for).  The row kernel takes 3.6e-7 us for each weight and activation row, limbs 3 to 5 us for each block of k, whose CTAs
 // share out the outputs: 3072 x 9984, 33 and 64 rows 389, 722 / 157, 227 us, 4096 x 11008, 16 and 64 rows 283, 1056 / 219, 251, 2048 x 5888 33 rows 156 / 133, 1024 x 3328 64 rows
 // 87 / 76, 16384 x 1280, 4 and 16 rows 36, 126 / 25, 32; but 1024 x 3328, 33 and 50 rows 47, 68 / 53, 75, 3072 x 9984 9 rows 132 / 146 (16 rows 191 / 153).
+// Rows of one block too: 1024 to 65536 x 256, 9 to 64 rows, none slower.
 unsigned long long light_b200_matmul_q_scratch_bytes(int t, const void *w, int64_t M, int64_t N, int K) {
   if (M > 64) return light_b200_q6k_scratch_bytes(t, w, M, K, 0);
   if (t != LB200_Q6_K || M < 2 || N < 16 || M * N < 60000 || K <= 0 || K % 256 || ((K >> 8) % 2 == 0 && !((uintptr_t)w & 3))) return 0;

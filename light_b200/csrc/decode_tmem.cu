@@ -568,7 +568,7 @@ int gguf_decode_tmem(int type, const float *x, const void *w, float *out, int M,
   if ((!q4 && type != LB200_Q6_K) || M < min_m || M > MAX_NT || K % 256 || !ws || N < 128 || size >> 8 > 1ll << 30 || ((uintptr_t)x & 15)) return 0;
   const long long tiles = (N + 127) / 128, U = tiles * (K >> 8), sms = sm_count();
   const long long runs = U < 2 * sms ? U / 2 : sms;  // (as run() has them)
-  if (size < (q4 && M <= 32 ? 16ll : 2ll) << 20) return 0;  // (below 2 Mi a matrix is one of several that share x: the token tiles take those in one launch)
+  if (size < (q4 && M <= 32 ? 16ll : 2ll) << 20) return 0;  // (smaller matrices were not compared, nor below 16 Mi the cluster kernel's, which needs no workspace)
   if (q4 && M <= 16 && U < 4 * sms && 4 * tiles < sms) return 0;
   if (!q4 && M <= 16 && runs > 9 * tiles) return 0;
   if (M > 32 && U < (q4 ? 5 : 6) * sms && runs > 8 * tiles) return 0;
